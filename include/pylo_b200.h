@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define PYLO_B200_ABI_VERSION 10
+#define PYLO_B200_ABI_VERSION 11
 
 /* optimizer families (which feature set / network geometry a launch uses) */
 #define PYLO_FAM_ADAFAC 0 /* AdafacLO_CUDA, ELO_CUDA: 28+11 features, 39-32-32-2 */
@@ -48,7 +48,7 @@ extern "C" {
 #define PYLO_MODE_VEC1D 2   /* fewer than two dims: accumulators are full size ("vector_like") */
 
 #define PYLO_STAT_STRIDE 40  /* floats per tile partial / per tensor sums: 30 feature slots + 8 VeLO statistics */
-#define PYLO_TILE_ELEMS 16384 /* elements per element-wise tile */
+#define PYLO_TILE_ELEMS 16384 /* elements per element-wise tile (at most) */
 #define PYLO_A_COLS 1024      /* columns per row/column-sum tile */
 #define PYLO_WFOLD_STRIDE 2432 /* floats reserved per tensor for the folded network */
 #define PYLO_MAX_PEERS 7       /* other GPUs of one box */
@@ -113,11 +113,13 @@ typedef struct pylo_tensor_desc {
   int32_t pad_;
 } pylo_tensor_desc;
 
-/* a unit of element-wise work: elements [start, start + PYLO_TILE_ELEMS) of tensor `tensor` */
+/* a unit of element-wise work: elements [start, start + elems) of tensor `tensor`.  elems <= 0 means PYLO_TILE_ELEMS; a
+ * host with little work cuts it into smaller tiles (multiples of 4) so that they fill the GPU.  A tensor's tiles in the
+ * list given to pylo_b200_state_moments all have one size, and desc.tile0 / n_tiles / tile_part go with that list. */
 typedef struct pylo_tile {
   int64_t start;
   int32_t tensor;
-  int32_t pad_;
+  int32_t elems;
 } pylo_tile;
 
 /* a unit of row/column-sum work: rows [row0, row0+rb) x columns [col0, col0+PYLO_A_COLS) */
@@ -209,14 +211,12 @@ int pylo_b200_grad_sumsq_static(const pylo_gvec* items, const pylo_tile* tiles, 
 
 /* Phase A: row and column sums of g'^2 + 1e-30 (the reductions inside
  * grad_sqr.mean(dim=dr / dc), AdafacLO_cuda.py:333-340, CELO2_cuda.py:218-224, velo_cuda.py:531-541).
- * atiles cover the FAST2D tensors (strip x 1024-column block each; they leave per-strip column partials);
- * rtiles, one per (FAST2D tensor, 1024-column block), drive the second-level sum of those partials over the
- * strips; generic_ids lists the GENERIC tensors. */
+ * atiles cover the FAST2D tensors (strip x 1024-column block each; they leave per-strip column partials, which
+ * pylo_b200_factor_update adds up); generic_ids lists the GENERIC tensors. */
 int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles,
-                          const pylo_atile* rtiles, int n_rtiles, const int32_t* generic_ids, int n_generic,
-                          const pylo_step_params* prm, void* stream);
+                          const int32_t* generic_ids, int n_generic, const pylo_step_params* prm, void* stream);
 
-/* Phase A2, one CTA per tensor: EMA of the factored accumulators, row_col_mean,
+/* Phase A2, one cluster of CTAs per tensor: the sums over strips and column blocks of phase A's partials, EMA of the factored accumulators, row_col_mean,
  * row/column rsqrt factors (AdafacLO_cuda.py:342-345, CELO2_cuda.py:229-231, velo_cuda.py:716-729)
  * and the closed-form feature moments of the twelve vector-only features. */
 int pylo_b200_factor_update(const pylo_tensor_desc* descs, int n_tensors, const pylo_step_params* prm,
@@ -233,13 +233,16 @@ int pylo_b200_state_moments(const pylo_tensor_desc* descs, const pylo_tile* tile
 /* Phase B2, one CTA per tensor: fixed-order reduction of the tile partials into desc.sums. */
 int pylo_b200_finalize_moments(const pylo_tensor_desc* descs, int n_tensors, void* stream);
 
-/* Phase P, gridDim (n_tensors, slices): fold the normalisers rsqrt(S_j/n + eps) and, for
+/* Phase P: fold the normalisers rsqrt(S_j/n + eps) and, for
  * AdafacLO/ELO, the time features tanh(t/tau - 1) (learned_optimizer.cu:27-32,245-248) into the
- * first layer, and tabulate the first-layer contribution of the vector-only features.
+ * first layer, and tabulate the first-layer contribution of the vector-only features.  items: tensor = unit, strip =
+ * index of the unit's item.  Item 0 of every unit writes the folded network; with tables, an item also makes
+ * 8192 / H entries of a table: items 0 .. ceil(X / (8192/H)) - 1 the per-row one, the following ceil(Y / (8192/H)) the
+ * per-column one (FAST2D units; the others have item 0 only).
  * desc.w layouts: ADAFAC  w_in[32][39] b_in[32] w_h[32][32] b_h[32] w_out[2][32] b_out[2] (out-major);
  *                 CELO2   w_in[30][8]  b_in[8]  w_h[8][8]   b_h[8]  w_out[8][3]  b_out[3] (in-major);
  *                 VELO    w_in[4][30]  b_in[4]  w_h[4][4]   b_h[4]  w_out[3][4]  b_out[3] (out-major). */
-int pylo_b200_prep_apply(const pylo_tensor_desc* descs, int n_tensors, const pylo_step_params* prm,
+int pylo_b200_prep_apply(const pylo_tensor_desc* descs, const pylo_atile* items, int n_items, const pylo_step_params* prm,
                          void* stream);
 
 /* Phase C: rebuild the features, run the network, write the parameter (ADAFAC, VELO) or the raw

@@ -15,8 +15,9 @@ STAT_STRIDE = 40
 SUMS_STRIDE = 48
 TILE_ELEMS = 16384
 A_COLS = 1024
+PREP_TABLE = 8192  # table entries (rows x hidden units) per item of pylo_b200_prep_apply
 WFOLD_STRIDE = 2432
-ABI_VERSION = 10
+ABI_VERSION = 11
 
 FAM_ADAFAC, FAM_CELO2, FAM_VELO = 0, 1, 2
 MODE_FAST2D, MODE_GENERIC, MODE_VEC1D = 0, 1, 2
@@ -36,7 +37,7 @@ DESC_DTYPE = np.dtype(
     + [(name, np.float32) for name in ("lr", "wd", "step", "clip_norm", "exp_mult", "step_mult")]
     + [("n_peer", np.int32), ("pad_", np.int32)]
 )
-TILE_DTYPE = np.dtype([("start", np.int64), ("tensor", np.int32), ("pad_", np.int32)])
+TILE_DTYPE = np.dtype([("start", np.int64), ("tensor", np.int32), ("elems", np.int32)])
 ATILE_DTYPE = np.dtype([("tensor", np.int32), ("strip", np.int32), ("cb", np.int32), ("pad_", np.int32)])
 GVEC_DTYPE = np.dtype([("g", np.uint64), ("n", np.int64)])
 POST_DTYPE = np.dtype(
@@ -104,11 +105,11 @@ def _load():
         "pylo_b200_workspace_bytes": [C.POINTER(WsLayout), i32, i32],
         "pylo_b200_grad_sumsq": [vp, vp, i32, vp, vp, vp],
         "pylo_b200_grad_sumsq_static": [vp, vp, i32, vp, vp],
-        "pylo_b200_rowcol_sums": [vp, vp, i32, vp, i32, vp, i32, C.POINTER(StepParams), vp],
+        "pylo_b200_rowcol_sums": [vp, vp, i32, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_factor_update": [vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_state_moments": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_finalize_moments": [vp, i32, vp],
-        "pylo_b200_prep_apply": [vp, i32, C.POINTER(StepParams), vp],
+        "pylo_b200_prep_apply": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply_adafac_cols": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply_adafac_tc": [vp, vp, i32, C.POINTER(StepParams), vp, vp],
@@ -136,7 +137,8 @@ def _load():
 lib, EXPORTED = _load()
 
 
-TC_WORKERS = 148 * 4  # warpgroups the tensor-core apply kernel runs at once (four per SM)
+SM_COUNT = 148        # of a B200; sizes of work lists only, the kernels ask the device
+TC_WORKERS = SM_COUNT * 4  # warpgroups the tensor-core apply kernel runs at once (four per SM)
 STATIC_SCRATCH_TILES = 65536
 ERR_STATIC_SCRATCH_TOO_SMALL = -4
 

@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
     const float gs = grad_scale_of(d, prm);
     const Fin fin{d.exp_mult, d.step_mult, d.wd, d.lr, d.wfold[L::SC + 1], 1.0f, prm.wd_mode};
     // no clipping, no nan_to_num, no global-norm scale (AdafacLO's defaults): the gradient is used as it is
-    const bool plain_grad = !prm.nan_to_num && prm.clip_val == CUDART_INF_F && gs == 1.0f;
+    const bool plain = plain_grad(gs, prm);
     const float fb0 = d.f_b[yc], fb1 = d.f_b[Y + yc], fb2 = d.f_b[2 * (int64_t)Y + yc];
     // the six features of this thread's column, high parts (then two ones) and low parts (then two zeros)
     uint32_t chi[8], clo[8];
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
       TC_CLK(9)  // bias vector written
       // ---- operand A of the first layer, high and low parts
       {
-        const float g = plain_grad ? cg : xform_grad(cg, gs, prm.clip_val, prm.nan_to_num);
+        const float g = plain ? cg : xform_grad(cg, gs, prm.clip_val, prm.nan_to_num);
         const float rs = rsqrt_pos(cv + prm.eps_feat);
         const float k0 = cfa.x * fb0, k1 = cfa.y * fb1, k2 = cfa.z * fb2;
         const float fe[16] = {g, cp, cm0, cm1, cm2, cv, cm0 * rs, cm1 * rs, cm2 * rs, rs,

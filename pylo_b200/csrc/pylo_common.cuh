@@ -13,6 +13,7 @@
 #define NWARP (NT / 32)
 #define SUMS_LO 38             // desc.sums: [0,30) feature sums, [30,38) VeLO statistics, [38,46) their low parts
 #define SUMS_STRIDE 48
+#define PYLO_A_ROWS_MAX 128    // rows of a row/column-sum strip
 
 // ----------------------------------------------------------------------------------------------
 // family traits: feature counts and where the twelve vector-only features sit in reference order
@@ -100,6 +101,17 @@ __device__ __forceinline__ float xform_grad(float g, float gs, float clip, int n
     else if (isinf(g)) g = g > 0 ? 3.4028234663852886e38f : -3.4028234663852886e38f;
   }
   return (g != g) ? g : fminf(fmaxf(g, -clip), clip);
+}
+
+// whether xform_grad changes nothing: no global-norm scale, no nan_to_num, no clamp (AdafacLO's defaults)
+__device__ __forceinline__ bool plain_grad(float gs, const pylo_step_params& prm) {
+  return !prm.nan_to_num && prm.clip_val == CUDART_INF_F && gs == 1.0f;
+}
+
+// elements of a tile of a tensor (or item) of n elements
+__device__ __forceinline__ int tile_count(const pylo_tile& t, int64_t n) {
+  const int64_t most = t.elems > 0 ? t.elems : PYLO_TILE_ELEMS, left = n - t.start;
+  return (int)(left < most ? left : most);
 }
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }

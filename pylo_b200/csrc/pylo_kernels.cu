@@ -52,8 +52,7 @@ __global__ void __launch_bounds__(NT) k_grad_sumsq(const pylo_gvec* __restrict__
   for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const pylo_tile tl = tiles[t];
     const float* g = descs[tl.tensor].g + tl.start;
-    const int64_t rem = descs[tl.tensor].n - tl.start;
-    const int cnt = rem < PYLO_TILE_ELEMS ? (int)rem : PYLO_TILE_ELEMS;
+    const int cnt = tile_count(tl, descs[tl.tensor].n);
     float acc = 0.f;
     if ((((uintptr_t)g) & 15) == 0) {
       const int c4 = cnt & ~3;
@@ -87,11 +86,17 @@ __global__ void __launch_bounds__(1024) k_sum_final(const float* __restrict__ sc
 // ================================================================================================
 // Phase A: row / column sums of g'^2 + 1e-30
 // ================================================================================================
-__global__ void __launch_bounds__(NT) k_rowcol_fast(const pylo_tensor_desc* __restrict__ descs,
-                                                    const pylo_atile* __restrict__ atiles, int n_atiles,
-                                                    const pylo_step_params prm) {
-  __shared__ float s_col[NWARP][PYLO_A_COLS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// Bound by HBM.  Of the CTA's eight warps, four pairs take every fourth row of the strip and the warps of a pair one half
+// (512 columns) of the block each, so that a lane keeps 16 column accumulators (not 32) and has room to request its next
+// row before it adds up the present one: the loads of the next row fly during the shuffles of this one's row sum.
+// 355 M elements (GPT-2-medium shapes): 417 us before (a warp per row, 32 accumulators, no row ahead).
+#define RC_GROUPS 4
+__global__ void __launch_bounds__(NT, 4) k_rowcol_fast(const pylo_tensor_desc* __restrict__ descs,
+                                                       const pylo_atile* __restrict__ atiles, int n_atiles,
+                                                       const pylo_step_params prm) {
+  __shared__ float s_col[RC_GROUPS][PYLO_A_COLS];
+  __shared__ float s_row[PYLO_A_ROWS_MAX][2];
+  const int lane = threadIdx.x & 31, half = (threadIdx.x >> 5) & 1, grp = threadIdx.x >> 6;
   for (int t = blockIdx.x; t < n_atiles; t += gridDim.x) {
     const pylo_atile at = atiles[t];
     const pylo_tensor_desc& d = descs[at.tensor];
@@ -100,74 +105,58 @@ __global__ void __launch_bounds__(NT) k_rowcol_fast(const pylo_tensor_desc* __re
     const int rows = min(rb, X - row0);
     const int col0 = at.cb * PYLO_A_COLS;
     const float gs = grad_scale_of(d, prm);
-    float colacc[32];
+    const bool plain = plain_grad(gs, prm);
+    const int c0 = half * 512 + lane * 4;
+    const float* base = d.g + (int64_t)row0 * Y + col0 + c0;
+    const int left = Y - col0 - c0;   // columns of this lane's pieces that exist: piece j is there if j * 128 < left
+    float colacc[16];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) colacc[j] = 0.f;
-    for (int r = warp; r < rows; r += NWARP) {
-      const int x = row0 + r;
-      const float* grow = d.g + (int64_t)x * Y + col0;
+    for (int j = 0; j < 16; ++j) colacc[j] = 0.f;
+    float4 cur[4], nxt[4];
+    auto load = [&](int r, float4 (&q)[4]) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j * 128 < left) q[j] = ldg4(base + (int64_t)r * Y + j * 128);
+    };
+    if (grp < rows) load(grp, cur);
+    for (int r = grp; r < rows; r += RC_GROUPS) {
+      if (r + RC_GROUPS < rows) load(r + RC_GROUPS, nxt);
       float rowsum = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int c = lane * 4 + j * 128;
-        if (col0 + c < Y) {
-          const float4 q = ldg4(grow + c);
-          const float e[4] = {q.x, q.y, q.z, q.w};
+      for (int j = 0; j < 4; ++j) {
+        if (j * 128 < left) {
+          const float e[4] = {cur[j].x, cur[j].y, cur[j].z, cur[j].w};
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            const float g = xform_grad(e[u], gs, prm.clip_val, prm.nan_to_num);
-            const float s = g * g + 1e-30f;
-            colacc[j * 4 + u] += s;
-            rowsum += s;
+            const float g = plain ? e[u] : xform_grad(e[u], gs, prm.clip_val, prm.nan_to_num);
+            const float q = g * g + 1e-30f;
+            colacc[j * 4 + u] += q;
+            rowsum += q;
           }
         }
       }
       rowsum = warp_sum(rowsum);
-      if (lane == 0) d.part_a[(int64_t)x * d.n_cb + at.cb] = rowsum;
+      if (lane == 0) s_row[r][half] = rowsum;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cur[j] = nxt[j];
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) st4(&s_col[warp][lane * 4 + j * 128], make_float4(colacc[j * 4], colacc[j * 4 + 1], colacc[j * 4 + 2], colacc[j * 4 + 3]));
+    for (int j = 0; j < 4; ++j) st4(&s_col[grp][c0 + j * 128], make_float4(colacc[j * 4], colacc[j * 4 + 1], colacc[j * 4 + 2], colacc[j * 4 + 3]));
     __syncthreads();
     {
       const int c = threadIdx.x * 4;
       if (col0 + c < Y) {
         float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int w = 0; w < NWARP; ++w) {
+        for (int w = 0; w < RC_GROUPS; ++w) {
           const float4 q = ld4(&s_col[w][c]);
           tot.x += q.x; tot.y += q.y; tot.z += q.z; tot.w += q.w;
         }
         st4(d.part_b + (int64_t)at.strip * Y + col0 + c, tot);
       }
+      if (threadIdx.x < rows) d.part_a[(int64_t)(row0 + threadIdx.x) * d.n_cb + at.cb] = s_row[threadIdx.x][0] + s_row[threadIdx.x][1];
     }
     __syncthreads();
-  }
-}
-
-// Second level of the column sums: sum_b[y] = sum over strips of part_b[strip][y], strips in order.
-// One work item = 1024 columns of one tensor; a thread owns a float4 of columns.
-__global__ void __launch_bounds__(NT) k_colpart_reduce(const pylo_tensor_desc* __restrict__ descs,
-                                                       const pylo_atile* __restrict__ rtiles, int n_rtiles) {
-  for (int t = blockIdx.x; t < n_rtiles; t += gridDim.x) {
-    const pylo_atile rt = rtiles[t];
-    const pylo_tensor_desc& d = descs[rt.tensor];
-    const int Y = d.Y, strips = d.n_strips;
-    const int y = rt.cb * PYLO_A_COLS + threadIdx.x * 4;
-    if (y >= Y) continue;
-    const float* __restrict__ src = d.part_b + y;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    int r = 0;
-    for (; r + 4 <= strips; r += 4) {  // four loads in flight, added in strip order
-      const float4 q0 = ld4(src + (int64_t)r * Y), q1 = ld4(src + (int64_t)(r + 1) * Y);
-      const float4 q2 = ld4(src + (int64_t)(r + 2) * Y), q3 = ld4(src + (int64_t)(r + 3) * Y);
-      acc.x = (((acc.x + q0.x) + q1.x) + q2.x) + q3.x; acc.y = (((acc.y + q0.y) + q1.y) + q2.y) + q3.y;
-      acc.z = (((acc.z + q0.z) + q1.z) + q2.z) + q3.z; acc.w = (((acc.w + q0.w) + q1.w) + q2.w) + q3.w;
-    }
-    for (; r < strips; ++r) {
-      const float4 q = ld4(src + (int64_t)r * Y);
-      acc.x += q.x; acc.y += q.y; acc.z += q.z; acc.w += q.w;
-    }
-    st4(d.sum_b + y, acc);
   }
 }
 
@@ -213,122 +202,182 @@ __global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* _
 }
 
 // ================================================================================================
-// Phase A2: factored accumulators, factors, closed-form vector-feature moments.  One CTA per tensor.
+// Phase A2: factored accumulators, factors, closed-form vector-feature moments.  One cluster of eight CTAs per tensor.
+//
+// Latency-bound: a tensor's vectors are a few ten thousand entries, but every column's sum runs over all strips of phase
+// A and the factors need the mean of the whole vector.  Eight CTAs share the tensor (one CTA took 185 us for the 50257
+// rows of a GPT-2 embedding) and exchange their partial sums through distributed shared memory; every CTA adds the eight
+// in rank order, so the result does not depend on timing.  The sum over the strips is part of this kernel: 128 columns
+// per pass, the strips dealt to eight groups of 128 threads.
 // ================================================================================================
 #define A2_NT 1024
+#define A2_CL 8
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// all threads of all CTAs of the cluster; orders shared, distributed shared and global memory accesses
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_store(float* p, uint32_t rank, float v) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+
 template <int FAM>
-__global__ void __launch_bounds__(A2_NT) k_factor_update(const pylo_tensor_desc* __restrict__ descs,
-                                                         const pylo_step_params prm) {
+__global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_factor_update(const pylo_tensor_desc* __restrict__ descs,
+                                                                                          const pylo_step_params prm) {
   using F = Fam<FAM>;
-  __shared__ float s_red[40];
-  __shared__ float s_mean[8];
-  const pylo_tensor_desc& d = descs[blockIdx.x];
-  const int tid = threadIdx.x;
-  if (tid < PYLO_STAT_STRIDE) d.closed[tid] = 0.f;
-  if (d.mode == PYLO_MODE_VEC1D) return;
-  const int64_t X = d.X, Y = d.Y;
+  constexpr int NS = 15;  // sums per CTA: row accumulator (its mean), then the four closed forms, three decays each
+  __shared__ float s_part[A2_NT / 128][128];
+  __shared__ float s_warp[A2_NT / 32][NS];
+  __shared__ float s_cta[A2_CL][NS + 1];
+  __shared__ float s_tot[NS + 1];
+  const pylo_tensor_desc& d = descs[blockIdx.x / A2_CL];
+  const int tid = threadIdx.x, rank = (int)cluster_rank();
+  if (d.mode == PYLO_MODE_VEC1D) {  // the same for all CTAs of the cluster
+    if (rank == 0 && tid < PYLO_STAT_STRIDE) d.closed[tid] = 0.f;
+    return;
+  }
+  const bool fast = d.mode == PYLO_MODE_FAST2D, r_is_a = d.r_is_a != 0;
   const int64_t La = d.La, Lb = d.Lb;
-
-  // 1. finish the row/column sums of the float4 path
-  if (d.mode == PYLO_MODE_FAST2D) {
-    for (int64_t x = tid; x < X; x += A2_NT) {
-      float s = 0.f;
-      for (int c = 0; c < d.n_cb; ++c) s += d.part_a[x * d.n_cb + c];
-      d.sum_a[x] = s;
-    }
-    // the column sums were finished by k_colpart_reduce
-  }
-  __syncthreads();
-
-  // 2. EMA of the two accumulators: lerp(acc, mean, 1 - beta_fac[k])
-  for (int64_t i = tid; i < La; i += A2_NT) {
-    const float mean = d.sum_a[i] / (float)Y;
+  const float inv_n_a = (float)d.Y, inv_n_b = (float)d.X;
+  float acc[NS];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) d.fac_a[k * La + i] = lerp_torch(d.fac_a[k * La + i], mean, prm.w_f[k]);
-  }
-  for (int64_t i = tid; i < Lb; i += A2_NT) {
-    const float mean = d.sum_b[i] / (float)X;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) d.fac_b[k * Lb + i] = lerp_torch(d.fac_b[k * Lb + i], mean, prm.w_f[k]);
-  }
-  __syncthreads();
+  for (int j = 0; j < NS; ++j) acc[j] = 0.f;
+  auto add = [&](bool is_r, int k, float v) {
+    const float q = rsqrtf(v + 1e-8f);
+    if (is_r) { acc[k] += v; acc[3 + k] = fmaf(v, v, acc[3 + k]); acc[6 + k] = fmaf(q, q, acc[6 + k]); }
+    else { acc[9 + k] = fmaf(v, v, acc[9 + k]); acc[12 + k] = fmaf(q, q, acc[12 + k]); }
+  };
 
-  // 3. row_factor = safe_rsqrt(fac_r / (mean over the reduce axis + 1e-9)), col_factor = safe_rsqrt(fac_c)
-  const float* fac_r = d.r_is_a ? d.fac_a : d.fac_b;
-  const float* fac_c = d.r_is_a ? d.fac_b : d.fac_a;
-  float* f_r = d.r_is_a ? d.f_a : d.f_b;
-  float* f_c = d.r_is_a ? d.f_b : d.f_a;
-  const int64_t Lr = d.r_is_a ? La : Lb, Lc = d.r_is_a ? Lb : La;
-  const int64_t pre = d.rcm_pre, A = d.rcm_A, post = d.rcm_post;
-  if (post == 1 && pre <= 8) {
-    for (int pr = 0; pr < pre; ++pr) {
-      float acc = 0.f;
-      for (int64_t a = tid; a < A; a += A2_NT) acc += fac_r[pr * A + a];
-      const float tot = block_sum(acc, s_red);
-      if (tid == 0) s_mean[pr] = tot / (float)A;
+  // 1. "a" vectors: finish the row sums, EMA of the accumulator lerp(acc, mean, 1 - beta_fac[k])
+  const int gtid = rank * A2_NT + tid;
+  for (int64_t i = gtid; i < La; i += A2_CL * A2_NT) {
+    float s;
+    if (fast) {
+      s = 0.f;
+      for (int c = 0; c < d.n_cb; ++c) s += d.part_a[i * d.n_cb + c];
+      d.sum_a[i] = s;
+    } else {
+      s = d.sum_a[i];
     }
-    __syncthreads();
-    for (int64_t e = tid; e < 3 * Lr; e += A2_NT) f_r[e] = safe_rsqrt(fac_r[e] / (s_mean[e / A] + 1e-9f));
-  } else if (post == 1) {
-    const int lane = tid & 31;
-    for (int64_t pr = tid >> 5; pr < pre; pr += A2_NT / 32) {
-      float acc = 0.f;
-      for (int64_t a = lane; a < A; a += 32) acc += fac_r[pr * A + a];
-      acc = warp_sum(acc);
-      acc = __shfl_sync(0xffffffffu, acc, 0) / (float)A;
-      for (int64_t a = lane; a < A; a += 32) f_r[pr * A + a] = safe_rsqrt(fac_r[pr * A + a] / (acc + 1e-9f));
-    }
-  } else {
-    for (int64_t o = tid; o < pre * post; o += A2_NT) {
-      const int64_t pr = o / post, po = o % post;
-      float acc = 0.f;
-      for (int64_t a = 0; a < A; ++a) acc += fac_r[(pr * A + a) * post + po];
-      acc /= (float)A;
-      for (int64_t a = 0; a < A; ++a) {
-        const int64_t e = (pr * A + a) * post + po;
-        f_r[e] = safe_rsqrt(fac_r[e] / (acc + 1e-9f));
-      }
-    }
-  }
-  for (int64_t e = tid; e < 3 * Lc; e += A2_NT) f_c[e] = safe_rsqrt(fac_c[e]);
-  __syncthreads();
-
-  // 4. "a" factors interleaved per index for the float4 path
-  if (d.mode == PYLO_MODE_FAST2D) {
-    for (int64_t i = tid; i < La; i += A2_NT)
-      st4(d.fx + 4 * i, make_float4(d.f_a[i], d.f_a[La + i], d.f_a[2 * La + i], 0.f));
-  }
-
-  // 5. closed-form sums of squares of the features that depend on one vector only: every
-  //    vector entry is seen by n / L elements of the tensor.
-  {
-    const float mult_r = (float)(d.n / Lr), mult_c = (float)(d.n / Lc);
+    const float mean = s / inv_n_a;
+    float f[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      float s1 = 0.f, s2 = 0.f, s3 = 0.f, s4 = 0.f;
-      for (int64_t i = tid; i < Lr; i += A2_NT) {
-        const float r = fac_r[k * Lr + i];
-        s1 += r * r;
-        const float q = rsqrtf(r + 1e-8f);
-        s2 += q * q;
-      }
-      for (int64_t i = tid; i < Lc; i += A2_NT) {
-        const float c = fac_c[k * Lc + i];
-        s3 += c * c;
-        const float q = rsqrtf(c + 1e-8f);
-        s4 += q * q;
-      }
-      s1 = block_sum(s1, s_red);
-      s2 = block_sum(s2, s_red);
-      s3 = block_sum(s3, s_red);
-      s4 = block_sum(s4, s_red);
-      if (tid == 0) {
-        d.closed[F::R + k] = s1 * mult_r;
-        d.closed[F::RR + k] = s2 * mult_r;
-        d.closed[F::C + k] = s3 * mult_c;
-        d.closed[F::RC + k] = s4 * mult_c;
+      const float v = lerp_torch(d.fac_a[k * La + i], mean, prm.w_f[k]);
+      d.fac_a[k * La + i] = v;
+      add(r_is_a, k, v);
+      f[k] = safe_rsqrt(v);
+    }
+    if (!r_is_a) {  // col_factor = safe_rsqrt(fac_c)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) d.f_a[k * La + i] = f[k];
+      if (fast) st4(d.fx + 4 * i, make_float4(f[0], f[1], f[2], 0.f));
+    }
+  }
+  // 2. "b" vectors: sum over the strips (in a fixed order), EMA
+  for (int64_t c0 = (int64_t)rank * 128; c0 < Lb; c0 += A2_CL * 128) {
+    const int64_t i = c0 + (tid & 127);
+    float s = 0.f;
+    if (i < Lb) {
+      if (fast) {
+        const float* __restrict__ src = d.part_b + i;
+#pragma unroll 8
+        for (int r = tid >> 7; r < d.n_strips; r += A2_NT / 128) s += src[(int64_t)r * Lb];
+      } else if (tid < 128) {
+        s = d.sum_b[i];
       }
     }
+    s_part[tid >> 7][tid & 127] = s;
+    __syncthreads();
+    if (tid < 128 && i < Lb) {
+      s = 0.f;
+#pragma unroll
+      for (int w = 0; w < A2_NT / 128; ++w) s += s_part[w][tid];
+      if (fast) d.sum_b[i] = s;
+      const float mean = s / inv_n_b;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const float v = lerp_torch(d.fac_b[k * Lb + i], mean, prm.w_f[k]);
+        d.fac_b[k * Lb + i] = v;
+        add(!r_is_a, k, v);
+        if (r_is_a) d.f_b[k * Lb + i] = safe_rsqrt(v);
+      }
+    }
+    __syncthreads();
+  }
+  // 3. the fifteen sums over the tensor, in every CTA
+#pragma unroll
+  for (int j = 0; j < NS; ++j) {
+    const float v = warp_sum(acc[j]);
+    if ((tid & 31) == 0) s_warp[tid >> 5][j] = v;
+  }
+  __syncthreads();
+  if (tid < NS) {
+    float v = 0.f;
+    for (int w = 0; w < A2_NT / 32; ++w) v += s_warp[w][tid];
+    for (uint32_t q = 0; q < A2_CL; ++q) cluster_store(&s_cta[rank][tid], q, v);
+  }
+  cluster_sync();  // also: every CTA's accumulators are visible to the others
+  if (tid < NS) {
+    float v = 0.f;
+    for (int q = 0; q < A2_CL; ++q) v += s_cta[q][tid];
+    s_tot[tid] = v;
+  }
+  __syncthreads();
+
+  // 4. row_factor = safe_rsqrt(fac_r / (mean over the reduce axis + 1e-9))
+  const float* fac_r = r_is_a ? d.fac_a : d.fac_b;
+  float* f_r = r_is_a ? d.f_a : d.f_b;
+  const int64_t Lr = r_is_a ? La : Lb;
+  const int64_t pre = d.rcm_pre, A = d.rcm_A, post = d.rcm_post;
+  if ((pre == 3 && A == Lr) || (pre == 1 && A == 3 && post == Lr)) {
+    // the mean of each decay's whole vector, or (the decay axis is the reduce axis) of each entry's three decays
+    const bool whole = pre == 3 && A == Lr;
+    for (int64_t i = gtid; i < Lr; i += A2_CL * A2_NT) {
+      const float v0 = fac_r[i], v1 = fac_r[Lr + i], v2 = fac_r[2 * Lr + i];
+      const float own = (v0 + v1 + v2) / 3.0f;
+      const float f0 = safe_rsqrt(v0 / ((whole ? s_tot[0] / (float)A : own) + 1e-9f));
+      const float f1 = safe_rsqrt(v1 / ((whole ? s_tot[1] / (float)A : own) + 1e-9f));
+      const float f2 = safe_rsqrt(v2 / ((whole ? s_tot[2] / (float)A : own) + 1e-9f));
+      f_r[i] = f0; f_r[Lr + i] = f1; f_r[2 * Lr + i] = f2;
+      if (fast && r_is_a) st4(d.fx + 4 * i, make_float4(f0, f1, f2, 0.f));
+    }
+  } else if (post == 1) {
+    const int lane = tid & 31;
+    for (int64_t pr = gtid >> 5; pr < pre; pr += A2_CL * A2_NT / 32) {
+      float m = 0.f;
+      for (int64_t a = lane; a < A; a += 32) m += fac_r[pr * A + a];
+      m = __shfl_sync(0xffffffffu, warp_sum(m), 0) / (float)A;
+      for (int64_t a = lane; a < A; a += 32) f_r[pr * A + a] = safe_rsqrt(fac_r[pr * A + a] / (m + 1e-9f));
+    }
+  } else {
+    for (int64_t o = gtid; o < pre * post; o += A2_CL * A2_NT) {
+      const int64_t pr = o / post, po = o % post;
+      float m = 0.f;
+      for (int64_t a = 0; a < A; ++a) m += fac_r[(pr * A + a) * post + po];
+      m /= (float)A;
+      for (int64_t a = 0; a < A; ++a) {
+        const int64_t e = (pr * A + a) * post + po;
+        f_r[e] = safe_rsqrt(fac_r[e] / (m + 1e-9f));
+      }
+    }
+  }
+  // 5. closed-form sums of squares of the features that depend on one vector only: every vector entry is seen by
+  //    n / L elements of the tensor
+  if (rank == 0 && tid < PYLO_STAT_STRIDE) {
+    const float mult_r = (float)(d.n / Lr), mult_c = (float)(d.n / (r_is_a ? Lb : La));
+    float v = 0.f;
+    if (tid >= F::R && tid < F::R + 3) v = s_tot[3 + tid - F::R] * mult_r;
+    else if (tid >= F::RR && tid < F::RR + 3) v = s_tot[6 + tid - F::RR] * mult_r;
+    else if (tid >= F::C && tid < F::C + 3) v = s_tot[9 + tid - F::C] * mult_c;
+    else if (tid >= F::RC && tid < F::RC + 3) v = s_tot[12 + tid - F::RC] * mult_c;
+    d.closed[tid] = v;
   }
 }
 
@@ -372,7 +421,7 @@ __global__ void __launch_bounds__(NT) k_state_moments(const pylo_tensor_desc* __
     const pylo_tile tl = tiles[t];
     const pylo_tensor_desc& d = descs[tl.tensor];
     const int64_t n = d.n, start = tl.start;
-    const int cnt = (int)min((int64_t)PYLO_TILE_ELEMS, n - start);
+    const int cnt = tile_count(tl, n);
     const float gs = grad_scale_of(d, prm);
     float acc[NACC];
 #pragma unroll
@@ -486,17 +535,26 @@ __global__ void __launch_bounds__(NT) k_state_moments(const pylo_tensor_desc* __
 // ================================================================================================
 // Phase B2: per-tensor fixed-order reduction of the tile partials
 // ================================================================================================
-__global__ void __launch_bounds__(NT) k_finalize_moments(const pylo_tensor_desc* __restrict__ descs) {
-  __shared__ double s_d[4][64];
+// Latency-bound: a 58 M-element tensor leaves 3584 rows of 40 partials.  The rows are read as one stretch of memory, 25
+// (or six) at a time, every thread keeping its column; eight rows ahead are in flight.
+__global__ void __launch_bounds__(1024) k_finalize_moments(const pylo_tensor_desc* __restrict__ descs) {
+  __shared__ double s_d[25][PYLO_STAT_STRIDE];
   const pylo_tensor_desc& d = descs[blockIdx.x];
-  const int j = threadIdx.x & 63, sub = threadIdx.x >> 6;  // 4 sub-sequences of tiles x 64 columns
-  double acc = 0.0;
-  if (j < PYLO_STAT_STRIDE)
-    for (int t = sub; t < d.n_tiles; t += 4) acc += (double)d.tile_part[(int64_t)t * PYLO_STAT_STRIDE + j];
-  s_d[sub][j] = acc;
+  const int rows = blockDim.x / PYLO_STAT_STRIDE;
+  const int j = threadIdx.x % PYLO_STAT_STRIDE, sub = threadIdx.x / PYLO_STAT_STRIDE;
+  if (sub < rows) {
+    double acc = 0.0;
+    const float* __restrict__ src = d.tile_part + j;
+    const int n = d.n_tiles;
+#pragma unroll 8
+    for (int t = sub; t < n; t += rows) acc += (double)src[(int64_t)t * PYLO_STAT_STRIDE];
+    s_d[sub][j] = acc;
+  }
   __syncthreads();
   if (threadIdx.x < PYLO_STAT_STRIDE) {
-    const double tot = ((s_d[0][j] + s_d[1][j]) + s_d[2][j]) + s_d[3][j] + (double)d.closed[j];
+    double tot = 0.0;
+    for (int q = 0; q < rows; ++q) tot += s_d[q][j];
+    tot += (double)d.closed[j];
     const float hi = (float)tot;
     d.sums[j] = hi;
     if (j >= 30 && j < 38) d.sums[SUMS_LO + (j - 30)] = (float)(tot - (double)hi);
@@ -513,17 +571,22 @@ __device__ __forceinline__ float w1_at(int fam, const float* w, int j, int k) {
   return w[j * 30 + k];
 }
 
+// One work item is PREP_TABLE / H entries of a unit's "a" or "b" table (the "a" items first); item 0 of a unit also writes
+// the folded network.  Items are dealt by the tables' sizes, so that a 50257-row table is spread over the GPU (a fixed
+// number of CTAs per unit took 537 us for it).
+#define PREP_TABLE 8192
 template <int FAM>
 __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __restrict__ descs,
-                                                   const pylo_step_params prm) {
+                                                   const pylo_atile* __restrict__ items, const pylo_step_params prm) {
   using F = Fam<FAM>;
   using L = Fold<FAM>;
   constexpr int H = F::H, NF = F::NF, NIN = F::NIN;
   __shared__ float s_scale[NF];
   __shared__ float s_w1[NF * H];
   __shared__ float s_b1[H];
-  const pylo_tensor_desc& d = descs[blockIdx.x];
-  const int tid = threadIdx.x, slice = blockIdx.y, slices = gridDim.y;
+  const pylo_atile it = items[blockIdx.x];
+  const pylo_tensor_desc& d = descs[it.tensor];
+  const int tid = threadIdx.x;
   const float* w = d.w;
   // source offsets in the family layout
   const int o_b1 = NIN * H, o_w2 = o_b1 + H, o_b2 = o_w2 + H * H, o_w3 = o_b2 + H, o_b3 = o_w3 + H * F::NOUT;
@@ -543,7 +606,7 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
     s_b1[tid] = b;
   }
   __syncthreads();
-  if (slice == 0) {
+  if (it.strip == 0) {
     float* o = d.wfold;
     for (int e = tid; e < NF * H; e += NT) o[L::W1 + e] = s_w1[e];
     if (tid < H) o[L::B1 + tid] = s_b1[tid];
@@ -569,34 +632,41 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
   }
   if (d.mode != PYLO_MODE_FAST2D || prm.no_tables == 1) return;
   // first-layer contribution of the features that depend only on the "a" index (plus bias) / "b" index
-  const int64_t La = d.X, Lb = d.Y;
+  constexpr int PER = PREP_TABLE / H;
+  const int La = d.X, Lb = d.Y;
   const int ka = d.r_is_a ? F::R : F::C, kra = d.r_is_a ? F::RR : F::RC;
   const int kb = d.r_is_a ? F::C : F::R, krb = d.r_is_a ? F::RC : F::RR;
-  for (int64_t e = (int64_t)slice * NT + tid; e < La * H; e += (int64_t)slices * NT) {
-    const int64_t i = e / H;
-    const int j = (int)(e % H);
-    float acc = s_b1[j];
+  const int items_a = (La + PER - 1) / PER;
+  const int j = tid % H;
+  if (it.strip < items_a) {
+    const int end = min(La, (it.strip + 1) * PER);
+    for (int i = it.strip * PER + tid / H; i < end; i += NT / H) {
+      float acc = s_b1[j];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float r = d.fac_a[k * La + i];
-      acc = fmaf(s_w1[(ka + k) * H + j], r, acc);
-      acc = fmaf(s_w1[(kra + k) * H + j], rsqrtf(r + 1e-8f), acc);
+      for (int k = 0; k < 3; ++k) {
+        const float r = d.fac_a[k * (int64_t)La + i];
+        acc = fmaf(s_w1[(ka + k) * H + j], r, acc);
+        acc = fmaf(s_w1[(kra + k) * H + j], rsqrtf(r + 1e-8f), acc);
+      }
+      const int64_t e = (int64_t)i * H + j;
+      if (FAM == PYLO_FAM_ADAFAC) d.h_a[e] = acc;
+      else { d.h_a[2 * e] = acc; d.h_a[2 * e + 1] = acc; }  // stored as (v, v) pairs for the packed kernel
     }
-    if (FAM == PYLO_FAM_ADAFAC) d.h_a[e] = acc;
-    else { d.h_a[2 * e] = acc; d.h_a[2 * e + 1] = acc; }  // stored as (v, v) pairs for the packed kernel
+    return;
   }
   if (prm.no_tables == 2) return;  // the per-row table only
-  for (int64_t e = (int64_t)slice * NT + tid; e < Lb * H; e += (int64_t)slices * NT) {
-    const int64_t i = e / H;
-    const int j = (int)(e % H);
+  const int i0 = (it.strip - items_a) * PER, end = min(Lb, i0 + PER);
+  for (int e = tid; e < PER * H; e += NT) {  // stored transposed, [H][Y]: a thread of the apply sweep reads its columns' terms with one float4
+    const int i = i0 + e % PER, jj = e / PER;
+    if (i >= end) continue;
     float acc = 0.f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float r = d.fac_b[k * Lb + i];
-      acc = fmaf(s_w1[(kb + k) * H + j], r, acc);
-      acc = fmaf(s_w1[(krb + k) * H + j], rsqrtf(r + 1e-8f), acc);
+      const float r = d.fac_b[k * (int64_t)Lb + i];
+      acc = fmaf(s_w1[(kb + k) * H + jj], r, acc);
+      acc = fmaf(s_w1[(krb + k) * H + jj], rsqrtf(r + 1e-8f), acc);
     }
-    d.h_b[(int64_t)j * Lb + i] = acc;  // transposed, [H][Y]: a thread reads its columns' terms with one float4
+    d.h_b[(int64_t)jj * Lb + i] = acc;
   }
 }
 
@@ -739,7 +809,7 @@ __global__ void __launch_bounds__(NT) k_apply(const pylo_tensor_desc* __restrict
       __syncthreads();
     }
     const int64_t n = d.n, start = tl.start;
-    const int cnt = (int)min((int64_t)PYLO_TILE_ELEMS, n - start);
+    const int cnt = tile_count(tl, n);
     const float gs = grad_scale_of(d, prm);
     const Fin fin = make_fin(d, s_w[L::SC], s_w[L::SC + 1], prm.wd_mode);
     const Peers peers = load_peers(d);
@@ -1276,7 +1346,7 @@ __global__ void __launch_bounds__(NT) k_post_sums(const pylo_post_item* __restri
     const pylo_tile tl = tiles[t];
     const pylo_post_item& it = items[tl.tensor];
     const float* s = it.step + tl.start;
-    const int cnt = (int)min((int64_t)PYLO_TILE_ELEMS, it.n - tl.start);
+    const int cnt = tile_count(tl, it.n);
     float acc = 0.f;
     if (((((uintptr_t)s) & 15) == 0)) {
       const int c4 = cnt & ~3;
@@ -1310,7 +1380,7 @@ __global__ void __launch_bounds__(NT) k_post_apply(const pylo_post_item* __restr
     const float sc = s_scale, lr = it.lr, wd = it.wd;
     const float* s = it.step + tl.start;
     float* p = it.p + tl.start;
-    const int cnt = (int)min((int64_t)PYLO_TILE_ELEMS, it.n - tl.start);
+    const int cnt = tile_count(tl, it.n);
     const bool al = (((((uintptr_t)s) | ((uintptr_t)p)) & 15) == 0);
     const int c4 = al ? (cnt & ~3) : 0;
     for (int i = threadIdx.x * 4; i < c4; i += NT * 4) {
@@ -1337,7 +1407,7 @@ __global__ void __launch_bounds__(NT) k_adamw(const pylo_adam_item* __restrict__
     const pylo_tile tl = tiles[t];
     const pylo_adam_item& it = items[tl.tensor];
     const int64_t n = it.n;
-    const int cnt = (int)min((int64_t)PYLO_TILE_ELEMS, n - tl.start);
+    const int cnt = tile_count(tl, n);
     float gs = 1.0f;
     if (it.clip_norm > 0.f && prm.gnorm_sq) {
       const float denom = fmaxf(sqrtf(*prm.gnorm_sq), it.clip_norm);
@@ -1626,8 +1696,10 @@ int pylo_b200_workspace_layout(int family, int mode, int64_t n, int64_t La, int6
   }
   if (mode == PYLO_MODE_FAST2D) {
     CHECK_ARG(X > 0 && Y > 0 && Y % 4 == 0 && La == X && Lb == Y);
-    int rb = (((X + 127) / 128 + 7) / 8) * 8;  // rows per strip: about X / 128, a multiple of 8, within [32, 128]
-    rb = rb < 32 ? 32 : (rb > 128 ? 128 : rb);
+    // rows per strip: about X / 128, a multiple of 8, within [32, 128].  Up to 512 rows a tensor gives too few strips of
+    // 32 to fill the GPU and the launch is all latency: strips of 8 (one or two rows per warp) there.
+    int rb = (((X + 127) / 128 + 7) / 8) * 8;
+    rb = X <= 512 ? 8 : (rb < 32 ? 32 : (rb > PYLO_A_ROWS_MAX ? PYLO_A_ROWS_MAX : rb));
     w.rb = rb;
     w.n_strips = (X + rb - 1) / rb;
     w.n_cb = (Y + PYLO_A_COLS - 1) / PYLO_A_COLS;
@@ -1717,14 +1789,12 @@ int pylo_b200_grad_sumsq_static(const pylo_gvec* items, const pylo_tile* tiles, 
 }
 
 int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles,
-                          const pylo_atile* rtiles, int n_rtiles, const int32_t* generic_ids, int n_generic,
-                          const pylo_step_params* prm, void* stream) {
-  CHECK_ARG(descs && prm && n_atiles >= 0 && n_rtiles >= 0 && n_generic >= 0);
+                          const int32_t* generic_ids, int n_generic, const pylo_step_params* prm, void* stream) {
+  CHECK_ARG(descs && prm && n_atiles >= 0 && n_generic >= 0);
   cudaStream_t s = (cudaStream_t)stream;
   if (n_atiles > 0) {
-    CHECK_ARG(atiles && rtiles && n_rtiles > 0);
+    CHECK_ARG(atiles);
     k_rowcol_fast<<<grid_for(n_atiles, 4), NT, 0, s>>>(descs, atiles, n_atiles, *prm);
-    k_colpart_reduce<<<grid_for(n_rtiles, 8), NT, 0, s>>>(descs, rtiles, n_rtiles);
   }
   if (n_generic > 0) {
     CHECK_ARG(generic_ids);
@@ -1738,9 +1808,9 @@ int pylo_b200_factor_update(const pylo_tensor_desc* descs, int n_tensors, const 
   if (n_tensors == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: k_factor_update<PYLO_FAM_ADAFAC><<<n_tensors, A2_NT, 0, s>>>(descs, *prm); break;
-    case PYLO_FAM_CELO2: k_factor_update<PYLO_FAM_CELO2><<<n_tensors, A2_NT, 0, s>>>(descs, *prm); break;
-    case PYLO_FAM_VELO: k_factor_update<PYLO_FAM_VELO><<<n_tensors, A2_NT, 0, s>>>(descs, *prm); break;
+    case PYLO_FAM_ADAFAC: k_factor_update<PYLO_FAM_ADAFAC><<<n_tensors * A2_CL, A2_NT, 0, s>>>(descs, *prm); break;
+    case PYLO_FAM_CELO2: k_factor_update<PYLO_FAM_CELO2><<<n_tensors * A2_CL, A2_NT, 0, s>>>(descs, *prm); break;
+    case PYLO_FAM_VELO: k_factor_update<PYLO_FAM_VELO><<<n_tensors * A2_CL, A2_NT, 0, s>>>(descs, *prm); break;
     default: return -2;
   }
   return launch_status();
@@ -1764,20 +1834,20 @@ int pylo_b200_state_moments(const pylo_tensor_desc* descs, const pylo_tile* tile
 int pylo_b200_finalize_moments(const pylo_tensor_desc* descs, int n_tensors, void* stream) {
   CHECK_ARG(descs && n_tensors >= 0);
   if (n_tensors == 0) return 0;
-  k_finalize_moments<<<n_tensors, NT, 0, (cudaStream_t)stream>>>(descs);
+  // many units (the slices of a CELO2 tensor) have few tiles each: small CTAs then
+  k_finalize_moments<<<n_tensors, n_tensors > 512 ? 6 * PYLO_STAT_STRIDE : 25 * PYLO_STAT_STRIDE, 0, (cudaStream_t)stream>>>(descs);
   return launch_status();
 }
 
-int pylo_b200_prep_apply(const pylo_tensor_desc* descs, int n_tensors, const pylo_step_params* prm, void* stream) {
-  CHECK_ARG(descs && prm && n_tensors >= 0);
-  if (n_tensors == 0) return 0;
+int pylo_b200_prep_apply(const pylo_tensor_desc* descs, const pylo_atile* items, int n_items, const pylo_step_params* prm,
+                         void* stream) {
+  CHECK_ARG(descs && items && prm && n_items >= 0);
+  if (n_items == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
-  // the table loops stride over grid.y slices; with few tensors in a launch the slices are what fills the GPU
-  const dim3 grid(n_tensors, n_tensors >= 64 ? 8 : 48);
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: k_prep_apply<PYLO_FAM_ADAFAC><<<grid, NT, 0, s>>>(descs, *prm); break;
-    case PYLO_FAM_CELO2: k_prep_apply<PYLO_FAM_CELO2><<<grid, NT, 0, s>>>(descs, *prm); break;
-    case PYLO_FAM_VELO: k_prep_apply<PYLO_FAM_VELO><<<grid, NT, 0, s>>>(descs, *prm); break;
+    case PYLO_FAM_ADAFAC: k_prep_apply<PYLO_FAM_ADAFAC><<<n_items, NT, 0, s>>>(descs, items, *prm); break;
+    case PYLO_FAM_CELO2: k_prep_apply<PYLO_FAM_CELO2><<<n_items, NT, 0, s>>>(descs, items, *prm); break;
+    case PYLO_FAM_VELO: k_prep_apply<PYLO_FAM_VELO><<<n_items, NT, 0, s>>>(descs, items, *prm); break;
     default: return -2;
   }
   return launch_status();

@@ -67,18 +67,25 @@ def _aligned16(*tensors) -> bool:
     return all(t is None or t.data_ptr() % 16 == 0 for t in tensors)
 
 
-def make_tiles(sizes: Sequence[int]) -> Tuple[np.ndarray, List[Tuple[int, int]]]:
-    """Element-wise tiles over items of the given sizes; returns (tiles, [(tile0, n_tiles)] per item)."""
-    ranges, total = [], 0
-    for n in sizes:
-        k = (int(n) + L.TILE_ELEMS - 1) // L.TILE_ELEMS
-        ranges.append((total, k))
-        total += k
-    tiles = np.zeros(total, dtype=L.TILE_DTYPE)
-    for i, (t0, k) in enumerate(ranges):
-        tiles["tensor"][t0:t0 + k] = i
-        tiles["start"][t0:t0 + k] = np.arange(k, dtype=np.int64) * L.TILE_ELEMS
-    return tiles, ranges
+def make_tiles(sizes: Sequence[int], elems: int = L.TILE_ELEMS) -> Tuple[np.ndarray, List[Tuple[int, int]]]:
+    """Element-wise tiles of ``elems`` elements over items of the given sizes; returns (tiles, [(tile0, n_tiles)] per item)."""
+    counts = (np.asarray(sizes, dtype=np.int64) + elems - 1) // elems
+    first = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    tiles = np.zeros(int(first[-1]), dtype=L.TILE_DTYPE)
+    owner = np.repeat(np.arange(len(counts)), counts)
+    tiles["tensor"] = owner
+    tiles["start"] = (np.arange(len(tiles), dtype=np.int64) - first[owner]) * elems
+    tiles["elems"] = elems
+    return tiles, list(zip(first[:-1].tolist(), counts.tolist()))
+
+
+def tile_elems(total: int, least: int, tiles_wanted: int) -> int:
+    """Elements per tile for ``total`` elements of work: the largest power of two up to ``L.TILE_ELEMS`` that still gives
+    ``tiles_wanted`` tiles (enough CTAs to fill the GPU), and never less than ``least`` (one pass of a CTA)."""
+    e = L.TILE_ELEMS
+    while e > least and total < e * tiles_wanted:
+        e //= 2
+    return e
 
 
 class DeviceTable:
@@ -159,7 +166,7 @@ class LoPlan:
         H = self.H[family]
         tdesc = np.zeros(T, dtype=L.DESC_DTYPE)
         ws_items = []  # (table, row, field, count)
-        atiles, rtiles, generic = [], [], []
+        atiles, generic = [], []
         ws_bytes = 0  # the library's own count of the workspace, checked against the layout below
         for i, t in enumerate(tensors):
             shape = tuple(t.p.shape)
@@ -210,12 +217,11 @@ class LoPlan:
                 ws_items += [("t", i, f, getattr(ws, f)) for f in ("f_a", "f_b", "sum_a", "sum_b")]
                 if fast:
                     d["rb"], d["n_strips"], d["n_cb"] = ws.rb, ws.n_strips, ws.n_cb
-                    assert ws.rb == min(128, max(32, ((X + 127) // 128 + 7) // 8 * 8)) and ws.h_a == La * H * 2
+                    assert ws.h_a == La * H * 2
                     ws_items += [("t", i, f, getattr(ws, f)) for f in ("fx", "part_a", "part_b", "h_a", "h_b")]
                     for s in range(ws.n_strips):
                         for cb in range(ws.n_cb):
                             atiles.append((i, s, cb, 0))
-                    rtiles += [(i, 0, cb, 0) for cb in range(ws.n_cb)]
                 else:
                     generic.append(i)
             ws_items.append(("t", i, "closed", L.STAT_STRIDE))
@@ -250,11 +256,13 @@ class LoPlan:
         else:
             udesc = tdesc
         sizes = [int(udesc["n"][u]) for u in range(U)]
-        tiles, ranges = make_tiles(sizes)
+        # phase B: four 256-thread CTAs per SM, one pass of a CTA is 1024 elements; below ~10 M elements smaller tiles
+        # fill the GPU, above they would only multiply the block reductions
+        tiles, ranges = make_tiles(sizes, tile_elems(sum(sizes), 1024, 4 * L.SM_COUNT))
         for u, (t0, k) in enumerate(ranges):
             udesc["tile0"][u], udesc["n_tiles"][u] = t0, k
             ws = L.workspace_layout(family, L.MODE_VEC1D, sizes[u])  # the per-unit part depends on the element count only
-            assert ws.n_tiles == k
+            ws.n_tiles, ws.tile_part = k, k * L.STAT_STRIDE
             ws_items += [("u", u, f, getattr(ws, f)) for f in ("sums", "wfold", "tile_part")]
             ws_bytes += L.lib.pylo_b200_workspace_bytes(C.byref(ws), 0, 1)
         # workspace: every sub-buffer starts on a 256-byte boundary
@@ -282,8 +290,6 @@ class LoPlan:
         self.n_tiles = len(tiles)
         self.atiles = DeviceTable(np.array(atiles, dtype=np.int32).reshape(-1, 4).view(L.ATILE_DTYPE).reshape(-1), self.device)
         self.n_atiles = len(atiles)
-        self.rtiles = DeviceTable(np.array(rtiles, dtype=np.int32).reshape(-1, 4).view(L.ATILE_DTYPE).reshape(-1), self.device)
-        self.n_rtiles = len(rtiles)
         self.generic = DeviceTable(np.array(generic, dtype=np.int32), self.device)
         self.n_generic = len(generic)
         self.n_tensors = T
@@ -292,17 +298,25 @@ class LoPlan:
         self._keepalive = []
         # FAST2D tensors take a tiled apply kernel (see apply_tile_shape); everything else the generic one
         ctiles = []
+        # phase P: item 0 of every unit folds the network, the further ones (and item 0) make the tables' parts
+        pitems = [(u, 0, 0, 0) for u in range(U)]
+        per = L.PREP_TABLE // H
         unit_of = {i: u for u, (i, _) in enumerate(unit_owner)}  # a FAST2D tensor is never sliced: one unit
         for i in range(T):
             if tdesc["mode"][i] != L.MODE_FAST2D:
                 continue
             X, Y = int(tdesc["X"][i]), int(tdesc["Y"][i])
+            # the tensor-core kernel reads the per-row table only, the CUDA-core kernels both
+            parts = (X + per - 1) // per + (0 if self.tensor_cores else (Y + per - 1) // per)
+            pitems += [(unit_of[i], k, 0, 0) for k in range(1, parts)]
             rt, width, tag = apply_tile_shape(family, X, Y, self.tensor_cores)
             for rtile in range((X + rt - 1) // rt):
                 for ctile in range((Y + width - 1) // width):
                     ctiles.append((unit_of[i], rtile, ctile, tag))
         self.ctiles = DeviceTable(np.array(ctiles, dtype=np.int32).reshape(-1, 4).view(L.ATILE_DTYPE).reshape(-1), self.device)
         self.n_ctiles = len(ctiles)
+        self.pitems = DeviceTable(np.array(pitems, dtype=np.int32).reshape(-1, 4).view(L.ATILE_DTYPE).reshape(-1), self.device)
+        self.n_pitems = len(pitems)
         #: the kernel that takes the FAST2D tensors' apply sweep (also the key of its timings in phase_times())
         if self.tensor_cores:
             self.apply_kernel = "k_apply_adafac_tc"
@@ -315,9 +329,13 @@ class LoPlan:
         # a pinned copy of the flag follows every launch without blocking; the next launch looks at it once it landed
         self._status_host = torch.zeros(1, dtype=torch.int32).pin_memory() if self.tensor_cores else None
         self._status_event = None
-        fast_unit = udesc["mode"] == L.MODE_FAST2D
-        slow = tiles[~fast_unit[tiles["tensor"]]] if len(tiles) else tiles
-        self.tiles_slow = DeviceTable(np.ascontiguousarray(slow), self.device)
+        # the other units' apply sweep: vectors are short and every element costs a whole network, so the tiles are as
+        # small as one element per thread where that is what fills the GPU (five 4096-vectors: 104 us as one tile each)
+        slow_units = [u for u in range(U) if udesc["mode"][u] != L.MODE_FAST2D]
+        slow_sizes = [sizes[u] for u in slow_units]
+        slow, _ = make_tiles(slow_sizes, tile_elems(sum(slow_sizes), 256, 4 * L.SM_COUNT))
+        slow["tensor"] = np.asarray(slow_units, dtype=np.int32)[slow["tensor"]] if len(slow) else slow["tensor"]
+        self.tiles_slow = DeviceTable(slow, self.device)
         self.n_tiles_slow = len(slow)
 
     # ------------------------------------------------------------------ per-step refresh
@@ -385,8 +403,8 @@ class LoPlan:
         pp = C.byref(prm)
         if self.n_atiles or self.n_generic:
             self._call("rowcol_sums", L.lib.pylo_b200_rowcol_sums, self.tdesc.ptr, self.atiles.ptr, self.n_atiles,
-                       self.rtiles.ptr, self.n_rtiles, self.generic.ptr, self.n_generic, pp, stream)
-            self.launch_count += (1 if self.n_atiles else 0) + (1 if self.n_atiles and self.n_generic else 0)
+                       self.generic.ptr, self.n_generic, pp, stream)
+            self.launch_count += 1 if self.n_atiles and self.n_generic else 0
         self._call("factor_update", L.lib.pylo_b200_factor_update, self.tdesc.ptr, self.n_tensors, pp, stream)
         self._call("state_moments", L.lib.pylo_b200_state_moments, self.desc.ptr, self.tiles.ptr, self.n_tiles,
                    int(reverse_b), pp, stream)
@@ -404,7 +422,7 @@ class LoPlan:
         # the tensor-core kernel needs the per-row table only (2); the CUDA-core kernels need both (0)
         prm.no_tables = 2 if self.tensor_cores else 0
         pp = C.byref(prm)
-        self._call("prep_apply", L.lib.pylo_b200_prep_apply, self.desc.ptr, self.n_units, pp, stream)
+        self._call("prep_apply", L.lib.pylo_b200_prep_apply, self.desc.ptr, self.pitems.ptr, self.n_pitems, pp, stream)
         if self.n_ctiles and self.tensor_cores:
             self._poll_status()
             self._call(self.apply_kernel, L.lib.pylo_b200_apply_adafac_tc, self.desc.ptr, self.ctiles.ptr, self.n_ctiles, pp, self.status.data_ptr(), stream)
