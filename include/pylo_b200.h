@@ -77,7 +77,7 @@ typedef struct pylo_tensor_desc {
   float* sum_a;   /* workspace [La]: sum over Y of g'^2 + 1e-30 */
   float* sum_b;   /* workspace [Lb]: sum over X */
   float* part_a;  /* workspace [X][n_cb]  row-sum partials (FAST2D) */
-  float* part_b;  /* workspace [n_strips][Y] column-sum partials (FAST2D) */
+  float* part_b;  /* workspace [n_strips][Lb] column-sum partials */
   float* h_a;     /* workspace [La][H] (ADAFAC) or [La][H][2] (CELO2, VELO): first-layer term of the "a" features (+ bias) */
   float* h_b;     /* workspace [H][Lb]: first-layer term of the "b" features */
   float* closed;  /* workspace [PYLO_STAT_STRIDE]: closed-form sums of squares of vector features */
@@ -100,7 +100,7 @@ typedef struct pylo_tensor_desc {
   int32_t mode;
   int32_t r_is_a;
   int32_t rcm_pre, rcm_A, rcm_post; /* row_col_mean: the row accumulator viewed [pre][A][post], mean over A */
-  int32_t rb, n_strips, n_cb;       /* FAST2D phase-A tiling: rows per strip, strips, column blocks */
+  int32_t rb, n_strips, n_cb;       /* phase-A tiling: rows per strip, strips, column blocks (FAST2D) */
   int32_t tile0, n_tiles;           /* this tensor's range in the element-wise tile list */
   int32_t vec_elementwise;          /* 1: this unit is a slice of a tensor (its normalisers cover the slice only),
                                        so the vector-only features are accumulated per element, not in closed form */
@@ -212,9 +212,11 @@ int pylo_b200_grad_sumsq_static(const pylo_gvec* items, const pylo_tile* tiles, 
 /* Phase A: row and column sums of g'^2 + 1e-30 (the reductions inside
  * grad_sqr.mean(dim=dr / dc), AdafacLO_cuda.py:333-340, CELO2_cuda.py:218-224, velo_cuda.py:531-541).
  * atiles cover the FAST2D tensors (strip x 1024-column block each; they leave per-strip column partials, which
- * pylo_b200_factor_update adds up); generic_ids lists the GENERIC tensors. */
+ * pylo_b200_factor_update adds up).  gitems cover the GENERIC tensors: items with pad_ = 1 take 256 of the Lb columns
+ * (cb) over the rows of a strip (desc.rb of the X rows), items with pad_ = 0 take cb of the La / I
+ * blocks that have I row sums each, from block strip * cb on. */
 int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles,
-                          const int32_t* generic_ids, int n_generic, const pylo_step_params* prm, void* stream);
+                          const pylo_atile* gitems, int n_gitems, const pylo_step_params* prm, void* stream);
 
 /* Phase A2, one cluster of CTAs per tensor: the sums over strips and column blocks of phase A's partials, EMA of the factored accumulators, row_col_mean,
  * row/column rsqrt factors (AdafacLO_cuda.py:342-345, CELO2_cuda.py:229-231, velo_cuda.py:716-729)
@@ -259,17 +261,19 @@ int pylo_b200_apply(const pylo_tensor_desc* descs, const pylo_tile* tiles, int n
 int pylo_b200_apply_adafac_cols(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles,
                                 const pylo_step_params* prm, void* stream);
 
-/* Phase C for the FAST2D tensors of the ADAFAC family on the tensor cores (no reference counterpart: the
+/* Phase C for the tensors of the ADAFAC family on the tensor cores (no reference counterpart: the
  * reference evaluates the network with scalar FMAs, lo_kernel_apply learned_optimizer.cu:236-284).  Same inputs
  * and outputs as pylo_b200_apply_adafac_cols, except that of the two first-layer tables it reads only desc.h_a
  * (run pylo_b200_prep_apply with no_tables = 2 or 0).  The two hidden layers run as tcgen05 TF32 products with
  * every operand split into a high and a low TF32 part (hi x hi + hi x lo + lo x hi), which keeps a 32-term dot
  * product within ~3e-7 of the sum of its terms' magnitudes; non-finite features give NaN where the scalar path may
  * give an infinity.  ttiles: strip = row-strip index, cb = block of 128 columns, pad_ = rows per work item (one
- * warpgroup of a CTA takes a whole item).  status: device int; the kernel ORs 1 into it if a wait on the tensor
+ * warpgroup of a CTA takes a whole item).  Units that are not FAST2D: pad_ = 0x10000 | tiles per work item, strip = item
+ * index, cb = 0; an item is that many runs of 128 consecutive elements; generic != 0 says that the list may hold such
+ * items.  status: device int; the kernel ORs 1 into it if a wait on the tensor
  * core ran out (the parameters it could not finish then keep their old values), and a launch that finds it
  * non-zero stores nothing; may be NULL. */
-int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* ttiles, int n_ttiles,
+int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* ttiles, int n_ttiles, int generic,
                               const pylo_step_params* prm, int* status, void* stream);
 
 /* Phase C for the FAST2D tensors of the CELO2 and VELO families (same arithmetic as pylo_b200_apply, done on

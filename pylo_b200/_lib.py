@@ -112,7 +112,7 @@ def _load():
         "pylo_b200_prep_apply": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply_adafac_cols": [vp, vp, i32, C.POINTER(StepParams), vp],
-        "pylo_b200_apply_adafac_tc": [vp, vp, i32, C.POINTER(StepParams), vp, vp],
+        "pylo_b200_apply_adafac_tc": [vp, vp, i32, i32, C.POINTER(StepParams), vp, vp],
         "pylo_b200_apply_packed": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_gemm_tn_3xtf32": [C.POINTER(GemmDesc), vp, vp],
         "pylo_b200_transpose": [vp, vp, i32, i32, i32, i32, C.c_int64, C.c_int64, i32, i32, vp],
@@ -139,6 +139,7 @@ lib, EXPORTED = _load()
 
 SM_COUNT = 148        # of a B200; sizes of work lists only, the kernels ask the device
 TC_WORKERS = SM_COUNT * 4  # warpgroups the tensor-core apply kernel runs at once (four per SM)
+TC_GEN_ITEM = 1 << 16  # tag bit of its items on tensors that are not FAST2D
 STATIC_SCRATCH_TILES = 65536
 ERR_STATIC_SCRATCH_TOO_SMALL = -4
 

@@ -1,4 +1,4 @@
-// Phase C for AdafacLO / ELO on FAST2D tensors on the tensor cores (included by pylo_kernels.cu).
+// Phase C for AdafacLO / ELO on the tensor cores (included by pylo_kernels.cu).
 //
 // The per-element network is a pair of small dense products, [elements x 29] x [29 x 32] and
 // [elements x 32] x [32 x 32]; on the CUDA cores they cost ~1600 fp32 FMAs per element and bound the whole
@@ -15,6 +15,10 @@
 //     three products per layer and K step (hi x hi, hi x lo, lo x hi) into one accumulator of 32 columns.  Operand
 //     B holds the high parts in rows 0..31 and the low parts in rows 32..63 of one block; a product addresses
 //     either half through its descriptor's start address.  A tile takes 9 + 13 = 22 products of width 32;
+//   * tensors that are not FAST2D (ragged rows, more than two dims, vectors) are taken as 128 consecutive elements that
+//     share nothing: all twelve vector features of an element are columns of operand A and the first-layer bias, now the
+//     same for the whole tensor, sits in operand B for good; K = 32 (the scalar kernel that took them before needed 752
+//     us for the 5 M parameters of a small convolutional network, FMA-bound);
 //   * the second-layer bias is one more product, of a constant operand A (ones, in shared memory) with a block of
 //     operand B that holds the bias's high and low parts;
 //   * relu, the split of the hidden activations, the two output heads and the parameter update stay on the CUDA
@@ -42,7 +46,9 @@
 #endif
 #define TC_COLS 128              // tensor columns per work item: one per lane of the accumulator tile
 #define TC_WG_TMEM 96            // tensor-memory columns per warpgroup: [0,32) operand A high parts, [32,64) low parts, [64,96) accumulator
-#define TC_K1 24                 // first-layer K: 16 element-wise + 6 column features + 2 constant columns
+#define TC_K1 24                 // first-layer K on FAST2D tensors: 16 element-wise + 6 column features + 2 constant columns
+#define TC_K1_GEN 32             // on the others: 16 element-wise + 12 vector features + 2 constant columns, two zero
+#define TC_GEN_ITEM (1 << 16)    // set in an item's tag: `strip` counts items of `rows` x 128 consecutive elements
 #define TC_SPIN_LIMIT (1 << 20)
 #ifndef TC_POLL_SLEEP_NS
 #define TC_POLL_SLEEP_NS 40
@@ -188,8 +194,9 @@ __device__ __forceinline__ void tc_split16(const float (&x)[16], uint32_t (&hi)[
 // One warpgroup's private shared memory: its copy of the weights and its tensor-core barrier.  Warpgroups never
 // wait on one another.
 struct __align__(128) TcWgSmem {
-  float b1[64 * TC_K1];   // first layer, rows 0..31 the high parts, 32..63 the low parts; K = 24 (K rows 22 and 23 of
+  float b1[64 * TC_K1_GEN];  // first layer, rows 0..31 the high parts, 32..63 the low parts; K = 24 (K rows 22 and 23 of
                           // the high half are rewritten for every tensor row: the row's bias vector, high and low part)
+                          // or K = 32 (K rows 28 and 29: the tensor's bias vector)
   float b2[64 * 32];      // second layer, laid out the same way; K = 32
   float b2bias[32 * 8];   // second-layer bias as a K = 8 block: (high part, low part, 0 ...)
   float w3[64 + 4];       // output layer, pair-major (Fold::W3P), then its two biases
@@ -202,6 +209,9 @@ struct TcSmem {
   int poisoned;  // the status word at launch: non-zero means an earlier launch reported a timed-out wait
 };
 
+// GENERIC: the launch may hold items on tensors that are not FAST2D.  The variant without them is the faster one on large
+// models (their body costs the other one registers: 1 % of the sweep over two Llama blocks).
+template <bool GENERIC>
 __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const pylo_tensor_desc* __restrict__ descs,
                                                               const pylo_atile* __restrict__ ttiles, int n_ttiles,
                                                               const pylo_step_params prm, int* __restrict__ status) {
@@ -242,27 +252,42 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
   for (int t = blockIdx.x * TC_WGS + wg; t < n_items; t += gridDim.x * TC_WGS) {
     const pylo_atile ct = ttiles[t];
     const pylo_tensor_desc& d = descs[ct.tensor];
+    const int rows_item = ct.pad_ & (TC_GEN_ITEM - 1);  // rows (tiles of 128 elements) per work item
+    // One item; GEN: the tensor is not FAST2D.  Two bodies, so that neither holds the other's registers.
+    auto item = [&](auto gen_tag) {
+    constexpr bool GEN = decltype(gen_tag)::value;
+    constexpr int KSTEPS = (GEN ? TC_K1_GEN : TC_K1) / 8;
     const int X = d.X, Y = d.Y;
-    const int rows_item = ct.pad_;  // rows per work item
+    const int64_t n = d.n;
     const int y = ct.cb * TC_COLS + col;
+    const int x0 = ct.strip * rows_item;
+    const int64_t e0 = (int64_t)x0 * TC_COLS + col;      // GEN: this thread's first element
     const bool colok = y < Y;
     const int yc = colok ? y : 0;
-    const int x0 = ct.strip * rows_item;
     wg_barrier(wg);  // the four warps are done with the previous item's weights
     if (loaded != ct.tensor) {
       // K order of the first layer: 16 element-wise features (0..12, 25..27), the six features of the column
-      // vector, then the two rows that carry the tensor row's bias vector (written per row below)
+      // vector, then the two rows that carry the tensor row's bias vector (written per row below); GEN: after the 16
+      // the twelve vector features (13..24), then the tensor's bias vector
       const int kb = d.r_is_a ? F::C : F::R, krb = d.r_is_a ? F::RC : F::RR;
-      for (int e = col; e < 32 * TC_K1; e += 128) {
+      for (int e = col; e < 32 * 8 * KSTEPS; e += 128) {
         const int n = e & 31, kk = e >> 5;
         float w = 0.f;
         if (kk < 13) w = d.wfold[L::W1 + kk * 32 + n];
         else if (kk < 16) w = d.wfold[L::W1 + (kk + 12) * 32 + n];
+        else if (GEN) {
+          if (kk < 28) w = d.wfold[L::W1 + (F::R + kk - 16) * 32 + n];
+        }
         else if (kk < 19) w = d.wfold[L::W1 + (kb + kk - 16) * 32 + n];
         else if (kk < 22) w = d.wfold[L::W1 + (krb + kk - 19) * 32 + n];
-        const float hi = tf32_hi(w);
+        float hi = tf32_hi(w), lo = w - hi;
+        if (GEN && (kk == 28 || kk == 29)) {
+          const float b = d.wfold[L::B1 + n];
+          hi = kk == 28 ? tf32_hi(b) : b - tf32_hi(b);
+          lo = 0.f;
+        }
         sm.b1[tc_b_index(n, kk, TC_LBO64)] = hi;
-        sm.b1[tc_b_index(32 + n, kk, TC_LBO64)] = w - hi;
+        sm.b1[tc_b_index(32 + n, kk, TC_LBO64)] = lo;
       }
       for (int e = col; e < 32 * 32; e += 128) {
         const int n = e & 31, k = e >> 5;
@@ -284,49 +309,75 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
     float* __restrict__ pp = d.p;
     const float* __restrict__ mp = d.m;
     const float* __restrict__ vp = d.v;
-    const float* __restrict__ fxp = d.fx;    // [X][4]: the row's three factors of the element-wise factored features
-    const float* __restrict__ hap = d.h_a;   // [X][32]: the row's first-layer bias vector (row features + bias)
-    const int64_t n = d.n;
     const Peers peers = load_peers(d);
     const float gs = grad_scale_of(d, prm);
     const Fin fin{d.exp_mult, d.step_mult, d.wd, d.lr, d.wfold[L::SC + 1], 1.0f, prm.wd_mode};
-    // no clipping, no nan_to_num, no global-norm scale (AdafacLO's defaults): the gradient is used as it is
     const bool plain = plain_grad(gs, prm);
-    const float fb0 = d.f_b[yc], fb1 = d.f_b[Y + yc], fb2 = d.f_b[2 * (int64_t)Y + yc];
-    // the six features of this thread's column, high parts (then two ones) and low parts (then two zeros)
+    // GEN: the accumulators of the "r" and "c" vectors and the "r" factor (the "c" factor is a function of its accumulator)
+    const bool vec1d = d.mode == PYLO_MODE_VEC1D, r_is_a = d.r_is_a != 0;
+    const float* __restrict__ facr = GEN ? (r_is_a ? d.fac_a : d.fac_b) : nullptr;
+    const float* __restrict__ facc = GEN ? (vec1d ? (d.fac_b ? d.fac_b : d.fac_a) : (r_is_a ? d.fac_b : d.fac_a)) : nullptr;
+    const float* __restrict__ frp = GEN && !vec1d ? (r_is_a ? d.f_a : d.f_b) : nullptr;
+    const int64_t Lr = vec1d ? n : (r_is_a ? d.La : d.Lb), Lc = vec1d ? n : (r_is_a ? d.Lb : d.La);
+    GenPos pos(d, GEN && !vec1d ? e0 : 0, TC_COLS);
+    // FAST2D: the row's three factors and its first-layer bias vector (row features + bias)
+    const float* __restrict__ fxp = d.fx;    // [X][4]
+    const float* __restrict__ hap = d.h_a;   // [X][32]
+    float fb0 = 0.f, fb1 = 0.f, fb2 = 0.f;
     uint32_t chi[8], clo[8];
+    if constexpr (!GEN) {
+      fb0 = d.f_b[yc]; fb1 = d.f_b[Y + yc]; fb2 = d.f_b[2 * (int64_t)Y + yc];
+      // the six features of this thread's column, high parts (then two ones) and low parts (then two zeros)
 #pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      const float r = colok ? d.fac_b[(int64_t)(j % 3) * Y + yc] : 0.f;
-      const float v = colok ? (j < 3 ? r : rsqrtf(r + 1e-8f)) : 0.f;
-      const float hi = tf32_hi(v);
-      chi[j] = __float_as_uint(hi);
-      clo[j] = __float_as_uint(v - hi);
+      for (int j = 0; j < 6; ++j) {
+        const float r = colok ? d.fac_b[(int64_t)(j % 3) * Y + yc] : 0.f;
+        const float v = colok ? (j < 3 ? r : rsqrtf(r + 1e-8f)) : 0.f;
+        const float hi = tf32_hi(v);
+        chi[j] = __float_as_uint(hi);
+        clo[j] = __float_as_uint(v - hi);
+      }
+      chi[6] = chi[7] = 0x3f800000u;
+      clo[6] = clo[7] = 0u;
     }
-    chi[6] = chi[7] = 0x3f800000u;
-    clo[6] = clo[7] = 0u;
     fence_async_smem();  // the tensor core reads the weights through the async proxy
     wg_barrier(wg);
     float cg, cp, cm0, cm1, cm2, cv;
-    float4 cfa;
+    float4 cfa;        // FAST2D: the row's factors.  GEN: the element's "r" factors (vectors: unused)
+    float cr[3], cc[3];  // GEN: the element's accumulators
     float hrow = 0.f;  // lanes 0..31 of the warpgroup's first warp: entry `col` of the row's bias vector
     auto load_row = [&](int x, float& g, float& p, float& m0, float& m1, float& m2, float& v, float4& fa, float& hr) {
-      const int xc = x < X ? x : 0;
-      const int64_t idx = (colok && x < X) ? (int64_t)x * Y + y : 0;
-      g = ldg_early(gp + idx); p = ldg_early(pp + idx); m0 = ldg_early(mp + idx);
-      m1 = ldg_early(mp + n + idx); m2 = ldg_early(mp + 2 * n + idx); v = ldg_early(vp + idx);
-      fa = ldg4_early(fxp + 4 * (int64_t)xc);
-      if (col < 32) hr = ldg_early(hap + (int64_t)xc * 32 + col);
+      if constexpr (GEN) {
+        const int64_t e = (int64_t)x * TC_COLS + col;
+        const int64_t idx = e < n ? e : 0;
+        g = ldg_early(gp + idx); p = ldg_early(pp + idx); m0 = ldg_early(mp + idx);
+        m1 = ldg_early(mp + n + idx); m2 = ldg_early(mp + 2 * n + idx); v = ldg_early(vp + idx);
+        int64_t ir = idx, ic = idx;
+        if (!vec1d) {
+          const int64_t a = e < n ? pos.a() : 0, b = e < n ? pos.b() : 0;
+          pos.next();
+          ir = r_is_a ? a : b; ic = r_is_a ? b : a;
+          fa.x = ldg_early(frp + ir); fa.y = ldg_early(frp + Lr + ir); fa.z = ldg_early(frp + 2 * Lr + ir);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { cr[k] = ldg_early(facr + k * Lr + ir); cc[k] = ldg_early(facc + k * Lc + ic); }
+      } else {
+        const int xc = x < X ? x : 0;
+        const int64_t idx = (colok && x < X) ? (int64_t)x * Y + y : 0;
+        g = ldg_early(gp + idx); p = ldg_early(pp + idx); m0 = ldg_early(mp + idx);
+        m1 = ldg_early(mp + n + idx); m2 = ldg_early(mp + 2 * n + idx); v = ldg_early(vp + idx);
+        fa = ldg4_early(fxp + 4 * (int64_t)xc);
+        if (col < 32) hr = ldg_early(hap + (int64_t)xc * 32 + col);
+      }
     };
     load_row(x0, cg, cp, cm0, cm1, cm2, cv, cfa, hrow);
     TC_CLK(7)  // item set-up
 #pragma unroll 1
     for (int i = 0; i < rows_item; ++i) {
       const int x = x0 + i;  // the same for the whole warpgroup
-      if (x >= X) break;
+      if (GEN ? (int64_t)x * TC_COLS >= n : x >= X) break;
       TC_CLK(8)  // loop overhead
       // ---- the row's bias vector into operand B (the previous row's first-layer products are complete)
-      if (col < 32) {
+      if (!GEN && col < 32) {
         const float hi = tf32_hi(hrow);
         *reinterpret_cast<float2*>(&sm.b1[tc_b_index(col, 22, TC_LBO64)]) = make_float2(hi, hrow - hi);
         fence_async_smem();
@@ -336,16 +387,31 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
       {
         const float g = plain ? cg : xform_grad(cg, gs, prm.clip_val, prm.nan_to_num);
         const float rs = rsqrt_pos(cv + prm.eps_feat);
-        const float k0 = cfa.x * fb0, k1 = cfa.y * fb1, k2 = cfa.z * fb2;
+        float k0, k1, k2;
+        if constexpr (GEN) {
+          k0 = vec1d ? safe_rsqrt(cr[0] + 1e-9f) : cfa.x * safe_rsqrt(cc[0]);
+          k1 = vec1d ? safe_rsqrt(cr[1] + 1e-9f) : cfa.y * safe_rsqrt(cc[1]);
+          k2 = vec1d ? safe_rsqrt(cr[2] + 1e-9f) : cfa.z * safe_rsqrt(cc[2]);
+        } else {
+          k0 = cfa.x * fb0; k1 = cfa.y * fb1; k2 = cfa.z * fb2;
+        }
         const float fe[16] = {g, cp, cm0, cm1, cm2, cv, cm0 * rs, cm1 * rs, cm2 * rs, rs,
                               k0 * g, k1 * g, k2 * g, k0 * cm0, k1 * cm1, k2 * cm2};
         uint32_t hi[16], lo[16];
         tc_split16(fe, hi, lo);
         TC_CLK(10)  // features and split
         tc_st16(tA, hi);
-        tc_st8(tA + 16, chi);
+        if constexpr (!GEN) tc_st8(tA + 16, chi);
         tc_st16(tA + 32, lo);
-        tc_st8(tA + 48, clo);
+        if constexpr (!GEN) tc_st8(tA + 48, clo);
+        if constexpr (GEN) {
+          const float fv[16] = {cr[0], cr[1], cr[2], cc[0], cc[1], cc[2],
+                                rsqrtf(cr[0] + 1e-8f), rsqrtf(cr[1] + 1e-8f), rsqrtf(cr[2] + 1e-8f),
+                                rsqrtf(cc[0] + 1e-8f), rsqrtf(cc[1] + 1e-8f), rsqrtf(cc[2] + 1e-8f), 1.0f, 1.0f, 0.0f, 0.0f};
+          tc_split16(fv, hi, lo);
+          tc_st16(tA + 16, hi);
+          tc_st16(tA + 48, lo);
+        }
       }
       // the next row's operands: requested now that this row's are consumed (only p is still needed, for the
       // update), so the two sets never share the register file; they land during the two products.  (Requesting
@@ -362,12 +428,12 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
           tc_fence_after();
           const uint64_t desc_b1 = tc_desc(smem_addr(sm.b1), TC_LBO64);
 #pragma unroll
-          for (int s = 0; s < 3; ++s) {
+          for (int s = 0; s < KSTEPS; ++s) {
             tc_mma(t_wg + 64, t_wg + 32 + 8 * s, desc_b1 + s * KSTEP64, TC_IDESC, s > 0);          // lo x hi
             tc_mma(t_wg + 64, t_wg + 8 * s, desc_b1 + TC_LOW_HALF + s * KSTEP64, TC_IDESC, 1);     // hi x lo
           }
 #pragma unroll
-          for (int s = 0; s < 3; ++s) tc_mma(t_wg + 64, t_wg + 8 * s, desc_b1 + s * KSTEP64, TC_IDESC, 1);   // hi x hi
+          for (int s = 0; s < KSTEPS; ++s) tc_mma(t_wg + 64, t_wg + 8 * s, desc_b1 + s * KSTEP64, TC_IDESC, 1);   // hi x hi
           tc_commit(&sm.bar);
         }
         __syncwarp();
@@ -446,15 +512,22 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
         unpack2(add2(od[0], od[1]), a, b);
         unpack2(add2(om[0], om[1]), c, dd);
         const float o0 = (a + b) + sm.w3[64], o1 = (c + dd) + sm.w3[65];
-        if (colok && !timed_out) {  // after a wait that ran out the accumulators are not to be trusted: keep the old value
+        const int64_t idx = GEN ? (int64_t)x * TC_COLS + col : (int64_t)x * Y + y;
+        if ((GEN ? idx < n : colok) && !timed_out) {  // after a wait that ran out the accumulators are not to be trusted: keep the old value
           const float pn = finish<PYLO_FAM_ADAFAC>(cp, o0, o1, fin);
-          const int64_t idx = (int64_t)x * Y + y;
           pp[idx] = pn;
           peer_store(peers, idx, pn);
         }
       }
       cp = np_;
       TC_CLK(6)  // heads, update, store
+    }
+    };
+    if constexpr (GENERIC) {
+      if (ct.pad_ & TC_GEN_ITEM) item(std::true_type{});
+      else item(std::false_type{});
+    } else {
+      item(std::false_type{});
     }
   }
   TC_CLK_FLUSH

@@ -184,19 +184,30 @@ __device__ __forceinline__ void block_reduce_store(float (&acc)[N], float* s_red
   __syncthreads();
 }
 
-// a / b vector indices of element idx of a [O,X,M,Y,I] tensor
-struct Geo {
-  uint32_t X, M, Y, I;
-  __device__ __forceinline__ void split(uint64_t idx, uint64_t& a, uint64_t& b) const {
-    const uint64_t i = idx % I;
-    uint64_t t = idx / I;
-    const uint64_t y = t % Y;
-    t /= Y;
-    const uint64_t m = t % M;
-    t /= M;
-    const uint64_t x = t % X;
-    const uint64_t o = t / X;
-    a = ((o * X + x) * M + m) * I + i;
-    b = ((o * M + m) * Y + y) * I + i;
+// Where an element of a [O,X,M,Y,I] tensor sits: R = o*X + x and c = (m*Y + y)*I + i, the tensor being a matrix of O*X rows
+// of C = M*Y*I.  A thread that walks through a tensor in equal strides moves its position by additions; one division pair
+// finds the first.  R and C fit 32 bits: X and Y are the two largest sides, so either would need a tensor of over 2^33
+// elements to overflow.
+struct GenPos {
+  uint32_t R, c, C, dR, dc, YI, Y, X, M, I;
+  bool plain;     // M == I == 1: a matrix
+  bool one;       // O == 1
+  __device__ __forceinline__ GenPos(const pylo_tensor_desc& d, int64_t first, uint32_t stride) {
+    X = d.X; Y = d.Y; M = d.M; I = d.I;
+    YI = Y * I; C = M * YI;
+    plain = M == 1 && I == 1;
+    one = d.O == 1;
+    if ((uint64_t)first < (1ull << 32)) { R = (uint32_t)first / C; c = (uint32_t)first - R * C; }
+    else { R = (uint32_t)((uint64_t)first / C); c = (uint32_t)((uint64_t)first - (uint64_t)R * C); }
+    dR = stride / C;
+    dc = stride - dR * C;
   }
+  __device__ __forceinline__ void next() {
+    R += dR;
+    c += dc;
+    if (c >= C) { c -= C; ++R; }
+  }
+  // index into the "a" vectors (which drop Y) and the "b" vectors (which drop X)
+  __device__ __forceinline__ int64_t a() const { return plain ? (int64_t)R : ((int64_t)R * M + c / YI) * I + c % I; }
+  __device__ __forceinline__ int64_t b() const { return one ? (int64_t)c : (int64_t)(R / X) * C + c; }
 };

@@ -160,43 +160,84 @@ __global__ void __launch_bounds__(NT, 4) k_rowcol_fast(const pylo_tensor_desc* _
   }
 }
 
-// GENERIC tensors: one warp per output vector element, lanes stride over the reduced axis.
+// GENERIC tensors, seen as a matrix of O*X rows of C = M*Y*I (see GenPos).  Two kinds of work item, told apart by pad_:
+//   1: column sums: 256 of the Lb columns, one per thread, over the rows of a strip (partials as on the float4 path);
+//   0: row sums: a row is M blocks of Y*I consecutive elements, every block has I sums over y.  A group of lanes takes a
+//      block and reads it front to back; with I > 1 a lane stays on one i because the group's stride is a multiple of I.
+// Both read whole lines.  (One warp per output with lanes along the reduced axis, as it was, read one element per line
+// wherever that axis is not the last: 211 us for 5 M parameters of 3x3 convolutions, 302 us for a ViT patch embedding.)
+#define GA_LONG 4096      // from this block length on (I == 1) a CTA, not a warp, takes a block
 __global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* __restrict__ descs,
-                                                       const int32_t* __restrict__ ids, int slices,
+                                                       const pylo_atile* __restrict__ items,
                                                        const pylo_step_params prm) {
-  const pylo_tensor_desc& d = descs[ids[blockIdx.x / slices]];
-  const int slice = blockIdx.x % slices;
-  const int lane = threadIdx.x & 31;
-  const int64_t wid = (int64_t)slice * NWARP + (threadIdx.x >> 5);
-  const int64_t nw = (int64_t)slices * NWARP;
-  const int64_t X = d.X, M = d.M, Y = d.Y, I = d.I;
-  const int64_t La = d.La, Lb = d.Lb;
+  __shared__ float s_red[40];
+  const pylo_atile it = items[blockIdx.x];
+  const pylo_tensor_desc& d = descs[it.tensor];
   const float gs = grad_scale_of(d, prm);
-  for (int64_t o = wid; o < La + Lb; o += nw) {
+  const bool plain = plain_grad(gs, prm);
+  auto square = [&](float e) {
+    const float g = plain ? e : xform_grad(e, gs, prm.clip_val, prm.nan_to_num);
+    return g * g + 1e-30f;
+  };
+  const int64_t L = (int64_t)d.Y * d.I;
+  if (it.pad_ == 1) {
+    const int64_t C = d.M * L, b = (int64_t)it.cb * NT + threadIdx.x;
+    if (b >= d.Lb) return;
+    const int64_t o = d.O == 1 ? 0 : b / C;
+    const int x0 = it.strip * d.rb, x1 = min(x0 + d.rb, d.X);
+    const float* __restrict__ g = d.g + (o * d.X + x0) * C + (b - o * C);
     float acc = 0.f;
-    if (o < La) {  // a = ((o*X + x)*M + m)*I + i ; sum over y
-      const int64_t i = o % I, omx = o / I;
-      const int64_t base = omx * Y * I + i;
-      for (int64_t y = lane; y < Y; y += 32) {
-        const float g = xform_grad(d.g[base + y * I], gs, prm.clip_val, prm.nan_to_num);
-        acc += g * g + 1e-30f;
+#pragma unroll 8
+    for (int x = x0; x < x1; ++x, g += C) acc += square(__ldg(g));
+    d.part_b[(int64_t)it.strip * d.Lb + b] = acc;
+    return;
+  }
+  const int64_t blocks = d.La / d.I, b0 = (int64_t)it.strip * it.cb, b1 = min(b0 + it.cb, blocks);
+  const int I = d.I;
+  const int lane = threadIdx.x & 31;
+  if (I == 1 && L >= GA_LONG) {
+    for (int64_t k = b0; k < b1; ++k) {
+      const float* __restrict__ g = d.g + k * L;
+      float acc = 0.f;
+#pragma unroll 4
+      for (int64_t e = threadIdx.x; e < L; e += NT) acc += square(__ldg(g + e));
+      acc = block_sum(acc, s_red);
+      if (threadIdx.x == 0) d.sum_a[k] = acc;
+    }
+  } else if (I == 1) {
+    const int w = L > 16 ? 32 : (L > 8 ? 16 : (L > 4 ? 8 : 4));   // lanes per block
+    for (int64_t k = b0 + threadIdx.x / w; k < b1 + NT / w; k += NT / w) {   // whole warps stay in the loop for the shuffles
+      float acc = 0.f;
+      if (k < b1) {
+        const float* __restrict__ g = d.g + k * L;
+#pragma unroll 4
+        for (int64_t e = lane & (w - 1); e < L; e += w) acc += square(__ldg(g + e));
       }
-      acc = warp_sum(acc);
-      if (lane == 0) d.sum_a[o] = acc;
-    } else {  // b = ((o*M + m)*Y + y)*I + i ; sum over x
-      const int64_t b = o - La;
-      const int64_t i = b % I;
-      int64_t t = b / I;
-      const int64_t y = t % Y;
-      t /= Y;
-      const int64_t m = t % M, oo = t / M;
-      for (int64_t x = lane; x < X; x += 32) {
-        const int64_t idx = ((((oo * X + x) * M + m) * Y + y) * I) + i;
-        const float g = xform_grad(d.g[idx], gs, prm.clip_val, prm.nan_to_num);
-        acc += g * g + 1e-30f;
+      for (int o = w >> 1; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, w);
+      if ((lane & (w - 1)) == 0 && k < b1) d.sum_a[k] = acc;
+      if (k - threadIdx.x / w + NT / w >= b1) break;   // the same for all threads
+    }
+  } else if (I <= 32) {
+    const int S = 32 / I * I;   // active lanes
+    for (int64_t k = b0 + (threadIdx.x >> 5); k < b1; k += NWARP) {
+      const float* __restrict__ g = d.g + k * L;
+      float acc = 0.f;
+      if (lane < S)
+#pragma unroll 4
+        for (int64_t e = lane; e < L; e += S) acc += square(__ldg(g + e));
+      float tot = acc;
+      for (int q = I; q < S; q += I) tot += __shfl_sync(0xffffffffu, acc, (lane + q) & 31);   // read by lanes < I only
+      if (lane < I) d.sum_a[k * I + lane] = tot;
+    }
+  } else {
+    for (int64_t k = b0 + (threadIdx.x >> 5); k < b1; k += NWARP) {
+      const float* __restrict__ g = d.g + k * L;
+      for (int i = lane; i < I; i += 32) {
+        float acc = 0.f;
+#pragma unroll 4
+        for (int y = 0; y < d.Y; ++y) acc += square(__ldg(g + (int64_t)y * I + i));
+        d.sum_a[k * I + i] = acc;
       }
-      acc = warp_sum(acc);
-      if (lane == 0) d.sum_b[b] = acc;
     }
   }
 }
@@ -285,13 +326,9 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
     const int64_t i = c0 + (tid & 127);
     float s = 0.f;
     if (i < Lb) {
-      if (fast) {
-        const float* __restrict__ src = d.part_b + i;
+      const float* __restrict__ src = d.part_b + i;
 #pragma unroll 8
-        for (int r = tid >> 7; r < d.n_strips; r += A2_NT / 128) s += src[(int64_t)r * Lb];
-      } else if (tid < 128) {
-        s = d.sum_b[i];
-      }
+      for (int r = tid >> 7; r < d.n_strips; r += A2_NT / 128) s += src[(int64_t)r * Lb];
     }
     s_part[tid >> 7][tid & 127] = s;
     __syncthreads();
@@ -299,7 +336,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
       s = 0.f;
 #pragma unroll
       for (int w = 0; w < A2_NT / 128; ++w) s += s_part[w][tid];
-      if (fast) d.sum_b[i] = s;
+      d.sum_b[i] = s;
       const float mean = s / inv_n_b;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
@@ -468,33 +505,59 @@ __global__ void __launch_bounds__(NT) k_state_moments(const pylo_tensor_desc* __
         st4(vp + i, make_float4(ve[0], ve[1], ve[2], ve[3]));
       }
     } else if (d.mode == PYLO_MODE_GENERIC) {
-      const Geo geo{(uint32_t)d.X, (uint32_t)d.M, (uint32_t)d.Y, (uint32_t)d.I};
       const int64_t La = d.La, Lb = d.Lb;
       const bool vecf = d.vec_elementwise != 0;
-      const float* fac_r = d.r_is_a ? d.fac_a : d.fac_b;
-      const float* fac_c = d.r_is_a ? d.fac_b : d.fac_a;
-      for (int i = tid; i < cnt; i += NT) {
-        uint64_t a, b;
-        geo.split((uint64_t)(d.idx0 + start + i), a, b);
-        const float g = xform_grad(gp[i], gs, prm.clip_val, prm.nan_to_num);
-        float m0 = m0p[i], m1 = m1p[i], m2 = m2p[i], v = vp[i];
+      GenPos pos(d, d.idx0 + start + tid, NT);
+      constexpr int U = 4;   // elements of a thread in flight
+      auto update = [&](float g, float& m0, float& m1, float& m2, float& v) {
         velo_stats<FAM>(acc, m0, m1, m2, v);
         m0 = lerp_torch(m0, g, prm.w_m[0]);
         m1 = lerp_torch(m1, g, prm.w_m[1]);
         m2 = lerp_torch(m2, g, prm.w_m[2]);
         v = lerp_torch(v, g * g + prm.eps_v, prm.w_v);
-        m0p[i] = m0; m1p[i] = m1; m2p[i] = m2; vp[i] = v;
-        const float rs = rsqrtf(v + prm.eps_feat);
-        float f[F::NF];
-        elem_features<FAM>(f, g, pp[i], m0, m1, m2, v, rs, d.f_a[a] * d.f_b[b], d.f_a[La + a] * d.f_b[Lb + b],
-                           d.f_a[2 * La + a] * d.f_b[2 * Lb + b]);
-        if (vecf) {
-          const uint64_t ir = d.r_is_a ? a : b, ic = d.r_is_a ? b : a;
+      };
+      if (!vecf) {
+        for (int i0 = tid; i0 < cnt; i0 += U * NT) {
+          float g[U], p[U], m0[U], m1[U], m2[U], v[U], k0[U], k1[U], k2[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * NT;
+            if (i < cnt) {
+              g[u] = __ldg(gp + i); p[u] = pp[i]; m0[u] = m0p[i]; m1[u] = m1p[i]; m2[u] = m2p[i]; v[u] = vp[i];
+              const int64_t a = pos.a(), b = pos.b();
+              k0[u] = d.f_a[a] * d.f_b[b]; k1[u] = d.f_a[La + a] * d.f_b[Lb + b]; k2[u] = d.f_a[2 * La + a] * d.f_b[2 * Lb + b];
+            }
+            pos.next();
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * NT;
+            if (i < cnt) {
+              const float gx = xform_grad(g[u], gs, prm.clip_val, prm.nan_to_num);
+              update(gx, m0[u], m1[u], m2[u], v[u]);
+              m0p[i] = m0[u]; m1p[i] = m1[u]; m2p[i] = m2[u]; vp[i] = v[u];
+              float f[F::NF];
+              elem_features<FAM>(f, gx, p[u], m0[u], m1[u], m2[u], v[u], rsqrtf(v[u] + prm.eps_feat), k0[u], k1[u], k2[u]);
+              accumulate<FAM, false>(acc, f);
+            }
+          }
+        }
+      } else {
+        const float* fac_r = d.r_is_a ? d.fac_a : d.fac_b;
+        const float* fac_c = d.r_is_a ? d.fac_b : d.fac_a;
+        for (int i = tid; i < cnt; i += NT, pos.next()) {
+          const int64_t a = pos.a(), b = pos.b();
+          const float g = xform_grad(gp[i], gs, prm.clip_val, prm.nan_to_num);
+          float m0 = m0p[i], m1 = m1p[i], m2 = m2p[i], v = vp[i];
+          update(g, m0, m1, m2, v);
+          m0p[i] = m0; m1p[i] = m1; m2p[i] = m2; vp[i] = v;
+          float f[F::NF];
+          elem_features<FAM>(f, g, pp[i], m0, m1, m2, v, rsqrtf(v + prm.eps_feat), d.f_a[a] * d.f_b[b], d.f_a[La + a] * d.f_b[Lb + b],
+                             d.f_a[2 * La + a] * d.f_b[2 * Lb + b]);
+          const int64_t ir = d.r_is_a ? a : b, ic = d.r_is_a ? b : a;
           const int64_t Lr = d.r_is_a ? La : Lb, Lc = d.r_is_a ? Lb : La;
           vec_features<FAM>(f, fac_r[ir], fac_r[Lr + ir], fac_r[2 * Lr + ir], fac_c[ic], fac_c[Lc + ic], fac_c[2 * Lc + ic]);
           accumulate<FAM, true>(acc, f);
-        } else {
-          accumulate<FAM, false>(acc, f);
         }
       }
     } else {  // VEC1D: full-size accumulators updated element-wise (AdafacLO_cuda.py:349-360, velo_cuda.py:543-546)
@@ -822,38 +885,52 @@ __global__ void __launch_bounds__(NT) k_apply(const pylo_tensor_desc* __restrict
     const float* vp = d.v + start;
 
     {
-      const Geo geo{(uint32_t)d.X, (uint32_t)d.M, (uint32_t)d.Y, (uint32_t)d.I};
+      // E elements of a thread side by side: every weight read from shared memory serves all of them.  Two where the
+      // network is small; the 32-wide one (reached with mlp_precision="fp32" only) has no registers for a second.
+      constexpr int E = FAM == PYLO_FAM_ADAFAC ? 1 : 2;
       const bool vec1d = d.mode == PYLO_MODE_VEC1D;
       const int64_t La = vec1d ? n : d.La, Lb = vec1d ? n : d.Lb;
       const float* fac_r = d.r_is_a ? d.fac_a : d.fac_b;
       const float* fac_c = d.r_is_a ? d.fac_b : d.fac_a;
-      for (int i = tid; i < cnt; i += NT) {
-        const float g = xform_grad(gp[i], gs, prm.clip_val, prm.nan_to_num);
-        const float p = pp[i], m0 = m0p[i], m1 = m1p[i], m2 = m2p[i], v = vp[i];
-        const float rs = rsqrtf(v + prm.eps_feat);
-        float f[1][F::NF];
-        if (vec1d) {
-          const int64_t e = start + i;
-          const float r0 = d.fac_a[e], r1 = d.fac_a[n + e], r2 = d.fac_a[2 * n + e];
-          const float* cb = d.fac_b ? d.fac_b : d.fac_a;
-          elem_features<FAM>(f[0], g, p, m0, m1, m2, v, rs, safe_rsqrt(r0 + 1e-9f), safe_rsqrt(r1 + 1e-9f), safe_rsqrt(r2 + 1e-9f));
-          vec_features<FAM>(f[0], r0, r1, r2, cb[e], cb[n + e], cb[2 * n + e]);
-        } else {
-          uint64_t a, b;
-          geo.split((uint64_t)(d.idx0 + start + i), a, b);
-          elem_features<FAM>(f[0], g, p, m0, m1, m2, v, rs, d.f_a[a] * d.f_b[b], d.f_a[La + a] * d.f_b[Lb + b],
-                             d.f_a[2 * La + a] * d.f_b[2 * Lb + b]);
-          const uint64_t ir = d.r_is_a ? a : b, ic = d.r_is_a ? b : a;
-          const int64_t Lr = d.r_is_a ? La : Lb, Lc = d.r_is_a ? Lb : La;
-          vec_features<FAM>(f[0], fac_r[ir], fac_r[Lr + ir], fac_r[2 * Lr + ir], fac_c[ic], fac_c[Lc + ic], fac_c[2 * Lc + ic]);
-        }
-        float h1[1][H], o0[1], o1[1];
+      GenPos pos(d, vec1d ? 0 : d.idx0 + start + tid, NT);
+      for (int i0 = tid; i0 < cnt; i0 += E * NT) {
+        float f[E][F::NF], p[E], h1[E][H], o0[E], o1[E];
 #pragma unroll
-        for (int j = 0; j < H; ++j) h1[0][j] = s_w[L::B1 + j];
-        network<FAM, true, 1>(s_wa, h1, f, o0, o1);
-        const float pn = finish<FAM>(p, o0[0], o1[0], fin);
-        op[i] = pn;
-        if (FAM != PYLO_FAM_CELO2) peer_store(peers, start + i, pn);
+        for (int u = 0; u < E; ++u) {
+          const bool ok = i0 + u * NT < cnt;
+          const int i = ok ? i0 + u * NT : i0;   // a thread without a second element repeats its first (in bounds)
+          const float g = xform_grad(gp[i], gs, prm.clip_val, prm.nan_to_num);
+          const float m0 = m0p[i], m1 = m1p[i], m2 = m2p[i], v = vp[i];
+          p[u] = pp[i];
+          const float rs = rsqrtf(v + prm.eps_feat);
+          if (vec1d) {
+            const int64_t e = start + i;
+            const float r0 = d.fac_a[e], r1 = d.fac_a[n + e], r2 = d.fac_a[2 * n + e];
+            const float* cb = d.fac_b ? d.fac_b : d.fac_a;
+            elem_features<FAM>(f[u], g, p[u], m0, m1, m2, v, rs, safe_rsqrt(r0 + 1e-9f), safe_rsqrt(r1 + 1e-9f), safe_rsqrt(r2 + 1e-9f));
+            vec_features<FAM>(f[u], r0, r1, r2, cb[e], cb[n + e], cb[2 * n + e]);
+          } else {
+            const int64_t a = ok ? pos.a() : 0, b = ok ? pos.b() : 0;
+            pos.next();
+            elem_features<FAM>(f[u], g, p[u], m0, m1, m2, v, rs, d.f_a[a] * d.f_b[b], d.f_a[La + a] * d.f_b[Lb + b],
+                               d.f_a[2 * La + a] * d.f_b[2 * Lb + b]);
+            const int64_t ir = d.r_is_a ? a : b, ic = d.r_is_a ? b : a;
+            const int64_t Lr = d.r_is_a ? La : Lb, Lc = d.r_is_a ? Lb : La;
+            vec_features<FAM>(f[u], fac_r[ir], fac_r[Lr + ir], fac_r[2 * Lr + ir], fac_c[ic], fac_c[Lc + ic], fac_c[2 * Lc + ic]);
+          }
+#pragma unroll
+          for (int j = 0; j < H; ++j) h1[u][j] = s_w[L::B1 + j];
+        }
+        network<FAM, true, E>(s_wa, h1, f, o0, o1);
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+          const int i = i0 + u * NT;
+          if (i < cnt) {
+            const float pn = finish<FAM>(p[u], o0[u], o1[u], fin);
+            op[i] = pn;
+            if (FAM != PYLO_FAM_CELO2) peer_store(peers, start + i, pn);
+          }
+        }
       }
     }
   }
@@ -1694,6 +1771,14 @@ int pylo_b200_workspace_layout(int family, int mode, int64_t n, int64_t La, int6
     CHECK_ARG(La > 0 && Lb > 0);
     w.f_a = 3 * La; w.f_b = 3 * Lb; w.sum_a = La; w.sum_b = Lb;
   }
+  if (mode == PYLO_MODE_GENERIC) {
+    CHECK_ARG(n % Lb == 0);
+    const int64_t rows = n / Lb;   // X
+    // rows per strip of the column sums: one thread adds up a strip's rows, and 256 columns are one item
+    w.rb = rows <= 512 ? 16 : (rows <= 2048 ? 32 : PYLO_A_ROWS_MAX);
+    w.n_strips = (int32_t)((rows + w.rb - 1) / w.rb);
+    w.part_b = w.n_strips * Lb;
+  }
   if (mode == PYLO_MODE_FAST2D) {
     CHECK_ARG(X > 0 && Y > 0 && Y % 4 == 0 && La == X && Lb == Y);
     // rows per strip: about X / 128, a multiple of 8, within [32, 128].  Up to 512 rows a tensor gives too few strips of
@@ -1789,16 +1874,16 @@ int pylo_b200_grad_sumsq_static(const pylo_gvec* items, const pylo_tile* tiles, 
 }
 
 int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles,
-                          const int32_t* generic_ids, int n_generic, const pylo_step_params* prm, void* stream) {
-  CHECK_ARG(descs && prm && n_atiles >= 0 && n_generic >= 0);
+                          const pylo_atile* gitems, int n_gitems, const pylo_step_params* prm, void* stream) {
+  CHECK_ARG(descs && prm && n_atiles >= 0 && n_gitems >= 0);
   cudaStream_t s = (cudaStream_t)stream;
   if (n_atiles > 0) {
     CHECK_ARG(atiles);
     k_rowcol_fast<<<grid_for(n_atiles, 4), NT, 0, s>>>(descs, atiles, n_atiles, *prm);
   }
-  if (n_generic > 0) {
-    CHECK_ARG(generic_ids);
-    k_rowcol_generic<<<n_generic * 16, NT, 0, s>>>(descs, generic_ids, 16, *prm);
+  if (n_gitems > 0) {
+    CHECK_ARG(gitems);
+    k_rowcol_generic<<<n_gitems, NT, 0, s>>>(descs, gitems, *prm);
   }
   return launch_status();
 }
@@ -1877,15 +1962,16 @@ int pylo_b200_apply_adafac_cols(const pylo_tensor_desc* descs, const pylo_atile*
   return launch_status();
 }
 
-int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* ttiles, int n_ttiles,
+int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* ttiles, int n_ttiles, int generic,
                               const pylo_step_params* prm, int* status, void* stream) {
   CHECK_ARG(descs && ttiles && prm && n_ttiles >= 0 && prm->family == PYLO_FAM_ADAFAC);
   if (n_ttiles == 0) return 0;
   // more than half an SM's shared memory is requested: one CTA per SM, which then owns all of the SM's tensor memory
   constexpr int smem = sizeof(TcSmem) > 120 * 1024 ? (int)sizeof(TcSmem) : 120 * 1024;
-  static bool configured[PYLO_MAX_DEVICES] = {};
-  if (int rc = allow_dynamic_smem(k_apply_adafac_tc, smem, configured)) return rc;
-  k_apply_adafac_tc<<<grid_for(n_ttiles, 1), TC_NT, smem, (cudaStream_t)stream>>>(descs, ttiles, n_ttiles, *prm, status);
+  static bool configured[2][PYLO_MAX_DEVICES] = {};
+  auto kernel = generic ? k_apply_adafac_tc<true> : k_apply_adafac_tc<false>;
+  if (int rc = allow_dynamic_smem(kernel, smem, configured[generic ? 1 : 0])) return rc;
+  kernel<<<grid_for(n_ttiles, 1), TC_NT, smem, (cudaStream_t)stream>>>(descs, ttiles, n_ttiles, *prm, status);
   return launch_status();
 }
 

@@ -88,14 +88,29 @@ def tile_elems(total: int, least: int, tiles_wanted: int) -> int:
     return e
 
 
+def atile_grid(tensor: int, n_strips: int, n_cb: int, tag: int = 0) -> np.ndarray:
+    """Work items (tensor, strip, cb, tag) for every strip and column block."""
+    a = np.empty((n_strips, n_cb, 4), dtype=np.int32)
+    a[..., 0], a[..., 3] = tensor, tag
+    a[..., 1] = np.arange(n_strips)[:, None]
+    a[..., 2] = np.arange(n_cb)
+    return a.reshape(-1, 4)
+
+
+def atile_list(parts: List[np.ndarray]) -> np.ndarray:
+    flat = np.concatenate(parts) if parts else np.empty((0, 4), dtype=np.int32)
+    return np.ascontiguousarray(flat).view(L.ATILE_DTYPE).reshape(-1)
+
+
 class DeviceTable:
-    """A numpy structured array mirrored in device memory through two pinned staging buffers."""
+    """A numpy structured array mirrored in device memory.  The first upload is an ordinary copy (most tables never see
+    another); later ones go through two pinned staging buffers and do not wait."""
 
     def __init__(self, host: np.ndarray, device):
         self.host = host
         self.nbytes = max(host.nbytes, 16)
         self.dev = torch.empty(self.nbytes, dtype=torch.uint8, device=device)
-        self._stage = [torch.empty(self.nbytes, dtype=torch.uint8).pin_memory() for _ in range(2)]
+        self._stage = None
         self._events = [None, None]
         self._turn = 0
         self._last = None
@@ -110,13 +125,19 @@ class DeviceTable:
         raw = self.host.view(np.uint8).reshape(-1) if self.host.nbytes else None
         if raw is not None and self._last is not None and np.array_equal(raw, self._last):
             return
-        self._last = None if raw is None else raw.copy()
+        first, self._last = self._last is None, None if raw is None else raw.copy()
+        if raw is None:
+            return
+        if first:
+            self.dev.copy_(torch.from_numpy(raw))
+            return
+        if self._stage is None:
+            self._stage = [torch.empty(self.nbytes, dtype=torch.uint8).pin_memory() for _ in range(2)]
         i = self._turn
         self._turn ^= 1
         if self._events[i] is not None:
             self._events[i].synchronize()
-        if self.host.nbytes:
-            self._stage[i].numpy()[: self.host.nbytes] = self.host.view(np.uint8).reshape(-1)
+        self._stage[i].numpy()[: self.host.nbytes] = raw
         self.dev.copy_(self._stage[i], non_blocking=True)
         ev = torch.cuda.Event()
         ev.record()
@@ -166,7 +187,7 @@ class LoPlan:
         H = self.H[family]
         tdesc = np.zeros(T, dtype=L.DESC_DTYPE)
         ws_items = []  # (table, row, field, count)
-        atiles, generic = [], []
+        atiles, gitems = [], []
         ws_bytes = 0  # the library's own count of the workspace, checked against the layout below
         for i, t in enumerate(tensors):
             shape = tuple(t.p.shape)
@@ -215,15 +236,18 @@ class LoPlan:
                 # this table and a table built by any other host of the C ABI agree
                 ws = L.workspace_layout(family, int(d["mode"]), n, La, Lb, X if fast else 0, Y if fast else 0)
                 ws_items += [("t", i, f, getattr(ws, f)) for f in ("f_a", "f_b", "sum_a", "sum_b")]
+                d["rb"], d["n_strips"], d["n_cb"] = ws.rb, ws.n_strips, ws.n_cb
                 if fast:
-                    d["rb"], d["n_strips"], d["n_cb"] = ws.rb, ws.n_strips, ws.n_cb
                     assert ws.h_a == La * H * 2
                     ws_items += [("t", i, f, getattr(ws, f)) for f in ("fx", "part_a", "part_b", "h_a", "h_b")]
-                    for s in range(ws.n_strips):
-                        for cb in range(ws.n_cb):
-                            atiles.append((i, s, cb, 0))
+                    atiles.append(atile_grid(i, ws.n_strips, ws.n_cb))
                 else:
-                    generic.append(i)
+                    ws_items.append(("t", i, "part_b", ws.part_b))
+                    gitems.append(atile_grid(i, ws.n_strips, (Lb + 255) // 256, 1))
+                    per = max(1, 16384 // (Y * I))  # blocks of Y*I elements per row-sum item: about 16 K elements
+                    rows = atile_grid(i, (La // I + per - 1) // per, 1)
+                    rows[:, 2] = per
+                    gitems.append(rows)
             ws_items.append(("t", i, "closed", L.STAT_STRIDE))
             ws_bytes += L.lib.pylo_b200_workspace_bytes(
                 C.byref(L.workspace_layout(family, int(d["mode"]), n, int(d["La"]), int(d["Lb"]),
@@ -288,18 +312,20 @@ class LoPlan:
         self.desc = DeviceTable(udesc, self.device) if self.sliced else self.tdesc
         self.tiles = DeviceTable(tiles, self.device)
         self.n_tiles = len(tiles)
-        self.atiles = DeviceTable(np.array(atiles, dtype=np.int32).reshape(-1, 4).view(L.ATILE_DTYPE).reshape(-1), self.device)
-        self.n_atiles = len(atiles)
-        self.generic = DeviceTable(np.array(generic, dtype=np.int32), self.device)
-        self.n_generic = len(generic)
+        self.atiles = DeviceTable(atile_list(atiles), self.device)
+        self.n_atiles = len(self.atiles.host)
+        self.gitems = DeviceTable(atile_list(gitems), self.device)
+        self.n_gitems = len(self.gitems.host)
         self.n_tensors = T
         self.n_units = U
         self.total_elems = int(sum(sizes))
         self._keepalive = []
-        # FAST2D tensors take a tiled apply kernel (see apply_tile_shape); everything else the generic one
-        ctiles = []
+        # FAST2D tensors take a tiled apply kernel (see apply_tile_shape); everything else the generic one, or, with
+        # tensor cores, items of the same kernel
+        ctiles, shapes_c = [], []
         # phase P: item 0 of every unit folds the network, the further ones (and item 0) make the tables' parts
-        pitems = [(u, 0, 0, 0) for u in range(U)]
+        pitems = [np.zeros((U, 4), dtype=np.int32)]
+        pitems[0][:, 0] = np.arange(U)
         per = L.PREP_TABLE // H
         unit_of = {i: u for u, (i, _) in enumerate(unit_owner)}  # a FAST2D tensor is never sliced: one unit
         for i in range(T):
@@ -308,15 +334,27 @@ class LoPlan:
             X, Y = int(tdesc["X"][i]), int(tdesc["Y"][i])
             # the tensor-core kernel reads the per-row table only, the CUDA-core kernels both
             parts = (X + per - 1) // per + (0 if self.tensor_cores else (Y + per - 1) // per)
-            pitems += [(unit_of[i], k, 0, 0) for k in range(1, parts)]
-            rt, width, tag = apply_tile_shape(family, X, Y, self.tensor_cores)
-            for rtile in range((X + rt - 1) // rt):
-                for ctile in range((Y + width - 1) // width):
-                    ctiles.append((unit_of[i], rtile, ctile, tag))
-        self.ctiles = DeviceTable(np.array(ctiles, dtype=np.int32).reshape(-1, 4).view(L.ATILE_DTYPE).reshape(-1), self.device)
-        self.n_ctiles = len(ctiles)
-        self.pitems = DeviceTable(np.array(pitems, dtype=np.int32).reshape(-1, 4).view(L.ATILE_DTYPE).reshape(-1), self.device)
-        self.n_pitems = len(pitems)
+            pitems.append(atile_grid(unit_of[i], parts, 1)[1:])
+            shapes_c.append((unit_of[i], X, Y) + apply_tile_shape(family, X, Y, self.tensor_cores))
+        slow_units = [u for u in range(U) if udesc["mode"][u] != L.MODE_FAST2D]
+        if self.tensor_cores:
+            # the tensor-core kernel takes every tensor: what is not FAST2D as runs of 128 elements, with as many per
+            # item as for a FAST2D tensor; a model too small to give every warpgroup an item gets smaller ones
+            gen = [(u, (sizes[u] + 127) // 128) for u in slow_units]
+            shapes_c = [(u, X, 128) + apply_tile_shape(family, X, 128, True)[:2] + (L.TC_GEN_ITEM,) for u, X in gen] + [
+                (u, X, Y, rt, width, 0) for u, X, Y, rt, width, _ in shapes_c]
+            n_items = lambda k: sum(-(-X // max(1, rt >> k)) * -(-Y // w) for _, X, Y, rt, w, _ in shapes_c)
+            k = next((k for k in range(3) if n_items(k + 1) > L.TC_WORKERS), 3)
+            shapes_c = [(u, X, Y, max(1, rt >> k), w, tag | max(1, rt >> k)) for u, X, Y, rt, w, tag in shapes_c]
+            slow_units = []
+        for u, X, Y, rt, width, tag in shapes_c:
+            ctiles.append(atile_grid(u, (X + rt - 1) // rt, (Y + width - 1) // width, tag))
+        self.ctiles = DeviceTable(atile_list(ctiles), self.device)
+        self.n_ctiles = len(self.ctiles.host)
+        #: how many of them, at the front of the list, are on tensors that are not FAST2D (tensor cores only)
+        self.n_ctiles_gen = int((self.ctiles.host["pad_"] >= L.TC_GEN_ITEM).sum())
+        self.pitems = DeviceTable(atile_list(pitems), self.device)
+        self.n_pitems = len(self.pitems.host)
         #: the kernel that takes the FAST2D tensors' apply sweep (also the key of its timings in phase_times())
         if self.tensor_cores:
             self.apply_kernel = "k_apply_adafac_tc"
@@ -331,7 +369,6 @@ class LoPlan:
         self._status_event = None
         # the other units' apply sweep: vectors are short and every element costs a whole network, so the tiles are as
         # small as one element per thread where that is what fills the GPU (five 4096-vectors: 104 us as one tile each)
-        slow_units = [u for u in range(U) if udesc["mode"][u] != L.MODE_FAST2D]
         slow_sizes = [sizes[u] for u in slow_units]
         slow, _ = make_tiles(slow_sizes, tile_elems(sum(slow_sizes), 256, 4 * L.SM_COUNT))
         slow["tensor"] = np.asarray(slow_units, dtype=np.int32)[slow["tensor"]] if len(slow) else slow["tensor"]
@@ -401,10 +438,10 @@ class LoPlan:
         self._poll_status()  # before any state of this step is touched
         prm.step_delta = getattr(self, "step_delta", 0.0)
         pp = C.byref(prm)
-        if self.n_atiles or self.n_generic:
+        if self.n_atiles or self.n_gitems:
             self._call("rowcol_sums", L.lib.pylo_b200_rowcol_sums, self.tdesc.ptr, self.atiles.ptr, self.n_atiles,
-                       self.generic.ptr, self.n_generic, pp, stream)
-            self.launch_count += 1 if self.n_atiles and self.n_generic else 0
+                       self.gitems.ptr, self.n_gitems, pp, stream)
+            self.launch_count += 1 if self.n_atiles and self.n_gitems else 0
         self._call("factor_update", L.lib.pylo_b200_factor_update, self.tdesc.ptr, self.n_tensors, pp, stream)
         self._call("state_moments", L.lib.pylo_b200_state_moments, self.desc.ptr, self.tiles.ptr, self.n_tiles,
                    int(reverse_b), pp, stream)
@@ -425,7 +462,14 @@ class LoPlan:
         self._call("prep_apply", L.lib.pylo_b200_prep_apply, self.desc.ptr, self.pitems.ptr, self.n_pitems, pp, stream)
         if self.n_ctiles and self.tensor_cores:
             self._poll_status()
-            self._call(self.apply_kernel, L.lib.pylo_b200_apply_adafac_tc, self.desc.ptr, self.ctiles.ptr, self.n_ctiles, pp, self.status.data_ptr(), stream)
+            # small models: one launch; large ones: what is not FAST2D first, then the rest through the leaner variant
+            first = self.n_ctiles if self.n_ctiles < 8 * L.TC_WORKERS else self.n_ctiles_gen
+            for at, count in ((0, first), (first, self.n_ctiles - first)):
+                if count:
+                    gen = at == 0 and self.n_ctiles_gen > 0
+                    self._call(self.apply_kernel if count > self.n_ctiles_gen else "k_apply", L.lib.pylo_b200_apply_adafac_tc,
+                               self.desc.ptr, self.ctiles.ptr + at * L.ATILE_DTYPE.itemsize, count, int(gen), pp,
+                               self.status.data_ptr(), stream)
             # a pinned copy of the status word follows the launch on the launch's own stream, without blocking
             ctx = (torch.cuda.stream(torch.cuda.ExternalStream(stream, device=self.device))
                    if stream != current_stream_ptr() else contextlib.nullcontext())
