@@ -239,7 +239,7 @@ int pylo_b200_finalize_moments(const pylo_tensor_desc* descs, int n_tensors, voi
  * AdafacLO/ELO, the time features tanh(t/tau - 1) (learned_optimizer.cu:27-32,245-248) into the
  * first layer, and tabulate the first-layer contribution of the vector-only features.  items: tensor = unit, strip =
  * index of the unit's item.  Item 0 of every unit writes the folded network; with tables, an item also makes
- * 8192 / H entries of a table: items 0 .. ceil(X / (8192/H)) - 1 the per-row one, the following ceil(Y / (8192/H)) the
+ * 2048 / H entries of a table: items 0 .. ceil(X / (2048/H)) - 1 the per-row one, the following ceil(Y / (2048/H)) the
  * per-column one (FAST2D units; the others have item 0 only).
  * desc.w layouts: ADAFAC  w_in[32][39] b_in[32] w_h[32][32] b_h[32] w_out[2][32] b_out[2] (out-major);
  *                 CELO2   w_in[30][8]  b_in[8]  w_h[8][8]   b_h[8]  w_out[8][3]  b_out[3] (in-major);

@@ -15,7 +15,7 @@ STAT_STRIDE = 40
 SUMS_STRIDE = 48
 TILE_ELEMS = 16384
 A_COLS = 1024
-PREP_TABLE = 8192  # table entries (rows x hidden units) per item of pylo_b200_prep_apply
+PREP_TABLE = 2048  # table entries (rows x hidden units) per item of pylo_b200_prep_apply
 WFOLD_STRIDE = 2432
 ABI_VERSION = 11
 

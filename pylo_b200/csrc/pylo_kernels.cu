@@ -298,9 +298,13 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
   // 1. "a" vectors: finish the row sums, EMA of the accumulator lerp(acc, mean, 1 - beta_fac[k])
   const int gtid = rank * A2_NT + tid;
   for (int64_t i = gtid; i < La; i += A2_CL * A2_NT) {
+    float old[3];  // requested before the partials are added up
+#pragma unroll
+    for (int k = 0; k < 3; ++k) old[k] = d.fac_a[k * La + i];
     float s;
     if (fast) {
       s = 0.f;
+#pragma unroll 4
       for (int c = 0; c < d.n_cb; ++c) s += d.part_a[i * d.n_cb + c];
       d.sum_a[i] = s;
     } else {
@@ -310,7 +314,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
     float f[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float v = lerp_torch(d.fac_a[k * La + i], mean, prm.w_f[k]);
+      const float v = lerp_torch(old[k], mean, prm.w_f[k]);
       d.fac_a[k * La + i] = v;
       add(r_is_a, k, v);
       f[k] = safe_rsqrt(v);
@@ -324,7 +328,11 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
   // 2. "b" vectors: sum over the strips (in a fixed order), EMA
   for (int64_t c0 = (int64_t)rank * 128; c0 < Lb; c0 += A2_CL * 128) {
     const int64_t i = c0 + (tid & 127);
-    float s = 0.f;
+    float s = 0.f, old[3] = {0.f, 0.f, 0.f};
+    if (tid < 128 && i < Lb) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) old[k] = d.fac_b[k * Lb + i];
+    }
     if (i < Lb) {
       const float* __restrict__ src = d.part_b + i;
 #pragma unroll 8
@@ -340,7 +348,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
       const float mean = s / inv_n_b;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        const float v = lerp_torch(d.fac_b[k * Lb + i], mean, prm.w_f[k]);
+        const float v = lerp_torch(old[k], mean, prm.w_f[k]);
         d.fac_b[k * Lb + i] = v;
         add(!r_is_a, k, v);
         if (r_is_a) d.f_b[k * Lb + i] = safe_rsqrt(v);
@@ -446,7 +454,7 @@ __device__ __forceinline__ void velo_stats(float (&acc)[BAcc<FAM>::N], float m0,
 }
 
 template <int FAM>
-__global__ void __launch_bounds__(NT) k_state_moments(const pylo_tensor_desc* __restrict__ descs,
+__global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc* __restrict__ descs,
                                                       const pylo_tile* __restrict__ tiles, int n_tiles, int reverse,
                                                       const pylo_step_params prm) {
   using F = Fam<FAM>;
@@ -508,7 +516,7 @@ __global__ void __launch_bounds__(NT) k_state_moments(const pylo_tensor_desc* __
       const int64_t La = d.La, Lb = d.Lb;
       const bool vecf = d.vec_elementwise != 0;
       GenPos pos(d, d.idx0 + start + tid, NT);
-      constexpr int U = 4;   // elements of a thread in flight
+      constexpr int U = 2;   // elements of a thread in flight (four cost the float4 path its second CTA per SM)
       auto update = [&](float g, float& m0, float& m1, float& m2, float& v) {
         velo_stats<FAM>(acc, m0, m1, m2, v);
         m0 = lerp_torch(m0, g, prm.w_m[0]);
@@ -634,10 +642,10 @@ __device__ __forceinline__ float w1_at(int fam, const float* w, int j, int k) {
   return w[j * 30 + k];
 }
 
-// One work item is PREP_TABLE / H entries of a unit's "a" or "b" table (the "a" items first); item 0 of a unit also writes
+// One work item is PREP_TABLE / H rows of a unit's "a" or "b" table (the "a" items first); item 0 of a unit also writes
 // the folded network.  Items are dealt by the tables' sizes, so that a 50257-row table is spread over the GPU (a fixed
 // number of CTAs per unit took 537 us for it).
-#define PREP_TABLE 8192
+#define PREP_TABLE 2048
 template <int FAM>
 __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __restrict__ descs,
                                                    const pylo_atile* __restrict__ items, const pylo_step_params prm) {
