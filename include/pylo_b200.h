@@ -278,8 +278,8 @@ int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* t
 
 /* Phase C for the FAST2D tensors of the CELO2 and VELO families (same arithmetic as pylo_b200_apply, done on
  * pairs of adjacent elements with packed fp32x2 instructions).  ctiles: strip = row-tile index, cb = column-tile
- * index, pad_ = threads per row (8 .. 256, a thread owns 4 columns); a tile has 16 * (256 / pad_) rows and
- * 4 * pad_ columns.  For these families pylo_b200_prep_apply stores desc.h_a as (v, v) pairs, [X][H][2], and
+ * index, pad_ = threads per row (8 .. 256, a thread owns 4 columns) | rows per thread << 16 (0: 16); a tile has
+ * rows * (256 / threads) rows and 4 * threads columns.  For these families pylo_b200_prep_apply stores desc.h_a as (v, v) pairs, [X][H][2], and
  * for every family desc.h_b transposed, [H][Y]. */
 int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles,
                            const pylo_step_params* prm, void* stream);
@@ -359,9 +359,9 @@ typedef struct pylo_velo_rnn {
   const float* bank;                              /* [B][159] */
   float *h, *c;                                   /* [T][H] LSTM state, updated in place */
   float *x_in;                                    /* [T][30] */
-  float *pooled;                                  /* workspace [H] */
+  float *pooled;                                  /* unused */
   float *xmix;                                    /* workspace [T][H] */
-  float *gates;                                   /* workspace [T][4H] */
+  float *gates;                                   /* workspace [2][T][4H] */
   float *controls;                                /* workspace [T][B] */
   float *weights;                                 /* out [T][160] */
   float *lr_mult;                                 /* out [T] */

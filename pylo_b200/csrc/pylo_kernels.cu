@@ -1256,7 +1256,7 @@ __device__ __forceinline__ uint64_t pk_feature(const PkBase& b) {
   else return mul2(b.k2, b.m2);
 }
 
-#define PK_ROWS 16  // rows per thread in a tile
+#define PK_ROWS 16  // rows per thread in a tile, unless the tag's upper half says fewer
 
 #ifndef PK_CTAS_VELO
 #define PK_CTAS_VELO 2
@@ -1277,9 +1277,10 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : 2) k
     const pylo_atile ct = ctiles[t];
     const pylo_tensor_desc& d = descs[ct.tensor];
     const int X = d.X, Y = d.Y;
-    const int tpr = ct.pad_;          // threads per row: 8 .. 256 (a thread owns 4 columns)
+    const int tpr = ct.pad_ & 0xffff; // threads per row: 8 .. 256 (a thread owns 4 columns)
+    const int rpt = ct.pad_ >> 16 ? ct.pad_ >> 16 : PK_ROWS;   // rows per thread
     const int ng = NT / tpr;          // row groups
-    const int rt = PK_ROWS * ng;      // rows per tile
+    const int rt = rpt * ng;          // rows per tile
     const int x0 = ct.strip * rt, y0 = ct.cb * tpr * 4;
     if (loaded != ct.tensor) {
       __syncthreads();
@@ -1330,9 +1331,9 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : 2) k
     };
     load_row(0, cg, cp, cm0, cm1, cm2, cv);
 #pragma unroll 1
-    for (int q = 0; q < PK_ROWS; ++q) {
+    for (int q = 0; q < rpt; ++q) {
       float4 ng_, np_, nm0, nm1, nm2, nv;
-      if (q + 1 < PK_ROWS) load_row(q + 1, ng_, np_, nm0, nm1, nm2, nv);
+      if (q + 1 < rpt) load_row(q + 1, ng_, np_, nm0, nm1, nm2, nv);
       const int x = x0 + rg + ng * q;
       const int xc = x < X ? x : 0;
       const float4 fa = ld4(fxp + 4 * (int64_t)xc);
@@ -1416,7 +1417,7 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : 2) k
         st4(op + (int64_t)x * Y + y, res);
         if (FAM != PYLO_FAM_CELO2) peer_store4(peers, (int64_t)x * Y + y, res);
       }
-      if (q + 1 < PK_ROWS) { cg = ng_; cp = np_; cm0 = nm0; cm1 = nm1; cm2 = nm2; cv = nv; }
+      if (q + 1 < rpt) { cg = ng_; cp = np_; cm0 = nm0; cm1 = nm1; cm2 = nm2; cv = nv; }
     }
   }
 }
@@ -1594,37 +1595,97 @@ __global__ void k_velo_loss(float* means, int32_t* iteration, float* running_min
   if (j == 0) *iteration = it + 1;
 }
 
-// x' = final_mix(x) + max_t relu(mix2(x)) ; two kernels: pooled (one thread per hidden unit), then xmix
-__global__ void k_velo_pool(const pylo_velo_rnn r) {
-  const int h = blockIdx.x * blockDim.x + threadIdx.x;
+// x' = final_mix(x) + max_t relu(mix2(x)).  One warp per hidden unit, lanes along the tensors (one thread per unit walked
+// through all tensors by itself: 203 us at 292 tensors).
+__global__ void __launch_bounds__(NT) k_velo_xmix(const pylo_velo_rnn r) {
+  const int h = blockIdx.x * NWARP + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (h >= r.H) return;
-  float w[30];
+  float best = 0.f;   // relu
+  const float b2 = r.mix2_b[h], bf = r.fmix_b[h];
+  const float2* __restrict__ w2 = reinterpret_cast<const float2*>(r.mix2_w + h * 30);
+  const float2* __restrict__ wf = reinterpret_cast<const float2*>(r.fmix_w + h * 30);
+  for (int t = lane; t < r.T; t += 32) {
+    const float2* __restrict__ x = reinterpret_cast<const float2*>(r.x_in + t * 30);
+    float m = b2, f = bf;
 #pragma unroll
-  for (int k = 0; k < 30; ++k) w[k] = r.mix2_w[h * 30 + k];
-  const float b = r.mix2_b[h];
-  float best = -CUDART_INF_F;
-  for (int t = 0; t < r.T; ++t) {
-    float acc = b;
-#pragma unroll
-    for (int k = 0; k < 30; ++k) acc = fmaf(w[k], r.x_in[t * 30 + k], acc);
-    best = fmaxf(best, fmaxf(acc, 0.f));
+    for (int k = 0; k < 15; ++k) {
+      const float2 v = x[k], a = w2[k], c = wf[k];
+      m = fmaf(a.y, v.y, fmaf(a.x, v.x, m));
+      f = fmaf(c.y, v.y, fmaf(c.x, v.x, f));
+    }
+    best = fmaxf(best, m);
+    r.xmix[(int64_t)t * r.H + h] = f;
   }
-  r.pooled[h] = best;
-}
-
-__global__ void k_velo_xmix(const pylo_velo_rnn r) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (int64_t)r.T * r.H) return;
-  const int t = (int)(e / r.H), h = (int)(e % r.H);
-  float acc = r.fmix_b[h];
 #pragma unroll
-  for (int k = 0; k < 30; ++k) acc = fmaf(r.fmix_w[h * 30 + k], r.x_in[t * 30 + k], acc);
-  r.xmix[e] = acc + r.pooled[h];
+  for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+  for (int t = lane; t < r.T; t += 32) r.xmix[(int64_t)t * r.H + h] += best;
 }
 
-// gates[t][q] = lstm_b[q] + sum_k lstm_w[q][k] * cat(x', h)[t][k]: a [T x 2H] x [2H x 4H] product.
-// Shared-memory tiled, 64 x 64 outputs per CTA, 16 deep, 4 x 4 outputs per thread; fp32 throughout
-// (the whole product is ~1 GFLOP, far too small to be worth a tensor-core path).
+// gates[t][q] = lstm_b[q] + sum_k lstm_w[q][k] * cat(x', h)[t][k]: a [T x 2H] x [2H x 4H] product, fp32 throughout.
+//
+// For few tensors it is a read of the 8.4 MB of weights, for a few hundred ~0.6 G FMAs.  A warp keeps four weight rows (one
+// half of their columns: those that meet x', or those that meet h) in registers and takes eight tensors at a time from
+// shared memory: 512 FMAs per lane on 32 shared-memory reads, then the 32 sums are reduced over the lanes together, 31
+// shuffles in all, and lane l ends with the sum of tensor l / 4 and row l % 4.  The two halves are left as two partial
+// sums that the cell kernel adds.  512 hidden units: 6 tensors 68.6 -> 3.6 us, 292 tensors 124 -> 46 us (the tiled kernel
+// below, which is kept for hidden sizes that are not multiples of 128, or above 512).
+#define GR_ROWS 16   // weight rows per CTA: four per pair of warps
+template <int NI>    // float4 per lane and row: H = 128 * NI
+__global__ void __launch_bounds__(NT, 2) k_velo_gates_rows(const pylo_velo_rnn r, int groups_per_cta) {
+  extern __shared__ __align__(16) float s_x[];   // [2][8][2H]
+  constexpr int H = 128 * NI;
+  const int tid = threadIdx.x, lane = tid & 31, half = (tid >> 5) & 1, q0 = blockIdx.x * GR_ROWS + (tid >> 6) * 4;
+  const int groups = (r.T + 7) / 8, g0 = blockIdx.y * groups_per_cta, g1 = min(g0 + groups_per_cta, groups);
+  auto stage = [&](int g) {
+    float* dst = s_x + (g & 1) * 16 * H;
+    for (int e = tid; e < 8 * 2 * (H / 4); e += NT) {
+      const int c = e % (H / 2), t = g * 8 + e / (H / 2);   // 2H / 4 pieces per tensor
+      const float* src = c < H / 4 ? r.xmix + (int64_t)t * H + 4 * c : r.h + (int64_t)t * H + 4 * (c - H / 4);
+      const uint32_t bytes = t < r.T ? 16 : 0;              // past the last tensor: zeros
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst + 4 * e)), "l"(t < r.T ? src : r.xmix), "r"(bytes) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (g0 < g1) stage(g0);
+  float4 w[4][NI];
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int i = 0; i < NI; ++i) w[u][i] = ldg4(r.lstm_w + (int64_t)(q0 + u) * 2 * H + half * H + (i * 32 + lane) * 4);
+  for (int g = g0; g < g1; ++g) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();   // this group has arrived, and the buffer of the next one is no longer read
+    if (g + 1 < g1) stage(g + 1);
+    const float* x = s_x + (g & 1) * 16 * H + half * H + lane * 4;
+    float acc[32];     // tensor * 4 + row
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[t * 4 + u] = 0.f;
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        const float4 v = ld4(x + t * 2 * H + i * 128);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          acc[t * 4 + u] = fmaf(w[u][i].w, v.w, fmaf(w[u][i].z, v.z, fmaf(w[u][i].y, v.y, fmaf(w[u][i].x, v.x, acc[t * 4 + u]))));
+      }
+    }
+    // fold the lanes: after the step of offset o a lane holds the o entries whose index agrees with its own in that bit
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int j = 0; j < o; ++j) {
+        const float keep = up ? acc[j + o] : acc[j], give = up ? acc[j] : acc[j + o];
+        acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    }
+    const int t = g * 8 + (lane >> 2), q = q0 + (lane & 3);
+    if (t < r.T) r.gates[((int64_t)half * r.T + t) * 4 * H + q] = acc[0] + (half ? 0.f : r.lstm_b[q]);
+  }
+}
+
+// Shared-memory tiled, 64 x 64 outputs per CTA, 16 deep, 4 x 4 outputs per thread.
 #define GT 64
 #define GK 16
 __global__ void __launch_bounds__(NT) k_velo_gates(const pylo_velo_rnn r) {
@@ -1678,12 +1739,21 @@ __global__ void __launch_bounds__(NT) k_velo_gates(const pylo_velo_rnn r) {
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // cell update; gate order i, g, f, o with f + 1 (VeLO_RNN.py:57-65)
-__global__ void k_velo_cell(const pylo_velo_rnn r) {
+// parts: 1, or 2 where the gates are left as two partial sums (the second [T][4H] block)
+__global__ void k_velo_cell(const pylo_velo_rnn r, int parts) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (int64_t)r.T * r.H) return;
   const int t = (int)(e / r.H), h = (int)(e % r.H), H = r.H;
-  const float* g4 = r.gates + (int64_t)t * 4 * H;
-  const float i = sigmoidf_(g4[h]), g = tanhf(g4[H + h]), f = sigmoidf_(g4[2 * H + h] + 1.0f), o = sigmoidf_(g4[3 * H + h]);
+  const float* g4 = r.gates + (int64_t)t * 4 * H + h;
+  float a[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) a[k] = g4[k * H];
+  if (parts == 2) {
+    const float* g5 = g4 + (int64_t)r.T * 4 * H;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a[k] += g5[k * H];
+  }
+  const float i = sigmoidf_(a[0]), g = tanhf(a[1]), f = sigmoidf_(a[2] + 1.0f), o = sigmoidf_(a[3]);
   const float c = f * r.c[e] + i * g;
   r.c[e] = c;
   r.h[e] = o * tanhf(c);
@@ -1706,17 +1776,26 @@ __global__ void __launch_bounds__(NT) k_velo_heads(const pylo_velo_rnn r) {
   }
 }
 
-// weights[tensor][e] = mean_b(control[b] * bank[b][e]) * 100 (VeLO_MLP.py:92-126); block per tensor
-__global__ void __launch_bounds__(160) k_velo_mix(const pylo_velo_rnn r) {
+// weights[tensor][e] = mean_b(control[b] * bank[b][e]) * 100 (VeLO_MLP.py:92-126); block per tensor, the bank dealt to four
+// groups of threads
+#define MIX_GROUPS 4
+__global__ void __launch_bounds__(160 * MIX_GROUPS) k_velo_mix(const pylo_velo_rnn r) {
   extern __shared__ float s_ctrl[];
+  __shared__ float s_part[MIX_GROUPS][160];
   const int tensor = blockIdx.x;
   const int row = r.T - 1 - tensor;
   for (int b = threadIdx.x; b < r.B; b += blockDim.x) s_ctrl[b] = r.controls[(int64_t)row * r.B + b];
   __syncthreads();
-  const int e = threadIdx.x;
+  const int e = threadIdx.x % 160, grp = threadIdx.x / 160;
+  float acc = 0.f;
   if (e < 159) {
-    float acc = 0.f;
-    for (int b = 0; b < r.B; ++b) acc = fmaf(s_ctrl[b], r.bank[(int64_t)b * 159 + e], acc);
+#pragma unroll 8
+    for (int b = grp; b < r.B; b += MIX_GROUPS) acc = fmaf(s_ctrl[b], r.bank[(int64_t)b * 159 + e], acc);
+  }
+  s_part[grp][e] = acc;
+  __syncthreads();
+  if (threadIdx.x < 159) {
+    acc = (s_part[0][e] + s_part[1][e]) + (s_part[2][e] + s_part[3][e]);
     r.weights[(int64_t)tensor * 160 + e] = acc / (float)r.B * 100.0f;
   }
 }
@@ -2067,13 +2146,24 @@ int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   const pylo_velo_rnn r = *rnn;
   const int64_t TH = (int64_t)r.T * r.H;
-  k_velo_pool<<<(r.H + 127) / 128, 128, 0, s>>>(r);
-  k_velo_xmix<<<(unsigned)((TH + 255) / 256), 256, 0, s>>>(r);
-  k_velo_gates<<<dim3((4 * r.H + GT - 1) / GT, (r.T + GT - 1) / GT), NT, 0, s>>>(r);
-  k_velo_cell<<<(unsigned)((TH + 255) / 256), 256, 0, s>>>(r);
+  k_velo_xmix<<<(r.H + NWARP - 1) / NWARP, NT, 0, s>>>(r);
+  int parts = 1;
+  if (r.H % 128 == 0 && r.H <= 512) {
+    parts = 2;
+    const int gx = 4 * r.H / GR_ROWS, groups = (r.T + 7) / 8;
+    const int gy = groups * gx <= 2 * sm_count() ? groups : (2 * sm_count() / gx > 0 ? 2 * sm_count() / gx : 1);   // two CTAs per SM
+    const int per = (groups + gy - 1) / gy, smem = 2 * 8 * 2 * r.H * (int)sizeof(float);
+    static bool configured[4][PYLO_MAX_DEVICES] = {};
+    auto kernel = r.H == 128 ? k_velo_gates_rows<1> : r.H == 256 ? k_velo_gates_rows<2> : r.H == 384 ? k_velo_gates_rows<3> : k_velo_gates_rows<4>;
+    if (int rc = allow_dynamic_smem(kernel, smem, configured[r.H / 128 - 1])) return rc;
+    kernel<<<dim3(gx, gy), NT, smem, s>>>(r, per);
+  } else {
+    k_velo_gates<<<dim3((4 * r.H + GT - 1) / GT, (r.T + GT - 1) / GT), NT, 0, s>>>(r);
+  }
+  k_velo_cell<<<(unsigned)((TH + 255) / 256), 256, 0, s>>>(r, parts);
   const int64_t hw = (int64_t)r.T * (r.B + 1);
   k_velo_heads<<<(unsigned)((hw + NWARP - 1) / NWARP), NT, 0, s>>>(r);
-  k_velo_mix<<<r.T, 160, r.B * sizeof(float), s>>>(r);
+  k_velo_mix<<<r.T, 160 * MIX_GROUPS, r.B * sizeof(float), s>>>(r);
   return launch_status();
 }
 

@@ -204,7 +204,7 @@ class VeLO_CUDA(Optimizer):
         f32 = dict(dtype=torch.float32, device=dev)
         buf = {
             "weights": torch.zeros(T, 160, **f32), "lr_mult": torch.zeros(T, **f32), "x_in": torch.zeros(T, 30, **f32),
-            "pooled": torch.zeros(H, **f32), "xmix": torch.zeros(T, H, **f32), "gates": torch.zeros(T, 4 * H, **f32),
+            "pooled": torch.zeros(H, **f32), "xmix": torch.zeros(T, H, **f32), "gates": torch.zeros(2, T, 4 * H, **f32),
             "controls": torch.zeros(T, B, **f32), "loss9": torch.zeros(9, **f32), "fraction9": torch.zeros(9, **f32),
             "rank": torch.stack([self.state[p]["rank_onehot"] for p in plist]).contiguous(),
             "loss": torch.zeros(1, **f32),

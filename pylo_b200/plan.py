@@ -347,6 +347,11 @@ class LoPlan:
             k = next((k for k in range(3) if n_items(k + 1) > L.TC_WORKERS), 3)
             shapes_c = [(u, X, Y, max(1, rt >> k), w, tag | max(1, rt >> k)) for u, X, Y, rt, w, tag in shapes_c]
             slow_units = []
+        elif family != L.FAM_ADAFAC:
+            # fewer rows per thread (16, 8, 4 or 2) while the model does not give every SM its two CTAs
+            n_items = lambda k: sum(-(-X // (rt >> k)) * -(-Y // w) for _, X, Y, rt, w, _ in shapes_c)
+            k = next((k for k in range(3) if n_items(k) >= 4 * L.SM_COUNT), 3)
+            shapes_c = [(u, X, Y, rt >> k, w, tag | (16 >> k) << 16) for u, X, Y, rt, w, tag in shapes_c]
         for u, X, Y, rt, width, tag in shapes_c:
             ctiles.append(atile_grid(u, (X + rt - 1) // rt, (Y + width - 1) // width, tag))
         self.ctiles = DeviceTable(atile_list(ctiles), self.device)
