@@ -272,9 +272,10 @@ int pylo_b200_apply_adafac_cols(const pylo_tensor_desc* descs, const pylo_atile*
  * index, cb = 0; an item is that many runs of 128 consecutive elements; generic != 0 says that the list may hold such
  * items.  status: device int; the kernel ORs 1 into it if a wait on the tensor
  * core ran out (the parameters it could not finish then keep their old values), and a launch that finds it
- * non-zero stores nothing; may be NULL. */
+ * non-zero stores nothing; may be NULL.  host_status: a word of pinned (device-accessible) host memory that both events
+ * are also written to, so that the host can look without asking the device; may be NULL. */
 int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* ttiles, int n_ttiles, int generic,
-                              const pylo_step_params* prm, int* status, void* stream);
+                              const pylo_step_params* prm, int* status, int* host_status, void* stream);
 
 /* Phase C for the FAST2D tensors of the CELO2 and VELO families (same arithmetic as pylo_b200_apply, done on
  * pairs of adjacent elements with packed fp32x2 instructions).  ctiles: strip = row-tile index, cb = column-tile
@@ -330,7 +331,8 @@ int pylo_b200_celo2_post_apply(const pylo_post_item* items, const pylo_tile* til
 
 /* AdamW branch for 1-D / embedding tensors.
  * independent != 0: CELO2_cuda.py:234-253 (own exp_avg/exp_avg_sq, betas b1,b2, bias correction with step t);
- * independent == 0: ELO_CELO2_cuda.py:244-253 (updates shared mom[3]/rms with prm, steps from mom[0], rms). */
+ * independent == 0: ELO_CELO2_cuda.py:244-253 (updates shared mom[3]/rms with prm, steps from mom[0], rms).
+ * bc1 > 0: bc1 and bc2 replace the items' own (all tensors are at the same step, no table to upload). */
 typedef struct pylo_adam_item {
   const float* g;
   float* p;
@@ -342,7 +344,7 @@ typedef struct pylo_adam_item {
 } pylo_adam_item;
 int pylo_b200_adamw(const pylo_adam_item* items, const pylo_tile* tiles, int n_tiles, int independent,
                     float beta1, float one_minus_beta1, float beta2, float one_minus_beta2, float eps,
-                    const pylo_step_params* prm, void* stream);
+                    float bc1, float bc2, const pylo_step_params* prm, void* stream);
 
 /* VeLO front end.  velo_tensor_features: desc.sums -> the [T][30] LSTM input rows, row T-1-t for
  * tensor t (velo_cuda.py:213-252,419-422); loss features and fraction features are passed in.
@@ -367,14 +369,45 @@ typedef struct pylo_velo_rnn {
   float *lr_mult;                                 /* out [T] */
   int32_t T, H, B, pad_;
 } pylo_velo_rnn;
+/* The loss buffer (BufferLossAccumulators, velo_cuda.py:170-211): means[10], iteration, running_min[10], decays[10], and
+ * the step's loss, a device scalar or (loss == NULL) value. */
+typedef struct pylo_velo_loss {
+  float* means;
+  int32_t* iteration;
+  float* running_min;
+  const float* decays;
+  const float* loss;
+  float value;
+  int32_t pad_;
+} pylo_velo_loss;
+/* fraction9 is a HOST array of 9.  lossbuf (HOST pointer): the same launch first advances the loss buffer and uses its
+ * features; NULL: loss9 holds them (device, [9]). */
 int pylo_b200_velo_tensor_features(const pylo_tensor_desc* descs, int n_local, const int32_t* layer_of,
                                    int n_total, const float* rank_onehot, const float* fraction9,
-                                   const float* loss9, float* x_in, void* stream);
+                                   const pylo_velo_loss* lossbuf, const float* loss9, float* x_in, void* stream);
 int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, void* stream);
-/* BufferLossAccumulators.update + features (velo_cuda.py:183-211) on device; state arrays are the
- * loss_buffer tensors means[10], iteration (int32), running_min[10], decays[10]; writes loss9[9]. */
+/* The loss buffer's update and features alone: writes loss9[9]. */
 int pylo_b200_velo_loss_features(float* means, int32_t* iteration, float* running_min, const float* decays,
                                  const float* loss, float* loss9, void* stream);
+
+/* All tables of one optimizer's tensors, and a step's phases over them in one call: PYLO_STEP_FRONT is rowcol_sums,
+ * factor_update, state_moments (tiles in reverse), finalize_moments; PYLO_STEP_BACK is prep_apply and the apply kernels.
+ * plan and prm are HOST pointers.  ctiles: items of pylo_b200_apply_adafac_tc where tensor_cores is set (the n_ctiles_gen
+ * on units that are not FAST2D first), else of apply_adafac_cols / apply_packed, with the other units in tiles_slow. */
+#define PYLO_STEP_FRONT 1
+#define PYLO_STEP_BACK 2
+#define PYLO_TC_ONE_LAUNCH 4736 /* items below which one launch takes both kinds of items of apply_adafac_tc */
+typedef struct pylo_step_plan {
+  const pylo_tensor_desc *tdesc, *desc; /* per tensor, per unit */
+  const pylo_atile *atiles, *gitems, *pitems, *ctiles;
+  const pylo_tile *tiles, *tiles_slow;
+  int *status, *host_status;
+  int32_t n_tensors, n_units, n_atiles, n_gitems, n_pitems, n_ctiles, n_ctiles_gen, n_tiles, n_tiles_slow, tensor_cores;
+} pylo_step_plan;
+int pylo_b200_step(const pylo_step_plan* plan, const pylo_step_params* prm, int phases, void* stream);
+/* Host only: adds 1 to n step counters (HOST pointers to doubles); first: the old value of the first, equal: whether all
+ * old values were the same. */
+int pylo_b200_advance_steps(double* const* steps, int n, double* first, int* equal);
 
 #ifdef __cplusplus
 }

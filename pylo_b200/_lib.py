@@ -82,6 +82,20 @@ class VeloRnn(C.Structure):
         ("T", C.c_int32), ("H", C.c_int32), ("B", C.c_int32), ("pad_", C.c_int32)]
 
 
+class VeloLoss(C.Structure):
+    """pylo_velo_loss: the loss buffer's tensors and the step's loss."""
+    _fields_ = [(name, C.c_void_p) for name in ("means", "iteration", "running_min", "decays", "loss")] + [
+        ("value", C.c_float), ("pad_", C.c_int32)]
+
+
+class StepPlan(C.Structure):
+    """pylo_step_plan: all tables of one optimizer's tensors."""
+    _fields_ = [(name, C.c_void_p) for name in (
+        "tdesc", "desc", "atiles", "gitems", "pitems", "ctiles", "tiles", "tiles_slow", "status", "host_status")] + [
+        (name, C.c_int32) for name in ("n_tensors", "n_units", "n_atiles", "n_gitems", "n_pitems", "n_ctiles", "n_ctiles_gen",
+                                       "n_tiles", "n_tiles_slow", "tensor_cores")]
+
+
 class PyloLibError(RuntimeError):
     pass
 
@@ -112,16 +126,18 @@ def _load():
         "pylo_b200_prep_apply": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply_adafac_cols": [vp, vp, i32, C.POINTER(StepParams), vp],
-        "pylo_b200_apply_adafac_tc": [vp, vp, i32, i32, C.POINTER(StepParams), vp, vp],
+        "pylo_b200_apply_adafac_tc": [vp, vp, i32, i32, C.POINTER(StepParams), vp, vp, vp],
         "pylo_b200_apply_packed": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_gemm_tn_3xtf32": [C.POINTER(GemmDesc), vp, vp],
         "pylo_b200_transpose": [vp, vp, i32, i32, i32, i32, C.c_int64, C.c_int64, i32, i32, vp],
         "pylo_b200_celo2_post_sums": [vp, vp, i32, vp],
         "pylo_b200_celo2_post_apply": [vp, vp, i32, vp],
-        "pylo_b200_adamw": [vp, vp, i32, i32, f32, f32, f32, f32, f32, C.POINTER(StepParams), vp],
-        "pylo_b200_velo_tensor_features": [vp, i32, vp, i32, vp, vp, vp, vp, vp],
+        "pylo_b200_adamw": [vp, vp, i32, i32] + [f32] * 7 + [C.POINTER(StepParams), vp],
+        "pylo_b200_velo_tensor_features": [vp, i32, vp, i32, vp, vp, C.POINTER(VeloLoss), vp, vp, vp],
         "pylo_b200_velo_rnn": [C.POINTER(VeloRnn), vp],
         "pylo_b200_velo_loss_features": [vp, vp, vp, vp, vp, vp, vp],
+        "pylo_b200_step": [C.POINTER(StepPlan), C.POINTER(StepParams), i32, vp],
+        "pylo_b200_advance_steps": [vp, i32, C.POINTER(C.c_double), C.POINTER(C.c_int)],
     }
     for name, argtypes in sigs.items():
         fn = getattr(lib, name)  # AttributeError if a declared symbol is missing
@@ -140,6 +156,8 @@ lib, EXPORTED = _load()
 SM_COUNT = 148        # of a B200; sizes of work lists only, the kernels ask the device
 TC_WORKERS = SM_COUNT * 4  # warpgroups the tensor-core apply kernel runs at once (four per SM)
 TC_GEN_ITEM = 1 << 16  # tag bit of its items on tensors that are not FAST2D
+STEP_FRONT, STEP_BACK = 1, 2
+TC_ONE_LAUNCH = 8 * TC_WORKERS  # items below which one launch of the tensor-core kernel takes both kinds of items
 STATIC_SCRATCH_TILES = 65536
 ERR_STATIC_SCRATCH_TOO_SMALL = -4
 

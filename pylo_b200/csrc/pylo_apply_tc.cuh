@@ -29,7 +29,8 @@
 //   * the products are issued by one elected lane inside a warp-uniform branch (the warp index is a broadcast
 //     from lane 0), so that their descriptors and tensor-memory addresses live in uniform registers: issued from
 //     a branch on the thread index, each product cost its thread ~52 cycles; this way ~24.
-// Every wait on the tensor core is bounded.  A thread whose wait ran out records it in *status, stops waiting
+// Every wait on the tensor core is bounded.  A thread whose wait ran out records it in *status (and in *host_status, a word
+// of pinned host memory that the host looks at without asking the device), stops waiting
 // and stops storing (its parameters, and their copies on the peers, keep their old values), and goes on to
 // the end, where the kernel frees its tensor memory.  A launch that finds *status already set stores nothing.
 #pragma once
@@ -214,7 +215,8 @@ struct TcSmem {
 template <bool GENERIC>
 __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const pylo_tensor_desc* __restrict__ descs,
                                                               const pylo_atile* __restrict__ ttiles, int n_ttiles,
-                                                              const pylo_step_params prm, int* __restrict__ status) {
+                                                              const pylo_step_params prm, int* __restrict__ status,
+                                                              int* __restrict__ host_status) {
   using F = Fam<PYLO_FAM_ADAFAC>;
   using L = Fold<PYLO_FAM_ADAFAC>;
   extern __shared__ __align__(128) unsigned char tc_raw[];
@@ -229,6 +231,7 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
   if (col == 0) mbar_init(&sm.bar, 1);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   for (int e = tid; e < TC_ONES_BYTES / 4; e += TC_NT) smem.ones[e] = (e & 3) < 2 ? 1.0f : 0.0f;
+  pdl_begin();  // the set-up so far overlaps the previous kernel's end
   if (tid == 32) smem.poisoned = status ? *reinterpret_cast<volatile int*>(status) : 0;
   if (warp == 0) { tc_alloc(&smem.tmem_base, 512); tc_relinquish(); }
   fence_async_smem();  // the constant operand is read by the tensor core through the async proxy
@@ -238,6 +241,7 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
   // A launch that finds the status word already set writes nothing (no parameter, no peer store): the
   // parameters stay as the last good step left them until the host has looked at the error and cleared it.
   const int n_items = smem.poisoned ? 0 : n_ttiles;
+  if (smem.poisoned && host_status && blockIdx.x == 0 && tid == 0) *reinterpret_cast<volatile int*>(host_status) = smem.poisoned;
   const uint32_t t_wg = __shfl_sync(0xffffffffu, smem.tmem_base, 0) + wg * TC_WG_TMEM;   // lane 0 of this warpgroup's columns
   const uint32_t t_lane = t_wg + ((uint32_t)((warp & 3) * 32) << 16);   // this warp's 32 lanes
   const uint32_t tA = t_lane, tD = t_lane + 64;
@@ -532,6 +536,7 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
   }
   TC_CLK_FLUSH
   if (timed_out && status) atomicOr(status, 1);
+  if (timed_out && host_status) *reinterpret_cast<volatile int*>(host_status) = 1;
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tc_dealloc(smem.tmem_base, 512);

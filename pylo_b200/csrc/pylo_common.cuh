@@ -67,6 +67,13 @@ __device__ __forceinline__ void static_for(Fn&& fn) {
   }
 }
 
+// First statement of every kernel: let the next kernel of the stream be set up, then wait until the previous one is
+// complete and its writes are visible.  Nothing that a predecessor may write is read before.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ----------------------------------------------------------------------------------------------
 // scalar helpers
 // ----------------------------------------------------------------------------------------------

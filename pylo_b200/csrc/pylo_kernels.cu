@@ -48,6 +48,7 @@ __device__ __forceinline__ void vec_features(float* f, float r0, float r1, float
 __global__ void __launch_bounds__(NT) k_grad_sumsq(const pylo_gvec* __restrict__ descs,
                                                    const pylo_tile* __restrict__ tiles, int n_tiles,
                                                    float* __restrict__ scratch) {
+  pdl_begin();
   __shared__ float s_red[40];
   for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const pylo_tile tl = tiles[t];
@@ -70,6 +71,7 @@ __global__ void __launch_bounds__(NT) k_grad_sumsq(const pylo_gvec* __restrict__
 }
 
 __global__ void __launch_bounds__(1024) k_sum_final(const float* __restrict__ scratch, int n, float* __restrict__ out) {
+  pdl_begin();
   __shared__ double s_d[32];
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) acc += (double)scratch[i];
@@ -94,6 +96,7 @@ __global__ void __launch_bounds__(1024) k_sum_final(const float* __restrict__ sc
 __global__ void __launch_bounds__(NT, 4) k_rowcol_fast(const pylo_tensor_desc* __restrict__ descs,
                                                        const pylo_atile* __restrict__ atiles, int n_atiles,
                                                        const pylo_step_params prm) {
+  pdl_begin();
   __shared__ float s_col[RC_GROUPS][PYLO_A_COLS];
   __shared__ float s_row[PYLO_A_ROWS_MAX][2];
   const int lane = threadIdx.x & 31, half = (threadIdx.x >> 5) & 1, grp = threadIdx.x >> 6;
@@ -170,6 +173,7 @@ __global__ void __launch_bounds__(NT, 4) k_rowcol_fast(const pylo_tensor_desc* _
 __global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* __restrict__ descs,
                                                        const pylo_atile* __restrict__ items,
                                                        const pylo_step_params prm) {
+  pdl_begin();
   __shared__ float s_red[40];
   const pylo_atile it = items[blockIdx.x];
   const pylo_tensor_desc& d = descs[it.tensor];
@@ -271,6 +275,7 @@ __device__ __forceinline__ void cluster_store(float* p, uint32_t rank, float v) 
 template <int FAM>
 __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_factor_update(const pylo_tensor_desc* __restrict__ descs,
                                                                                           const pylo_step_params prm) {
+  pdl_begin();
   using F = Fam<FAM>;
   constexpr int NS = 15;  // sums per CTA: row accumulator (its mean), then the four closed forms, three decays each
   __shared__ float s_part[A2_NT / 128][128];
@@ -457,6 +462,7 @@ template <int FAM>
 __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc* __restrict__ descs,
                                                       const pylo_tile* __restrict__ tiles, int n_tiles, int reverse,
                                                       const pylo_step_params prm) {
+  pdl_begin();
   using F = Fam<FAM>;
   constexpr int NACC = BAcc<FAM>::N;
   __shared__ float s_red[NWARP * NACC];
@@ -609,6 +615,7 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
 // Latency-bound: a 58 M-element tensor leaves 3584 rows of 40 partials.  The rows are read as one stretch of memory, 25
 // (or six) at a time, every thread keeping its column; eight rows ahead are in flight.
 __global__ void __launch_bounds__(1024) k_finalize_moments(const pylo_tensor_desc* __restrict__ descs) {
+  pdl_begin();
   __shared__ double s_d[25][PYLO_STAT_STRIDE];
   const pylo_tensor_desc& d = descs[blockIdx.x];
   const int rows = blockDim.x / PYLO_STAT_STRIDE;
@@ -649,6 +656,7 @@ __device__ __forceinline__ float w1_at(int fam, const float* w, int j, int k) {
 template <int FAM>
 __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __restrict__ descs,
                                                    const pylo_atile* __restrict__ items, const pylo_step_params prm) {
+  pdl_begin();
   using F = Fam<FAM>;
   using L = Fold<FAM>;
   constexpr int H = F::H, NF = F::NF, NIN = F::NIN;
@@ -862,6 +870,7 @@ template <int FAM>
 __global__ void __launch_bounds__(NT) k_apply(const pylo_tensor_desc* __restrict__ descs,
                                               const pylo_tile* __restrict__ tiles, int n_tiles, int reverse,
                                               const pylo_step_params prm) {
+  pdl_begin();
   using F = Fam<FAM>;
   using L = Fold<FAM>;
   constexpr int H = F::H;
@@ -1005,6 +1014,7 @@ struct CcSmem {
 __global__ void __launch_bounds__(NT, CC_CTAS_PER_SM) k_apply_adafac_cols(const pylo_tensor_desc* __restrict__ descs,
                                                               const pylo_atile* __restrict__ ctiles, int n_ctiles,
                                                               const pylo_step_params prm) {
+  pdl_begin();
   using F = Fam<PYLO_FAM_ADAFAC>;
   using L = Fold<PYLO_FAM_ADAFAC>;
   constexpr int E = CC_E;
@@ -1265,6 +1275,7 @@ template <int FAM>
 __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : 2) k_apply_packed(const pylo_tensor_desc* __restrict__ descs,
                                                         const pylo_atile* __restrict__ ctiles, int n_ctiles,
                                                         const pylo_step_params prm) {
+  pdl_begin();
   using F = Fam<FAM>;
   using L = Fold<FAM>;
   using W = PkW<FAM>;
@@ -1427,6 +1438,7 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : 2) k
 // ================================================================================================
 __global__ void __launch_bounds__(NT) k_post_sums(const pylo_post_item* __restrict__ items,
                                                   const pylo_tile* __restrict__ tiles, int n_tiles) {
+  pdl_begin();
   __shared__ float s_red[40];
   for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const pylo_tile tl = tiles[t];
@@ -1451,6 +1463,7 @@ __global__ void __launch_bounds__(NT) k_post_sums(const pylo_post_item* __restri
 
 __global__ void __launch_bounds__(NT) k_post_apply(const pylo_post_item* __restrict__ items,
                                                    const pylo_tile* __restrict__ tiles, int n_tiles) {
+  pdl_begin();
   __shared__ float s_scale;
   for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const pylo_tile tl = tiles[t];
@@ -1485,10 +1498,15 @@ __global__ void __launch_bounds__(NT) k_post_apply(const pylo_post_item* __restr
 // ================================================================================================
 // AdamW branch
 // ================================================================================================
+// Bound by HBM (28 or 44 B per element): float4 where every stream allows it, two pieces of a thread in flight.  262 M
+// elements: 1829 us (4.0 TB/s) with scalar loads before.
+template <bool INDEPENDENT>
 __global__ void __launch_bounds__(NT) k_adamw(const pylo_adam_item* __restrict__ items,
-                                              const pylo_tile* __restrict__ tiles, int n_tiles, int independent,
-                                              float beta1, float omb1, float beta2, float omb2, float eps,
+                                              const pylo_tile* __restrict__ tiles, int n_tiles,
+                                              float beta1, float omb1, float beta2, float omb2, float eps, float bc1_all, float bc2_all,
                                               const pylo_step_params prm) {
+  pdl_begin();
+  constexpr int NM = INDEPENDENT ? 1 : 3;
   for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const pylo_tile tl = tiles[t];
     const pylo_adam_item& it = items[tl.tensor];
@@ -1499,28 +1517,52 @@ __global__ void __launch_bounds__(NT) k_adamw(const pylo_adam_item* __restrict__
       const float denom = fmaxf(sqrtf(*prm.gnorm_sq), it.clip_norm);
       gs = denom > 0.f ? it.clip_norm / denom : 1.0f;
     }
-    const float* gp = it.g + tl.start;
-    float* pp = it.p + tl.start;
-    float* vp = it.v + tl.start;
-    float* mp = it.m + tl.start;
-    for (int i = threadIdx.x; i < cnt; i += NT) {
-      const float g = xform_grad(gp[i], gs, prm.clip_val, prm.nan_to_num);
-      const float p = pp[i];
-      float m, v;
-      if (independent) {  // exp_avg.mul_(b1).add_(g, alpha=1-b1); exp_avg_sq.mul_(b2).addcmul_(g, g, value=1-b2)
-        m = fmaf(g, omb1, mp[i] * beta1);
-        v = fmaf(g * g, omb2, vp[i] * beta2);
-        mp[i] = m;
+    const float bc1 = bc1_all > 0.f ? bc1_all : it.bc1, bc2 = bc1_all > 0.f ? bc2_all : it.bc2;
+    const float lr = it.lr, wd = it.wd;
+    const float* __restrict__ gp = it.g + tl.start;
+    float* __restrict__ pp = it.p + tl.start;
+    float* __restrict__ vp = it.v + tl.start;
+    float* __restrict__ mp = it.m + tl.start;
+    auto element = [&](float g, float& p, float& v, float (&m)[NM]) {
+      g = xform_grad(g, gs, prm.clip_val, prm.nan_to_num);
+      if (INDEPENDENT) {  // exp_avg.mul_(b1).add_(g, alpha=1-b1); exp_avg_sq.mul_(b2).addcmul_(g, g, value=1-b2)
+        m[0] = fmaf(g, omb1, m[0] * beta1);
+        v = fmaf(g * g, omb2, v * beta2);
       } else {  // shared accumulators: all three momenta advance, the step uses decay 0
-        m = lerp_torch(mp[i], g, prm.w_m[0]);
-        mp[i] = m;
-        mp[n + i] = lerp_torch(mp[n + i], g, prm.w_m[1]);
-        mp[2 * n + i] = lerp_torch(mp[2 * n + i], g, prm.w_m[2]);
-        v = lerp_torch(vp[i], g * g, prm.w_v);
+#pragma unroll
+        for (int k = 0; k < NM; ++k) m[k] = lerp_torch(m[k], g, prm.w_m[k]);
+        v = lerp_torch(v, g * g, prm.w_v);
       }
+      const float upd = (m[0] / bc1) / (sqrtf(v / bc2) + eps);
+      p = fmaf(-lr, fmaf(wd, p, upd), p);
+    };
+    const bool al = ((((uintptr_t)gp | (uintptr_t)pp | (uintptr_t)vp | (uintptr_t)mp) & 15) == 0) && (INDEPENDENT || (n & 3) == 0);
+    const int c4 = al ? (cnt & ~3) : 0;
+#pragma unroll 2
+    for (int i = threadIdx.x * 4; i < c4; i += NT * 4) {
+      const float4 g4 = ldg4(gp + i), p4 = ld4(pp + i), v4 = ld4(vp + i);
+      float4 m4[NM];
+#pragma unroll
+      for (int k = 0; k < NM; ++k) m4[k] = ld4(mp + k * n + i);
+      float g[4] = {g4.x, g4.y, g4.z, g4.w}, p[4] = {p4.x, p4.y, p4.z, p4.w}, v[4] = {v4.x, v4.y, v4.z, v4.w}, m[4][NM];
+#pragma unroll
+      for (int k = 0; k < NM; ++k) { m[0][k] = m4[k].x; m[1][k] = m4[k].y; m[2][k] = m4[k].z; m[3][k] = m4[k].w; }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) element(g[u], p[u], v[u], m[u]);
+      st4(pp + i, make_float4(p[0], p[1], p[2], p[3]));
+      st4(vp + i, make_float4(v[0], v[1], v[2], v[3]));
+#pragma unroll
+      for (int k = 0; k < NM; ++k) st4(mp + k * n + i, make_float4(m[0][k], m[1][k], m[2][k], m[3][k]));
+    }
+    for (int i = c4 + threadIdx.x; i < cnt; i += NT) {
+      float p = pp[i], v = vp[i], m[NM];
+#pragma unroll
+      for (int k = 0; k < NM; ++k) m[k] = mp[k * n + i];
+      element(gp[i], p, v, m);
+      pp[i] = p;
       vp[i] = v;
-      const float upd = (m / it.bc1) / (sqrtf(v / it.bc2) + eps);
-      pp[i] = fmaf(-it.lr, fmaf(it.wd, p, upd), p);
+#pragma unroll
+      for (int k = 0; k < NM; ++k) mp[k * n + i] = m[k];
     }
   }
 }
@@ -1532,72 +1574,92 @@ __device__ __forceinline__ float clip_log_abs10(float v) {
   return fminf(fmaxf(logf(1e-8f + fabsf(v * 10.0f)), -5.f), 5.f) * 0.5f;
 }
 
-// one thread per tensor: the 30 LSTM inputs from the statistics gathered in phase B (velo_cuda.py:213-252)
-__global__ void k_velo_tensor_features(const pylo_tensor_desc* __restrict__ descs, int n_local,
-                                       const int32_t* __restrict__ layer_of, int T,
-                                       const float* __restrict__ rank_onehot, const float* __restrict__ fraction9,
-                                       const float* __restrict__ loss9, float* __restrict__ x_in) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_local) return;
-  const int layer = layer_of ? layer_of[t] : t;  // position of this tensor among all T tensors of the model
-  const pylo_tensor_desc& d = descs[t];
-  const double n = (double)d.n;
-  auto stat = [&](int j) { return (double)d.sums[30 + j] + (double)d.sums[SUMS_LO + j]; };
-  const float mean_p2 = (float)((double)d.sums[2] / n);
-  const double norm = (double)rsqrtf(fmaxf(mean_p2, 1e-9f));
-  float* o = x_in + (int64_t)(T - 1 - layer) * 30;  // rows are flipped (velo_cuda.py:422)
-#pragma unroll
-  for (int j = 0; j < 9; ++j) { o[j] = fraction9[j]; o[9 + j] = loss9[j]; }
-  const double mean_v = stat(6) / n, e_v2 = stat(7) / n;
-  o[18] = clip_log_abs10((float)(norm * mean_v));
-#pragma unroll
-  for (int j = 0; j < 5; ++j) o[19 + j] = rank_onehot[t * 5 + j];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const double mu = stat(k) / n, e_m2 = stat(3 + k) / n;
-    const double var_m = fmax(e_m2 - mu * mu, 0.0);
-    const double var_v = fmax(e_v2 - 2.0 * mu * mean_v + mu * mu, 0.0);  // mean((rms - mean_m)^2), velo_cuda.py:243
-    o[24 + k] = clip_log_abs10((float)(norm * norm * var_m));
-    o[27 + k] = clip_log_abs10((float)(norm * norm * var_v));
-  }
-}
-
-// BufferLossAccumulators.update followed by .features (velo_cuda.py:183-211); one warp
-__global__ void k_velo_loss(float* means, int32_t* iteration, float* running_min, const float* __restrict__ decays,
-                            const float* __restrict__ loss_in, float* __restrict__ loss9) {
+// BufferLossAccumulators.update followed by .features (velo_cuda.py:183-211); one warp, loss9 may be shared memory
+__device__ __forceinline__ void velo_loss_update(const pylo_velo_loss& b, float* loss9) {
   __shared__ float s_cor[10];
-  const int j = threadIdx.x;
-  const int it = *iteration;
+  const int j = threadIdx.x & 31;
+  const int it = *b.iteration;
+  const float loss_in = b.loss ? b.loss[0] : b.value;
   float cor = -CUDART_INF_F;
-  if (j < 10) cor = means[j] / (1.0f - powf(decays[j], (float)(it + 1)));
+  if (j < 10) cor = b.means[j] / (1.0f - powf(b.decays[j], (float)(it + 1)));
   float mx = cor;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const float approx_max = it == 0 ? loss_in[0] : mx;
-  const float loss = fminf(fabsf(approx_max) * 2.0f, loss_in[0]);
+  const float approx_max = it == 0 ? loss_in : mx;
+  const float loss = fminf(fabsf(approx_max) * 2.0f, loss_in);
+  float rmin = 0.f;
   if (j < 10) {
-    const float dj = decays[j];
-    const float mnew = means[j] * dj + loss * (1.0f - dj);
-    const float c2 = mnew / (1.0f - powf(dj, (float)(it + 1)));
-    const float rmin = fminf(running_min[j], c2);
-    means[j] = mnew;
-    running_min[j] = rmin;
-    s_cor[j] = mnew / (1.0f - powf(dj, (float)(it + 1)));  // features() uses iteration after the increment
+    const float dj = b.decays[j];
+    const float mnew = b.means[j] * dj + loss * (1.0f - dj);
+    const float c2 = mnew / (1.0f - powf(dj, (float)(it + 1)));  // features() uses iteration after the increment
+    rmin = fminf(b.running_min[j], c2);
+    b.means[j] = mnew;
+    b.running_min[j] = rmin;
+    s_cor[j] = c2;
   }
   __syncwarp();
   if (j < 9) {
-    const float rmin = running_min[j];
     const float den = fmaxf(1e-8f, s_cor[j + 1] - rmin);
     float f = fminf(fmaxf((s_cor[j] - rmin) / den - 1.0f, -1.f), 1.f);
     loss9[j] = (it + 1 <= 2) ? f * 0.f : f;
   }
   __syncwarp();
-  if (j == 0) *iteration = it + 1;
+  if (j == 0) *b.iteration = it + 1;
+}
+
+__global__ void k_velo_loss(const pylo_velo_loss b, float* __restrict__ loss9) {
+  pdl_begin();
+  velo_loss_update(b, loss9);
+}
+
+// One CTA: its first warp advances the loss buffer (where it is given), then one thread per tensor makes the 30 LSTM inputs
+// from the statistics gathered in phase B (velo_cuda.py:213-252).
+struct VeloFraction { float f[9]; };
+__global__ void __launch_bounds__(512) k_velo_tensor_features(const pylo_tensor_desc* __restrict__ descs, int n_local,
+                                       const int32_t* __restrict__ layer_of, int T,
+                                       const float* __restrict__ rank_onehot, const VeloFraction fraction9,
+                                       const pylo_velo_loss lossbuf, const float* __restrict__ loss9, float* __restrict__ x_in) {
+  pdl_begin();
+  __shared__ float s_loss9[9];
+  if (lossbuf.means) {
+    if (threadIdx.x < 32) velo_loss_update(lossbuf, s_loss9);
+  } else if (threadIdx.x < 9) {
+    s_loss9[threadIdx.x] = loss9[threadIdx.x];
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < n_local; t += blockDim.x) {
+    const int layer = layer_of ? layer_of[t] : t;  // position of this tensor among all T tensors of the model
+    const pylo_tensor_desc& d = descs[t];
+    const double n = (double)d.n;
+    const float* __restrict__ sums = d.sums;
+    float st[8], lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { st[j] = sums[30 + j]; lo[j] = sums[SUMS_LO + j]; }
+    auto stat = [&](int j) { return (double)st[j] + (double)lo[j]; };
+    const float mean_p2 = (float)((double)sums[2] / n);
+    const double norm = (double)rsqrtf(fmaxf(mean_p2, 1e-9f));
+    float* o = x_in + (int64_t)(T - 1 - layer) * 30;  // rows are flipped (velo_cuda.py:422)
+#pragma unroll
+    for (int j = 0; j < 9; ++j) { o[j] = fraction9.f[j]; o[9 + j] = s_loss9[j]; }
+    const double mean_v = stat(6) / n, e_v2 = stat(7) / n;
+    o[18] = clip_log_abs10((float)(norm * mean_v));
+#pragma unroll
+    for (int j = 0; j < 5; ++j) o[19 + j] = rank_onehot[t * 5 + j];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double mu = stat(k) / n, e_m2 = stat(3 + k) / n;
+      const double var_m = fmax(e_m2 - mu * mu, 0.0);
+      const double var_v = fmax(e_v2 - 2.0 * mu * mean_v + mu * mu, 0.0);  // mean((rms - mean_m)^2), velo_cuda.py:243
+      o[24 + k] = clip_log_abs10((float)(norm * norm * var_m));
+      o[27 + k] = clip_log_abs10((float)(norm * norm * var_v));
+    }
+  }
 }
 
 // x' = final_mix(x) + max_t relu(mix2(x)).  One warp per hidden unit, lanes along the tensors (one thread per unit walked
 // through all tensors by itself: 203 us at 292 tensors).
 __global__ void __launch_bounds__(NT) k_velo_xmix(const pylo_velo_rnn r) {
+  pdl_begin();
   const int h = blockIdx.x * NWARP + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (h >= r.H) return;
   float best = 0.f;   // relu
@@ -1632,6 +1694,7 @@ __global__ void __launch_bounds__(NT) k_velo_xmix(const pylo_velo_rnn r) {
 #define GR_ROWS 16   // weight rows per CTA: four per pair of warps
 template <int NI>    // float4 per lane and row: H = 128 * NI
 __global__ void __launch_bounds__(NT, 2) k_velo_gates_rows(const pylo_velo_rnn r, int groups_per_cta) {
+  pdl_begin();
   extern __shared__ __align__(16) float s_x[];   // [2][8][2H]
   constexpr int H = 128 * NI;
   const int tid = threadIdx.x, lane = tid & 31, half = (tid >> 5) & 1, q0 = blockIdx.x * GR_ROWS + (tid >> 6) * 4;
@@ -1689,6 +1752,7 @@ __global__ void __launch_bounds__(NT, 2) k_velo_gates_rows(const pylo_velo_rnn r
 #define GT 64
 #define GK 16
 __global__ void __launch_bounds__(NT) k_velo_gates(const pylo_velo_rnn r) {
+  pdl_begin();
   __shared__ float s_a[GK][GT + 4];
   __shared__ float s_w[GK][GT + 4];
   const int H = r.H, Q = 4 * H, K = 2 * H, T = r.T;
@@ -1741,6 +1805,7 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf
 // cell update; gate order i, g, f, o with f + 1 (VeLO_RNN.py:57-65)
 // parts: 1, or 2 where the gates are left as two partial sums (the second [T][4H] block)
 __global__ void k_velo_cell(const pylo_velo_rnn r, int parts) {
+  pdl_begin();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (int64_t)r.T * r.H) return;
   const int t = (int)(e / r.H), h = (int)(e % r.H), H = r.H;
@@ -1761,6 +1826,7 @@ __global__ void k_velo_cell(const pylo_velo_rnn r, int parts) {
 
 // controls[t][b] and lr_mult[t]; one warp per output
 __global__ void __launch_bounds__(NT) k_velo_heads(const pylo_velo_rnn r) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t wid = (int64_t)blockIdx.x * NWARP + (threadIdx.x >> 5);
   const int H = r.H, B1 = r.B + 1;
@@ -1780,6 +1846,7 @@ __global__ void __launch_bounds__(NT) k_velo_heads(const pylo_velo_rnn r) {
 // groups of threads
 #define MIX_GROUPS 4
 __global__ void __launch_bounds__(160 * MIX_GROUPS) k_velo_mix(const pylo_velo_rnn r) {
+  pdl_begin();
   extern __shared__ float s_ctrl[];
   __shared__ float s_part[MIX_GROUPS][160];
   const int tensor = blockIdx.x;
@@ -1821,6 +1888,24 @@ static int grid_for(int n_items, int ctas_per_sm) {
   return n_items < cap ? n_items : cap;
 }
 static int launch_status() { return (int)cudaGetLastError(); }
+
+// Every kernel of this library is launched so that it may become resident while its predecessor in the stream drains
+// (programmatic dependent launch) and waits in pdl_begin() until that one is complete.  A step is a chain of small launches;
+// on a small model the gaps between them are as long as the kernels.
+template <class... P, class... A>
+static void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // Opt a kernel in to more than 48 KB of dynamic shared memory, once per device (the attribute belongs to the
 // device's copy of the function); flags[] is the caller's per-kernel record.
@@ -1905,8 +1990,8 @@ int pylo_b200_grad_sumsq(const pylo_gvec* descs, const pylo_tile* tiles, int n_t
                          float* out, void* stream) {
   CHECK_ARG(descs && tiles && scratch && out && n_tiles >= 0);
   cudaStream_t s = (cudaStream_t)stream;
-  if (n_tiles > 0) k_grad_sumsq<<<grid_for(n_tiles, 8), NT, 0, s>>>(descs, tiles, n_tiles, scratch);
-  k_sum_final<<<1, 1024, 0, s>>>(scratch, n_tiles, out);
+  if (n_tiles > 0) launch(k_grad_sumsq, grid_for(n_tiles, 8), NT, 0, s, descs, tiles, n_tiles, scratch);
+  launch(k_sum_final, 1, 1024, 0, s, scratch, n_tiles, out);
   return launch_status();
 }
 
@@ -1955,8 +2040,8 @@ int pylo_b200_grad_sumsq_static(const pylo_gvec* items, const pylo_tile* tiles, 
   cudaStream_t s = (cudaStream_t)stream;
   // every slot that the final sum reads is written by the partial kernel of this same call, so
   // nothing left over from an earlier call needs clearing
-  if (n_tiles > 0) k_grad_sumsq<<<grid_for(n_tiles, 8), NT, 0, s>>>(items, tiles, n_tiles, scratch);
-  k_sum_final<<<1, 1024, 0, s>>>(scratch, n_tiles, out);
+  if (n_tiles > 0) launch(k_grad_sumsq, grid_for(n_tiles, 8), NT, 0, s, items, tiles, n_tiles, scratch);
+  launch(k_sum_final, 1, 1024, 0, s, scratch, n_tiles, out);
   return launch_status();
 }
 
@@ -1966,11 +2051,11 @@ int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atile
   cudaStream_t s = (cudaStream_t)stream;
   if (n_atiles > 0) {
     CHECK_ARG(atiles);
-    k_rowcol_fast<<<grid_for(n_atiles, 4), NT, 0, s>>>(descs, atiles, n_atiles, *prm);
+    launch(k_rowcol_fast, grid_for(n_atiles, 4), NT, 0, s, descs, atiles, n_atiles, *prm);
   }
   if (n_gitems > 0) {
     CHECK_ARG(gitems);
-    k_rowcol_generic<<<n_gitems, NT, 0, s>>>(descs, gitems, *prm);
+    launch(k_rowcol_generic, n_gitems, NT, 0, s, descs, gitems, *prm);
   }
   return launch_status();
 }
@@ -1980,9 +2065,9 @@ int pylo_b200_factor_update(const pylo_tensor_desc* descs, int n_tensors, const 
   if (n_tensors == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: k_factor_update<PYLO_FAM_ADAFAC><<<n_tensors * A2_CL, A2_NT, 0, s>>>(descs, *prm); break;
-    case PYLO_FAM_CELO2: k_factor_update<PYLO_FAM_CELO2><<<n_tensors * A2_CL, A2_NT, 0, s>>>(descs, *prm); break;
-    case PYLO_FAM_VELO: k_factor_update<PYLO_FAM_VELO><<<n_tensors * A2_CL, A2_NT, 0, s>>>(descs, *prm); break;
+    case PYLO_FAM_ADAFAC: launch(k_factor_update<PYLO_FAM_ADAFAC>, n_tensors * A2_CL, A2_NT, 0, s, descs, *prm); break;
+    case PYLO_FAM_CELO2: launch(k_factor_update<PYLO_FAM_CELO2>, n_tensors * A2_CL, A2_NT, 0, s, descs, *prm); break;
+    case PYLO_FAM_VELO: launch(k_factor_update<PYLO_FAM_VELO>, n_tensors * A2_CL, A2_NT, 0, s, descs, *prm); break;
     default: return -2;
   }
   return launch_status();
@@ -1995,9 +2080,9 @@ int pylo_b200_state_moments(const pylo_tensor_desc* descs, const pylo_tile* tile
   cudaStream_t s = (cudaStream_t)stream;
   const int grid = grid_for(n_tiles, 4);
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: k_state_moments<PYLO_FAM_ADAFAC><<<grid, NT, 0, s>>>(descs, tiles, n_tiles, reverse, *prm); break;
-    case PYLO_FAM_CELO2: k_state_moments<PYLO_FAM_CELO2><<<grid, NT, 0, s>>>(descs, tiles, n_tiles, reverse, *prm); break;
-    case PYLO_FAM_VELO: k_state_moments<PYLO_FAM_VELO><<<grid, NT, 0, s>>>(descs, tiles, n_tiles, reverse, *prm); break;
+    case PYLO_FAM_ADAFAC: launch(k_state_moments<PYLO_FAM_ADAFAC>, grid, NT, 0, s, descs, tiles, n_tiles, reverse, *prm); break;
+    case PYLO_FAM_CELO2: launch(k_state_moments<PYLO_FAM_CELO2>, grid, NT, 0, s, descs, tiles, n_tiles, reverse, *prm); break;
+    case PYLO_FAM_VELO: launch(k_state_moments<PYLO_FAM_VELO>, grid, NT, 0, s, descs, tiles, n_tiles, reverse, *prm); break;
     default: return -2;
   }
   return launch_status();
@@ -2007,7 +2092,7 @@ int pylo_b200_finalize_moments(const pylo_tensor_desc* descs, int n_tensors, voi
   CHECK_ARG(descs && n_tensors >= 0);
   if (n_tensors == 0) return 0;
   // many units (the slices of a CELO2 tensor) have few tiles each: small CTAs then
-  k_finalize_moments<<<n_tensors, n_tensors > 512 ? 6 * PYLO_STAT_STRIDE : 25 * PYLO_STAT_STRIDE, 0, (cudaStream_t)stream>>>(descs);
+  launch(k_finalize_moments, n_tensors, n_tensors > 512 ? 6 * PYLO_STAT_STRIDE : 25 * PYLO_STAT_STRIDE, 0, (cudaStream_t)stream, descs);
   return launch_status();
 }
 
@@ -2017,9 +2102,9 @@ int pylo_b200_prep_apply(const pylo_tensor_desc* descs, const pylo_atile* items,
   if (n_items == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: k_prep_apply<PYLO_FAM_ADAFAC><<<n_items, NT, 0, s>>>(descs, items, *prm); break;
-    case PYLO_FAM_CELO2: k_prep_apply<PYLO_FAM_CELO2><<<n_items, NT, 0, s>>>(descs, items, *prm); break;
-    case PYLO_FAM_VELO: k_prep_apply<PYLO_FAM_VELO><<<n_items, NT, 0, s>>>(descs, items, *prm); break;
+    case PYLO_FAM_ADAFAC: launch(k_prep_apply<PYLO_FAM_ADAFAC>, n_items, NT, 0, s, descs, items, *prm); break;
+    case PYLO_FAM_CELO2: launch(k_prep_apply<PYLO_FAM_CELO2>, n_items, NT, 0, s, descs, items, *prm); break;
+    case PYLO_FAM_VELO: launch(k_prep_apply<PYLO_FAM_VELO>, n_items, NT, 0, s, descs, items, *prm); break;
     default: return -2;
   }
   return launch_status();
@@ -2031,9 +2116,9 @@ int pylo_b200_apply(const pylo_tensor_desc* descs, const pylo_tile* tiles, int n
   if (n_tiles == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: k_apply<PYLO_FAM_ADAFAC><<<grid_for(n_tiles, 2), NT, 0, s>>>(descs, tiles, n_tiles, reverse, *prm); break;
-    case PYLO_FAM_CELO2: k_apply<PYLO_FAM_CELO2><<<grid_for(n_tiles, 4), NT, 0, s>>>(descs, tiles, n_tiles, reverse, *prm); break;
-    case PYLO_FAM_VELO: k_apply<PYLO_FAM_VELO><<<grid_for(n_tiles, 4), NT, 0, s>>>(descs, tiles, n_tiles, reverse, *prm); break;
+    case PYLO_FAM_ADAFAC: launch(k_apply<PYLO_FAM_ADAFAC>, grid_for(n_tiles, 2), NT, 0, s, descs, tiles, n_tiles, reverse, *prm); break;
+    case PYLO_FAM_CELO2: launch(k_apply<PYLO_FAM_CELO2>, grid_for(n_tiles, 4), NT, 0, s, descs, tiles, n_tiles, reverse, *prm); break;
+    case PYLO_FAM_VELO: launch(k_apply<PYLO_FAM_VELO>, grid_for(n_tiles, 4), NT, 0, s, descs, tiles, n_tiles, reverse, *prm); break;
     default: return -2;
   }
   return launch_status();
@@ -2045,12 +2130,12 @@ int pylo_b200_apply_adafac_cols(const pylo_tensor_desc* descs, const pylo_atile*
   if (n_ctiles == 0) return 0;
   static bool configured[PYLO_MAX_DEVICES] = {};
   if (int rc = allow_dynamic_smem(k_apply_adafac_cols, (int)sizeof(CcSmem), configured)) return rc;
-  k_apply_adafac_cols<<<grid_for(n_ctiles, CC_CTAS_PER_SM), NT, sizeof(CcSmem), (cudaStream_t)stream>>>(descs, ctiles, n_ctiles, *prm);
+  launch(k_apply_adafac_cols, grid_for(n_ctiles, CC_CTAS_PER_SM), NT, sizeof(CcSmem), (cudaStream_t)stream, descs, ctiles, n_ctiles, *prm);
   return launch_status();
 }
 
 int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* ttiles, int n_ttiles, int generic,
-                              const pylo_step_params* prm, int* status, void* stream) {
+                              const pylo_step_params* prm, int* status, int* host_status, void* stream) {
   CHECK_ARG(descs && ttiles && prm && n_ttiles >= 0 && prm->family == PYLO_FAM_ADAFAC);
   if (n_ttiles == 0) return 0;
   // more than half an SM's shared memory is requested: one CTA per SM, which then owns all of the SM's tensor memory
@@ -2058,7 +2143,7 @@ int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* t
   static bool configured[2][PYLO_MAX_DEVICES] = {};
   auto kernel = generic ? k_apply_adafac_tc<true> : k_apply_adafac_tc<false>;
   if (int rc = allow_dynamic_smem(kernel, smem, configured[generic ? 1 : 0])) return rc;
-  kernel<<<grid_for(n_ttiles, 1), TC_NT, smem, (cudaStream_t)stream>>>(descs, ttiles, n_ttiles, *prm, status);
+  launch(kernel, grid_for(n_ttiles, 1), TC_NT, smem, (cudaStream_t)stream, descs, ttiles, n_ttiles, *prm, status, host_status);
   return launch_status();
 }
 
@@ -2080,7 +2165,7 @@ int pylo_b200_gemm_tn_3xtf32(const pylo_gemm_desc* g, int* status, void* stream)
   constexpr int smem = (int)sizeof(NsSmem) + 1024;  // room to start the tiles on a 1024-byte boundary
   if (int rc = allow_dynamic_smem(k_gemm_tn_3xtf32, smem, configured)) return rc;
   const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-  k_gemm_tn_3xtf32<<<grid, NS_THREADS, smem, (cudaStream_t)stream>>>(a, status);
+  launch(k_gemm_tn_3xtf32, grid, NS_THREADS, smem, (cudaStream_t)stream, a, status);
   return launch_status();
 }
 
@@ -2091,7 +2176,7 @@ int pylo_b200_transpose(const float* src, float* dst, int rows, int cols, int ld
   else CHECK_ARG(src != dst && ld_dst >= rows);
   const dim3 grid((cols + 31) / 32, (rows + 31) / 32, batch);
   CHECK_ARG(grid.y <= 65535);
-  k_transpose32<<<grid, 256, 0, (cudaStream_t)stream>>>(src, dst, rows, cols, ld_src, ld_dst, stride_src, stride_dst, mirror ? 1 : 0);
+  launch(k_transpose32, grid, 256, 0, (cudaStream_t)stream, src, dst, rows, cols, ld_src, ld_dst, stride_src, stride_dst, mirror ? 1 : 0);
   return launch_status();
 }
 
@@ -2101,8 +2186,8 @@ int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctil
   if (n_ctiles == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_CELO2: k_apply_packed<PYLO_FAM_CELO2><<<grid_for(n_ctiles, 2), NT, 0, s>>>(descs, ctiles, n_ctiles, *prm); break;
-    case PYLO_FAM_VELO: k_apply_packed<PYLO_FAM_VELO><<<grid_for(n_ctiles, PK_CTAS_VELO), NT, 0, s>>>(descs, ctiles, n_ctiles, *prm); break;
+    case PYLO_FAM_CELO2: launch(k_apply_packed<PYLO_FAM_CELO2>, grid_for(n_ctiles, 2), NT, 0, s, descs, ctiles, n_ctiles, *prm); break;
+    case PYLO_FAM_VELO: launch(k_apply_packed<PYLO_FAM_VELO>, grid_for(n_ctiles, PK_CTAS_VELO), NT, 0, s, descs, ctiles, n_ctiles, *prm); break;
     default: return -2;
   }
   return launch_status();
@@ -2111,33 +2196,37 @@ int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctil
 int pylo_b200_celo2_post_sums(const pylo_post_item* items, const pylo_tile* tiles, int n_tiles, void* stream) {
   CHECK_ARG(items && tiles && n_tiles >= 0);
   if (n_tiles == 0) return 0;
-  k_post_sums<<<grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream>>>(items, tiles, n_tiles);
+  launch(k_post_sums, grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream, items, tiles, n_tiles);
   return launch_status();
 }
 
 int pylo_b200_celo2_post_apply(const pylo_post_item* items, const pylo_tile* tiles, int n_tiles, void* stream) {
   CHECK_ARG(items && tiles && n_tiles >= 0);
   if (n_tiles == 0) return 0;
-  k_post_apply<<<grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream>>>(items, tiles, n_tiles);
+  launch(k_post_apply, grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream, items, tiles, n_tiles);
   return launch_status();
 }
 
 int pylo_b200_adamw(const pylo_adam_item* items, const pylo_tile* tiles, int n_tiles, int independent, float beta1,
-                    float one_minus_beta1, float beta2, float one_minus_beta2, float eps,
+                    float one_minus_beta1, float beta2, float one_minus_beta2, float eps, float bc1, float bc2,
                     const pylo_step_params* prm, void* stream) {
   CHECK_ARG(items && tiles && prm && n_tiles >= 0);
   if (n_tiles == 0) return 0;
-  k_adamw<<<grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream>>>(items, tiles, n_tiles, independent, beta1, one_minus_beta1, beta2,
-                                                              one_minus_beta2, eps, *prm);
+  launch(independent ? k_adamw<true> : k_adamw<false>, grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream, items, tiles, n_tiles,
+         beta1, one_minus_beta1, beta2, one_minus_beta2, eps, bc1, bc2, *prm);
   return launch_status();
 }
 
 int pylo_b200_velo_tensor_features(const pylo_tensor_desc* descs, int n_local, const int32_t* layer_of,
                                    int n_total, const float* rank_onehot, const float* fraction9,
-                                   const float* loss9, float* x_in, void* stream) {
-  CHECK_ARG(descs && rank_onehot && fraction9 && loss9 && x_in && n_local > 0 && n_total >= n_local);
-  k_velo_tensor_features<<<(n_local + 127) / 128, 128, 0, (cudaStream_t)stream>>>(descs, n_local, layer_of, n_total,
-                                                                                 rank_onehot, fraction9, loss9, x_in);
+                                   const pylo_velo_loss* lossbuf, const float* loss9, float* x_in, void* stream) {
+  CHECK_ARG(descs && rank_onehot && fraction9 && x_in && n_local > 0 && n_total >= n_local);
+  CHECK_ARG(lossbuf ? lossbuf->means && lossbuf->iteration && lossbuf->running_min && lossbuf->decays : loss9 != nullptr);
+  VeloFraction f;
+  memcpy(&f, fraction9, sizeof(f));
+  const pylo_velo_loss none = {};
+  launch(k_velo_tensor_features, 1, n_local > 256 ? 512 : 256, 0, (cudaStream_t)stream, descs, n_local, layer_of, n_total,
+         rank_onehot, f, lossbuf ? *lossbuf : none, loss9, x_in);
   return launch_status();
 }
 
@@ -2146,7 +2235,7 @@ int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   const pylo_velo_rnn r = *rnn;
   const int64_t TH = (int64_t)r.T * r.H;
-  k_velo_xmix<<<(r.H + NWARP - 1) / NWARP, NT, 0, s>>>(r);
+  launch(k_velo_xmix, (r.H + NWARP - 1) / NWARP, NT, 0, s, r);
   int parts = 1;
   if (r.H % 128 == 0 && r.H <= 512) {
     parts = 2;
@@ -2156,22 +2245,67 @@ int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, void* stream) {
     static bool configured[4][PYLO_MAX_DEVICES] = {};
     auto kernel = r.H == 128 ? k_velo_gates_rows<1> : r.H == 256 ? k_velo_gates_rows<2> : r.H == 384 ? k_velo_gates_rows<3> : k_velo_gates_rows<4>;
     if (int rc = allow_dynamic_smem(kernel, smem, configured[r.H / 128 - 1])) return rc;
-    kernel<<<dim3(gx, gy), NT, smem, s>>>(r, per);
+    launch(kernel, dim3(gx, gy), NT, smem, s, r, per);
   } else {
-    k_velo_gates<<<dim3((4 * r.H + GT - 1) / GT, (r.T + GT - 1) / GT), NT, 0, s>>>(r);
+    launch(k_velo_gates, dim3((4 * r.H + GT - 1) / GT, (r.T + GT - 1) / GT), NT, 0, s, r);
   }
-  k_velo_cell<<<(unsigned)((TH + 255) / 256), 256, 0, s>>>(r, parts);
+  launch(k_velo_cell, (unsigned)((TH + 255) / 256), 256, 0, s, r, parts);
   const int64_t hw = (int64_t)r.T * (r.B + 1);
-  k_velo_heads<<<(unsigned)((hw + NWARP - 1) / NWARP), NT, 0, s>>>(r);
-  k_velo_mix<<<r.T, 160 * MIX_GROUPS, r.B * sizeof(float), s>>>(r);
+  launch(k_velo_heads, (unsigned)((hw + NWARP - 1) / NWARP), NT, 0, s, r);
+  launch(k_velo_mix, r.T, 160 * MIX_GROUPS, r.B * sizeof(float), s, r);
   return launch_status();
 }
 
 int pylo_b200_velo_loss_features(float* means, int32_t* iteration, float* running_min, const float* decays,
                                  const float* loss, float* loss9, void* stream) {
   CHECK_ARG(means && iteration && running_min && decays && loss && loss9);
-  k_velo_loss<<<1, 32, 0, (cudaStream_t)stream>>>(means, iteration, running_min, decays, loss, loss9);
+  const pylo_velo_loss b = {means, iteration, running_min, decays, loss, 0.f, 0};
+  launch(k_velo_loss, 1, 32, 0, (cudaStream_t)stream, b, loss9);
   return launch_status();
+}
+
+// ------------------------------------------------------------------------------------------------
+// A step's phases in one call, for hosts whose own call overhead counts (a ctypes call costs about as much as a launch).
+// ------------------------------------------------------------------------------------------------
+int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int phases, void* stream) {
+  CHECK_ARG(p && prm);
+  int rc = 0;
+  if (phases & PYLO_STEP_FRONT) {
+    if (p->n_atiles || p->n_gitems)
+      if ((rc = pylo_b200_rowcol_sums(p->tdesc, p->atiles, p->n_atiles, p->gitems, p->n_gitems, prm, stream))) return rc;
+    if ((rc = pylo_b200_factor_update(p->tdesc, p->n_tensors, prm, stream))) return rc;
+    if ((rc = pylo_b200_state_moments(p->desc, p->tiles, p->n_tiles, 1, prm, stream))) return rc;
+    if ((rc = pylo_b200_finalize_moments(p->desc, p->n_units, stream))) return rc;
+  }
+  if (phases & PYLO_STEP_BACK) {
+    pylo_step_params q = *prm;
+    q.no_tables = p->tensor_cores ? 2 : 0;   // the tensor-core kernel reads the per-row table only
+    if ((rc = pylo_b200_prep_apply(p->desc, p->pitems, p->n_pitems, &q, stream))) return rc;
+    if (p->tensor_cores) {
+      // small models: one launch; large ones: what is not FAST2D first, then the rest through the leaner variant
+      const int first = p->n_ctiles < PYLO_TC_ONE_LAUNCH ? p->n_ctiles : p->n_ctiles_gen;
+      if ((rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles, first, p->n_ctiles_gen > 0, &q, p->status, p->host_status, stream))) return rc;
+      if ((rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles + first, p->n_ctiles - first, 0, &q, p->status, p->host_status, stream))) return rc;
+    } else if (p->n_ctiles) {
+      rc = q.family == PYLO_FAM_ADAFAC ? pylo_b200_apply_adafac_cols(p->desc, p->ctiles, p->n_ctiles, &q, stream)
+                                       : pylo_b200_apply_packed(p->desc, p->ctiles, p->n_ctiles, &q, stream);
+      if (rc) return rc;
+    }
+    if (p->n_tiles_slow)
+      if ((rc = pylo_b200_apply(p->desc, p->tiles_slow, p->n_tiles_slow, 0, &q, stream))) return rc;
+  }
+  return 0;
+}
+
+int pylo_b200_advance_steps(double* const* steps, int n, double* first, int* equal) {
+  CHECK_ARG(steps && n >= 0 && first && equal);
+  *first = n ? *steps[0] : 0.0;
+  *equal = 1;
+  for (int i = 0; i < n; ++i) {
+    if (*steps[i] != *first) *equal = 0;
+    *steps[i] += 1.0;
+  }
+  return 0;
 }
 
 }  // extern "C"

@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(NS_THREADS, 1) k_gemm_tn_3xtf32(const pylo_gem
     sm.abort = 0;
   }
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  pdl_begin();
   if (warp == NS_EPI_WARPS) { tc_alloc(&sm.tmem_base, 512); tc_relinquish(); }
   tc_fence_before();
   __syncthreads();
@@ -311,6 +312,7 @@ __global__ void __launch_bounds__(NS_THREADS, 1) k_gemm_tn_3xtf32(const pylo_gem
 //           it (completes the symmetric products; the diagonal tiles are mirrored inside the tile).
 __global__ void __launch_bounds__(256) k_transpose32(const float* __restrict__ src, float* __restrict__ dst, int R, int C,
                                                      int lds, int ldd, long long ss, long long sd, int mode) {
+  pdl_begin();
   __shared__ float tile[32][33];
   const int b = blockIdx.z, ti = blockIdx.y, tj = blockIdx.x;
   if (mode == 1 && tj < ti) return;  // source tiles: on and above the diagonal

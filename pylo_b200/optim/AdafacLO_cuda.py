@@ -31,8 +31,8 @@ from torch.optim import Optimizer
 
 from .. import _lib as L
 from ..models.Meta_MLP import MetaMLP
-from ..plan import GradNorm, LoPlan, LoTensor, current_stream_ptr, one_minus
-from ._common import factored_dims_sorted, require_cuda_param
+from ..plan import GradNorm, LoPlan, LoTensor, current_stream_ptr, one_minus, with_gradients
+from ._common import StepCounters, factored_dims_sorted, require_cuda_param
 
 
 def _decay_to_param(x):
@@ -66,6 +66,7 @@ class _AdafacFamily(Optimizer):
         # fp32 values of 1 - beta, read back once (the reference evaluates them on the device every step)
         self._w_m, self._w_f = one_minus(self.beta_m), one_minus(self.beta_adafactor)
         self._w_v = one_minus(self.beta_rms)[0]
+        self._prm = None   # the launch constants, made once
 
     def _init_state(self, state, p):
         """AdafacLO_cuda.py:227-256 / ELO_cuda.py:160-176."""
@@ -120,42 +121,34 @@ class _AdafacFamily(Optimizer):
         for _, plan in self._plans.values():
             plan.clear_status()
 
-    def _run_group(self, gi, group, plist, prm, lr, wd, exp_mult, step_mult, clip_norm, stream):
-        sig = tuple(p.data_ptr() for p in plist)
+    def _run_group(self, gi, plist, grads, prm, stream, **hyper):
+        sig = [p.data_ptr() for p in plist]
         cached = self._plans.get(gi)
         if cached is None or cached[0] != sig:
             cached = (sig, self._build_plan(plist))
             self._plans[gi] = cached
+            cached[1].counters = StepCounters([self.state[p] for p in plist])
         plan: LoPlan = cached[1]
         plan._poll_status()  # refuse the step before any state (the step counters included) is advanced
-        steps = []
-        for p in plist:
-            st = self.state[p]["step"]
-            st += 1
-            steps.append(float(st) - 1.0)
-        plan.set_field("lr", lr)
-        plan.set_field("wd", wd)
-        plan.set_field("exp_mult", exp_mult)
-        plan.set_field("step_mult", step_mult)
-        plan.set_field("clip_norm", clip_norm)
-        plan.refresh([p.grad for p in plist], steps=steps)
+        plan.set_hyper(**hyper)
+        plan.refresh(grads, plan.counters)
         if self.before_group is not None:
             self.before_group(gi)
-        plan.run_front(prm, stream)
-        plan.run_back(prm, stream)
+        plan.run(prm, stream)
         if self.after_group is not None:
             self.after_group(gi)
 
-    def _params_struct(self, gnorm_ptr, wd_mode, nan_to_num):
-        prm = L.StepParams()
-        prm.family = L.FAM_ADAFAC
-        prm.nan_to_num, prm.wd_mode = int(nan_to_num), int(wd_mode)
-        for k in range(3):
-            prm.w_m[k], prm.w_f[k] = self._w_m[k], self._w_f[k]
-        prm.w_v = self._w_v
-        prm.eps_v, prm.eps_feat, prm.eps_norm = 1e-30, 1e-6, 1e-5
-        prm.clip_val = float("inf")
-        prm.gnorm_sq = gnorm_ptr
+    def _params_struct(self, gnorm_ptr, wd_mode, nan_to_num, eps_v=1e-30):
+        prm = self._prm
+        if prm is None:
+            prm = self._prm = L.StepParams()
+            prm.family = L.FAM_ADAFAC
+            for k in range(3):
+                prm.w_m[k], prm.w_f[k] = self._w_m[k], self._w_f[k]
+            prm.w_v = self._w_v
+            prm.eps_feat, prm.eps_norm = 1e-6, 1e-5
+            prm.clip_val = float("inf")
+        prm.nan_to_num, prm.wd_mode, prm.eps_v, prm.gnorm_sq = nan_to_num, wd_mode, eps_v, gnorm_ptr
         return prm
 
 
@@ -235,20 +228,17 @@ class AdafacLO_CUDA(_AdafacFamily):
             if group["max_grad_norm"] is not None:
                 for p in group["params"]:
                     torch.nn.utils.clip_grad_norm_(p, group["max_grad_norm"])  # per tensor, as AdafacLO_cuda.py:214-215
-            plist = [p for p in group["params"] if p.grad is not None]
+            plist, grads = with_gradients(group["params"])
             if not plist:
                 # a sharded step hangs collectives on this hook: every rank must reach it for every group, in order,
                 # also a rank that owns nothing of the group
                 if self.after_group is not None:
                     self.after_group(gi)
                 continue
-            if any(p.grad.is_sparse for p in plist):
-                raise RuntimeError("Sparse gradients not supported")
-            wd = float(group["weight_decay"])
-            prm = self._params_struct(None, wd_mode=1 if wd > 0 else 0, nan_to_num=False)
-            if group["eps"] is not None:
-                prm.eps_v = float(group["eps"])
-            self._run_group(gi, group, plist, prm, float(group["lr"]), wd, self.exp_mult, self.step_mult, 0.0, stream)
+            wd, eps = float(group["weight_decay"]), group["eps"]
+            prm = self._params_struct(None, 1 if wd > 0 else 0, 0, 1e-30 if eps is None else float(eps))
+            self._run_group(gi, plist, grads, prm, stream, lr=float(group["lr"]), wd=wd, exp_mult=self.exp_mult,
+                            step_mult=self.step_mult, clip_norm=0.0)
         return loss
 
 
@@ -291,26 +281,24 @@ class ELO_CUDA(_AdafacFamily):
         stream = current_stream_ptr()
         gnorm_ptr = None
         if any(g["clip_grad"] for g in self.param_groups):
-            all_p = [p for g in self.param_groups for p in g["params"] if p.grad is not None]
-            sig = tuple(p.numel() for p in all_p)
+            all_p, all_g = with_gradients([p for g in self.param_groups for p in g["params"]])
+            sig = [p.numel() for p in all_p]
             if self._gnorm is None or self._gnorm[0] != sig:
                 self._gnorm = (sig, GradNorm(sig, self.device))
-            total = self._gnorm[1].run([p.grad for p in all_p], stream)
+            total = self._gnorm[1].run(all_g, stream)
             if self.process_group is not None or (torch.distributed.is_initialized() and self._sharded):
                 torch.distributed.all_reduce(total, group=self.process_group)  # each rank holds its own tensors' share
             gnorm_ptr = total.data_ptr()
         for gi, group in enumerate(self.param_groups):
-            plist = [p for p in group["params"] if p.grad is not None]
+            plist, grads = with_gradients(group["params"])
             if not plist:
                 # a sharded step hangs collectives on this hook: every rank must reach it for every group, in order,
                 # also a rank that owns nothing of the group
                 if self.after_group is not None:
                     self.after_group(gi)
                 continue
-            if any(p.grad.is_sparse for p in plist):
-                raise RuntimeError("Sparse gradients not supported")
             wd = float(group["weight_decay"])
-            prm = self._params_struct(gnorm_ptr, wd_mode=2 if wd > 0 else 0, nan_to_num=True)
-            clip_norm = float(group["clip_norm"]) if group["clip_grad"] else 0.0
-            self._run_group(gi, group, plist, prm, float(group["lr"]), wd, float(group["exp_mult"]), 1.0, clip_norm, stream)
+            prm = self._params_struct(gnorm_ptr, 2 if wd > 0 else 0, 1)
+            self._run_group(gi, plist, grads, prm, stream, lr=float(group["lr"]), wd=wd, exp_mult=float(group["exp_mult"]),
+                            step_mult=1.0, clip_norm=float(group["clip_norm"]) if group["clip_grad"] else 0.0)
         return loss

@@ -28,7 +28,8 @@ from torch.optim import Optimizer
 
 from .. import _lib as L
 from ..models.CELO2_MLP import CELO2MLP
-from ..plan import GradNorm, LoPlan, LoTensor, current_stream_ptr, one_minus
+from ..plan import (GradNorm, LoPlan, LoTensor, current_stream_ptr, grad_pointers, one_minus, tile_elems,
+                    with_gradients)
 from ._common import (ItemPlan, factored_dims_argsort, newton_schulz, newton_schulz_eligible, newton_schulz_tc,
                       require_cuda_param)
 
@@ -87,6 +88,7 @@ class _Celo2Family(Optimizer):
         # fp32 values of 1 - beta, read back once (the reference evaluates them on the device every step)
         self._w_m, self._w_f = one_minus(self.beta_m), one_minus(self.beta_fac)
         self._w_v = float(1 - self.beta_rms[-1])
+        self._prm = None   # the launch constants, made once
         self._b1_shared, self._b2_shared = float(self.beta_m[0]), float(self.beta_rms[-1])
 
     # ------------------------------------------------------------------ state
@@ -133,7 +135,9 @@ class _Celo2Family(Optimizer):
                 if "mom" not in st:
                     self._init_lo_state(st, p)
             (adam if to_adam else lo).append(p)
-        plan = {"lo_params": lo, "adam_params": adam, "lo": None, "adam": None, "post": None}
+        in_lo = [not (group["use_adamw_for_1d"] and (p.dim() <= 1 or group["is_embedding"])) for p in plist]
+        plan = {"lo_params": lo, "adam_params": adam, "lo": None, "adam": None, "post": None, "in_lo": in_lo,
+                "post_key": None, "adam_key": None}
         if lo:
             # raw-step buffers of equally shaped tensors are slices of one stacked tensor, so that
             # Newton-Schulz runs once per shape as a batched product instead of once per tensor
@@ -164,28 +168,36 @@ class _Celo2Family(Optimizer):
                 for k in range(p.numel() // mat):
                     post_sizes.append(mat)
                     post_owner.append((ti, k * mat))
-            post = ItemPlan(L.POST_DTYPE, post_sizes, self.device)
+            post = ItemPlan(L.POST_DTYPE, post_sizes, self.device, tile_elems(sum(post_sizes), 1024, 4 * L.SM_COUNT))
             post.owner = post_owner
             post.owner_t = np.array([t for t, _ in post_owner], dtype=np.int64)
             post.owner_off = np.array([4 * o for _, o in post_owner], dtype=np.uint64)
             post.part = torch.zeros(max(post.n_tiles, 1), dtype=torch.float32, device=self.device)
-            for i, (t0, k) in enumerate(post.ranges):
-                post.items["part"][i] = post.part.data_ptr() + 4 * t0
+            post.items["part"] = post.part.data_ptr() + 4 * post.items["tile0"].astype(np.uint64)
             plan["post"] = post
+            base_p = np.array([p.data_ptr() for p in lo], dtype=np.uint64)
+            post.items["p"][:] = base_p[post.owner_t] + post.owner_off
         if adam:
-            plan["adam"] = ItemPlan(L.ADAM_DTYPE, [p.numel() for p in adam], self.device)
+            sizes = [p.numel() for p in adam]
+            plan["adam"] = ItemPlan(L.ADAM_DTYPE, sizes, self.device, tile_elems(sum(sizes), 1024, 4 * L.SM_COUNT))
+            it = plan["adam"].items
+            keys = ("mom", "rms") if self._shared_adam else ("exp_avg", "exp_avg_sq")
+            plan["adam_states"] = [self.state[p] for p in adam]
+            it["p"][:] = [p.data_ptr() for p in adam]
+            it["m"][:] = [st[keys[0]].data_ptr() for st in plan["adam_states"]]
+            it["v"][:] = [st[keys[1]].data_ptr() for st in plan["adam_states"]]
         return plan
 
     def _params_struct(self, group, gnorm_ptr):
-        prm = L.StepParams()
-        prm.family = L.FAM_CELO2
-        prm.nan_to_num, prm.wd_mode = 0, 0
-        for k in range(3):
-            prm.w_m[k], prm.w_f[k] = self._w_m[k], self._w_f[k]
-        prm.w_v = self._w_v
-        prm.eps_v, prm.eps_feat, prm.eps_norm = 0.0, 1e-8, 1e-9
-        prm.clip_val = float(group["grad_clip_val"])
-        prm.gnorm_sq = gnorm_ptr
+        prm = self._prm
+        if prm is None:
+            prm = self._prm = L.StepParams()
+            prm.family = L.FAM_CELO2
+            for k in range(3):
+                prm.w_m[k], prm.w_f[k] = self._w_m[k], self._w_f[k]
+            prm.w_v = self._w_v
+            prm.eps_feat, prm.eps_norm = 1e-8, 1e-9
+        prm.clip_val, prm.gnorm_sq = float(group["grad_clip_val"]), gnorm_ptr
         return prm
 
     def check_status(self):
@@ -199,11 +211,11 @@ class _Celo2Family(Optimizer):
         stream = current_stream_ptr()
         gnorm_ptr = None
         if any(g["clip_grad"] for g in self.param_groups):
-            all_p = [p for g in self.param_groups for p in g["params"] if p.grad is not None]
-            sig = tuple(p.numel() for p in all_p)
+            all_p, all_g = with_gradients([p for g in self.param_groups for p in g["params"]])
+            sig = [p.numel() for p in all_p]
             if self._gnorm is None or self._gnorm[0] != sig:
                 self._gnorm = (sig, GradNorm(sig, self.device))
-            total = self._gnorm[1].run([p.grad for p in all_p], stream)
+            total = self._gnorm[1].run(all_g, stream)
             if self.process_group is not None or (torch.distributed.is_initialized() and self._sharded):
                 torch.distributed.all_reduce(total, group=self.process_group)  # each rank holds its own tensors' share
             gnorm_ptr = total.data_ptr()
@@ -212,14 +224,14 @@ class _Celo2Family(Optimizer):
             if self._shared_adam:
                 # every group advances on every step, with or without gradients (ELO_CELO2_cuda.py:215-216)
                 group["step"] = group.get("step", 0) + 1
-            plist = [p for p in group["params"] if p.grad is not None]
+            plist, grads = with_gradients(group["params"])
             if not plist:
                 # a sharded step hangs collectives on this hook: every rank must reach it for every group, in order,
                 # also a rank that owns nothing of the group
                 if self.after_group is not None:
                     self.after_group(gi)
                 continue
-            sig = tuple((p.data_ptr(), bool(group["is_embedding"]), bool(group["use_adamw_for_1d"])) for p in plist)
+            sig = [p.data_ptr() for p in plist] + [bool(group["is_embedding"]), bool(group["use_adamw_for_1d"])]
             cached = self._plans.get(gi)
             if cached is None or cached[0] != sig:
                 cached = (sig, self._build_group_plan(gi, group, plist))
@@ -229,79 +241,78 @@ class _Celo2Family(Optimizer):
                 self.before_group(gi)
             prm = self._params_struct(group, gnorm_ptr)
             clip_norm = float(group["clip_norm"]) if group["clip_grad"] else 0.0
-            lr = float(group["lr"])
-
-            lo: Optional[LoPlan] = plan["lo"]
-            if lo is not None:
-                lo.set_field("lr", lr)
-                lo.set_field("wd", group["weight_decay"])
-                lo.set_field("clip_norm", clip_norm)
-                lo.set_field("exp_mult", group["exp_mult"])
-                lo.refresh([p.grad for p in plan["lo_params"]])
-                lo.run_front(prm, stream)
-                lo.run_back(prm, stream)
-                post = plan["post"]
-                keep = [t.out for t in lo.tensors]
-                if group["orthogonalize"]:
-                    for stacked, members in plan["stacks"]:
-                        on_tc = self.ns_precision == "3xtf32" and newton_schulz_eligible(*stacked.shape[-2:])
-                        # batches of at most ~64 M elements keep the iteration's temporaries small
-                        per = max(1, (64 << 20) // max(1, stacked[0].numel()))
-                        for c0 in range(0, len(members), per):
-                            part = stacked[c0:c0 + per]
-                            if on_tc:
-                                res = newton_schulz_tc(part, self.ns_coeffs, self.ns_iters, self.ns_eps, self._ns_status, stream)
-                                self.extra_launches += 3 * self.ns_iters
-                            else:
-                                res = newton_schulz(part, self.ns_coeffs, self.ns_iters, self.ns_eps)
-                            res = res.contiguous()
-                            for j, ti in enumerate(members[c0:c0 + per]):
-                                keep[ti] = res[j]
-                it = post.items
-                base_s = np.fromiter((k.data_ptr() for k in keep), dtype=np.uint64, count=len(keep))
-                base_p = np.fromiter((p.data_ptr() for p in plan["lo_params"]), dtype=np.uint64, count=len(keep))
-                it["step"][:] = base_s[post.owner_t] + post.owner_off
-                it["p"][:] = base_p[post.owner_t] + post.owner_off
-                it["lr"][:] = lr
-                it["wd"][:] = group["weight_decay"]
-                it["rmsmult"][:] = group["rmsmult"]
-                post.upload()
-                L.check(L.lib.pylo_b200_celo2_post_sums(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_sums")
-                L.check(L.lib.pylo_b200_celo2_post_apply(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_apply")
-                self._keep = keep
-
-            adam: Optional[ItemPlan] = plan["adam"]
-            if adam is not None:
-                it = adam.items
-                keepg = []
-                for i, p in enumerate(plan["adam_params"]):
-                    st = self.state[p]
-                    g = p.grad
-                    if not (g.dtype == torch.float32 and g.is_contiguous()):
-                        g = g.to(torch.float32).contiguous()
-                        keepg.append(g)
-                    it["g"][i], it["p"][i] = g.data_ptr(), p.data_ptr()
-                    if self._shared_adam:
-                        t = group["step"]
-                        b1, b2 = self._b1_shared, self._b2_shared
-                        it["m"][i], it["v"][i] = st["mom"].data_ptr(), st["rms"].data_ptr()
-                    else:
-                        st["adam_step"] += 1
-                        t = st["adam_step"]
-                        b1, b2 = self.adam_beta1, self.adam_beta2
-                        it["m"][i], it["v"][i] = st["exp_avg"].data_ptr(), st["exp_avg_sq"].data_ptr()
-                    it["bc1"][i], it["bc2"][i] = 1.0 - b1 ** t, 1.0 - b2 ** t
-                it["lr"][:] = group["adam_lr_mult"] * lr
-                it["wd"][:] = group["adam_weight_decay"]
-                it["clip_norm"][:] = clip_norm
-                adam.upload()
-                eps = 1e-8 if self._shared_adam else self.adam_eps
-                L.check(L.lib.pylo_b200_adamw(adam.table.ptr, adam.tiles.ptr, adam.n_tiles, int(not self._shared_adam),
-                                              b1, 1 - b1, b2, 1 - b2, eps, C.byref(prm), stream), "adamw")
-                self._keepg = keepg
+            lr, wd = float(group["lr"]), group["weight_decay"]
+            if plan["lo"] is not None:
+                self._lo_step(group, plan, [g for g, lo in zip(grads, plan["in_lo"]) if lo], prm, clip_norm, lr, wd, stream)
+            if plan["adam"] is not None:
+                self._adam_step(group, plan, [g for g, lo in zip(grads, plan["in_lo"]) if not lo], prm, clip_norm, lr, stream)
             if self.after_group is not None:
                 self.after_group(gi)
         return loss
+
+
+    def _lo_step(self, group, plan, grads, prm, clip_norm, lr, wd, stream):
+        lo: LoPlan = plan["lo"]
+        lo.set_hyper(lr=lr, wd=wd, clip_norm=clip_norm, exp_mult=group["exp_mult"])
+        lo.refresh(grads)
+        lo.run(prm, stream)
+        post: ItemPlan = plan["post"]
+        keep = [t.out for t in lo.tensors]
+        if group["orthogonalize"]:
+            for stacked, members in plan["stacks"]:
+                on_tc = self.ns_precision == "3xtf32" and newton_schulz_eligible(*stacked.shape[-2:])
+                # batches of at most ~64 M elements keep the iteration's temporaries small
+                per = max(1, (64 << 20) // max(1, stacked[0].numel()))
+                for c0 in range(0, len(members), per):
+                    part = stacked[c0:c0 + per]
+                    if on_tc:
+                        res = newton_schulz_tc(part, self.ns_coeffs, self.ns_iters, self.ns_eps, self._ns_status, stream)
+                        self.extra_launches += 3 * self.ns_iters
+                    else:
+                        res = newton_schulz(part, self.ns_coeffs, self.ns_iters, self.ns_eps)
+                    res = res.contiguous()
+                    for j, ti in enumerate(members[c0:c0 + per]):
+                        keep[ti] = res[j]
+        steps = [k.data_ptr() for k in keep]
+        key = (steps, lr, wd, group["rmsmult"])
+        if key != plan["post_key"]:
+            it = post.items
+            it["step"][:] = np.array(steps, dtype=np.uint64)[post.owner_t] + post.owner_off
+            it["lr"][:], it["wd"][:], it["rmsmult"][:] = lr, wd, group["rmsmult"]
+            post.upload()
+            plan["post_key"] = key
+        L.check(L.lib.pylo_b200_celo2_post_sums(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_sums")
+        L.check(L.lib.pylo_b200_celo2_post_apply(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_apply")
+        self._keep = keep
+
+    def _adam_step(self, group, plan, grads, prm, clip_norm, lr, stream):
+        adam: ItemPlan = plan["adam"]
+        it = adam.items
+        ptrs = grad_pointers(grads)
+        copies = []
+        if ptrs is None:   # a gradient that is not contiguous is copied, which gives it a new address on every step
+            grads = [g if g.is_contiguous() else g.contiguous() for g in grads]
+            copies, ptrs = grads, [g.data_ptr() for g in grads]
+        if self._shared_adam:
+            b1, b2, eps = self._b1_shared, self._b2_shared, 1e-8
+            ts = [group["step"]]
+        else:
+            b1, b2, eps = self.adam_beta1, self.adam_beta2, self.adam_eps
+            for st in plan["adam_states"]:
+                st["adam_step"] += 1
+            ts = [st["adam_step"] for st in plan["adam_states"]]
+        same = min(ts) == max(ts)   # one step count: the bias corrections go with the launch, not through the table
+        key = (ptrs, group["adam_lr_mult"] * lr, group["adam_weight_decay"], clip_norm)
+        if key != plan["adam_key"] or not same:
+            it["g"][:] = ptrs
+            it["lr"][:], it["wd"][:], it["clip_norm"][:] = key[1:]
+            it["bc1"][:], it["bc2"][:] = [1.0 - b1 ** t for t in ts], [1.0 - b2 ** t for t in ts]
+            adam.upload()
+            plan["adam_key"] = key
+        bc1, bc2 = (1.0 - b1 ** ts[0], 1.0 - b2 ** ts[0]) if same else (0.0, 0.0)
+        L.check(L.lib.pylo_b200_adamw(adam.table.ptr, adam.tiles.ptr, adam.n_tiles, int(not self._shared_adam),
+                                      b1, 1 - b1, b2, 1 - b2, eps, bc1, bc2, C.byref(prm), stream), "adamw")
+        self._keepg = copies
 
 
 class CELO2_CUDA(_Celo2Family):

@@ -139,16 +139,44 @@ def require_cuda_param(p: torch.Tensor, who: str):
         raise RuntimeError(f"{who}: parameters must be contiguous")
 
 
+class StepCounters:
+    """The ``step`` entries of some parameters' states, advanced together.
+
+    The usual ones, 0-d fp64 tensors on the CPU, are counted up through their addresses in one native call (one torch
+    operation per tensor was most of the host's time on a small model); anything else one by one."""
+
+    def __init__(self, states):
+        self.states = states
+        self.tensors = [None] * len(states)
+        self.first, self.equal = C_.c_double(), C_.c_int()
+
+    def advance(self):
+        """Add one to every counter; returns the old values: a float where they are all the same, else a list."""
+        if not all([st["step"] is t for st, t in zip(self.states, self.tensors)]):
+            self.tensors = [st["step"] for st in self.states]
+            plain = all(torch.is_tensor(t) and t.device.type == "cpu" and t.dtype == torch.float64 and t.dim() == 0 for t in self.tensors)
+            self.table = (C_.c_void_p * len(self.tensors))(*[t.data_ptr() for t in self.tensors]) if plain else None
+        if self.table is not None:
+            L.check(L.lib.pylo_b200_advance_steps(self.table, len(self.tensors), C_.byref(self.first), C_.byref(self.equal)), "advance_steps")
+            if self.equal.value:
+                return self.first.value
+            return [float(t) - 1.0 for t in self.tensors]
+        old = []
+        for st in self.states:
+            st["step"] += 1
+            old.append(float(st["step"]) - 1.0)
+        return old
+
+
 class ItemPlan:
     """Tile list + item table for the simple element-wise kernels (AdamW, CELO2 tail)."""
 
-    def __init__(self, dtype, sizes: Sequence[int], device):
+    def __init__(self, dtype, sizes: Sequence[int], device, elems: int = L.TILE_ELEMS):
         self.items = np.zeros(len(sizes), dtype=dtype)
         self.items["n"] = sizes
-        tiles, ranges = make_tiles(sizes)
+        tiles, ranges = make_tiles(sizes, elems)
         if "tile0" in dtype.names:
-            for i, (t0, k) in enumerate(ranges):
-                self.items["tile0"][i], self.items["n_tiles"][i] = t0, k
+            self.items["tile0"], self.items["n_tiles"] = [t0 for t0, _ in ranges], [k for _, k in ranges]
         self.ranges = ranges
         self.tiles = DeviceTable(tiles, device)
         self.n_tiles = len(tiles)

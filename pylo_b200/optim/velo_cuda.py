@@ -20,6 +20,7 @@ and the apply sweep, which reads each tensor's mixed weights and its
 from __future__ import annotations
 
 import ctypes as C
+import math
 
 import numpy as np
 import torch
@@ -41,10 +42,12 @@ def _param_to_decay(x):
     return 1 - torch.exp(x * 10.0)
 
 
-def fractional_tanh_embed(x: float) -> torch.Tensor:
-    """tanh((x - t) * 10) for the nine time fractions of velo_cuda.py:155-162."""
-    ts = torch.tensor([0.03, 0.1, 0.2, 0.4, 0.6, 0.8, 0.9, 1.0, 1.1], dtype=torch.float32)
-    return torch.tanh((x - ts) * 10)
+_FRACTIONS = np.array([0.03, 0.1, 0.2, 0.4, 0.6, 0.8, 0.9, 1.0, 1.1], dtype=np.float32)
+
+
+def fractional_tanh_embed(x: float):
+    """tanh((x - t) * 10) in fp32 for the nine time fractions of velo_cuda.py:155-162."""
+    return [math.tanh(v) for v in ((np.float32(x) - _FRACTIONS) * np.float32(10)).tolist()]
 
 
 def init_loss_buffer(num_steps, device):
@@ -123,6 +126,7 @@ class VeLO_CUDA(Optimizer):
         if (self._all_shapes is None) != (self._owned is None):
             raise ValueError("VeLO_CUDA: pass all_shapes and owned together")
         self._plan = None
+        self._prm = None   # the launch constants, made once
         g0 = self.param_groups[0]
         self._w_m, self._w_f = one_minus(g0["initial_momentum_decays"]), one_minus(g0["initial_adafactor_decays"])
         self._w_v = one_minus(g0["initial_rms_decays"])[0]
@@ -205,15 +209,10 @@ class VeLO_CUDA(Optimizer):
         buf = {
             "weights": torch.zeros(T, 160, **f32), "lr_mult": torch.zeros(T, **f32), "x_in": torch.zeros(T, 30, **f32),
             "pooled": torch.zeros(H, **f32), "xmix": torch.zeros(T, H, **f32), "gates": torch.zeros(2, T, 4 * H, **f32),
-            "controls": torch.zeros(T, B, **f32), "loss9": torch.zeros(9, **f32), "fraction9": torch.zeros(9, **f32),
+            "controls": torch.zeros(T, B, **f32),
             "rank": torch.stack([self.state[p]["rank_onehot"] for p in plist]).contiguous(),
             "loss": torch.zeros(1, **f32),
         }
-        # the nine time features are computed on the host (as the reference does) and cross through pinned staging
-        # buffers, two in turn, so that the copy never stalls the host
-        buf["frac_stage"] = [torch.zeros(9, dtype=torch.float32).pin_memory() for _ in range(2)]
-        buf["frac_event"] = [None, None]
-        buf["frac_turn"] = 0
         layers = [self.state[p]["layer_idx"] for p in plist]
         buf["layer_of"] = torch.tensor(layers, dtype=torch.int32, device=dev)
         tensors = []
@@ -243,70 +242,64 @@ class VeLO_CUDA(Optimizer):
         for k in ("x_in", "pooled", "xmix", "gates", "controls", "weights", "lr_mult"):
             setattr(r, k, buf[k].data_ptr())
         r.T, r.H, r.B = T, H, B
-        return {"plan": plan, "buf": buf, "rnn": r}
+        return {"plan": plan, "buf": buf, "rnn": r, "loss": L.VeloLoss(), "fraction": (C.c_float * 9)(), "hyper": None}
 
     # ------------------------------------------------------------------ step
     @torch.no_grad()
     def step(self, loss):
         stream = current_stream_ptr()
         dev = self.device
-        plist, lrs, wds, ems, sms = [], [], [], [], []
+        plist, counts, hyper = [], [], []
         fraction = None
         for group in self.param_groups:
             frac = group["step"] / self.num_steps
             if fraction is not None and frac != fraction:
                 raise RuntimeError("VeLO_CUDA: param groups must advance in lock step")
             fraction = frac
-            for p in group["params"]:
-                if p.requires_grad is False:
-                    continue
-                if p.grad is None:
-                    raise RuntimeError("VeLO_CUDA: every parameter needs a gradient on every step "
-                                       "(the per-tensor LSTM sees all tensors, velo_cuda.py:399-418)")
-                plist.append(p)
-                lrs.append(group["lr"]); wds.append(group["weight_decay"])
-                ems.append(group["exp_mult"]); sms.append(group["step_mult"])
-        sig = tuple(p.data_ptr() for p in plist)
+            mine = [p for p in group["params"] if p.requires_grad]
+            plist += mine
+            counts.append(len(mine))
+            hyper.append((group["lr"], group["weight_decay"], group["exp_mult"], group["step_mult"]))
+        grads = [p.grad for p in plist]
+        if any([g is None for g in grads]):
+            raise RuntimeError("VeLO_CUDA: every parameter needs a gradient on every step "
+                               "(the per-tensor LSTM sees all tensors, velo_cuda.py:399-418)")
+        sig = [p.data_ptr() for p in plist]
         if self._plan is None or self._plan[0] != sig:
             self._plan = (sig, self._build_plan(plist))
         ctx = self._plan[1]
         plan: LoPlan = ctx["plan"]
         buf, r = ctx["buf"], ctx["rnn"]
+        if ctx["hyper"] != (counts, hyper):
+            per = lambda k: [h[k] for h, n in zip(hyper, counts) for _ in range(n)]
+            plan.set_hyper(lr=per(0), wd=per(1), exp_mult=per(2), step_mult=per(3))
+            ctx["hyper"] = (counts, hyper)
+        plan.refresh(grads)
 
-        # loss features (velo_cuda.py:183-211)
+        # loss features (velo_cuda.py:183-211): the kernel reads the loss where it is, or takes a host number as an argument
+        lb, loss_arg = self.loss_buffer, ctx["loss"]
         if torch.is_tensor(loss):
-            buf["loss"].copy_(loss.detach().reshape(-1)[:1].to(torch.float32), non_blocking=True)
+            loss = loss.detach()
+            if not (loss.is_cuda and loss.dtype == torch.float32 and loss.device == dev):
+                buf["loss"].copy_(loss.reshape(-1)[:1].to(torch.float32), non_blocking=True)
+                loss = buf["loss"]
+            loss_arg.loss = loss.data_ptr()
         else:
-            buf["loss"].fill_(float(loss))
-        lb = self.loss_buffer
-        L.check(L.lib.pylo_b200_velo_loss_features(lb["means"].data_ptr(), lb["iteration"].data_ptr(),
-                                                   lb["running_min"].data_ptr(), lb["decays"].data_ptr(),
-                                                   buf["loss"].data_ptr(), buf["loss9"].data_ptr(), stream), "velo_loss_features")
-        turn = buf["frac_turn"]
-        buf["frac_turn"] = turn ^ 1
-        if buf["frac_event"][turn] is not None:
-            buf["frac_event"][turn].synchronize()  # the copy issued two steps ago has long finished
-        buf["frac_stage"][turn].copy_(fractional_tanh_embed(fraction))
-        buf["fraction9"].copy_(buf["frac_stage"][turn], non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record()
-        buf["frac_event"][turn] = ev
+            loss_arg.loss, loss_arg.value = None, float(loss)
+        loss_arg.means, loss_arg.iteration = lb["means"].data_ptr(), lb["iteration"].data_ptr()
+        loss_arg.running_min, loss_arg.decays = lb["running_min"].data_ptr(), lb["decays"].data_ptr()
+        ctx["fraction"][:] = fractional_tanh_embed(fraction)
 
-        prm = L.StepParams()
-        prm.family, prm.nan_to_num, prm.wd_mode = L.FAM_VELO, 0, 3
-        for k in range(3):
-            prm.w_m[k], prm.w_f[k] = self._w_m[k], self._w_f[k]
-        prm.w_v = self._w_v
-        prm.eps_v, prm.eps_feat, prm.eps_norm = 0.0, 1e-6, 1e-5
-        prm.clip_val = 1000.0
-        prm.gnorm_sq = None
-
-        plan.set_field("lr", lrs)
-        plan.set_field("wd", wds)
-        plan.set_field("exp_mult", ems)
-        plan.set_field("step_mult", sms)
-        plan.refresh([p.grad for p in plist])
-        plan.run_front(prm, stream)
+        prm = self._prm
+        if prm is None:
+            prm = self._prm = L.StepParams()
+            prm.family, prm.nan_to_num, prm.wd_mode = L.FAM_VELO, 0, 3
+            for k in range(3):
+                prm.w_m[k], prm.w_f[k] = self._w_m[k], self._w_f[k]
+            prm.w_v = self._w_v
+            prm.eps_v, prm.eps_feat, prm.eps_norm = 0.0, 1e-6, 1e-5
+            prm.clip_val = 1000.0
+        plan.run(prm, stream, L.STEP_FRONT)
 
         h, c = self.lstm_hidden_state
         r.h, r.c = h.data_ptr(), c.data_ptr()
@@ -314,13 +307,13 @@ class VeLO_CUDA(Optimizer):
         if sharded:
             buf["x_in"].zero_()
         L.check(L.lib.pylo_b200_velo_tensor_features(plan.desc.ptr, plan.n_tensors, buf["layer_of"].data_ptr(), int(r.T),
-                                                     buf["rank"].data_ptr(), buf["fraction9"].data_ptr(),
-                                                     buf["loss9"].data_ptr(), buf["x_in"].data_ptr(), stream),
+                                                     buf["rank"].data_ptr(), ctx["fraction"], C.byref(loss_arg), None,
+                                                     buf["x_in"].data_ptr(), stream),
                 "velo_tensor_features")
         if sharded and torch.distributed.is_initialized() and torch.distributed.get_world_size(self._pg) > 1:
             torch.distributed.all_reduce(buf["x_in"], group=self._pg)
         L.check(L.lib.pylo_b200_velo_rnn(C.byref(r), stream), "velo_rnn")
-        plan.run_back(prm, stream)
+        plan.run(prm, stream, L.STEP_BACK)
         for group in self.param_groups:
             group["step"] += 1
         return None

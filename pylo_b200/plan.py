@@ -8,7 +8,6 @@ sequence of one step.  Nothing here touches tensor values on the host.
 
 from __future__ import annotations
 
-import contextlib
 import ctypes as C
 import math
 from dataclasses import dataclass
@@ -369,9 +368,9 @@ class LoPlan:
             self.apply_kernel = "k_apply_packed<CELO2>" if family == L.FAM_CELO2 else "k_apply_packed<VELO>"
         #: device flag the tensor-core kernel raises when one of its bounded waits ran out
         self.status = torch.zeros(128, dtype=torch.int32, device=self.device) if self.tensor_cores else None
-        # a pinned copy of the flag follows every launch without blocking; the next launch looks at it once it landed
+        # its twin in pinned host memory, written by the kernel itself: the next step looks at it without asking the device
         self._status_host = torch.zeros(1, dtype=torch.int32).pin_memory() if self.tensor_cores else None
-        self._status_event = None
+        self._status_view = self._status_host.numpy() if self.tensor_cores else None
         # the other units' apply sweep: vectors are short and every element costs a whole network, so the tiles are as
         # small as one element per thread where that is what fills the GPU (five 4096-vectors: 104 us as one tile each)
         slow_sizes = [sizes[u] for u in slow_units]
@@ -379,6 +378,23 @@ class LoPlan:
         slow["tensor"] = np.asarray(slow_units, dtype=np.int32)[slow["tensor"]] if len(slow) else slow["tensor"]
         self.tiles_slow = DeviceTable(slow, self.device)
         self.n_tiles_slow = len(slow)
+        #: everything pylo_b200_step needs for a step over these tensors
+        self.step_plan = L.StepPlan(
+            tdesc=self.tdesc.ptr, desc=self.desc.ptr, atiles=self.atiles.ptr, gitems=self.gitems.ptr, pitems=self.pitems.ptr,
+            ctiles=self.ctiles.ptr, tiles=self.tiles.ptr, tiles_slow=self.tiles_slow.ptr,
+            status=self.status.data_ptr() if self.tensor_cores else None,
+            host_status=self._status_host.data_ptr() if self.tensor_cores else None,
+            n_tensors=T, n_units=U, n_atiles=self.n_atiles, n_gitems=self.n_gitems, n_pitems=self.n_pitems,
+            n_ctiles=self.n_ctiles, n_ctiles_gen=self.n_ctiles_gen, n_tiles=self.n_tiles, n_tiles_slow=self.n_tiles_slow,
+            tensor_cores=int(self.tensor_cores))
+        self._step_plan_ref = C.byref(self.step_plan)
+        self._hyper = None          # what set_hyper last wrote
+        self._grad_ptrs = None      # the gradient addresses the table holds
+        self._step_base = None      # the step count the table holds for every tensor, where it is one
+        self._dirty = True          # the host table is ahead of the device's
+        self.step_delta = 0.0
+        self._prof = None
+        self.launch_count = 0
 
     # ------------------------------------------------------------------ per-step refresh
     def set_field(self, name, values):
@@ -388,29 +404,57 @@ class LoPlan:
             vals = np.broadcast_to(np.asarray(values), (self.n_tensors,))
             self.desc.host[name][:] = [vals[i] for i, _ in self.unit_owner]
 
-    def refresh(self, grads: Sequence[torch.Tensor], steps=None):
-        """Point the descriptors at this step's gradients (and step counts) and upload the tables."""
-        self._keepalive = []
-        ptrs = np.zeros(self.n_tensors, dtype=np.uint64)
-        for i, g in enumerate(grads):
-            if not (g.is_cuda and g.dtype == torch.float32 and g.is_contiguous() and g.data_ptr() % 16 == 0):
-                g = g.to(torch.float32).contiguous().clone()
-                self._keepalive.append(g)
-            ptrs[i] = g.data_ptr()
-        self.tdesc.host["g"][:] = ptrs
+    def set_hyper(self, **fields):
+        """Per-tensor fields (scalar or one value per tensor) as :meth:`set_field`, skipped where they are what they were."""
+        if fields != self._hyper:
+            for name, values in fields.items():
+                self.set_field(name, values)
+            self._hyper, self._dirty = fields, True
+
+    def refresh(self, grads: Sequence[torch.Tensor], counters=None):
+        """Point the descriptors at this step's gradients (and step counts) and upload the tables where that changed them.
+
+        ``counters.advance()``, called once the gradients are accepted, gives the step count: one value for all tensors,
+        or one per tensor."""
+        ptrs = grad_pointers(grads)
+        if ptrs is None or ptrs != self._grad_ptrs:
+            self._grad_ptrs = ptrs
+            self._keepalive = []
+            at = np.zeros(self.n_tensors, dtype=np.uint64)
+            for i, g in enumerate(grads):
+                if not (g.is_cuda and g.dtype == torch.float32 and g.is_contiguous() and g.data_ptr() % 16 == 0):
+                    g = g.to(torch.float32).contiguous().clone()
+                    self._keepalive.append(g)
+                    self._grad_ptrs = None   # the copy is this step's: look again at the next
+                at[i] = g.data_ptr()
+            if not np.array_equal(self.tdesc.host["g"], at):
+                self.tdesc.host["g"][:] = at
+                if self.sliced:
+                    self.desc.host["g"][:] = [at[i] + np.uint64(4 * off) for i, off in self.unit_owner]
+                self._dirty = True
         self.step_delta = 0.0
-        if steps is not None:
+        if counters is not None:
+            steps = counters.advance()
             # when every tensor advanced by the same amount since the table was last written, leave the
             # table alone and hand the kernels the difference (no upload on the step path)
-            delta = np.asarray(steps, dtype=np.float64) - self.tdesc.host["step"].astype(np.float64)
-            if len(delta) and np.all(delta == delta[0]) and 0 <= delta[0] < 2**20 and self.tdesc._last is not None:
-                self.step_delta = float(delta[0])
+            one = isinstance(steps, float)
+            delta = None
+            if one and self._step_base is not None:
+                delta = steps - self._step_base
+            elif self.tdesc._last is not None:
+                diff = np.asarray(steps, dtype=np.float64) - self.tdesc.host["step"].astype(np.float64)
+                delta = float(diff[0]) if len(diff) and np.all(diff == diff[0]) else None
+            if delta is not None and 0 <= delta < 2**20:
+                self.step_delta = delta
             else:
                 self.set_field("step", steps)
-        self.tdesc.upload()
-        if self.sliced:
-            self.desc.host["g"][:] = [ptrs[i] + np.uint64(4 * off) for i, off in self.unit_owner]
-            self.desc.upload()
+                self._dirty = True
+            self._step_base = steps - self.step_delta if one else None
+        if self._dirty:
+            self.tdesc.upload()
+            if self.sliced:
+                self.desc.upload()
+            self._dirty = False
 
     # ------------------------------------------------------------------ launch sequence
     #: the kernel that dominates each timed phase, for reports
@@ -428,65 +472,71 @@ class LoPlan:
         return {k: [a.elapsed_time(b) for a, b in v] for k, v in (self._prof or {}).items()}
 
     def _call(self, name, fn, *args):
-        prof = getattr(self, "_prof", None)
+        prof = self._prof
         if prof is not None:
             a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             a.record()
         L.check(fn(*args), name)
-        self.launch_count = getattr(self, "launch_count", 0) + self.LAUNCHES.get(name, 1)
+        self.launch_count += self.LAUNCHES.get(name, 1)
         if prof is not None:
             b.record()
             prof.setdefault(name, []).append((a, b))
 
-    def run_front(self, prm: L.StepParams, stream: int, reverse_b: bool = True):
-        """Phases A, A2, B, B2."""
+    def run(self, prm: L.StepParams, stream: int, phases: int = L.STEP_FRONT | L.STEP_BACK):
+        """The phases of a step (all of them, or only those before or after the caller's own work in between)."""
         self._poll_status()  # before any state of this step is touched
-        prm.step_delta = getattr(self, "step_delta", 0.0)
+        prm.step_delta = self.step_delta
+        if self._prof is None:
+            L.check(L.lib.pylo_b200_step(self._step_plan_ref, C.byref(prm), phases, stream), "step")
+            if phases & L.STEP_FRONT:
+                self.launch_count += 3 + (self.n_atiles > 0) + (self.n_gitems > 0)
+            if phases & L.STEP_BACK:
+                two = self.tensor_cores and 0 < self.n_ctiles_gen < self.n_ctiles and self.n_ctiles >= L.TC_ONE_LAUNCH
+                self.launch_count += 1 + (self.n_ctiles > 0) + two + (self.n_tiles_slow > 0)
+            return
+        if phases & L.STEP_FRONT:
+            self._front(prm, stream)
+        if phases & L.STEP_BACK:
+            self._back(prm, stream)
+
+    def _front(self, prm, stream):
+        """Phases A, A2, B, B2, one call each (timed)."""
         pp = C.byref(prm)
         if self.n_atiles or self.n_gitems:
             self._call("rowcol_sums", L.lib.pylo_b200_rowcol_sums, self.tdesc.ptr, self.atiles.ptr, self.n_atiles,
                        self.gitems.ptr, self.n_gitems, pp, stream)
             self.launch_count += 1 if self.n_atiles and self.n_gitems else 0
         self._call("factor_update", L.lib.pylo_b200_factor_update, self.tdesc.ptr, self.n_tensors, pp, stream)
-        self._call("state_moments", L.lib.pylo_b200_state_moments, self.desc.ptr, self.tiles.ptr, self.n_tiles,
-                   int(reverse_b), pp, stream)
+        self._call("state_moments", L.lib.pylo_b200_state_moments, self.desc.ptr, self.tiles.ptr, self.n_tiles, 1, pp, stream)
         self._call("finalize_moments", L.lib.pylo_b200_finalize_moments, self.desc.ptr, self.n_units, stream)
 
     def _poll_status(self):
-        """Raise if the copy of the status word that followed an earlier tensor-core launch has landed non-zero."""
-        if self._status_event is not None and self._status_event.query() and int(self._status_host[0]) != 0:
+        """Raise if a tensor-core launch of an earlier step has written its status word."""
+        if self._status_view is not None and self._status_view[0] != 0:
             raise L.PyloLibError("apply_adafac_tc: a wait on the tensor core timed out in an earlier step; the kernel "
                                  "kept the old values of the parameters it could not finish, and launches write "
                                  "nothing until clear_status() is called")
 
-    def run_back(self, prm: L.StepParams, stream: int, reverse_c: bool = False):
-        """Phases P, C."""
+    def _back(self, prm, stream):
+        """Phases P, C, one call each (timed)."""
         # the tensor-core kernel needs the per-row table only (2); the CUDA-core kernels need both (0)
         prm.no_tables = 2 if self.tensor_cores else 0
         pp = C.byref(prm)
         self._call("prep_apply", L.lib.pylo_b200_prep_apply, self.desc.ptr, self.pitems.ptr, self.n_pitems, pp, stream)
         if self.n_ctiles and self.tensor_cores:
-            self._poll_status()
             # small models: one launch; large ones: what is not FAST2D first, then the rest through the leaner variant
-            first = self.n_ctiles if self.n_ctiles < 8 * L.TC_WORKERS else self.n_ctiles_gen
+            first = self.n_ctiles if self.n_ctiles < L.TC_ONE_LAUNCH else self.n_ctiles_gen
             for at, count in ((0, first), (first, self.n_ctiles - first)):
                 if count:
                     gen = at == 0 and self.n_ctiles_gen > 0
                     self._call(self.apply_kernel if count > self.n_ctiles_gen else "k_apply", L.lib.pylo_b200_apply_adafac_tc,
                                self.desc.ptr, self.ctiles.ptr + at * L.ATILE_DTYPE.itemsize, count, int(gen), pp,
-                               self.status.data_ptr(), stream)
-            # a pinned copy of the status word follows the launch on the launch's own stream, without blocking
-            ctx = (torch.cuda.stream(torch.cuda.ExternalStream(stream, device=self.device))
-                   if stream != current_stream_ptr() else contextlib.nullcontext())
-            with ctx:
-                self._status_host.copy_(self.status[:1], non_blocking=True)
-                self._status_event = torch.cuda.Event()
-                self._status_event.record()
+                               self.status.data_ptr(), self._status_host.data_ptr(), stream)
         elif self.n_ctiles:
             fn = L.lib.pylo_b200_apply_adafac_cols if self.family == L.FAM_ADAFAC else L.lib.pylo_b200_apply_packed
             self._call(self.apply_kernel, fn, self.desc.ptr, self.ctiles.ptr, self.n_ctiles, pp, stream)
         if self.n_tiles_slow:
-            self._call("k_apply", L.lib.pylo_b200_apply, self.desc.ptr, self.tiles_slow.ptr, self.n_tiles_slow, int(reverse_c), pp, stream)
+            self._call("k_apply", L.lib.pylo_b200_apply, self.desc.ptr, self.tiles_slow.ptr, self.n_tiles_slow, 0, pp, stream)
 
     def check_status(self):
         """Synchronise and raise if the tensor-core kernel reported a wait that ran out.
@@ -502,8 +552,8 @@ class LoPlan:
         """Acknowledge a reported timeout: the next launches store again."""
         if self.status is not None:
             self.status.zero_()
+            torch.cuda.synchronize(self.device)   # a launch in flight may still write the host's word
             self._status_host.zero_()
-            self._status_event = None
 
 
 class GradNorm:
@@ -512,6 +562,7 @@ class GradNorm:
     def __init__(self, sizes: Sequence[int], device):
         self.out = torch.zeros(1, dtype=torch.float32, device=device)
         self._keepalive = []
+        self._grad_ptrs = None
         self.n_tiles = 0
         if len(sizes) == 0:   # a rank that owns no tensor still takes part in the all-reduce of the sum: with zero
             return
@@ -524,23 +575,48 @@ class GradNorm:
         self.scratch = torch.zeros(max(self.n_tiles, 1), dtype=torch.float32, device=device)
 
     def run(self, grads: Sequence[torch.Tensor], stream: int):
-        self._keepalive = []
         if self.n_tiles == 0:
             self.out.zero_()
             return self.out
-        for i, g in enumerate(grads):
-            if not (g.dtype == torch.float32 and g.is_contiguous()):
-                g = g.to(torch.float32).contiguous()
-                self._keepalive.append(g)
-            self.items["g"][i] = g.data_ptr()
-        self.table.upload()
+        ptrs = grad_pointers(grads)
+        if ptrs is None or ptrs != self._grad_ptrs:
+            self._grad_ptrs = ptrs
+            self._keepalive = []
+            for i, g in enumerate(grads):
+                if not (g.dtype == torch.float32 and g.is_contiguous()):
+                    g = g.to(torch.float32).contiguous()
+                    self._keepalive.append(g)
+                    self._grad_ptrs = None
+                self.items["g"][i] = g.data_ptr()
+            self.table.upload()
         L.check(L.lib.pylo_b200_grad_sumsq(self.table.ptr, self.tiles.ptr, self.n_tiles, self.scratch.data_ptr(),
                                            self.out.data_ptr(), stream), "grad_sumsq")
         return self.out
 
 
+def with_gradients(params):
+    """(parameters that have a gradient, their gradients)."""
+    grads = [p.grad for p in params]
+    if any([g is None for g in grads]):
+        params = [p for p, g in zip(params, grads) if g is not None]
+        grads = [g for g in grads if g is not None]
+    return params, grads
+
+
+def grad_pointers(grads: Sequence[torch.Tensor]):
+    """The gradients' addresses, or None where one of them is not contiguous and has to be looked at."""
+    try:
+        ptrs = [g.data_ptr() for g in grads]
+    except RuntimeError:
+        if any(g.is_sparse for g in grads):
+            raise RuntimeError("Sparse gradients not supported") from None
+        raise
+    return ptrs if all([g.is_contiguous() for g in grads]) else None
+
+
 def current_stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device (what ``torch.cuda.current_stream().cuda_stream`` says, without the object)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def f32(x) -> float:
