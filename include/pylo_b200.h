@@ -146,6 +146,8 @@ typedef struct pylo_step_params {
   int32_t no_tables;      /* prep_apply: 0 = make the per-row (desc.h_a) and per-column (desc.h_b) first-layer tables,
                              1 = neither, 2 = the per-row table only (what the tensor-core apply kernel reads) */
   const float* gnorm_sq;  /* device scalar: sum of squares of all gradients, or NULL */
+  int32_t sum_tiles;      /* prep_apply: 1 = add the tile partials up itself (finalize_moments was not called) */
+  int32_t pad_;
 } pylo_step_params;
 
 int pylo_b200_abi_version(void);
@@ -316,6 +318,26 @@ int pylo_b200_gemm_tn_3xtf32(const pylo_gemm_desc* g, int* status, void* stream)
 int pylo_b200_transpose(const float* src, float* dst, int rows, int cols, int ld_src, int ld_dst, int64_t stride_src,
                         int64_t stride_dst, int batch, int mirror, void* stream);
 
+/* The whole Newton-Schulz chain of n stacks of equally shaped matrices (CELO2_naive.py:59-73), the products of up to eight
+ * stacks side by side in one launch:
+ *     x /= ||x||_F + eps;  iters times  { a = x x^T;  b = c1 a + c2 a a;  x = c0 x + b x }   (a tall x from the right side)
+ * x and out are [batch][rows][cols], contiguous, different; x is left as it is.  Operands are kept as two fp16 planes of one
+ * power-of-two scale (22 significant bits, as many as a TF32 high and low part), which is sound while every |x| of the chain
+ * stays below 10: the caller checks its coefficients.  Matrices of a few thousand elements run in plain fp32 instead.
+ * work: pylo_b200_newton_schulz_workspace(...) bytes of device memory (may be NULL where that is 0), 256-byte aligned.
+ * descs is a HOST array; all stacks run the same number of iterations.  status: device int, bit 2 is ORed in if a bounded wait ran out; may be NULL.  Returns -5 where the
+ * driver offers no tensor maps. */
+typedef struct pylo_ns_desc {
+  const float* x;
+  float* out;
+  void* work;
+  int64_t work_bytes;
+  int32_t rows, cols, batch, iters;
+  float c0, c1, c2, eps;
+} pylo_ns_desc;
+int64_t pylo_b200_newton_schulz_workspace(int rows, int cols, int batch, int iters);
+int pylo_b200_newton_schulz(const pylo_ns_desc* descs, int n, int* status, void* stream);
+
 /* CELO2 tail (CELO2_cuda.py:336-339): step * rsqrt(mean(step^2 over the last two axes) + 1e-9) * rmsmult,
  * then p -= lr * (step + wd * p).  Items are matrices (the last two axes of a tensor). */
 typedef struct pylo_post_item {
@@ -380,12 +402,13 @@ typedef struct pylo_velo_loss {
   float value;
   int32_t pad_;
 } pylo_velo_loss;
-/* fraction9 is a HOST array of 9.  lossbuf (HOST pointer): the same launch first advances the loss buffer and uses its
- * features; NULL: loss9 holds them (device, [9]). */
+/* velo_tensor_features also does finalize_moments for its tensors (leave that call out).  fraction9 is a HOST array of 9,
+ * lossbuf a HOST pointer: the launch uses the features the buffer has after this step's loss, and velo_rnn, which must
+ * follow with the same lossbuf, advances it (NULL there: it is left as it is). */
 int pylo_b200_velo_tensor_features(const pylo_tensor_desc* descs, int n_local, const int32_t* layer_of,
                                    int n_total, const float* rank_onehot, const float* fraction9,
-                                   const pylo_velo_loss* lossbuf, const float* loss9, float* x_in, void* stream);
-int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, void* stream);
+                                   const pylo_velo_loss* lossbuf, float* x_in, void* stream);
+int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, const pylo_velo_loss* lossbuf, void* stream);
 /* The loss buffer's update and features alone: writes loss9[9]. */
 int pylo_b200_velo_loss_features(float* means, int32_t* iteration, float* running_min, const float* decays,
                                  const float* loss, float* loss9, void* stream);
@@ -403,6 +426,9 @@ typedef struct pylo_step_plan {
   const pylo_tile *tiles, *tiles_slow;
   int *status, *host_status;
   int32_t n_tensors, n_units, n_atiles, n_gitems, n_pitems, n_ctiles, n_ctiles_gen, n_tiles, n_tiles_slow, tensor_cores;
+  int32_t sum_tiles; /* 1: leave finalize_moments out and let prep_apply add up the tile partials, for units of a few dozen
+                        tiles at most (VELO, of any size: velo_tensor_features does it) */
+  int32_t pad_;
 } pylo_step_plan;
 int pylo_b200_step(const pylo_step_plan* plan, const pylo_step_params* prm, int phases, void* stream);
 /* Host only: adds 1 to n step counters (HOST pointers to doubles); first: the old value of the first, equal: whether all

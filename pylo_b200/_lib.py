@@ -56,7 +56,7 @@ class StepParams(C.Structure):
         ("family", C.c_int32), ("nan_to_num", C.c_int32), ("wd_mode", C.c_int32), ("step_delta", C.c_float),
         ("w_m", C.c_float * 3), ("w_v", C.c_float), ("w_f", C.c_float * 3),
         ("eps_v", C.c_float), ("eps_feat", C.c_float), ("eps_norm", C.c_float), ("clip_val", C.c_float),
-        ("no_tables", C.c_int32), ("gnorm_sq", C.c_void_p),
+        ("no_tables", C.c_int32), ("gnorm_sq", C.c_void_p), ("sum_tiles", C.c_int32), ("pad_", C.c_int32),
     ]
 
 
@@ -73,6 +73,12 @@ class GemmDesc(C.Structure):
                 ("strideA", C.c_int64), ("strideB", C.c_int64), ("strideC", C.c_int64), ("strideD", C.c_int64)] + [
         (name, C.c_int32) for name in ("M", "N", "K", "lda", "ldb", "ldc", "ldd", "batch")] + [
         ("alpha", C.c_float), ("beta", C.c_float), ("symmetric", C.c_int32), ("pad_", C.c_int32)]
+
+
+class NsDesc(C.Structure):
+    """pylo_ns_desc: a batch of matrices and the coefficients of their Newton-Schulz chain."""
+    _fields_ = [("x", C.c_void_p), ("out", C.c_void_p), ("work", C.c_void_p), ("work_bytes", C.c_int64)] + [
+        (name, C.c_int32) for name in ("rows", "cols", "batch", "iters")] + [(name, C.c_float) for name in ("c0", "c1", "c2", "eps")]
 
 
 class VeloRnn(C.Structure):
@@ -93,7 +99,7 @@ class StepPlan(C.Structure):
     _fields_ = [(name, C.c_void_p) for name in (
         "tdesc", "desc", "atiles", "gitems", "pitems", "ctiles", "tiles", "tiles_slow", "status", "host_status")] + [
         (name, C.c_int32) for name in ("n_tensors", "n_units", "n_atiles", "n_gitems", "n_pitems", "n_ctiles", "n_ctiles_gen",
-                                       "n_tiles", "n_tiles_slow", "tensor_cores")]
+                                       "n_tiles", "n_tiles_slow", "tensor_cores", "sum_tiles", "pad_")]
 
 
 class PyloLibError(RuntimeError):
@@ -130,11 +136,13 @@ def _load():
         "pylo_b200_apply_packed": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_gemm_tn_3xtf32": [C.POINTER(GemmDesc), vp, vp],
         "pylo_b200_transpose": [vp, vp, i32, i32, i32, i32, C.c_int64, C.c_int64, i32, i32, vp],
+        "pylo_b200_newton_schulz_workspace": [i32, i32, i32, i32],
+        "pylo_b200_newton_schulz": [C.POINTER(NsDesc), i32, vp, vp],
         "pylo_b200_celo2_post_sums": [vp, vp, i32, vp],
         "pylo_b200_celo2_post_apply": [vp, vp, i32, vp],
         "pylo_b200_adamw": [vp, vp, i32, i32] + [f32] * 7 + [C.POINTER(StepParams), vp],
-        "pylo_b200_velo_tensor_features": [vp, i32, vp, i32, vp, vp, C.POINTER(VeloLoss), vp, vp, vp],
-        "pylo_b200_velo_rnn": [C.POINTER(VeloRnn), vp],
+        "pylo_b200_velo_tensor_features": [vp, i32, vp, i32, vp, vp, C.POINTER(VeloLoss), vp, vp],
+        "pylo_b200_velo_rnn": [C.POINTER(VeloRnn), C.POINTER(VeloLoss), vp],
         "pylo_b200_velo_loss_features": [vp, vp, vp, vp, vp, vp, vp],
         "pylo_b200_step": [C.POINTER(StepPlan), C.POINTER(StepParams), i32, vp],
         "pylo_b200_advance_steps": [vp, i32, C.POINTER(C.c_double), C.POINTER(C.c_int)],
@@ -142,7 +150,7 @@ def _load():
     for name, argtypes in sigs.items():
         fn = getattr(lib, name)  # AttributeError if a declared symbol is missing
         fn.argtypes = argtypes
-        fn.restype = C.c_int64 if name == "pylo_b200_workspace_bytes" else C.c_int
+        fn.restype = C.c_int64 if name in ("pylo_b200_workspace_bytes", "pylo_b200_newton_schulz_workspace") else C.c_int
     if lib.pylo_b200_abi_version() != ABI_VERSION:
         raise ImportError("libpylo_b200.so was built from a different ABI version; rebuild it")
     if lib.pylo_b200_sizeof_desc() != DESC_DTYPE.itemsize or lib.pylo_b200_sizeof_params() != C.sizeof(StepParams):

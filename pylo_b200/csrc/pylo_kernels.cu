@@ -169,12 +169,12 @@ __global__ void __launch_bounds__(NT, 4) k_rowcol_fast(const pylo_tensor_desc* _
 //      block and reads it front to back; with I > 1 a lane stays on one i because the group's stride is a multiple of I.
 // Both read whole lines.  (One warp per output with lanes along the reduced axis, as it was, read one element per line
 // wherever that axis is not the last: 211 us for 5 M parameters of 3x3 convolutions, 302 us for a ViT patch embedding.)
-#define GA_LONG 4096      // from this block length on (I == 1) a CTA, not a warp, takes a block
+#define GA_LONG 1024      // from this block length on (I <= 32) a CTA, not a warp, takes a block: the loads of a block are a serial chain
 __global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* __restrict__ descs,
                                                        const pylo_atile* __restrict__ items,
                                                        const pylo_step_params prm) {
   pdl_begin();
-  __shared__ float s_red[40];
+  __shared__ float s_red[NT];
   const pylo_atile it = items[blockIdx.x];
   const pylo_tensor_desc& d = descs[it.tensor];
   const float gs = grad_scale_of(d, prm);
@@ -199,14 +199,26 @@ __global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* _
   const int64_t blocks = d.La / d.I, b0 = (int64_t)it.strip * it.cb, b1 = min(b0 + it.cb, blocks);
   const int I = d.I;
   const int lane = threadIdx.x & 31;
-  if (I == 1 && L >= GA_LONG) {
+  if (I <= 32 && L >= GA_LONG) {
+    const int S = NT / I * I;   // active threads: a thread stays on one i
     for (int64_t k = b0; k < b1; ++k) {
       const float* __restrict__ g = d.g + k * L;
       float acc = 0.f;
-#pragma unroll 4
-      for (int64_t e = threadIdx.x; e < L; e += NT) acc += square(__ldg(g + e));
-      acc = block_sum(acc, s_red);
-      if (threadIdx.x == 0) d.sum_a[k] = acc;
+      if (threadIdx.x < S)
+#pragma unroll 8
+        for (int64_t e = threadIdx.x; e < L; e += S) acc += square(__ldg(g + e));
+      if (I == 1) {
+        acc = block_sum(acc, s_red);
+        if (threadIdx.x == 0) d.sum_a[k] = acc;
+      } else {
+        __syncthreads();   // the previous block's sums have been read
+        s_red[threadIdx.x] = acc;
+        __syncthreads();
+        if (threadIdx.x < I) {
+          for (int q = threadIdx.x + I; q < S; q += I) acc += s_red[q];
+          d.sum_a[k * I + threadIdx.x] = acc;
+        }
+      }
     }
   } else if (I == 1) {
     const int w = L > 16 ? 32 : (L > 8 ? 16 : (L > 4 ? 8 : 4));   // lanes per block
@@ -214,7 +226,7 @@ __global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* _
       float acc = 0.f;
       if (k < b1) {
         const float* __restrict__ g = d.g + k * L;
-#pragma unroll 4
+#pragma unroll 8
         for (int64_t e = lane & (w - 1); e < L; e += w) acc += square(__ldg(g + e));
       }
       for (int o = w >> 1; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, w);
@@ -227,7 +239,7 @@ __global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* _
       const float* __restrict__ g = d.g + k * L;
       float acc = 0.f;
       if (lane < S)
-#pragma unroll 4
+#pragma unroll 8
         for (int64_t e = lane; e < L; e += S) acc += square(__ldg(g + e));
       float tot = acc;
       for (int q = I; q < S; q += I) tot += __shfl_sync(0xffffffffu, acc, (lane + q) & 31);   // read by lanes < I only
@@ -612,31 +624,41 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
 // ================================================================================================
 // Phase B2: per-tensor fixed-order reduction of the tile partials
 // ================================================================================================
-// Latency-bound: a 58 M-element tensor leaves 3584 rows of 40 partials.  The rows are read as one stretch of memory, 25
-// (or six) at a time, every thread keeping its column; eight rows ahead are in flight.
-__global__ void __launch_bounds__(1024) k_finalize_moments(const pylo_tensor_desc* __restrict__ descs) {
-  pdl_begin();
-  __shared__ double s_d[25][PYLO_STAT_STRIDE];
-  const pylo_tensor_desc& d = descs[blockIdx.x];
-  const int rows = blockDim.x / PYLO_STAT_STRIDE;
+// A unit's sums from its tiles' partials, in a fixed order; valid in threads j < PYLO_STAT_STRIDE, which hold sum j.
+// Latency-bound: a 58 M-element tensor leaves 3584 rows of 40 partials.  The rows are read as one stretch of memory, ROWS at
+// a time, every thread keeping its column; eight rows ahead are in flight.
+template <int ROWS>
+__device__ __forceinline__ double unit_sum(const pylo_tensor_desc& d, double (&s_d)[ROWS][PYLO_STAT_STRIDE]) {
   const int j = threadIdx.x % PYLO_STAT_STRIDE, sub = threadIdx.x / PYLO_STAT_STRIDE;
-  if (sub < rows) {
+  if (sub < ROWS) {
     double acc = 0.0;
     const float* __restrict__ src = d.tile_part + j;
     const int n = d.n_tiles;
 #pragma unroll 8
-    for (int t = sub; t < n; t += rows) acc += (double)src[(int64_t)t * PYLO_STAT_STRIDE];
+    for (int t = sub; t < n; t += ROWS) acc += (double)src[(int64_t)t * PYLO_STAT_STRIDE];
     s_d[sub][j] = acc;
   }
   __syncthreads();
+  double tot = 0.0;
   if (threadIdx.x < PYLO_STAT_STRIDE) {
-    double tot = 0.0;
-    for (int q = 0; q < rows; ++q) tot += s_d[q][j];
+    for (int q = 0; q < ROWS; ++q) tot += s_d[q][j];
     tot += (double)d.closed[j];
-    const float hi = (float)tot;
-    d.sums[j] = hi;
-    if (j >= 30 && j < 38) d.sums[SUMS_LO + (j - 30)] = (float)(tot - (double)hi);
   }
+  return tot;
+}
+__device__ __forceinline__ void store_unit_sum(const pylo_tensor_desc& d, double tot) {
+  const int j = threadIdx.x;
+  const float hi = (float)tot;
+  d.sums[j] = hi;
+  if (j >= 30 && j < 38) d.sums[SUMS_LO + (j - 30)] = (float)(tot - (double)hi);
+}
+template <int ROWS>
+__global__ void __launch_bounds__(ROWS * PYLO_STAT_STRIDE) k_finalize_moments(const pylo_tensor_desc* __restrict__ descs) {
+  pdl_begin();
+  __shared__ double s_d[ROWS][PYLO_STAT_STRIDE];
+  const pylo_tensor_desc& d = descs[blockIdx.x];
+  const double tot = unit_sum<ROWS>(d, s_d);
+  if (threadIdx.x < PYLO_STAT_STRIDE) store_unit_sum(d, tot);
 }
 
 // ================================================================================================
@@ -661,15 +683,25 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
   using L = Fold<FAM>;
   constexpr int H = F::H, NF = F::NF, NIN = F::NIN;
   __shared__ float s_scale[NF];
+  __shared__ double s_d[6][PYLO_STAT_STRIDE];
   __shared__ float s_w1[NF * H];
   __shared__ float s_b1[H];
+  __shared__ float s_p2;
   const pylo_atile it = items[blockIdx.x];
   const pylo_tensor_desc& d = descs[it.tensor];
   const int tid = threadIdx.x;
   const float* w = d.w;
   // source offsets in the family layout
   const int o_b1 = NIN * H, o_w2 = o_b1 + H, o_b2 = o_w2 + H * H, o_w3 = o_b2 + H, o_b3 = o_w3 + H * F::NOUT;
-  if (tid < NF) s_scale[tid] = rsqrtf(d.sums[tid] / (float)d.n + prm.eps_norm);
+  if (prm.sum_tiles) {   // small models: no finalize launch, every item adds its unit's few partials up itself
+    const double tot = unit_sum<6>(d, s_d);
+    if (tid < NF) s_scale[tid] = rsqrtf((float)tot / (float)d.n + prm.eps_norm);
+    if (tid == 2) s_p2 = (float)tot;
+    if (it.strip == 0 && tid < PYLO_STAT_STRIDE) store_unit_sum(d, tot);
+  } else {
+    if (tid < NF) s_scale[tid] = rsqrtf(d.sums[tid] / (float)d.n + prm.eps_norm);
+    if (tid == 2) s_p2 = d.sums[2];
+  }
   __syncthreads();
   for (int e = tid; e < NF * H; e += NT) {
     const int k = e / H, j = e % H;
@@ -705,7 +737,7 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
     }
     if (tid == 0) {
       // VeLO: param_scale = sqrt(mean(p^2) + 1e-9) from the p feature's sum (velo_kernel.cu:297)
-      o[L::SC + 0] = (FAM == PYLO_FAM_VELO) ? sqrtf(d.sums[2] / (float)d.n + 1e-9f) : 1.0f;
+      o[L::SC + 0] = (FAM == PYLO_FAM_VELO) ? sqrtf(s_p2 / (float)d.n + 1e-9f) : 1.0f;
       o[L::SC + 1] = d.lr_mult ? d.lr * d.lr_mult[0] : d.lr;
     }
   }
@@ -719,6 +751,7 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
   const int j = tid % H;
   if (it.strip < items_a) {
     const int end = min(La, (it.strip + 1) * PER);
+#pragma unroll 4
     for (int i = it.strip * PER + tid / H; i < end; i += NT / H) {
       float acc = s_b1[j];
 #pragma unroll
@@ -1216,6 +1249,7 @@ __global__ void __launch_bounds__(NT, CC_CTAS_PER_SM) k_apply_adafac_cols(const 
 
 #include "pylo_apply_tc.cuh"
 #include "pylo_ns_gemm.cuh"
+#include "pylo_ns_f16.cuh"
 
 // ================================================================================================
 // Phase C for CELO2 / ELO_CELO2 / VeLO on FAST2D tensors: packed kernel.
@@ -1227,7 +1261,9 @@ __global__ void __launch_bounds__(NT, CC_CTAS_PER_SM) k_apply_adafac_cols(const 
 //   * weights sit in shared memory as (w, w) pairs, one 128-bit read feeds four elements;
 //   * a thread keeps four columns for all rows of its tile, so the columns' tabulated first-layer
 //     terms and factors stay in registers; the rows' terms arrive as broadcast loads;
-//   * the next row's six float4 operands are requested before the current row is computed.
+//   * the next row's six float4 operands are requested before the current row is computed;
+//   * the rows' first-layer terms and factors are staged in shared memory, up to 256 rows at a time: read from global memory
+//     row by row, every row began with their latency.
 // ================================================================================================
 template <int FAM>
 struct PkW {  // duplicated-weight layout in shared memory (floats)
@@ -1266,7 +1302,8 @@ __device__ __forceinline__ uint64_t pk_feature(const PkBase& b) {
   else return mul2(b.k2, b.m2);
 }
 
-#define PK_ROWS 16  // rows per thread in a tile, unless the tag's upper half says fewer
+#define PK_ROWS 16  // rows per thread in a tile, unless the tag's upper half says otherwise
+#define PK_STAGE 256  // rows staged at once
 
 #ifndef PK_CTAS_VELO
 #define PK_CTAS_VELO 2
@@ -1280,7 +1317,9 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : 2) k
   using L = Fold<FAM>;
   using W = PkW<FAM>;
   constexpr int H = F::H;
+  constexpr int RP = 2 * H + 4;     // floats of a staged row: H pairs (v, v), then its three factors
   __shared__ __align__(16) float s_w[W::SIZE];
+  __shared__ __align__(16) float s_row[PK_STAGE * RP];
   __shared__ float s_sc[2];
   const int tid = threadIdx.x;
   int loaded = -1;
@@ -1341,13 +1380,24 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : 2) k
       g = ldg4(gp + idx); p = ld4(pp + idx); m0 = ld4(mp + idx); m1 = ld4(mp + n + idx); m2 = ld4(mp + 2 * n + idx); v = ld4(vp + idx);
     };
     load_row(0, cg, cp, cm0, cm1, cm2, cv);
+    const int sub = min(PK_ROWS, PK_STAGE / ng);   // rows per thread and stage
 #pragma unroll 1
     for (int q = 0; q < rpt; ++q) {
+      if (x0 + q * ng >= X) break;   // the same for the whole CTA
+      if (q % sub == 0) {
+        __syncthreads();   // the previous stage is no longer read
+        const int first = x0 + q * ng, rows = min(sub * ng, X - first);
+        for (int e = tid; e < rows * (RP / 4); e += NT) {
+          const int r = e / (RP / 4), k = e - r * (RP / 4);
+          st4(s_row + r * RP + 4 * k, k < H / 2 ? ld4(hap + (int64_t)(first + r) * 2 * H + 4 * k) : ld4(fxp + 4 * (int64_t)(first + r)));
+        }
+        __syncthreads();
+      }
       float4 ng_, np_, nm0, nm1, nm2, nv;
       if (q + 1 < rpt) load_row(q + 1, ng_, np_, nm0, nm1, nm2, nv);
       const int x = x0 + rg + ng * q;
-      const int xc = x < X ? x : 0;
-      const float4 fa = ld4(fxp + 4 * (int64_t)xc);
+      const float* const row = s_row + (x < X ? rg + ng * (q % sub) : 0) * RP;
+      const float4 fa = ld4(row + 2 * H);
       PkBase b[2];
       {
         float ge[4] = {cg.x, cg.y, cg.z, cg.w};
@@ -1365,7 +1415,7 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : 2) k
       uint64_t h1[2][H];
 #pragma unroll
       for (int j = 0; j < H; j += 2) {
-        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(hap + ((int64_t)xc * H + j) * 2);
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(row + 2 * j);
         h1[0][j] = add2(hb[0][j], a.x); h1[0][j + 1] = add2(hb[0][j + 1], a.y);
         h1[1][j] = add2(hb[1][j], a.x); h1[1][j + 1] = add2(hb[1][j + 1], a.y);
       }
@@ -1574,8 +1624,9 @@ __device__ __forceinline__ float clip_log_abs10(float v) {
   return fminf(fmaxf(logf(1e-8f + fabsf(v * 10.0f)), -5.f), 5.f) * 0.5f;
 }
 
-// BufferLossAccumulators.update followed by .features (velo_cuda.py:183-211); one warp, loss9 may be shared memory
-__device__ __forceinline__ void velo_loss_update(const pylo_velo_loss& b, float* loss9) {
+// BufferLossAccumulators.update followed by .features (velo_cuda.py:183-211); one warp.  loss9 (may be shared memory, may be
+// NULL) gets the features, the buffer is advanced where `write` says so.
+__device__ __forceinline__ void velo_loss_update(const pylo_velo_loss& b, float* loss9, bool write) {
   __shared__ float s_cor[10];
   const int j = threadIdx.x & 31;
   const int it = *b.iteration;
@@ -1593,73 +1644,77 @@ __device__ __forceinline__ void velo_loss_update(const pylo_velo_loss& b, float*
     const float mnew = b.means[j] * dj + loss * (1.0f - dj);
     const float c2 = mnew / (1.0f - powf(dj, (float)(it + 1)));  // features() uses iteration after the increment
     rmin = fminf(b.running_min[j], c2);
-    b.means[j] = mnew;
-    b.running_min[j] = rmin;
+    if (write) {
+      b.means[j] = mnew;
+      b.running_min[j] = rmin;
+    }
     s_cor[j] = c2;
   }
   __syncwarp();
-  if (j < 9) {
+  if (loss9 && j < 9) {
     const float den = fmaxf(1e-8f, s_cor[j + 1] - rmin);
     float f = fminf(fmaxf((s_cor[j] - rmin) / den - 1.0f, -1.f), 1.f);
     loss9[j] = (it + 1 <= 2) ? f * 0.f : f;
   }
   __syncwarp();
-  if (j == 0) *b.iteration = it + 1;
+  if (write && j == 0) *b.iteration = it + 1;
 }
 
 __global__ void k_velo_loss(const pylo_velo_loss b, float* __restrict__ loss9) {
   pdl_begin();
-  velo_loss_update(b, loss9);
+  velo_loss_update(b, loss9, true);
 }
 
-// One CTA: its first warp advances the loss buffer (where it is given), then one thread per tensor makes the 30 LSTM inputs
-// from the statistics gathered in phase B (velo_cuda.py:213-252).
+// The 30 LSTM inputs of a tensor from the statistics gathered in phase B (velo_cuda.py:213-252).  One CTA per tensor, which
+// first does phase B2 for it (a launch less), while its last warp works out the loss features: every CTA for itself and
+// without advancing the loss buffer, which is left to a kernel that runs when all of them are done (k_velo_xmix).
 struct VeloFraction { float f[9]; };
-__global__ void __launch_bounds__(512) k_velo_tensor_features(const pylo_tensor_desc* __restrict__ descs, int n_local,
+template <int ROWS>
+__global__ void __launch_bounds__(ROWS * PYLO_STAT_STRIDE + 32) k_velo_tensor_features(const pylo_tensor_desc* __restrict__ descs,
                                        const int32_t* __restrict__ layer_of, int T,
                                        const float* __restrict__ rank_onehot, const VeloFraction fraction9,
-                                       const pylo_velo_loss lossbuf, const float* __restrict__ loss9, float* __restrict__ x_in) {
+                                       const pylo_velo_loss lossbuf, float* __restrict__ x_in) {
   pdl_begin();
+  __shared__ double s_d[ROWS][PYLO_STAT_STRIDE];
+  __shared__ double s_sum[PYLO_STAT_STRIDE];
   __shared__ float s_loss9[9];
-  if (lossbuf.means) {
-    if (threadIdx.x < 32) velo_loss_update(lossbuf, s_loss9);
-  } else if (threadIdx.x < 9) {
-    s_loss9[threadIdx.x] = loss9[threadIdx.x];
+  const int t = blockIdx.x, tid = threadIdx.x;
+  const pylo_tensor_desc& d = descs[t];
+  if (tid >= ROWS * PYLO_STAT_STRIDE) velo_loss_update(lossbuf, s_loss9, false);
+  const double tot = unit_sum<ROWS>(d, s_d);
+  if (tid < PYLO_STAT_STRIDE) {
+    store_unit_sum(d, tot);
+    s_sum[tid] = tot;
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < n_local; t += blockDim.x) {
-    const int layer = layer_of ? layer_of[t] : t;  // position of this tensor among all T tensors of the model
-    const pylo_tensor_desc& d = descs[t];
-    const double n = (double)d.n;
-    const float* __restrict__ sums = d.sums;
-    float st[8], lo[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { st[j] = sums[30 + j]; lo[j] = sums[SUMS_LO + j]; }
-    auto stat = [&](int j) { return (double)st[j] + (double)lo[j]; };
-    const float mean_p2 = (float)((double)sums[2] / n);
-    const double norm = (double)rsqrtf(fmaxf(mean_p2, 1e-9f));
-    float* o = x_in + (int64_t)(T - 1 - layer) * 30;  // rows are flipped (velo_cuda.py:422)
-#pragma unroll
-    for (int j = 0; j < 9; ++j) { o[j] = fraction9.f[j]; o[9 + j] = s_loss9[j]; }
-    const double mean_v = stat(6) / n, e_v2 = stat(7) / n;
-    o[18] = clip_log_abs10((float)(norm * mean_v));
-#pragma unroll
-    for (int j = 0; j < 5; ++j) o[19 + j] = rank_onehot[t * 5 + j];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const double mu = stat(k) / n, e_m2 = stat(3 + k) / n;
-      const double var_m = fmax(e_m2 - mu * mu, 0.0);
-      const double var_v = fmax(e_v2 - 2.0 * mu * mean_v + mu * mu, 0.0);  // mean((rms - mean_m)^2), velo_cuda.py:243
-      o[24 + k] = clip_log_abs10((float)(norm * norm * var_m));
-      o[27 + k] = clip_log_abs10((float)(norm * norm * var_v));
-    }
+  if (tid >= 32) return;
+  const int layer = layer_of ? layer_of[t] : t;  // position of this tensor among all T tensors of the model
+  const double n = (double)d.n;
+  // as the stored sums have them: 32 bits, the VeLO statistics 32 + 32
+  auto stat = [&](int j) { const float hi = (float)s_sum[30 + j]; return (double)hi + (double)(float)(s_sum[30 + j] - (double)hi); };
+  const float mean_p2 = (float)((double)(float)s_sum[2] / n);
+  const double norm = (double)rsqrtf(fmaxf(mean_p2, 1e-9f));
+  const double mean_v = stat(6) / n, e_v2 = stat(7) / n;
+  float o = 0.f;
+  if (tid < 9) o = fraction9.f[tid];
+  else if (tid < 18) o = s_loss9[tid - 9];
+  else if (tid == 18) o = clip_log_abs10((float)(norm * mean_v));
+  else if (tid < 24) o = rank_onehot[t * 5 + tid - 19];
+  else if (tid < 30) {
+    const int k = (tid - 24) % 3;
+    const double mu = stat(k) / n, e_m2 = stat(3 + k) / n;
+    const double var = tid < 27 ? fmax(e_m2 - mu * mu, 0.0)
+                                : fmax(e_v2 - 2.0 * mu * mean_v + mu * mu, 0.0);  // mean((rms - mean_m)^2), velo_cuda.py:243
+    o = clip_log_abs10((float)(norm * norm * var));
   }
+  if (tid < 30) x_in[(int64_t)(T - 1 - layer) * 30 + tid] = o;  // rows are flipped (velo_cuda.py:422)
 }
 
 // x' = final_mix(x) + max_t relu(mix2(x)).  One warp per hidden unit, lanes along the tensors (one thread per unit walked
 // through all tensors by itself: 203 us at 292 tensors).
-__global__ void __launch_bounds__(NT) k_velo_xmix(const pylo_velo_rnn r) {
+__global__ void __launch_bounds__(NT) k_velo_xmix(const pylo_velo_rnn r, const pylo_velo_loss lossbuf) {
   pdl_begin();
+  if (lossbuf.means && blockIdx.x == 0 && threadIdx.x < 32) velo_loss_update(lossbuf, nullptr, true);
   const int h = blockIdx.x * NWARP + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (h >= r.H) return;
   float best = 0.f;   // relu
@@ -1891,7 +1946,15 @@ static int launch_status() { return (int)cudaGetLastError(); }
 
 // Every kernel of this library is launched so that it may become resident while its predecessor in the stream drains
 // (programmatic dependent launch) and waits in pdl_begin() until that one is complete.  A step is a chain of small launches;
-// on a small model the gaps between them are as long as the kernels.
+// on a small model the gaps between them are as long as the kernels (AdafacLO over a 118 K MLP: 47.5 -> 38.8 us per step).
+// On large ones there is nothing to gain (GPT-2-medium shapes: 0.7 % slower with it), so a step of more than 134 M elements
+// launches plainly: PlainLaunches says so for the calls of one scope on one host thread.
+static thread_local bool t_plain_launches = false;
+struct PlainLaunches {
+  bool before;
+  explicit PlainLaunches(int n_tiles) : before(t_plain_launches) { t_plain_launches = before || n_tiles > 8192; }
+  ~PlainLaunches() { t_plain_launches = before; }
+};
 template <class... P, class... A>
 static void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchAttribute attr;
@@ -1903,7 +1966,7 @@ static void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cud
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = t_plain_launches ? 0 : 1;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
@@ -1925,6 +1988,26 @@ static int allow_dynamic_smem(K kernel, int bytes, bool (&flags)[PYLO_MAX_DEVICE
   do {                  \
     if (!(cond)) return -1; \
   } while (0)
+
+template <int BN>
+static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
+  static bool configured[PYLO_MAX_DEVICES] = {};
+  constexpr int smem = (int)sizeof(NfSmem<BN>) + 1024;  // room to start the stages on a 1024-byte boundary
+  if (int rc = allow_dynamic_smem(k_gemm_f16x2<BN>, smem, configured)) return rc;
+  long long tiles = 0;
+  for (int k = 0; k < grp.n; ++k) {
+    nf_args& g = grp.p[k].g;
+    g.per = nf_tiles_per_matrix<BN>((g.M + NF_BM - 1) / NF_BM, (g.N + BN - 1) / BN, g.symmetric);
+    g.tile0 = (int)tiles;
+    tiles += (long long)g.per * g.batch;
+  }
+  if (tiles > 0x7fffffff) return -1;
+  // tiles of 128 x 256 where they fill the GPU; else half as wide ones: a small product is as long as its longest tile
+  if (BN == 256 && tiles < sm_count()) return ns_gemm<128>(grp, status, s);
+  grp.tiles = (int)tiles;
+  launch(k_gemm_f16x2<BN>, grp.tiles < sm_count() ? grp.tiles : sm_count(), NF_THREADS, smem, s, grp, status);
+  return launch_status();
+}
 
 extern "C" {
 
@@ -2092,7 +2175,8 @@ int pylo_b200_finalize_moments(const pylo_tensor_desc* descs, int n_tensors, voi
   CHECK_ARG(descs && n_tensors >= 0);
   if (n_tensors == 0) return 0;
   // many units (the slices of a CELO2 tensor) have few tiles each: small CTAs then
-  launch(k_finalize_moments, n_tensors, n_tensors > 512 ? 6 * PYLO_STAT_STRIDE : 25 * PYLO_STAT_STRIDE, 0, (cudaStream_t)stream, descs);
+  if (n_tensors > 512) launch(k_finalize_moments<6>, n_tensors, 6 * PYLO_STAT_STRIDE, 0, (cudaStream_t)stream, descs);
+  else launch(k_finalize_moments<25>, n_tensors, 25 * PYLO_STAT_STRIDE, 0, (cudaStream_t)stream, descs);
   return launch_status();
 }
 
@@ -2180,6 +2264,181 @@ int pylo_b200_transpose(const float* src, float* dst, int rows, int cols, int ld
   return launch_status();
 }
 
+// ------------------------------------------------------------------------------------------------
+// Newton-Schulz chain
+// ------------------------------------------------------------------------------------------------
+static long long ns_small_floats(int rows, int cols) {
+  const long long r = rows < cols ? rows : cols, c = rows < cols ? cols : rows;
+  return 2 * r * (c + 1) + 2 * r * (r + 1);
+}
+// One CTA does about 1e5 FMAs per microsecond: beyond a few million, or where it does not fit into shared memory, the
+// tensor-core chain (15 launches of 4 us at least) is faster.
+static bool ns_is_small(int rows, int cols, int iters) {
+  const long long r = rows < cols ? rows : cols, c = rows < cols ? cols : rows;
+  return r <= 64 && iters * (2 * r * r * c + r * r * r) <= 3000000 && ns_small_floats(rows, cols) * 4 <= 200 * 1024;
+}
+
+struct NsWork {   // byte offsets into the workspace, every buffer on a 1024-byte boundary
+  int64_t xp[2], ap, bp, a, x, part, inv, total;
+  int r, c, ldx, lda_p, lda, slices;
+};
+static NsWork ns_work(int rows, int cols, int batch) {
+  NsWork w = {};
+  w.r = rows < cols ? rows : cols;
+  w.c = rows < cols ? cols : rows;
+  w.ldx = (cols + 7) / 8 * 8;
+  w.lda_p = (w.r + 7) / 8 * 8;
+  w.lda = (w.r + 3) / 4 * 4;
+  const int64_t n = (int64_t)rows * cols;
+  w.slices = (int)((n + NF_SLICE - 1) / NF_SLICE);
+  int64_t at = 0;
+  auto take = [&](int64_t bytes) { const int64_t o = at; at += (bytes + 1023) / 1024 * 1024; return o; };
+  const int64_t planes_x = (int64_t)batch * rows * w.ldx * 4, planes_a = (int64_t)batch * w.r * w.lda_p * 4;
+  w.xp[0] = take(planes_x);
+  w.xp[1] = take(planes_x);
+  w.ap = take(planes_a);
+  w.bp = take(planes_a);
+  w.a = take((int64_t)batch * w.r * w.lda * 4);
+  w.x = take((int64_t)batch * n * 4);
+  w.part = take((int64_t)batch * w.slices * 4);
+  w.inv = take((int64_t)batch * 4);
+  w.total = at;
+  return w;
+}
+
+int64_t pylo_b200_newton_schulz_workspace(int rows, int cols, int batch, int iters) {
+  if (rows <= 0 || cols <= 0 || batch <= 0 || iters < 0) return -1;
+  return ns_is_small(rows, cols, iters) ? 0 : ns_work(rows, cols, batch).total;
+}
+
+typedef CUresult (*TensorMapEncode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                    const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static TensorMapEncode tensor_map_encode() {
+  static TensorMapEncode fn = [] {   // initialised once, also with several threads
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
+    return (TensorMapEncode)p;
+  }();
+  return fn;
+}
+// planes [2][batch][rows][ld] of fp16, boxes of 64 x 64; what a box reaches beyond a matrix reads as zero
+static int ns_map(CUtensorMap* map, void* base, int rows, int cols, int ld, int batch) {
+  TensorMapEncode fn = tensor_map_encode();
+  if (!fn) return -5;
+  const cuuint64_t dims[4] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch, 2};
+  const cuuint64_t strides[3] = {(cuuint64_t)ld * 2, (cuuint64_t)rows * ld * 2, (cuuint64_t)batch * rows * ld * 2};
+  const cuuint32_t box[4] = {64, 64, 1, 1}, unit[4] = {1, 1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, base, dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -5;
+}
+
+// the chain of up to NF_GROUP stacks of matrices, step by step side by side
+static int ns_chain(const pylo_ns_desc* const* ds, int n, int* status, cudaStream_t s) {
+  struct Stack { NsWork w; CUtensorMap x[2], a, b; char* base; };
+  Stack st[NF_GROUP];
+  // |x|, |a|, |b| stay below about 1.3, 1.5 and 3 for the usual coefficients and below 10, 15 and 15 for whatever this is
+  // called with (the caller checks): 2^12 keeps them inside fp16's range
+  constexpr float SX = 4096.f, SA = 4096.f, SB = 4096.f;
+  nf_prep_group prep = {};
+  prep.n = n;
+  long long ctas = 0;
+  for (int k = 0; k < n; ++k) {
+    const pylo_ns_desc& d = *ds[k];
+    Stack& t = st[k];
+    t.w = ns_work(d.rows, d.cols, d.batch);
+    t.base = (char*)d.work;
+    for (int q = 0; q < 2; ++q)
+      if (int rc = ns_map(&t.x[q], t.base + t.w.xp[q], d.rows, d.cols, t.w.ldx, d.batch)) return rc;
+    if (int rc = ns_map(&t.a, t.base + t.w.ap, t.w.r, t.w.r, t.w.lda_p, d.batch)) return rc;
+    if (int rc = ns_map(&t.b, t.base + t.w.bp, t.w.r, t.w.r, t.w.lda_p, d.batch)) return rc;
+    nf_prep& p = prep.p[k];
+    p.x = d.x; p.n = (long long)d.rows * d.cols;
+    p.part = (float*)(t.base + t.w.part); p.inv = (float*)(t.base + t.w.inv); p.P = (__half*)(t.base + t.w.xp[0]);
+    p.sP = (long long)d.rows * t.w.ldx; p.planeP = p.sP * d.batch;
+    p.cols = d.cols; p.ldp = t.w.ldx; p.slices = t.w.slices; p.cta0 = (int)ctas; p.eps = d.eps; p.scale = SX;
+    ctas += (long long)t.w.slices * d.batch;
+  }
+  if (ctas > 0x7fffffff) return -1;
+  launch(k_ns_sumsq, (int)ctas, NT, 0, s, prep);
+  launch(k_ns_split, (int)ctas, NT, 0, s, prep);
+  const int iters = ds[0]->iters;
+  nf_group grp;
+  grp.n = n;
+  for (int it = 0; it < iters; ++it) {
+    const int cur = it & 1;
+    const bool last = it == iters - 1;
+    for (int step = 0; step < 3; ++step) {
+      for (int k = 0; k < n; ++k) {
+        const pylo_ns_desc& d = *ds[k];
+        Stack& t = st[k];
+        const NsWork& w = t.w;
+        const bool wide = d.rows <= d.cols;
+        const long long size = (long long)d.rows * d.cols, sA = (long long)w.r * w.lda, sAp = (long long)w.r * w.lda_p;
+        nf_problem& q = grp.p[k];
+        nf_args g = {};
+        g.batch = d.batch;
+        if (step == 0) {          // a = x x^T (wide), x^T x (tall)
+          q.A = q.B = t.x[cur];
+          g.C = (float*)(t.base + w.a); g.sC = sA; g.ldc = w.lda;
+          g.P = (__half*)(t.base + w.ap); g.sP = sAp; g.ldp = w.lda_p; g.planeP = sAp * d.batch;
+          g.M = g.N = w.r; g.K = w.c;
+          g.alpha = 1.0f / (SX * SX); g.scale = SA; g.a_mn = g.b_mn = !wide; g.symmetric = 1;
+        } else if (step == 1) {   // b = c1 a + c2 a a
+          q.A = q.B = t.a;
+          g.D = (float*)(t.base + w.a); g.sD = sA; g.ldd = w.lda;
+          g.P = (__half*)(t.base + w.bp); g.sP = sAp; g.ldp = w.lda_p; g.planeP = sAp * d.batch;
+          g.M = g.N = g.K = w.r;
+          g.alpha = d.c2 / (SA * SA); g.beta = d.c1; g.scale = SB; g.symmetric = 1;
+        } else {                  // x' = c0 x + b x (wide), c0 x + x b (tall); the first round's x is d.x times inv
+          q.A = wide ? t.b : t.x[cur];
+          q.B = wide ? t.x[cur] : t.b;
+          float* const even = (float*)(t.base + w.x);
+          g.C = ((iters - it) & 1) ? d.out : even; g.sC = size; g.ldc = d.cols;   // the last round writes d.out
+          g.D = it == 0 ? d.x : ((iters - it) & 1) ? even : d.out; g.sD = size; g.ldd = d.cols;
+          g.d_scale = it == 0 ? (float*)(t.base + w.inv) : nullptr;
+          if (!last) { g.P = (__half*)(t.base + w.xp[cur ^ 1]); g.sP = (long long)d.rows * w.ldx; g.ldp = w.ldx; g.planeP = g.sP * d.batch; }
+          g.M = d.rows; g.N = d.cols; g.K = w.r;
+          g.alpha = 1.0f / (SB * SX); g.beta = d.c0; g.scale = SX; g.b_mn = wide;
+        }
+        q.g = g;
+      }
+      if (int rc = ns_gemm<256>(grp, status, s)) return rc;
+    }
+  }
+  return 0;
+}
+
+int pylo_b200_newton_schulz(const pylo_ns_desc* descs, int n, int* status, void* stream) {
+  CHECK_ARG(descs && n >= 0);
+  cudaStream_t s = (cudaStream_t)stream;
+  for (int k = 0; k < n; ++k) {
+    const pylo_ns_desc& d = descs[k];
+    CHECK_ARG(d.x && d.out && d.x != d.out && d.rows > 0 && d.cols > 0 && d.batch > 0 && d.iters >= 1 && d.iters == descs[0].iters);
+    CHECK_ARG(d.cols % 4 != 0 || (((uintptr_t)d.x | (uintptr_t)d.out) & 15) == 0);   // rows are moved in 16-byte pieces where they can
+    if (!ns_is_small(d.rows, d.cols, d.iters)) CHECK_ARG(d.work && ((uintptr_t)d.work & 255) == 0 && d.work_bytes >= ns_work(d.rows, d.cols, d.batch).total);
+  }
+  const pylo_ns_desc* group[NF_GROUP];
+  int m = 0;
+  for (int k = 0; k < n; ++k) {
+    const pylo_ns_desc& d = descs[k];
+    if (ns_is_small(d.rows, d.cols, d.iters)) {
+      static bool configured[PYLO_MAX_DEVICES] = {};
+      if (int rc = allow_dynamic_smem(k_ns_small, 200 * 1024, configured)) return rc;
+      launch(k_ns_small, d.batch, NT, (size_t)ns_small_floats(d.rows, d.cols) * 4, s, d.x, d.out, d.rows, d.cols, d.iters, d.c0, d.c1, d.c2, d.eps);
+      continue;
+    }
+    group[m++] = &d;
+    if (m == NF_GROUP) {
+      if (int rc = ns_chain(group, m, status, s)) return rc;
+      m = 0;
+    }
+  }
+  if (m)
+    if (int rc = ns_chain(group, m, status, s)) return rc;
+  return launch_status();
+}
+
 int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles,
                            const pylo_step_params* prm, void* stream) {
   CHECK_ARG(descs && ctiles && prm && n_ctiles >= 0);
@@ -2196,6 +2455,7 @@ int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctil
 int pylo_b200_celo2_post_sums(const pylo_post_item* items, const pylo_tile* tiles, int n_tiles, void* stream) {
   CHECK_ARG(items && tiles && n_tiles >= 0);
   if (n_tiles == 0) return 0;
+  const PlainLaunches plain(n_tiles);
   launch(k_post_sums, grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream, items, tiles, n_tiles);
   return launch_status();
 }
@@ -2203,6 +2463,7 @@ int pylo_b200_celo2_post_sums(const pylo_post_item* items, const pylo_tile* tile
 int pylo_b200_celo2_post_apply(const pylo_post_item* items, const pylo_tile* tiles, int n_tiles, void* stream) {
   CHECK_ARG(items && tiles && n_tiles >= 0);
   if (n_tiles == 0) return 0;
+  const PlainLaunches plain(n_tiles);
   launch(k_post_apply, grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream, items, tiles, n_tiles);
   return launch_status();
 }
@@ -2212,6 +2473,7 @@ int pylo_b200_adamw(const pylo_adam_item* items, const pylo_tile* tiles, int n_t
                     const pylo_step_params* prm, void* stream) {
   CHECK_ARG(items && tiles && prm && n_tiles >= 0);
   if (n_tiles == 0) return 0;
+  const PlainLaunches plain(n_tiles);
   launch(independent ? k_adamw<true> : k_adamw<false>, grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream, items, tiles, n_tiles,
          beta1, one_minus_beta1, beta2, one_minus_beta2, eps, bc1, bc2, *prm);
   return launch_status();
@@ -2219,23 +2481,23 @@ int pylo_b200_adamw(const pylo_adam_item* items, const pylo_tile* tiles, int n_t
 
 int pylo_b200_velo_tensor_features(const pylo_tensor_desc* descs, int n_local, const int32_t* layer_of,
                                    int n_total, const float* rank_onehot, const float* fraction9,
-                                   const pylo_velo_loss* lossbuf, const float* loss9, float* x_in, void* stream) {
+                                   const pylo_velo_loss* lossbuf, float* x_in, void* stream) {
   CHECK_ARG(descs && rank_onehot && fraction9 && x_in && n_local > 0 && n_total >= n_local);
-  CHECK_ARG(lossbuf ? lossbuf->means && lossbuf->iteration && lossbuf->running_min && lossbuf->decays : loss9 != nullptr);
+  CHECK_ARG(lossbuf && lossbuf->means && lossbuf->iteration && lossbuf->running_min && lossbuf->decays);
   VeloFraction f;
   memcpy(&f, fraction9, sizeof(f));
-  const pylo_velo_loss none = {};
-  launch(k_velo_tensor_features, 1, n_local > 256 ? 512 : 256, 0, (cudaStream_t)stream, descs, n_local, layer_of, n_total,
-         rank_onehot, f, lossbuf ? *lossbuf : none, loss9, x_in);
+  launch(k_velo_tensor_features<20>, n_local, 20 * PYLO_STAT_STRIDE + 32, 0, (cudaStream_t)stream, descs, layer_of, n_total,
+         rank_onehot, f, *lossbuf, x_in);
   return launch_status();
 }
 
-int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, void* stream) {
+int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, const pylo_velo_loss* lossbuf, void* stream) {
   CHECK_ARG(rnn && rnn->T > 0 && rnn->H > 0 && rnn->B > 0 && rnn->B <= 1024);
   cudaStream_t s = (cudaStream_t)stream;
   const pylo_velo_rnn r = *rnn;
   const int64_t TH = (int64_t)r.T * r.H;
-  launch(k_velo_xmix, (r.H + NWARP - 1) / NWARP, NT, 0, s, r);
+  const pylo_velo_loss none = {};
+  launch(k_velo_xmix, (r.H + NWARP - 1) / NWARP, NT, 0, s, r, lossbuf ? *lossbuf : none);
   int parts = 1;
   if (r.H % 128 == 0 && r.H <= 512) {
     parts = 2;
@@ -2269,16 +2531,18 @@ int pylo_b200_velo_loss_features(float* means, int32_t* iteration, float* runnin
 // ------------------------------------------------------------------------------------------------
 int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int phases, void* stream) {
   CHECK_ARG(p && prm);
+  const PlainLaunches plain(p->n_tiles);
   int rc = 0;
   if (phases & PYLO_STEP_FRONT) {
     if (p->n_atiles || p->n_gitems)
       if ((rc = pylo_b200_rowcol_sums(p->tdesc, p->atiles, p->n_atiles, p->gitems, p->n_gitems, prm, stream))) return rc;
     if ((rc = pylo_b200_factor_update(p->tdesc, p->n_tensors, prm, stream))) return rc;
     if ((rc = pylo_b200_state_moments(p->desc, p->tiles, p->n_tiles, 1, prm, stream))) return rc;
-    if ((rc = pylo_b200_finalize_moments(p->desc, p->n_units, stream))) return rc;
+    if (!p->sum_tiles && (rc = pylo_b200_finalize_moments(p->desc, p->n_units, stream))) return rc;
   }
   if (phases & PYLO_STEP_BACK) {
     pylo_step_params q = *prm;
+    q.sum_tiles = p->sum_tiles && q.family != PYLO_FAM_VELO;
     q.no_tables = p->tensor_cores ? 2 : 0;   // the tensor-core kernel reads the per-row table only
     if ((rc = pylo_b200_prep_apply(p->desc, p->pitems, p->n_pitems, &q, stream))) return rc;
     if (p->tensor_cores) {

@@ -11,8 +11,9 @@ What differs is where the work runs.  The reference does the accumulator
 updates with ~10 torch ops per tensor and then calls a two-kernel extension per
 tensor.  Here every tensor of a param group goes through one multi-tensor
 launch per phase: row/column sums of g^2, factor update, fused EMA + feature
-moments, normaliser folding, network + raw step; then Newton-Schulz (still
-``torch.matmul``), and one fused kernel pair for the final normalise-and-apply.
+moments, normaliser folding, network + raw step; then Newton-Schulz, one native
+call per stack of equally shaped matrices, and one fused kernel pair for the
+final normalise-and-apply.
 The global-norm clip factor is computed and consumed on the device, so the step
 has no host synchronisation.
 """
@@ -30,10 +31,11 @@ from .. import _lib as L
 from ..models.CELO2_MLP import CELO2MLP
 from ..plan import (GradNorm, LoPlan, LoTensor, current_stream_ptr, grad_pointers, one_minus, tile_elems,
                     with_gradients)
-from ._common import (ItemPlan, factored_dims_argsort, newton_schulz, newton_schulz_eligible, newton_schulz_tc,
-                      require_cuda_param)
+from ._common import (ItemPlan, factored_dims_argsort, newton_schulz, newton_schulz_bounded, newton_schulz_buffers,
+                      newton_schulz_native, newton_schulz_tc, require_cuda_param)
 
 _IN, _HID = 30, 8
+_KEPT_FLOATS = 4 << 20  # elements up to which a plan keeps Newton-Schulz results and workspaces between steps
 
 
 class _Celo2Family(Optimizer):
@@ -74,8 +76,9 @@ class _Celo2Family(Optimizer):
         self._w_flat = torch.cat([t.reshape(-1) for t in (self.w_in, self.b_in, self.w_h, self.b_h, self.w_out, self.b_out)]).contiguous()
         self._plans = {}
         self._gnorm = None
-        # "3xtf32" (default): the Newton-Schulz products on the tensor cores (this library's kernel, operands split
-        # into TF32 high and low parts, as accurate as fp32 products); "fp32": torch.matmul, the reference's arithmetic
+        # "3xtf32" (default): the Newton-Schulz products on the tensor cores (this library's kernels, operands split
+        # into a high and a low part of eleven bits each, as accurate as fp32 products); "fp32": torch.matmul, the
+        # reference's arithmetic
         self.ns_precision = "3xtf32"
         #: device word the Newton-Schulz kernel ORs 4 into if one of its bounded waits ran out
         self._ns_status = torch.zeros(1, dtype=torch.int32, device=dev)
@@ -144,13 +147,22 @@ class _Celo2Family(Optimizer):
             by_shape = {}
             for ti, p in enumerate(lo):
                 by_shape.setdefault(tuple(p.shape), []).append(ti)
-            stacks, out_of = [], {}
+            parts, out_of = [], {}
             for shape, members in by_shape.items():
                 stacked = torch.empty((len(members),) + shape, dtype=torch.float32, device=self.device)
-                stacks.append((stacked, members))
+                # parts of at most ~64 M elements keep Newton-Schulz's temporaries small
+                per = max(1, (64 << 20) // stacked[0].numel())
+                parts += [(stacked[c0:c0 + per], members[c0:c0 + per]) for c0 in range(0, len(members), per)]
                 for j, ti in enumerate(members):
                     out_of[ti] = stacked[j]
-            plan["stacks"] = stacks
+            # what goes into one native Newton-Schulz call: up to eight parts, up to ~96 M elements
+            groups = []
+            for part in parts:
+                if not groups or len(groups[-1]["parts"]) == 8 or groups[-1]["floats"] + part[0].numel() > (96 << 20):
+                    groups.append({"parts": [], "floats": 0, "kept": None})
+                groups[-1]["parts"].append(part)
+                groups[-1]["floats"] += part[0].numel()
+            plan["ns_groups"] = groups
             tensors = []
             for ti, p in enumerate(lo):
                 st = self.state[p]
@@ -259,21 +271,9 @@ class _Celo2Family(Optimizer):
         post: ItemPlan = plan["post"]
         keep = [t.out for t in lo.tensors]
         if group["orthogonalize"]:
-            for stacked, members in plan["stacks"]:
-                on_tc = self.ns_precision == "3xtf32" and newton_schulz_eligible(*stacked.shape[-2:])
-                # batches of at most ~64 M elements keep the iteration's temporaries small
-                per = max(1, (64 << 20) // max(1, stacked[0].numel()))
-                for c0 in range(0, len(members), per):
-                    part = stacked[c0:c0 + per]
-                    if on_tc:
-                        res = newton_schulz_tc(part, self.ns_coeffs, self.ns_iters, self.ns_eps, self._ns_status, stream)
-                        self.extra_launches += 3 * self.ns_iters
-                    else:
-                        res = newton_schulz(part, self.ns_coeffs, self.ns_iters, self.ns_eps)
-                    res = res.contiguous()
-                    for j, ti in enumerate(members[c0:c0 + per]):
-                        keep[ti] = res[j]
-        steps = [k.data_ptr() for k in keep]
+            keep, steps = self._orthogonalise(plan, stream)
+        else:
+            steps = [k.data_ptr() for k in keep]
         key = (steps, lr, wd, group["rmsmult"])
         if key != plan["post_key"]:
             it = post.items
@@ -284,6 +284,35 @@ class _Celo2Family(Optimizer):
         L.check(L.lib.pylo_b200_celo2_post_sums(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_sums")
         L.check(L.lib.pylo_b200_celo2_post_apply(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_apply")
         self._keep = keep
+
+    def _orthogonalise(self, plan, stream):
+        """Newton-Schulz over the plan's stacks of raw steps: (the results to keep alive, address of every tensor's)."""
+        keep, steps = [], [0] * len(plan["lo_params"])
+        native = self.ns_precision == "3xtf32" and newton_schulz_bounded(self.ns_coeffs, self.ns_iters)
+        for group in plan["ns_groups"]:
+            results = group["kept"]
+            if native:
+                if results is None:
+                    results = [newton_schulz_buffers(part, self.ns_iters) for part, _ in group["parts"]]
+                    if group["floats"] <= _KEPT_FLOATS:
+                        # small models: results and workspaces stay with the plan; large ones take them from the allocator
+                        # on every step, so that the training step can have the memory in between
+                        group["kept"] = results
+                newton_schulz_native([part for part, _ in group["parts"]], [r for r, _ in results], [w for _, w in results],
+                                     self.ns_coeffs, self.ns_iters, self.ns_eps, self._ns_status, stream)
+                outs = [r for r, _ in results]
+            else:
+                args = (self.ns_coeffs, self.ns_iters, self.ns_eps)
+                outs = [(newton_schulz_tc(part, *args, self._ns_status, stream) if self.ns_precision == "3xtf32"
+                         else newton_schulz(part, *args)).contiguous() for part, _ in group["parts"]]
+            if self.ns_precision == "3xtf32":
+                self.extra_launches += 3 * self.ns_iters
+            keep += outs
+            for res, (part, members) in zip(outs, group["parts"]):
+                at, n = res.data_ptr(), 4 * part[0].numel()
+                for j, ti in enumerate(members):
+                    steps[ti] = at + n * j
+        return keep, steps
 
     def _adam_step(self, group, plan, grads, prm, clip_norm, lr, stream):
         adam: ItemPlan = plan["adam"]

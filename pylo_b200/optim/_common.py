@@ -3,6 +3,7 @@
 from __future__ import annotations
 
 import ctypes as C_
+import functools
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -88,23 +89,73 @@ def _transpose(src, dst, stream):
 
 
 def newton_schulz_eligible(rows: int, cols: int) -> bool:
-    """Whether :func:`newton_schulz_tc` takes a matrix of this shape (else it goes to ``torch.matmul``): both sides
-    multiples of 4 (rows are moved in 16-byte pieces) and the short side at least 64 (the kernel's tiles have 128
-    rows; below half a tile the library product is the better tool)."""
+    """Whether the TF32 product kernel takes a matrix of this shape: both sides multiples of 4 (rows are moved in 16-byte
+    pieces) and the short side at least 64 (half a tile)."""
     r, c = min(rows, cols), max(rows, cols)
     return r % 4 == 0 and c % 4 == 0 and r >= 64
 
 
-def newton_schulz_tc(x: torch.Tensor, coeffs, iters: int = 5, eps: float = 1e-8, status=None, stream=None) -> torch.Tensor:
-    """:func:`newton_schulz` with the three products of every round on the tensor cores.
+@functools.lru_cache(maxsize=64)
+def newton_schulz_bounded(coeffs, iters: int) -> bool:
+    """Whether the iteration keeps every matrix small enough for planes of fp16 (|x| < 10, |a|, |b| < 15).
 
-    Same chain as CELO2_naive.py:59-73.  Each product is one launch of the library's own batched kernel
-    (``pylo_b200_gemm_tn_3xtf32``: operands split into TF32 high and low parts inside the kernel, three tcgen05
-    products accumulated in fp32, the scaled additions ``c1 a + c2 (a a)`` and ``c0 x + (b x)`` as its epilogue),
-    which needs both operands with the contraction index contiguous; x^T is therefore kept beside x and refreshed
-    once per round.  Not bit-identical to the fp32 products of ``torch.matmul`` (neither are two builds of cuBLAS);
-    against an fp64 evaluation it is as close as they are.
+    All of them are polynomials of the singular values, which start in [0, 1]; their largest values are followed through
+    the iterations on a fine grid.  The usual coefficients stay below 1.3."""
+    c0, c1, c2 = coeffs
+    top = 1.0
+    for _ in range(iters):
+        s = np.linspace(0.0, top, 4001)
+        if top * top > 14.0 or np.abs(c1 * s**2 + c2 * s**4).max() > 14.0:
+            return False
+        top = float(np.abs(c0 * s + c1 * s**3 + c2 * s**5).max()) * 1.01
+        if not top < 9.0:
+            return False
+    return iters >= 1
+
+
+def newton_schulz_native(stacks, outs, works, coeffs, iters, eps, status, stream):
+    """One native call for the chains of several stacks of matrices (contiguous, 16-byte aligned): ``outs`` the results,
+    ``works`` uint8 tensors of at least :func:`newton_schulz_workspace` bytes (None where that is 0)."""
+    descs = (L.NsDesc * len(stacks))()
+    for d, x, out, work in zip(descs, stacks, outs, works):
+        d.x, d.out = x.data_ptr(), out.data_ptr()
+        d.rows, d.cols, d.iters, d.eps = x.shape[-2], x.shape[-1], iters, eps
+        d.batch = x.numel() // (d.rows * d.cols)
+        d.c0, d.c1, d.c2 = coeffs
+        if work is not None:
+            d.work, d.work_bytes = work.data_ptr(), work.numel()
+    L.check(L.lib.pylo_b200_newton_schulz(descs, len(stacks), status.data_ptr() if status is not None else None, stream), "newton_schulz")
+
+
+def newton_schulz_buffers(x: torch.Tensor, iters: int):
+    """(result, workspace or None) for one stack of :func:`newton_schulz_native`."""
+    r, c = x.shape[-2:]
+    n = int(L.lib.pylo_b200_newton_schulz_workspace(r, c, x.numel() // (r * c), iters))
+    return torch.empty_like(x), torch.empty(n, dtype=torch.uint8, device=x.device) if n else None
+
+
+def newton_schulz_tc(x: torch.Tensor, coeffs, iters: int = 5, eps: float = 1e-8, status=None, stream=None) -> torch.Tensor:
+    """:func:`newton_schulz` on the tensor cores.
+
+    Same chain as CELO2_naive.py:59-73.  Where the coefficients keep the iterates bounded (the usual ones do), the whole
+    chain is one native call (``pylo_b200_newton_schulz``): every matrix is kept as two fp16 planes of one power-of-two
+    scale, 22 significant bits, and every product is three tcgen05 products of planes accumulated in fp32.  Else each
+    product is a launch of ``pylo_b200_gemm_tn_3xtf32`` on plain fp32 matrices, with x^T kept beside x, for the shapes it
+    takes.  Not bit-identical to the fp32 products of ``torch.matmul`` (neither are two builds of cuBLAS); against an fp64
+    evaluation both are as close as they are.
     """
+    coeffs = tuple(float(v) for v in coeffs)
+    if stream is None:
+        stream = torch.cuda.current_stream().cuda_stream
+    if newton_schulz_bounded(coeffs, iters):
+        x = x.contiguous()
+        if x.data_ptr() % 16:
+            x = x.clone()
+        out, work = newton_schulz_buffers(x, iters)
+        newton_schulz_native([x], [out], [work], coeffs, iters, eps, status, stream)
+        return out
+    if not newton_schulz_eligible(*x.shape[-2:]):
+        return newton_schulz(x, coeffs, iters, eps)
     shape = x.shape
     x = x.reshape((-1,) + tuple(shape[-2:]))
     tall = x.shape[-2] > x.shape[-1]
@@ -112,9 +163,7 @@ def newton_schulz_tc(x: torch.Tensor, coeffs, iters: int = 5, eps: float = 1e-8,
         x = x.transpose(-2, -1)
     x = (x / (torch.linalg.norm(x, dim=(-2, -1), keepdim=True) + eps)).contiguous()
     n_b, r, c = x.shape
-    if stream is None:
-        stream = torch.cuda.current_stream().cuda_stream
-    c0, c1, c2 = (float(v) for v in coeffs)
+    c0, c1, c2 = coeffs
     xt = torch.empty((n_b, c, r), dtype=torch.float32, device=x.device)
     a = torch.empty((n_b, r, r), dtype=torch.float32, device=x.device)
     b = torch.empty_like(a)

@@ -307,12 +307,12 @@ class VeLO_CUDA(Optimizer):
         if sharded:
             buf["x_in"].zero_()
         L.check(L.lib.pylo_b200_velo_tensor_features(plan.desc.ptr, plan.n_tensors, buf["layer_of"].data_ptr(), int(r.T),
-                                                     buf["rank"].data_ptr(), ctx["fraction"], C.byref(loss_arg), None,
+                                                     buf["rank"].data_ptr(), ctx["fraction"], C.byref(loss_arg),
                                                      buf["x_in"].data_ptr(), stream),
                 "velo_tensor_features")
         if sharded and torch.distributed.is_initialized() and torch.distributed.get_world_size(self._pg) > 1:
             torch.distributed.all_reduce(buf["x_in"], group=self._pg)
-        L.check(L.lib.pylo_b200_velo_rnn(C.byref(r), stream), "velo_rnn")
+        L.check(L.lib.pylo_b200_velo_rnn(C.byref(r), C.byref(loss_arg), stream), "velo_rnn")
         plan.run(prm, stream, L.STEP_BACK)
         for group in self.param_groups:
             group["step"] += 1

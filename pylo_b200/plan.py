@@ -243,7 +243,7 @@ class LoPlan:
                 else:
                     ws_items.append(("t", i, "part_b", ws.part_b))
                     gitems.append(atile_grid(i, ws.n_strips, (Lb + 255) // 256, 1))
-                    per = max(1, 16384 // (Y * I))  # blocks of Y*I elements per row-sum item: about 16 K elements
+                    per = max(1, 4096 // (Y * I))  # blocks of Y*I elements per row-sum item: about 4 K elements
                     rows = atile_grid(i, (La // I + per - 1) // per, 1)
                     rows[:, 2] = per
                     gitems.append(rows)
@@ -347,10 +347,11 @@ class LoPlan:
             shapes_c = [(u, X, Y, max(1, rt >> k), w, tag | max(1, rt >> k)) for u, X, Y, rt, w, tag in shapes_c]
             slow_units = []
         elif family != L.FAM_ADAFAC:
-            # fewer rows per thread (16, 8, 4 or 2) while the model does not give every SM its two CTAs
-            n_items = lambda k: sum(-(-X // (rt >> k)) * -(-Y // w) for _, X, Y, rt, w, _ in shapes_c)
-            k = next((k for k in range(3) if n_items(k) >= 4 * L.SM_COUNT), 3)
-            shapes_c = [(u, X, Y, rt >> k, w, tag | (16 >> k) << 16) for u, X, Y, rt, w, tag in shapes_c]
+            # rows per thread: 64 (a tile's start costs about a row's time), fewer while the model does not give every SM
+            # its two CTAs several tiles each; the shape's own height is 16 rows
+            n_items = lambda k: sum(-(-X // (rt * k // 16)) * -(-Y // w) for _, X, Y, rt, w, _ in shapes_c)
+            k = next((k for k in (64, 32, 16, 8, 4) if n_items(k) >= (16 if k > 16 else 4) * L.SM_COUNT), 2)
+            shapes_c = [(u, X, Y, rt * k // 16, w, tag | k << 16) for u, X, Y, rt, w, tag in shapes_c]
         for u, X, Y, rt, width, tag in shapes_c:
             ctiles.append(atile_grid(u, (X + rt - 1) // rt, (Y + width - 1) // width, tag))
         self.ctiles = DeviceTable(atile_list(ctiles), self.device)
@@ -378,6 +379,8 @@ class LoPlan:
         slow["tensor"] = np.asarray(slow_units, dtype=np.int32)[slow["tensor"]] if len(slow) else slow["tensor"]
         self.tiles_slow = DeviceTable(slow, self.device)
         self.n_tiles_slow = len(slow)
+        #: no launch for phase B2: of small units phase P adds the tile partials up, for VeLO the LSTM's input kernel does
+        self.sum_tiles = family == L.FAM_VELO or max((k for _, k in ranges), default=0) <= 48
         #: everything pylo_b200_step needs for a step over these tensors
         self.step_plan = L.StepPlan(
             tdesc=self.tdesc.ptr, desc=self.desc.ptr, atiles=self.atiles.ptr, gitems=self.gitems.ptr, pitems=self.pitems.ptr,
@@ -386,7 +389,7 @@ class LoPlan:
             host_status=self._status_host.data_ptr() if self.tensor_cores else None,
             n_tensors=T, n_units=U, n_atiles=self.n_atiles, n_gitems=self.n_gitems, n_pitems=self.n_pitems,
             n_ctiles=self.n_ctiles, n_ctiles_gen=self.n_ctiles_gen, n_tiles=self.n_tiles, n_tiles_slow=self.n_tiles_slow,
-            tensor_cores=int(self.tensor_cores))
+            tensor_cores=int(self.tensor_cores), sum_tiles=int(self.sum_tiles))
         self._step_plan_ref = C.byref(self.step_plan)
         self._hyper = None          # what set_hyper last wrote
         self._grad_ptrs = None      # the gradient addresses the table holds
@@ -489,7 +492,7 @@ class LoPlan:
         if self._prof is None:
             L.check(L.lib.pylo_b200_step(self._step_plan_ref, C.byref(prm), phases, stream), "step")
             if phases & L.STEP_FRONT:
-                self.launch_count += 3 + (self.n_atiles > 0) + (self.n_gitems > 0)
+                self.launch_count += 3 - self.sum_tiles + (self.n_atiles > 0) + (self.n_gitems > 0)
             if phases & L.STEP_BACK:
                 two = self.tensor_cores and 0 < self.n_ctiles_gen < self.n_ctiles and self.n_ctiles >= L.TC_ONE_LAUNCH
                 self.launch_count += 1 + (self.n_ctiles > 0) + two + (self.n_tiles_slow > 0)
@@ -508,7 +511,8 @@ class LoPlan:
             self.launch_count += 1 if self.n_atiles and self.n_gitems else 0
         self._call("factor_update", L.lib.pylo_b200_factor_update, self.tdesc.ptr, self.n_tensors, pp, stream)
         self._call("state_moments", L.lib.pylo_b200_state_moments, self.desc.ptr, self.tiles.ptr, self.n_tiles, 1, pp, stream)
-        self._call("finalize_moments", L.lib.pylo_b200_finalize_moments, self.desc.ptr, self.n_units, stream)
+        if self.family != L.FAM_VELO:
+            self._call("finalize_moments", L.lib.pylo_b200_finalize_moments, self.desc.ptr, self.n_units, stream)
 
     def _poll_status(self):
         """Raise if a tensor-core launch of an earlier step has written its status word."""
@@ -520,7 +524,7 @@ class LoPlan:
     def _back(self, prm, stream):
         """Phases P, C, one call each (timed)."""
         # the tensor-core kernel needs the per-row table only (2); the CUDA-core kernels need both (0)
-        prm.no_tables = 2 if self.tensor_cores else 0
+        prm.no_tables, prm.sum_tiles = 2 if self.tensor_cores else 0, 0
         pp = C.byref(prm)
         self._call("prep_apply", L.lib.pylo_b200_prep_apply, self.desc.ptr, self.pitems.ptr, self.n_pitems, pp, stream)
         if self.n_ctiles and self.tensor_cores:

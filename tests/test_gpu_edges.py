@@ -1,0 +1,166 @@
+"""GPU checks at the sizes where the work lists, the generic paths and the Newton-Schulz chain can go wrong: edges of tiles,
+remainders, the smallest and the largest of a range; against the CPU oracle or an fp64 evaluation."""
+
+import pytest
+import torch
+
+import cases
+import cuda_util as CU
+from test_gpu_properties import _make, _nets, _step
+
+pytestmark = pytest.mark.gpu
+
+COEFFS = (3.4445, -4.7750, 2.0315)
+
+# inner axes after the factored ones (1 < I <= 32, I > 32), before and between them, rows that are longer than a warp takes
+# (4096 on, unaligned), short blocks (Y*I = 4), strips of 8, 16 and 32 rows with remainders, a partial table item
+SHAPES = {
+    "inner": [(40, 24, 3, 3), (9, 50, 5), (64, 70, 40), (33, 35, 33)],
+    "outer": [(3, 40, 5, 24), (2, 3, 37, 41), (30, 3, 4, 4)],
+    "long": [(3, 4099), (5, 8193), (600, 7), (1100, 3)],
+    "rows": [(513, 64), (512, 68), (9, 1028), (65, 2052), (2049, 36)],
+}
+
+
+def _oracle(family, net, shapes):
+    from oracle import pylo_oracle as O
+
+    if family == "adafaclo":
+        return O.AdafacLOOracle(net.flat_weights(), lr=1e-2)
+    if family == "celo2":
+        return O.CELO2Oracle(net.flat_weights(), lr=1e-2, weight_decay=0.1, clip_grad=True, orthogonalize=False)
+    rnn, mlp = net
+    return O.VeLOOracle(O.rnn_weights_from_module(rnn), O.bank_from_module(mlp), shapes, lr=1.0, num_steps=100)
+
+
+@pytest.mark.parametrize("which", sorted(SHAPES))
+@pytest.mark.parametrize("family,extra", [("adafaclo", {}), ("adafaclo", {"mlp_precision": "fp32"}), ("celo2", {"orthogonalize": False}),
+                                          ("velo", {})])
+def test_shapes_at_the_edges_match_the_oracle(family, extra, which):
+    shapes = SHAPES[which] + [(13,)]
+    case = dict(shapes=shapes, init_seed=51, init_scale=0.1, grad_seed=52, grad_scale=0.3)
+    params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+    init = [v.clone() for v in cases.init_values(case)]
+    ref = [v.clone() for v in init]
+    opt, ora = _make(family, params, **extra), _oracle(family, _nets(family), shapes)
+    for t in (1, 2):
+        grads = cases.grads_at(case, t)
+        for p, g in zip(params, grads):
+            p.grad = g.cuda()
+        _step(opt, family, t)
+        ora.step(ref, grads, cases.velo_loss(t)) if family == "velo" else ora.step(ref, grads)
+    res = CU.compare({2: [p.detach().cpu() for p in params]}, {2: ref}, init)
+    assert res[2][0] < 1e-5 and res[2][1] < 2e-5, res
+
+
+# matrices of the shared-memory kernel, of the 128- and 256-wide tiles, with K tails and odd pitches, wide and tall
+STACKS = [[(1, 5)], [(64, 64), (3, 16, 16), (10, 128)], [(65, 67), (67, 65), (2, 129, 257)], [(128, 128), (7, 3001), (3001, 7), (100, 260)],
+          [(1024, 1030), (258, 1024), (2, 200, 392), (33, 1000), (1000, 33), (5, 5), (96, 96), (300, 300), (131, 70), (70, 131)]]
+
+
+@pytest.mark.parametrize("shapes", STACKS, ids=[str(len(s)) + "x" + str(s[0]) for s in STACKS])
+def test_newton_schulz_chains_side_by_side(shapes):
+    """Several stacks in one call (also more than one launch takes): every result against fp64, and the same bits as alone."""
+    from pylo_b200.optim import _common as K
+
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    xs = [torch.randn(s, device="cuda", generator=gen) for s in shapes]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    bufs = [K.newton_schulz_buffers(x, 5) for x in xs]
+    stream = torch.cuda.current_stream().cuda_stream
+    K.newton_schulz_native(xs, [o for o, _ in bufs], [w for _, w in bufs], COEFFS, 5, 1e-8, status, stream)
+    for x, (out, _) in zip(xs, bufs):
+        exact = K.newton_schulz(x.double(), COEFFS)
+        e32 = float((K.newton_schulz(x, COEFFS).double() - exact).norm() / exact.norm())
+        err = float((out.double() - exact).norm() / exact.norm())
+        assert err < max(4 * e32, 1e-5), (tuple(x.shape), err, e32)
+    assert int(status.item()) == 0
+
+
+def test_newton_schulz_with_unbounded_coefficients_leaves_the_fp16_planes():
+    from pylo_b200.optim import _common as K
+
+    assert K.newton_schulz_bounded(COEFFS, 5) and not K.newton_schulz_bounded((9.0, -2.0, 1.0), 5)
+    x = torch.randn(128, 256, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    coeffs = (4.0, -3.0, 1.0)
+    assert not K.newton_schulz_bounded(coeffs, 2)
+    exact = K.newton_schulz(x.double(), coeffs, 2)
+    assert float((K.newton_schulz_tc(x, coeffs, 2).double() - exact).norm() / exact.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("T", [1, 8, 9])
+def test_velo_gates_at_group_edges(T):
+    """One tensor, exactly one group of eight, one more than a group; 512 hidden units (weight rows in registers)."""
+    from oracle import pylo_oracle as O
+    from pylo_b200 import models, optim
+
+    shapes = [(12 + i, 8) for i in range(T)]
+    torch.manual_seed(0)
+    rnn, mlp = models.VeLORNN(), models.VeLOMLP()
+    with torch.no_grad():
+        for name, p in mlp.named_parameters():
+            if name.endswith("_") or "_." in name:
+                p.mul_(0.05)
+    ora = O.VeLOOracle(O.rnn_weights_from_module(rnn), O.bank_from_module(mlp), shapes, lr=1.0, num_steps=100)
+    case = dict(shapes=shapes, init_seed=61, init_scale=0.1, grad_seed=62, grad_scale=0.3)
+    params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+    ref = [v.clone() for v in cases.init_values(case)]
+    opt = optim.VeLO_CUDA(params, lr=1.0, num_steps=100, rnn=rnn, mlp=mlp)
+    for t in (1, 2):
+        grads = cases.grads_at(case, t)
+        for p, g in zip(params, grads):
+            p.grad = g.cuda()
+        # a loss on the device, then a host number
+        opt.step(torch.tensor(cases.velo_loss(t), device="cuda") if t == 1 else cases.velo_loss(t))
+        ora.step(ref, grads, cases.velo_loss(t))
+    e = float((opt.lstm_hidden_state[0].cpu() - ora.lstm_hidden_state[0]).abs().max())
+    assert e < 1e-5, e
+    res = CU.compare({2: [p.detach().cpu() for p in params]}, {2: ref}, cases.init_values(case))
+    assert res[2][0] < 1e-5, res
+
+
+def test_steps_that_changed_hands():
+    """Step counters that differ between tensors, that are replaced, and gradients that move or are not contiguous."""
+    shapes = [(40, 24), (24, 40), (24,)]
+    runs = []
+    for variant in (0, 1):
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(dict(shapes=shapes, init_seed=71))]
+        opt = _make("adafaclo", params)
+        for t in (1, 2, 3, 4):
+            grads = [g.cuda() for g in cases.grads_at(dict(grad_seed=72, grad_scale=0.3, shapes=shapes), t)]
+            for k, (p, g) in enumerate(zip(params, grads)):
+                if t == 2 and k == 1:
+                    p.grad = None                      # this tensor falls a step behind
+                elif variant and p.dim() == 2:
+                    p.grad = g.t().contiguous().t()    # the same values with other strides
+                else:
+                    p.grad = g
+            if t == 4 and variant:
+                for p in params:                       # the same count in another tensor, as a loaded checkpoint has it
+                    opt.state[p]["step"] = opt.state[p]["step"].clone()
+            opt.step()
+        assert [float(opt.state[p]["step"]) for p in params] == [4.0, 3.0, 4.0]
+        runs.append([p.detach().clone() for p in params])
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+
+
+@pytest.mark.parametrize("cls", ["celo2", "elo_celo2"])
+def test_adamw_tensors_of_any_length(cls):
+    """Whole pieces of four, tails, and a length that keeps the three shared momenta unaligned."""
+    from oracle import pylo_oracle as O
+
+    shapes = [(4096,), (5,), (1027,), (1,), (2050,)]
+    case = dict(shapes=shapes, init_seed=81, init_scale=0.1, grad_seed=82, grad_scale=0.3)
+    params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+    ref = [v.clone() for v in cases.init_values(case)]
+    opt = _make(cls, params)
+    kw = dict(weight_decay=0.1, clip_grad=True) if cls == "celo2" else dict(weight_decay=0.1, clip_grad=True, adam_lr_mult=20.0)
+    ora = O.CELO2Oracle(_nets(cls).flat_weights(), lr=1e-2, shared_adam=(cls == "elo_celo2"), **kw)
+    for t in (1, 2, 3):
+        grads = cases.grads_at(case, t)
+        for p, g in zip(params, grads):
+            p.grad = g.cuda()
+        opt.step()
+        ora.step(ref, grads)
+    res = CU.compare({3: [p.detach().cpu() for p in params]}, {3: ref}, cases.init_values(case))
+    assert res[3][0] < 1e-5 and res[3][1] < 2e-5, res
