@@ -1308,8 +1308,11 @@ __device__ __forceinline__ uint64_t pk_feature(const PkBase& b) {
 #ifndef PK_CTAS_VELO
 #define PK_CTAS_VELO 2
 #endif
+#ifndef PK_CTAS_CELO2
+#define PK_CTAS_CELO2 2
+#endif
 template <int FAM>
-__global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : 2) k_apply_packed(const pylo_tensor_desc* __restrict__ descs,
+__global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_CTAS_CELO2) k_apply_packed(const pylo_tensor_desc* __restrict__ descs,
                                                         const pylo_atile* __restrict__ ctiles, int n_ctiles,
                                                         const pylo_step_params prm) {
   pdl_begin();
@@ -1989,24 +1992,40 @@ static int allow_dynamic_smem(K kernel, int bytes, bool (&flags)[PYLO_MAX_DEVICE
     if (!(cond)) return -1; \
   } while (0)
 
-template <int BN>
-static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
-  static bool configured[PYLO_MAX_DEVICES] = {};
-  constexpr int smem = (int)sizeof(NfSmem<BN>) + 1024;  // room to start the stages on a 1024-byte boundary
-  if (int rc = allow_dynamic_smem(k_gemm_f16x2<BN>, smem, configured)) return rc;
+template <int BM, int BN>
+static long long ns_deal(nf_group& grp) {
   long long tiles = 0;
   for (int k = 0; k < grp.n; ++k) {
     nf_args& g = grp.p[k].g;
-    g.per = nf_tiles_per_matrix<BN>((g.M + NF_BM - 1) / NF_BM, (g.N + BN - 1) / BN, g.symmetric);
+    g.per = nf_tiles_per_matrix<BM, BN>(g.M, g.N, g.symmetric);
     g.tile0 = (int)tiles;
     tiles += (long long)g.per * g.batch;
   }
-  if (tiles > 0x7fffffff) return -1;
-  // tiles of 128 x 256 where they fill the GPU; else half as wide ones: a small product is as long as its longest tile
-  if (BN == 256 && tiles < sm_count()) return ns_gemm<128>(grp, status, s);
   grp.tiles = (int)tiles;
-  launch(k_gemm_f16x2<BN>, grp.tiles < sm_count() ? grp.tiles : sm_count(), NF_THREADS, smem, s, grp, status);
+  return tiles;
+}
+template <class Smem, class K>
+static int ns_launch(K kernel, nf_group& grp, int ctas, int* status, cudaStream_t s) {
+  static bool configured[PYLO_MAX_DEVICES] = {};
+  constexpr int smem = (int)sizeof(Smem) + 1024;  // room to start the stages on a 1024-byte boundary
+  if (int rc = allow_dynamic_smem(kernel, smem, configured)) return rc;
+  launch(kernel, ctas, NF_THREADS, smem, s, grp, status);
   return launch_status();
+}
+// The tile by what fills the GPU: a launch is as long as the SM with the most tiles, and a pair's tile is worth it from about
+// one per pair of SMs on; below one per SM, half as wide ones.
+static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
+  const int sms = sm_count();
+  long long tiles = ns_deal<256, 256>(grp);
+  if (tiles > 0x3fffffff) return -1;
+  if (tiles * 8 >= sms / 2 * 7) {
+    const int ctas = (int)(2 * tiles < sms ? 2 * tiles : sms & ~1);
+    return ns_launch<NfSmem<256, true>>(k_gemm_f16x2_pair, grp, ctas, status, s);
+  }
+  tiles = ns_deal<NF_BM, 256>(grp);
+  if (tiles >= sms) return ns_launch<NfSmem<256, false>>(k_gemm_f16x2<256>, grp, sms, status, s);
+  tiles = ns_deal<NF_BM, 128>(grp);
+  return ns_launch<NfSmem<128, false>>(k_gemm_f16x2<128>, grp, (int)(tiles < sms ? tiles : sms), status, s);
 }
 
 extern "C" {
@@ -2390,6 +2409,7 @@ static int ns_chain(const pylo_ns_desc* const* ds, int n, int* status, cudaStrea
           g.P = (__half*)(t.base + w.bp); g.sP = sAp; g.ldp = w.lda_p; g.planeP = sAp * d.batch;
           g.M = g.N = g.K = w.r;
           g.alpha = d.c2 / (SA * SA); g.beta = d.c1; g.scale = SB; g.symmetric = 1;
+          if (d.c2 == 0.f) { g.K = 0; g.alpha = 1.0f; }   // no product: b = c1 a
         } else {                  // x' = c0 x + b x (wide), c0 x + x b (tall); the first round's x is d.x times inv
           q.A = wide ? t.b : t.x[cur];
           q.B = wide ? t.x[cur] : t.b;
@@ -2403,7 +2423,7 @@ static int ns_chain(const pylo_ns_desc* const* ds, int n, int* status, cudaStrea
         }
         q.g = g;
       }
-      if (int rc = ns_gemm<256>(grp, status, s)) return rc;
+      if (int rc = ns_gemm(grp, status, s)) return rc;
     }
   }
   return 0;
@@ -2445,7 +2465,7 @@ int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctil
   if (n_ctiles == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_CELO2: launch(k_apply_packed<PYLO_FAM_CELO2>, grid_for(n_ctiles, 2), NT, 0, s, descs, ctiles, n_ctiles, *prm); break;
+    case PYLO_FAM_CELO2: launch(k_apply_packed<PYLO_FAM_CELO2>, grid_for(n_ctiles, PK_CTAS_CELO2), NT, 0, s, descs, ctiles, n_ctiles, *prm); break;
     case PYLO_FAM_VELO: launch(k_apply_packed<PYLO_FAM_VELO>, grid_for(n_ctiles, PK_CTAS_VELO), NT, 0, s, descs, ctiles, n_ctiles, *prm); break;
     default: return -2;
   }

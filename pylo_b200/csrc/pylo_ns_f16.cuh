@@ -19,8 +19,8 @@
 // The same product of several stacks of matrices (a model has one stack per shape) goes into one launch: the tiles of all of
 // them are dealt over the SMs together, and a model of small matrices pays for one chain of launches, not one per shape.
 //
-// One persistent CTA per SM, ten warps: one lane issues the TMA copies, one lane the products (M = 128, N = 256, K steps of
-// 16), eight warps run the epilogue.  The tensor core truncates when it accumulates, so the contraction is cut into
+// One persistent CTA per SM, ten warps: one lane issues the TMA copies, one lane the products (K steps of 16), eight warps run
+// the epilogue.  The tensor core truncates when it accumulates, so the contraction is cut into
 // chunks of 256 that start from zero, alternating between two accumulators of 256 columns; the epilogue warps add the
 // chunks up with round-to-nearest in registers (128 per thread) while the next chunk is multiplied.  Results leave through
 // shared memory, 16 columns at a time, so that a warp's loads and stores cover whole sectors of four rows (straight from
@@ -34,7 +34,6 @@
 
 #define NF_BM 128
 #define NF_BK 64
-#define NF_STAGES 2
 #define NF_EPI_WARPS 8
 #define NF_THREADS ((NF_EPI_WARPS + 2) * 32)
 #define NF_CHUNK_BLOCKS 4       // K blocks per accumulation chunk (256 terms)
@@ -42,11 +41,16 @@
 #define NF_OUT_PITCH 20         // floats: 16 columns, rows 16-byte aligned and spread over the banks
 #define NF_GROUP 8              // products of one launch at most
 
-template <int BN>
-struct NfSmem {   // per stage: A hi, A lo (128 x 64 each), B hi, B lo (BN x 64 each)
-  unsigned char st[NF_STAGES][2 * (NF_BM / 64) * NF_BOX + 2 * (BN / 64) * NF_BOX];
+// PAIR: two CTAs on two SMs share a tile of 256 x 256 (cta_group::2): each holds its own 128 rows of A and one half of B's
+// columns, and the tensor cores of both read both halves.  Per product and SM a third less operand data crosses from L2 than
+// for a tile of 128 x 256 (64 instead of 96 KB per 64 terms; at that rate L2 is what binds), and a third stage fits.
+template <int BN, bool PAIR>
+struct NfSmem {   // per stage: A hi, A lo (128 x 64 each), B hi, B lo (BN x 64 each, of a pair one half)
+  static constexpr int STAGES = PAIR ? 3 : 2;
+  static constexpr int BROWS = PAIR ? BN / 2 : BN;
+  unsigned char st[STAGES][2 * (NF_BM / 64) * NF_BOX + 2 * (BROWS / 64) * NF_BOX];
   float out[NF_EPI_WARPS][32 * NF_OUT_PITCH];   // per epilogue warp: 32 rows x 16 columns on their way out
-  uint64_t full[NF_STAGES], empty[NF_STAGES], acc_ready[2], acc_free[2];
+  uint64_t full[STAGES], empty[STAGES], acc_ready[2], acc_free[2];
   uint32_t tmem_base;
   volatile int abort;
 };
@@ -70,68 +74,105 @@ struct nf_group { nf_problem p[NF_GROUP]; int n, tiles; };
 __device__ __forceinline__ void nf_expect(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void nf_tma(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int b, int plane) {
-  asm volatile("cp.async.bulk.tensor.4d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-               ::"r"(dst), "l"(map), "r"(smem_addr(bar)), "r"(x), "r"(y), "r"(b), "r"(plane) : "memory");
+template <bool PAIR>
+__device__ __forceinline__ void nf_tma(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int b, int plane) {
+  if constexpr (PAIR)   // the barrier may be the other CTA's
+    asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(b), "r"(plane) : "memory");
+  else
+    asm volatile("cp.async.bulk.tensor.4d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(b), "r"(plane) : "memory");
+}
+// the address of another CTA's copy of a shared variable
+__device__ __forceinline__ uint32_t nf_at_rank(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+  return a;
+}
+template <bool PAIR>
+__device__ __forceinline__ void nf_commit(uint64_t* bar) {
+  if constexpr (PAIR)   // arrives at the barrier of both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_addr(bar)), "h"((uint16_t)3) : "memory");
+  else
+    tc_commit(bar);
 }
 // descriptor of a 128-byte-swizzled operand of 64 x 64 boxes.  K-major: rows of 64 k, 8-row groups 1024 bytes apart (boxes
 // follow one another).  MN-major: rows are k, a row holds 64 mn; 8-k groups 1024 bytes apart, 64-mn boxes NF_BOX apart.
 __device__ __forceinline__ uint64_t nf_desc(uint32_t saddr, int mn) {
   return (uint64_t)((saddr >> 4) & 0x3fff) | ((uint64_t)(mn ? NF_BOX >> 4 : 1) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
+template <bool PAIR>
 __device__ __forceinline__ void nf_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+  if constexpr (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// fp32 accumulate, fp16 x fp16, M = 128
-__device__ __forceinline__ uint32_t nf_idesc(uint32_t n, int a_mn, int b_mn) {
-  return (1u << 4) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+// fp32 accumulate, fp16 x fp16, M = 128 or (a pair) 256
+__device__ __forceinline__ uint32_t nf_idesc(uint32_t m, uint32_t n, int a_mn, int b_mn) {
+  return (1u << 4) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
-// tiles of one matrix; symmetric: those whose columns are not all below the diagonal of their rows
-template <int BN>
-__host__ __device__ inline int nf_tiles_per_matrix(int tiles_m, int tiles_n, int symmetric) {
+// tiles of one matrix of BM x BN; symmetric: those whose columns are not all below the diagonal of their rows
+template <int BM, int BN>
+__host__ __device__ inline int nf_tiles_per_matrix(int M, int N, int symmetric) {
+  const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
   if (!symmetric) return tiles_m * tiles_n;
   int n = 0;
-  for (int tm = 0; tm < tiles_m; ++tm) n += tiles_n - tm * NF_BM / BN;
+  for (int tm = 0; tm < tiles_m; ++tm) n += tiles_n - tm * BM / BN;
   return n;
 }
-template <int BN>
-__device__ __forceinline__ void nf_tile_coords(int r, int tiles_m, int tiles_n, int symmetric, int& tm, int& tn) {
+template <int BM, int BN>
+__device__ __forceinline__ void nf_tile_coords(int r, int M, int N, int symmetric, int& tm, int& tn) {
+  const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
   if (!symmetric) { tm = r / tiles_n; tn = r % tiles_n; return; }
   for (tm = 0; tm < tiles_m; ++tm) {
-    const int first = tm * NF_BM / BN, cnt = tiles_n - first;
+    const int first = tm * BM / BN, cnt = tiles_n - first;
     if (r < cnt) { tn = first + r; return; }
     r -= cnt;
   }
   tm = 0; tn = 0;
 }
 
-// BN: 256, or 128 where 256 would not give every SM a tile
-template <int BN>
-__global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_constant__ nf_group grp, int* __restrict__ status) {
+template <int BN, bool PAIR>
+__device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restrict__ status) {
   extern __shared__ unsigned char nf_raw[];
-  using Smem = NfSmem<BN>;
-  Smem& sm = *reinterpret_cast<Smem*>(nf_raw + ((1024 - (smem_addr(nf_raw) & 1023)) & 1023));
-  constexpr int A_PLANE = (NF_BM / 64) * NF_BOX, B_PLANE = (BN / 64) * NF_BOX, STAGE = 2 * A_PLANE + 2 * B_PLANE;
+  using Smem = NfSmem<BN, PAIR>;
+  constexpr int STAGES = Smem::STAGES, TILE_M = PAIR ? 2 * NF_BM : NF_BM;
+  Smem& sm = *reinterpret_cast<Smem*>(nf_raw + ((1024 - (smem_addr(nf_raw) & 1023)) & 1023));   // at the same place in both CTAs of a pair
+  constexpr int A_PLANE = (NF_BM / 64) * NF_BOX, B_PLANE = (Smem::BROWS / 64) * NF_BOX, STAGE = 2 * A_PLANE + 2 * B_PLANE;
   // the warp index as a broadcast from lane 0: the role branches are warp-uniform and the issuing branch keeps its
   // descriptors in uniform registers
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int rank = PAIR ? (int)cluster_rank() : 0;
   if (tid == 0) {
-    for (int s = 0; s < NF_STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&sm.acc_ready[s], 1); mbar_init(&sm.acc_free[s], NF_EPI_WARPS); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&sm.acc_ready[s], 1); mbar_init(&sm.acc_free[s], (PAIR ? 2 : 1) * NF_EPI_WARPS); }
     sm.abort = 0;
   }
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  if (warp == 1) { tc_alloc(&sm.tmem_base, 512); tc_relinquish(); }
+  if (warp == 1) {
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sm.tmem_base)), "r"(512) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      tc_alloc(&sm.tmem_base, 512);
+      tc_relinquish();
+    }
+  }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync();   // the other CTA's barriers exist
   tc_fence_after();
   pdl_begin();
   const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);   // two accumulators of 256 columns
-  const int n_tiles = grp.tiles;
+  const int n_tiles = grp.tiles, first_tile = PAIR ? blockIdx.x >> 1 : blockIdx.x, tile_step = PAIR ? gridDim.x >> 1 : gridDim.x;
   // the product a tile belongs to, and its place there
   auto locate = [&](int tile, int& b, int& tm, int& tn) -> const nf_problem& {
     int k = 0;
@@ -139,7 +180,7 @@ __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_const
     const nf_args& g = grp.p[k].g;
     const int r = tile - g.tile0;
     b = r / g.per;
-    nf_tile_coords<BN>(r - b * g.per, (g.M + NF_BM - 1) / NF_BM, (g.N + BN - 1) / BN, g.symmetric, tm, tn);
+    nf_tile_coords<TILE_M, BN>(r - b * g.per, g.M, g.N, g.symmetric, tm, tn);
     return grp.p[k];
   };
 
@@ -149,40 +190,43 @@ __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_const
       asm volatile("fence.proxy.async;" ::: "memory");   // what earlier kernels stored is read through the async proxy
       long long kbc = 0;
       bool dead = false;
-      for (int tile = blockIdx.x; tile < n_tiles && !dead && !sm.abort; tile += gridDim.x) {
+      for (int tile = first_tile; tile < n_tiles && !dead && !sm.abort; tile += tile_step) {
         int b, tm, tn;
         const nf_problem& q = locate(tile, b, tm, tn);
         const int a_mn = q.g.a_mn, b_mn = q.g.b_mn, n_kb = (q.g.K + NF_BK - 1) / NF_BK;
         for (int kb = 0; kb < n_kb; ++kb, ++kbc) {
-          const int s = (int)(kbc % NF_STAGES);
-          const long long use = kbc / NF_STAGES;
+          const int s = (int)(kbc % STAGES);
+          const long long use = kbc / STAGES;
           if (use > 0 && !ns_wait(&sm.empty[s], (uint32_t)((use - 1) & 1), &sm.abort)) { dead = true; break; }
-          nf_expect(&sm.full[s], STAGE);   // boxes that reach beyond the matrix are filled with zeros and count in full
+          // boxes that reach beyond the matrix are filled with zeros and count in full; of a pair the first CTA's barrier
+          // takes the bytes of both
+          if (rank == 0) nf_expect(&sm.full[s], (PAIR ? 2 : 1) * STAGE);
+          const uint32_t bar = PAIR ? nf_at_rank(&sm.full[s], 0) : smem_addr(&sm.full[s]);
           uint32_t dst = smem_addr(sm.st[s]);
           const int k = kb * NF_BK;
           for (int plane = 0; plane < 2; ++plane)
 #pragma unroll
             for (int u = 0; u < NF_BM / 64; ++u, dst += NF_BOX) {
-              const int mn = tm * NF_BM + 64 * u;
-              nf_tma(dst, &q.A, &sm.full[s], a_mn ? mn : k, a_mn ? k : mn, b, plane);
+              const int mn = tm * TILE_M + rank * NF_BM + 64 * u;
+              nf_tma<PAIR>(dst, &q.A, bar, a_mn ? mn : k, a_mn ? k : mn, b, plane);
             }
           for (int plane = 0; plane < 2; ++plane)
 #pragma unroll
-            for (int u = 0; u < BN / 64; ++u, dst += NF_BOX) {
-              const int mn = tn * BN + 64 * u;
-              nf_tma(dst, &q.B, &sm.full[s], b_mn ? mn : k, b_mn ? k : mn, b, plane);
+            for (int u = 0; u < Smem::BROWS / 64; ++u, dst += NF_BOX) {
+              const int mn = tn * BN + rank * Smem::BROWS + 64 * u;
+              nf_tma<PAIR>(dst, &q.B, bar, b_mn ? mn : k, b_mn ? k : mn, b, plane);
             }
         }
       }
       // the CTA must not end while a copy into its shared memory is in flight: normally the issuing lane has waited for
       // every stage; after an abort wait (bounded) for the stages filled last
-      if (dead || sm.abort) {
-        for (long long f = kbc > NF_STAGES ? kbc - NF_STAGES : 0; f < kbc; ++f) {
-          const uint32_t a = smem_addr(&sm.full[f % NF_STAGES]);
+      if (rank == 0 && (dead || sm.abort)) {
+        for (long long f = kbc > STAGES ? kbc - STAGES : 0; f < kbc; ++f) {
+          const uint32_t a = smem_addr(&sm.full[f % STAGES]);
           for (int it = 0; it < NS_SPIN_LIMIT; ++it) {
             uint32_t ok;
             asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                         : "=r"(ok) : "r"(a), "r"((uint32_t)((f / NF_STAGES) & 1)) : "memory");
+                         : "=r"(ok) : "r"(a), "r"((uint32_t)((f / STAGES) & 1)) : "memory");
             if (ok) break;
           }
         }
@@ -190,15 +234,15 @@ __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_const
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ products
-    if (elect_one()) {
+    // ------------------------------------------------------------------ products (of a pair the first CTA issues them)
+    if (rank == 0 && elect_one()) {
       long long kbc = 0, cc = 0;
       bool dead = false;
-      for (int tile = blockIdx.x; tile < n_tiles && !dead && !sm.abort; tile += gridDim.x) {
+      for (int tile = first_tile; tile < n_tiles && !dead && !sm.abort; tile += tile_step) {
         int b, tm, tn;
         const nf_problem& q = locate(tile, b, tm, tn);
         const int a_mn = q.g.a_mn, b_mn = q.g.b_mn, n_kb = (q.g.K + NF_BK - 1) / NF_BK;
-        const uint32_t idesc = nf_idesc(BN, a_mn, b_mn);
+        const uint32_t idesc = nf_idesc(TILE_M, BN, a_mn, b_mn);
         const uint64_t a_step = (a_mn ? 2048 : 32) >> 4, b_step = (b_mn ? 2048 : 32) >> 4;   // 16 terms further along K
         for (int kb = 0; kb < n_kb; ++kb, ++kbc) {
           const int in_chunk = kb % NF_CHUNK_BLOCKS;
@@ -207,20 +251,20 @@ __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_const
             if (!ns_wait(&sm.acc_free[cc & 1], (uint32_t)(((cc >> 1) - 1) & 1), &sm.abort)) { dead = true; break; }
             tc_fence_after();
           }
-          const int s = (int)(kbc % NF_STAGES);
-          if (!ns_wait(&sm.full[s], (uint32_t)((kbc / NF_STAGES) & 1), &sm.abort)) { dead = true; break; }
+          const int s = (int)(kbc % STAGES);
+          if (!ns_wait(&sm.full[s], (uint32_t)((kbc / STAGES) & 1), &sm.abort)) { dead = true; break; }
           tc_fence_after();
           const uint32_t base = smem_addr(sm.st[s]);
           const uint64_t ah = nf_desc(base, a_mn), al = nf_desc(base + A_PLANE, a_mn);
           const uint64_t bh = nf_desc(base + 2 * A_PLANE, b_mn), bl = nf_desc(base + 2 * A_PLANE + B_PLANE, b_mn);
 #pragma unroll
-          for (int ks = 0; ks < NF_BK / 16; ++ks) nf_mma(acc, al + ks * a_step, bh + ks * b_step, idesc, (in_chunk > 0 || ks > 0) ? 1u : 0u);
+          for (int ks = 0; ks < NF_BK / 16; ++ks) nf_mma<PAIR>(acc, al + ks * a_step, bh + ks * b_step, idesc, (in_chunk > 0 || ks > 0) ? 1u : 0u);
 #pragma unroll
-          for (int ks = 0; ks < NF_BK / 16; ++ks) nf_mma(acc, ah + ks * a_step, bl + ks * b_step, idesc, 1u);
+          for (int ks = 0; ks < NF_BK / 16; ++ks) nf_mma<PAIR>(acc, ah + ks * a_step, bl + ks * b_step, idesc, 1u);
 #pragma unroll
-          for (int ks = 0; ks < NF_BK / 16; ++ks) nf_mma(acc, ah + ks * a_step, bh + ks * b_step, idesc, 1u);
-          tc_commit(&sm.empty[s]);
-          if (in_chunk == NF_CHUNK_BLOCKS - 1 || kb == n_kb - 1) { tc_commit(&sm.acc_ready[cc & 1]); ++cc; }
+          for (int ks = 0; ks < NF_BK / 16; ++ks) nf_mma<PAIR>(acc, ah + ks * a_step, bh + ks * b_step, idesc, 1u);
+          nf_commit<PAIR>(&sm.empty[s]);
+          if (in_chunk == NF_CHUNK_BLOCKS - 1 || kb == n_kb - 1) { nf_commit<PAIR>(&sm.acc_ready[cc & 1]); ++cc; }
         }
       }
     }
@@ -234,13 +278,51 @@ __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_const
     const int sr = lane >> 2, sc = (lane & 3) * 4;   // on the way out: row sr + 8 i, columns sc .. sc + 3 of 16
     long long cc = 0;
     bool dead = false;
-    for (int tile = blockIdx.x; tile < n_tiles && !dead && !sm.abort; tile += gridDim.x) {
+    for (int tile = first_tile; tile < n_tiles && !dead && !sm.abort; tile += tile_step) {
       int b, tm, tn;
       const nf_args& g = locate(tile, b, tm, tn).g;
       const int n_kb = (g.K + NF_BK - 1) / NF_BK, n_chunks = (n_kb + NF_CHUNK_BLOCKS - 1) / NF_CHUNK_BLOCKS;
+      const int M = g.M, N = g.N, ldc = g.ldc, ldd = g.ldd, ldp = g.ldp, sym = g.symmetric;
+      const int m0 = tm * TILE_M + rank * NF_BM + quarter * 32;
+      const float alpha = g.alpha, scale = g.scale;
       float run[HALF];
+      if (g.D) {
+        // beta D / alpha is what the sum starts from: read while the first products run.  alpha is a power of two where D is
+        // large (x'), so nothing is rounded that would not be rounded at the end.
+        const float f = (g.d_scale ? g.beta * g.d_scale[b] : g.beta) / alpha;
+        const float* const D = g.D + (long long)b * g.sD;
+        const bool dvec = (ldd & 3) == 0;
 #pragma unroll
-      for (int j = 0; j < HALF; ++j) run[j] = 0.f;
+        for (int q = 0; q < HALF / 16; ++q) {
+          const int n0 = tn * BN + col0 + 16 * q, n = n0 + sc;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int m = m0 + sr + 8 * i;
+            float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (m < M && n < N && (!sym || n + 3 >= m)) {
+              const float* drow = D + (long long)m * ldd + n;
+              if (dvec && n + 3 < ldd) d = ld4(drow);
+              else {
+                d.x = drow[0];
+                if (n + 1 < N) d.y = drow[1];
+                if (n + 2 < N) d.z = drow[2];
+                if (n + 3 < N) d.w = drow[3];
+              }
+            }
+            st4(stage + (sr + 8 * i) * NF_OUT_PITCH + sc, d);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            const float4 d = ld4(stage + lane * NF_OUT_PITCH + 4 * h);
+            run[16 * q + 4 * h] = f * d.x; run[16 * q + 4 * h + 1] = f * d.y; run[16 * q + 4 * h + 2] = f * d.z; run[16 * q + 4 * h + 3] = f * d.w;
+          }
+          __syncwarp();
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < HALF; ++j) run[j] = 0.f;
+      }
       for (int c = 0; c < n_chunks; ++c, ++cc) {
         if (!ns_wait(&sm.acc_ready[cc & 1], (uint32_t)((cc >> 1) & 1), &sm.abort)) { dead = true; break; }
         tc_fence_after();
@@ -255,17 +337,16 @@ __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_const
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) ns_arrive(&sm.acc_free[cc & 1]);
+        if (lane == 0) {
+          if constexpr (PAIR) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(nf_at_rank(&sm.acc_free[cc & 1], 0)) : "memory");
+          else ns_arrive(&sm.acc_free[cc & 1]);
+        }
       }
       if (dead) break;
-      const int M = g.M, N = g.N, ldc = g.ldc, ldd = g.ldd, ldp = g.ldp, sym = g.symmetric;
-      const int m0 = tm * NF_BM + quarter * 32;
-      const float alpha = g.alpha, scale = g.scale, beta = g.d_scale ? g.beta * g.d_scale[b] : g.beta;
-      const float* const D = g.D ? g.D + (long long)b * g.sD : nullptr;
       float* const C = g.C ? g.C + (long long)b * g.sC : nullptr;
       __half* const P = g.P ? g.P + (long long)b * g.sP : nullptr;
       const long long planeP = g.planeP;
-      const bool dvec = (ldd & 3) == 0, cvec = (ldc & 3) == 0;
+      const bool cvec = (ldc & 3) == 0;
 #pragma unroll
       for (int q = 0; q < HALF / 16; ++q) {
         const int n0 = tn * BN + col0 + 16 * q;
@@ -282,17 +363,6 @@ __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_const
             if (m < M && n < N && (!sym || n + 3 >= m)) {
               float4 o = ld4(stage + rr * NF_OUT_PITCH + sc);
               float v[4] = {o.x, o.y, o.z, o.w};
-              if (D) {
-                const float* drow = D + (long long)m * ldd + n;
-                if (dvec && n + 3 < ldd) {
-                  const float4 d = ld4(drow);
-                  v[0] = fmaf(beta, d.x, v[0]); v[1] = fmaf(beta, d.y, v[1]); v[2] = fmaf(beta, d.z, v[2]); v[3] = fmaf(beta, d.w, v[3]);
-                } else {
-#pragma unroll
-                  for (int j = 0; j < 4; ++j) if (n + j < N) v[j] = fmaf(beta, drow[j], v[j]);
-                }
-                if (sym) st4(stage + rr * NF_OUT_PITCH + sc, make_float4(v[0], v[1], v[2], v[3]));   // for the mirror below
-              }
               if (C) {
                 float* crow = C + (long long)m * ldc + n;
                 if (cvec && n + 3 < ldc) st4(crow, make_float4(v[0], v[1], v[2], v[3]));
@@ -322,26 +392,19 @@ __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_const
           }
           __syncwarp();
           if (sym && P) {
-            // the mirror image: a row per lane again, so the lanes of a warp write neighbours of row n0 + j
+            // the mirror image, from the accumulators: the lanes of a warp write neighbours of row n0 + j
             const int m = m0 + lane;
-            float w[16];
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              const float4 o = ld4(stage + lane * NF_OUT_PITCH + 4 * h);
-              w[4 * h] = o.x; w[4 * h + 1] = o.y; w[4 * h + 2] = o.z; w[4 * h + 3] = o.w;
-            }
             if (m < M) {
               __half* pcol = P + m;
 #pragma unroll
               for (int j = 0; j < 16; ++j)
                 if (n0 + j > m && n0 + j < N) {
-                  const float s = w[j] * scale;
+                  const float s = alpha * run[16 * q + j] * scale;
                   const __half hi = __float2half_rn(s);
                   pcol[(long long)(n0 + j) * ldp] = hi;
                   pcol[planeP + (long long)(n0 + j) * ldp] = __float2half_rn(s - __half2float(hi));
                 }
             }
-            __syncwarp();
           }
         }
       }
@@ -349,8 +412,21 @@ __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_const
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync();   // neither CTA leaves while the other's products may read its shared memory
   if (tid == 0 && sm.abort && status) atomicOr(status, 4);
-  if (warp == 1) tc_dealloc(tmem, 512);
+  if (warp == 1) {
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    else tc_dealloc(tmem, 512);
+  }
+}
+
+// 256 x 256 on pairs of SMs where that fills the GPU, else 128 x 256, else 128 x 128 on one SM
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2_pair(const __grid_constant__ nf_group grp, int* __restrict__ status) {
+  nf_gemm_body<256, true>(grp, status);
+}
+template <int BN>
+__global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_constant__ nf_group grp, int* __restrict__ status) {
+  nf_gemm_body<BN, false>(grp, status);
 }
 
 // ------------------------------------------------------------------------------------------------

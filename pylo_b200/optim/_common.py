@@ -102,6 +102,8 @@ def newton_schulz_bounded(coeffs, iters: int) -> bool:
     All of them are polynomials of the singular values, which start in [0, 1]; their largest values are followed through
     the iterations on a fine grid.  The usual coefficients stay below 1.3."""
     c0, c1, c2 = coeffs
+    if c2 != 0.0 and abs(c1) > 1e6 * abs(c2):   # the kernel adds c1 a / c2 to a a
+        return False
     top = 1.0
     for _ in range(iters):
         s = np.linspace(0.0, top, 4001)

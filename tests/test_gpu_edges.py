@@ -53,9 +53,10 @@ def test_shapes_at_the_edges_match_the_oracle(family, extra, which):
     assert res[2][0] < 1e-5 and res[2][1] < 2e-5, res
 
 
-# matrices of the shared-memory kernel, of the 128- and 256-wide tiles, with K tails and odd pitches, wide and tall
+# matrices of the shared-memory kernel, of the 128- and 256-wide tiles and of tiles on pairs of SMs, with K tails and odd
+# pitches, wide and tall
 STACKS = [[(1, 5)], [(64, 64), (3, 16, 16), (10, 128)], [(65, 67), (67, 65), (2, 129, 257)], [(128, 128), (7, 3001), (3001, 7), (100, 260)],
-          [(1024, 1030), (258, 1024), (2, 200, 392), (33, 1000), (1000, 33), (5, 5), (96, 96), (300, 300), (131, 70), (70, 131)]]
+          [(2, 1300, 1290), (1290, 2050)], [(1024, 1030), (258, 1024), (2, 200, 392), (33, 1000), (1000, 33), (5, 5), (96, 96), (300, 300), (131, 70), (70, 131)]]
 
 
 @pytest.mark.parametrize("shapes", STACKS, ids=[str(len(s)) + "x" + str(s[0]) for s in STACKS])
@@ -85,6 +86,8 @@ def test_newton_schulz_with_unbounded_coefficients_leaves_the_fp16_planes():
     coeffs = (4.0, -3.0, 1.0)
     assert not K.newton_schulz_bounded(coeffs, 2)
     exact = K.newton_schulz(x.double(), coeffs, 2)
+    cubic = K.newton_schulz(x.double(), (1.5, -0.5, 0.0), 3)   # no quintic term: one product less per round
+    assert float((K.newton_schulz_tc(x, (1.5, -0.5, 0.0), 3).double() - cubic).norm() / cubic.norm()) < 1e-5
     assert float((K.newton_schulz_tc(x, coeffs, 2).double() - exact).norm() / exact.norm()) < 1e-5
 
 
