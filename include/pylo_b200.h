@@ -402,11 +402,11 @@ typedef struct pylo_velo_loss {
   float value;
   int32_t pad_;
 } pylo_velo_loss;
-/* velo_tensor_features also does finalize_moments for its tensors (leave that call out).  fraction9 is a HOST array of 9,
- * lossbuf a HOST pointer: the launch uses the features the buffer has after this step's loss, and velo_rnn, which must
+/* velo_tensor_features also does finalize_moments for its tensors (leave that call out).  fraction: step / num_steps, of
+ * which the nine time features are made (velo_cuda.py:155-162); lossbuf is a HOST pointer: the launch uses the features the buffer has after this step's loss, and velo_rnn, which must
  * follow with the same lossbuf, advances it (NULL there: it is left as it is). */
 int pylo_b200_velo_tensor_features(const pylo_tensor_desc* descs, int n_local, const int32_t* layer_of,
-                                   int n_total, const float* rank_onehot, const float* fraction9,
+                                   int n_total, const float* rank_onehot, float fraction,
                                    const pylo_velo_loss* lossbuf, float* x_in, void* stream);
 int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, const pylo_velo_loss* lossbuf, void* stream);
 /* The loss buffer's update and features alone: writes loss9[9]. */

@@ -141,7 +141,7 @@ def _load():
         "pylo_b200_celo2_post_sums": [vp, vp, i32, vp],
         "pylo_b200_celo2_post_apply": [vp, vp, i32, vp],
         "pylo_b200_adamw": [vp, vp, i32, i32] + [f32] * 7 + [C.POINTER(StepParams), vp],
-        "pylo_b200_velo_tensor_features": [vp, i32, vp, i32, vp, vp, C.POINTER(VeloLoss), vp, vp],
+        "pylo_b200_velo_tensor_features": [vp, i32, vp, i32, vp, f32, C.POINTER(VeloLoss), vp, vp],
         "pylo_b200_velo_rnn": [C.POINTER(VeloRnn), C.POINTER(VeloLoss), vp],
         "pylo_b200_velo_loss_features": [vp, vp, vp, vp, vp, vp, vp],
         "pylo_b200_step": [C.POINTER(StepPlan), C.POINTER(StepParams), i32, vp],

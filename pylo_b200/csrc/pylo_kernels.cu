@@ -1309,7 +1309,7 @@ __device__ __forceinline__ uint64_t pk_feature(const PkBase& b) {
 #define PK_CTAS_VELO 2
 #endif
 #ifndef PK_CTAS_CELO2
-#define PK_CTAS_CELO2 2
+#define PK_CTAS_CELO2 1   // its 8-wide layers want registers more than a second CTA: 2989 -> 2753 us over a Llama block
 #endif
 template <int FAM>
 __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_CTAS_CELO2) k_apply_packed(const pylo_tensor_desc* __restrict__ descs,
@@ -1671,11 +1671,10 @@ __global__ void k_velo_loss(const pylo_velo_loss b, float* __restrict__ loss9) {
 // The 30 LSTM inputs of a tensor from the statistics gathered in phase B (velo_cuda.py:213-252).  One CTA per tensor, which
 // first does phase B2 for it (a launch less), while its last warp works out the loss features: every CTA for itself and
 // without advancing the loss buffer, which is left to a kernel that runs when all of them are done (k_velo_xmix).
-struct VeloFraction { float f[9]; };
 template <int ROWS>
 __global__ void __launch_bounds__(ROWS * PYLO_STAT_STRIDE + 32) k_velo_tensor_features(const pylo_tensor_desc* __restrict__ descs,
                                        const int32_t* __restrict__ layer_of, int T,
-                                       const float* __restrict__ rank_onehot, const VeloFraction fraction9,
+                                       const float* __restrict__ rank_onehot, float fraction,
                                        const pylo_velo_loss lossbuf, float* __restrict__ x_in) {
   pdl_begin();
   __shared__ double s_d[ROWS][PYLO_STAT_STRIDE];
@@ -1699,7 +1698,11 @@ __global__ void __launch_bounds__(ROWS * PYLO_STAT_STRIDE + 32) k_velo_tensor_fe
   const double norm = (double)rsqrtf(fmaxf(mean_p2, 1e-9f));
   const double mean_v = stat(6) / n, e_v2 = stat(7) / n;
   float o = 0.f;
-  if (tid < 9) o = fraction9.f[tid];
+  if (tid < 9) {  // tanh((x - t) * 10) (velo_cuda.py:155-162)
+    const float at[9] = {0.03f, 0.1f, 0.2f, 0.4f, 0.6f, 0.8f, 0.9f, 1.0f, 1.1f};
+#pragma unroll
+    for (int j = 0; j < 9; ++j) if (tid == j) o = tanhf((fraction - at[j]) * 10.0f);
+  }
   else if (tid < 18) o = s_loss9[tid - 9];
   else if (tid == 18) o = clip_log_abs10((float)(norm * mean_v));
   else if (tid < 24) o = rank_onehot[t * 5 + tid - 19];
@@ -2500,14 +2503,12 @@ int pylo_b200_adamw(const pylo_adam_item* items, const pylo_tile* tiles, int n_t
 }
 
 int pylo_b200_velo_tensor_features(const pylo_tensor_desc* descs, int n_local, const int32_t* layer_of,
-                                   int n_total, const float* rank_onehot, const float* fraction9,
+                                   int n_total, const float* rank_onehot, float fraction,
                                    const pylo_velo_loss* lossbuf, float* x_in, void* stream) {
-  CHECK_ARG(descs && rank_onehot && fraction9 && x_in && n_local > 0 && n_total >= n_local);
+  CHECK_ARG(descs && rank_onehot && x_in && n_local > 0 && n_total >= n_local);
   CHECK_ARG(lossbuf && lossbuf->means && lossbuf->iteration && lossbuf->running_min && lossbuf->decays);
-  VeloFraction f;
-  memcpy(&f, fraction9, sizeof(f));
   launch(k_velo_tensor_features<20>, n_local, 20 * PYLO_STAT_STRIDE + 32, 0, (cudaStream_t)stream, descs, layer_of, n_total,
-         rank_onehot, f, *lossbuf, x_in);
+         rank_onehot, fraction, *lossbuf, x_in);
   return launch_status();
 }
 

@@ -32,7 +32,7 @@ from torch.optim import Optimizer
 from .. import _lib as L
 from ..models.Meta_MLP import MetaMLP
 from ..plan import GradNorm, LoPlan, LoTensor, current_stream_ptr, one_minus, with_gradients
-from ._common import StepCounters, factored_dims_sorted, require_cuda_param
+from ._common import StepCounters, factored_dims_sorted, optimizer_step, require_cuda_param
 
 
 def _decay_to_param(x):
@@ -221,7 +221,7 @@ class AdafacLO_CUDA(_AdafacFamily):
                     st["step"] = torch.tensor(float(st["step"]), dtype=torch.float64)
         self._plans = {}
 
-    @torch.no_grad()
+    @optimizer_step
     def step(self, loss=None):
         stream = current_stream_ptr()
         for gi, group in enumerate(self.param_groups):
@@ -276,7 +276,7 @@ class ELO_CUDA(_AdafacFamily):
         self.mlp_precision = mlp_precision
         self._finish_init(self.network)
 
-    @torch.no_grad()
+    @optimizer_step
     def step(self, loss=None):
         stream = current_stream_ptr()
         gnorm_ptr = None

@@ -32,7 +32,7 @@ from ..models.CELO2_MLP import CELO2MLP
 from ..plan import (GradNorm, LoPlan, LoTensor, current_stream_ptr, grad_pointers, one_minus, tile_elems,
                     with_gradients)
 from ._common import (ItemPlan, factored_dims_argsort, newton_schulz, newton_schulz_bounded, newton_schulz_buffers,
-                      newton_schulz_native, newton_schulz_tc, require_cuda_param)
+                      newton_schulz_native, newton_schulz_tc, optimizer_step, require_cuda_param)
 
 _IN, _HID = 30, 8
 _KEPT_FLOATS = 4 << 20  # elements up to which a plan keeps Newton-Schulz results and workspaces between steps
@@ -218,7 +218,7 @@ class _Celo2Family(Optimizer):
             raise L.PyloLibError(f"{self._name}: a wait inside the Newton-Schulz kernel timed out; the step is invalid")
 
     # ------------------------------------------------------------------ step
-    @torch.no_grad()
+    @optimizer_step
     def step(self, loss=None):
         stream = current_stream_ptr()
         gnorm_ptr = None

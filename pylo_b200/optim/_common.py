@@ -4,10 +4,12 @@ from __future__ import annotations
 
 import ctypes as C_
 import functools
+import sys
 from typing import List, Optional, Sequence
 
 import numpy as np
 import torch
+from torch.optim import Optimizer
 
 from .. import _lib as L
 from ..plan import DeviceTable, make_tiles
@@ -188,6 +190,29 @@ def require_cuda_param(p: torch.Tensor, who: str):
         raise RuntimeError(f"{who}: only fp32 parameters are supported, got {p.dtype}")
     if not p.is_contiguous():
         raise RuntimeError(f"{who}: parameters must be contiguous")
+
+
+def optimizer_step(step):
+    """Decorator of an optimizer's ``step``: torch's own wrapper (profiler range, step hooks) and ``no_grad``, but only where
+    something can see them.
+
+    The wrapper costs as much as all launches of a small model's step.  The steps of this package run no differentiable
+    operation on a parameter, so without hooks and without a profiler a plain call does the same."""
+    watched = Optimizer.profile_hook_step(torch.no_grad()(step))
+    module = sys.modules[Optimizer.__module__]
+    hooks = [getattr(module, name, None) for name in ("_global_optimizer_pre_hooks", "_global_optimizer_post_hooks")]
+    profiling = getattr(torch.autograd, "_profiler_enabled", None)
+
+    @functools.wraps(step)
+    def run(self, *args, **kwargs):
+        own = self.__dict__
+        if (profiling is None or profiling() or None in hooks or hooks[0] or hooks[1]
+                or own.get("_optimizer_step_pre_hooks", True) or own.get("_optimizer_step_post_hooks", True)):
+            return watched(self, *args, **kwargs)
+        return step(self, *args, **kwargs)
+
+    run.hooked = True   # tells the base class that the wrapper is there
+    return run
 
 
 class StepCounters:

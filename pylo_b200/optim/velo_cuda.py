@@ -20,7 +20,6 @@ and the apply sweep, which reads each tensor's mixed weights and its
 from __future__ import annotations
 
 import ctypes as C
-import math
 
 import numpy as np
 import torch
@@ -31,7 +30,7 @@ from .. import _lib as L
 from ..models.VeLO_MLP import VeLOMLP
 from ..models.VeLO_RNN import VeLORNN
 from ..plan import LoPlan, LoTensor, current_stream_ptr, one_minus
-from ._common import factored_dims_velo, require_cuda_param
+from ._common import factored_dims_velo, optimizer_step, require_cuda_param
 
 
 def _decay_to_param(x):
@@ -40,14 +39,6 @@ def _decay_to_param(x):
 
 def _param_to_decay(x):
     return 1 - torch.exp(x * 10.0)
-
-
-_FRACTIONS = np.array([0.03, 0.1, 0.2, 0.4, 0.6, 0.8, 0.9, 1.0, 1.1], dtype=np.float32)
-
-
-def fractional_tanh_embed(x: float):
-    """tanh((x - t) * 10) in fp32 for the nine time fractions of velo_cuda.py:155-162."""
-    return [math.tanh(v) for v in ((np.float32(x) - _FRACTIONS) * np.float32(10)).tolist()]
 
 
 def init_loss_buffer(num_steps, device):
@@ -242,10 +233,10 @@ class VeLO_CUDA(Optimizer):
         for k in ("x_in", "pooled", "xmix", "gates", "controls", "weights", "lr_mult"):
             setattr(r, k, buf[k].data_ptr())
         r.T, r.H, r.B = T, H, B
-        return {"plan": plan, "buf": buf, "rnn": r, "loss": L.VeloLoss(), "fraction": (C.c_float * 9)(), "hyper": None}
+        return {"plan": plan, "buf": buf, "rnn": r, "loss": L.VeloLoss(), "hyper": None}
 
     # ------------------------------------------------------------------ step
-    @torch.no_grad()
+    @optimizer_step
     def step(self, loss):
         stream = current_stream_ptr()
         dev = self.device
@@ -288,7 +279,6 @@ class VeLO_CUDA(Optimizer):
             loss_arg.loss, loss_arg.value = None, float(loss)
         loss_arg.means, loss_arg.iteration = lb["means"].data_ptr(), lb["iteration"].data_ptr()
         loss_arg.running_min, loss_arg.decays = lb["running_min"].data_ptr(), lb["decays"].data_ptr()
-        ctx["fraction"][:] = fractional_tanh_embed(fraction)
 
         prm = self._prm
         if prm is None:
@@ -307,7 +297,7 @@ class VeLO_CUDA(Optimizer):
         if sharded:
             buf["x_in"].zero_()
         L.check(L.lib.pylo_b200_velo_tensor_features(plan.desc.ptr, plan.n_tensors, buf["layer_of"].data_ptr(), int(r.T),
-                                                     buf["rank"].data_ptr(), ctx["fraction"], C.byref(loss_arg),
+                                                     buf["rank"].data_ptr(), float(fraction), C.byref(loss_arg),
                                                      buf["x_in"].data_ptr(), stream),
                 "velo_tensor_features")
         if sharded and torch.distributed.is_initialized() and torch.distributed.get_world_size(self._pg) > 1:

@@ -337,14 +337,17 @@ class LoPlan:
             shapes_c.append((unit_of[i], X, Y) + apply_tile_shape(family, X, Y, self.tensor_cores))
         slow_units = [u for u in range(U) if udesc["mode"][u] != L.MODE_FAST2D]
         if self.tensor_cores:
-            # the tensor-core kernel takes every tensor: what is not FAST2D as runs of 128 elements, with as many per
-            # item as for a FAST2D tensor; a model too small to give every warpgroup an item gets smaller ones
+            # The tensor-core kernel takes every tensor: what is not FAST2D as runs of 128 elements.  The height of the
+            # items is the one that makes the busiest worker's share shortest, over all tensors together (the shape's own
+            # rule looks at one tensor): an item's set-up costs about one and a half rows.  86 M ViT-B/16 parameters: 64
+            # rows instead of 8, sweep 2050 -> 1750 us.
             gen = [(u, (sizes[u] + 127) // 128) for u in slow_units]
-            shapes_c = [(u, X, 128) + apply_tile_shape(family, X, 128, True)[:2] + (L.TC_GEN_ITEM,) for u, X in gen] + [
-                (u, X, Y, rt, width, 0) for u, X, Y, rt, width, _ in shapes_c]
-            n_items = lambda k: sum(-(-X // max(1, rt >> k)) * -(-Y // w) for _, X, Y, rt, w, _ in shapes_c)
-            k = next((k for k in range(3) if n_items(k + 1) > L.TC_WORKERS), 3)
-            shapes_c = [(u, X, Y, max(1, rt >> k), w, tag | max(1, rt >> k)) for u, X, Y, rt, w, tag in shapes_c]
+            shapes_c = [(u, X, 128, L.TC_GEN_ITEM) for u, X in gen] + [(u, X, Y, 0) for u, X, Y, *_ in shapes_c]
+            xs = np.array([X for _, X, _, _ in shapes_c])
+            cols = np.array([-(-Y // 128) for _, _, Y, _ in shapes_c])
+            share = lambda R: -(-int((-(-xs // R) * cols).sum()) // L.TC_WORKERS) * (R + 1.5)
+            rt = min((64, 32, 16, 8, 4, 2, 1), key=share)
+            shapes_c = [(u, X, Y, rt, 128, tag | rt) for u, X, Y, tag in shapes_c]
             slow_units = []
         elif family != L.FAM_ADAFAC:
             # rows per thread: 64 (a tile's start costs about a row's time), fewer while the model does not give every SM
