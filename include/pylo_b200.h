@@ -148,6 +148,9 @@ typedef struct pylo_step_params {
   const float* gnorm_sq;  /* device scalar: sum of squares of all gradients, or NULL */
   int32_t sum_tiles;      /* prep_apply: 1 = add the tile partials up itself (finalize_moments was not called) */
   int32_t pad_;
+  int* status;            /* device int: state_moments ORs 8 in if a bounded wait for its own copies ran out (the step is
+                             then incomplete); may be NULL */
+  int* host_status;       /* the same in pinned host memory; may be NULL */
 } pylo_step_params;
 
 int pylo_b200_abi_version(void);

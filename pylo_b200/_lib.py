@@ -57,6 +57,7 @@ class StepParams(C.Structure):
         ("w_m", C.c_float * 3), ("w_v", C.c_float), ("w_f", C.c_float * 3),
         ("eps_v", C.c_float), ("eps_feat", C.c_float), ("eps_norm", C.c_float), ("clip_val", C.c_float),
         ("no_tables", C.c_int32), ("gnorm_sq", C.c_void_p), ("sum_tiles", C.c_int32), ("pad_", C.c_int32),
+        ("status", C.c_void_p), ("host_status", C.c_void_p),
     ]
 
 

@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "pylo_common.cuh"
+#include "pylo_pipe.cuh"
 
 // ================================================================================================
 // feature construction (reference order; learned_optimizer.cu:59-96, celo2_kernel.cu:87-124)
@@ -470,22 +471,57 @@ __device__ __forceinline__ void velo_stats(float (&acc)[BAcc<FAM>::N], float m0,
   }
 }
 
+// Bound by HBM on large models.  FAST2D tiles come through the ring of pylo_pipe.cuh: the copies run ahead over tile borders,
+// so that neither the next loads nor the block reduction at a tile's end leave the memory idle.  The other tiles are read
+// into registers.
 template <int FAM>
 __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc* __restrict__ descs,
                                                       const pylo_tile* __restrict__ tiles, int n_tiles, int reverse,
                                                       const pylo_step_params prm) {
-  pdl_begin();
   using F = Fam<FAM>;
   constexpr int NACC = BAcc<FAM>::N;
+  extern __shared__ __align__(128) unsigned char pipe_raw[];
+  PipeSmem& pipe = *reinterpret_cast<PipeSmem*>(pipe_raw);
   __shared__ float s_red[NWARP * NACC];
   const int tid = threadIdx.x;
-  for (int tt = blockIdx.x; tt < n_tiles; tt += gridDim.x) {
+  pipe_init(pipe);
+  pdl_begin();
+  uint32_t k = 0;   // stages consumed
+  // the first warp's cursor, PIPE_STAGES - 1 stages ahead of the consumers: lane u < 6 copies stream u
+  int ptt = blockIdx.x - gridDim.x, pc = 0, pcnt = 0;
+  uint32_t pk = 0;
+  const float* psrc = nullptr;
+  auto produce = [&]() -> bool {
+    while (pc >= pcnt) {   // on to the next FAST2D tile
+      ptt += gridDim.x;
+      if (ptt >= n_tiles) { ptt = n_tiles; return true; }
+      const pylo_tile tl = tiles[reverse ? (n_tiles - 1 - ptt) : ptt];
+      const pylo_tensor_desc& d = descs[tl.tensor];
+      if (d.mode != PYLO_MODE_FAST2D) continue;
+      pc = 0;
+      pcnt = tile_count(tl, d.n);
+      psrc = (tid == 0 ? d.g : tid == 1 ? d.p : tid == 5 ? d.v : d.m + (tid - 2) * d.m_stride) + tl.start;
+    }
+    const uint32_t bytes = 4u * min(PIPE_ELEMS, pcnt - pc);
+    if (!pipe_begin(pipe, pk, PIPE_STREAMS * bytes)) return false;
+    if (tid < PIPE_STREAMS) pipe_copy(pipe, pk, tid, 0, psrc + pc, bytes);
+    pc += PIPE_ELEMS;
+    ++pk;
+    return true;
+  };
+  if (tid < 32) {
+    asm volatile("fence.proxy.async;" ::: "memory");   // what earlier kernels stored is read through the async proxy
+    for (int s = 0; s < PIPE_STAGES - 1; ++s) produce();
+  }
+  bool dead = false;
+  for (int tt = blockIdx.x; tt < n_tiles && !dead; tt += gridDim.x) {
     const int t = reverse ? (n_tiles - 1 - tt) : tt;
     const pylo_tile tl = tiles[t];
     const pylo_tensor_desc& d = descs[tl.tensor];
     const int64_t n = d.n, start = tl.start;
     const int cnt = tile_count(tl, n);
     const float gs = grad_scale_of(d, prm);
+    const bool plain = plain_grad(gs, prm);
     float acc[NACC];
 #pragma unroll
     for (int j = 0; j < NACC; ++j) acc[j] = 0.f;
@@ -498,37 +534,50 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
 
     if (d.mode == PYLO_MODE_FAST2D) {
       const uint32_t Y = d.Y;
-      const bool small = n < (1ll << 32);
-      for (int i = tid * 4; i < cnt; i += NT * 4) {
-        const int64_t idx = start + i;
-        uint32_t x, y;
-        if (small) { x = (uint32_t)idx / Y; y = (uint32_t)idx - x * Y; }
-        else { x = (uint32_t)(idx / Y); y = (uint32_t)(idx - (int64_t)x * Y); }
-        const float4 g4 = ldg4(gp + i), p4 = ld4(pp + i);
-        float4 a0 = ld4(m0p + i), a1 = ld4(m1p + i), a2 = ld4(m2p + i), v4 = ld4(vp + i);
-        const float4 fa = ld4(d.fx + 4 * (int64_t)x);
-        const float4 b0 = ld4(d.f_b + y), b1 = ld4(d.f_b + Y + y), b2 = ld4(d.f_b + 2 * (int64_t)Y + y);
-        float ge[4] = {g4.x, g4.y, g4.z, g4.w}, pe[4] = {p4.x, p4.y, p4.z, p4.w};
-        float m0e[4] = {a0.x, a0.y, a0.z, a0.w}, m1e[4] = {a1.x, a1.y, a1.z, a1.w}, m2e[4] = {a2.x, a2.y, a2.z, a2.w};
-        float ve[4] = {v4.x, v4.y, v4.z, v4.w};
-        const float b0e[4] = {b0.x, b0.y, b0.z, b0.w}, b1e[4] = {b1.x, b1.y, b1.z, b1.w}, b2e[4] = {b2.x, b2.y, b2.z, b2.w};
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float g = xform_grad(ge[u], gs, prm.clip_val, prm.nan_to_num);
-          velo_stats<FAM>(acc, m0e[u], m1e[u], m2e[u], ve[u]);
-          m0e[u] = lerp_torch(m0e[u], g, prm.w_m[0]);
-          m1e[u] = lerp_torch(m1e[u], g, prm.w_m[1]);
-          m2e[u] = lerp_torch(m2e[u], g, prm.w_m[2]);
-          ve[u] = lerp_torch(ve[u], g * g + prm.eps_v, prm.w_v);
-          const float rs = rsqrtf(ve[u] + prm.eps_feat);
-          float f[F::NF];
-          elem_features<FAM>(f, g, pe[u], m0e[u], m1e[u], m2e[u], ve[u], rs, fa.x * b0e[u], fa.y * b1e[u], fa.z * b2e[u]);
-          accumulate<FAM, false>(acc, f);
+      // this thread's row and column (n < 2^31 here), moved on by a stage's length
+      const uint32_t first = (uint32_t)start + tid * 4;
+      uint32_t x = first / Y, y = first - x * Y;
+      const uint32_t dx = PIPE_ELEMS / Y, dy = PIPE_ELEMS - dx * Y;
+      const float* __restrict__ fxp = d.fx;
+      const float* __restrict__ fbp = d.f_b;
+      for (int i = tid * 4; i - tid * 4 < cnt; i += PIPE_ELEMS, ++k) {
+        const bool ok = i < cnt;
+        float4 fa = make_float4(0.f, 0.f, 0.f, 0.f), b0 = fa, b1 = fa, b2 = fa;
+        if (ok) {
+          fa = ld4(fxp + 4 * (int64_t)x);
+          b0 = ld4(fbp + y); b1 = ld4(fbp + Y + y); b2 = ld4(fbp + 2 * (int64_t)Y + y);
         }
-        st4(m0p + i, make_float4(m0e[0], m0e[1], m0e[2], m0e[3]));
-        st4(m1p + i, make_float4(m1e[0], m1e[1], m1e[2], m1e[3]));
-        st4(m2p + i, make_float4(m2e[0], m2e[1], m2e[2], m2e[3]));
-        st4(vp + i, make_float4(ve[0], ve[1], ve[2], ve[3]));
+        x += dx; y += dy;
+        if (y >= Y) { y -= Y; ++x; }
+        if (tid < 32 && !produce()) { dead = true; break; }
+        if (!pipe_wait_full(pipe, k)) { dead = true; break; }
+        if (ok) {
+          const float(*st)[PIPE_ELEMS] = pipe.st[k % PIPE_STAGES];
+          const float4 g4 = ld4(&st[0][tid * 4]), p4 = ld4(&st[1][tid * 4]);
+          const float4 a0 = ld4(&st[2][tid * 4]), a1 = ld4(&st[3][tid * 4]), a2 = ld4(&st[4][tid * 4]), v4 = ld4(&st[5][tid * 4]);
+          float ge[4] = {g4.x, g4.y, g4.z, g4.w}, pe[4] = {p4.x, p4.y, p4.z, p4.w};
+          float m0e[4] = {a0.x, a0.y, a0.z, a0.w}, m1e[4] = {a1.x, a1.y, a1.z, a1.w}, m2e[4] = {a2.x, a2.y, a2.z, a2.w};
+          float ve[4] = {v4.x, v4.y, v4.z, v4.w};
+          const float b0e[4] = {b0.x, b0.y, b0.z, b0.w}, b1e[4] = {b1.x, b1.y, b1.z, b1.w}, b2e[4] = {b2.x, b2.y, b2.z, b2.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float g = plain ? ge[u] : xform_grad(ge[u], gs, prm.clip_val, prm.nan_to_num);
+            velo_stats<FAM>(acc, m0e[u], m1e[u], m2e[u], ve[u]);
+            m0e[u] = lerp_torch(m0e[u], g, prm.w_m[0]);
+            m1e[u] = lerp_torch(m1e[u], g, prm.w_m[1]);
+            m2e[u] = lerp_torch(m2e[u], g, prm.w_m[2]);
+            ve[u] = lerp_torch(ve[u], g * g + prm.eps_v, prm.w_v);
+            const float rs = rsqrtf(ve[u] + prm.eps_feat);
+            float f[F::NF];
+            elem_features<FAM>(f, g, pe[u], m0e[u], m1e[u], m2e[u], ve[u], rs, fa.x * b0e[u], fa.y * b1e[u], fa.z * b2e[u]);
+            accumulate<FAM, false>(acc, f);
+          }
+          st4(m0p + i, make_float4(m0e[0], m0e[1], m0e[2], m0e[3]));
+          st4(m1p + i, make_float4(m1e[0], m1e[1], m1e[2], m1e[3]));
+          st4(m2p + i, make_float4(m2e[0], m2e[1], m2e[2], m2e[3]));
+          st4(vp + i, make_float4(ve[0], ve[1], ve[2], ve[3]));
+        }
+        pipe_release(pipe, k);
       }
     } else if (d.mode == PYLO_MODE_GENERIC) {
       const int64_t La = d.La, Lb = d.Lb;
@@ -619,6 +668,8 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
     block_reduce_store<NACC>(acc, s_red, out);
     if (tid >= NACC && tid < PYLO_STAT_STRIDE) out[tid] = 0.f;
   }
+  if (dead && (tid & 31) == 0) pipe_failed(prm);
+  if (dead && tid < 32) pipe_drain(pipe, pk);
 }
 
 // ================================================================================================
@@ -2031,6 +2082,14 @@ static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
   return ns_launch<NfSmem<128, false>>(k_gemm_f16x2<128>, grp, (int)(tiles < sms ? tiles : sms), status, s);
 }
 
+template <class K>
+static int state_moments_launch(K kernel, const pylo_tensor_desc* descs, const pylo_tile* tiles, int n_tiles, int reverse,
+                                const pylo_step_params& prm, bool (&configured)[PYLO_MAX_DEVICES], cudaStream_t s) {
+  if (int rc = allow_dynamic_smem(kernel, (int)sizeof(PipeSmem), configured)) return rc;
+  launch(kernel, grid_for(n_tiles, 2), NT, sizeof(PipeSmem), s, descs, tiles, n_tiles, reverse, prm);
+  return 0;
+}
+
 extern "C" {
 
 int pylo_b200_abi_version(void) { return PYLO_B200_ABI_VERSION; }
@@ -2183,13 +2242,15 @@ int pylo_b200_state_moments(const pylo_tensor_desc* descs, const pylo_tile* tile
   CHECK_ARG(descs && tiles && prm && n_tiles >= 0);
   if (n_tiles == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
-  const int grid = grid_for(n_tiles, 4);
+  static bool configured[3][PYLO_MAX_DEVICES] = {};
+  int rc = 0;
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: launch(k_state_moments<PYLO_FAM_ADAFAC>, grid, NT, 0, s, descs, tiles, n_tiles, reverse, *prm); break;
-    case PYLO_FAM_CELO2: launch(k_state_moments<PYLO_FAM_CELO2>, grid, NT, 0, s, descs, tiles, n_tiles, reverse, *prm); break;
-    case PYLO_FAM_VELO: launch(k_state_moments<PYLO_FAM_VELO>, grid, NT, 0, s, descs, tiles, n_tiles, reverse, *prm); break;
+    case PYLO_FAM_ADAFAC: rc = state_moments_launch(k_state_moments<PYLO_FAM_ADAFAC>, descs, tiles, n_tiles, reverse, *prm, configured[PYLO_FAM_ADAFAC], s); break;
+    case PYLO_FAM_CELO2: rc = state_moments_launch(k_state_moments<PYLO_FAM_CELO2>, descs, tiles, n_tiles, reverse, *prm, configured[PYLO_FAM_CELO2], s); break;
+    case PYLO_FAM_VELO: rc = state_moments_launch(k_state_moments<PYLO_FAM_VELO>, descs, tiles, n_tiles, reverse, *prm, configured[PYLO_FAM_VELO], s); break;
     default: return -2;
   }
+  if (rc) return rc;
   return launch_status();
 }
 

@@ -213,7 +213,10 @@ class _Celo2Family(Optimizer):
         return prm
 
     def check_status(self):
-        """Synchronise and raise if the Newton-Schulz kernel reported a wait that ran out (its output is incomplete)."""
+        """Synchronise and raise if a kernel reported a wait that ran out (its output is incomplete)."""
+        for _, plan in self._plans.values():
+            if plan["lo"] is not None:
+                plan["lo"].check_status()
         if int(self._ns_status.item()) != 0:
             raise L.PyloLibError(f"{self._name}: a wait inside the Newton-Schulz kernel timed out; the step is invalid")
 

@@ -191,6 +191,11 @@ class VeLO_CUDA(Optimizer):
         super().add_param_group(param_group)
         self._plan = None
 
+    def check_status(self):
+        """Synchronise and raise if a kernel of an earlier step reported a wait that ran out."""
+        if self._plan is not None:
+            self._plan[1]["plan"].check_status()
+
     # ------------------------------------------------------------------ planning
     def _build_plan(self, plist):
         dev = self.device

@@ -370,11 +370,11 @@ class LoPlan:
             self.apply_kernel = "k_apply_adafac_cols"
         else:
             self.apply_kernel = "k_apply_packed<CELO2>" if family == L.FAM_CELO2 else "k_apply_packed<VELO>"
-        #: device flag the tensor-core kernel raises when one of its bounded waits ran out
-        self.status = torch.zeros(128, dtype=torch.int32, device=self.device) if self.tensor_cores else None
+        #: device flag that a kernel raises when one of its bounded waits ran out
+        self.status = torch.zeros(128, dtype=torch.int32, device=self.device)
         # its twin in pinned host memory, written by the kernel itself: the next step looks at it without asking the device
-        self._status_host = torch.zeros(1, dtype=torch.int32).pin_memory() if self.tensor_cores else None
-        self._status_view = self._status_host.numpy() if self.tensor_cores else None
+        self._status_host = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self._status_view = self._status_host.numpy()
         # the other units' apply sweep: vectors are short and every element costs a whole network, so the tiles are as
         # small as one element per thread where that is what fills the GPU (five 4096-vectors: 104 us as one tile each)
         slow_sizes = [sizes[u] for u in slow_units]
@@ -388,8 +388,7 @@ class LoPlan:
         self.step_plan = L.StepPlan(
             tdesc=self.tdesc.ptr, desc=self.desc.ptr, atiles=self.atiles.ptr, gitems=self.gitems.ptr, pitems=self.pitems.ptr,
             ctiles=self.ctiles.ptr, tiles=self.tiles.ptr, tiles_slow=self.tiles_slow.ptr,
-            status=self.status.data_ptr() if self.tensor_cores else None,
-            host_status=self._status_host.data_ptr() if self.tensor_cores else None,
+            status=self.status.data_ptr(), host_status=self._status_host.data_ptr(),
             n_tensors=T, n_units=U, n_atiles=self.n_atiles, n_gitems=self.n_gitems, n_pitems=self.n_pitems,
             n_ctiles=self.n_ctiles, n_ctiles_gen=self.n_ctiles_gen, n_tiles=self.n_tiles, n_tiles_slow=self.n_tiles_slow,
             tensor_cores=int(self.tensor_cores), sum_tiles=int(self.sum_tiles))
@@ -492,6 +491,7 @@ class LoPlan:
         """The phases of a step (all of them, or only those before or after the caller's own work in between)."""
         self._poll_status()  # before any state of this step is touched
         prm.step_delta = self.step_delta
+        prm.status, prm.host_status = self.step_plan.status, self.step_plan.host_status
         if self._prof is None:
             L.check(L.lib.pylo_b200_step(self._step_plan_ref, C.byref(prm), phases, stream), "step")
             if phases & L.STEP_FRONT:
@@ -518,11 +518,11 @@ class LoPlan:
             self._call("finalize_moments", L.lib.pylo_b200_finalize_moments, self.desc.ptr, self.n_units, stream)
 
     def _poll_status(self):
-        """Raise if a tensor-core launch of an earlier step has written its status word."""
-        if self._status_view is not None and self._status_view[0] != 0:
-            raise L.PyloLibError("apply_adafac_tc: a wait on the tensor core timed out in an earlier step; the kernel "
-                                 "kept the old values of the parameters it could not finish, and launches write "
-                                 "nothing until clear_status() is called")
+        """Raise if a launch of an earlier step has written its status word."""
+        if self._status_view[0] != 0:
+            raise L.PyloLibError("a bounded wait inside a kernel timed out in an earlier step (apply_adafac_tc: the kernel kept "
+                                 "the old values of the parameters it could not finish, and launches write nothing until "
+                                 "clear_status() is called)")
 
     def _back(self, prm, stream):
         """Phases P, C, one call each (timed)."""
@@ -546,21 +546,23 @@ class LoPlan:
             self._call("k_apply", L.lib.pylo_b200_apply, self.desc.ptr, self.tiles_slow.ptr, self.n_tiles_slow, 0, pp, stream)
 
     def check_status(self):
-        """Synchronise and raise if the tensor-core kernel reported a wait that ran out.
+        """Synchronise and raise if a kernel reported a wait that ran out.
 
-        The kernel keeps the old value of every parameter it could not finish, so nothing invalid was written, but
-        the step is incomplete; until :meth:`clear_status` the kernel stores nothing at all.  Call this before a
+        The tensor-core kernel keeps the old value of every parameter it could not finish, so nothing invalid was
+        written, but the step is incomplete; until :meth:`clear_status` it stores nothing at all.  Call this before a
         checkpoint is written."""
-        if self.status is not None and int(self.status[0].item()) != 0:
+        code = int(self.status[0].item())
+        if code & 8:
+            raise L.PyloLibError("a wait for a kernel's own copies timed out; this step is incomplete")
+        if code != 0:
             raise L.PyloLibError("apply_adafac_tc: a wait on the tensor core timed out; this step is incomplete "
                                  "(unfinished parameters kept their old values)")
 
     def clear_status(self):
         """Acknowledge a reported timeout: the next launches store again."""
-        if self.status is not None:
-            self.status.zero_()
-            torch.cuda.synchronize(self.device)   # a launch in flight may still write the host's word
-            self._status_host.zero_()
+        self.status.zero_()
+        torch.cuda.synchronize(self.device)   # a launch in flight may still write the host's word
+        self._status_host.zero_()
 
 
 class GradNorm:
