@@ -147,7 +147,8 @@ typedef struct pylo_step_params {
                              1 = neither, 2 = the per-row table only (what the tensor-core apply kernel reads) */
   const float* gnorm_sq;  /* device scalar: sum of squares of all gradients, or NULL */
   int32_t sum_tiles;      /* prep_apply: 1 = add the tile partials up itself (finalize_moments was not called) */
-  int32_t pad_;
+  int32_t bulk_copies;    /* state_moments: 1 = FAST2D tiles come through a ring of bulk copies, for large models that consist
+                             of them; 0 = all tiles are read into registers */
   int* status;            /* device int: state_moments ORs 8 in if a bounded wait for its own copies ran out (the step is
                              then incomplete); may be NULL */
   int* host_status;       /* the same in pinned host memory; may be NULL */

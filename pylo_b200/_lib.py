@@ -56,7 +56,7 @@ class StepParams(C.Structure):
         ("family", C.c_int32), ("nan_to_num", C.c_int32), ("wd_mode", C.c_int32), ("step_delta", C.c_float),
         ("w_m", C.c_float * 3), ("w_v", C.c_float), ("w_f", C.c_float * 3),
         ("eps_v", C.c_float), ("eps_feat", C.c_float), ("eps_norm", C.c_float), ("clip_val", C.c_float),
-        ("no_tables", C.c_int32), ("gnorm_sq", C.c_void_p), ("sum_tiles", C.c_int32), ("pad_", C.c_int32),
+        ("no_tables", C.c_int32), ("gnorm_sq", C.c_void_p), ("sum_tiles", C.c_int32), ("bulk_copies", C.c_int32),
         ("status", C.c_void_p), ("host_status", C.c_void_p),
     ]
 
@@ -167,6 +167,7 @@ TC_WORKERS = SM_COUNT * 4  # warpgroups the tensor-core apply kernel runs at onc
 TC_GEN_ITEM = 1 << 16  # tag bit of its items on tensors that are not FAST2D
 STEP_FRONT, STEP_BACK = 1, 2
 TC_ONE_LAUNCH = 8 * TC_WORKERS  # items below which one launch of the tensor-core kernel takes both kinds of items
+BULK_COPY_ELEMS = 1 << 26  # FAST2D elements from which the state sweep reads through a ring of bulk copies
 STATIC_SCRATCH_TILES = 65536
 ERR_STATIC_SCRATCH_TOO_SMALL = -4
 

@@ -471,20 +471,21 @@ __device__ __forceinline__ void velo_stats(float (&acc)[BAcc<FAM>::N], float m0,
   }
 }
 
-// Bound by HBM on large models.  FAST2D tiles come through the ring of pylo_pipe.cuh: the copies run ahead over tile borders,
-// so that neither the next loads nor the block reduction at a tile's end leave the memory idle.  The other tiles are read
-// into registers.
-template <int FAM>
+// Bound by HBM on large models.  With RING, FAST2D tiles come through the ring of pylo_pipe.cuh: the copies run ahead over tile
+// borders, so that neither the next loads nor the block reduction at a tile's end leave the memory idle.  Everything else is
+// read into registers; without RING all tiles are, and the memory that the ring would take is the L1 cache in which the
+// factor vectors of strided tensors are found.
+template <int FAM, bool RING>
 __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc* __restrict__ descs,
                                                       const pylo_tile* __restrict__ tiles, int n_tiles, int reverse,
                                                       const pylo_step_params prm) {
   using F = Fam<FAM>;
   constexpr int NACC = BAcc<FAM>::N;
   extern __shared__ __align__(128) unsigned char pipe_raw[];
-  PipeSmem& pipe = *reinterpret_cast<PipeSmem*>(pipe_raw);
+  PipeSmem& pipe = *reinterpret_cast<PipeSmem*>(pipe_raw);   // RING only
   __shared__ float s_red[NWARP * NACC];
   const int tid = threadIdx.x;
-  pipe_init(pipe);
+  if constexpr (RING) pipe_init(pipe);
   pdl_begin();
   uint32_t k = 0;   // stages consumed
   // the first warp's cursor, PIPE_STAGES - 1 stages ahead of the consumers: lane u < 6 copies stream u
@@ -509,7 +510,7 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
     ++pk;
     return true;
   };
-  if (tid < 32) {
+  if (RING && tid < 32) {
     asm volatile("fence.proxy.async;" ::: "memory");   // what earlier kernels stored is read through the async proxy
     for (int s = 0; s < PIPE_STAGES - 1; ++s) produce();
   }
@@ -540,7 +541,30 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
       const uint32_t dx = PIPE_ELEMS / Y, dy = PIPE_ELEMS - dx * Y;
       const float* __restrict__ fxp = d.fx;
       const float* __restrict__ fbp = d.f_b;
-      for (int i = tid * 4; i - tid * 4 < cnt; i += PIPE_ELEMS, ++k) {
+      auto update4 = [&](int i, float4 g4, float4 p4, float4 a0, float4 a1, float4 a2, float4 v4, float4 fa, float4 b0, float4 b1, float4 b2) {
+        float ge[4] = {g4.x, g4.y, g4.z, g4.w}, pe[4] = {p4.x, p4.y, p4.z, p4.w};
+        float m0e[4] = {a0.x, a0.y, a0.z, a0.w}, m1e[4] = {a1.x, a1.y, a1.z, a1.w}, m2e[4] = {a2.x, a2.y, a2.z, a2.w};
+        float ve[4] = {v4.x, v4.y, v4.z, v4.w};
+        const float b0e[4] = {b0.x, b0.y, b0.z, b0.w}, b1e[4] = {b1.x, b1.y, b1.z, b1.w}, b2e[4] = {b2.x, b2.y, b2.z, b2.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float g = plain ? ge[u] : xform_grad(ge[u], gs, prm.clip_val, prm.nan_to_num);
+          velo_stats<FAM>(acc, m0e[u], m1e[u], m2e[u], ve[u]);
+          m0e[u] = lerp_torch(m0e[u], g, prm.w_m[0]);
+          m1e[u] = lerp_torch(m1e[u], g, prm.w_m[1]);
+          m2e[u] = lerp_torch(m2e[u], g, prm.w_m[2]);
+          ve[u] = lerp_torch(ve[u], g * g + prm.eps_v, prm.w_v);
+          const float rs = rsqrtf(ve[u] + prm.eps_feat);
+          float f[F::NF];
+          elem_features<FAM>(f, g, pe[u], m0e[u], m1e[u], m2e[u], ve[u], rs, fa.x * b0e[u], fa.y * b1e[u], fa.z * b2e[u]);
+          accumulate<FAM, false>(acc, f);
+        }
+        st4(m0p + i, make_float4(m0e[0], m0e[1], m0e[2], m0e[3]));
+        st4(m1p + i, make_float4(m1e[0], m1e[1], m1e[2], m1e[3]));
+        st4(m2p + i, make_float4(m2e[0], m2e[1], m2e[2], m2e[3]));
+        st4(vp + i, make_float4(ve[0], ve[1], ve[2], ve[3]));
+      };
+      for (int i = tid * 4; i - tid * 4 < cnt; i += PIPE_ELEMS) {
         const bool ok = i < cnt;
         float4 fa = make_float4(0.f, 0.f, 0.f, 0.f), b0 = fa, b1 = fa, b2 = fa;
         if (ok) {
@@ -549,35 +573,16 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
         }
         x += dx; y += dy;
         if (y >= Y) { y -= Y; ++x; }
-        if (tid < 32 && !produce()) { dead = true; break; }
-        if (!pipe_wait_full(pipe, k)) { dead = true; break; }
-        if (ok) {
+        if constexpr (RING) {
+          if (tid < 32 && !produce()) { dead = true; break; }
+          if (!pipe_wait_full(pipe, k)) { dead = true; break; }
           const float(*st)[PIPE_ELEMS] = pipe.st[k % PIPE_STAGES];
-          const float4 g4 = ld4(&st[0][tid * 4]), p4 = ld4(&st[1][tid * 4]);
-          const float4 a0 = ld4(&st[2][tid * 4]), a1 = ld4(&st[3][tid * 4]), a2 = ld4(&st[4][tid * 4]), v4 = ld4(&st[5][tid * 4]);
-          float ge[4] = {g4.x, g4.y, g4.z, g4.w}, pe[4] = {p4.x, p4.y, p4.z, p4.w};
-          float m0e[4] = {a0.x, a0.y, a0.z, a0.w}, m1e[4] = {a1.x, a1.y, a1.z, a1.w}, m2e[4] = {a2.x, a2.y, a2.z, a2.w};
-          float ve[4] = {v4.x, v4.y, v4.z, v4.w};
-          const float b0e[4] = {b0.x, b0.y, b0.z, b0.w}, b1e[4] = {b1.x, b1.y, b1.z, b1.w}, b2e[4] = {b2.x, b2.y, b2.z, b2.w};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float g = plain ? ge[u] : xform_grad(ge[u], gs, prm.clip_val, prm.nan_to_num);
-            velo_stats<FAM>(acc, m0e[u], m1e[u], m2e[u], ve[u]);
-            m0e[u] = lerp_torch(m0e[u], g, prm.w_m[0]);
-            m1e[u] = lerp_torch(m1e[u], g, prm.w_m[1]);
-            m2e[u] = lerp_torch(m2e[u], g, prm.w_m[2]);
-            ve[u] = lerp_torch(ve[u], g * g + prm.eps_v, prm.w_v);
-            const float rs = rsqrtf(ve[u] + prm.eps_feat);
-            float f[F::NF];
-            elem_features<FAM>(f, g, pe[u], m0e[u], m1e[u], m2e[u], ve[u], rs, fa.x * b0e[u], fa.y * b1e[u], fa.z * b2e[u]);
-            accumulate<FAM, false>(acc, f);
-          }
-          st4(m0p + i, make_float4(m0e[0], m0e[1], m0e[2], m0e[3]));
-          st4(m1p + i, make_float4(m1e[0], m1e[1], m1e[2], m1e[3]));
-          st4(m2p + i, make_float4(m2e[0], m2e[1], m2e[2], m2e[3]));
-          st4(vp + i, make_float4(ve[0], ve[1], ve[2], ve[3]));
+          if (ok) update4(i, ld4(&st[0][tid * 4]), ld4(&st[1][tid * 4]), ld4(&st[2][tid * 4]), ld4(&st[3][tid * 4]), ld4(&st[4][tid * 4]),
+                          ld4(&st[5][tid * 4]), fa, b0, b1, b2);
+          pipe_release(pipe, k++);
+        } else if (ok) {
+          update4(i, ldg4(gp + i), ld4(pp + i), ld4(m0p + i), ld4(m1p + i), ld4(m2p + i), ld4(vp + i), fa, b0, b1, b2);
         }
-        pipe_release(pipe, k);
       }
     } else if (d.mode == PYLO_MODE_GENERIC) {
       const int64_t La = d.La, Lb = d.Lb;
@@ -668,8 +673,10 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
     block_reduce_store<NACC>(acc, s_red, out);
     if (tid >= NACC && tid < PYLO_STAT_STRIDE) out[tid] = 0.f;
   }
-  if (dead && (tid & 31) == 0) pipe_failed(prm);
-  if (dead && tid < 32) pipe_drain(pipe, pk);
+  if constexpr (RING) {
+    if (dead && (tid & 31) == 0) pipe_failed(prm);
+    if (dead && tid < 32) pipe_drain(pipe, pk);
+  }
 }
 
 // ================================================================================================
@@ -2012,6 +2019,11 @@ struct PlainLaunches {
   explicit PlainLaunches(int n_tiles) : before(t_plain_launches) { t_plain_launches = before || n_tiles > 8192; }
   ~PlainLaunches() { t_plain_launches = before; }
 };
+// The SMs' memory is split between L1 cache and shared memory anew only when they are idle, which programmatic launches never
+// let them be: the kernels after one with a large share of shared memory would run with what L1 it left (the apply sweep of
+// 6 x 4096 x 4096 VeLO parameters: 921 us after the state sweep's ring, 755 us without).  Such a kernel has itself and the next
+// launch of its thread made plainly.
+static thread_local bool t_plain_next = false;
 template <class... P, class... A>
 static void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchAttribute attr;
@@ -2023,7 +2035,8 @@ static void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cud
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = &attr;
-  cfg.numAttrs = t_plain_launches ? 0 : 1;
+  cfg.numAttrs = t_plain_launches || t_plain_next ? 0 : 1;
+  t_plain_next = false;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
@@ -2082,11 +2095,18 @@ static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
   return ns_launch<NfSmem<128, false>>(k_gemm_f16x2<128>, grp, (int)(tiles < sms ? tiles : sms), status, s);
 }
 
-template <class K>
-static int state_moments_launch(K kernel, const pylo_tensor_desc* descs, const pylo_tile* tiles, int n_tiles, int reverse,
-                                const pylo_step_params& prm, bool (&configured)[PYLO_MAX_DEVICES], cudaStream_t s) {
-  if (int rc = allow_dynamic_smem(kernel, (int)sizeof(PipeSmem), configured)) return rc;
-  launch(kernel, grid_for(n_tiles, 2), NT, sizeof(PipeSmem), s, descs, tiles, n_tiles, reverse, prm);
+template <int FAM>
+static int state_moments_launch(const pylo_tensor_desc* descs, const pylo_tile* tiles, int n_tiles, int reverse,
+                                const pylo_step_params& prm, cudaStream_t s) {
+  if (!prm.bulk_copies) {
+    launch(k_state_moments<FAM, false>, grid_for(n_tiles, 4), NT, 0, s, descs, tiles, n_tiles, reverse, prm);
+    return 0;
+  }
+  static bool configured[PYLO_MAX_DEVICES] = {};
+  if (int rc = allow_dynamic_smem(k_state_moments<FAM, true>, (int)sizeof(PipeSmem), configured)) return rc;
+  t_plain_next = true;
+  launch(k_state_moments<FAM, true>, grid_for(n_tiles, 2), NT, sizeof(PipeSmem), s, descs, tiles, n_tiles, reverse, prm);
+  t_plain_next = true;
   return 0;
 }
 
@@ -2242,12 +2262,11 @@ int pylo_b200_state_moments(const pylo_tensor_desc* descs, const pylo_tile* tile
   CHECK_ARG(descs && tiles && prm && n_tiles >= 0);
   if (n_tiles == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
-  static bool configured[3][PYLO_MAX_DEVICES] = {};
   int rc = 0;
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: rc = state_moments_launch(k_state_moments<PYLO_FAM_ADAFAC>, descs, tiles, n_tiles, reverse, *prm, configured[PYLO_FAM_ADAFAC], s); break;
-    case PYLO_FAM_CELO2: rc = state_moments_launch(k_state_moments<PYLO_FAM_CELO2>, descs, tiles, n_tiles, reverse, *prm, configured[PYLO_FAM_CELO2], s); break;
-    case PYLO_FAM_VELO: rc = state_moments_launch(k_state_moments<PYLO_FAM_VELO>, descs, tiles, n_tiles, reverse, *prm, configured[PYLO_FAM_VELO], s); break;
+    case PYLO_FAM_ADAFAC: rc = state_moments_launch<PYLO_FAM_ADAFAC>(descs, tiles, n_tiles, reverse, *prm, s); break;
+    case PYLO_FAM_CELO2: rc = state_moments_launch<PYLO_FAM_CELO2>(descs, tiles, n_tiles, reverse, *prm, s); break;
+    case PYLO_FAM_VELO: rc = state_moments_launch<PYLO_FAM_VELO>(descs, tiles, n_tiles, reverse, *prm, s); break;
     default: return -2;
   }
   if (rc) return rc;

@@ -384,6 +384,11 @@ class LoPlan:
         self.n_tiles_slow = len(slow)
         #: no launch for phase B2: of small units phase P adds the tile partials up, for VeLO the LSTM's input kernel does
         self.sum_tiles = family == L.FAM_VELO or max((k for _, k in ranges), default=0) <= 48
+        # The state sweep's ring of bulk copies leaves little L1 cache to the units that are not FAST2D and keeps the launches
+        # around it apart, so it has to have enough to do: from 64 M elements on (VeLO on 100 M: 1615 -> 1580 us per step, on
+        # 17 M: 341 -> 351; AdafacLO on 25 M: 837 -> 851, on 86 M even), nearly all of them FAST2D.
+        fast_elems = sum(sizes[u] for u in range(U) if udesc["mode"][u] == L.MODE_FAST2D)
+        self.bulk_copies = int(fast_elems >= L.BULK_COPY_ELEMS and 8 * fast_elems >= 7 * self.total_elems)
         #: everything pylo_b200_step needs for a step over these tensors
         self.step_plan = L.StepPlan(
             tdesc=self.tdesc.ptr, desc=self.desc.ptr, atiles=self.atiles.ptr, gitems=self.gitems.ptr, pitems=self.pitems.ptr,
@@ -492,6 +497,7 @@ class LoPlan:
         self._poll_status()  # before any state of this step is touched
         prm.step_delta = self.step_delta
         prm.status, prm.host_status = self.step_plan.status, self.step_plan.host_status
+        prm.bulk_copies = self.bulk_copies
         if self._prof is None:
             L.check(L.lib.pylo_b200_step(self._step_plan_ref, C.byref(prm), phases, stream), "step")
             if phases & L.STEP_FRONT:

@@ -6,6 +6,7 @@ import torch
 
 import cases
 import cuda_util as CU
+from pylo_b200 import _lib as pylo_lib
 from test_gpu_properties import _make, _nets, _step
 
 pytestmark = pytest.mark.gpu
@@ -51,6 +52,24 @@ def test_shapes_at_the_edges_match_the_oracle(family, extra, which):
         ora.step(ref, grads, cases.velo_loss(t)) if family == "velo" else ora.step(ref, grads)
     res = CU.compare({2: [p.detach().cpu() for p in params]}, {2: ref}, init)
     assert res[2][0] < 1e-5 and res[2][1] < 2e-5, res
+
+
+@pytest.mark.parametrize("family", ["adafaclo", "celo2", "velo"])
+def test_state_sweep_through_the_ring(family, monkeypatch):
+    """Large models' state sweep on small ones: tiles shorter than a stage, partial stages, tiles of other kinds in between."""
+    shapes = [(513, 64), (7,), (9, 1028), (3, 4), (600, 1040), (65, 7), (300, 4100)]
+    runs = []
+    for least in (pylo_lib.BULK_COPY_ELEMS, 1):
+        monkeypatch.setattr(pylo_lib, "BULK_COPY_ELEMS", least)
+        case = dict(shapes=shapes, init_seed=61, init_scale=0.1, grad_seed=62, grad_scale=0.3)
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+        opt = _make(family, params, **({"orthogonalize": False} if family == "celo2" else {}))
+        for t in (1, 2):
+            for p, g in zip(params, cases.grads_at(case, t)):
+                p.grad = g.cuda()
+            _step(opt, family, t)
+        runs.append([p.detach().clone() for p in params])
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
 
 
 # matrices of the shared-memory kernel, of the 128- and 256-wide tiles and of tiles on pairs of SMs, with K tails and odd
