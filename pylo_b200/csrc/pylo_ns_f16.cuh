@@ -19,10 +19,11 @@
 // The same product of several stacks of matrices (a model has one stack per shape) goes into one launch: the tiles of all of
 // them are dealt over the SMs together, and a model of small matrices pays for one chain of launches, not one per shape.
 //
-// One persistent CTA per SM, ten warps: one lane issues the TMA copies, one lane the products (K steps of 16), eight warps run
-// the epilogue.  The tensor core truncates when it accumulates, so the contraction is cut into
+// One persistent CTA per SM, eighteen warps: one lane issues the TMA copies, one lane the products (K steps of 16), sixteen
+// warps run the epilogue (its instructions wait for one another; eight warps were too few to hide that under a product with a
+// short K: chain on 12 x 768 x 3072 1317 us with eight, 1229 with sixteen; 4 x 768 x 3072 656 and 547).  The tensor core truncates when it accumulates, so the contraction is cut into
 // chunks of 256 that start from zero, alternating between two accumulators of 256 columns; the epilogue warps add the
-// chunks up with round-to-nearest in registers (128 per thread) while the next chunk is multiplied.  Results leave through
+// chunks up with round-to-nearest in registers (64 per thread) while the next chunk is multiplied.  Results leave through
 // shared memory, 16 columns at a time, so that a warp's loads and stores cover whole sectors of four rows (straight from
 // the accumulator layout, a row per lane, they touch 32 lines each and bound every product with K < 1000).
 //
@@ -34,11 +35,10 @@
 
 #define NF_BM 128
 #define NF_BK 64
-#define NF_EPI_WARPS 8
+#define NF_EPI_WARPS 16
 #define NF_THREADS ((NF_EPI_WARPS + 2) * 32)
 #define NF_CHUNK_BLOCKS 4       // K blocks per accumulation chunk (256 terms)
 #define NF_BOX 8192             // bytes of one TMA box: 64 x 64 fp16
-#define NF_OUT_PITCH 20         // floats: 16 columns, rows 16-byte aligned and spread over the banks
 #define NF_GROUP 8              // products of one launch at most
 
 // PAIR: two CTAs on two SMs share a tile of 256 x 256 (cta_group::2): each holds its own 128 rows of A and one half of B's
@@ -49,7 +49,7 @@ struct NfSmem {   // per stage: A hi, A lo (128 x 64 each), B hi, B lo (BN x 64 
   static constexpr int STAGES = PAIR ? 3 : 2;
   static constexpr int BROWS = PAIR ? BN / 2 : BN;
   unsigned char st[STAGES][2 * (NF_BM / 64) * NF_BOX + 2 * (BROWS / 64) * NF_BOX];
-  float out[NF_EPI_WARPS][32 * NF_OUT_PITCH];   // per epilogue warp: 32 rows x 16 columns on their way out
+  float out[NF_EPI_WARPS][32 * 16];   // per epilogue warp: 32 rows x 16 columns on their way out
   uint64_t full[STAGES], empty[STAGES], acc_ready[2], acc_free[2];
   uint32_t tmem_base;
   volatile int abort;
@@ -89,6 +89,15 @@ __device__ __forceinline__ uint32_t nf_at_rank(const void* p, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
   return a;
 }
+__device__ __forceinline__ void nf_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+}
+// four columns (quad 0..3) of a row of a warp's 32 x 16 stage; neighbouring rows' quads are spread over the banks
+__device__ __forceinline__ float* nf_out(float* stage, int row, int quad) { return stage + row * 16 + 4 * (quad ^ ((row >> 1) & 3)); }
 template <bool PAIR>
 __device__ __forceinline__ void nf_commit(uint64_t* bar) {
   if constexpr (PAIR)   // arrives at the barrier of both CTAs
@@ -274,9 +283,9 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
     }
     __syncwarp();
   } else {
-    // ------------------------------------------------------------------ epilogue: a thread adds up half a row of the tile
-    constexpr int HALF = BN / 2;           // columns per thread
-    const int quarter = warp & 3, col0 = ((warp - 2) >> 2) * HALF;
+    // ------------------------------------------------------------------ epilogue: a thread adds up a quarter of a row of the tile
+    constexpr int COLS = BN * 4 / NF_EPI_WARPS;   // columns per thread
+    const int quarter = warp & 3, col0 = ((warp - 2) >> 2) * COLS;
     const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
     float* const stage = sm.out[warp - 2];
     const int sr = lane >> 2, sc = (lane & 3) * 4;   // on the way out: row sr + 8 i, columns sc .. sc + 3 of 16
@@ -289,7 +298,7 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
       const int M = g.M, N = g.N, ldc = g.ldc, ldd = g.ldd, ldp = g.ldp, sym = g.symmetric;
       const int m0 = tm * TILE_M + rank * NF_BM + quarter * 32;
       const float alpha = g.alpha, scale = g.scale;
-      float run[HALF];
+      float run[COLS];
       if (g.D) {
         // beta D / alpha is what the sum starts from: read while the first products run.  alpha is a power of two where D is
         // large (x'), so nothing is rounded that would not be rounded at the end.
@@ -299,7 +308,7 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
         // all of this thread's pieces are requested before the first is turned (they wait in the registers of the sum): four
         // loads in flight at a time kept the 12 products of 768 x 3072 with an addition at 209 us, all of them take 164
 #pragma unroll
-        for (int q = 0; q < HALF / 16; ++q) {
+        for (int q = 0; q < COLS / 16; ++q) {
           const int n = tn * BN + col0 + 16 * q + sc;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -319,33 +328,33 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
           }
         }
 #pragma unroll
-        for (int q = 0; q < HALF / 16; ++q) {   // from rows of four lanes to a row per lane
+        for (int q = 0; q < COLS / 16; ++q) {   // from rows of four lanes to a row per lane
 #pragma unroll
           for (int i = 0; i < 4; ++i)
-            st4(stage + (sr + 8 * i) * NF_OUT_PITCH + sc, make_float4(run[16 * q + 4 * i], run[16 * q + 4 * i + 1], run[16 * q + 4 * i + 2], run[16 * q + 4 * i + 3]));
+            st4(nf_out(stage, sr + 8 * i, lane & 3), make_float4(run[16 * q + 4 * i], run[16 * q + 4 * i + 1], run[16 * q + 4 * i + 2], run[16 * q + 4 * i + 3]));
           __syncwarp();
 #pragma unroll
           for (int h = 0; h < 4; ++h) {
-            const float4 d = ld4(stage + lane * NF_OUT_PITCH + 4 * h);
+            const float4 d = ld4(nf_out(stage, lane, h));
             run[16 * q + 4 * h] = f * d.x; run[16 * q + 4 * h + 1] = f * d.y; run[16 * q + 4 * h + 2] = f * d.z; run[16 * q + 4 * h + 3] = f * d.w;
           }
           __syncwarp();
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < HALF; ++j) run[j] = 0.f;
+        for (int j = 0; j < COLS; ++j) run[j] = 0.f;
       }
       for (int c = 0; c < n_chunks; ++c, ++cc) {
         if (!ns_wait(&sm.acc_ready[cc & 1], (uint32_t)((cc >> 1) & 1), &sm.abort)) { dead = true; break; }
         tc_fence_after();
         const uint32_t t_acc = t_lane + (uint32_t)(cc & 1) * 256;
 #pragma unroll
-        for (int q = 0; q < HALF / 32; ++q) {
-          uint32_t v[32];
-          tc_ld32(t_acc + 32 * q, v);
+        for (int q = 0; q < COLS / 16; ++q) {
+          uint32_t v[16];
+          nf_ld16(t_acc + 16 * q, v);
           tc_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) run[32 * q + j] += __uint_as_float(v[j]);
+          for (int j = 0; j < 16; ++j) run[16 * q + j] += __uint_as_float(v[j]);
         }
         tc_fence_before();
         __syncwarp();
@@ -360,12 +369,12 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
       const long long planeP = g.planeP;
       const bool cvec = (ldc & 3) == 0;
 #pragma unroll
-      for (int q = 0; q < HALF / 16; ++q) {
+      for (int q = 0; q < COLS / 16; ++q) {
         const int n0 = tn * BN + col0 + 16 * q;
         if (n0 < N && m0 < M && (!sym || n0 + 15 >= m0)) {   // the same for the whole warp
 #pragma unroll
           for (int h = 0; h < 4; ++h)
-            st4(stage + lane * NF_OUT_PITCH + 4 * h, make_float4(alpha * run[16 * q + 4 * h], alpha * run[16 * q + 4 * h + 1],
+            st4(nf_out(stage, lane, h), make_float4(alpha * run[16 * q + 4 * h], alpha * run[16 * q + 4 * h + 1],
                                                                  alpha * run[16 * q + 4 * h + 2], alpha * run[16 * q + 4 * h + 3]));
           __syncwarp();
           const int n = n0 + sc;
@@ -373,7 +382,7 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
           for (int i = 0; i < 4; ++i) {
             const int rr = sr + 8 * i, m = m0 + rr;
             if (m < M && n < N && (!sym || n + 3 >= m)) {
-              float4 o = ld4(stage + rr * NF_OUT_PITCH + sc);
+              float4 o = ld4(nf_out(stage, rr, lane & 3));
               float v[4] = {o.x, o.y, o.z, o.w};
               if (C) {
                 float* crow = C + (long long)m * ldc + n;
