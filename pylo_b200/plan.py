@@ -382,8 +382,10 @@ class LoPlan:
         slow["tensor"] = np.asarray(slow_units, dtype=np.int32)[slow["tensor"]] if len(slow) else slow["tensor"]
         self.tiles_slow = DeviceTable(slow, self.device)
         self.n_tiles_slow = len(slow)
-        #: no launch for phase B2: of small units phase P adds the tile partials up, for VeLO the LSTM's input kernel does
-        self.sum_tiles = family == L.FAM_VELO or max((k for _, k in ranges), default=0) <= 48
+        #: no launch for phase B2: of small units phase P adds the tile partials up, for VeLO the LSTM's input kernel does.
+        #: Every item of phase P repeats its unit's sum: about a hundred tiles are read in the time that a launch takes
+        #: (AdafacLO on a 118 K perceptron, 98 tiles: 39.6 -> 38.0 us per step)
+        self.sum_tiles = family == L.FAM_VELO or max((k for _, k in ranges), default=0) <= 112
         # The state sweep's ring of bulk copies leaves little L1 cache to the units that are not FAST2D and keeps the launches
         # around it apart, so it has to have enough to do: from 64 M elements on (VeLO on 100 M: 1615 -> 1580 us per step, on
         # 17 M: 341 -> 351; AdafacLO on 25 M: 837 -> 851, on 86 M even), nearly all of them FAST2D.
