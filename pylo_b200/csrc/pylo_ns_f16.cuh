@@ -46,7 +46,7 @@
 // for a tile of 128 x 256 (64 instead of 96 KB per 64 terms; at that rate L2 is what binds), and a third stage fits.
 template <int BN, bool PAIR>
 struct NfSmem {   // per stage: A hi, A lo (128 x 64 each), B hi, B lo (BN x 64 each, of a pair one half)
-  static constexpr int STAGES = PAIR ? 3 : 2;
+  static constexpr int STAGES = PAIR || BN == 128 ? 3 : 2;   // of 64 or 96 KB
   static constexpr int BROWS = PAIR ? BN / 2 : BN;
   unsigned char st[STAGES][2 * (NF_BM / 64) * NF_BOX + 2 * (BROWS / 64) * NF_BOX];
   float out[NF_EPI_WARPS][32 * 16];   // per epilogue warp: 32 rows x 16 columns on their way out
