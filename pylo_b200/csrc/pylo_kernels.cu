@@ -276,6 +276,11 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   return r;
 }
 // all threads of all CTAs of the cluster; orders shared, distributed shared and global memory accesses
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t n;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  return n;
+}
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -2025,19 +2030,32 @@ struct PlainLaunches {
 // launch of its thread made plainly.
 static thread_local bool t_plain_next = false;
 template <class... P, class... A>
-static void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+static void launch_clusters(void (*kernel)(P...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (!t_plain_launches && !t_plain_next) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  t_plain_next = false;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = t_plain_launches || t_plain_next ? 0 : 1;
-  t_plain_next = false;
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+static void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  launch_clusters(kernel, grid, block, 0, smem, stream, static_cast<A&&>(args)...);
 }
 
 // Opt a kernel in to more than 48 KB of dynamic shared memory, once per device (the attribute belongs to the
@@ -2071,28 +2089,36 @@ static long long ns_deal(nf_group& grp) {
   grp.tiles = (int)tiles;
   return tiles;
 }
-template <class Smem, class K>
-static int ns_launch(K kernel, nf_group& grp, int ctas, int* status, cudaStream_t s) {
+template <class Smem, void (*kernel)(nf_group, int*)>
+static int ns_launch(nf_group& grp, int ctas, int* status, cudaStream_t s, int cluster = 0) {
   static bool configured[PYLO_MAX_DEVICES] = {};
   constexpr int smem = (int)sizeof(Smem) + 1024;  // room to start the stages on a 1024-byte boundary
   if (int rc = allow_dynamic_smem(kernel, smem, configured)) return rc;
-  launch(kernel, ctas, NF_THREADS, smem, s, grp, status);
+  launch_clusters(kernel, ctas, NF_THREADS, cluster, smem, s, grp, status);
   return launch_status();
 }
 // The tile by what fills the GPU: a launch is as long as the SM with the most tiles, and a pair's tile is worth it from about
-// one per pair of SMs on; below one per SM, half as wide ones.
+// one per pair of SMs on; below one per SM, half as wide ones, the longest contractions split.
 static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
   const int sms = sm_count();
   long long tiles = ns_deal<256, 256>(grp);
   if (tiles > 0x3fffffff) return -1;
   if (tiles * 8 >= sms / 2 * 7) {
     const int ctas = (int)(2 * tiles < sms ? 2 * tiles : sms & ~1);
-    return ns_launch<NfSmem<256, true>>(k_gemm_f16x2_pair, grp, ctas, status, s);
+    return ns_launch<NfSmem<256, true>, k_gemm_f16x2_pair>(grp, ctas, status, s);
   }
   tiles = ns_deal<NF_BM, 256>(grp);
-  if (tiles >= sms) return ns_launch<NfSmem<256, false>>(k_gemm_f16x2<256>, grp, sms, status, s);
+  if (tiles >= sms) return ns_launch<NfSmem<256, false>, k_gemm_f16x2<256>>(grp, sms, status, s);
   tiles = ns_deal<NF_BM, 128>(grp);
-  return ns_launch<NfSmem<128, false>>(k_gemm_f16x2<128>, grp, (int)(tiles < sms ? tiles : sms), status, s);
+  // An SM fetches a K block of 64 in half a microsecond or more, so a few tiles with a long contraction are shared by clusters
+  // of CTAs: from eight blocks each on (below, bringing the sums together costs what is gained: 197 x 768, 12 blocks, 171 us
+  // per chain unsplit, 174 in two), as far as three quarters of the SMs go (1001 x 1433 in 36 clusters of four found no room
+  // for all of them at once: 342 -> 446).  128 x 3000: 293 -> 194 us, 768 x 2304: 308 -> 259, 10 x 3000: 215 -> 140.
+  int blocks = 0, split = 1;
+  for (int k = 0; k < grp.n; ++k) blocks = max(blocks, (grp.p[k].g.K + NF_BK - 1) / NF_BK);
+  while (split < 8 && blocks >= 16 * split && tiles * 2 * split <= sms * 3 / 4) split *= 2;
+  if (split > 1) return ns_launch<NfSmem<128, false>, k_gemm_f16x2_split>(grp, (int)tiles * split, status, s, split);
+  return ns_launch<NfSmem<128, false>, k_gemm_f16x2<128>>(grp, (int)(tiles < sms ? tiles : sms), status, s);
 }
 
 template <int FAM>

@@ -50,7 +50,7 @@ struct NfSmem {   // per stage: A hi, A lo (128 x 64 each), B hi, B lo (BN x 64 
   static constexpr int BROWS = PAIR ? BN / 2 : BN;
   unsigned char st[STAGES][2 * (NF_BM / 64) * NF_BOX + 2 * (BROWS / 64) * NF_BOX];
   float out[NF_EPI_WARPS][32 * 16];   // per epilogue warp: 32 rows x 16 columns on their way out
-  uint64_t full[STAGES], empty[STAGES], acc_ready[2], acc_free[2];
+  uint64_t full[STAGES], empty[STAGES], acc_ready[2], acc_free[2], parts;
   uint32_t tmem_base;
   volatile int abort;
 };
@@ -149,7 +149,9 @@ __device__ __forceinline__ void nf_tile_coords(int r, int M, int N, int symmetri
   tm = 0; tn = 0;
 }
 
-template <int BN, bool PAIR>
+// SPLIT: the CTAs of a cluster share one tile, each with its part of the contraction; the first adds their sums up through
+// distributed shared memory, in rank order, and carries on alone.  One tile per cluster.
+template <int BN, bool PAIR, bool SPLIT>
 __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restrict__ status) {
   extern __shared__ unsigned char nf_raw[];
   using Smem = NfSmem<BN, PAIR>;
@@ -160,9 +162,11 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
   // descriptors in uniform registers
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int rank = PAIR ? (int)cluster_rank() : 0;
+  const int part = SPLIT ? (int)cluster_rank() : 0, parts = SPLIT ? (int)cluster_size() : 1;
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(&sm.acc_ready[s], 1); mbar_init(&sm.acc_free[s], (PAIR ? 2 : 1) * NF_EPI_WARPS); }
+    if constexpr (SPLIT) mbar_init(&sm.parts, (parts - 1) * NF_EPI_WARPS);
     sm.abort = 0;
   }
   if (tid < 2 * grp.n) {   // the tensor maps' first use would wait for them
@@ -181,11 +185,11 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync();   // the other CTA's barriers exist
+  if constexpr (PAIR || SPLIT) cluster_sync();   // the other CTAs' barriers exist
   tc_fence_after();
   pdl_begin();
   const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);   // two accumulators of 256 columns
-  const int n_tiles = grp.tiles, first_tile = PAIR ? blockIdx.x >> 1 : blockIdx.x, tile_step = PAIR ? gridDim.x >> 1 : gridDim.x;
+  const int n_tiles = grp.tiles, ctas = PAIR ? 2 : parts, first_tile = blockIdx.x / ctas, tile_step = gridDim.x / ctas;
   // the product a tile belongs to, and its place there
   auto locate = [&](int tile, int& b, int& tm, int& tn) -> const nf_problem& {
     int k = 0;
@@ -197,6 +201,13 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
     return grp.p[k];
   };
 
+  // the K blocks of a tile that are this CTA's
+  auto blocks = [&](const nf_args& g, int& kb0, int& kb1) {
+    const int n_kb = (g.K + NF_BK - 1) / NF_BK, per = SPLIT ? (n_kb + parts - 1) / parts : n_kb;
+    kb0 = SPLIT ? min(part * per, n_kb) : 0;
+    kb1 = SPLIT ? min(kb0 + per, n_kb) : n_kb;
+  };
+
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA
     if (elect_one()) {
@@ -206,8 +217,10 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
       for (int tile = first_tile; tile < n_tiles && !dead && !sm.abort; tile += tile_step) {
         int b, tm, tn;
         const nf_problem& q = locate(tile, b, tm, tn);
-        const int a_mn = q.g.a_mn, b_mn = q.g.b_mn, n_kb = (q.g.K + NF_BK - 1) / NF_BK;
-        for (int kb = 0; kb < n_kb; ++kb, ++kbc) {
+        const int a_mn = q.g.a_mn, b_mn = q.g.b_mn;
+        int kb0, kb1;
+        blocks(q.g, kb0, kb1);
+        for (int kb = kb0; kb < kb1; ++kb, ++kbc) {
           const int s = (int)(kbc % STAGES);
           const long long use = kbc / STAGES;
           if (use > 0 && !ns_wait(&sm.empty[s], (uint32_t)((use - 1) & 1), &sm.abort)) { dead = true; break; }
@@ -254,11 +267,13 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
       for (int tile = first_tile; tile < n_tiles && !dead && !sm.abort; tile += tile_step) {
         int b, tm, tn;
         const nf_problem& q = locate(tile, b, tm, tn);
-        const int a_mn = q.g.a_mn, b_mn = q.g.b_mn, n_kb = (q.g.K + NF_BK - 1) / NF_BK;
+        const int a_mn = q.g.a_mn, b_mn = q.g.b_mn;
+        int kb0, kb1;
+        blocks(q.g, kb0, kb1);
         const uint32_t idesc = nf_idesc(TILE_M, BN, a_mn, b_mn);
         const uint64_t a_step = (a_mn ? 2048 : 32) >> 4, b_step = (b_mn ? 2048 : 32) >> 4;   // 16 terms further along K
-        for (int kb = 0; kb < n_kb; ++kb, ++kbc) {
-          const int in_chunk = kb % NF_CHUNK_BLOCKS;
+        for (int kb = kb0; kb < kb1; ++kb, ++kbc) {
+          const int in_chunk = (kb - kb0) % NF_CHUNK_BLOCKS;
           const uint32_t acc = tmem + (uint32_t)(cc & 1) * 256;
           if (in_chunk == 0 && cc >= 2) {   // this accumulator's previous chunk must have been added up
             if (!ns_wait(&sm.acc_free[cc & 1], (uint32_t)(((cc >> 1) - 1) & 1), &sm.abort)) { dead = true; break; }
@@ -277,7 +292,7 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
 #pragma unroll
           for (int ks = 0; ks < NF_BK / 16; ++ks) nf_mma<PAIR>(acc, ah + ks * a_step, bh + ks * b_step, idesc, 1u);
           nf_commit<PAIR>(&sm.empty[s]);
-          if (in_chunk == NF_CHUNK_BLOCKS - 1 || kb == n_kb - 1) { nf_commit<PAIR>(&sm.acc_ready[cc & 1]); ++cc; }
+          if (in_chunk == NF_CHUNK_BLOCKS - 1 || kb == kb1 - 1) { nf_commit<PAIR>(&sm.acc_ready[cc & 1]); ++cc; }
         }
       }
     }
@@ -294,12 +309,14 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
     for (int tile = first_tile; tile < n_tiles && !dead && !sm.abort; tile += tile_step) {
       int b, tm, tn;
       const nf_args& g = locate(tile, b, tm, tn).g;
-      const int n_kb = (g.K + NF_BK - 1) / NF_BK, n_chunks = (n_kb + NF_CHUNK_BLOCKS - 1) / NF_CHUNK_BLOCKS;
+      int kb0, kb1;
+      blocks(g, kb0, kb1);
+      const int n_chunks = (kb1 - kb0 + NF_CHUNK_BLOCKS - 1) / NF_CHUNK_BLOCKS;
       const int M = g.M, N = g.N, ldc = g.ldc, ldd = g.ldd, ldp = g.ldp, sym = g.symmetric;
       const int m0 = tm * TILE_M + rank * NF_BM + quarter * 32;
       const float alpha = g.alpha, scale = g.scale;
       float run[COLS];
-      if (g.D) {
+      if (g.D && part == 0) {
         // beta D / alpha is what the sum starts from: read while the first products run.  alpha is a power of two where D is
         // large (x'), so nothing is rounded that would not be rounded at the end.
         const float f = (g.d_scale ? g.beta * g.d_scale[b] : g.beta) / alpha;
@@ -364,6 +381,28 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
         }
       }
       if (dead) break;
+      if constexpr (SPLIT) {
+        // the stages are free: this CTA's products are done.  A thread's sums, four floats of a warp's lanes side by side
+        float4* const box = reinterpret_cast<float4*>(sm.st) + (warp - 2) * (COLS / 4) * 32 + lane;
+        if (part > 0) {
+#pragma unroll
+          for (int h = 0; h < COLS / 4; ++h) box[32 * h] = make_float4(run[4 * h], run[4 * h + 1], run[4 * h + 2], run[4 * h + 3]);
+          __syncwarp();
+          if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(nf_at_rank(&sm.parts, 0)) : "memory");
+          continue;
+        }
+        if (!ns_wait(&sm.parts, 0, &sm.abort)) break;
+        asm volatile("fence.acq_rel.cluster;" ::: "memory");
+        for (int r = 1; r < parts; ++r) {
+          const uint32_t src = nf_at_rank(box, r);
+#pragma unroll
+          for (int h = 0; h < COLS / 4; ++h) {
+            float4 v;
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(src + 512 * h) : "memory");
+            run[4 * h] += v.x; run[4 * h + 1] += v.y; run[4 * h + 2] += v.z; run[4 * h + 3] += v.w;
+          }
+        }
+      }
       float* const C = g.C ? g.C + (long long)b * g.sC : nullptr;
       __half* const P = g.P ? g.P + (long long)b * g.sP : nullptr;
       const long long planeP = g.planeP;
@@ -433,7 +472,7 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync();   // neither CTA leaves while the other's products may read its shared memory
+  if constexpr (PAIR || SPLIT) cluster_sync();   // no CTA leaves while another may read its shared memory
   if (tid == 0 && sm.abort && status) atomicOr(status, 4);
   if (warp == 1) {
     if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
@@ -443,11 +482,15 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
 
 // 256 x 256 on pairs of SMs where that fills the GPU, else 128 x 256, else 128 x 128 on one SM
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2_pair(const __grid_constant__ nf_group grp, int* __restrict__ status) {
-  nf_gemm_body<256, true>(grp, status);
+  nf_gemm_body<256, true, false>(grp, status);
 }
 template <int BN>
 __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_constant__ nf_group grp, int* __restrict__ status) {
-  nf_gemm_body<BN, false>(grp, status);
+  nf_gemm_body<BN, false, false>(grp, status);
+}
+// few tiles with a long contraction: launched in clusters of 2, 4 or 8
+__global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2_split(const __grid_constant__ nf_group grp, int* __restrict__ status) {
+  nf_gemm_body<128, false, true>(grp, status);
 }
 
 // ------------------------------------------------------------------------------------------------
