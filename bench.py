@@ -258,7 +258,7 @@ def config_of(args, shapes, n_gpus):
         "params": W.total_params(shapes), "grads": f"randn*{gscale} ({gkind}), one buffer per distinct shape",
         "orthogonalize": (not args.no_orthogonalize) if "celo2" in args.optimizer else None,
         "newton_schulz": (None if "celo2" not in args.optimizer or args.no_orthogonalize else
-                          ("k_gemm_tn_3xtf32 (this library, tcgen05)" if args.ns_precision == "3xtf32" else "torch.matmul fp32 (library)")),
+                          ("k_gemm_f16x2 (this library, tcgen05, fp16 planes of split fp32)" if args.ns_precision == "3xtf32" else "torch.matmul fp32 (library)")),
         "mlp_precision": args.mlp_precision if args.optimizer in ("adafaclo", "elo") else None,
         "cache": "inputs larger than L2 (no flush needed)" if W.total_params(shapes) * 24 / max(n_gpus, 1) > 2e9
                  else "L2 flushed between steps by writing a 512 MiB buffer",
