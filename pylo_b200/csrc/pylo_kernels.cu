@@ -1552,11 +1552,14 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
 // ================================================================================================
 // CELO2 tail: second-moment normaliser over a matrix, then the parameter update
 // ================================================================================================
+// From the last tile to the first: what the sweep before wrote last is still in L2, and k_post_apply, which goes the other way,
+// finds the first steps there.
 __global__ void __launch_bounds__(NT) k_post_sums(const pylo_post_item* __restrict__ items,
                                                   const pylo_tile* __restrict__ tiles, int n_tiles) {
   pdl_begin();
   __shared__ float s_red[40];
-  for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+  for (int tt = blockIdx.x; tt < n_tiles; tt += gridDim.x) {
+    const int t = n_tiles - 1 - tt;
     const pylo_tile tl = tiles[t];
     const pylo_post_item& it = items[tl.tensor];
     const float* s = it.step + tl.start;
