@@ -2100,8 +2100,8 @@ static int ns_launch(nf_group& grp, int ctas, int* status, cudaStream_t s, int c
   launch_clusters(kernel, ctas, NF_THREADS, cluster, smem, s, grp, status);
   return launch_status();
 }
-// The tile by what fills the GPU: a launch is as long as the SM with the most tiles, and a pair's tile is worth it from about
-// one per pair of SMs on; below one per SM, half as wide ones, the longest contractions split.
+// The tile by what fills the GPU: a launch is as long as the SM with the most tiles, and a pair's tile of 256 x 256 is worth it
+// from about one per pair of SMs on; below, tiles of 128 x 128 on single SMs, the longest contractions split.
 static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
   const int sms = sm_count();
   long long tiles = ns_deal<256, 256>(grp);
@@ -2110,8 +2110,6 @@ static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
     const int ctas = (int)(2 * tiles < sms ? 2 * tiles : sms & ~1);
     return ns_launch<NfSmem<256, true>, k_gemm_f16x2_pair>(grp, ctas, status, s);
   }
-  tiles = ns_deal<NF_BM, 256>(grp);
-  if (tiles >= sms) return ns_launch<NfSmem<256, false>, k_gemm_f16x2<256>>(grp, sms, status, s);
   tiles = ns_deal<NF_BM, 128>(grp);
   // An SM fetches a K block of 64 in half a microsecond or more, so a few tiles with a long contraction are shared by clusters
   // of CTAs: from eight blocks each on (below, bringing the sums together costs what is gained: 197 x 768, 12 blocks, 171 us
@@ -2121,7 +2119,7 @@ static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
   for (int k = 0; k < grp.n; ++k) blocks = max(blocks, (grp.p[k].g.K + NF_BK - 1) / NF_BK);
   while (split < 8 && blocks >= 16 * split && tiles * 2 * split <= sms * 3 / 4) split *= 2;
   if (split > 1) return ns_launch<NfSmem<128, false>, k_gemm_f16x2_split>(grp, (int)tiles * split, status, s, split);
-  return ns_launch<NfSmem<128, false>, k_gemm_f16x2<128>>(grp, (int)(tiles < sms ? tiles : sms), status, s);
+  return ns_launch<NfSmem<128, false>, k_gemm_f16x2>(grp, (int)(tiles < sms ? tiles : sms), status, s);
 }
 
 template <int FAM>

@@ -27,7 +27,8 @@
 // shared memory, 16 columns at a time, so that a warp's loads and stores cover whole sectors of four rows (straight from
 // the accumulator layout, a row per lane, they touch 32 lines each and bound every product with K < 1000).
 //
-// What binds it: the tensor pipe (12 products of 128 cycles per 96 KB stage) and tile quantisation.
+// What binds it: the tensor pipe (a pair: 12 products of 128 cycles per 64 KB stage), tile quantisation, and below K = 1000 a
+// tile's way out.
 #pragma once
 
 #include <cuda.h>
@@ -46,7 +47,7 @@
 // for a tile of 128 x 256 (64 instead of 96 KB per 64 terms; at that rate L2 is what binds), and a third stage fits.
 template <int BN, bool PAIR>
 struct NfSmem {   // per stage: A hi, A lo (128 x 64 each), B hi, B lo (BN x 64 each, of a pair one half)
-  static constexpr int STAGES = PAIR || BN == 128 ? 3 : 2;   // of 64 or 96 KB
+  static constexpr int STAGES = 3;   // of 64 KB
   static constexpr int BROWS = PAIR ? BN / 2 : BN;
   unsigned char st[STAGES][2 * (NF_BM / 64) * NF_BOX + 2 * (BROWS / 64) * NF_BOX];
   float out[NF_EPI_WARPS][32 * 16];   // per epilogue warp: 32 rows x 16 columns on their way out
@@ -480,13 +481,12 @@ __device__ __forceinline__ void nf_gemm_body(const nf_group& grp, int* __restric
   }
 }
 
-// 256 x 256 on pairs of SMs where that fills the GPU, else 128 x 256, else 128 x 128 on one SM
+// 256 x 256 on pairs of SMs where that fills the GPU, else 128 x 128 on one SM
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2_pair(const __grid_constant__ nf_group grp, int* __restrict__ status) {
   nf_gemm_body<256, true, false>(grp, status);
 }
-template <int BN>
 __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2(const __grid_constant__ nf_group grp, int* __restrict__ status) {
-  nf_gemm_body<BN, false, false>(grp, status);
+  nf_gemm_body<128, false, false>(grp, status);
 }
 // few tiles with a long contraction: launched in clusters of 2, 4 or 8
 __global__ void __launch_bounds__(NF_THREADS, 1) k_gemm_f16x2_split(const __grid_constant__ nf_group grp, int* __restrict__ status) {
