@@ -2578,7 +2578,9 @@ int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctil
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
     case PYLO_FAM_CELO2: launch(k_apply_packed<PYLO_FAM_CELO2>, grid_for(n_ctiles, PK_CTAS_CELO2), NT, 0, s, descs, ctiles, n_ctiles, *prm); break;
-    case PYLO_FAM_VELO: launch(k_apply_packed<PYLO_FAM_VELO>, grid_for(n_ctiles, PK_CTAS_VELO), NT, 0, s, descs, ctiles, n_ctiles, *prm); break;
+    // four times the CTAs that fit: an SM that is done takes the next (17 M parameters: 341 -> 327 us per step, 67 M: 1104 ->
+    // 1091); CELO2's larger network is loaded by every CTA, which costs more than that gives
+    case PYLO_FAM_VELO: launch(k_apply_packed<PYLO_FAM_VELO>, grid_for(n_ctiles, 4 * PK_CTAS_VELO), NT, 0, s, descs, ctiles, n_ctiles, *prm); break;
     default: return -2;
   }
   return launch_status();
