@@ -2126,9 +2126,7 @@ template <int FAM>
 static int state_moments_launch(const pylo_tensor_desc* descs, const pylo_tile* tiles, int n_tiles, int reverse,
                                 const pylo_step_params& prm, cudaStream_t s) {
   if (!prm.bulk_copies) {
-    // more CTAs than fit at once: an SM that is done takes the next one, instead of a fixed share of the tiles each
-    // (AdafacLO on 8.4 M parameters 314 -> 304 us per step, VeLO on 17 M unaligned ones 435 -> 415)
-    launch(k_state_moments<FAM, false>, grid_for(n_tiles, 16), NT, 0, s, descs, tiles, n_tiles, reverse, prm);
+    launch(k_state_moments<FAM, false>, grid_for(n_tiles, 4), NT, 0, s, descs, tiles, n_tiles, reverse, prm);
     return 0;
   }
   static bool configured[PYLO_MAX_DEVICES] = {};
