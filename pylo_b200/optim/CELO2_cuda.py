@@ -29,7 +29,7 @@ from torch.optim import Optimizer
 
 from .. import _lib as L
 from ..models.CELO2_MLP import CELO2MLP
-from ..plan import (GradNorm, LoPlan, LoTensor, current_stream_ptr, grad_pointers, one_minus, tile_elems,
+from ..plan import (GradNorm, LoPlan, LoTensor, current_stream_ptr, fp32_gradient, grad_pointers, one_minus, tile_elems,
                     with_gradients)
 from ._common import (ItemPlan, factored_dims_argsort, newton_schulz, newton_schulz_bounded, newton_schulz_buffers,
                       newton_schulz_native, newton_schulz_tc, optimizer_step, require_cuda_param)
@@ -322,9 +322,9 @@ class _Celo2Family(Optimizer):
         it = adam.items
         ptrs = grad_pointers(grads)
         copies = []
-        if ptrs is None:   # a gradient that is not contiguous is copied, which gives it a new address on every step
-            grads = [g if g.is_contiguous() else g.contiguous() for g in grads]
-            copies, ptrs = grads, [g.data_ptr() for g in grads]
+        if ptrs is None:   # a gradient that is not contiguous fp32 is copied, which gives it a new address on every step
+            copies = [fp32_gradient(g) for g in grads]
+            ptrs = [g.data_ptr() for g in copies]
         if self._shared_adam:
             b1, b2, eps = self._b1_shared, self._b2_shared, 1e-8
             ts = [group["step"]]

@@ -435,7 +435,7 @@ class LoPlan:
             at = np.zeros(self.n_tensors, dtype=np.uint64)
             for i, g in enumerate(grads):
                 if not (g.is_cuda and g.dtype == torch.float32 and g.is_contiguous() and g.data_ptr() % 16 == 0):
-                    g = g.to(torch.float32).contiguous().clone()
+                    g = g.detach().to(torch.float32).contiguous().clone()
                     self._keepalive.append(g)
                     self._grad_ptrs = None   # the copy is this step's: look again at the next
                 at[i] = g.data_ptr()
@@ -600,11 +600,11 @@ class GradNorm:
             self._grad_ptrs = ptrs
             self._keepalive = []
             for i, g in enumerate(grads):
-                if not (g.dtype == torch.float32 and g.is_contiguous()):
-                    g = g.to(torch.float32).contiguous()
-                    self._keepalive.append(g)
+                plain = fp32_gradient(g)
+                if plain is not g:
+                    self._keepalive.append(plain)
                     self._grad_ptrs = None
-                self.items["g"][i] = g.data_ptr()
+                self.items["g"][i] = plain.data_ptr()
             self.table.upload()
         L.check(L.lib.pylo_b200_grad_sumsq(self.table.ptr, self.tiles.ptr, self.n_tiles, self.scratch.data_ptr(),
                                            self.out.data_ptr(), stream), "grad_sumsq")
@@ -621,14 +621,21 @@ def with_gradients(params):
 
 
 def grad_pointers(grads: Sequence[torch.Tensor]):
-    """The gradients' addresses, or None where one of them is not contiguous and has to be looked at."""
+    """The gradients' addresses, or None where one of them is not contiguous fp32 and has to be looked at (an fp32 parameter
+    may have a gradient of another type: ``p.grad_dtype``).  Looked at on every step: an address says nothing about the type
+    of what lies there now."""
     try:
         ptrs = [g.data_ptr() for g in grads]
     except RuntimeError:
         if any(g.is_sparse for g in grads):
             raise RuntimeError("Sparse gradients not supported") from None
         raise
-    return ptrs if all([g.is_contiguous() for g in grads]) else None
+    return ptrs if all([g.dtype is torch.float32 and g.is_contiguous() for g in grads]) else None
+
+
+def fp32_gradient(g: torch.Tensor) -> torch.Tensor:
+    """``g`` as contiguous fp32: itself, or a copy."""
+    return g if g.dtype is torch.float32 and g.is_contiguous() else g.detach().to(torch.float32).contiguous()
 
 
 def current_stream_ptr() -> int:

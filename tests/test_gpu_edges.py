@@ -187,3 +187,28 @@ def test_adamw_tensors_of_any_length(cls):
         ora.step(ref, grads)
     res = CU.compare({3: [p.detach().cpu() for p in params]}, {3: ref}, cases.init_values(case))
     assert res[3][0] < 1e-5 and res[3][1] < 2e-5, res
+
+
+@pytest.mark.parametrize("family", ["adafaclo", "elo", "celo2", "elo_celo2", "velo"])
+def test_gradients_of_another_type_are_converted(family):
+    """bf16 gradients of fp32 parameters (``grad_dtype``), through every path of a step (the norm, the sweeps, AdamW), give
+    what the same values in fp32 give: also where a bf16 gradient comes to lie at an address that held an fp32 one."""
+    shapes = [(40, 24), (24,), (300, 260), (1027,)]
+    runs = []
+    for half in (False, True):
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(dict(shapes=shapes, init_seed=91, init_scale=0.1))]
+        pool = [torch.zeros(p.shape, device="cuda") for p in params]
+        opt = _make(family, params)
+        for t in (1, 2, 3):
+            for k, (p, g) in enumerate(zip(params, cases.grads_at(dict(grad_seed=92, grad_scale=0.3, shapes=shapes), t))):
+                g = g.cuda().to(torch.bfloat16)
+                if half and t > 1 and k != 0:
+                    p.grad_dtype = torch.bfloat16
+                    p.grad = pool[k].view(-1).view(torch.bfloat16)[:p.numel()].view(p.shape).copy_(g)
+                else:
+                    p.grad = pool[k].copy_(g)
+            _step(opt, family, t)
+            for p in params:
+                p.grad = None
+        runs.append([p.detach().clone() for p in params])
+    assert all(torch.equal(a, b) for a, b in zip(*runs))

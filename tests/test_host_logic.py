@@ -175,3 +175,18 @@ def test_a_rank_without_tensors_still_gets_a_param_group():
     ps = [torch.zeros(4), torch.zeros(8), torch.zeros(4)]
     groups = split_in_groups(ps, 2)
     assert [len(g["params"]) for g in groups] == [2, 1]
+
+
+def test_gradients_of_another_type_are_not_taken_by_their_address():
+    """An fp32 parameter may have a bf16 gradient (``grad_dtype``); its address alone would be read as fp32, beyond its end."""
+    full, half = torch.arange(8.0), torch.arange(8.0).to(torch.bfloat16)
+    assert plan.grad_pointers([full, full]) == [full.data_ptr()] * 2
+    assert plan.grad_pointers([full, half]) is None
+    assert plan.grad_pointers([full.view(2, 4).t()]) is None
+    # the same address with another type in it: not what it was
+    assert plan.grad_pointers([full[:4].view(torch.int32)]) is None
+    assert plan.fp32_gradient(full) is full
+    got = plan.fp32_gradient(half)
+    assert got.dtype == torch.float32 and torch.equal(got, full)
+    strided = plan.fp32_gradient(full.view(2, 4).t())
+    assert strided.is_contiguous() and torch.equal(strided, full.view(2, 4).t())
