@@ -237,8 +237,8 @@ class AdafacLO_CUDA(_AdafacFamily):
                 continue
             wd, eps = float(group["weight_decay"]), group["eps"]
             prm = self._params_struct(None, 1 if wd > 0 else 0, 0, 1e-30 if eps is None else float(eps))
-            self._run_group(gi, plist, grads, prm, stream, lr=float(group["lr"]), wd=wd, exp_mult=self.exp_mult,
-                            step_mult=self.step_mult, clip_norm=0.0)
+            self._run_group(gi, plist, grads, prm, stream, lr=float(group["lr"]), wd=wd, exp_mult=float(self.exp_mult),
+                            step_mult=float(self.step_mult), clip_norm=0.0)
         return loss
 
 

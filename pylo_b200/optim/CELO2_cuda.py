@@ -31,7 +31,7 @@ from .. import _lib as L
 from ..models.CELO2_MLP import CELO2MLP
 from ..plan import (GradNorm, LoPlan, LoTensor, current_stream_ptr, fp32_gradient, grad_pointers, one_minus, tile_elems,
                     with_gradients)
-from ._common import (ItemPlan, factored_dims_argsort, newton_schulz, newton_schulz_bounded, newton_schulz_buffers,
+from ._common import (ItemPlan, factored_dims_argsort, group_floats, newton_schulz, newton_schulz_bounded, newton_schulz_buffers,
                       newton_schulz_native, newton_schulz_tc, optimizer_step, require_cuda_param)
 
 _IN, _HID = 30, 8
@@ -256,7 +256,7 @@ class _Celo2Family(Optimizer):
                 self.before_group(gi)
             prm = self._params_struct(group, gnorm_ptr)
             clip_norm = float(group["clip_norm"]) if group["clip_grad"] else 0.0
-            lr, wd = float(group["lr"]), group["weight_decay"]
+            lr, wd = group_floats(group, "lr", "weight_decay")
             if plan["lo"] is not None:
                 self._lo_step(group, plan, [g for g, lo in zip(grads, plan["in_lo"]) if lo], prm, clip_norm, lr, wd, stream)
             if plan["adam"] is not None:
@@ -268,7 +268,8 @@ class _Celo2Family(Optimizer):
 
     def _lo_step(self, group, plan, grads, prm, clip_norm, lr, wd, stream):
         lo: LoPlan = plan["lo"]
-        lo.set_hyper(lr=lr, wd=wd, clip_norm=clip_norm, exp_mult=group["exp_mult"])
+        exp_mult, rmsmult = group_floats(group, "exp_mult", "rmsmult")
+        lo.set_hyper(lr=lr, wd=wd, clip_norm=clip_norm, exp_mult=exp_mult)
         lo.refresh(grads)
         lo.run(prm, stream)
         post: ItemPlan = plan["post"]
@@ -277,11 +278,11 @@ class _Celo2Family(Optimizer):
             keep, steps = self._orthogonalise(plan, stream)
         else:
             steps = [k.data_ptr() for k in keep]
-        key = (steps, lr, wd, group["rmsmult"])
+        key = (steps, lr, wd, rmsmult)
         if key != plan["post_key"]:
             it = post.items
             it["step"][:] = np.array(steps, dtype=np.uint64)[post.owner_t] + post.owner_off
-            it["lr"][:], it["wd"][:], it["rmsmult"][:] = lr, wd, group["rmsmult"]
+            it["lr"][:], it["wd"][:], it["rmsmult"][:] = lr, wd, rmsmult
             post.upload()
             plan["post_key"] = key
         L.check(L.lib.pylo_b200_celo2_post_sums(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_sums")
@@ -334,7 +335,8 @@ class _Celo2Family(Optimizer):
                 st["adam_step"] += 1
             ts = [st["adam_step"] for st in plan["adam_states"]]
         same = min(ts) == max(ts)   # one step count: the bias corrections go with the launch, not through the table
-        key = (ptrs, group["adam_lr_mult"] * lr, group["adam_weight_decay"], clip_norm)
+        adam_lr_mult, adam_wd = group_floats(group, "adam_lr_mult", "adam_weight_decay")
+        key = (ptrs, adam_lr_mult * lr, adam_wd, clip_norm)
         if key != plan["adam_key"] or not same:
             it["g"][:] = ptrs
             it["lr"][:], it["wd"][:], it["clip_norm"][:] = key[1:]

@@ -192,6 +192,13 @@ def require_cuda_param(p: torch.Tensor, who: str):
         raise RuntimeError(f"{who}: parameters must be contiguous")
 
 
+def group_floats(group, *names):
+    """The values of some of a param group's entries as floats, to be compared with the next step's.
+
+    An entry may be a tensor that a scheduler changes in place: kept as it is, it would always equal itself."""
+    return tuple([float(group[name]) for name in names])
+
+
 def optimizer_step(step):
     """Decorator of an optimizer's ``step``: torch's own wrapper (profiler range, step hooks) and ``no_grad``, but only where
     something can see them.

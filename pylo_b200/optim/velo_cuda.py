@@ -30,7 +30,7 @@ from .. import _lib as L
 from ..models.VeLO_MLP import VeLOMLP
 from ..models.VeLO_RNN import VeLORNN
 from ..plan import LoPlan, LoTensor, current_stream_ptr, one_minus
-from ._common import factored_dims_velo, optimizer_step, require_cuda_param
+from ._common import factored_dims_velo, group_floats, optimizer_step, require_cuda_param
 
 
 def _decay_to_param(x):
@@ -255,7 +255,7 @@ class VeLO_CUDA(Optimizer):
             mine = [p for p in group["params"] if p.requires_grad]
             plist += mine
             counts.append(len(mine))
-            hyper.append((group["lr"], group["weight_decay"], group["exp_mult"], group["step_mult"]))
+            hyper.append(group_floats(group, "lr", "weight_decay", "exp_mult", "step_mult"))
         grads = [p.grad for p in plist]
         if any([g is None for g in grads]):
             raise RuntimeError("VeLO_CUDA: every parameter needs a gradient on every step "

@@ -212,3 +212,27 @@ def test_gradients_of_another_type_are_converted(family):
                 p.grad = None
         runs.append([p.detach().clone() for p in params])
     assert all(torch.equal(a, b) for a, b in zip(*runs))
+
+
+@pytest.mark.parametrize("family", ["adafaclo", "elo", "celo2", "elo_celo2", "velo"])
+def test_a_scheduled_tensor_learning_rate_is_followed(family):
+    """A tensor learning rate that a scheduler changes in place gives what the same float learning rates give."""
+    shapes = [(40, 24), (24,)]
+    runs = []
+    for tensor_lr in (False, True):
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(dict(shapes=shapes, init_seed=95, init_scale=0.1))]
+        opt = _make(family, params)
+        if tensor_lr:
+            for group in opt.param_groups:
+                group["lr"] = torch.tensor(0.5)
+        for t in (1, 2, 3):
+            for p, g in zip(params, cases.grads_at(dict(grad_seed=96, grad_scale=0.3, shapes=shapes), t)):
+                p.grad = g.cuda()
+            for group in opt.param_groups:
+                if tensor_lr:
+                    group["lr"].fill_(0.5 ** t)
+                else:
+                    group["lr"] = 0.5 ** t
+            _step(opt, family, t)
+        runs.append([p.detach().clone() for p in params])
+    assert all(torch.equal(a, b) for a, b in zip(*runs))

@@ -190,3 +190,20 @@ def test_gradients_of_another_type_are_not_taken_by_their_address():
     assert got.dtype == torch.float32 and torch.equal(got, full)
     strided = plan.fp32_gradient(full.view(2, 4).t())
     assert strided.is_contiguous() and torch.equal(strided, full.view(2, 4).t())
+
+
+def test_a_tensor_learning_rate_that_a_scheduler_changes_in_place_is_seen():
+    """torch's schedulers ``fill_`` a tensor learning rate: what a step keeps for comparison must be its value."""
+    from pylo_b200.optim._common import group_floats
+
+    p = torch.nn.Parameter(torch.zeros(3))
+    opt = torch.optim.SGD([p], lr=torch.tensor(0.5), weight_decay=0.1)
+    sched = torch.optim.lr_scheduler.ExponentialLR(opt, gamma=0.5)
+    group = opt.param_groups[0]
+    lr = group["lr"]
+    kept = group_floats(group, "lr", "weight_decay")
+    p.grad = torch.zeros(3)
+    opt.step()
+    sched.step()
+    assert group["lr"] is lr, "the scheduler changes the tensor in place"
+    assert kept == (0.5, 0.1) and group_floats(group, "lr", "weight_decay") == (0.25, 0.1)
