@@ -275,14 +275,25 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// all threads of all CTAs of the cluster; orders shared, distributed shared and global memory accesses
 __device__ __forceinline__ uint32_t cluster_size() {
   uint32_t n;
   asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
   return n;
 }
+// all threads of all CTAs of the cluster; orders shared, distributed shared and global memory accesses
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The same in two parts that order nothing: after cluster_wait() every CTA of the cluster is known to be running.  Until then
+// none may reach into another's shared memory.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void cluster_store(float* p, uint32_t rank, float v) {
   uint32_t a;
@@ -306,6 +317,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
     if (rank == 0 && tid < PYLO_STAT_STRIDE) d.closed[tid] = 0.f;
     return;
   }
+  cluster_arrive();   // waited for below, before the first store into another CTA
   const bool fast = d.mode == PYLO_MODE_FAST2D, r_is_a = d.r_is_a != 0;
   const int64_t La = d.La, Lb = d.Lb;
   const float inv_n_a = (float)d.Y, inv_n_b = (float)d.X;
@@ -386,6 +398,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
     if ((tid & 31) == 0) s_warp[tid >> 5][j] = v;
   }
   __syncthreads();
+  cluster_wait();
   if (tid < NS) {
     float v = 0.f;
     for (int w = 0; w < A2_NT / 32; ++w) v += s_warp[w][tid];

@@ -1,0 +1,35 @@
+"""Rules that the device code has to keep and that no run can show to be broken: checked on the source text."""
+
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "pylo_b200", "csrc")
+
+
+def functions():
+    """{name: body} of the device functions and kernels in the sources."""
+    out = {}
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+        text = re.sub(r"__(?:launch_bounds|cluster_dims)__\([^()]*\)", "", text)
+        for head in re.finditer(r"(?:__global__|__device__ __forceinline__)[^;{]*?(\w+)\s*\([^;{]*\)\s*\{", text):
+            depth, at = 1, head.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[at], 0)
+                at += 1
+            out[head.group(1)] = text[head.end():at]
+    return out
+
+
+def test_no_cta_reaches_into_another_before_it_is_known_to_run():
+    """Distributed shared memory may be accessed only once every CTA of the cluster has started (a cluster barrier)."""
+    bodies = functions()
+    assert {"k_factor_update", "nf_gemm_body"} <= set(bodies)
+    for name, body in bodies.items():
+        reach = re.search(r"\b(cluster_store|nf_at_rank)\(", body)
+        if name in ("cluster_store", "nf_at_rank") or not reach or "cluster_rank()" not in body:
+            continue
+        before = body[:reach.start()]
+        assert "cluster_sync();" in before or re.search(r"cluster_arrive\(\);.*cluster_wait\(\);", before, re.S), name
