@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define PYLO_B200_ABI_VERSION 11
+#define PYLO_B200_ABI_VERSION 12
 
 /* optimizer families (which feature set / network geometry a launch uses) */
 #define PYLO_FAM_ADAFAC 0 /* AdafacLO_CUDA, ELO_CUDA: 28+11 features, 39-32-32-2 */
@@ -150,8 +150,9 @@ typedef struct pylo_step_params {
   int32_t bulk_copies;    /* state_moments: 1 = FAST2D tiles come through a ring of bulk copies, for large models that consist
                              of them; 0 = all tiles are read into registers */
   int* status;            /* device int: state_moments ORs 8 in if a bounded wait for its own copies ran out (the step is
-                             then incomplete); may be NULL */
-  int* host_status;       /* the same in pinned host memory; may be NULL */
+                             then incomplete); the apply kernels that write parameters (ADAFAC, VELO) write none while it
+                             is not zero; may be NULL */
+  int* host_status;       /* a word of pinned host memory that both events are written to; may be NULL */
 } pylo_step_params;
 
 int pylo_b200_abi_version(void);
@@ -353,7 +354,10 @@ typedef struct pylo_post_item {
   float lr, wd, rmsmult, pad_;
 } pylo_post_item;
 int pylo_b200_celo2_post_sums(const pylo_post_item* items, const pylo_tile* tiles, int n_tiles, void* stream);
-int pylo_b200_celo2_post_apply(const pylo_post_item* items, const pylo_tile* tiles, int n_tiles, void* stream);
+/* status, host_status: as in pylo_step_params: no parameter is written while *status is not zero (the words that were given to
+ * state_moments and newton_schulz); may be NULL */
+int pylo_b200_celo2_post_apply(const pylo_post_item* items, const pylo_tile* tiles, int n_tiles, const int* status, int* host_status,
+                               void* stream);
 
 /* AdamW branch for 1-D / embedding tensors.
  * independent != 0: CELO2_cuda.py:234-253 (own exp_avg/exp_avg_sq, betas b1,b2, bias correction with step t);
@@ -387,7 +391,8 @@ typedef struct pylo_velo_rnn {
   const float* bank;                              /* [B][159] */
   float *h, *c;                                   /* [T][H] LSTM state, updated in place */
   float *x_in;                                    /* [T][30] */
-  float *pooled;                                  /* unused */
+  const int *status;                              /* device int: while it is not zero, h, c and the loss buffer are left as
+                                                     they are (tensor_features' input was incomplete); may be NULL */
   float *xmix;                                    /* workspace [T][H] */
   float *gates;                                   /* workspace [2][T][4H] */
   float *controls;                                /* workspace [T][B] */

@@ -17,7 +17,7 @@ TILE_ELEMS = 16384
 A_COLS = 1024
 PREP_TABLE = 2048  # table entries (rows x hidden units) per item of pylo_b200_prep_apply
 WFOLD_STRIDE = 2432
-ABI_VERSION = 11
+ABI_VERSION = 12
 
 FAM_ADAFAC, FAM_CELO2, FAM_VELO = 0, 1, 2
 MODE_FAST2D, MODE_GENERIC, MODE_VEC1D = 0, 1, 2
@@ -85,7 +85,7 @@ class NsDesc(C.Structure):
 class VeloRnn(C.Structure):
     _fields_ = [(name, C.c_void_p) for name in (
         "mix2_w", "mix2_b", "fmix_w", "fmix_b", "lstm_w", "lstm_b", "ctrl_w", "ctrl_b", "step_w", "step_b",
-        "bank", "h", "c", "x_in", "pooled", "xmix", "gates", "controls", "weights", "lr_mult")] + [
+        "bank", "h", "c", "x_in", "status", "xmix", "gates", "controls", "weights", "lr_mult")] + [
         ("T", C.c_int32), ("H", C.c_int32), ("B", C.c_int32), ("pad_", C.c_int32)]
 
 
@@ -140,7 +140,7 @@ def _load():
         "pylo_b200_newton_schulz_workspace": [i32, i32, i32, i32],
         "pylo_b200_newton_schulz": [C.POINTER(NsDesc), i32, vp, vp],
         "pylo_b200_celo2_post_sums": [vp, vp, i32, vp],
-        "pylo_b200_celo2_post_apply": [vp, vp, i32, vp],
+        "pylo_b200_celo2_post_apply": [vp, vp, i32, vp, vp, vp],
         "pylo_b200_adamw": [vp, vp, i32, i32] + [f32] * 7 + [C.POINTER(StepParams), vp],
         "pylo_b200_velo_tensor_features": [vp, i32, vp, i32, vp, f32, C.POINTER(VeloLoss), vp, vp],
         "pylo_b200_velo_rnn": [C.POINTER(VeloRnn), C.POINTER(VeloLoss), vp],

@@ -74,6 +74,14 @@ __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// The status word of a step: set by a kernel whose bounded wait ran out.  A kernel that writes parameters (or the LSTM's state)
+// and finds it set leaves them as they are, since its inputs are incomplete, and passes the word on to the host.  It is asked
+// for at the kernel's start and looked at behind the first barrier, where it has arrived with everything else.
+__device__ __forceinline__ int reported(const int* status) { return status ? *reinterpret_cast<const volatile int*>(status) : 0; }
+__device__ __forceinline__ void pass_on(int word, int* host_status) {
+  if (word && host_status && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<volatile int*>(host_status) = word;
+}
+
 // ----------------------------------------------------------------------------------------------
 // scalar helpers
 // ----------------------------------------------------------------------------------------------

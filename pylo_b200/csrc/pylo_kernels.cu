@@ -992,10 +992,15 @@ __global__ void __launch_bounds__(NT) k_apply(const pylo_tensor_desc* __restrict
     const pylo_tile tl = tiles[t];
     const pylo_tensor_desc& d = descs[tl.tensor];
     if (loaded != tl.tensor) {
+      const int word = FAM == PYLO_FAM_CELO2 ? 0 : reported(prm.status);   // CELO2's parameters are written by k_post_apply
       __syncthreads();
       for (int e = tid; e < L::SIZE; e += NT) s_w[e] = d.wfold[e];
       loaded = tl.tensor;
       __syncthreads();
+      if (word) {
+        pass_on(word, prm.host_status);
+        return;
+      }
     }
     const int64_t n = d.n, start = tl.start;
     const int cnt = tile_count(tl, n);
@@ -1130,6 +1135,9 @@ __global__ void __launch_bounds__(NT, CC_CTAS_PER_SM) k_apply_adafac_cols(const 
   extern __shared__ __align__(16) unsigned char cc_raw[];
   CcSmem& sm = *reinterpret_cast<CcSmem*>(cc_raw);
   const int tid = threadIdx.x;
+  const int word = reported(prm.status);
+  pass_on(word, prm.host_status);
+  if (word) return;
   int loaded = -1;
   for (int t = blockIdx.x; t < n_ctiles; t += gridDim.x) {
     const pylo_atile ct = ctiles[t];
@@ -1412,6 +1420,7 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
     const int rt = rpt * ng;          // rows per tile
     const int x0 = ct.strip * rt, y0 = ct.cb * tpr * 4;
     if (loaded != ct.tensor) {
+      const int word = FAM == PYLO_FAM_CELO2 ? 0 : reported(prm.status);
       __syncthreads();
       const float* __restrict__ wf = d.wfold;
       for (int e = tid; e < 30 * H; e += NT) { const float w = wf[L::W1 + e]; s_w[W::W1 + 2 * e] = w; s_w[W::W1 + 2 * e + 1] = w; }
@@ -1421,6 +1430,10 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
       for (int e = tid; e < 2; e += NT) { const float w = wf[L::B3 + e]; s_w[W::B3 + 2 * e] = w; s_w[W::B3 + 2 * e + 1] = w; s_sc[e] = wf[L::SC + e]; }
       loaded = ct.tensor;
       __syncthreads();
+      if (word) {
+        pass_on(word, prm.host_status);
+        return;
+      }
     }
     const int y = y0 + 4 * (tid % tpr), rg = tid / tpr;
     const bool colok = y < Y;
@@ -1594,8 +1607,10 @@ __global__ void __launch_bounds__(NT) k_post_sums(const pylo_post_item* __restri
 }
 
 __global__ void __launch_bounds__(NT) k_post_apply(const pylo_post_item* __restrict__ items,
-                                                   const pylo_tile* __restrict__ tiles, int n_tiles) {
+                                                   const pylo_tile* __restrict__ tiles, int n_tiles,
+                                                   const int* __restrict__ status, int* __restrict__ host_status) {
   pdl_begin();
+  const int word = reported(status);
   __shared__ float s_scale;
   for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const pylo_tile tl = tiles[t];
@@ -1608,6 +1623,10 @@ __global__ void __launch_bounds__(NT) k_post_apply(const pylo_post_item* __restr
       if (threadIdx.x == 0) s_scale = rsqrtf(1e-9f + (float)acc / (float)it.n) * it.rmsmult;
     }
     __syncthreads();
+    if (word) {
+      pass_on(word, host_status);
+      return;
+    }
     const float sc = s_scale, lr = it.lr, wd = it.wd;
     const float* s = it.step + tl.start;
     float* p = it.p + tl.start;
@@ -1799,7 +1818,7 @@ __global__ void __launch_bounds__(ROWS * PYLO_STAT_STRIDE + 32) k_velo_tensor_fe
 // through all tensors by itself: 203 us at 292 tensors).
 __global__ void __launch_bounds__(NT) k_velo_xmix(const pylo_velo_rnn r, const pylo_velo_loss lossbuf) {
   pdl_begin();
-  if (lossbuf.means && blockIdx.x == 0 && threadIdx.x < 32) velo_loss_update(lossbuf, nullptr, true);
+  if (lossbuf.means && blockIdx.x == 0 && threadIdx.x < 32) velo_loss_update(lossbuf, nullptr, !reported(r.status));
   const int h = blockIdx.x * NWARP + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (h >= r.H) return;
   float best = 0.f;   // relu
@@ -1948,6 +1967,7 @@ __global__ void k_velo_cell(const pylo_velo_rnn r, int parts) {
   pdl_begin();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (int64_t)r.T * r.H) return;
+  const int word = reported(r.status);
   const int t = (int)(e / r.H), h = (int)(e % r.H), H = r.H;
   const float* g4 = r.gates + (int64_t)t * 4 * H + h;
   float a[4];
@@ -1960,6 +1980,7 @@ __global__ void k_velo_cell(const pylo_velo_rnn r, int parts) {
   }
   const float i = sigmoidf_(a[0]), g = tanhf(a[1]), f = sigmoidf_(a[2] + 1.0f), o = sigmoidf_(a[3]);
   const float c = f * r.c[e] + i * g;
+  if (word) return;
   r.c[e] = c;
   r.h[e] = o * tanhf(c);
 }
@@ -2605,11 +2626,12 @@ int pylo_b200_celo2_post_sums(const pylo_post_item* items, const pylo_tile* tile
   return launch_status();
 }
 
-int pylo_b200_celo2_post_apply(const pylo_post_item* items, const pylo_tile* tiles, int n_tiles, void* stream) {
+int pylo_b200_celo2_post_apply(const pylo_post_item* items, const pylo_tile* tiles, int n_tiles, const int* status, int* host_status,
+                               void* stream) {
   CHECK_ARG(items && tiles && n_tiles >= 0);
   if (n_tiles == 0) return 0;
   const PlainLaunches plain(n_tiles);
-  launch(k_post_apply, grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream, items, tiles, n_tiles);
+  launch(k_post_apply, grid_for(n_tiles, 8), NT, 0, (cudaStream_t)stream, items, tiles, n_tiles, status, host_status);
   return launch_status();
 }
 

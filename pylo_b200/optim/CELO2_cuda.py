@@ -80,8 +80,6 @@ class _Celo2Family(Optimizer):
         # into a high and a low part of eleven bits each, as accurate as fp32 products); "fp32": torch.matmul, the
         # reference's arithmetic
         self.ns_precision = "3xtf32"
-        #: device word the Newton-Schulz kernel ORs 4 into if one of its bounded waits ran out
-        self._ns_status = torch.zeros(1, dtype=torch.int32, device=dev)
         #: Newton-Schulz launches of this library since construction (for the benchmark's launch count)
         self.extra_launches = 0
         self.process_group = None   # set (or set _sharded) when the tensors of the model are split over ranks
@@ -217,8 +215,6 @@ class _Celo2Family(Optimizer):
         for _, plan in self._plans.values():
             if plan["lo"] is not None:
                 plan["lo"].check_status()
-        if int(self._ns_status.item()) != 0:
-            raise L.PyloLibError(f"{self._name}: a wait inside the Newton-Schulz kernel timed out; the step is invalid")
 
     # ------------------------------------------------------------------ step
     @optimizer_step
@@ -286,12 +282,14 @@ class _Celo2Family(Optimizer):
             post.upload()
             plan["post_key"] = key
         L.check(L.lib.pylo_b200_celo2_post_sums(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_sums")
-        L.check(L.lib.pylo_b200_celo2_post_apply(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_apply")
+        L.check(L.lib.pylo_b200_celo2_post_apply(post.table.ptr, post.tiles.ptr, post.n_tiles, lo.step_plan.status,
+                                                 lo.step_plan.host_status, stream), "celo2_post_apply")
         self._keep = keep
 
     def _orthogonalise(self, plan, stream):
         """Newton-Schulz over the plan's stacks of raw steps: (the results to keep alive, address of every tensor's)."""
         keep, steps = [], [0] * len(plan["lo_params"])
+        status = plan["lo"].status   # the products OR 4 in if one of their bounded waits ran out
         native = self.ns_precision == "3xtf32" and newton_schulz_bounded(self.ns_coeffs, self.ns_iters)
         for group in plan["ns_groups"]:
             results = group["kept"]
@@ -303,11 +301,11 @@ class _Celo2Family(Optimizer):
                         # on every step, so that the training step can have the memory in between
                         group["kept"] = results
                 newton_schulz_native([part for part, _ in group["parts"]], [r for r, _ in results], [w for _, w in results],
-                                     self.ns_coeffs, self.ns_iters, self.ns_eps, self._ns_status, stream)
+                                     self.ns_coeffs, self.ns_iters, self.ns_eps, status, stream)
                 outs = [r for r, _ in results]
             else:
                 args = (self.ns_coeffs, self.ns_iters, self.ns_eps)
-                outs = [(newton_schulz_tc(part, *args, self._ns_status, stream) if self.ns_precision == "3xtf32"
+                outs = [(newton_schulz_tc(part, *args, status, stream) if self.ns_precision == "3xtf32"
                          else newton_schulz(part, *args)).contiguous() for part, _ in group["parts"]]
             if self.ns_precision == "3xtf32":
                 self.extra_launches += 3 * self.ns_iters

@@ -204,7 +204,7 @@ class VeLO_CUDA(Optimizer):
         f32 = dict(dtype=torch.float32, device=dev)
         buf = {
             "weights": torch.zeros(T, 160, **f32), "lr_mult": torch.zeros(T, **f32), "x_in": torch.zeros(T, 30, **f32),
-            "pooled": torch.zeros(H, **f32), "xmix": torch.zeros(T, H, **f32), "gates": torch.zeros(2, T, 4 * H, **f32),
+            "xmix": torch.zeros(T, H, **f32), "gates": torch.zeros(2, T, 4 * H, **f32),
             "controls": torch.zeros(T, B, **f32),
             "rank": torch.stack([self.state[p]["rank_onehot"] for p in plist]).contiguous(),
             "loss": torch.zeros(1, **f32),
@@ -235,7 +235,8 @@ class VeLO_CUDA(Optimizer):
         r.ctrl_w, r.ctrl_b = w["rnn_to_controls.weight"].data_ptr(), w["rnn_to_controls.bias"].data_ptr()
         r.step_w, r.step_b = w["step_size.weight"].data_ptr(), w["step_size.bias"].data_ptr()
         r.bank = self._bank.data_ptr()
-        for k in ("x_in", "pooled", "xmix", "gates", "controls", "weights", "lr_mult"):
+        r.status = plan.status.data_ptr()
+        for k in ("x_in", "xmix", "gates", "controls", "weights", "lr_mult"):
             setattr(r, k, buf[k].data_ptr())
         r.T, r.H, r.B = T, H, B
         return {"plan": plan, "buf": buf, "rnn": r, "loss": L.VeloLoss(), "hyper": None}

@@ -528,9 +528,9 @@ class LoPlan:
     def _poll_status(self):
         """Raise if a launch of an earlier step has written its status word."""
         if self._status_view[0] != 0:
-            raise L.PyloLibError("a bounded wait inside a kernel timed out in an earlier step (apply_adafac_tc: the kernel kept "
-                                 "the old values of the parameters it could not finish, and launches write nothing until "
-                                 "clear_status() is called)")
+            raise L.PyloLibError("a bounded wait inside a kernel timed out in an earlier step: that step is incomplete, the "
+                                 "parameters it could not finish kept their old values, and launches write no parameters until "
+                                 "clear_status() is called")
 
     def _back(self, prm, stream):
         """Phases P, C, one call each (timed)."""
@@ -556,12 +556,15 @@ class LoPlan:
     def check_status(self):
         """Synchronise and raise if a kernel reported a wait that ran out.
 
-        The tensor-core kernel keeps the old value of every parameter it could not finish, so nothing invalid was
-        written, but the step is incomplete; until :meth:`clear_status` it stores nothing at all.  Call this before a
-        checkpoint is written."""
+        Every kernel that writes parameters keeps the old value of those it could not finish, and of all of them where what
+        it reads is incomplete, so no invalid parameter was written; but the step is incomplete (the accumulators may have
+        advanced in part), and until :meth:`clear_status` no parameter is written at all.  Call this before a checkpoint
+        is written."""
         code = int(self.status[0].item())
         if code & 8:
             raise L.PyloLibError("a wait for a kernel's own copies timed out; this step is incomplete")
+        if code & 4:
+            raise L.PyloLibError("a wait inside a Newton-Schulz kernel timed out; this step is incomplete")
         if code != 0:
             raise L.PyloLibError("apply_adafac_tc: a wait on the tensor core timed out; this step is incomplete "
                                  "(unfinished parameters kept their old values)")

@@ -236,3 +236,38 @@ def test_a_scheduled_tensor_learning_rate_is_followed(family):
             _step(opt, family, t)
         runs.append([p.detach().clone() for p in params])
     assert all(torch.equal(a, b) for a, b in zip(*runs))
+
+
+def _plans(opt):
+    if getattr(opt, "_plan", None):
+        return [opt._plan[1]["plan"]]
+    return [v[1]["lo"] if isinstance(v[1], dict) else v[1] for v in opt._plans.values()]
+
+
+@pytest.mark.parametrize("family,extra", [("adafaclo", {}), ("adafaclo", {"mlp_precision": "fp32"}), ("elo", {}), ("celo2", {}),
+                                          ("elo_celo2", {}), ("velo", {})])
+def test_a_reported_wait_keeps_the_parameters(family, extra):
+    """The status word is set from the host (no wait runs out here): every kernel that writes parameters, on matrices of both
+    kinds, must leave them, VeLO's LSTM must keep its state, and check_status() and the next step must say so."""
+    shapes = [(40, 24), (33, 7)]
+    params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(dict(shapes=shapes, init_seed=97, init_scale=0.1))]
+    opt = _make(family, params, **extra)
+    for p, g in zip(params, cases.grads_at(dict(grad_seed=98, grad_scale=0.3, shapes=shapes), 1)):
+        p.grad = g.cuda()
+    _step(opt, family, 1)
+    opt.check_status()
+    plan, = _plans(opt)
+    plan.status[0] = 4 if "celo2" in family else 8
+    with pytest.raises(pylo_lib.PyloLibError):
+        opt.check_status()
+
+    def kept():
+        lstm = [*opt.lstm_hidden_state, *opt.loss_buffer.values()] if family == "velo" else []
+        return [t.detach().clone() for t in params + lstm]
+
+    before = kept()
+    _step(opt, family, 2)      # its launches find the word set and pass it on to the host
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(before, kept()))
+    with pytest.raises(pylo_lib.PyloLibError):
+        _step(opt, family, 3)

@@ -33,3 +33,12 @@ def test_no_cta_reaches_into_another_before_it_is_known_to_run():
             continue
         before = body[:reach.start()]
         assert "cluster_sync();" in before or re.search(r"cluster_arrive\(\);.*cluster_wait\(\);", before, re.S), name
+
+
+def test_kernels_that_write_parameters_look_at_the_status_word():
+    """After a wait that ran out the step's sums are incomplete; no kernel may write parameters from them.  (k_adamw reads
+    nothing that an earlier kernel of the step makes.)"""
+    bodies = functions()
+    for name in ("k_apply", "k_apply_adafac_cols", "k_apply_packed", "k_post_apply", "k_velo_cell", "k_velo_xmix"):
+        assert "reported(" in bodies[name], name
+    assert "poisoned" in bodies["k_apply_adafac_tc"]
