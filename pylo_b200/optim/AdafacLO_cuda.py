@@ -112,12 +112,12 @@ class _AdafacFamily(Optimizer):
         return LoPlan(L.FAM_ADAFAC, tensors, self.device, tensor_cores=(self.mlp_precision == "3xtf32"))
 
     def check_status(self):
-        """Synchronise and raise if a tensor-core launch of an earlier step reported a timed-out wait."""
+        """Synchronise and raise if a kernel of an earlier step reported a wait that ran out."""
         for _, plan in self._plans.values():
             plan.check_status()
 
     def clear_status(self):
-        """Acknowledge a reported tensor-core timeout so that the apply kernels store again."""
+        """Acknowledge a reported timeout: the next steps write parameters again."""
         for _, plan in self._plans.values():
             plan.clear_status()
 

@@ -216,6 +216,12 @@ class _Celo2Family(Optimizer):
             if plan["lo"] is not None:
                 plan["lo"].check_status()
 
+    def clear_status(self):
+        """Acknowledge a reported timeout: the next steps write parameters again."""
+        for _, plan in self._plans.values():
+            if plan["lo"] is not None:
+                plan["lo"].clear_status()
+
     # ------------------------------------------------------------------ step
     @optimizer_step
     def step(self, loss=None):

@@ -196,6 +196,11 @@ class VeLO_CUDA(Optimizer):
         if self._plan is not None:
             self._plan[1]["plan"].check_status()
 
+    def clear_status(self):
+        """Acknowledge a reported timeout: the next steps write parameters again."""
+        if self._plan is not None:
+            self._plan[1]["plan"].clear_status()
+
     # ------------------------------------------------------------------ planning
     def _build_plan(self, plist):
         dev = self.device

@@ -570,7 +570,7 @@ class LoPlan:
                                  "(unfinished parameters kept their old values)")
 
     def clear_status(self):
-        """Acknowledge a reported timeout: the next launches store again."""
+        """Acknowledge a reported timeout: the next launches write parameters again."""
         self.status.zero_()
         torch.cuda.synchronize(self.device)   # a launch in flight may still write the host's word
         self._status_host.zero_()

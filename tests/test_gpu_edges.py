@@ -271,3 +271,7 @@ def test_a_reported_wait_keeps_the_parameters(family, extra):
     assert all(torch.equal(a, b) for a, b in zip(before, kept()))
     with pytest.raises(pylo_lib.PyloLibError):
         _step(opt, family, 3)
+    opt.clear_status()
+    _step(opt, family, 4)
+    opt.check_status()
+    assert not any(torch.equal(a, p) for a, p in zip(before, params)), "a cleared optimizer goes on"

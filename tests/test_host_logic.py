@@ -207,3 +207,11 @@ def test_a_tensor_learning_rate_that_a_scheduler_changes_in_place_is_seen():
     sched.step()
     assert group["lr"] is lr, "the scheduler changes the tensor in place"
     assert kept == (0.5, 0.1) and group_floats(group, "lr", "weight_decay") == (0.25, 0.1)
+
+
+@pytest.mark.parametrize("name", ["AdafacLO_CUDA", "ELO_CUDA", "CELO2_CUDA", "ELO_CELO2_CUDA", "VeLO_CUDA"])
+def test_every_class_that_reports_a_timeout_can_be_cleared(name):
+    from pylo_b200 import optim
+
+    cls = getattr(optim, name)
+    assert callable(cls.check_status) and callable(cls.clear_status)
