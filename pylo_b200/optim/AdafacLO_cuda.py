@@ -121,6 +121,11 @@ class _AdafacFamily(Optimizer):
         for _, plan in self._plans.values():
             plan.clear_status()
 
+    def _poll_status(self):
+        """Refuse the step before anything (gradients, step counters, an earlier group) is touched."""
+        for _, plan in self._plans.values():
+            plan.poll_status()
+
     def _run_group(self, gi, plist, grads, prm, stream, **hyper):
         sig = [p.data_ptr() for p in plist]
         cached = self._plans.get(gi)
@@ -129,7 +134,6 @@ class _AdafacFamily(Optimizer):
             self._plans[gi] = cached
             cached[1].counters = StepCounters([self.state[p] for p in plist])
         plan: LoPlan = cached[1]
-        plan._poll_status()  # refuse the step before any state (the step counters included) is advanced
         plan.set_hyper(**hyper)
         plan.refresh(grads, plan.counters)
         if self.before_group is not None:
@@ -223,6 +227,7 @@ class AdafacLO_CUDA(_AdafacFamily):
 
     @optimizer_step
     def step(self, loss=None):
+        self._poll_status()
         stream = current_stream_ptr()
         for gi, group in enumerate(self.param_groups):
             if group["max_grad_norm"] is not None:
@@ -278,6 +283,7 @@ class ELO_CUDA(_AdafacFamily):
 
     @optimizer_step
     def step(self, loss=None):
+        self._poll_status()
         stream = current_stream_ptr()
         gnorm_ptr = None
         if any(g["clip_grad"] for g in self.param_groups):

@@ -225,6 +225,9 @@ class _Celo2Family(Optimizer):
     # ------------------------------------------------------------------ step
     @optimizer_step
     def step(self, loss=None):
+        for _, plan in self._plans.values():
+            if plan["lo"] is not None:
+                plan["lo"].poll_status()
         stream = current_stream_ptr()
         gnorm_ptr = None
         if any(g["clip_grad"] for g in self.param_groups):

@@ -249,6 +249,8 @@ class VeLO_CUDA(Optimizer):
     # ------------------------------------------------------------------ step
     @optimizer_step
     def step(self, loss):
+        if self._plan is not None:
+            self._plan[1]["plan"].poll_status()
         stream = current_stream_ptr()
         dev = self.device
         plist, counts, hyper = [], [], []

@@ -496,7 +496,6 @@ class LoPlan:
 
     def run(self, prm: L.StepParams, stream: int, phases: int = L.STEP_FRONT | L.STEP_BACK):
         """The phases of a step (all of them, or only those before or after the caller's own work in between)."""
-        self._poll_status()  # before any state of this step is touched
         prm.step_delta = self.step_delta
         prm.status, prm.host_status = self.step_plan.status, self.step_plan.host_status
         prm.bulk_copies = self.bulk_copies
@@ -525,8 +524,9 @@ class LoPlan:
         if self.family != L.FAM_VELO:
             self._call("finalize_moments", L.lib.pylo_b200_finalize_moments, self.desc.ptr, self.n_units, stream)
 
-    def _poll_status(self):
-        """Raise if a launch of an earlier step has written its status word."""
+    def poll_status(self):
+        """Raise if a launch of an earlier step has written its status word: every optimizer's step begins with this, for all
+        of its plans, before it advances anything of its own."""
         if self._status_view[0] != 0:
             raise L.PyloLibError("a bounded wait inside a kernel timed out in an earlier step: that step is incomplete, the "
                                  "parameters it could not finish kept their old values, and launches write no parameters until "

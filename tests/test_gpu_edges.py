@@ -275,3 +275,35 @@ def test_a_reported_wait_keeps_the_parameters(family, extra):
     _step(opt, family, 4)
     opt.check_status()
     assert not any(torch.equal(a, p) for a, p in zip(before, params)), "a cleared optimizer goes on"
+
+
+@pytest.mark.parametrize("family", ["adafaclo", "elo", "celo2", "elo_celo2", "velo"])
+def test_a_refused_step_has_advanced_nothing(family):
+    """A reported timeout of the second param group: the first group, the step counters, the gradients and the state stay."""
+    shapes = [(40, 24), (33, 20)]
+    params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(dict(shapes=shapes, init_seed=97, init_scale=0.1))]
+    opt = _make(family, [{"params": [p]} for p in params])
+    if family == "adafaclo":
+        for group in opt.param_groups:
+            group["max_grad_norm"] = 1e-3   # scales the gradients in place
+    grads = [g.cuda() for g in cases.grads_at(dict(grad_seed=98, grad_scale=0.3, shapes=shapes), 1)]
+    for p, g in zip(params, grads):
+        p.grad = g
+    _step(opt, family, 1)
+    torch.cuda.synchronize()
+    for g in grads:
+        g.mul_(1e6)
+
+    def everything():
+        out = [t.clone() for t in grads] + [p.detach().clone() for p in params]
+        for p in params:
+            out += [v.clone() if torch.is_tensor(v) else torch.tensor(float(v)) for v in opt.state[p].values()]
+        return out + [torch.tensor(float(g.get("step", 0))) for g in opt.param_groups]
+
+    before = everything()
+    _plans(opt)[-1]._status_view[0] = 8
+    with pytest.raises(pylo_lib.PyloLibError):
+        _step(opt, family, 2)
+    torch.cuda.synchronize()
+    after = everything()
+    assert len(before) == len(after) and all(torch.equal(a, b) for a, b in zip(before, after))
