@@ -690,6 +690,7 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
     float* out = d.tile_part + (int64_t)(t - d.tile0) * PYLO_STAT_STRIDE;
     block_reduce_store<NACC>(acc, s_red, out);
     if (tid >= NACC && tid < PYLO_STAT_STRIDE) out[tid] = 0.f;
+    if constexpr (RING) dead = __syncthreads_or(dead);   // a warp whose wait ran out takes the whole CTA with it: the barriers above are everyone's
   }
   if constexpr (RING) {
     if (dead && (tid & 31) == 0) pipe_failed(prm);

@@ -27,16 +27,14 @@ __device__ __forceinline__ void pipe_init(PipeSmem& p) {
   }
   __syncthreads();
 }
-// bounded wait for the phase with the given parity; false if it ran out
+// bounded wait of a whole warp for the phase with the given parity; false, in all of its lanes, if it ran out
 __device__ __forceinline__ bool pipe_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t a = smem_addr(bar);
-  for (int it = 0; it < PIPE_SPIN_LIMIT; ++it) {
-    uint32_t ok;
+  uint32_t ok = 0;
+  for (int it = 0; it < PIPE_SPIN_LIMIT && !ok; ++it)
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok) : "r"(a), "r"(parity) : "memory");
-    if (ok) return true;
-  }
-  return false;
+  return __all_sync(0xffffffffu, ok);
 }
 __device__ __forceinline__ bool pipe_wait_full(PipeSmem& p, uint32_t k) { return pipe_wait(&p.full[k % PIPE_STAGES], (k / PIPE_STAGES) & 1); }
 // the calling warp has read stage k

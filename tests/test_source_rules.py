@@ -42,3 +42,11 @@ def test_kernels_that_write_parameters_look_at_the_status_word():
     for name in ("k_apply", "k_apply_adafac_cols", "k_apply_packed", "k_post_apply", "k_velo_cell", "k_velo_xmix"):
         assert "reported(" in bodies[name], name
     assert "poisoned" in bodies["k_apply_adafac_tc"]
+
+
+def test_a_failed_wait_of_the_ring_ends_the_whole_cta():
+    """A wait that runs out is one answer for the warp (shuffles and barriers follow) and, at the tile's end, for the CTA."""
+    bodies = functions()
+    assert "__all_sync(0xffffffffu, ok)" in bodies["pipe_wait"]
+    sweep = bodies["k_state_moments"]
+    assert sweep.index("block_reduce_store<NACC>") < sweep.index("dead = __syncthreads_or(dead)")
