@@ -423,11 +423,19 @@ int pylo_b200_velo_loss_features(float* means, int32_t* iteration, float* runnin
                                  const float* loss, float* loss9, void* stream);
 
 /* All tables of one optimizer's tensors, and a step's phases over them in one call: PYLO_STEP_FRONT is rowcol_sums,
- * factor_update, state_moments (tiles in reverse), finalize_moments; PYLO_STEP_BACK is prep_apply and the apply kernels.
- * plan and prm are HOST pointers.  ctiles: items of pylo_b200_apply_adafac_tc where tensor_cores is set (the n_ctiles_gen
+ * factor_update, state_moments (tiles in reverse), finalize_moments; PYLO_STEP_BACK is prep_apply and the apply kernels
+ * (PYLO_STEP_APPLY_REST: the launch, if there is one of its own, of what is not FAST2D).  A host that times the phases gives
+ * them one by one.  plan and prm are HOST pointers.  ctiles: items of pylo_b200_apply_adafac_tc where tensor_cores is set (the n_ctiles_gen
  * on units that are not FAST2D first), else of apply_adafac_cols / apply_packed, with the other units in tiles_slow. */
-#define PYLO_STEP_FRONT 1
-#define PYLO_STEP_BACK 2
+#define PYLO_STEP_SUMS 1
+#define PYLO_STEP_FACTORS 2
+#define PYLO_STEP_STATE 4
+#define PYLO_STEP_MOMENTS 8
+#define PYLO_STEP_PREP 16
+#define PYLO_STEP_APPLY 32
+#define PYLO_STEP_APPLY_REST 64
+#define PYLO_STEP_FRONT (PYLO_STEP_SUMS | PYLO_STEP_FACTORS | PYLO_STEP_STATE | PYLO_STEP_MOMENTS)
+#define PYLO_STEP_BACK (PYLO_STEP_PREP | PYLO_STEP_APPLY | PYLO_STEP_APPLY_REST)
 #define PYLO_TC_ONE_LAUNCH 4736 /* items below which one launch takes both kinds of items of apply_adafac_tc */
 typedef struct pylo_step_plan {
   const pylo_tensor_desc *tdesc, *desc; /* per tensor, per unit */

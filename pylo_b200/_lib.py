@@ -165,7 +165,9 @@ lib, EXPORTED = _load()
 SM_COUNT = 148        # of a B200; sizes of work lists only, the kernels ask the device
 TC_WORKERS = SM_COUNT * 4  # warpgroups the tensor-core apply kernel runs at once (four per SM)
 TC_GEN_ITEM = 1 << 16  # tag bit of its items on tensors that are not FAST2D
-STEP_FRONT, STEP_BACK = 1, 2
+STEP_SUMS, STEP_FACTORS, STEP_STATE, STEP_MOMENTS, STEP_PREP, STEP_APPLY, STEP_APPLY_REST = (1 << k for k in range(7))
+STEP_FRONT = STEP_SUMS | STEP_FACTORS | STEP_STATE | STEP_MOMENTS
+STEP_BACK = STEP_PREP | STEP_APPLY | STEP_APPLY_REST
 TC_ONE_LAUNCH = 8 * TC_WORKERS  # items below which one launch of the tensor-core kernel takes both kinds of items
 BULK_COPY_ELEMS = 1 << 26  # FAST2D elements from which the state sweep reads through a ring of bulk copies
 STATIC_SCRATCH_TILES = 65536

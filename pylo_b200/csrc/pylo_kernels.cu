@@ -2699,31 +2699,34 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
   CHECK_ARG(p && prm);
   const PlainLaunches plain(p->n_tiles);
   int rc = 0;
-  if (phases & PYLO_STEP_FRONT) {
-    if (p->n_atiles || p->n_gitems)
-      if ((rc = pylo_b200_rowcol_sums(p->tdesc, p->atiles, p->n_atiles, p->gitems, p->n_gitems, prm, stream))) return rc;
+  if ((phases & PYLO_STEP_SUMS) && (p->n_atiles || p->n_gitems))
+    if ((rc = pylo_b200_rowcol_sums(p->tdesc, p->atiles, p->n_atiles, p->gitems, p->n_gitems, prm, stream))) return rc;
+  if (phases & PYLO_STEP_FACTORS)
     if ((rc = pylo_b200_factor_update(p->tdesc, p->n_tensors, prm, stream))) return rc;
+  if (phases & PYLO_STEP_STATE)
     if ((rc = pylo_b200_state_moments(p->desc, p->tiles, p->n_tiles, 1, prm, stream))) return rc;
-    if (!p->sum_tiles && (rc = pylo_b200_finalize_moments(p->desc, p->n_units, stream))) return rc;
-  }
-  if (phases & PYLO_STEP_BACK) {
-    pylo_step_params q = *prm;
-    q.sum_tiles = p->sum_tiles && q.family != PYLO_FAM_VELO;
-    q.no_tables = p->tensor_cores ? 2 : 0;   // the tensor-core kernel reads the per-row table only
+  if ((phases & PYLO_STEP_MOMENTS) && !p->sum_tiles)
+    if ((rc = pylo_b200_finalize_moments(p->desc, p->n_units, stream))) return rc;
+  if (!(phases & PYLO_STEP_BACK)) return 0;
+  pylo_step_params q = *prm;
+  q.sum_tiles = p->sum_tiles && q.family != PYLO_FAM_VELO;
+  q.no_tables = p->tensor_cores ? 2 : 0;   // the tensor-core kernel reads the per-row table only
+  if (phases & PYLO_STEP_PREP)
     if ((rc = pylo_b200_prep_apply(p->desc, p->pitems, p->n_pitems, &q, stream))) return rc;
-    if (p->tensor_cores) {
-      // small models: one launch; large ones: what is not FAST2D first, then the rest through the leaner variant
-      const int first = p->n_ctiles < PYLO_TC_ONE_LAUNCH ? p->n_ctiles : p->n_ctiles_gen;
-      if ((rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles, first, p->n_ctiles_gen > 0, &q, p->status, p->host_status, stream))) return rc;
-      if ((rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles + first, p->n_ctiles - first, 0, &q, p->status, p->host_status, stream))) return rc;
-    } else if (p->n_ctiles) {
-      rc = q.family == PYLO_FAM_ADAFAC ? pylo_b200_apply_adafac_cols(p->desc, p->ctiles, p->n_ctiles, &q, stream)
-                                       : pylo_b200_apply_packed(p->desc, p->ctiles, p->n_ctiles, &q, stream);
-      if (rc) return rc;
-    }
-    if (p->n_tiles_slow)
-      if ((rc = pylo_b200_apply(p->desc, p->tiles_slow, p->n_tiles_slow, 0, &q, stream))) return rc;
+  const bool main = phases & PYLO_STEP_APPLY, rest = phases & PYLO_STEP_APPLY_REST;
+  if (p->tensor_cores) {
+    // small models: one launch; large ones: what is not FAST2D first, then the others through the leaner variant
+    const int first = p->n_ctiles < PYLO_TC_ONE_LAUNCH ? 0 : p->n_ctiles_gen;
+    if (rest && (rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles, first, 1, &q, p->status, p->host_status, stream))) return rc;
+    if (main && (rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles + first, p->n_ctiles - first, p->n_ctiles_gen > first, &q, p->status, p->host_status, stream))) return rc;
+    return 0;
   }
+  if (main && p->n_ctiles) {
+    rc = q.family == PYLO_FAM_ADAFAC ? pylo_b200_apply_adafac_cols(p->desc, p->ctiles, p->n_ctiles, &q, stream)
+                                     : pylo_b200_apply_packed(p->desc, p->ctiles, p->n_ctiles, &q, stream);
+    if (rc) return rc;
+  }
+  if (rest && p->n_tiles_slow) return pylo_b200_apply(p->desc, p->tiles_slow, p->n_tiles_slow, 0, &q, stream);
   return 0;
 }
 

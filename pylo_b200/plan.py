@@ -406,7 +406,9 @@ class LoPlan:
         self._dirty = True          # the host table is ahead of the device's
         self.step_delta = 0.0
         self._prof = None
+        #: launches since construction (or since the caller zeroed it), and what each call of :meth:`run` adds
         self.launch_count = 0
+        self._launches = {k: sum(n for ph, _, n in self._phases() if ph & k) for k in (L.STEP_FRONT, L.STEP_BACK, L.STEP_FRONT | L.STEP_BACK)}
 
     # ------------------------------------------------------------------ per-step refresh
     def set_field(self, name, values):
@@ -472,57 +474,44 @@ class LoPlan:
     #: the kernel that dominates each timed phase, for reports
     KERNEL_OF = {"rowcol_sums": "k_rowcol_fast", "factor_update": "k_factor_update", "state_moments": "k_state_moments",
                  "finalize_moments": "k_finalize_moments", "prep_apply": "k_prep_apply"}
-    #: kernels each C-ABI call launches (for the launch count the benchmark reports)
-    LAUNCHES = {"rowcol_sums": 1, "factor_update": 1, "state_moments": 1, "finalize_moments": 1, "prep_apply": 1}
+
+    def _phases(self):
+        """[(phase of pylo_b200_step, name, launches)] in the step's order, without those that launch nothing."""
+        split = self.tensor_cores and self.n_ctiles >= L.TC_ONE_LAUNCH   # a launch of its own for what is not FAST2D
+        rest = int(split and self.n_ctiles_gen > 0) if self.tensor_cores else int(self.n_tiles_slow > 0)
+        main = int(self.n_ctiles > (self.n_ctiles_gen if split else 0))
+        apply = [(L.STEP_APPLY, self.apply_kernel, main)]
+        apply.insert(0 if self.tensor_cores else 1, (L.STEP_APPLY_REST, "k_apply_adafac_tc<true>" if self.tensor_cores else "k_apply", rest))
+        phases = [(L.STEP_SUMS, "rowcol_sums", (self.n_atiles > 0) + (self.n_gitems > 0)), (L.STEP_FACTORS, "factor_update", 1),
+                  (L.STEP_STATE, "state_moments", 1), (L.STEP_MOMENTS, "finalize_moments", int(not self.sum_tiles)),
+                  (L.STEP_PREP, "prep_apply", 1)] + apply
+        return [ph for ph in phases if ph[2]]
 
     def enable_profile(self, on: bool = True):
-        """Record a CUDA-event pair around every phase launch (read back with :meth:`phase_times`)."""
+        """Record a CUDA-event pair around every phase (read back with :meth:`phase_times`): the launches are those of any
+        other step, but each phase then waits for the end of the one before."""
         self._prof = {} if on else None
 
     def phase_times(self):
         """{phase: [ms, ...]} of the recorded launches; call after a device synchronisation."""
         return {k: [a.elapsed_time(b) for a, b in v] for k, v in (self._prof or {}).items()}
 
-    def _call(self, name, fn, *args):
-        prof = self._prof
-        if prof is not None:
-            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a.record()
-        L.check(fn(*args), name)
-        self.launch_count += self.LAUNCHES.get(name, 1)
-        if prof is not None:
-            b.record()
-            prof.setdefault(name, []).append((a, b))
-
     def run(self, prm: L.StepParams, stream: int, phases: int = L.STEP_FRONT | L.STEP_BACK):
         """The phases of a step (all of them, or only those before or after the caller's own work in between)."""
         prm.step_delta = self.step_delta
         prm.status, prm.host_status = self.step_plan.status, self.step_plan.host_status
         prm.bulk_copies = self.bulk_copies
+        self.launch_count += self._launches[phases]
         if self._prof is None:
             L.check(L.lib.pylo_b200_step(self._step_plan_ref, C.byref(prm), phases, stream), "step")
-            if phases & L.STEP_FRONT:
-                self.launch_count += 3 - self.sum_tiles + (self.n_atiles > 0) + (self.n_gitems > 0)
-            if phases & L.STEP_BACK:
-                two = self.tensor_cores and 0 < self.n_ctiles_gen < self.n_ctiles and self.n_ctiles >= L.TC_ONE_LAUNCH
-                self.launch_count += 1 + (self.n_ctiles > 0) + two + (self.n_tiles_slow > 0)
             return
-        if phases & L.STEP_FRONT:
-            self._front(prm, stream)
-        if phases & L.STEP_BACK:
-            self._back(prm, stream)
-
-    def _front(self, prm, stream):
-        """Phases A, A2, B, B2, one call each (timed)."""
-        pp = C.byref(prm)
-        if self.n_atiles or self.n_gitems:
-            self._call("rowcol_sums", L.lib.pylo_b200_rowcol_sums, self.tdesc.ptr, self.atiles.ptr, self.n_atiles,
-                       self.gitems.ptr, self.n_gitems, pp, stream)
-            self.launch_count += 1 if self.n_atiles and self.n_gitems else 0
-        self._call("factor_update", L.lib.pylo_b200_factor_update, self.tdesc.ptr, self.n_tensors, pp, stream)
-        self._call("state_moments", L.lib.pylo_b200_state_moments, self.desc.ptr, self.tiles.ptr, self.n_tiles, 1, pp, stream)
-        if self.family != L.FAM_VELO:
-            self._call("finalize_moments", L.lib.pylo_b200_finalize_moments, self.desc.ptr, self.n_units, stream)
+        for phase, name, _ in self._phases():
+            if phases & phase:
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record()
+                L.check(L.lib.pylo_b200_step(self._step_plan_ref, C.byref(prm), phase, stream), name)
+                b.record()
+                self._prof.setdefault(name, []).append((a, b))
 
     def poll_status(self):
         """Raise if a launch of an earlier step has written its status word: every optimizer's step begins with this, for all
@@ -531,27 +520,6 @@ class LoPlan:
             raise L.PyloLibError("a bounded wait inside a kernel timed out in an earlier step: that step is incomplete, the "
                                  "parameters it could not finish kept their old values, and launches write no parameters until "
                                  "clear_status() is called")
-
-    def _back(self, prm, stream):
-        """Phases P, C, one call each (timed)."""
-        # the tensor-core kernel needs the per-row table only (2); the CUDA-core kernels need both (0)
-        prm.no_tables, prm.sum_tiles = 2 if self.tensor_cores else 0, 0
-        pp = C.byref(prm)
-        self._call("prep_apply", L.lib.pylo_b200_prep_apply, self.desc.ptr, self.pitems.ptr, self.n_pitems, pp, stream)
-        if self.n_ctiles and self.tensor_cores:
-            # small models: one launch; large ones: what is not FAST2D first, then the rest through the leaner variant
-            first = self.n_ctiles if self.n_ctiles < L.TC_ONE_LAUNCH else self.n_ctiles_gen
-            for at, count in ((0, first), (first, self.n_ctiles - first)):
-                if count:
-                    gen = at == 0 and self.n_ctiles_gen > 0
-                    self._call(self.apply_kernel if count > self.n_ctiles_gen else "k_apply", L.lib.pylo_b200_apply_adafac_tc,
-                               self.desc.ptr, self.ctiles.ptr + at * L.ATILE_DTYPE.itemsize, count, int(gen), pp,
-                               self.status.data_ptr(), self._status_host.data_ptr(), stream)
-        elif self.n_ctiles:
-            fn = L.lib.pylo_b200_apply_adafac_cols if self.family == L.FAM_ADAFAC else L.lib.pylo_b200_apply_packed
-            self._call(self.apply_kernel, fn, self.desc.ptr, self.ctiles.ptr, self.n_ctiles, pp, stream)
-        if self.n_tiles_slow:
-            self._call("k_apply", L.lib.pylo_b200_apply, self.desc.ptr, self.tiles_slow.ptr, self.n_tiles_slow, 0, pp, stream)
 
     def check_status(self):
         """Synchronise and raise if a kernel reported a wait that ran out.

@@ -307,3 +307,29 @@ def test_a_refused_step_has_advanced_nothing(family):
     torch.cuda.synchronize()
     after = everything()
     assert len(before) == len(after) and all(torch.equal(a, b) for a, b in zip(before, after))
+
+
+@pytest.mark.parametrize("family,extra", [("adafaclo", {}), ("adafaclo", {"mlp_precision": "fp32"}), ("celo2", {"orthogonalize": False}),
+                                          ("velo", {})])
+@pytest.mark.parametrize("shapes", [[(40, 24), (33, 7)], [(2048, 1024), (33, 7)]], ids=["small", "many_tiles"])
+def test_timed_phases_are_the_step_that_users_get(family, extra, shapes):
+    """Timed phase by phase, a step launches what it launches otherwise (counted, and by its result bit for bit)."""
+    case = dict(shapes=shapes, init_seed=97, init_scale=0.1, grad_seed=98, grad_scale=0.3)
+    runs = []
+    for timed in (False, True):
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+        opt = _make(family, params, **extra)
+        for t in (1, 2):
+            for p, g in zip(params, cases.grads_at(case, t)):
+                p.grad = g.cuda()
+            _step(opt, family, t)
+            plan, = _plans(opt)
+            if t == 1:
+                plan.enable_profile(timed)
+                plan.launch_count = 0
+        torch.cuda.synchronize()
+        runs.append(([p.detach().clone() for p in params], plan.launch_count))
+    assert all(torch.equal(a, b) for a, b in zip(runs[0][0], runs[1][0])) and runs[0][1] == runs[1][1]
+    times = plan.phase_times()
+    assert ("finalize_moments" in times) == (not plan.sum_tiles) and plan.apply_kernel in times
+    assert all(len(v) == 1 and v[0] > 0 for v in times.values())
