@@ -443,8 +443,8 @@ typedef struct pylo_step_plan {
   const pylo_tile *tiles, *tiles_slow;
   int *status, *host_status;
   int32_t n_tensors, n_units, n_atiles, n_gitems, n_pitems, n_ctiles, n_ctiles_gen, n_tiles, n_tiles_slow, tensor_cores;
-  int32_t sum_tiles; /* 1: leave finalize_moments out and let prep_apply add up the tile partials, for units of about a
-                        hundred tiles at most (VELO, of any size: velo_tensor_features does it) */
+  int32_t sum_tiles; /* 1: leave finalize_moments out and let prep_apply add up the tile partials, for units of up to
+                        about 200 tiles (VELO, of any size: velo_tensor_features does it) */
   int32_t pad_;
 } pylo_step_plan;
 int pylo_b200_step(const pylo_step_plan* plan, const pylo_step_params* prm, int phases, void* stream);

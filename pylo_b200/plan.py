@@ -19,6 +19,14 @@ import torch
 from . import _lib as L
 
 
+#: Tiles of a unit up to which phase P adds their partials up itself instead of a launch before it.  Every item of phase P
+#: repeats its unit's sum (six rows at a time, a chain that grows with the tiles), the launch costs a fixed time.  AdafacLO and
+#: CELO2, one to five units, us per step without and with the launch: 98 tiles 36.0 / 37.4, 112: 41.4 / 42.3, 160: 46.1 / 47.3,
+#: 192: 45.5 / 47.2 and 75.3 / 75.7; 224: 48.3 / 48.0, 256: 43.1 / 42.4, 512: 58.8 / 56.4.  Ten to forty units of up to 112
+#: tiles: 1.6 us less to 1.4 more.
+SUM_TILES_MOST = 192
+
+
 def _prod(xs) -> int:
     out = 1
     for x in xs:
@@ -383,9 +391,7 @@ class LoPlan:
         self.tiles_slow = DeviceTable(slow, self.device)
         self.n_tiles_slow = len(slow)
         #: no launch for phase B2: of small units phase P adds the tile partials up, for VeLO the LSTM's input kernel does.
-        #: Every item of phase P repeats its unit's sum: about a hundred tiles are read in the time that a launch takes
-        #: (AdafacLO on a 118 K perceptron, 98 tiles: 39.6 -> 38.0 us per step)
-        self.sum_tiles = family == L.FAM_VELO or max((k for _, k in ranges), default=0) <= 112
+        self.sum_tiles = family == L.FAM_VELO or max((k for _, k in ranges), default=0) <= SUM_TILES_MOST
         # The state sweep's ring of bulk copies leaves little L1 cache to the units that are not FAST2D and keeps the launches
         # around it apart, so it has to have enough to do: from 64 M elements on (VeLO on 100 M: 1615 -> 1580 us per step, on
         # 17 M: 341 -> 351; AdafacLO on 25 M: 837 -> 851, on 86 M even), nearly all of them FAST2D.

@@ -333,3 +333,27 @@ def test_timed_phases_are_the_step_that_users_get(family, extra, shapes):
     times = plan.phase_times()
     assert ("finalize_moments" in times) == (not plan.sum_tiles) and plan.apply_kernel in times
     assert all(len(v) == 1 and v[0] > 0 for v in times.values())
+
+
+@pytest.mark.parametrize("family,extra", [("adafaclo", {}), ("celo2", {"orthogonalize": False})])
+@pytest.mark.parametrize("rows", [8 * 192, 8 * 192 + 8])
+def test_tile_sums_on_both_sides_of_the_launch(family, extra, rows):
+    """The most tiles that phase P adds up itself, and one more: the step with the other way of adding them."""
+    case = dict(shapes=[(rows, 128)], init_seed=97, init_scale=0.1, grad_seed=98, grad_scale=0.3)
+    runs = []
+    for flip in (False, True):
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+        opt = _make(family, params, **extra)
+        for t in (1, 2, 3):
+            params[0].grad = cases.grads_at(case, t)[0].cuda()
+            _step(opt, family, t)
+            plan, = _plans(opt)
+            if t == 1:
+                assert plan.sum_tiles == (rows == 8 * 192) and plan.n_tiles == rows // 8
+                if flip:
+                    plan.step_plan.sum_tiles = int(not plan.sum_tiles)
+        runs.append(params[0].detach().clone())
+    # the partials are added up in fp64 on both ways and rounded once: they differ by the last bit of a sum at most, which
+    # moves a normalised feature by 2^-24 of itself and the network's output, and so the step, by a few times that
+    move = float((runs[0] - cases.init_values(case)[0].cuda()).abs().max())
+    assert float((runs[0] - runs[1]).abs().max()) <= 1e-5 * move + 2 ** -23 * float(runs[0].abs().max())
