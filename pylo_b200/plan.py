@@ -151,20 +151,14 @@ class DeviceTable:
         self._events[i] = ev
 
 
-def apply_tile_shape(family: int, X: int, Y: int, tensor_cores=None):
-    """(rows per work item, columns per work item, tag for ``pylo_atile.pad_``) of a FAST2D tensor's apply sweep.
+def apply_tile_shape(family: int, X: int, Y: int):
+    """(rows per work item, columns per work item, tag for ``pylo_atile.pad_``) of a FAST2D tensor's apply sweep on the CUDA
+    cores.
 
-    * tensor-core kernel (AdafacLO family, ``tensor_cores`` true): an item is rt rows x 128 columns, taken by one
-      warpgroup (four per SM); as many rows as possible (the column terms are loaded once per item) while the
-      tensor still yields >= 8 items per warpgroup; tag = rt;
-    * AdafacLO family on the CUDA cores: n_sub sub-tiles of 32 rows in one block of 32..256 columns, as long as
-      possible while the tensor still yields >= 8 items per SM; tag = columns | n_sub << 16;
-    * CELO2 / VeLO: four columns per thread, tag = threads per row.
+    * AdafacLO family: n_sub sub-tiles of 32 rows in one block of 32..256 columns, as long as possible while the tensor
+      still yields >= 8 items per SM; tag = columns | n_sub << 16;
+    * CELO2 / VeLO: four columns per thread, 16 rows per thread (see :func:`packed_rows`), tag = threads per row.
     """
-    if tensor_cores:
-        ncol = (Y + 127) // 128
-        rt = next((r for r in (64, 32, 16) if ((X + r - 1) // r) * ncol >= 8 * L.TC_WORKERS), 8)
-        return rt, 128, rt
     if family == L.FAM_ADAFAC:
         cw = min((256, 128, 64, 32), key=lambda c: ((Y + c - 1) // c * c - Y, -c))
         ncol = (Y + cw - 1) // cw
@@ -172,6 +166,39 @@ def apply_tile_shape(family: int, X: int, Y: int, tensor_cores=None):
         return 32 * n_sub, cw, cw | (n_sub << 16)
     tpr = min((256, 128, 64, 32, 16, 8), key=lambda c: ((Y + 4 * c - 1) // (4 * c) * 4 * c - Y, -c))
     return 16 * (256 // tpr), 4 * tpr, tpr
+
+
+def tensor_core_rows(shapes: Sequence[Tuple[int, int]]) -> int:
+    """Rows of an item of the tensor-core sweep (rows x 128 columns, taken by one warpgroup) over tensors of these (rows,
+    columns): the height that makes the busiest worker's share shortest, over all tensors together; an item's set-up costs
+    about one and a half rows.  86 M ViT-B/16 parameters: 64 rows instead of 8, sweep 2050 -> 1750 us."""
+    xs = np.array([X for X, _ in shapes], dtype=np.int64)
+    cols = np.array([-(-Y // 128) for _, Y in shapes], dtype=np.int64)
+    share = lambda R: -(-int((-(-xs // R) * cols).sum()) // L.TC_WORKERS) * (R + 1.5)
+    return min((64, 32, 16, 8, 4, 2, 1), key=share)
+
+
+def packed_rows(tiles: Sequence[Tuple[int, int, int, int]]) -> int:
+    """Rows per thread of the packed sweep (CELO2, VeLO) over tensors of these (rows, columns, rows and columns of a tile at 16
+    rows per thread): 64 (a tile's start costs about a row's time), fewer while the model does not give every SM its two
+    CTAs several tiles each."""
+    n_items = lambda k: sum(-(-X // (rt * k // 16)) * -(-Y // w) for X, Y, rt, w in tiles)
+    return next((k for k in (64, 32, 16, 8, 4) if n_items(k) >= (16 if k > 16 else 4) * L.SM_COUNT), 2)
+
+
+def apply_items(family: int, tensor_cores: bool, fast, slow) -> np.ndarray:
+    """Work list of the tiled apply sweep: ``fast`` = [(unit, rows, columns)] of the FAST2D units, ``slow`` = [(unit,
+    elements)] of the others, which only the tensor-core kernel takes (as runs of 128 elements, first in the list)."""
+    if tensor_cores:
+        parts = [(u, -(-n // 128), 128, L.TC_GEN_ITEM) for u, n in slow] + [(u, X, Y, 0) for u, X, Y in fast]
+        rt = tensor_core_rows([(X, Y) for _, X, Y, _ in parts])
+        parts = [(u, X, Y, rt, 128, tag | rt) for u, X, Y, tag in parts]
+    else:
+        parts = [(u, X, Y) + apply_tile_shape(family, X, Y) for u, X, Y in fast]
+        if family != L.FAM_ADAFAC:
+            k = packed_rows([(X, Y, rt, w) for _, X, Y, rt, w, _ in parts])
+            parts = [(u, X, Y, rt * k // 16, w, tag | k << 16) for u, X, Y, rt, w, tag in parts]
+    return atile_list([atile_grid(u, -(-X // rt), -(-Y // w), tag) for u, X, Y, rt, w, tag in parts])
 
 
 class LoPlan:
@@ -327,9 +354,9 @@ class LoPlan:
         self.n_units = U
         self.total_elems = int(sum(sizes))
         self._keepalive = []
-        # FAST2D tensors take a tiled apply kernel (see apply_tile_shape); everything else the generic one, or, with
+        # FAST2D tensors take a tiled apply kernel (see apply_items); everything else the generic one, or, with
         # tensor cores, items of the same kernel
-        ctiles, shapes_c = [], []
+        fast = []
         # phase P: item 0 of every unit folds the network, the further ones (and item 0) make the tables' parts
         pitems = [np.zeros((U, 4), dtype=np.int32)]
         pitems[0][:, 0] = np.arange(U)
@@ -342,33 +369,12 @@ class LoPlan:
             # the tensor-core kernel reads the per-row table only, the CUDA-core kernels both
             parts = (X + per - 1) // per + (0 if self.tensor_cores else (Y + per - 1) // per)
             pitems.append(atile_grid(unit_of[i], parts, 1)[1:])
-            shapes_c.append((unit_of[i], X, Y) + apply_tile_shape(family, X, Y, self.tensor_cores))
+            fast.append((unit_of[i], X, Y))
         slow_units = [u for u in range(U) if udesc["mode"][u] != L.MODE_FAST2D]
-        if self.tensor_cores:
-            # The tensor-core kernel takes every tensor: what is not FAST2D as runs of 128 elements.  The height of the
-            # items is the one that makes the busiest worker's share shortest, over all tensors together (the shape's own
-            # rule looks at one tensor): an item's set-up costs about one and a half rows.  86 M ViT-B/16 parameters: 64
-            # rows instead of 8, sweep 2050 -> 1750 us.
-            gen = [(u, (sizes[u] + 127) // 128) for u in slow_units]
-            shapes_c = [(u, X, 128, L.TC_GEN_ITEM) for u, X in gen] + [(u, X, Y, 0) for u, X, Y, *_ in shapes_c]
-            xs = np.array([X for _, X, _, _ in shapes_c])
-            cols = np.array([-(-Y // 128) for _, _, Y, _ in shapes_c])
-            share = lambda R: -(-int((-(-xs // R) * cols).sum()) // L.TC_WORKERS) * (R + 1.5)
-            rt = min((64, 32, 16, 8, 4, 2, 1), key=share)
-            shapes_c = [(u, X, Y, rt, 128, tag | rt) for u, X, Y, tag in shapes_c]
-            slow_units = []
-        elif family != L.FAM_ADAFAC:
-            # rows per thread: 64 (a tile's start costs about a row's time), fewer while the model does not give every SM
-            # its two CTAs several tiles each; the shape's own height is 16 rows
-            n_items = lambda k: sum(-(-X // (rt * k // 16)) * -(-Y // w) for _, X, Y, rt, w, _ in shapes_c)
-            k = next((k for k in (64, 32, 16, 8, 4) if n_items(k) >= (16 if k > 16 else 4) * L.SM_COUNT), 2)
-            shapes_c = [(u, X, Y, rt * k // 16, w, tag | k << 16) for u, X, Y, rt, w, tag in shapes_c]
-        for u, X, Y, rt, width, tag in shapes_c:
-            ctiles.append(atile_grid(u, (X + rt - 1) // rt, (Y + width - 1) // width, tag))
-        self.ctiles = DeviceTable(atile_list(ctiles), self.device)
+        self.ctiles = DeviceTable(apply_items(family, self.tensor_cores, fast, [(u, sizes[u]) for u in slow_units]), self.device)
         self.n_ctiles = len(self.ctiles.host)
         #: how many of them, at the front of the list, are on tensors that are not FAST2D (tensor cores only)
-        self.n_ctiles_gen = int((self.ctiles.host["pad_"] >= L.TC_GEN_ITEM).sum())
+        self.n_ctiles_gen = int((self.ctiles.host["pad_"] >= L.TC_GEN_ITEM).sum()) if self.tensor_cores else 0
         self.pitems = DeviceTable(atile_list(pitems), self.device)
         self.n_pitems = len(self.pitems.host)
         #: the kernel that takes the FAST2D tensors' apply sweep (also the key of its timings in phase_times())
@@ -385,6 +391,7 @@ class LoPlan:
         self._status_view = self._status_host.numpy()
         # the other units' apply sweep: vectors are short and every element costs a whole network, so the tiles are as
         # small as one element per thread where that is what fills the GPU (five 4096-vectors: 104 us as one tile each)
+        slow_units = [] if self.tensor_cores else slow_units
         slow_sizes = [sizes[u] for u in slow_units]
         slow, _ = make_tiles(slow_sizes, tile_elems(sum(slow_sizes), 256, 4 * L.SM_COUNT))
         slow["tensor"] = np.asarray(slow_units, dtype=np.int32)[slow["tensor"]] if len(slow) else slow["tensor"]

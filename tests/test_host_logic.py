@@ -116,20 +116,61 @@ def test_apply_items_cover_a_tensor_exactly_once(family, X, Y, tc):
     """Work items of the tiled apply sweeps: whole rows x column blocks, every element in exactly one item."""
     if tc and family != L.FAM_ADAFAC:
         pytest.skip("tensor-core kernels exist for the AdafacLO family only")
-    rt, width, tag = plan.apply_tile_shape(family, X, Y, tc)
+    rt, width, tag = (plan.tensor_core_rows([(X, Y)]), 128, 0) if tc else plan.apply_tile_shape(family, X, Y)
     n_r, n_c = (X + rt - 1) // rt, (Y + width - 1) // width
     assert (n_r - 1) * rt < X <= n_r * rt and (n_c - 1) * width < Y <= n_c * width
     if tc:
-        assert width == 128 and tag == rt and rt in (8, 16, 32, 64)
-        # as many rows per item as leave every warpgroup at least eight items, never below eight rows
-        workers = L.TC_WORKERS
-        assert rt == 8 or n_r * n_c >= 8 * workers
-        if rt < 64:
-            assert ((X + 2 * rt - 1) // (2 * rt)) * n_c < 8 * workers
+        # the busiest worker's items, each its rows and a row and a half of set-up: no other height makes it shorter
+        share = lambda r: -(-(-(-X // r) * n_c) // L.TC_WORKERS) * (r + 1.5)
+        assert rt in (1, 2, 4, 8, 16, 32, 64) and share(rt) == min(share(r) for r in (1, 2, 4, 8, 16, 32, 64))
     elif family == L.FAM_ADAFAC:
         assert width in (32, 64, 128, 256) and tag & 0xffff == width and rt == 32 * (tag >> 16)
     else:
         assert width == 4 * tag and rt == 16 * (256 // tag)
+
+
+@pytest.mark.parametrize("family,tc", [(L.FAM_ADAFAC, True), (L.FAM_ADAFAC, False), (L.FAM_CELO2, False), (L.FAM_VELO, False)])
+@pytest.mark.parametrize("fast,slow", [
+    ([(1, 64, 128)], []),
+    ([], [127, 129, 1]),
+    ([(3, 129, 300), (2, 40, 4100)], [5, 4096, 70001]),
+    ([(0, 1025, 4096), (1, 1, 4), (2, 33, 260)], [1]),
+])
+def test_apply_work_lists_cover_all_units_exactly_once(family, tc, fast, slow):
+    """The whole list as the kernels decode it (tags, rows per thread, runs of 128 elements)."""
+    slow = [(10 + k, n) for k, n in enumerate(slow)]
+    seen = {u: np.zeros((X, Y), dtype=np.int32) for u, X, Y in fast}
+    runs = {u: np.zeros(n, dtype=np.int32) for u, n in slow if tc}   # the CUDA-core sweeps leave these to another kernel
+    n_gen = 0
+    for k, it in enumerate(plan.apply_items(family, tc, fast, slow)):
+        u, tag = int(it["tensor"]), int(it["pad_"])
+        if tc and tag >= L.TC_GEN_ITEM:
+            assert k == n_gen and it["cb"] == 0, "items on units that are not FAST2D come first"
+            n_gen += 1
+            step = 128 * (tag & 0xffff)
+            runs[u][it["strip"] * step:(it["strip"] + 1) * step] += 1
+            assert it["strip"] * step < len(runs[u])
+            continue
+        if tc:
+            rt, w = tag, 128
+        elif family == L.FAM_ADAFAC:
+            rt, w = 32 * (tag >> 16), tag & 0xffff
+        else:
+            rt, w = (tag >> 16) * (256 // (tag & 0xffff)), 4 * (tag & 0xffff)
+        r, c = int(it["strip"]) * rt, int(it["cb"]) * w
+        assert rt > 0 and r < seen[u].shape[0] and c < seen[u].shape[1]
+        seen[u][r:r + rt, c:c + w] += 1
+    assert all((x == 1).all() for x in list(seen.values()) + list(runs.values()))
+
+
+def test_packed_rows_give_every_sm_its_tiles():
+    """Rows per thread of the packed sweep: the most that still leave sixteen tiles per SM (four below 32 rows)."""
+    for X, Y in ((4096, 4096), (1024, 1024), (300, 260), (16, 8), (50257, 768)):
+        rt, w, _ = plan.apply_tile_shape(L.FAM_VELO, X, Y)
+        items = lambda k: -(-X // (rt * k // 16)) * -(-Y // w)
+        enough = lambda k: items(k) >= (16 if k > 16 else 4) * L.SM_COUNT
+        k = plan.packed_rows([(X, Y, rt, w)])
+        assert k in (2, 4, 8, 16, 32, 64) and (k == 2 or enough(k)) and not any(enough(q) for q in (4, 8, 16, 32, 64) if q > k)
 
 
 def test_mulo_groups_follow_the_infinite_width_shapes():
