@@ -418,7 +418,7 @@ int pylo_b200_velo_tensor_features(const pylo_tensor_desc* descs, int n_local, c
                                    int n_total, const float* rank_onehot, float fraction,
                                    const pylo_velo_loss* lossbuf, float* x_in, void* stream);
 int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, const pylo_velo_loss* lossbuf, void* stream);
-/* The loss buffer's update and features alone: writes loss9[9]. */
+/* The loss buffer's update and features alone, for a host with a front end of its own: writes loss9[9]. */
 int pylo_b200_velo_loss_features(float* means, int32_t* iteration, float* running_min, const float* decays,
                                  const float* loss, float* loss9, void* stream);
 

@@ -9,7 +9,6 @@ sequence of one step.  Nothing here touches tensor values on the host.
 from __future__ import annotations
 
 import ctypes as C
-import math
 from dataclasses import dataclass
 from typing import List, Optional, Sequence, Tuple
 
@@ -627,14 +626,6 @@ def current_stream_ptr() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def f32(x) -> float:
-    """Round a Python float to fp32 the way a torch fp32 tensor element would hold it."""
-    return float(np.float32(x))
-
-
 def one_minus(beta: torch.Tensor) -> List[float]:
     """``1 - beta`` evaluated in fp32, as ``1 - tensor`` does in the reference classes."""
     return [float(x) for x in (1 - beta.detach().to("cpu", torch.float32)).tolist()]
-
-
-INF = math.inf

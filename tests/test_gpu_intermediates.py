@@ -80,3 +80,34 @@ def test_states_and_feature_moments_after_two_steps(family):
             rel = ((got - want).abs() / (want.abs() + 1e-30)).max()
             assert rel < 2e-5, (family, i, float(rel))
         lo_index += 1
+
+
+def test_loss_buffer_entry_point():
+    """pylo_b200_velo_loss_features, the loss buffer alone, against the oracle's buffer in 64 bits: the first step, the two steps
+    without features, a loss that jumps (and is capped) and one that falls."""
+    from oracle import pylo_oracle as O
+    from pylo_b200 import _lib as L
+    from pylo_b200.optim.velo_cuda import init_loss_buffer
+
+    buf, ref = init_loss_buffer(100, "cuda"), O.LossBuffer(100)
+    ref.decays, ref.means, ref.running_min = buf["decays"].cpu().double(), ref.means.double(), ref.running_min.double()
+    out = torch.empty(9, device="cuda")
+    for it, value in enumerate([5.0, 4.5, 4.75, 80.0, 3.0, 2.5, 2.0, 2.25, 1.0]):
+        loss = torch.tensor(value, device="cuda")
+        L.check(L.lib.pylo_b200_velo_loss_features(
+            buf["means"].data_ptr(), buf["iteration"].data_ptr(), buf["running_min"].data_ptr(), buf["decays"].data_ptr(),
+            loss.data_ptr(), out.data_ptr(), torch.cuda.current_stream().cuda_stream), "velo_loss_features")
+        ref.update(value)
+        want = ref.features()
+        assert int(buf["iteration"]) == it + 1
+        assert float((buf["means"].cpu().double() - ref.means).abs().max() / ref.means.abs().max()) < 4 * (it + 1) * 2 ** -24
+        # a corrected mean is a quotient by 1 - decay^k, which carries powf's error (2 units in the last place of a value
+        # near 1) magnified by its own smallness; a feature is a difference of two of them over another difference
+        cor = ref.means / (1 - ref.decays ** (it + 1))
+        e = (4 / (1 - ref.decays ** (it + 1)) + 2 * (it + 1)) * 2 ** -24 * cor.abs()
+        den = torch.clamp(cor[1:] - ref.running_min[:-1], min=1e-8)
+        tol = 2 * (e[:-1] + e[1:]) / den * (1 + (cor[:-1] - ref.running_min[:-1]).abs() / den) + 1e-6
+        assert ((out.cpu().double() - want).abs() <= torch.clamp(tol, max=2.0)).all(), (it, out, want, tol)
+        if it < 2:
+            assert (out == 0).all()
+    assert (tol < 1e-2).any(), "the bound says something"
