@@ -10,7 +10,7 @@ kept out of version control.
 The built modules are used by ``oracle/ref_cuda.py`` as a second checker (the output of the reference's own
 kernels on a GPU) and as the "kernel to beat" timing; never by the product path.
 
-    python oracle/build_ref.py [/path/to/reference]      # default /root/reference; skips what is already built
+    python oracle/build_ref.py /path/to/reference      # or PYLO_REFERENCE=/path/to/reference; skips what is already built
 """
 
 import os
@@ -54,9 +54,9 @@ def build_one(args):
 
 
 def main():
-    ref = sys.argv[1] if len(sys.argv) > 1 else "/root/reference"
-    if not os.path.isdir(os.path.join(ref, "pylo", "csrc")):
-        print(f"no reference checkout at {ref}: nothing built (prebuilt modules in {OUT} are used as they are)")
+    ref = sys.argv[1] if len(sys.argv) > 1 else os.environ.get("PYLO_REFERENCE", "")
+    if not ref or not os.path.isdir(os.path.join(ref, "pylo", "csrc")):
+        print(f"no reference checkout at {ref!r}: nothing built (prebuilt modules in {OUT} are used as they are)")
         return 0
     os.makedirs(OUT, exist_ok=True)
     jobs = [(name, os.path.join(ref, rel)) for name, rel in EXTENSIONS.items()]

@@ -35,7 +35,7 @@ def load(name):
     if name not in _loaded:
         path = os.path.join(REF_DIR, name + ".so")
         if not os.path.exists(path):
-            raise FileNotFoundError(f"{path} is missing: run `python oracle/build_ref.py` where the reference checkout is")
+            raise FileNotFoundError(f"{path} is missing: run `python oracle/build_ref.py /path/to/reference`")
         loader = importlib.machinery.ExtensionFileLoader(name, path)
         spec = importlib.util.spec_from_loader(name, loader)
         mod = importlib.util.module_from_spec(spec)

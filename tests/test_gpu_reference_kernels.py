@@ -33,7 +33,7 @@ def _ref_cuda():
     from oracle import ref_cuda
 
     if not ref_cuda.available():
-        pytest.skip("the reference's CUDA extensions are not built (python oracle/build_ref.py)")
+        pytest.skip("the reference's CUDA extensions are not built (python oracle/build_ref.py /path/to/reference)")
     return ref_cuda
 
 

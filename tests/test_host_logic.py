@@ -256,3 +256,17 @@ def test_every_class_that_reports_a_timeout_can_be_cleared(name):
 
     cls = getattr(optim, name)
     assert callable(cls.check_status) and callable(cls.clear_status)
+
+
+def test_no_source_file_names_a_path_of_one_machine():
+    """Where the reference checkout lies comes from an argument or PYLO_REFERENCE."""
+    import os
+    import re
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for folder, dirs, files in os.walk(root):
+        dirs[:] = [d for d in dirs if not d.startswith((".", "_")) and d not in ("build", "baseline", "gpurun_out")]
+        for name in files:
+            if name.endswith((".py", ".cu", ".cuh", ".h")):
+                text = open(os.path.join(folder, name)).read()
+                assert not re.search(r"/(root|home)/\w", text), os.path.join(folder, name)
