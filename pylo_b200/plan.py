@@ -492,8 +492,9 @@ class LoPlan:
         split = self.tensor_cores and self.n_ctiles >= L.TC_ONE_LAUNCH   # a launch of its own for what is not FAST2D
         rest = int(split and self.n_ctiles_gen > 0) if self.tensor_cores else int(self.n_tiles_slow > 0)
         main = int(self.n_ctiles > (self.n_ctiles_gen if split else 0))
-        apply = [(L.STEP_APPLY, self.apply_kernel, main)]
-        apply.insert(0 if self.tensor_cores else 1, (L.STEP_APPLY_REST, "k_apply_adafac_tc<true>" if self.tensor_cores else "k_apply", rest))
+        other = "k_apply_adafac_tc<true>" if self.tensor_cores else "k_apply"
+        apply = [(L.STEP_APPLY, self.apply_kernel if self.n_ctiles > self.n_ctiles_gen else other, main)]
+        apply.insert(0 if self.tensor_cores else 1, (L.STEP_APPLY_REST, other, rest))
         phases = [(L.STEP_SUMS, "rowcol_sums", (self.n_atiles > 0) + (self.n_gitems > 0)), (L.STEP_FACTORS, "factor_update", 1),
                   (L.STEP_STATE, "state_moments", 1), (L.STEP_MOMENTS, "finalize_moments", int(not self.sum_tiles)),
                   (L.STEP_PREP, "prep_apply", 1)] + apply

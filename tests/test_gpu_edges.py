@@ -335,6 +335,19 @@ def test_timed_phases_are_the_step_that_users_get(family, extra, shapes):
     assert all(len(v) == 1 and v[0] > 0 for v in times.values())
 
 
+def test_a_launch_without_factored_matrices_is_not_reported_as_the_main_kernel():
+    """The benchmark sets the main kernel's mean time against its bytes: a bias' own launch is not one of them."""
+    params = [torch.nn.Parameter(torch.randn(33, device="cuda"))]
+    opt = _make("adafaclo", params)
+    params[0].grad = torch.ones(33, device="cuda")
+    opt.step()
+    plan, = _plans(opt)
+    plan.enable_profile()
+    opt.step()
+    torch.cuda.synchronize()
+    assert plan.apply_kernel not in plan.phase_times() and "k_apply_adafac_tc<true>" in plan.phase_times()
+
+
 @pytest.mark.parametrize("family,extra", [("adafaclo", {}), ("celo2", {"orthogonalize": False})])
 @pytest.mark.parametrize("rows", [8 * 192, 8 * 192 + 8])
 def test_tile_sums_on_both_sides_of_the_launch(family, extra, rows):
