@@ -433,7 +433,7 @@ def measure(args, dev, world, rank, local, headline):
     barrier()
     elapsed_ms = ev[0].elapsed_time(ev[1])
     if hasattr(opt, "check_status"):
-        opt.check_status()  # raises if a bounded wait of the tensor-core kernel ran out during the timed steps
+        opt.check_status()  # raises if a bounded wait of a kernel ran out during the timed steps
     clocks = sampler.stop() if rank == 0 else None
     phase = {}
     launches = getattr(opt, "extra_launches", 0) - extra_launches0

@@ -29,6 +29,10 @@
 //   * the products are issued by one elected lane inside a warp-uniform branch (the warp index is a broadcast
 //     from lane 0), so that their descriptors and tensor-memory addresses live in uniform registers: issued from
 //     a branch on the thread index, each product cost its thread ~52 cycles; this way ~24.
+// What bounds it: one 4096 x 4096 tensor takes 365 us (21.8 ps, 5.75 SM cycles and 378 instructions per element; 28 B of
+// memory traffic); issue slots 54 %, tensor pipe 51 %, ALU pipe 43 %, DRAM 15 % busy: none is full.  A tile's stages are one
+// serial chain (operand stores, products, read-back, split and stores, products, read-back, heads) and four tiles per SM
+// are in flight, one per warpgroup.
 // Every wait on the tensor core is bounded.  A thread whose wait ran out records it in *status (and in *host_status, a word
 // of pinned host memory that the host looks at without asking the device), stops waiting
 // and stops storing (its parameters, and their copies on the peers, keep their old values), and goes on to

@@ -11,9 +11,9 @@ What differs is where the work runs.  The reference does the accumulator
 updates with ~10 torch ops per tensor and then calls a two-kernel extension per
 tensor.  Here every tensor of a param group goes through one multi-tensor
 launch per phase: row/column sums of g^2, factor update, fused EMA + feature
-moments, normaliser folding, network + raw step; then Newton-Schulz, one native
-call per stack of equally shaped matrices, and one fused kernel pair for the
-final normalise-and-apply.
+moments, normaliser folding, network + raw step; then Newton-Schulz, one native call
+per up to eight stacks of equally shaped matrices, and one fused kernel pair
+for the final normalise-and-apply.
 The global-norm clip factor is computed and consumed on the device, so the step
 has no host synchronisation.
 """
