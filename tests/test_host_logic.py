@@ -264,9 +264,9 @@ def test_no_source_file_names_a_path_of_one_machine():
     import re
 
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    for folder, dirs, files in os.walk(root):
-        dirs[:] = [d for d in dirs if not d.startswith((".", "_")) and d not in ("build", "baseline", "gpurun_out")]
-        for name in files:
-            if name.endswith((".py", ".cu", ".cuh", ".h")):
-                text = open(os.path.join(folder, name)).read()
-                assert not re.search(r"/(root|home)/\w", text), os.path.join(folder, name)
+    paths = [os.path.join(root, name) for name in os.listdir(root)]
+    for top in ("include", "oracle", "perf", "pylo_b200", "tests"):
+        paths += [os.path.join(folder, name) for folder, _, files in os.walk(os.path.join(root, top)) for name in files]
+    for path in paths:
+        if path.endswith((".py", ".cu", ".cuh", ".h")):
+            assert not re.search(r"/(root|home)/\w", open(path).read()), path
