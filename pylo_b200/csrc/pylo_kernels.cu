@@ -8,6 +8,7 @@
 // All reductions go through fixed-slot partials and fixed-order final sums, so
 // results are bit-reproducible from run to run (no floating-point atomics).
 
+#include <stddef.h>
 #include <string.h>
 
 #include <mutex>
@@ -1335,6 +1336,7 @@ __global__ void __launch_bounds__(NT, CC_CTAS_PER_SM) k_apply_adafac_cols(const 
 #include "pylo_apply_tc.cuh"
 #include "pylo_ns_gemm.cuh"
 #include "pylo_ns_f16.cuh"
+#include "pylo_ns_cluster.cuh"
 
 // ================================================================================================
 // Phase C for CELO2 / ELO_CELO2 / VeLO on FAST2D tensors: packed kernel.
@@ -2076,7 +2078,7 @@ static void launch_clusters(void (*kernel)(P...), dim3 grid, dim3 block, int clu
     attr[n++].val.programmaticStreamSerializationAllowed = 1;
   }
   t_plain_next = false;
-  if (cluster > 1) {
+  if (cluster >= 1) {
     attr[n].id = cudaLaunchAttributeClusterDimension;
     attr[n].val.clusterDim.x = cluster;
     attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
@@ -2105,6 +2107,19 @@ static int allow_dynamic_smem(K kernel, int bytes, bool (&flags)[PYLO_MAX_DEVICE
   if (e != cudaSuccess) return (int)e;
   if (dev >= 0 && dev < PYLO_MAX_DEVICES && flags[dev]) return 0;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return (int)e;
+  if (dev >= 0 && dev < PYLO_MAX_DEVICES) flags[dev] = true;
+  return 0;
+}
+
+// The same for clusters of more than eight CTAs.
+template <class K>
+static int allow_wide_clusters(K kernel, bool (&flags)[PYLO_MAX_DEVICES]) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return (int)e;
+  if (dev >= 0 && dev < PYLO_MAX_DEVICES && flags[dev]) return 0;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return (int)e;
   if (dev >= 0 && dev < PYLO_MAX_DEVICES) flags[dev] = true;
   return 0;
@@ -2170,6 +2185,66 @@ static int state_moments_launch(const pylo_tensor_desc* descs, const pylo_tile* 
   launch(k_state_moments<FAM, true>, grid_for(n_tiles, 2), NT, sizeof(PipeSmem), s, descs, tiles, n_tiles, reverse, prm);
   t_plain_next = true;
   return 0;
+}
+
+static long long ns_small_floats(int rows, int cols) {
+  const long long r = rows < cols ? rows : cols, c = rows < cols ? cols : rows;
+  return 2 * r * (c + 1) + 2 * r * (r + 1);
+}
+// One CTA does about 1e5 FMAs per microsecond: beyond a few million, or where it does not fit into shared memory, the
+// tensor-core chain (15 launches of 4 us at least) is faster.
+static bool ns_is_small(int rows, int cols, int iters) {
+  const long long r = rows < cols ? rows : cols, c = rows < cols ? cols : rows;
+  return r <= 64 && iters * (2 * r * r * c + r * r * r) <= 3000000 && ns_small_floats(rows, cols) * 4 <= 200 * 1024;
+}
+
+// How a stack is run: 0, by single CTAs in plain fp32; 1 to 16, by so many CTAs a matrix (k_ns_cluster); -1, as a chain of
+// launches.  What fits clusters is faster there for any number of matrices (us per chain, launches / clusters, two of each run
+// within 1 %: 128 x 784 155 / 64, 128 x 3072 184 / 83, 24 x 128 x 1000 288 / 140, 48 x 128 x 1000 413 / 280, 400 x 128 x 128
+// 833 / 120, 300 x 64 x 256 642 / 205), with as few CTAs a matrix as hold it (48 matrices of 128 x 128 to 128 x 512, with
+// up to 192 columns per CTA 73, with 128 125).
+static int ns_parts(int rows, int cols, int iters) {
+  if (ns_is_small(rows, cols, iters)) return 0;
+  const int r = rows < cols ? rows : cols, c = rows < cols ? cols : rows;
+  if (r > NC_SIDE || c > 16 * NC_COLS) return -1;
+  int parts = 1;
+  while ((c + parts - 1) / parts > NC_COLS) parts *= 2;
+  return parts;
+}
+// Whether a stack goes into the launch of clusters: what they take, and, where there is such a launch, a few small matrices.
+static bool ns_any_clusters(const pylo_ns_desc* descs, int n) {
+  for (int k = 0; k < n; ++k) if (ns_parts(descs[k].rows, descs[k].cols, descs[k].iters) > 0) return true;
+  return false;
+}
+static bool ns_in_clusters(const pylo_ns_desc& d, bool clusters) {
+  const int parts = ns_parts(d.rows, d.cols, d.iters);
+  return parts > 0 || (clusters && parts == 0 && d.batch <= 16);
+}
+// One launch: clusters as large as the most CTAs that share a matrix.
+template <int COLS>
+static int nc_launch(const nc_group& grp, int ctas, int cluster, int* status, cudaStream_t s) {
+  static bool configured[PYLO_MAX_DEVICES] = {}, wide[PYLO_MAX_DEVICES] = {};
+  constexpr int smem = (int)sizeof(NcSmem<COLS>) + 1024;   // room to start the boxes on a 1024-byte boundary
+  if (int rc = allow_dynamic_smem(k_ns_cluster<COLS>, smem, configured)) return rc;
+  if (cluster > 8)
+    if (int rc = allow_wide_clusters(k_ns_cluster<COLS>, wide)) return rc;
+  launch_clusters(k_ns_cluster<COLS>, ctas, NC_THREADS, cluster, smem, s, grp, status);
+  return launch_status();
+}
+static int ns_clusters(nc_group& grp, int* status, cudaStream_t s) {
+  int cluster = 1;
+  for (int k = 0; k < grp.n; ++k) cluster = max(cluster, grp.p[k].parts);
+  long long ctas = 0;
+  bool wide = false;   // whether 128 columns per CTA (a register less in three: 64 instead of 69 us for 128 x 784) do not do
+  for (int k = 0; k < grp.n; ++k) {
+    nc_item& p = grp.p[k];
+    const int c = max(p.rows, p.cols);
+    p.cta0 = (int)ctas;
+    ctas += ((long long)p.batch * max(1, p.parts) + cluster - 1) / cluster * cluster;
+    wide |= p.parts ? (c + p.parts - 1) / p.parts > 128 : ns_small_floats(p.rows, p.cols) * 4 > (long long)offsetof(NcSmem<128>, red);
+  }
+  if (ctas > 0x7fffffff) return -1;
+  return wide ? nc_launch<NC_COLS>(grp, (int)ctas, cluster, status, s) : nc_launch<128>(grp, (int)ctas, cluster, status, s);
 }
 
 extern "C" {
@@ -2431,17 +2506,6 @@ int pylo_b200_transpose(const float* src, float* dst, int rows, int cols, int ld
 // ------------------------------------------------------------------------------------------------
 // Newton-Schulz chain
 // ------------------------------------------------------------------------------------------------
-static long long ns_small_floats(int rows, int cols) {
-  const long long r = rows < cols ? rows : cols, c = rows < cols ? cols : rows;
-  return 2 * r * (c + 1) + 2 * r * (r + 1);
-}
-// One CTA does about 1e5 FMAs per microsecond: beyond a few million, or where it does not fit into shared memory, the
-// tensor-core chain (15 launches of 4 us at least) is faster.
-static bool ns_is_small(int rows, int cols, int iters) {
-  const long long r = rows < cols ? rows : cols, c = rows < cols ? cols : rows;
-  return r <= 64 && iters * (2 * r * r * c + r * r * r) <= 3000000 && ns_small_floats(rows, cols) * 4 <= 200 * 1024;
-}
-
 struct NsWork {   // byte offsets into the workspace, every buffer on a 1024-byte boundary
   int64_t xp[2], ap, bp, a, x, part, inv, total;
   int r, c, ldx, lda_p, lda, slices;
@@ -2472,7 +2536,7 @@ static NsWork ns_work(int rows, int cols, int batch) {
 
 int64_t pylo_b200_newton_schulz_workspace(int rows, int cols, int batch, int iters) {
   if (rows <= 0 || cols <= 0 || batch <= 0 || iters < 0) return -1;
-  return ns_is_small(rows, cols, iters) ? 0 : ns_work(rows, cols, batch).total;
+  return ns_parts(rows, cols, iters) >= 0 ? 0 : ns_work(rows, cols, batch).total;
 }
 
 typedef CUresult (*TensorMapEncode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -2581,27 +2645,51 @@ int pylo_b200_newton_schulz(const pylo_ns_desc* descs, int n, int* status, void*
     const pylo_ns_desc& d = descs[k];
     CHECK_ARG(d.x && d.out && d.x != d.out && d.rows > 0 && d.cols > 0 && d.batch > 0 && d.iters >= 1 && d.iters == descs[0].iters);
     CHECK_ARG(d.cols % 4 != 0 || (((uintptr_t)d.x | (uintptr_t)d.out) & 15) == 0);   // rows are moved in 16-byte pieces where they can
-    if (!ns_is_small(d.rows, d.cols, d.iters)) CHECK_ARG(d.work && ((uintptr_t)d.work & 255) == 0 && d.work_bytes >= ns_work(d.rows, d.cols, d.batch).total);
+    if (ns_parts(d.rows, d.cols, d.iters) < 0) CHECK_ARG(d.work && ((uintptr_t)d.work & 255) == 0 && d.work_bytes >= ns_work(d.rows, d.cols, d.batch).total);
   }
+  // what clusters take goes first, and with it, beside it, what single CTAs take
   const pylo_ns_desc* group[NF_GROUP];
   int m = 0;
+  nc_group small = {};
+  small.iters = n ? descs[0].iters : 0;
+  auto run_clusters = [&]() { const int rc = small.n ? ns_clusters(small, status, s) : 0; small.n = 0; return rc; };
+  const bool clusters = ns_any_clusters(descs, n);
   for (int k = 0; k < n; ++k) {
     const pylo_ns_desc& d = descs[k];
-    if (ns_is_small(d.rows, d.cols, d.iters)) {
+    const int parts = ns_parts(d.rows, d.cols, d.iters);
+    if (ns_in_clusters(d, clusters)) {
+      small.p[small.n++] = {d.x, d.out, d.rows, d.cols, d.batch, parts, 0, d.c0, d.c1, d.c2, d.eps};
+      if (small.n == NF_GROUP)
+        if (int rc = run_clusters()) return rc;
+    } else if (parts == 0) {
       static bool configured[PYLO_MAX_DEVICES] = {};
       if (int rc = allow_dynamic_smem(k_ns_small, 200 * 1024, configured)) return rc;
       launch(k_ns_small, d.batch, NT, (size_t)ns_small_floats(d.rows, d.cols) * 4, s, d.x, d.out, d.rows, d.cols, d.iters, d.c0, d.c1, d.c2, d.eps);
-      continue;
-    }
-    group[m++] = &d;
-    if (m == NF_GROUP) {
-      if (int rc = ns_chain(group, m, status, s)) return rc;
-      m = 0;
+    } else {
+      group[m++] = &d;
+      if (m == NF_GROUP) {
+        if (int rc = ns_chain(group, m, status, s)) return rc;
+        m = 0;
+      }
     }
   }
+  if (int rc = run_clusters()) return rc;
   if (m)
     if (int rc = ns_chain(group, m, status, s)) return rc;
   return launch_status();
+}
+
+int pylo_b200_newton_schulz_launches(const pylo_ns_desc* descs, int n) {
+  CHECK_ARG(descs && n >= 0);
+  const bool clusters = ns_any_clusters(descs, n);
+  int in_clusters = 0, single = 0, chains = 0;
+  for (int k = 0; k < n; ++k) {
+    if (ns_in_clusters(descs[k], clusters)) ++in_clusters;
+    else if (ns_parts(descs[k].rows, descs[k].cols, descs[k].iters) == 0) ++single;
+    else ++chains;
+  }
+  auto groups = [](int m) { return (m + NF_GROUP - 1) / NF_GROUP; };
+  return groups(in_clusters) + single + groups(chains) * (2 + 3 * (n ? descs[0].iters : 0));
 }
 
 int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles,

@@ -590,34 +590,32 @@ __global__ void __launch_bounds__(NT) k_ns_split(const __grid_constant__ nf_prep
 // A tile of the tensor-core kernel would be mostly padding (a 16 x 16 slice of a ViT patch embedding fills 1/64 of it), and
 // fifteen launches would cost more than the arithmetic.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NT) k_ns_small(const float* __restrict__ x, float* __restrict__ out, int rows, int cols, int iters,
-                                                 float c0, float c1, float c2, float eps) {
-  pdl_begin();
-  extern __shared__ __align__(16) float ns_s[];
-  __shared__ float s_red[40];
+// One matrix by a CTA of THREADS threads.  smem: ns_small_floats(rows, cols) floats of shared memory, s_red: 33.
+template <int THREADS>
+__device__ __forceinline__ void ns_small_body(const float* __restrict__ src, float* __restrict__ dst, int rows, int cols, int iters,
+                                              float c0, float c1, float c2, float eps, float* smem, float* s_red) {
   const bool tall = rows > cols;
   const int r = tall ? cols : rows, c = tall ? rows : cols, n = rows * cols, pitch = c + 1, pa = r + 1;
-  float* X = ns_s;
+  float* X = smem;
   float* Y = X + r * pitch;
   float* A = Y + r * pitch;
   float* B = A + r * pa;
-  const float* src = x + (long long)blockIdx.x * n;
   const int tid = threadIdx.x;
   float acc = 0.f;
-  for (int i = tid; i < n; i += NT) {
+  for (int i = tid; i < n; i += THREADS) {
     const float v = src[i];
     acc = fmaf(v, v, acc);
     const int a = i / cols, b = i - a * cols;
     X[tall ? b * pitch + a : a * pitch + b] = v;
   }
   const float f = 1.0f / (sqrtf(block_sum(acc, s_red)) + eps);
-  for (int i = tid; i < r * pitch; i += NT) if (i % pitch < c) X[i] *= f;
+  for (int i = tid; i < r * pitch; i += THREADS) if (i % pitch < c) X[i] *= f;
   // lanes per entry of a (r x r): as many as keep all threads busy
   int L = 1;
-  while (L < 32 && r * r * L * 2 <= NT) L *= 2;
+  while (L < 32 && r * r * L * 2 <= THREADS) L *= 2;
   __syncthreads();
   for (int it = 0; it < iters; ++it) {
-    for (int p0 = 0; p0 < r * r; p0 += NT / L) {       // the same trip count for all threads
+    for (int p0 = 0; p0 < r * r; p0 += THREADS / L) {       // the same trip count for all threads
       const int p = p0 + tid / L, i = p / r, j = p - i * r;
       float s = 0.f;
       if (p < r * r)
@@ -626,14 +624,14 @@ __global__ void __launch_bounds__(NT) k_ns_small(const float* __restrict__ x, fl
       if (p < r * r && tid % L == 0) A[i * pa + j] = s;
     }
     __syncthreads();
-    for (int p = tid; p < r * r; p += NT) {
+    for (int p = tid; p < r * r; p += THREADS) {
       const int i = p / r, j = p - i * r;
       float s = 0.f;
       for (int k = 0; k < r; ++k) s = fmaf(A[i * pa + k], A[k * pa + j], s);
       B[i * pa + j] = fmaf(c2, s, c1 * A[i * pa + j]);
     }
     __syncthreads();
-    for (int p = tid; p < r * c; p += NT) {
+    for (int p = tid; p < r * c; p += THREADS) {
       const int i = p / c, k = p - i * c;
       float s = c0 * X[i * pitch + k];
       for (int j = 0; j < r; ++j) s = fmaf(B[i * pa + j], X[j * pitch + k], s);
@@ -642,9 +640,16 @@ __global__ void __launch_bounds__(NT) k_ns_small(const float* __restrict__ x, fl
     __syncthreads();
     float* t = X; X = Y; Y = t;
   }
-  float* dst = out + (long long)blockIdx.x * n;
-  for (int i = tid; i < n; i += NT) {
+  for (int i = tid; i < n; i += THREADS) {
     const int a = i / cols, b = i - a * cols;
     dst[i] = X[tall ? b * pitch + a : a * pitch + b];
   }
+}
+__global__ void __launch_bounds__(NT) k_ns_small(const float* __restrict__ x, float* __restrict__ out, int rows, int cols, int iters,
+                                                 float c0, float c1, float c2, float eps) {
+  pdl_begin();
+  extern __shared__ __align__(16) float ns_s[];
+  __shared__ float s_red[40];
+  const long long at = (long long)blockIdx.x * rows * cols;
+  ns_small_body<NT>(x + at, out + at, rows, cols, iters, c0, c1, c2, eps, ns_s, s_red);
 }

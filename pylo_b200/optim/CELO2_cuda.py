@@ -309,15 +309,16 @@ class _Celo2Family(Optimizer):
                         # small models: results and workspaces stay with the plan; large ones take them from the allocator
                         # on every step, so that the training step can have the memory in between
                         group["kept"] = results
-                newton_schulz_native([part for part, _ in group["parts"]], [r for r, _ in results], [w for _, w in results],
-                                     self.ns_coeffs, self.ns_iters, self.ns_eps, status, stream)
+                launches = newton_schulz_native([part for part, _ in group["parts"]], [r for r, _ in results], [w for _, w in results],
+                                                self.ns_coeffs, self.ns_iters, self.ns_eps, status, stream)
                 outs = [r for r, _ in results]
             else:
                 args = (self.ns_coeffs, self.ns_iters, self.ns_eps)
                 outs = [(newton_schulz_tc(part, *args, status, stream) if self.ns_precision == "3xtf32"
                          else newton_schulz(part, *args)).contiguous() for part, _ in group["parts"]]
+                launches = 3 * self.ns_iters
             if self.ns_precision == "3xtf32":
-                self.extra_launches += 3 * self.ns_iters
+                self.extra_launches += launches
             keep += outs
             for res, (part, members) in zip(outs, group["parts"]):
                 at, n = res.data_ptr(), 4 * part[0].numel()

@@ -119,7 +119,8 @@ def newton_schulz_bounded(coeffs, iters: int) -> bool:
 
 def newton_schulz_native(stacks, outs, works, coeffs, iters, eps, status, stream):
     """One native call for the chains of several stacks of matrices (contiguous, 16-byte aligned): ``outs`` the results,
-    ``works`` uint8 tensors of at least :func:`newton_schulz_workspace` bytes (None where that is 0)."""
+    ``works`` uint8 tensors of at least :func:`newton_schulz_workspace` bytes (None where that is 0).  Returns the number of
+    launches."""
     descs = (L.NsDesc * len(stacks))()
     for d, x, out, work in zip(descs, stacks, outs, works):
         d.x, d.out = x.data_ptr(), out.data_ptr()
@@ -129,6 +130,7 @@ def newton_schulz_native(stacks, outs, works, coeffs, iters, eps, status, stream
         if work is not None:
             d.work, d.work_bytes = work.data_ptr(), work.numel()
     L.check(L.lib.pylo_b200_newton_schulz(descs, len(stacks), status.data_ptr() if status is not None else None, stream), "newton_schulz")
+    return int(L.lib.pylo_b200_newton_schulz_launches(descs, len(stacks)))
 
 
 def newton_schulz_buffers(x: torch.Tensor, iters: int):

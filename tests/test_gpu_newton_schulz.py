@@ -140,3 +140,36 @@ def test_transpose_kernel():
         out = torch.full((shape[0], shape[2], shape[1]), float("nan"), device="cuda")
         _transpose(x, out, torch.cuda.current_stream().cuda_stream)
         assert torch.equal(out, x.transpose(1, 2))
+
+
+# a cluster's chain: sides at and beside the edges of CTAs (192 columns), of 32 rows and of clusters of 1 to 16, odd pitches,
+# wide and tall; several stacks in one launch, some CTAs of the last cluster idle, a single-CTA matrix beside them
+CLUSTERED = [[(65, 65)], [(128, 128)], [(128, 192)], [(5, 97, 193)], [(33, 769)], [(127, 1537)], [(128, 3072)], [(3071, 128)],
+             [(3, 128, 100), (128, 3000), (10, 128), (1001, 126), (2, 40, 500)]]
+
+
+@pytest.mark.parametrize("shapes", CLUSTERED, ids=[str(s[0]) for s in CLUSTERED])
+@pytest.mark.parametrize("coeffs,iters", [(COEFFS, 5), ((1.5, -0.5, 0.0), 3)])
+def test_chain_in_one_launch(shapes, coeffs, iters):
+    """Against fp64, as close as the fp32 chain (both round every entry of three products a round to 2^-22 or less of its
+    largest terms: the same bound as for the chain of launches); and what a matrix gives does not depend on its company."""
+    from pylo_b200.optim import _common as K
+
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    xs = [torch.randn(s, device="cuda", generator=gen) * torch.exp(torch.randn(s[:-1] + (1,), device="cuda", generator=gen)) for s in shapes]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def run(stacks):
+        bufs = [K.newton_schulz_buffers(x, iters) for x in stacks]
+        assert all(work is None for _, work in bufs)   # no workspace: none of them goes through the chain of launches
+        assert K.newton_schulz_native(stacks, [o for o, _ in bufs], [None] * len(bufs), coeffs, iters, 1e-8, status, stream) == 1
+        return [o for o, _ in bufs]
+
+    for x, out in zip(xs, run(xs)):
+        exact = K.newton_schulz(x.double(), coeffs, iters)
+        e32 = float((K.newton_schulz(x, coeffs, iters).double() - exact).norm() / exact.norm())
+        assert float((out.double() - exact).norm() / exact.norm()) < max(4 * e32, 1e-5)
+        if max(x.shape) > 128:
+            assert torch.equal(run([x])[0], out)
+    assert int(status.item()) == 0
