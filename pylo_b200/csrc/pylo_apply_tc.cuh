@@ -281,16 +281,16 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
       for (int e = col; e < 32 * 8 * KSTEPS; e += 128) {
         const int n = e & 31, kk = e >> 5;
         float w = 0.f;
-        if (kk < 13) w = d.wfold[L::W1 + kk * 32 + n];
-        else if (kk < 16) w = d.wfold[L::W1 + (kk + 12) * 32 + n];
+        if (kk < 13) w = __ldg(d.wfold + L::W1 + kk * 32 + n);
+        else if (kk < 16) w = __ldg(d.wfold + L::W1 + (kk + 12) * 32 + n);
         else if (GEN) {
-          if (kk < 28) w = d.wfold[L::W1 + (F::R + kk - 16) * 32 + n];
+          if (kk < 28) w = __ldg(d.wfold + L::W1 + (F::R + kk - 16) * 32 + n);
         }
-        else if (kk < 19) w = d.wfold[L::W1 + (kb + kk - 16) * 32 + n];
-        else if (kk < 22) w = d.wfold[L::W1 + (krb + kk - 19) * 32 + n];
+        else if (kk < 19) w = __ldg(d.wfold + L::W1 + (kb + kk - 16) * 32 + n);
+        else if (kk < 22) w = __ldg(d.wfold + L::W1 + (krb + kk - 19) * 32 + n);
         float hi = tf32_hi(w), lo = w - hi;
         if (GEN && (kk == 28 || kk == 29)) {
-          const float b = d.wfold[L::B1 + n];
+          const float b = __ldg(d.wfold + L::B1 + n);
           hi = kk == 28 ? tf32_hi(b) : b - tf32_hi(b);
           lo = 0.f;
         }
@@ -299,17 +299,17 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
       }
       for (int e = col; e < 32 * 32; e += 128) {
         const int n = e & 31, k = e >> 5;
-        const float w = d.wfold[L::W2 + k * 32 + n], hi = tf32_hi(w);
+        const float w = __ldg(d.wfold + L::W2 + k * 32 + n), hi = tf32_hi(w);
         sm.b2[tc_b_index(n, k, TC_LBO64)] = hi;
         sm.b2[tc_b_index(32 + n, k, TC_LBO64)] = w - hi;
       }
       for (int e = col; e < 32 * 8; e += 128) {
         const int n = e & 31, k = e >> 5;
-        const float w = d.wfold[L::B2 + n], hi = tf32_hi(w);
+        const float w = __ldg(d.wfold + L::B2 + n), hi = tf32_hi(w);
         sm.b2bias[tc_b_index(n, k)] = k == 0 ? hi : (k == 1 ? w - hi : 0.f);
       }
-      if (col < 64) sm.w3[col] = d.wfold[L::W3P + col];
-      if (col < 2) sm.w3[64 + col] = d.wfold[L::B3 + col];
+      if (col < 64) sm.w3[col] = __ldg(d.wfold + L::W3P + col);
+      if (col < 2) sm.w3[64 + col] = __ldg(d.wfold + L::B3 + col);
       loaded = ct.tensor;
     }
     // per-item constants: in registers for all rows of the item
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
     const float* __restrict__ vp = d.v;
     const Peers peers = load_peers(d);
     const float gs = grad_scale_of(d, prm);
-    const Fin fin{d.exp_mult, d.step_mult, d.wd, d.lr, d.wfold[L::SC + 1], 1.0f, prm.wd_mode};
+    const Fin fin{d.exp_mult, d.step_mult, d.wd, d.lr, __ldg(d.wfold + L::SC + 1), 1.0f, prm.wd_mode};
     const bool plain = plain_grad(gs, prm);
     // GEN: the accumulators of the "r" and "c" vectors and the "r" factor (the "c" factor is a function of its accumulator)
     const bool vec1d = d.mode == PYLO_MODE_VEC1D, r_is_a = d.r_is_a != 0;
@@ -334,11 +334,11 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
     float fb0 = 0.f, fb1 = 0.f, fb2 = 0.f;
     uint32_t chi[8], clo[8];
     if constexpr (!GEN) {
-      fb0 = d.f_b[yc]; fb1 = d.f_b[Y + yc]; fb2 = d.f_b[2 * (int64_t)Y + yc];
+      fb0 = __ldg(d.f_b + yc); fb1 = __ldg(d.f_b + Y + yc); fb2 = __ldg(d.f_b + 2 * (int64_t)Y + yc);
       // the six features of this thread's column, high parts (then two ones) and low parts (then two zeros)
 #pragma unroll
       for (int j = 0; j < 6; ++j) {
-        const float r = colok ? d.fac_b[(int64_t)(j % 3) * Y + yc] : 0.f;
+        const float r = colok ? __ldg(d.fac_b + (int64_t)(j % 3) * Y + yc) : 0.f;
         const float v = colok ? (j < 3 ? r : rsqrtf(r + 1e-8f)) : 0.f;
         const float hi = tf32_hi(v);
         chi[j] = __float_as_uint(hi);

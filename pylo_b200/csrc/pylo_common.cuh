@@ -179,21 +179,46 @@ __device__ __forceinline__ float block_sum(float v, float* s_red) {
   return s_red[32];
 }
 
+// Sums of accumulators FIRST .. FIRST + WIDTH - 1 over the lanes of a warp, lane l (and l + WIDTH, ...) ending with that of
+// accumulator FIRST + l % WIDTH: after the step of offset o a lane holds the o of them whose index agrees with its own in that
+// bit.  WIDTH - 1 shuffles (and one per halving of the lanes left), where one sum after the other takes five each.
+template <int FIRST, int WIDTH, int N>
+__device__ __forceinline__ float warp_fold(const float (&acc)[N]) {
+  const int lane = threadIdx.x & 31;
+  float a[WIDTH];
+#pragma unroll
+  for (int j = 0; j < WIDTH; ++j) a[j] = FIRST + j < N ? acc[FIRST + j < N ? FIRST + j : 0] : 0.f;
+#pragma unroll
+  for (int o = WIDTH / 2; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int j = 0; j < o; ++j) {
+      const float keep = up ? a[j + o] : a[j], give = up ? a[j] : a[j + o];
+      a[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+#pragma unroll
+  for (int o = WIDTH; o < 32; o <<= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+  return a[0];
+}
+
 // Deterministic block reduction of N per-thread accumulators; thread j < N writes out[j].
-// s_red: NWARP * N floats.
-template <int N>
+// s_red: WARPS * N floats.
+template <int N, int WARPS = NWARP>
 __device__ __forceinline__ void block_reduce_store(float (&acc)[N], float* s_red, float* out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    const float v = warp_sum(acc[j]);
-    if (lane == 0) s_red[warp * N + j] = v;
+  static_assert(N > 16 && N <= 40, "one fold of 32, and one of 8");
+  const float v = warp_fold<0, 32>(acc);
+  if (lane < N) s_red[warp * N + lane] = v;
+  if constexpr (N > 32) {
+    const float w = warp_fold<32, 8>(acc);
+    if (lane < N - 32) s_red[warp * N + 32 + lane] = w;
   }
   __syncthreads();
   if (threadIdx.x < N) {
     float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < NWARP; ++w) t += s_red[w * N + threadIdx.x];
+    for (int w = 0; w < WARPS; ++w) t += s_red[w * N + threadIdx.x];
     out[threadIdx.x] = t;
   }
   __syncthreads();
