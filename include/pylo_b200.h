@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define PYLO_B200_ABI_VERSION 12
+#define PYLO_B200_ABI_VERSION 13
 
 /* optimizer families (which feature set / network geometry a launch uses) */
 #define PYLO_FAM_ADAFAC 0 /* AdafacLO_CUDA, ELO_CUDA: 28+11 features, 39-32-32-2 */
@@ -51,6 +51,7 @@ extern "C" {
 #define PYLO_TILE_ELEMS 16384 /* elements per element-wise tile (at most) */
 #define PYLO_A_COLS 1024      /* columns per row/column-sum tile */
 #define PYLO_WFOLD_STRIDE 2432 /* floats reserved per tensor for the folded network */
+#define PYLO_SMALL_FLOATS 52224 /* shared memory of pylo_b200_small_front, in floats */
 #define PYLO_MAX_PEERS 7       /* other GPUs of one box */
 
 /*
@@ -238,6 +239,14 @@ int pylo_b200_factor_update(const pylo_tensor_desc* descs, int n_tensors, const 
  * lstm_features_for_tensor needs (velo_cuda.py:213-252). */
 int pylo_b200_state_moments(const pylo_tensor_desc* descs, const pylo_tile* tiles, int n_tiles,
                             int reverse, const pylo_step_params* prm, void* stream);
+
+/* Phases A, A2 and B of a small model in one launch, a cluster of 1, 2, 4, 8 or 16 CTAs per tensor.  Every tensor is VEC1D, or a
+ * contiguous matrix (O = M = I = 1) whose row_col_mean is over the whole vector (rcm_pre = 3) or over the decays (rcm_pre = 1,
+ * rcm_A = 3); the units are the tensors.  slice: the most elements of a CTA's ceil(X / cluster) rows, up to 8192 (of a vector:
+ * any); rows, cols: the most such rows and columns; 6 slice + 4 rows + 5 cols, each rounded up to 4, fit PYLO_SMALL_FLOATS.
+ * Every tensor leaves `cluster` rows of tile_part, so desc.n_tiles has to be that. */
+int pylo_b200_small_front(const pylo_tensor_desc* descs, int n_tensors, int cluster, int slice, int rows, int cols,
+                          const pylo_step_params* prm, void* stream);
 
 /* Phase B2, one CTA per tensor: fixed-order reduction of the tile partials into desc.sums. */
 int pylo_b200_finalize_moments(const pylo_tensor_desc* descs, int n_tensors, void* stream);
@@ -448,6 +457,8 @@ typedef struct pylo_step_plan {
   int32_t n_tensors, n_units, n_atiles, n_gitems, n_pitems, n_ctiles, n_ctiles_gen, n_tiles, n_tiles_slow, tensor_cores;
   int32_t sum_tiles; /* 1: leave finalize_moments out and let prep_apply add up the tile partials, for units of up to
                         about 200 tiles (VELO, of any size: velo_tensor_features does it) */
+  int32_t small_cluster, small_slice, small_rows, small_cols; /* small_cluster > 0: SUMS, FACTORS and STATE, asked for together,
+                        are one launch of pylo_b200_small_front */
   int32_t pad_;
 } pylo_step_plan;
 int pylo_b200_step(const pylo_step_plan* plan, const pylo_step_params* prm, int phases, void* stream);

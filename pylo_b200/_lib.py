@@ -17,7 +17,7 @@ TILE_ELEMS = 16384
 A_COLS = 1024
 PREP_TABLE = 2048  # table entries (rows x hidden units) per item of pylo_b200_prep_apply
 WFOLD_STRIDE = 2432
-ABI_VERSION = 12
+ABI_VERSION = 13
 
 FAM_ADAFAC, FAM_CELO2, FAM_VELO = 0, 1, 2
 MODE_FAST2D, MODE_GENERIC, MODE_VEC1D = 0, 1, 2
@@ -100,7 +100,8 @@ class StepPlan(C.Structure):
     _fields_ = [(name, C.c_void_p) for name in (
         "tdesc", "desc", "atiles", "gitems", "pitems", "ctiles", "tiles", "tiles_slow", "status", "host_status")] + [
         (name, C.c_int32) for name in ("n_tensors", "n_units", "n_atiles", "n_gitems", "n_pitems", "n_ctiles", "n_ctiles_gen",
-                                       "n_tiles", "n_tiles_slow", "tensor_cores", "sum_tiles", "pad_")]
+                                       "n_tiles", "n_tiles_slow", "tensor_cores", "sum_tiles", "small_cluster", "small_slice",
+                                       "small_rows", "small_cols", "pad_")]
 
 
 class PyloLibError(RuntimeError):
@@ -129,6 +130,7 @@ def _load():
         "pylo_b200_rowcol_sums": [vp, vp, i32, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_factor_update": [vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_state_moments": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
+        "pylo_b200_small_front": [vp, i32, i32, i32, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_finalize_moments": [vp, i32, vp],
         "pylo_b200_prep_apply": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
@@ -171,6 +173,7 @@ STEP_FRONT = STEP_SUMS | STEP_FACTORS | STEP_STATE | STEP_MOMENTS
 STEP_BACK = STEP_PREP | STEP_APPLY | STEP_APPLY_REST
 TC_ONE_LAUNCH = 8 * TC_WORKERS  # items below which one launch of the tensor-core kernel takes both kinds of items
 BULK_COPY_ELEMS = 1 << 26  # FAST2D elements from which the state sweep reads through a ring of bulk copies
+SMALL_SLICE, SMALL_FLOATS = 8192, 52224   # of pylo_b200_small_front: elements of a CTA's rows, floats of shared memory
 STATIC_SCRATCH_TILES = 65536
 ERR_STATIC_SCRATCH_TOO_SMALL = -4
 

@@ -10,7 +10,7 @@ INCLUDE = os.path.join(os.path.dirname(PKG_DIR), "include")
 LIB_PATH = os.path.join(CSRC, "libpylo_b200.so")
 LOCK_PATH = os.path.join(CSRC, ".build.lock")
 SOURCES = [os.path.join(CSRC, "pylo_kernels.cu")]
-HEADERS = [os.path.join(CSRC, "pylo_common.cuh"), os.path.join(CSRC, "pylo_pipe.cuh"), os.path.join(CSRC, "pylo_apply_tc.cuh"), os.path.join(CSRC, "pylo_ns_gemm.cuh"), os.path.join(CSRC, "pylo_ns_f16.cuh"), os.path.join(CSRC, "pylo_ns_cluster.cuh"), os.path.join(INCLUDE, "pylo_b200.h")]
+HEADERS = [os.path.join(CSRC, "pylo_common.cuh"), os.path.join(CSRC, "pylo_pipe.cuh"), os.path.join(CSRC, "pylo_small_front.cuh"), os.path.join(CSRC, "pylo_apply_tc.cuh"), os.path.join(CSRC, "pylo_ns_gemm.cuh"), os.path.join(CSRC, "pylo_ns_f16.cuh"), os.path.join(CSRC, "pylo_ns_cluster.cuh"), os.path.join(INCLUDE, "pylo_b200.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -302,6 +302,14 @@ __device__ __forceinline__ void cluster_store(float* p, uint32_t rank, float v) 
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
 
+__device__ __forceinline__ float cluster_load(const float* p, uint32_t rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
 template <int FAM>
 __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_factor_update(const pylo_tensor_desc* __restrict__ descs,
                                                                                           const pylo_step_params prm) {
@@ -1360,6 +1368,7 @@ __global__ void __launch_bounds__(NT, CC_CTAS_PER_SM) k_apply_adafac_cols(const 
   }
 }
 
+#include "pylo_small_front.cuh"
 #include "pylo_apply_tc.cuh"
 #include "pylo_ns_gemm.cuh"
 #include "pylo_ns_f16.cuh"
@@ -2277,6 +2286,16 @@ static int ns_clusters(nc_group& grp, int* status, cudaStream_t s) {
   return wide ? nc_launch<NC_COLS>(grp, (int)ctas, cluster, status, s) : nc_launch<128>(grp, (int)ctas, cluster, status, s);
 }
 
+template <int FAM>
+static int small_front_launch(const pylo_tensor_desc* descs, int ctas, int cluster, const SfShape& q, const pylo_step_params& prm, cudaStream_t s) {
+  static bool configured[PYLO_MAX_DEVICES] = {}, wide[PYLO_MAX_DEVICES] = {};
+  if (int rc = allow_dynamic_smem(k_small_front<FAM>, PYLO_SMALL_FLOATS * 4, configured)) return rc;
+  if (cluster > 8)
+    if (int rc = allow_wide_clusters(k_small_front<FAM>, wide)) return rc;
+  launch_clusters(k_small_front<FAM>, ctas, SF_NT, cluster, (size_t)sf_floats(q) * 4, s, descs, q, prm);
+  return launch_status();
+}
+
 extern "C" {
 
 int pylo_b200_abi_version(void) { return PYLO_B200_ABI_VERSION; }
@@ -2438,6 +2457,23 @@ int pylo_b200_state_moments(const pylo_tensor_desc* descs, const pylo_tile* tile
   }
   if (rc) return rc;
   return launch_status();
+}
+
+int pylo_b200_small_front(const pylo_tensor_desc* descs, int n_tensors, int cluster, int slice, int rows, int cols,
+                          const pylo_step_params* prm, void* stream) {
+  CHECK_ARG(descs && prm && n_tensors >= 0);
+  CHECK_ARG(((uintptr_t)descs & 15) == 0);   // a descriptor is read in pieces of 16 bytes
+  CHECK_ARG(cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8 || cluster == 16);
+  const SfShape q = {(slice + 3) & ~3, (rows + 3) & ~3, (cols + 3) & ~3};   // the arrays start on 16-byte boundaries
+  CHECK_ARG(slice >= 0 && rows >= 0 && cols >= 0 && slice <= SF_SLICE && sf_floats(q) <= PYLO_SMALL_FLOATS);
+  if (n_tensors == 0) return 0;
+  cudaStream_t s = (cudaStream_t)stream;
+  switch (prm->family) {
+    case PYLO_FAM_ADAFAC: return small_front_launch<PYLO_FAM_ADAFAC>(descs, n_tensors * cluster, cluster, q, *prm, s);
+    case PYLO_FAM_CELO2: return small_front_launch<PYLO_FAM_CELO2>(descs, n_tensors * cluster, cluster, q, *prm, s);
+    case PYLO_FAM_VELO: return small_front_launch<PYLO_FAM_VELO>(descs, n_tensors * cluster, cluster, q, *prm, s);
+    default: return -2;
+  }
 }
 
 int pylo_b200_finalize_moments(const pylo_tensor_desc* descs, int n_tensors, void* stream) {
@@ -2817,6 +2853,11 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
   CHECK_ARG(p && prm);
   const PlainLaunches plain(p->n_tiles);
   int rc = 0;
+  constexpr int front = PYLO_STEP_SUMS | PYLO_STEP_FACTORS | PYLO_STEP_STATE;
+  if (p->small_cluster && (phases & front) == front) {
+    if ((rc = pylo_b200_small_front(p->tdesc, p->n_tensors, p->small_cluster, p->small_slice, p->small_rows, p->small_cols, prm, stream))) return rc;
+    phases &= ~front;
+  }
   if ((phases & PYLO_STEP_SUMS) && (p->n_atiles || p->n_gitems))
     if ((rc = pylo_b200_rowcol_sums(p->tdesc, p->atiles, p->n_atiles, p->gitems, p->n_gitems, prm, stream))) return rc;
   if (phases & PYLO_STEP_FACTORS)

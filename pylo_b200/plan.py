@@ -27,6 +27,10 @@ from . import _lib as L
 SUM_TILES_MOST = 192
 
 
+#: CTAs of the launch that takes phases A to B of a small model, a cluster per tensor, that run at once (one per SM).
+SMALL_CTAS = L.SM_COUNT
+
+
 def _prod(xs) -> int:
     out = 1
     for x in xs:
@@ -84,6 +88,23 @@ def make_tiles(sizes: Sequence[int], elems: int = L.TILE_ELEMS) -> Tuple[np.ndar
     tiles["start"] = (np.arange(len(tiles), dtype=np.int64) - first[owner]) * elems
     tiles["elems"] = elems
     return tiles, list(zip(first[:-1].tolist(), counts.tolist()))
+
+
+def equal_tiles(sizes: Sequence[int], k: int) -> Tuple[np.ndarray, List[Tuple[int, int]]]:
+    """:func:`make_tiles` with exactly ``k`` tiles per item (the last ones may be empty), of a multiple of four elements."""
+    elems = -(-np.asarray(sizes, dtype=np.int64) // (4 * k)) * 4
+    tiles = np.zeros(len(sizes) * k, dtype=L.TILE_DTYPE)
+    tiles["tensor"], tiles["elems"] = np.repeat(np.arange(len(sizes)), k), np.repeat(elems, k)
+    tiles["start"] = (elems[:, None] * np.arange(k)).reshape(-1)
+    return tiles, [(k * i, k) for i in range(len(sizes))]
+
+
+def plain_matrices(d: np.ndarray) -> np.ndarray:
+    """Which descriptors are of contiguous matrices whose row_col_mean is over a whole vector or over the decays."""
+    Lr = np.where(d["r_is_a"] != 0, d["La"], d["Lb"])
+    whole = (d["rcm_pre"] == 3) & (d["rcm_A"] == Lr) & (d["rcm_post"] == 1)
+    decays = (d["rcm_pre"] == 1) & (d["rcm_A"] == 3) & (d["rcm_post"] == Lr)
+    return (d["O"] == 1) & (d["M"] == 1) & (d["I"] == 1) & (whole | decays)
 
 
 def tile_elems(total: int, least: int, tiles_wanted: int) -> int:
@@ -201,6 +222,28 @@ def apply_items(family: int, tensor_cores: bool, fast, slow) -> np.ndarray:
     return atile_list([atile_grid(u, -(-X // rt), -(-Y // w), tag) for u, X, Y, rt, w, tag in parts])
 
 
+def small_front(mats: Sequence[Tuple[int, int]], vectors: Sequence[int]):
+    """(CTAs per tensor, elements, rows and columns of the largest share) with which ``pylo_b200_small_front`` takes tensors of
+    these (rows, columns) and these vectors, or None: as many CTAs a tensor as all run at once, or as few as hold it where two
+    turns do.
+
+    us per step, three launches / one: six tensors (118 K elements, 16 CTAs each) 33.9 / 28.5, fourteen (26 K) with 8 CTAs
+    30.7 / 23.7 (with 16, two turns: 29.2), 28 (462 K, 8 CTAs, two turns) 48.3 / 46.6, 124 (533 K, 2 CTAs, two turns) 83.7 /
+    63.0, eight of odd sizes (325 K, 16 CTAs) 56.8 / 43.1; three turns: 76 (1.3 M, 16 CTAs) 98 / 137."""
+    T = len(mats) + len(vectors)
+
+    def share(cl):
+        rows = max([-(-X // cl) for X, _ in mats], default=0)
+        cols = max([Y for _, Y in mats], default=0)
+        most = max([-(-X // cl) * Y for X, Y in mats], default=0)
+        floats = 6 * (-(-most // 4) * 4) + 4 * (-(-rows // 4) * 4) + 5 * (-(-cols // 4) * 4)
+        fits = most <= L.SMALL_SLICE and floats <= L.SMALL_FLOATS and max(vectors, default=0) <= cl * L.SMALL_SLICE
+        return (cl, most, rows, cols) if fits else None
+
+    found = next((q for q in map(share, [cl for cl in (16, 8, 4, 2, 1) if T * cl <= SMALL_CTAS]) if q), None)
+    return found or next((q for q in map(share, [cl for cl in (1, 2, 4, 8, 16) if T * cl <= 2 * SMALL_CTAS]) if q), None)
+
+
 class LoPlan:
     """Descriptor tables, tile lists and workspace for the tensors of one optimizer instance.
 
@@ -316,7 +359,15 @@ class LoPlan:
         sizes = [int(udesc["n"][u]) for u in range(U)]
         # phase B: four 256-thread CTAs per SM, one pass of a CTA is 1024 elements; below ~10 M elements smaller tiles
         # fill the GPU, above they would only multiply the block reductions
-        tiles, ranges = make_tiles(sizes, tile_elems(sum(sizes), 1024, 4 * L.SM_COUNT))
+        self.small = None
+        if not self.sliced and sum(sizes) <= 2 * SMALL_CTAS * L.SMALL_SLICE:
+            vectors = tdesc["mode"] == L.MODE_VEC1D
+            if (vectors | plain_matrices(tdesc)).all():
+                self.small = small_front(list(zip(tdesc["X"][~vectors].tolist(), tdesc["Y"][~vectors].tolist())), tdesc["n"][vectors].tolist())
+        if self.small:   # as many tiles a tensor as CTAs take its rows
+            tiles, ranges = equal_tiles(sizes, self.small[0])
+        else:
+            tiles, ranges = make_tiles(sizes, tile_elems(sum(sizes), 1024, 4 * L.SM_COUNT))
         for u, (t0, k) in enumerate(ranges):
             udesc["tile0"][u], udesc["n_tiles"][u] = t0, k
             ws = L.workspace_layout(family, L.MODE_VEC1D, sizes[u])  # the per-unit part depends on the element count only
@@ -412,6 +463,8 @@ class LoPlan:
             n_tensors=T, n_units=U, n_atiles=self.n_atiles, n_gitems=self.n_gitems, n_pitems=self.n_pitems,
             n_ctiles=self.n_ctiles, n_ctiles_gen=self.n_ctiles_gen, n_tiles=self.n_tiles, n_tiles_slow=self.n_tiles_slow,
             tensor_cores=int(self.tensor_cores), sum_tiles=int(self.sum_tiles))
+        if self.small:
+            (self.step_plan.small_cluster, self.step_plan.small_slice, self.step_plan.small_rows, self.step_plan.small_cols) = self.small
         self._step_plan_ref = C.byref(self.step_plan)
         self._hyper = None          # what set_hyper last wrote
         self._grad_ptrs = None      # the gradient addresses the table holds
@@ -486,7 +539,7 @@ class LoPlan:
     # ------------------------------------------------------------------ launch sequence
     #: the kernel that dominates each timed phase, for reports
     KERNEL_OF = {"rowcol_sums": "k_rowcol_fast", "factor_update": "k_factor_update", "state_moments": "k_state_moments",
-                 "finalize_moments": "k_finalize_moments", "prep_apply": "k_prep_apply"}
+                 "finalize_moments": "k_finalize_moments", "prep_apply": "k_prep_apply", "small_front": "k_small_front"}
 
     def _phases(self):
         """[(phase of pylo_b200_step, name, launches)] in the step's order, without those that launch nothing."""
@@ -496,8 +549,11 @@ class LoPlan:
         other = "k_apply_adafac_tc<true>" if self.tensor_cores else "k_apply"
         apply = [(L.STEP_APPLY, self.apply_kernel if self.n_ctiles > self.n_ctiles_gen else other, main)]
         apply.insert(0 if self.tensor_cores else 1, (L.STEP_APPLY_REST, other, rest))
-        phases = [(L.STEP_SUMS, "rowcol_sums", (self.n_atiles > 0) + (self.n_gitems > 0)), (L.STEP_FACTORS, "factor_update", 1),
-                  (L.STEP_STATE, "state_moments", 1), (L.STEP_MOMENTS, "finalize_moments", int(not self.sum_tiles)),
+        front = [(L.STEP_SUMS, "rowcol_sums", (self.n_atiles > 0) + (self.n_gitems > 0)), (L.STEP_FACTORS, "factor_update", 1),
+                 (L.STEP_STATE, "state_moments", 1)]
+        if self.small:
+            front = [(L.STEP_SUMS | L.STEP_FACTORS | L.STEP_STATE, "small_front", 1)]
+        phases = front + [(L.STEP_MOMENTS, "finalize_moments", int(not self.sum_tiles)),
                   (L.STEP_PREP, "prep_apply", 1)] + apply
         return [ph for ph in phases if ph[2]]
 

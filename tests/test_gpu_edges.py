@@ -370,3 +370,40 @@ def test_tile_sums_on_both_sides_of_the_launch(family, extra, rows):
     # moves a normalised feature by 2^-24 of itself and the network's output, and so the step, by a few times that
     move = float((runs[0] - cases.init_values(case)[0].cuda()).abs().max())
     assert float((runs[0] - runs[1]).abs().max()) <= 1e-5 * move + 2 ** -23 * float(runs[0].abs().max())
+
+
+# matrices and vectors of a small model: rows fewer than CTAs, one CTA's share full, odd sizes (no piece of 16 bytes), one row, one
+# column, a single element; 1, 2, 8 and 16 CTAs a tensor
+SMALL = [[(128, 784), (128,), (10, 128), (10,)], [(1, 4744), (3, 4), (1, 1)], [(5000, 1), (7, 1001), (1001, 7), (4099,)], [(512, 256)],
+         [(64, 64)] * 40 + [(13,)] * 30, [(9, 20), (33, 7)] * 30]
+
+
+@pytest.mark.parametrize("shapes", SMALL, ids=[str(s[0]) + "x" + str(len(s)) for s in SMALL])
+@pytest.mark.parametrize("family,extra", [("adafaclo", {}), ("adafaclo", {"initial_momentum_decays": (0.2, 0.9, 0.99)}), ("elo", {}),
+                                          ("celo2", {"orthogonalize": False}), ("velo", {})])
+def test_small_models_front_in_one_launch(family, extra, shapes, monkeypatch):
+    """Sums, factors and state of a small model by clusters, against the three launches that other models take."""
+    from pylo_b200 import plan as pylo_plan
+
+    case = dict(shapes=shapes, init_seed=51, init_scale=0.1, grad_seed=52, grad_scale=0.3)
+    runs = []
+    for ctas in (pylo_plan.SMALL_CTAS, 0):
+        monkeypatch.setattr(pylo_plan, "SMALL_CTAS", ctas)
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+        opt = _make(family, params, **extra)
+        for t in (1, 2):
+            for p, g in zip(params, cases.grads_at(case, t)):
+                p.grad = g.cuda()
+            _step(opt, family, t)
+        plan, = _plans(opt)
+        assert bool(plan.small) == bool(ctas)
+        runs.append(([p.detach().clone() for p in params], [opt.state[p] for p in params]))
+    for (a, b, init) in zip(runs[0][0], runs[1][0], cases.init_values(case)):
+        # sums of positive terms in another order: relative differences of a few 2^-24 (a thousand terms, in trees), which move
+        # a factor by half of that and the network's output by a few times as much
+        move = float((b - init.cuda()).abs().max())
+        assert float((a - b).abs().max()) <= 2e-5 * move + 2 ** -23 * float(b.abs().max())
+    for sa, sb in zip(runs[0][1], runs[1][1]):
+        for key, x in sa.items():
+            if torch.is_tensor(x) and x.is_floating_point() and x.numel():
+                assert torch.allclose(x, sb[key], rtol=4e-6, atol=1e-12), key

@@ -270,3 +270,29 @@ def test_no_source_file_names_a_path_of_one_machine():
     for path in paths:
         if path.endswith((".py", ".cu", ".cuh", ".h")):
             assert not re.search(r"/(root|home)/\w", open(path).read()), path
+
+
+def test_small_models_are_dealt_to_clusters_that_hold_them():
+    """Every share fits, all clusters run at once (or, with the fewest CTAs that hold the tensors, in two turns)."""
+    cases = [([(128, 784), (128, 128), (10, 128)], [128, 128, 10]), ([(64, 64)] * 40, [13] * 30), ([(512, 256)], []), ([], [5]),
+             ([(1, 4747)], []), ([(1, 4748)], []), ([(1, 8193)], []), ([(513, 256)], []), ([(4096, 4096)], []), ([(64, 64)] * 296, []), ([(64, 64)] * 297, [])]
+    for mats, vectors in cases:
+        got, T = plan.small_front(mats, vectors), len(mats) + len(vectors)
+        up = lambda n: -(-n // 4) * 4
+        fits = lambda cl: (all(-(-X // cl) * Y <= L.SMALL_SLICE for X, Y in mats) and all(-(-n // cl) <= L.SMALL_SLICE for n in vectors)
+                           and 6 * up(max([-(-X // cl) * Y for X, Y in mats], default=0)) + 4 * up(max([-(-X // cl) for X, _ in mats], default=0))
+                           + 5 * up(max([Y for _, Y in mats], default=0)) <= L.SMALL_FLOATS)
+        if got is None:
+            assert not any(fits(cl) and T * cl <= 2 * plan.SMALL_CTAS for cl in (1, 2, 4, 8, 16))
+            continue
+        cl, share, rows, cols = got
+        assert cl in (1, 2, 4, 8, 16) and fits(cl)
+        assert T * cl <= plan.SMALL_CTAS or not any(fits(c) for c in (1, 2, 4, 8) if c < cl)
+    assert plan.small_front([(128, 784)], [10])[0] == 16 and plan.small_front([(64, 64)] * 40, [13] * 30)[0] == 2
+
+    for sizes, k in (([1], 16), ([100352, 10, 7], 16), ([8192], 1)):
+        tiles, ranges = plan.equal_tiles(sizes, k)
+        for i, (n, (t0, m)) in enumerate(zip(sizes, ranges)):
+            mine = tiles[t0:t0 + m]
+            assert m == k and (mine["tensor"] == i).all() and (mine["elems"] % 4 == 0).all()
+            assert int(np.clip(n - mine["start"], 0, mine["elems"]).sum()) == n
