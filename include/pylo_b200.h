@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define PYLO_B200_ABI_VERSION 13
+#define PYLO_B200_ABI_VERSION 14
 
 /* optimizer families (which feature set / network geometry a launch uses) */
 #define PYLO_FAM_ADAFAC 0 /* AdafacLO_CUDA, ELO_CUDA: 28+11 features, 39-32-32-2 */
@@ -154,6 +154,8 @@ typedef struct pylo_step_params {
                              then incomplete); the apply kernels that write parameters (ADAFAC, VELO) write none while it
                              is not zero; may be NULL */
   int* host_status;       /* a word of pinned host memory that both events are written to; may be NULL */
+  const float* w_host;    /* HOST pointer to the network of desc.w, where it is the same for all units, or NULL.  CELO2: apply_packed
+                             then takes it as an argument of its launch instead of reading the folded one of every unit */
 } pylo_step_params;
 
 int pylo_b200_abi_version(void);

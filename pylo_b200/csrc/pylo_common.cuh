@@ -54,9 +54,10 @@ struct Fold {
   static constexpr int B3 = W3 + F::H * 2;        // [2]
   static constexpr int SC = B3 + 2;               // [0] param_scale (VeLO), [1] lr_eff
   static constexpr int W3P = SC + 2;              // [H/2][4]: (dir[2j], dir[2j+1], mag[2j], mag[2j+1]) for packed dot products
-  static constexpr int SIZE = W3P + 2 * F::H;
+  static constexpr int SN = W3P + 2 * F::H;       // [NF]: the features' normalisers
+  static constexpr int SIZE = SN;                 // of what a kernel with the folded network needs
 };
-static_assert(Fold<PYLO_FAM_ADAFAC>::SIZE <= PYLO_WFOLD_STRIDE, "wfold too small");
+static_assert(Fold<PYLO_FAM_ADAFAC>::SN + Fam<PYLO_FAM_ADAFAC>::NF <= PYLO_WFOLD_STRIDE, "wfold too small");
 
 // compile-time loop: guarantees static register indexing however large the unrolled body gets
 template <int I, int N, class Fn>
@@ -115,7 +116,9 @@ __device__ __forceinline__ float xform_grad(float g, float gs, float clip, int n
     if (g != g) g = 0.0f;
     else if (isinf(g)) g = g > 0 ? 3.4028234663852886e38f : -3.4028234663852886e38f;
   }
-  return (g != g) ? g : fminf(fmaxf(g, -clip), clip);
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(g) : "f"(-clip));
+  asm("min.NaN.f32 %0, %0, %1;" : "+f"(g) : "f"(clip));
+  return g;
 }
 
 // whether xform_grad changes nothing: no global-norm scale, no nan_to_num, no clamp (AdafacLO's defaults)

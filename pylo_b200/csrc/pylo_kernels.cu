@@ -837,6 +837,7 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
   if (it.strip == 0) {
     float* const o = d.wfold;
     for (int e = tid; e < NF * H; e += NT) o[L::W1 + e] = s_w1[e];
+    if (tid < NF) o[L::SN + tid] = s_scale[tid];
     if (tid < H) o[L::B1 + tid] = s_b1[tid];
     for (int e = tid; e < H * H; e += NT) {
       const int k = e / H, j = e % H;
@@ -1378,26 +1379,36 @@ __global__ void __launch_bounds__(NT, CC_CTAS_PER_SM) k_apply_adafac_cols(const 
 // Phase C for CELO2 / ELO_CELO2 / VeLO on FAST2D tensors: packed kernel.
 //
 // These networks are small (30-8-8-3, 30-4-4-3), so the sweep should run at HBM speed; what stands
-// in the way is the instruction count per element.  This kernel halves it:
+// in the way is the work per element.  218 M CELO2 parameters (a Llama block) take 2197 us (2747 before constant weights and
+// early requests), 10.1 ps per element, of which the multiply-adds' pipe needs 8; 355 M VeLO parameters (GPT-2-medium) 1986 us
+// (2345) = 5.0 TB/s.
 //   * all arithmetic is done on PAIRS OF ADJACENT ELEMENTS with packed fp32x2 instructions: a
 //     float4 load already is two such pairs, so no register moves are needed to form them;
-//   * weights sit in shared memory as (w, w) pairs, one 128-bit read feeds four elements;
+//   * a weight is a pair (w, w) of one register, or of a constant: four weights per read from shared memory, each feeds four elements;
 //   * a thread keeps four columns for all rows of its tile, so the columns' tabulated first-layer
 //     terms and factors stay in registers; the rows' terms arrive as broadcast loads;
 //   * the next row's six float4 operands are requested before the current row is computed;
+//   * a packed multiply-add with three operands in registers occupies the pipe for 3.3 cycles (six registers to read), with one
+//     of them a constant for 2.3: where one network serves all units (CELO2) its weights are arguments of the launch, and the
+//     eighteen features are normalised instead of the weights; where every tensor has its own (VeLO) a weight is one register
+//     taken twice (3.0 cycles), and a read from shared memory brings four of them, not two;
 //   * the rows' first-layer terms and factors are staged in shared memory, up to 256 rows at a time: read from global memory
 //     row by row, every row began with their latency.
 // ================================================================================================
 template <int FAM>
-struct PkW {  // duplicated-weight layout in shared memory (floats)
-  static constexpr int H = Fam<FAM>::H;
-  static constexpr int W1 = 0;                   // [30][H] pairs
-  static constexpr int W2 = W1 + 30 * H * 2;     // [H][H] pairs, k-major
-  static constexpr int B2 = W2 + H * H * 2;      // [H] pairs
-  static constexpr int W3 = B2 + H * 2;          // [H][2] pairs
-  static constexpr int B3 = W3 + H * 4;          // [2] pairs
+struct PkW {  // the network in shared memory (floats), or as an argument of the launch
+  static constexpr int H = Fam<FAM>::H, NE = 18;  // NE: element-wise features
+  static constexpr int W1 = 0;                    // [NE][H]
+  static constexpr int W2 = W1 + NE * H;          // [H][H], k-major
+  static constexpr int B2 = W2 + H * H;           // [H]
+  static constexpr int W3 = B2 + H;               // [H][2]
+  static constexpr int B3 = W3 + H * 2;           // [2], two unused
   static constexpr int SIZE = B3 + 4;
 };
+template <int FAM>
+struct PkNet { float w[PkW<FAM>::SIZE]; };
+// place of an element-wise feature among them
+__host__ __device__ constexpr int pk_index(int k) { return k < 15 ? k : k - 12; }
 
 struct PkBase {  // packed per-pair operands the features are made of
   uint64_t g, cg, p, m0, m1, m2, v, rs, k0, k1, k2;
@@ -1425,6 +1436,12 @@ __device__ __forceinline__ uint64_t pk_feature(const PkBase& b) {
   else return mul2(b.k2, b.m2);
 }
 
+// a 128-bit load issued where it is written: the compiler moves the next row's loads down to their use (CELO2 3023 us instead of 2197)
+__device__ __forceinline__ float4 ld4_early(const float* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
 #define PK_ROWS 16  // rows per thread in a tile, unless the tag's upper half says otherwise
 #define PK_STAGE 256  // rows staged at once
 
@@ -1432,22 +1449,24 @@ __device__ __forceinline__ uint64_t pk_feature(const PkBase& b) {
 #define PK_CTAS_VELO 2
 #endif
 #ifndef PK_CTAS_CELO2
-#define PK_CTAS_CELO2 1   // its 8-wide layers want registers more than a second CTA: 2989 -> 2753 us over a Llama block
+#define PK_CTAS_CELO2 1   // its 8-wide layers want registers more than a second CTA (224 bytes of spills: 2357 -> 2435 us over a Llama block)
 #endif
-template <int FAM>
+// ARG: one network for all units, which comes as an argument of the launch; the features are normalised instead of the weights.
+template <int FAM, bool ARG>
 __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_CTAS_CELO2) k_apply_packed(const pylo_tensor_desc* __restrict__ descs,
                                                         const pylo_atile* __restrict__ ctiles, int n_ctiles,
-                                                        const pylo_step_params prm) {
+                                                        const pylo_step_params prm, const __grid_constant__ PkNet<FAM> net) {
   pdl_begin();
   using F = Fam<FAM>;
   using L = Fold<FAM>;
   using W = PkW<FAM>;
   constexpr int H = F::H;
   constexpr int RP = 2 * H + 4;     // floats of a staged row: H pairs (v, v), then its three factors
-  __shared__ __align__(16) float s_w[W::SIZE];
+  __shared__ __align__(16) float s_w[ARG ? 20 : W::SIZE];   // ARG: the normalisers of the element-wise features
   __shared__ __align__(16) float s_row[PK_STAGE * RP];
   __shared__ float s_sc[2];
   const int tid = threadIdx.x;
+  const uint32_t s_wa = smem_addr(s_w);
   int loaded = -1;
   for (int t = blockIdx.x; t < n_ctiles; t += gridDim.x) {
     const pylo_atile ct = ctiles[t];
@@ -1462,11 +1481,16 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
       const int word = FAM == PYLO_FAM_CELO2 ? 0 : reported(prm.status);
       __syncthreads();
       const float* __restrict__ wf = d.wfold;
-      for (int e = tid; e < 30 * H; e += NT) { const float w = __ldg(wf + L::W1 + e); s_w[W::W1 + 2 * e] = w; s_w[W::W1 + 2 * e + 1] = w; }
-      for (int e = tid; e < H * H; e += NT) { const float w = __ldg(wf + L::W2 + e); s_w[W::W2 + 2 * e] = w; s_w[W::W2 + 2 * e + 1] = w; }
-      for (int e = tid; e < H; e += NT) { const float w = __ldg(wf + L::B2 + e); s_w[W::B2 + 2 * e] = w; s_w[W::B2 + 2 * e + 1] = w; }
-      for (int e = tid; e < H * 2; e += NT) { const float w = __ldg(wf + L::W3 + e); s_w[W::W3 + 2 * e] = w; s_w[W::W3 + 2 * e + 1] = w; }
-      for (int e = tid; e < 2; e += NT) { const float w = __ldg(wf + L::B3 + e); s_w[W::B3 + 2 * e] = w; s_w[W::B3 + 2 * e + 1] = w; s_sc[e] = __ldg(wf + L::SC + e); }
+      if (ARG) {
+        if (tid < W::NE) s_w[tid] = __ldg(wf + L::SN + (tid < 15 ? tid : tid + 12));
+      } else {
+        for (int e = tid; e < W::NE * H; e += NT) { const int k = e / H; s_w[W::W1 + e] = __ldg(wf + L::W1 + (k < 15 ? e : e + 12 * H)); }
+        for (int e = tid; e < H * H; e += NT) s_w[W::W2 + e] = __ldg(wf + L::W2 + e);
+        if (tid < H) s_w[W::B2 + tid] = __ldg(wf + L::B2 + tid);
+        if (tid < H * 2) s_w[W::W3 + tid] = __ldg(wf + L::W3 + tid);
+        if (tid < 2) s_w[W::B3 + tid] = __ldg(wf + L::B3 + tid);
+      }
+      if (tid < 2) s_sc[tid] = __ldg(wf + L::SC + tid);
       loaded = ct.tensor;
       __syncthreads();
       if (word) {
@@ -1477,7 +1501,8 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
     const int y = y0 + 4 * (tid % tpr), rg = tid / tpr;
     const bool colok = y < Y;
     const int yc = colok ? y : 0;
-    const Fin fin = make_fin(d, s_sc[0], s_sc[1], prm.wd_mode);
+    // VeLO: p + rate * (...), then + decay * that (lr_eff may have either sign)
+    const float exp_mult = d.exp_mult, rate = -(s_sc[1] * s_sc[0] * d.step_mult), decay = d.wd > 0.f ? -(d.wd * s_sc[1]) : 0.f;
     const float gs = grad_scale_of(d, prm);
     const float eps_feat = prm.eps_feat, clip = prm.clip_val;
     const int64_t n = d.n;
@@ -1508,7 +1533,7 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
     auto load_row = [&](int q, float4& g, float4& p, float4& m0, float4& m1, float4& m2, float4& v) {
       const int x = x0 + rg + ng * q;
       const int64_t idx = (colok && x < X) ? (int64_t)x * Y + y : 0;
-      g = ldg4(gp + idx); p = ld4(pp + idx); m0 = ld4(mp + idx); m1 = ld4(mp + n + idx); m2 = ld4(mp + 2 * n + idx); v = ld4(vp + idx);
+      g = ld4_early(gp + idx); p = ld4_early(pp + idx); m0 = ld4_early(mp + idx); m1 = ld4_early(mp + n + idx); m2 = ld4_early(mp + 2 * n + idx); v = ld4_early(vp + idx);
     };
     load_row(0, cg, cp, cm0, cm1, cm2, cv);
     const int sub = min(PK_ROWS, PK_STAGE / ng);   // rows per thread and stage
@@ -1550,25 +1575,44 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
         h1[0][j] = add2(hb[0][j], a.x); h1[0][j + 1] = add2(hb[0][j + 1], a.y);
         h1[1][j] = add2(hb[1][j], a.x); h1[1][j + 1] = add2(hb[1][j + 1], a.y);
       }
+      // four weights at a time, each as a pair (w, w): constants where they are an argument, which leaves a product two operands
+      // to read from registers (three cost it 3.3 cycles instead of 2.3), else from shared memory
+      auto weights = [&](auto at) -> float4 {
+        constexpr int A = decltype(at)::value;
+        if constexpr (ARG) return make_float4(net.w[A], net.w[A + 1], net.w[A + 2], net.w[A + 3]);
+        else return lds4<A>(s_wa);
+      };
+      float4 scales;
       static_for<0, F::NF>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
         if constexpr (!is_vec_feature<FAM>(k)) {
-          const uint64_t f0 = pk_feature<k>(b[0]), f1 = pk_feature<k>(b[1]);
-#pragma unroll
-          for (int j = 0; j < H; j += 2) {
-            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&s_w[W::W1 + (k * H + j) * 2]);
-            h1[0][j] = fma2(w.x, f0, h1[0][j]); h1[0][j + 1] = fma2(w.y, f0, h1[0][j + 1]);
-            h1[1][j] = fma2(w.x, f1, h1[1][j]); h1[1][j + 1] = fma2(w.y, f1, h1[1][j + 1]);
+          constexpr int i = pk_index(k);
+          uint64_t f0 = pk_feature<k>(b[0]), f1 = pk_feature<k>(b[1]);
+          if constexpr (ARG) {
+            if constexpr (i % 4 == 0) scales = lds4<i>(s_wa);
+            const float sc = i % 4 == 0 ? scales.x : i % 4 == 1 ? scales.y : i % 4 == 2 ? scales.z : scales.w;
+            f0 = mul2(f0, pack2(sc, sc));
+            f1 = mul2(f1, pack2(sc, sc));
           }
+          static_for<0, H / 4>([&](auto jc) {
+            constexpr int j = decltype(jc)::value * 4;
+            const float4 w = weights(std::integral_constant<int, W::W1 + i * H + j>{});
+            const uint64_t w0 = pack2(w.x, w.x), w1 = pack2(w.y, w.y), w2 = pack2(w.z, w.z), w3 = pack2(w.w, w.w);
+            h1[0][j] = fma2(w0, f0, h1[0][j]); h1[1][j] = fma2(w0, f1, h1[1][j]);
+            h1[0][j + 1] = fma2(w1, f0, h1[0][j + 1]); h1[1][j + 1] = fma2(w1, f1, h1[1][j + 1]);
+            h1[0][j + 2] = fma2(w2, f0, h1[0][j + 2]); h1[1][j + 2] = fma2(w2, f1, h1[1][j + 2]);
+            h1[0][j + 3] = fma2(w3, f0, h1[0][j + 3]); h1[1][j + 3] = fma2(w3, f1, h1[1][j + 3]);
+          });
         }
       });
       // second layer
       uint64_t h2[2][H];
+      static_for<0, H / 4>([&](auto jc) {
+        constexpr int j = decltype(jc)::value * 4;
+        const float4 w = weights(std::integral_constant<int, W::B2 + j>{});
 #pragma unroll
-      for (int j = 0; j < H; j += 2) {
-        const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(&s_w[W::B2 + j * 2]);
-        h2[0][j] = bb.x; h2[0][j + 1] = bb.y; h2[1][j] = bb.x; h2[1][j + 1] = bb.y;
-      }
+        for (int e = 0; e < 2; ++e) { h2[e][j] = pack2(w.x, w.x); h2[e][j + 1] = pack2(w.y, w.y); h2[e][j + 2] = pack2(w.z, w.z); h2[e][j + 3] = pack2(w.w, w.w); }
+      });
       static_for<0, H>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
         uint64_t r[2];
@@ -1578,34 +1622,51 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
           unpack2(h1[e][k], lo, hi);
           r[e] = pack2(fmaxf(lo, 0.f), fmaxf(hi, 0.f));
         }
-#pragma unroll
-        for (int j = 0; j < H; j += 2) {
-          const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&s_w[W::W2 + (k * H + j) * 2]);
-          h2[0][j] = fma2(w.x, r[0], h2[0][j]); h2[0][j + 1] = fma2(w.y, r[0], h2[0][j + 1]);
-          h2[1][j] = fma2(w.x, r[1], h2[1][j]); h2[1][j + 1] = fma2(w.y, r[1], h2[1][j + 1]);
-        }
+        static_for<0, H / 4>([&](auto jc) {
+          constexpr int j = decltype(jc)::value * 4;
+          const float4 w = weights(std::integral_constant<int, W::W2 + k * H + j>{});
+          const uint64_t w0 = pack2(w.x, w.x), w1 = pack2(w.y, w.y), w2 = pack2(w.z, w.z), w3 = pack2(w.w, w.w);
+          h2[0][j] = fma2(w0, r[0], h2[0][j]); h2[1][j] = fma2(w0, r[1], h2[1][j]);
+          h2[0][j + 1] = fma2(w1, r[0], h2[0][j + 1]); h2[1][j + 1] = fma2(w1, r[1], h2[1][j + 1]);
+          h2[0][j + 2] = fma2(w2, r[0], h2[0][j + 2]); h2[1][j + 2] = fma2(w2, r[1], h2[1][j + 2]);
+          h2[0][j + 3] = fma2(w3, r[0], h2[0][j + 3]); h2[1][j + 3] = fma2(w3, r[1], h2[1][j + 3]);
+        });
       });
       // output layer: direction and magnitude
-      const ulonglong2 b3 = *reinterpret_cast<const ulonglong2*>(&s_w[W::B3]);
-      uint64_t o0[2] = {b3.x, b3.x}, o1[2] = {b3.y, b3.y};
-      static_for<0, H>([&](auto kc) {
-        constexpr int k = decltype(kc)::value;
-        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&s_w[W::W3 + k * 4]);
+      const float4 b3 = weights(std::integral_constant<int, W::B3>{});
+      uint64_t o0[2] = {pack2(b3.x, b3.x), pack2(b3.x, b3.x)}, o1[2] = {pack2(b3.y, b3.y), pack2(b3.y, b3.y)};
+      static_for<0, H / 2>([&](auto kc) {
+        constexpr int k = decltype(kc)::value * 2;
+        const float4 w = weights(std::integral_constant<int, W::W3 + k * 2>{});   // (dir, mag) of two units
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           float lo, hi;
           unpack2(h2[e][k], lo, hi);
-          const uint64_t r = pack2(fmaxf(lo, 0.f), fmaxf(hi, 0.f));
-          o0[e] = fma2(w.x, r, o0[e]);
-          o1[e] = fma2(w.y, r, o1[e]);
+          uint64_t r = pack2(fmaxf(lo, 0.f), fmaxf(hi, 0.f));
+          o0[e] = fma2(pack2(w.x, w.x), r, o0[e]);
+          o1[e] = fma2(pack2(w.y, w.y), r, o1[e]);
+          unpack2(h2[e][k + 1], lo, hi);
+          r = pack2(fmaxf(lo, 0.f), fmaxf(hi, 0.f));
+          o0[e] = fma2(pack2(w.z, w.z), r, o0[e]);
+          o1[e] = fma2(pack2(w.w, w.w), r, o1[e]);
         }
       });
       if (colok && x < X) {
         float d0, d1, d2, d3, m0, m1, m2, m3;
         unpack2(o0[0], d0, d1); unpack2(o0[1], d2, d3);
         unpack2(o1[0], m0, m1); unpack2(o1[1], m2, m3);
-        const float4 res = make_float4(finish<FAM>(cp.x, d0, m0, fin), finish<FAM>(cp.y, d1, m1, fin),
-                                       finish<FAM>(cp.z, d2, m2, fin), finish<FAM>(cp.w, d3, m3, fin));
+        float4 res;
+        if constexpr (FAM == PYLO_FAM_VELO) {   // finish(), two elements at a time and its constants made once per tile
+          auto two = [&](float p0, float p1, float a, float b, float m, float n, float& r0, float& r1) {
+            uint64_t pn = fma2(mul2(pack2(a, b), pack2(__expf(m * exp_mult), __expf(n * exp_mult))), pack2(rate, rate), pack2(p0, p1));
+            if (decay != 0.f) pn = fma2(pack2(decay, decay), pn, pn);
+            unpack2(pn, r0, r1);
+          };
+          two(cp.x, cp.y, d0, d1, m0, m1, res.x, res.y);
+          two(cp.z, cp.w, d2, d3, m2, m3, res.z, res.w);
+        } else {
+          res = make_float4(d0 * __expf(m0 * exp_mult), d1 * __expf(m1 * exp_mult), d2 * __expf(m2 * exp_mult), d3 * __expf(m3 * exp_mult));
+        }
         st4(op + (int64_t)x * Y + y, res);
         if (FAM != PYLO_FAM_CELO2) peer_store4(peers, (int64_t)x * Y + y, res);
       }
@@ -2764,10 +2825,24 @@ int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctil
   if (n_ctiles == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_CELO2: launch(k_apply_packed<PYLO_FAM_CELO2>, grid_for(n_ctiles, PK_CTAS_CELO2), NT, 0, s, descs, ctiles, n_ctiles, *prm); break;
+    case PYLO_FAM_CELO2: {
+      PkNet<PYLO_FAM_CELO2> net = {};
+      if (prm->w_host) {
+        using W = PkW<PYLO_FAM_CELO2>;
+        const float* w = prm->w_host;   // w_in[30][8] b_in[8] w_h[8][8] b_h[8] w_out[8][3] b_out[3]
+        for (int e = 0; e < 18 * 8; ++e) net.w[W::W1 + e] = w[e < 15 * 8 ? e : e + 12 * 8];
+        for (int e = 0; e < 64; ++e) net.w[W::W2 + e] = w[248 + e];
+        for (int e = 0; e < 8; ++e) { net.w[W::B2 + e] = w[312 + e]; net.w[W::W3 + 2 * e] = w[320 + 3 * e]; net.w[W::W3 + 2 * e + 1] = w[321 + 3 * e]; }
+        net.w[W::B3] = w[344]; net.w[W::B3 + 1] = w[345];
+        launch(k_apply_packed<PYLO_FAM_CELO2, true>, grid_for(n_ctiles, PK_CTAS_CELO2), NT, 0, s, descs, ctiles, n_ctiles, *prm, net);
+      } else {
+        launch(k_apply_packed<PYLO_FAM_CELO2, false>, grid_for(n_ctiles, PK_CTAS_CELO2), NT, 0, s, descs, ctiles, n_ctiles, *prm, net);
+      }
+      break;
+    }
     // four times the CTAs that fit: an SM that is done takes the next (17 M parameters: 341 -> 327 us per step, 67 M: 1104 ->
     // 1091); CELO2's larger network is loaded by every CTA, which costs more than that gives
-    case PYLO_FAM_VELO: launch(k_apply_packed<PYLO_FAM_VELO>, grid_for(n_ctiles, 4 * PK_CTAS_VELO), NT, 0, s, descs, ctiles, n_ctiles, *prm); break;
+    case PYLO_FAM_VELO: launch(k_apply_packed<PYLO_FAM_VELO, false>, grid_for(n_ctiles, 4 * PK_CTAS_VELO), NT, 0, s, descs, ctiles, n_ctiles, *prm, PkNet<PYLO_FAM_VELO>{}); break;
     default: return -2;
   }
   return launch_status();

@@ -74,6 +74,7 @@ class _Celo2Family(Optimizer):
         self.w_in, self.b_in, self.w_h, self.b_h, self.w_out, self.b_out = (
             t.to(dev) for t in self.network.flat_weights())
         self._w_flat = torch.cat([t.reshape(-1) for t in (self.w_in, self.b_in, self.w_h, self.b_h, self.w_out, self.b_out)]).contiguous()
+        self._w_host = self._w_flat.cpu().numpy()   # the apply sweep's launch carries it
         self._plans = {}
         self._gnorm = None
         # "3xtf32" (default): the Newton-Schulz products on the tensor cores (this library's kernels, operands split
@@ -207,6 +208,7 @@ class _Celo2Family(Optimizer):
                 prm.w_m[k], prm.w_f[k] = self._w_m[k], self._w_f[k]
             prm.w_v = self._w_v
             prm.eps_feat, prm.eps_norm = 1e-8, 1e-9
+            prm.w_host = self._w_host.ctypes.data
         prm.clip_val, prm.gnorm_sq = float(group["grad_clip_val"]), gnorm_ptr
         return prm
 
