@@ -155,7 +155,8 @@ typedef struct pylo_step_params {
                              is not zero; may be NULL */
   int* host_status;       /* a word of pinned host memory that both events are written to; may be NULL */
   const float* w_host;    /* HOST pointer to the network of desc.w, where it is the same for all units, or NULL.  CELO2: apply_packed
-                             then takes it as an argument of its launch instead of reading the folded one of every unit */
+                             then takes it as an argument of its launch instead of reading the folded one of every unit;
+                             ADAFAC: apply_adafac_tc its output layer */
 } pylo_step_params;
 
 int pylo_b200_abi_version(void);

@@ -29,10 +29,12 @@
 //   * the products are issued by one elected lane inside a warp-uniform branch (the warp index is a broadcast
 //     from lane 0), so that their descriptors and tensor-memory addresses live in uniform registers: issued from
 //     a branch on the thread index, each product cost its thread ~52 cycles; this way ~24.
-// What bounds it: one 4096 x 4096 tensor takes 365 us (21.8 ps, 5.75 SM cycles and 378 instructions per element; 28 B of
-// memory traffic); issue slots 54 %, tensor pipe 51 %, ALU pipe 43 %, DRAM 15 % busy: none is full.  A tile's stages are one
-// serial chain (operand stores, products, read-back, split and stores, products, read-back, heads) and four tiles per SM
-// are in flight, one per warpgroup.
+//   * the output layer, one network's for all units, is an argument of the launch: read from shared memory, with no registers
+//     to ask ahead, each pair of units waited for its weights (the heads took 700 of a tile's 2970 cycles, now 500 of 2795; ViT-B/16
+//     sweep 1827 -> 1689 us, two Llama blocks 9640 -> 9190).
+// What bounds it: a tile's stages are one serial chain (operand stores, products, read-back, split and stores, products,
+// read-back, heads; 2795 cycles with four tiles per SM in flight, one per warpgroup), and the GPU's power limit: with the heads
+// moved under the next row's products, or the bias vector's store under the second layer's, the sweep was not faster.
 // Every wait on the tensor core is bounded.  A thread whose wait ran out records it in *status (and in *host_status, a word
 // of pinned host memory that the host looks at without asking the device), stops waiting
 // and stops storing (its parameters, and their copies on the peers, keep their old values), and goes on to
@@ -214,13 +216,17 @@ struct TcSmem {
   int poisoned;  // the status word at launch: non-zero means an earlier launch reported a timed-out wait
 };
 
+// The output layer as an argument of the launch, where one network serves all units: pairs of units' direction and magnitude weights
+// (Fold::W3P), then the two biases.
+struct TcHeads { float w[64], b[2]; };
+
 // GENERIC: the launch may hold items on tensors that are not FAST2D.  The variant without them is the faster one on large
 // models (their body costs the other one registers: 1 % of the sweep over two Llama blocks).
-template <bool GENERIC>
+template <bool GENERIC, bool ARG>
 __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const pylo_tensor_desc* __restrict__ descs,
                                                               const pylo_atile* __restrict__ ttiles, int n_ttiles,
                                                               const pylo_step_params prm, int* __restrict__ status,
-                                                              int* __restrict__ host_status) {
+                                                              int* __restrict__ host_status, const __grid_constant__ TcHeads heads_arg) {
   using F = Fam<PYLO_FAM_ADAFAC>;
   using L = Fold<PYLO_FAM_ADAFAC>;
   extern __shared__ __align__(128) unsigned char tc_raw[];
@@ -308,8 +314,8 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
         const float w = __ldg(d.wfold + L::B2 + n), hi = tf32_hi(w);
         sm.b2bias[tc_b_index(n, k)] = k == 0 ? hi : (k == 1 ? w - hi : 0.f);
       }
-      if (col < 64) sm.w3[col] = __ldg(d.wfold + L::W3P + col);
-      if (col < 2) sm.w3[64 + col] = __ldg(d.wfold + L::B3 + col);
+      if (!ARG && col < 64) sm.w3[col] = __ldg(d.wfold + L::W3P + col);
+      if (!ARG && col < 2) sm.w3[64 + col] = __ldg(d.wfold + L::B3 + col);
       loaded = ct.tensor;
     }
     // per-item constants: in registers for all rows of the item
@@ -506,7 +512,13 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
         auto heads = [&](const uint32_t (&a)[16], int half) {
 #pragma unroll
           for (int jp = 0; jp < 8; ++jp) {
-            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&sm.w3[4 * (half * 8 + jp)]);  // (dir pair, mag pair)
+            ulonglong2 w;   // (dir pair, mag pair)
+            if constexpr (ARG) {
+              const float* q = &heads_arg.w[4 * (half * 8 + jp)];
+              w = make_ulonglong2(pack2(q[0], q[1]), pack2(q[2], q[3]));
+            } else {
+              w = *reinterpret_cast<const ulonglong2*>(&sm.w3[4 * (half * 8 + jp)]);
+            }
             const uint64_t r = pack2(fmaxf(__uint_as_float(a[2 * jp]), 0.f), fmaxf(__uint_as_float(a[2 * jp + 1]), 0.f));
             od[jp & 1] = fma2(w.x, r, od[jp & 1]);
             om[jp & 1] = fma2(w.y, r, om[jp & 1]);
@@ -519,7 +531,7 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
         float a, b, c, dd;
         unpack2(add2(od[0], od[1]), a, b);
         unpack2(add2(om[0], om[1]), c, dd);
-        const float o0 = (a + b) + sm.w3[64], o1 = (c + dd) + sm.w3[65];
+        const float o0 = (a + b) + (ARG ? heads_arg.b[0] : sm.w3[64]), o1 = (c + dd) + (ARG ? heads_arg.b[1] : sm.w3[65]);
         const int64_t idx = GEN ? (int64_t)x * TC_COLS + col : (int64_t)x * Y + y;
         if ((GEN ? idx < n : colok) && !timed_out) {  // after a wait that ran out the accumulators are not to be trusted: keep the old value
           const float pn = finish<PYLO_FAM_ADAFAC>(cp, o0, o1, fin);

@@ -2590,10 +2590,19 @@ int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* t
   if (n_ttiles == 0) return 0;
   // more than half an SM's shared memory is requested: one CTA per SM, which then owns all of the SM's tensor memory
   constexpr int smem = sizeof(TcSmem) > 120 * 1024 ? (int)sizeof(TcSmem) : 120 * 1024;
-  static bool configured[2][PYLO_MAX_DEVICES] = {};
-  auto kernel = generic ? k_apply_adafac_tc<true> : k_apply_adafac_tc<false>;
-  if (int rc = allow_dynamic_smem(kernel, smem, configured[generic ? 1 : 0])) return rc;
-  launch(kernel, grid_for(n_ttiles, 1), TC_NT, smem, (cudaStream_t)stream, descs, ttiles, n_ttiles, *prm, status, host_status);
+  static bool configured[4][PYLO_MAX_DEVICES] = {};
+  TcHeads heads = {};
+  if (prm->w_host) {   // w_in[32][39] b_in[32] w_h[32][32] b_h[32] w_out[2][32] b_out[2]
+    const float* w = prm->w_host + 32 * 39 + 32 + 32 * 32 + 32;
+    for (int k = 0; k < 32; ++k)
+      for (int q = 0; q < 2; ++q) heads.w[4 * (k / 2) + 2 * q + k % 2] = w[32 * q + k];
+    heads.b[0] = w[64];
+    heads.b[1] = w[65];
+  }
+  auto kernel = prm->w_host ? (generic ? k_apply_adafac_tc<true, true> : k_apply_adafac_tc<false, true>)
+                            : (generic ? k_apply_adafac_tc<true, false> : k_apply_adafac_tc<false, false>);
+  if (int rc = allow_dynamic_smem(kernel, smem, configured[(generic ? 1 : 0) + (prm->w_host ? 2 : 0)])) return rc;
+  launch(kernel, grid_for(n_ttiles, 1), TC_NT, smem, (cudaStream_t)stream, descs, ttiles, n_ttiles, *prm, status, host_status, heads);
   return launch_status();
 }
 

@@ -55,6 +55,7 @@ class _AdafacFamily(Optimizer):
         if tuple(flat[0].shape) != (32, 39):
             raise ValueError(f"{self._name} kernel only supports the 39->32->32->2 MetaMLP.")
         self._w_flat = torch.cat([t.reshape(-1) for t in flat]).to(self.device).contiguous()
+        self._w_host = self._w_flat.cpu().numpy()   # the apply sweep's launch carries its output layer
         self._plans = {}
         self._gnorm = None
         if self.mlp_precision not in ("fp32", "3xtf32"):
@@ -146,6 +147,7 @@ class _AdafacFamily(Optimizer):
         prm = self._prm
         if prm is None:
             prm = self._prm = L.StepParams()
+            prm.w_host = self._w_host.ctypes.data
             prm.family = L.FAM_ADAFAC
             for k in range(3):
                 prm.w_m[k], prm.w_f[k] = self._w_m[k], self._w_f[k]

@@ -410,14 +410,16 @@ def test_small_models_front_in_one_launch(family, extra, shapes, monkeypatch):
 
 
 @pytest.mark.parametrize("shapes", [[(40, 24), (33, 28)], [(300, 1028), (7, 4)]], ids=["small", "blocks"])
-def test_network_as_an_argument_is_the_folded_one(shapes):
-    """The packed sweep with CELO2's network as constants (features normalised) and with every unit's folded one (weights
-    normalised): a product is rounded once more or less, 2^-24 of each of 30 terms."""
+@pytest.mark.parametrize("family,extra", [("celo2", {"orthogonalize": False}), ("adafaclo", {})])
+def test_network_as_an_argument_is_the_folded_one(family, extra, shapes):
+    """CELO2's packed sweep with the network as constants (features normalised) and with every unit's folded one (weights
+    normalised): a product is rounded once more or less, 2^-24 of each of 30 terms.  AdafacLO's output layer as constants: the
+    same numbers."""
     case = dict(shapes=shapes, init_seed=51, init_scale=0.1, grad_seed=52, grad_scale=0.3)
     runs = []
     for arg in (True, False):
         params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
-        opt = _make("celo2", params, orthogonalize=False)
+        opt = _make(family, params, **extra)
         for t in (1, 2):
             for p, g in zip(params, cases.grads_at(case, t)):
                 p.grad = g.cuda()
@@ -426,4 +428,6 @@ def test_network_as_an_argument_is_the_folded_one(shapes):
             opt.step()
         runs.append([p.detach().clone() for p in params])
     for a, b, init in zip(runs[0], runs[1], cases.init_values(case)):
+        if family == "adafaclo":
+            assert torch.equal(a, b)
         assert float((a - b).abs().max()) <= 1e-5 * float((b - init.cuda()).abs().max()) + 2 ** -23 * float(b.abs().max())
