@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define PYLO_B200_ABI_VERSION 14
+#define PYLO_B200_ABI_VERSION 15
 
 /* optimizer families (which feature set / network geometry a launch uses) */
 #define PYLO_FAM_ADAFAC 0 /* AdafacLO_CUDA, ELO_CUDA: 28+11 features, 39-32-32-2 */
@@ -74,10 +74,10 @@ typedef struct pylo_tensor_desc {
   float* fac_b;   /* factored accumulator state, [3][Lb] (VEC1D: the column one or NULL) */
   float* f_a;     /* workspace [3][La]: rsqrt factor in "a" orientation */
   float* f_b;     /* workspace [3][Lb] */
-  float* fx;      /* workspace [La][4]: f_a interleaved per index (FAST2D only) */
+  float* fx;      /* workspace [La][4]: f_a interleaved per index (FAST2D, and GENERIC matrices with tables, see workspace_layout; else NULL) */
   float* sum_a;   /* workspace [La]: sum over Y of g'^2 + 1e-30 */
   float* sum_b;   /* workspace [Lb]: sum over X */
-  float* part_a;  /* workspace [X][n_cb]  row-sum partials (FAST2D) */
+  float* part_a;  /* workspace [X][n_cb]  row-sum partials (tensors in atiles; else NULL) */
   float* part_b;  /* workspace [n_strips][Lb] column-sum partials */
   float* h_a;     /* workspace [La][H] (ADAFAC) or [La][H][2] (CELO2, VELO): first-layer term of the "a" features (+ bias) */
   float* h_b;     /* workspace [H][Lb]: first-layer term of the "b" features */
@@ -169,7 +169,9 @@ int pylo_b200_sizeof_params(void);
  *
  * pylo_b200_workspace_layout fills, for one tensor of the given family, traversal mode and geometry, the size
  * in floats of every workspace sub-buffer that pylo_tensor_desc points at (0 where the mode does not use it),
- * and the phase-A tiling (rb, n_strips, n_cb) and the number of element-wise tiles that go into the descriptor.
+ * and the phase-A tiling (rb, n_strips, n_cb) and the number of element-wise tiles that go into the descriptor.  A GENERIC tensor
+ * that is a plain matrix (O = M = I = 1) may be given with its X and Y: its sums then go into the items of FAST2D tensors (atiles),
+ * and for CELO2 and VELO it has the tables of pylo_b200_apply_packed's ragged items.
  * A unit of element-wise work that is a slice of a tensor (vec_elementwise = 1) owns only the last three
  * sub-buffers (sums, wfold, tile_part), sized with n = the slice's elements, plus a zero-filled `closed`; the
  * others belong to its tensor.  Every sub-buffer must start on a 256-byte boundary and the whole workspace
@@ -222,11 +224,11 @@ int pylo_b200_grad_sumsq_static(const pylo_gvec* items, const pylo_tile* tiles, 
 
 /* Phase A: row and column sums of g'^2 + 1e-30 (the reductions inside
  * grad_sqr.mean(dim=dr / dc), AdafacLO_cuda.py:333-340, CELO2_cuda.py:218-224, velo_cuda.py:531-541).
- * atiles cover the FAST2D tensors (strip x 1024-column block each; they leave per-strip column partials, which
+ * atiles cover the FAST2D tensors, and GENERIC matrices laid out like them (the first n_ragged; strip x 1024-column block each; they leave per-strip column partials, which
  * pylo_b200_factor_update adds up).  gitems cover the GENERIC tensors: items with pad_ = 1 take 256 of the Lb columns
  * (cb) over the rows of a strip (desc.rb of the X rows), items with pad_ = 0 take cb of the La / I
  * blocks that have I row sums each, from block strip * cb on. */
-int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles,
+int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles, int n_ragged,
                           const pylo_atile* gitems, int n_gitems, const pylo_step_params* prm, void* stream);
 
 /* Phase A2, one cluster of CTAs per tensor: the sums over strips and column blocks of phase A's partials, EMA of the factored accumulators, row_col_mean,
@@ -299,9 +301,10 @@ int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* t
 /* Phase C for the FAST2D tensors of the CELO2 and VELO families (same arithmetic as pylo_b200_apply, done on
  * pairs of adjacent elements with packed fp32x2 instructions).  ctiles: strip = row-tile index, cb = column-tile
  * index, pad_ = threads per row (8 .. 256, a thread owns 4 columns) | rows per thread << 16 (0: 16); a tile has
- * rows * (256 / threads) rows and 4 * threads columns.  For these families pylo_b200_prep_apply stores desc.h_a as (v, v) pairs, [X][H][2], and
+ * rows * (256 / threads) rows and 4 * threads columns.  ragged != 0: the items are on GENERIC matrices with tables (any Y, any
+ * alignment).  For these families pylo_b200_prep_apply stores desc.h_a as (v, v) pairs, [X][H][2], and
  * for every family desc.h_b transposed, [H][Y]. */
-int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles,
+int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles, int ragged,
                            const pylo_step_params* prm, void* stream);
 
 /* Batched fp32-faithful matrix product on the tensor cores, for the Newton-Schulz orthogonalisation of the CELO2
@@ -456,10 +459,12 @@ typedef struct pylo_step_plan {
   const pylo_tensor_desc *tdesc, *desc; /* per tensor, per unit */
   const pylo_atile *atiles, *gitems, *pitems, *ctiles;
   const pylo_tile *tiles, *tiles_slow;
+  const pylo_atile* rtiles; /* CELO2, VELO: items of apply_packed on matrices with tables whose rows are not aligned */
   int *status, *host_status;
   int32_t n_tensors, n_units, n_atiles, n_gitems, n_pitems, n_ctiles, n_ctiles_gen, n_tiles, n_tiles_slow, tensor_cores;
   int32_t sum_tiles; /* 1: leave finalize_moments out and let prep_apply add up the tile partials, for units of up to
                         about 200 tiles (VELO, of any size: velo_tensor_features does it) */
+  int32_t n_ragged, n_rtiles; /* of atiles, the first that are not on FAST2D tensors; of rtiles */
   int32_t small_cluster, small_slice, small_rows, small_cols; /* small_cluster > 0: SUMS, FACTORS and STATE, asked for together,
                         are one launch of pylo_b200_small_front */
   int32_t pad_;

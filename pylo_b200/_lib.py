@@ -17,7 +17,7 @@ TILE_ELEMS = 16384
 A_COLS = 1024
 PREP_TABLE = 2048  # table entries (rows x hidden units) per item of pylo_b200_prep_apply
 WFOLD_STRIDE = 2432
-ABI_VERSION = 14
+ABI_VERSION = 15
 
 FAM_ADAFAC, FAM_CELO2, FAM_VELO = 0, 1, 2
 MODE_FAST2D, MODE_GENERIC, MODE_VEC1D = 0, 1, 2
@@ -98,9 +98,9 @@ class VeloLoss(C.Structure):
 class StepPlan(C.Structure):
     """pylo_step_plan: all tables of one optimizer's tensors."""
     _fields_ = [(name, C.c_void_p) for name in (
-        "tdesc", "desc", "atiles", "gitems", "pitems", "ctiles", "tiles", "tiles_slow", "status", "host_status")] + [
+        "tdesc", "desc", "atiles", "gitems", "pitems", "ctiles", "tiles", "tiles_slow", "rtiles", "status", "host_status")] + [
         (name, C.c_int32) for name in ("n_tensors", "n_units", "n_atiles", "n_gitems", "n_pitems", "n_ctiles", "n_ctiles_gen",
-                                       "n_tiles", "n_tiles_slow", "tensor_cores", "sum_tiles", "small_cluster", "small_slice",
+                                       "n_tiles", "n_tiles_slow", "tensor_cores", "sum_tiles", "n_ragged", "n_rtiles", "small_cluster", "small_slice",
                                        "small_rows", "small_cols", "pad_")]
 
 
@@ -127,7 +127,7 @@ def _load():
         "pylo_b200_workspace_bytes": [C.POINTER(WsLayout), i32, i32],
         "pylo_b200_grad_sumsq": [vp, vp, i32, vp, vp, vp],
         "pylo_b200_grad_sumsq_static": [vp, vp, i32, vp, vp],
-        "pylo_b200_rowcol_sums": [vp, vp, i32, vp, i32, C.POINTER(StepParams), vp],
+        "pylo_b200_rowcol_sums": [vp, vp, i32, i32, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_factor_update": [vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_state_moments": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_small_front": [vp, i32, i32, i32, i32, i32, C.POINTER(StepParams), vp],
@@ -136,7 +136,7 @@ def _load():
         "pylo_b200_apply": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply_adafac_cols": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply_adafac_tc": [vp, vp, i32, i32, C.POINTER(StepParams), vp, vp, vp],
-        "pylo_b200_apply_packed": [vp, vp, i32, C.POINTER(StepParams), vp],
+        "pylo_b200_apply_packed": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_gemm_tn_3xtf32": [C.POINTER(GemmDesc), vp, vp],
         "pylo_b200_transpose": [vp, vp, i32, i32, i32, i32, C.c_int64, C.c_int64, i32, i32, vp],
         "pylo_b200_newton_schulz_workspace": [i32, i32, i32, i32],

@@ -94,8 +94,10 @@ __global__ void __launch_bounds__(1024) k_sum_final(const float* __restrict__ sc
 // (512 columns) of the block each, so that a lane keeps 16 column accumulators (not 32) and has room to request its next
 // row before it adds up the present one: the loads of the next row fly during the shuffles of this one's row sum.
 // 355 M elements (GPT-2-medium shapes): 417 us before (a warp per row, 32 accumulators, no row ahead).
+// Matrices whose rows are not aligned (GENERIC, with part_a) go the same way with single loads (not VEC), a piece's columns 32 apart.
 #define RC_GROUPS 4
-__global__ void __launch_bounds__(NT, 4) k_rowcol_fast(const pylo_tensor_desc* __restrict__ descs,
+template <bool VEC>
+__global__ void __launch_bounds__(NT, VEC ? 4 : 3) k_rowcol_fast(const pylo_tensor_desc* __restrict__ descs,
                                                        const pylo_atile* __restrict__ atiles, int n_atiles,
                                                        const pylo_step_params prm) {
   pdl_begin();
@@ -111,17 +113,26 @@ __global__ void __launch_bounds__(NT, 4) k_rowcol_fast(const pylo_tensor_desc* _
     const int col0 = at.cb * PYLO_A_COLS;
     const float gs = grad_scale_of(d, prm);
     const bool plain = plain_grad(gs, prm);
-    const int c0 = half * 512 + lane * 4;
+    const int c0 = half * 512 + (VEC ? lane * 4 : lane);
     const float* base = d.g + (int64_t)row0 * Y + col0 + c0;
-    const int left = Y - col0 - c0;   // columns of this lane's pieces that exist: piece j is there if j * 128 < left
+    const int left = Y - col0 - c0;   // columns of this lane's pieces that exist: VEC: piece j is there if j * 128 < left, else column k if k * 32 is
     float colacc[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) colacc[j] = 0.f;
     float4 cur[4], nxt[4];
     auto load = [&](int r, float4 (&q)[4]) {
+      const float* p = base + (int64_t)r * Y;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j * 128 < left) q[j] = ldg4(base + (int64_t)r * Y + j * 128);
+      for (int j = 0; j < 4; ++j) {
+        if constexpr (VEC) {
+          if (j * 128 < left) q[j] = ldg4(p + j * 128);
+        } else {
+          if (j * 128 < left) q[j].x = __ldg(p + j * 128);
+          if (j * 128 + 32 < left) q[j].y = __ldg(p + j * 128 + 32);
+          if (j * 128 + 64 < left) q[j].z = __ldg(p + j * 128 + 64);
+          if (j * 128 + 96 < left) q[j].w = __ldg(p + j * 128 + 96);
+        }
+      }
     };
     if (grp < rows) load(grp, cur);
     for (int r = grp; r < rows; r += RC_GROUPS) {
@@ -133,6 +144,7 @@ __global__ void __launch_bounds__(NT, 4) k_rowcol_fast(const pylo_tensor_desc* _
           const float e[4] = {cur[j].x, cur[j].y, cur[j].z, cur[j].w};
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
+            if (!VEC && j * 128 + u * 32 >= left) continue;
             const float g = plain ? e[u] : xform_grad(e[u], gs, prm.clip_val, prm.nan_to_num);
             const float q = g * g + 1e-30f;
             colacc[j * 4 + u] += q;
@@ -146,9 +158,14 @@ __global__ void __launch_bounds__(NT, 4) k_rowcol_fast(const pylo_tensor_desc* _
       for (int j = 0; j < 4; ++j) cur[j] = nxt[j];
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) st4(&s_col[grp][c0 + j * 128], make_float4(colacc[j * 4], colacc[j * 4 + 1], colacc[j * 4 + 2], colacc[j * 4 + 3]));
+    for (int j = 0; j < 4; ++j) {
+      if constexpr (VEC) st4(&s_col[grp][c0 + j * 128], make_float4(colacc[j * 4], colacc[j * 4 + 1], colacc[j * 4 + 2], colacc[j * 4 + 3]));
+      else
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s_col[grp][c0 + j * 128 + u * 32] = colacc[j * 4 + u];
+    }
     __syncthreads();
-    {
+    if constexpr (VEC) {
       const int c = threadIdx.x * 4;
       if (col0 + c < Y) {
         float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -159,8 +176,15 @@ __global__ void __launch_bounds__(NT, 4) k_rowcol_fast(const pylo_tensor_desc* _
         }
         st4(d.part_b + (int64_t)at.strip * Y + col0 + c, tot);
       }
-      if (threadIdx.x < rows) d.part_a[(int64_t)(row0 + threadIdx.x) * d.n_cb + at.cb] = s_row[threadIdx.x][0] + s_row[threadIdx.x][1];
+    } else {
+      for (int c = threadIdx.x; c < PYLO_A_COLS && col0 + c < Y; c += NT) {
+        float tot = 0.f;
+#pragma unroll
+        for (int w = 0; w < RC_GROUPS; ++w) tot += s_col[w][c];
+        d.part_b[(int64_t)at.strip * Y + col0 + c] = tot;
+      }
     }
+    if (threadIdx.x < rows) d.part_a[(int64_t)(row0 + threadIdx.x) * d.n_cb + at.cb] = s_row[threadIdx.x][0] + s_row[threadIdx.x][1];
     __syncthreads();
   }
 }
@@ -327,7 +351,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
     return;
   }
   cluster_arrive();   // waited for below, before the first store into another CTA
-  const bool fast = d.mode == PYLO_MODE_FAST2D, r_is_a = d.r_is_a != 0;
+  const bool blocks = d.part_a != nullptr, r_is_a = d.r_is_a != 0;   // blocks: phase A has left row sums per block of columns
   const int64_t La = d.La, Lb = d.Lb;
   const float inv_n_a = (float)d.Y, inv_n_b = (float)d.X;
   float acc[NS];
@@ -346,7 +370,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
 #pragma unroll
     for (int k = 0; k < 3; ++k) old[k] = d.fac_a[k * La + i];
     float s;
-    if (fast) {
+    if (blocks) {
       s = 0.f;
 #pragma unroll 4
       for (int c = 0; c < d.n_cb; ++c) s += d.part_a[i * d.n_cb + c];
@@ -366,7 +390,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
     if (!r_is_a) {  // col_factor = safe_rsqrt(fac_c)
 #pragma unroll
       for (int k = 0; k < 3; ++k) d.f_a[k * La + i] = f[k];
-      if (fast) st4(d.fx + 4 * i, make_float4(f[0], f[1], f[2], 0.f));
+      if (d.fx) st4(d.fx + 4 * i, make_float4(f[0], f[1], f[2], 0.f));
     }
   }
   // 2. "b" vectors: sum over the strips (in a fixed order), EMA
@@ -436,7 +460,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
       const float f1 = safe_rsqrt(v1 / ((whole ? s_tot[1] / (float)A : own) + 1e-9f));
       const float f2 = safe_rsqrt(v2 / ((whole ? s_tot[2] / (float)A : own) + 1e-9f));
       f_r[i] = f0; f_r[Lr + i] = f1; f_r[2 * Lr + i] = f2;
-      if (fast && r_is_a) st4(d.fx + 4 * i, make_float4(f0, f1, f2, 0.f));
+      if (d.fx && r_is_a) st4(d.fx + 4 * i, make_float4(f0, f1, f2, 0.f));
     }
   } else if (post == 1) {
     const int lane = tid & 31;
@@ -651,7 +675,7 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
       const int64_t La = d.La, Lb = d.Lb;
       const bool vecf = d.vec_elementwise != 0;
       GenPos pos(d, d.idx0 + start + tid, NT);
-      constexpr int U = 2;   // elements of a thread in flight (four cost the float4 path its second CTA per SM)
+      constexpr int U = 4;   // elements of a thread in flight; their factors, from L1, are fetched when they are needed
       auto update = [&](float g, float& m0, float& m1, float& m2, float& v) {
         velo_stats<FAM>(acc, m0, m1, m2, v);
         m0 = lerp_torch(m0, g, prm.w_m[0]);
@@ -661,28 +685,27 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
       };
       if (!vecf) {
         for (int i0 = tid; i0 < cnt; i0 += U * NT) {
-          float g[U], p[U], m0[U], m1[U], m2[U], v[U], k0[U], k1[U], k2[U];
+          float g[U], p[U], m0[U], m1[U], m2[U], v[U];
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const int i = i0 + u * NT;
-            if (i < cnt) {
-              g[u] = __ldg(gp + i); p[u] = pp[i]; m0[u] = m0p[i]; m1[u] = m1p[i]; m2[u] = m2p[i]; v[u] = vp[i];
-              const int64_t a = pos.a(), b = pos.b();
-              k0[u] = d.f_a[a] * d.f_b[b]; k1[u] = d.f_a[La + a] * d.f_b[Lb + b]; k2[u] = d.f_a[2 * La + a] * d.f_b[2 * Lb + b];
-            }
-            pos.next();
+            if (i < cnt) { g[u] = __ldg(gp + i); p[u] = pp[i]; m0[u] = m0p[i]; m1[u] = m1p[i]; m2[u] = m2p[i]; v[u] = vp[i]; }
           }
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const int i = i0 + u * NT;
             if (i < cnt) {
+              const int64_t a = pos.a(), b = pos.b();
+              const float k0 = __ldg(d.f_a + a) * __ldg(d.f_b + b), k1 = __ldg(d.f_a + La + a) * __ldg(d.f_b + Lb + b),
+                          k2 = __ldg(d.f_a + 2 * La + a) * __ldg(d.f_b + 2 * Lb + b);
               const float gx = xform_grad(g[u], gs, prm.clip_val, prm.nan_to_num);
               update(gx, m0[u], m1[u], m2[u], v[u]);
               m0p[i] = m0[u]; m1p[i] = m1[u]; m2p[i] = m2[u]; vp[i] = v[u];
               float f[F::NF];
-              elem_features<FAM>(f, gx, p[u], m0[u], m1[u], m2[u], v[u], rsqrtf(v[u] + prm.eps_feat), k0[u], k1[u], k2[u]);
+              elem_features<FAM>(f, gx, p[u], m0[u], m1[u], m2[u], v[u], rsqrtf(v[u] + prm.eps_feat), k0, k1, k2);
               accumulate<FAM, false>(acc, f);
             }
+            pos.next();
           }
         }
       } else {
@@ -801,7 +824,7 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
   for (int e = tid; e < o_end; e += NT) copy(s_net + e, d.w + e);
   // the table entries of this item: of the "a" or of the "b" index
   const int La = d.X, Lb = d.Y, items_a = (La + PER - 1) / PER;
-  const bool tables = d.mode == PYLO_MODE_FAST2D && prm.no_tables != 1, of_a = it.strip < items_a;
+  const bool tables = d.fx && prm.no_tables != 1, of_a = it.strip < items_a;
   const int i0 = (of_a ? it.strip : it.strip - items_a) * PER, end = tables && (of_a || prm.no_tables != 2) ? min(of_a ? La : Lb, i0 + PER) : 0;
   for (int e = tid; e < 3 * PER; e += NT) {
     const int k = e / PER, i = i0 + e % PER;
@@ -1452,7 +1475,9 @@ __device__ __forceinline__ float4 ld4_early(const float* p) {
 #define PK_CTAS_CELO2 1   // its 8-wide layers want registers more than a second CTA (224 bytes of spills: 2357 -> 2435 us over a Llama block)
 #endif
 // ARG: one network for all units, which comes as an argument of the launch; the features are normalised instead of the weights.
-template <int FAM, bool ARG>
+// RAGGED: matrices whose rows do not start on 16-byte boundaries: a thread's four columns are a tile's quarter apart, so that a
+// warp's single accesses are to neighbouring elements.
+template <int FAM, bool ARG, bool RAGGED>
 __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_CTAS_CELO2) k_apply_packed(const pylo_tensor_desc* __restrict__ descs,
                                                         const pylo_atile* __restrict__ ctiles, int n_ctiles,
                                                         const pylo_step_params prm, const __grid_constant__ PkNet<FAM> net) {
@@ -1498,9 +1523,13 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
         return;
       }
     }
-    const int y = y0 + 4 * (tid % tpr), rg = tid / tpr;
+    const int y = y0 + (RAGGED ? tid % tpr : 4 * (tid % tpr)), rg = tid / tpr;
     const bool colok = y < Y;
     const int yc = colok ? y : 0;
+    int yu[4];   // RAGGED: the thread's columns, or 0 where there is none
+#pragma unroll
+    for (int u = 0; u < 4; ++u) yu[u] = y + u * tpr < Y ? y + u * tpr : 0;
+    auto columns = [&](const float* p) { return RAGGED ? make_float4(__ldg(p + yu[0]), __ldg(p + yu[1]), __ldg(p + yu[2]), __ldg(p + yu[3])) : ldg4(p + yc); };
     // VeLO: p + rate * (...), then + decay * that (lr_eff may have either sign)
     const float exp_mult = d.exp_mult, rate = -(s_sc[1] * s_sc[0] * d.step_mult), decay = d.wd > 0.f ? -(d.wd * s_sc[1]) : 0.f;
     const float gs = grad_scale_of(d, prm);
@@ -1510,13 +1539,13 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
     uint64_t hb[2][H], fb[2][3];
 #pragma unroll
     for (int j = 0; j < H; ++j) {
-      const float4 q = ldg4(d.h_b + (int64_t)j * Y + yc);
+      const float4 q = columns(d.h_b + (int64_t)j * Y);
       hb[0][j] = pack2(q.x, q.y);
       hb[1][j] = pack2(q.z, q.w);
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float4 q = ldg4(d.f_b + (int64_t)k * Y + yc);
+      const float4 q = columns(d.f_b + (int64_t)k * Y);
       fb[0][k] = pack2(q.x, q.y);
       fb[1][k] = pack2(q.z, q.w);
     }
@@ -1532,8 +1561,14 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
     float4 cg, cp, cm0, cm1, cm2, cv;
     auto load_row = [&](int q, float4& g, float4& p, float4& m0, float4& m1, float4& m2, float4& v) {
       const int x = x0 + rg + ng * q;
-      const int64_t idx = (colok && x < X) ? (int64_t)x * Y + y : 0;
-      g = ld4_early(gp + idx); p = ld4_early(pp + idx); m0 = ld4_early(mp + idx); m1 = ld4_early(mp + n + idx); m2 = ld4_early(mp + 2 * n + idx); v = ld4_early(vp + idx);
+      if constexpr (RAGGED) {
+        const int64_t at = x < X ? (int64_t)x * Y : 0;
+        auto four = [&](const float* p) { return make_float4(ldg_early(p + yu[0]), ldg_early(p + yu[1]), ldg_early(p + yu[2]), ldg_early(p + yu[3])); };
+        g = four(gp + at); p = four(pp + at); m0 = four(mp + at); m1 = four(mp + n + at); m2 = four(mp + 2 * n + at); v = four(vp + at);
+      } else {
+        const int64_t idx = (colok && x < X) ? (int64_t)x * Y + y : 0;
+        g = ld4_early(gp + idx); p = ld4_early(pp + idx); m0 = ld4_early(mp + idx); m1 = ld4_early(mp + n + idx); m2 = ld4_early(mp + 2 * n + idx); v = ld4_early(vp + idx);
+      }
     };
     load_row(0, cg, cp, cm0, cm1, cm2, cv);
     const int sub = min(PK_ROWS, PK_STAGE / ng);   // rows per thread and stage
@@ -1667,8 +1702,19 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
         } else {
           res = make_float4(d0 * __expf(m0 * exp_mult), d1 * __expf(m1 * exp_mult), d2 * __expf(m2 * exp_mult), d3 * __expf(m3 * exp_mult));
         }
-        st4(op + (int64_t)x * Y + y, res);
-        if (FAM != PYLO_FAM_CELO2) peer_store4(peers, (int64_t)x * Y + y, res);
+        if constexpr (RAGGED) {
+          const float r4[4] = {res.x, res.y, res.z, res.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (y + u * tpr < Y) {
+              const int64_t at = (int64_t)x * Y + y + u * tpr;
+              op[at] = r4[u];
+              if (FAM != PYLO_FAM_CELO2) peer_store(peers, at, r4[u]);
+            }
+        } else {
+          st4(op + (int64_t)x * Y + y, res);
+          if (FAM != PYLO_FAM_CELO2) peer_store4(peers, (int64_t)x * Y + y, res);
+        }
       }
       if (q + 1 < rpt) { cg = ng_; cp = np_; cm0 = nm0; cm1 = nm1; cm2 = nm2; cv = nv; }
     }
@@ -2374,16 +2420,15 @@ int pylo_b200_workspace_layout(int family, int mode, int64_t n, int64_t La, int6
     CHECK_ARG(La > 0 && Lb > 0);
     w.f_a = 3 * La; w.f_b = 3 * Lb; w.sum_a = La; w.sum_b = Lb;
   }
-  if (mode == PYLO_MODE_GENERIC) {
+  if (mode == PYLO_MODE_GENERIC && X <= 0) {
     CHECK_ARG(n % Lb == 0);
     const int64_t rows = n / Lb;   // X
     // rows per strip of the column sums: one thread adds up a strip's rows, and 256 columns are one item
     w.rb = rows <= 512 ? 16 : (rows <= 2048 ? 32 : PYLO_A_ROWS_MAX);
     w.n_strips = (int32_t)((rows + w.rb - 1) / w.rb);
     w.part_b = w.n_strips * Lb;
-  }
-  if (mode == PYLO_MODE_FAST2D) {
-    CHECK_ARG(X > 0 && Y > 0 && Y % 4 == 0 && La == X && Lb == Y);
+  } else if (mode != PYLO_MODE_VEC1D) {
+    CHECK_ARG(X > 0 && Y > 0 && La == X && Lb == Y && (Y % 4 == 0 || mode == PYLO_MODE_GENERIC));
     // rows per strip: about X / 128, a multiple of 8, within [32, 128].  Up to 512 rows a tensor gives too few strips of
     // 32 to fill the GPU and the launch is all latency: strips of 8 (one or two rows per warp) there.
     int rb = (((X + 127) / 128 + 7) / 8) * 8;
@@ -2391,11 +2436,13 @@ int pylo_b200_workspace_layout(int family, int mode, int64_t n, int64_t La, int6
     w.rb = rb;
     w.n_strips = (X + rb - 1) / rb;
     w.n_cb = (Y + PYLO_A_COLS - 1) / PYLO_A_COLS;
-    w.fx = 4 * La;
     w.part_a = (int64_t)X * w.n_cb;
     w.part_b = (int64_t)w.n_strips * Y;
-    w.h_a = La * H * 2;
-    w.h_b = Lb * H;
+    if (mode == PYLO_MODE_FAST2D || family != PYLO_FAM_ADAFAC) {   // what the tiled apply sweeps read
+      w.fx = 4 * La;
+      w.h_a = La * H * 2;
+      w.h_b = Lb * H;
+    }
   }
   w.closed = PYLO_STAT_STRIDE;
   w.n_tiles = (int32_t)((n + PYLO_TILE_ELEMS - 1) / PYLO_TILE_ELEMS);
@@ -2476,14 +2523,12 @@ int pylo_b200_grad_sumsq_static(const pylo_gvec* items, const pylo_tile* tiles, 
   return launch_status();
 }
 
-int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles,
+int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles, int n_ragged,
                           const pylo_atile* gitems, int n_gitems, const pylo_step_params* prm, void* stream) {
-  CHECK_ARG(descs && prm && n_atiles >= 0 && n_gitems >= 0);
+  CHECK_ARG(descs && prm && n_ragged >= 0 && n_atiles >= n_ragged && n_gitems >= 0 && (atiles || !n_atiles));
   cudaStream_t s = (cudaStream_t)stream;
-  if (n_atiles > 0) {
-    CHECK_ARG(atiles);
-    launch(k_rowcol_fast, grid_for(n_atiles, 4), NT, 0, s, descs, atiles, n_atiles, *prm);
-  }
+  if (n_ragged > 0) launch(k_rowcol_fast<false>, grid_for(n_ragged, 3), NT, 0, s, descs, atiles, n_ragged, *prm);
+  if (n_atiles > n_ragged) launch(k_rowcol_fast<true>, grid_for(n_atiles - n_ragged, 4), NT, 0, s, descs, atiles + n_ragged, n_atiles - n_ragged, *prm);
   if (n_gitems > 0) {
     CHECK_ARG(gitems);
     launch(k_rowcol_generic, n_gitems, NT, 0, s, descs, gitems, *prm);
@@ -2828,7 +2873,7 @@ int pylo_b200_newton_schulz_launches(const pylo_ns_desc* descs, int n) {
   return groups(in_clusters) + single + groups(chains) * (2 + 3 * (n ? descs[0].iters : 0));
 }
 
-int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles,
+int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles, int ragged,
                            const pylo_step_params* prm, void* stream) {
   CHECK_ARG(descs && ctiles && prm && n_ctiles >= 0);
   if (n_ctiles == 0) return 0;
@@ -2843,15 +2888,18 @@ int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctil
         for (int e = 0; e < 64; ++e) net.w[W::W2 + e] = w[248 + e];
         for (int e = 0; e < 8; ++e) { net.w[W::B2 + e] = w[312 + e]; net.w[W::W3 + 2 * e] = w[320 + 3 * e]; net.w[W::W3 + 2 * e + 1] = w[321 + 3 * e]; }
         net.w[W::B3] = w[344]; net.w[W::B3 + 1] = w[345];
-        launch(k_apply_packed<PYLO_FAM_CELO2, true>, grid_for(n_ctiles, PK_CTAS_CELO2), NT, 0, s, descs, ctiles, n_ctiles, *prm, net);
-      } else {
-        launch(k_apply_packed<PYLO_FAM_CELO2, false>, grid_for(n_ctiles, PK_CTAS_CELO2), NT, 0, s, descs, ctiles, n_ctiles, *prm, net);
       }
+      auto kernel = prm->w_host ? (ragged ? k_apply_packed<PYLO_FAM_CELO2, true, true> : k_apply_packed<PYLO_FAM_CELO2, true, false>)
+                                : (ragged ? k_apply_packed<PYLO_FAM_CELO2, false, true> : k_apply_packed<PYLO_FAM_CELO2, false, false>);
+      launch(kernel, grid_for(n_ctiles, PK_CTAS_CELO2), NT, 0, s, descs, ctiles, n_ctiles, *prm, net);
       break;
     }
     // four times the CTAs that fit: an SM that is done takes the next (17 M parameters: 341 -> 327 us per step, 67 M: 1104 ->
     // 1091); CELO2's larger network is loaded by every CTA, which costs more than that gives
-    case PYLO_FAM_VELO: launch(k_apply_packed<PYLO_FAM_VELO, false>, grid_for(n_ctiles, 4 * PK_CTAS_VELO), NT, 0, s, descs, ctiles, n_ctiles, *prm, PkNet<PYLO_FAM_VELO>{}); break;
+    case PYLO_FAM_VELO:
+      launch(ragged ? k_apply_packed<PYLO_FAM_VELO, false, true> : k_apply_packed<PYLO_FAM_VELO, false, false>, grid_for(n_ctiles, 4 * PK_CTAS_VELO), NT, 0, s,
+             descs, ctiles, n_ctiles, *prm, PkNet<PYLO_FAM_VELO>{});
+      break;
     default: return -2;
   }
   return launch_status();
@@ -2943,7 +2991,7 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
     phases &= ~front;
   }
   if ((phases & PYLO_STEP_SUMS) && (p->n_atiles || p->n_gitems))
-    if ((rc = pylo_b200_rowcol_sums(p->tdesc, p->atiles, p->n_atiles, p->gitems, p->n_gitems, prm, stream))) return rc;
+    if ((rc = pylo_b200_rowcol_sums(p->tdesc, p->atiles, p->n_atiles, p->n_ragged, p->gitems, p->n_gitems, prm, stream))) return rc;
   if (phases & PYLO_STEP_FACTORS)
     if ((rc = pylo_b200_factor_update(p->tdesc, p->n_tensors, prm, stream))) return rc;
   if (phases & PYLO_STEP_STATE)
@@ -2966,9 +3014,11 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
   }
   if (main && p->n_ctiles) {
     rc = q.family == PYLO_FAM_ADAFAC ? pylo_b200_apply_adafac_cols(p->desc, p->ctiles, p->n_ctiles, &q, stream)
-                                     : pylo_b200_apply_packed(p->desc, p->ctiles, p->n_ctiles, &q, stream);
+                                     : pylo_b200_apply_packed(p->desc, p->ctiles, p->n_ctiles, 0, &q, stream);
     if (rc) return rc;
   }
+  if (rest && p->n_rtiles)
+    if ((rc = pylo_b200_apply_packed(p->desc, p->rtiles, p->n_rtiles, 1, &q, stream))) return rc;
   if (rest && p->n_tiles_slow) return pylo_b200_apply(p->desc, p->tiles_slow, p->n_tiles_slow, 0, &q, stream);
   return 0;
 }

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(SF_NT, 1) k_small_front(const pylo_tensor_desc
     float f[3];
     factors(r_is_a, X, s_fa + i, shape.rows, d.fac_a + row0 + i, d.f_a + row0 + i, true, f);
     d.sum_a[row0 + i] = s_rs[i];
-    if (fast) st4(d.fx + 4 * (int64_t)(row0 + i), make_float4(f[0], f[1], f[2], 0.f));
+    if (d.fx) st4(d.fx + 4 * (int64_t)(row0 + i), make_float4(f[0], f[1], f[2], 0.f));
   }
   for (int y = tid; y < Y; y += SF_NT) {   // every CTA all columns
     float f[3];

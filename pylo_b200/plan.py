@@ -172,20 +172,21 @@ class DeviceTable:
         self._events[i] = ev
 
 
-def apply_tile_shape(family: int, X: int, Y: int):
+def apply_tile_shape(family: int, X: int, Y: int, least: int = 8):
     """(rows per work item, columns per work item, tag for ``pylo_atile.pad_``) of a FAST2D tensor's apply sweep on the CUDA
     cores.
 
     * AdafacLO family: n_sub sub-tiles of 32 rows in one block of 32..256 columns, as long as possible while the tensor
       still yields >= 8 items per SM; tag = columns | n_sub << 16;
-    * CELO2 / VeLO: four columns per thread, 16 rows per thread (see :func:`packed_rows`), tag = threads per row.
+    * CELO2 / VeLO: four columns per thread, 16 rows per thread (see :func:`packed_rows`), tag = threads per row (at least
+      ``least``).
     """
     if family == L.FAM_ADAFAC:
         cw = min((256, 128, 64, 32), key=lambda c: ((Y + c - 1) // c * c - Y, -c))
         ncol = (Y + cw - 1) // cw
         n_sub = next((k for k in (8, 4, 2) if ((X + 32 * k - 1) // (32 * k)) * ncol >= 1184), 1)
         return 32 * n_sub, cw, cw | (n_sub << 16)
-    tpr = min((256, 128, 64, 32, 16, 8), key=lambda c: ((Y + 4 * c - 1) // (4 * c) * 4 * c - Y, -c))
+    tpr = min([c for c in (256, 128, 64, 32, 16, 8) if c >= least], key=lambda c: ((Y + 4 * c - 1) // (4 * c) * 4 * c - Y, -c))
     return 16 * (256 // tpr), 4 * tpr, tpr
 
 
@@ -207,7 +208,16 @@ def packed_rows(tiles: Sequence[Tuple[int, int, int, int]]) -> int:
     return next((k for k in (64, 32, 16, 8, 4) if n_items(k) >= (16 if k > 16 else 4) * L.SM_COUNT), 2)
 
 
-def apply_items(family: int, tensor_cores: bool, fast, slow) -> np.ndarray:
+def ragged_rows(family: int, tiles: Sequence[Tuple[int, int, int, int]]) -> int:
+    """Rows per thread of the packed sweep over matrices whose rows are not aligned: the number that makes the longest share of a
+    CTA shortest; a tile's start counts as a row (VeLO over 3.4 M parameters, us per step with 4, 8, 16, 32 rows: 128.3, 128.8,
+    134.9, 171.2, over 33 M 576.9, 551.2, 550.1, 557.2; CELO2 over 3.4 M 141.1, 134.7, 144.1, 144.6)."""
+    ctas = L.SM_COUNT * (2 if family == L.FAM_VELO else 1)
+    n_items = lambda k: sum(-(-X // (rt * k // 16)) * -(-Y // w) for X, Y, rt, w in tiles)
+    return min((64, 32, 16, 8, 4), key=lambda k: -(-n_items(k) // ctas) * (k + 1))
+
+
+def apply_items(family: int, tensor_cores: bool, fast, slow, least: int = 8) -> np.ndarray:
     """Work list of the tiled apply sweep: ``fast`` = [(unit, rows, columns)] of the FAST2D units, ``slow`` = [(unit,
     elements)] of the others, which only the tensor-core kernel takes (as runs of 128 elements, first in the list)."""
     if tensor_cores:
@@ -215,9 +225,10 @@ def apply_items(family: int, tensor_cores: bool, fast, slow) -> np.ndarray:
         rt = tensor_core_rows([(X, Y) for _, X, Y, _ in parts])
         parts = [(u, X, Y, rt, 128, tag | rt) for u, X, Y, tag in parts]
     else:
-        parts = [(u, X, Y) + apply_tile_shape(family, X, Y) for u, X, Y in fast]
+        parts = [(u, X, Y) + apply_tile_shape(family, X, Y, least) for u, X, Y in fast]
         if family != L.FAM_ADAFAC:
-            k = packed_rows([(X, Y, rt, w) for _, X, Y, rt, w, _ in parts])
+            shapes = [(X, Y, rt, w) for _, X, Y, rt, w, _ in parts]
+            k = packed_rows(shapes) if least == 8 else ragged_rows(family, shapes)
             parts = [(u, X, Y, rt * k // 16, w, tag | k << 16) for u, X, Y, rt, w, tag in parts]
     return atile_list([atile_grid(u, -(-X // rt), -(-Y // w), tag) for u, X, Y, rt, w, tag in parts])
 
@@ -264,8 +275,9 @@ class LoPlan:
         H = self.H[family]
         tdesc = np.zeros(T, dtype=L.DESC_DTYPE)
         ws_items = []  # (table, row, field, count)
-        atiles, gitems = [], []
+        atiles, ratiles, gitems = [], [], []
         ws_bytes = 0  # the library's own count of the workspace, checked against the layout below
+        plain = []    # per tensor: whether it is a matrix that phase A takes in strips and blocks of columns
         for i, t in enumerate(tensors):
             shape = tuple(t.p.shape)
             n = t.p.numel()
@@ -289,6 +301,7 @@ class LoPlan:
                 d["p_peer"][: len(t.peer_ptrs)] = list(t.peer_ptrs)
                 d["n_peer"] = -1 if t.peer_multicast else len(t.peer_ptrs)
             if t.fdims is None:
+                plain.append(False)
                 d["mode"] = L.MODE_VEC1D
                 d["O"] = d["X"] = d["M"] = d["I"] = 1
                 d["Y"] = min(n, 2**31 - 1)
@@ -309,15 +322,19 @@ class LoPlan:
                 fast = (O == 1 and M == 1 and I == 1 and Y % 4 == 0 and n < 2**31
                         and not (t.slice_last2 and t.p.dim() > 2) and _aligned16(t.p, t.m, t.v, t.out))
                 d["mode"] = L.MODE_FAST2D if fast else L.MODE_GENERIC
+                # matrices whose rows are not aligned go the way of the others with single accesses, where a warp finds its 32
+                # columns twice: 3.4 M VeLO parameters in rows of 1433 and 1001, sums 25.8 -> 13.5 us, apply sweep 68 -> 33
+                sliced = t.slice_last2 and t.p.dim() > 2
+                ragged = not fast and not sliced and O == M == I == 1 and Y >= 64
+                plain.append(fast or ragged)
                 # sub-buffer sizes and the phase-A tiling come from the library (pylo_b200_workspace_layout), so that
                 # this table and a table built by any other host of the C ABI agree
-                ws = L.workspace_layout(family, int(d["mode"]), n, La, Lb, X if fast else 0, Y if fast else 0)
+                ws = L.workspace_layout(family, int(d["mode"]), n, La, Lb, X if fast or ragged else 0, Y if fast or ragged else 0)
                 ws_items += [("t", i, f, getattr(ws, f)) for f in ("f_a", "f_b", "sum_a", "sum_b")]
                 d["rb"], d["n_strips"], d["n_cb"] = ws.rb, ws.n_strips, ws.n_cb
-                if fast:
-                    assert ws.h_a == La * H * 2
-                    ws_items += [("t", i, f, getattr(ws, f)) for f in ("fx", "part_a", "part_b", "h_a", "h_b")]
-                    atiles.append(atile_grid(i, ws.n_strips, ws.n_cb))
+                if fast or ragged:
+                    ws_items += [("t", i, f, getattr(ws, f)) for f in ("fx", "part_a", "part_b", "h_a", "h_b") if getattr(ws, f)]
+                    (atiles if fast else ratiles).append(atile_grid(i, ws.n_strips, ws.n_cb))
                 else:
                     ws_items.append(("t", i, "part_b", ws.part_b))
                     gitems.append(atile_grid(i, ws.n_strips, (Lb + 255) // 256, 1))
@@ -328,8 +345,7 @@ class LoPlan:
             ws_items.append(("t", i, "closed", L.STAT_STRIDE))
             ws_bytes += L.lib.pylo_b200_workspace_bytes(
                 C.byref(L.workspace_layout(family, int(d["mode"]), n, int(d["La"]), int(d["Lb"]),
-                                           int(d["X"]) if d["mode"] == L.MODE_FAST2D else 0,
-                                           int(d["Y"]) if d["mode"] == L.MODE_FAST2D else 0)), 1, 0)
+                                           int(d["X"]) if plain[i] else 0, int(d["Y"]) if plain[i] else 0)), 1, 0)
 
         # units of element-wise work
         self.sliced = any(t.slice_last2 and t.p.dim() > 2 for t in tensors)
@@ -397,8 +413,8 @@ class LoPlan:
         self.desc = DeviceTable(udesc, self.device) if self.sliced else self.tdesc
         self.tiles = DeviceTable(tiles, self.device)
         self.n_tiles = len(tiles)
-        self.atiles = DeviceTable(atile_list(atiles), self.device)
-        self.n_atiles = len(self.atiles.host)
+        self.atiles = DeviceTable(atile_list(ratiles + atiles), self.device)
+        self.n_atiles, self.n_ragged = len(self.atiles.host), len(atile_list(ratiles))
         self.gitems = DeviceTable(atile_list(gitems), self.device)
         self.n_gitems = len(self.gitems.host)
         self.n_tensors = T
@@ -413,17 +429,20 @@ class LoPlan:
         pitems[0][:, 0] = np.arange(U)
         per = L.PREP_TABLE // H
         unit_of = {i: u for u, (i, _) in enumerate(unit_owner)}  # a FAST2D tensor is never sliced: one unit
+        ragged = []
         for i in range(T):
-            if tdesc["mode"][i] != L.MODE_FAST2D:
+            if not tdesc["h_a"][i]:
                 continue
             X, Y = int(tdesc["X"][i]), int(tdesc["Y"][i])
             # the tensor-core kernel reads the per-row table only, the CUDA-core kernels both
             parts = (X + per - 1) // per + (0 if self.tensor_cores else (Y + per - 1) // per)
             pitems.append(atile_grid(unit_of[i], parts, 1)[1:])
-            fast.append((unit_of[i], X, Y))
-        slow_units = [u for u in range(U) if udesc["mode"][u] != L.MODE_FAST2D]
+            (fast if tdesc["mode"][i] == L.MODE_FAST2D else ragged).append((unit_of[i], X, Y))
+        slow_units = [u for u in range(U) if not tdesc["h_a"][unit_owner[u][0]]]
         self.ctiles = DeviceTable(apply_items(family, self.tensor_cores, fast, [(u, sizes[u]) for u in slow_units]), self.device)
         self.n_ctiles = len(self.ctiles.host)
+        self.rtiles = DeviceTable(apply_items(family, False, ragged, [], 32), self.device)
+        self.n_rtiles = len(self.rtiles.host)
         #: how many of them, at the front of the list, are on tensors that are not FAST2D (tensor cores only)
         self.n_ctiles_gen = int((self.ctiles.host["pad_"] >= L.TC_GEN_ITEM).sum()) if self.tensor_cores else 0
         self.pitems = DeviceTable(atile_list(pitems), self.device)
@@ -458,10 +477,10 @@ class LoPlan:
         #: everything pylo_b200_step needs for a step over these tensors
         self.step_plan = L.StepPlan(
             tdesc=self.tdesc.ptr, desc=self.desc.ptr, atiles=self.atiles.ptr, gitems=self.gitems.ptr, pitems=self.pitems.ptr,
-            ctiles=self.ctiles.ptr, tiles=self.tiles.ptr, tiles_slow=self.tiles_slow.ptr,
+            ctiles=self.ctiles.ptr, tiles=self.tiles.ptr, tiles_slow=self.tiles_slow.ptr, rtiles=self.rtiles.ptr,
             status=self.status.data_ptr(), host_status=self._status_host.data_ptr(),
             n_tensors=T, n_units=U, n_atiles=self.n_atiles, n_gitems=self.n_gitems, n_pitems=self.n_pitems,
-            n_ctiles=self.n_ctiles, n_ctiles_gen=self.n_ctiles_gen, n_tiles=self.n_tiles, n_tiles_slow=self.n_tiles_slow,
+            n_ctiles=self.n_ctiles, n_ctiles_gen=self.n_ctiles_gen, n_tiles=self.n_tiles, n_tiles_slow=self.n_tiles_slow, n_ragged=self.n_ragged, n_rtiles=self.n_rtiles,
             tensor_cores=int(self.tensor_cores), sum_tiles=int(self.sum_tiles))
         if self.small:
             (self.step_plan.small_cluster, self.step_plan.small_slice, self.step_plan.small_rows, self.step_plan.small_cols) = self.small
@@ -544,12 +563,12 @@ class LoPlan:
     def _phases(self):
         """[(phase of pylo_b200_step, name, launches)] in the step's order, without those that launch nothing."""
         split = self.tensor_cores and self.n_ctiles >= L.TC_ONE_LAUNCH   # a launch of its own for what is not FAST2D
-        rest = int(split and self.n_ctiles_gen > 0) if self.tensor_cores else int(self.n_tiles_slow > 0)
+        rest = int(split and self.n_ctiles_gen > 0) if self.tensor_cores else int(self.n_tiles_slow > 0) + int(self.n_rtiles > 0)
         main = int(self.n_ctiles > (self.n_ctiles_gen if split else 0))
         other = "k_apply_adafac_tc<true>" if self.tensor_cores else "k_apply"
         apply = [(L.STEP_APPLY, self.apply_kernel if self.n_ctiles > self.n_ctiles_gen else other, main)]
         apply.insert(0 if self.tensor_cores else 1, (L.STEP_APPLY_REST, other, rest))
-        front = [(L.STEP_SUMS, "rowcol_sums", (self.n_atiles > 0) + (self.n_gitems > 0)), (L.STEP_FACTORS, "factor_update", 1),
+        front = [(L.STEP_SUMS, "rowcol_sums", (self.n_ragged > 0) + (self.n_atiles > self.n_ragged) + (self.n_gitems > 0)), (L.STEP_FACTORS, "factor_update", 1),
                  (L.STEP_STATE, "state_moments", 1)]
         if self.small:
             front = [(L.STEP_SUMS | L.STEP_FACTORS | L.STEP_STATE, "small_front", 1)]

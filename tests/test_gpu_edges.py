@@ -431,3 +431,32 @@ def test_network_as_an_argument_is_the_folded_one(family, extra, shapes):
         if family == "adafaclo":
             assert torch.equal(a, b)
         assert float((a - b).abs().max()) <= 1e-5 * float((b - init.cuda()).abs().max()) + 2 ** -23 * float(b.abs().max())
+
+
+# rows that are not aligned: from the first width that goes with the others (64 columns) on, one and several blocks of 1024 columns,
+# strips of 8 and 32 rows with remainders, a tile's last columns missing; narrower ones and aligned ones beside them
+UNALIGNED = [(65, 65), (9, 1025), (33, 2051), (600, 67), (70, 63), (1, 101), (40, 24), (13,)]
+
+
+@pytest.mark.parametrize("family,extra", [("adafaclo", {}), ("celo2", {"orthogonalize": False}), ("velo", {})])
+def test_unaligned_rows_go_the_way_of_the_aligned_ones(family, extra, monkeypatch):
+    """Sums and apply sweep of unaligned matrices against the oracle (small models' single launch off), and their work lists."""
+    from pylo_b200 import plan as pylo_plan
+
+    monkeypatch.setattr(pylo_plan, "SMALL_CTAS", 0)
+    case = dict(shapes=UNALIGNED, init_seed=51, init_scale=0.1, grad_seed=52, grad_scale=0.3)
+    params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+    init = [v.clone() for v in cases.init_values(case)]
+    ref = [v.clone() for v in init]
+    opt, ora = _make(family, params, **extra), _oracle(family, _nets(family), UNALIGNED)
+    for t in (1, 2):
+        grads = cases.grads_at(case, t)
+        for p, g in zip(params, grads):
+            p.grad = g.cuda()
+        _step(opt, family, t)
+        ora.step(ref, grads, cases.velo_loss(t)) if family == "velo" else ora.step(ref, grads)
+    res = CU.compare({2: [p.detach().cpu() for p in params]}, {2: ref}, init)
+    assert res[2][0] < 1e-5 and res[2][1] < 2e-5, res
+    plan, = _plans(opt)
+    taken = {int(t) for t in plan.atiles.host["tensor"][:plan.n_ragged]}
+    assert taken == {0, 1, 2, 3, 5} and len({int(u) for u in plan.rtiles.host["tensor"]}) == (0 if family == "adafaclo" else 5)
