@@ -172,6 +172,25 @@ class DeviceTable:
         self._events[i] = ev
 
 
+class FixedTable:
+    """A table that stays as it is: its place is in one device buffer with the plan's others, copied there once (seven copies of a
+    few hundred bytes each took a tenth of the time to build a small model's plan)."""
+
+    def __init__(self, host: np.ndarray):
+        self.host, self.ptr = host, 0
+
+    @staticmethod
+    def place(tables: Sequence["FixedTable"], device) -> torch.Tensor:
+        ends = np.cumsum([(max(t.host.nbytes, 16) + 255) // 256 * 256 for t in tables])
+        raw = np.zeros(int(ends[-1]), dtype=np.uint8)
+        buffer = torch.empty(len(raw), dtype=torch.uint8, device=device)
+        for t, at in zip(tables, [0] + ends[:-1].tolist()):
+            raw[at:at + t.host.nbytes] = t.host.view(np.uint8).reshape(-1)
+            t.ptr = buffer.data_ptr() + at
+        buffer.copy_(torch.from_numpy(raw))
+        return buffer
+
+
 def apply_tile_shape(family: int, X: int, Y: int, least: int = 8):
     """(rows per work item, columns per work item, tag for ``pylo_atile.pad_``) of a FAST2D tensor's apply sweep on the CUDA
     cores.
@@ -411,11 +430,11 @@ class LoPlan:
         self.unit_owner = unit_owner
         self.tdesc = DeviceTable(tdesc, self.device)
         self.desc = DeviceTable(udesc, self.device) if self.sliced else self.tdesc
-        self.tiles = DeviceTable(tiles, self.device)
+        self.tiles = FixedTable(tiles)
         self.n_tiles = len(tiles)
-        self.atiles = DeviceTable(atile_list(ratiles + atiles), self.device)
+        self.atiles = FixedTable(atile_list(ratiles + atiles))
         self.n_atiles, self.n_ragged = len(self.atiles.host), len(atile_list(ratiles))
-        self.gitems = DeviceTable(atile_list(gitems), self.device)
+        self.gitems = FixedTable(atile_list(gitems))
         self.n_gitems = len(self.gitems.host)
         self.n_tensors = T
         self.n_units = U
@@ -439,13 +458,13 @@ class LoPlan:
             pitems.append(atile_grid(unit_of[i], parts, 1)[1:])
             (fast if tdesc["mode"][i] == L.MODE_FAST2D else ragged).append((unit_of[i], X, Y))
         slow_units = [u for u in range(U) if not tdesc["h_a"][unit_owner[u][0]]]
-        self.ctiles = DeviceTable(apply_items(family, self.tensor_cores, fast, [(u, sizes[u]) for u in slow_units]), self.device)
+        self.ctiles = FixedTable(apply_items(family, self.tensor_cores, fast, [(u, sizes[u]) for u in slow_units]))
         self.n_ctiles = len(self.ctiles.host)
-        self.rtiles = DeviceTable(apply_items(family, False, ragged, [], 32), self.device)
+        self.rtiles = FixedTable(apply_items(family, False, ragged, [], 32))
         self.n_rtiles = len(self.rtiles.host)
         #: how many of them, at the front of the list, are on tensors that are not FAST2D (tensor cores only)
         self.n_ctiles_gen = int((self.ctiles.host["pad_"] >= L.TC_GEN_ITEM).sum()) if self.tensor_cores else 0
-        self.pitems = DeviceTable(atile_list(pitems), self.device)
+        self.pitems = FixedTable(atile_list(pitems))
         self.n_pitems = len(self.pitems.host)
         #: the kernel that takes the FAST2D tensors' apply sweep (also the key of its timings in phase_times())
         if self.tensor_cores:
@@ -465,8 +484,9 @@ class LoPlan:
         slow_sizes = [sizes[u] for u in slow_units]
         slow, _ = make_tiles(slow_sizes, tile_elems(sum(slow_sizes), 256, 4 * L.SM_COUNT))
         slow["tensor"] = np.asarray(slow_units, dtype=np.int32)[slow["tensor"]] if len(slow) else slow["tensor"]
-        self.tiles_slow = DeviceTable(slow, self.device)
+        self.tiles_slow = FixedTable(slow)
         self.n_tiles_slow = len(slow)
+        self._fixed = FixedTable.place([self.tiles, self.atiles, self.gitems, self.ctiles, self.rtiles, self.pitems, self.tiles_slow], self.device)
         #: no launch for phase B2: of small units phase P adds the tile partials up, for VeLO the LSTM's input kernel does.
         self.sum_tiles = family == L.FAM_VELO or max((k for _, k in ranges), default=0) <= SUM_TILES_MOST
         # The state sweep's ring of bulk copies leaves little L1 cache to the units that are not FAST2D and keeps the launches
