@@ -1988,21 +1988,32 @@ __global__ void __launch_bounds__(NT) k_velo_xmix(const pylo_velo_rnn r, const p
   for (int t = lane; t < r.T; t += 32) r.xmix[(int64_t)t * r.H + h] += best;
 }
 
-// gates[t][q] = lstm_b[q] + sum_k lstm_w[q][k] * cat(x', h)[t][k]: a [T x 2H] x [2H x 4H] product, fp32 throughout.
+__device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
+// cell update of one hidden unit; gate order i, g, f, o with f + 1 (VeLO_RNN.py:57-65)
+__device__ __forceinline__ float velo_cell(float i, float g, float f, float o, float& c) {
+  c = sigmoidf_(f + 1.0f) * c + sigmoidf_(i) * tanhf(g);
+  return sigmoidf_(o) * tanhf(c);
+}
+
+// The LSTM's gates, gates[t][q] = lstm_b[q] + sum_k lstm_w[q][k] * cat(x', h)[t][k], a [T x 2H] x [2H x 4H] product, fp32
+// throughout, and its cell.
 //
-// For few tensors it is a read of the 8.4 MB of weights, for a few hundred ~0.6 G FMAs.  A warp keeps four weight rows (one
-// half of their columns: those that meet x', or those that meet h) in registers and takes eight tensors at a time from
-// shared memory: 512 FMAs per lane on 32 shared-memory reads, then the 32 sums are reduced over the lanes together, 31
-// shuffles in all, and lane l ends with the sum of tensor l / 4 and row l % 4.  The two halves are left as two partial
-// sums that the cell kernel adds.  512 hidden units: 6 tensors 68.6 -> 3.6 us, 292 tensors 124 -> 46 us (the tiled kernel
-// below, which is kept for hidden sizes that are not multiples of 128, or above 512).
-#define GR_ROWS 16   // weight rows per CTA: four per pair of warps
+// For few tensors it is a read of the 8.4 MB of weights, for a few hundred ~0.6 G FMAs.  A warp keeps the four weight rows of a
+// hidden unit (one half of their columns: those that meet x', or those that meet h) in registers and takes eight tensors at a time
+// from shared memory: 512 FMAs per lane on 32 shared-memory reads, then the 32 sums are reduced over the lanes together, 31
+// shuffles in all, and lane l ends with the sum of tensor l / 4 and gate l % 4.  The other half's sums come from the warp beside
+// it, the four gates of a tensor from the lanes beside.  512 hidden units: 6 tensors 68.6 -> 3.6 us, 292 tensors 124 -> 46 us (the
+// tiled kernel below, which is kept for hidden sizes that are not multiples of 128, or above 512), and the cell was another launch
+// of 2.8.  Other CTAs still read h: the new one is left in `gates` ([T][H]), k_velo_mix takes it over.
+#define GR_UNITS 4   // hidden units per CTA: one per pair of warps
 template <int NI>    // float4 per lane and row: H = 128 * NI
-__global__ void __launch_bounds__(NT, 2) k_velo_gates_rows(const pylo_velo_rnn r, int groups_per_cta) {
+__global__ void __launch_bounds__(NT, 2) k_velo_lstm(const pylo_velo_rnn r, int groups_per_cta) {
   pdl_begin();
   extern __shared__ __align__(16) float s_x[];   // [2][8][2H]
+  __shared__ float s_half[GR_UNITS][32];
   constexpr int H = 128 * NI;
-  const int tid = threadIdx.x, lane = tid & 31, half = (tid >> 5) & 1, q0 = blockIdx.x * GR_ROWS + (tid >> 6) * 4;
+  const int tid = threadIdx.x, lane = tid & 31, half = (tid >> 5) & 1, unit = tid >> 6, h = blockIdx.x * GR_UNITS + unit;
+  const int word = reported(r.status);
   const int groups = (r.T + 7) / 8, g0 = blockIdx.y * groups_per_cta, g1 = min(g0 + groups_per_cta, groups);
   auto stage = [&](int g) {
     float* dst = s_x + (g & 1) * 16 * H;
@@ -2019,13 +2030,16 @@ __global__ void __launch_bounds__(NT, 2) k_velo_gates_rows(const pylo_velo_rnn r
 #pragma unroll
   for (int u = 0; u < 4; ++u)
 #pragma unroll
-    for (int i = 0; i < NI; ++i) w[u][i] = ldg4(r.lstm_w + (int64_t)(q0 + u) * 2 * H + half * H + (i * 32 + lane) * 4);
+    for (int i = 0; i < NI; ++i) w[u][i] = ldg4(r.lstm_w + (int64_t)(u * H + h) * 2 * H + half * H + (i * 32 + lane) * 4);
+  const float bias = r.lstm_b[(lane & 3) * H + h];
   for (int g = g0; g < g1; ++g) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();   // this group has arrived, and the buffer of the next one is no longer read
     if (g + 1 < g1) stage(g + 1);
+    const int t = g * 8 + (lane >> 2);
+    const float c_old = !half && t < r.T ? r.c[(int64_t)t * H + h] : 0.f;
     const float* x = s_x + (g & 1) * 16 * H + half * H + lane * 4;
-    float acc[32];     // tensor * 4 + row
+    float acc[32];     // tensor * 4 + gate
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
 #pragma unroll
@@ -2038,18 +2052,20 @@ __global__ void __launch_bounds__(NT, 2) k_velo_gates_rows(const pylo_velo_rnn r
           acc[t * 4 + u] = fmaf(w[u][i].w, v.w, fmaf(w[u][i].z, v.z, fmaf(w[u][i].y, v.y, fmaf(w[u][i].x, v.x, acc[t * 4 + u]))));
       }
     }
-    // fold the lanes: after the step of offset o a lane holds the o entries whose index agrees with its own in that bit
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const bool up = lane & o;
-#pragma unroll
-      for (int j = 0; j < o; ++j) {
-        const float keep = up ? acc[j + o] : acc[j], give = up ? acc[j] : acc[j + o];
-        acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    const float sum = warp_fold<0, 32>(acc);
+    if (half) s_half[unit][lane] = sum;
+    __syncthreads();
+    if (!half) {
+      const float gate = (sum + bias) + s_half[unit][lane];
+      const int first = lane & ~3;
+      const float gi = __shfl_sync(0xffffffffu, gate, first), gg = __shfl_sync(0xffffffffu, gate, first + 1),
+                  gf = __shfl_sync(0xffffffffu, gate, first + 2), go = __shfl_sync(0xffffffffu, gate, first + 3);
+      if ((lane & 3) == 0 && t < r.T && !word) {
+        float c = c_old;
+        r.gates[(int64_t)t * H + h] = velo_cell(gi, gg, gf, go, c);
+        r.c[(int64_t)t * H + h] = c;
       }
     }
-    const int t = g * 8 + (lane >> 2), q = q0 + (lane & 3);
-    if (t < r.T) r.gates[((int64_t)half * r.T + t) * 4 * H + q] = acc[0] + (half ? 0.f : r.lstm_b[q]);
   }
 }
 
@@ -2105,34 +2121,24 @@ __global__ void __launch_bounds__(NT) k_velo_gates(const pylo_velo_rnn r) {
   }
 }
 
-__device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
-
-// cell update; gate order i, g, f, o with f + 1 (VeLO_RNN.py:57-65)
-// parts: 1, or 2 where the gates are left as two partial sums (the second [T][4H] block)
-__global__ void k_velo_cell(const pylo_velo_rnn r, int parts) {
+// the cell behind k_velo_gates
+__global__ void k_velo_cell(const pylo_velo_rnn r) {
   pdl_begin();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (int64_t)r.T * r.H) return;
   const int word = reported(r.status);
   const int t = (int)(e / r.H), h = (int)(e % r.H), H = r.H;
   const float* g4 = r.gates + (int64_t)t * 4 * H + h;
-  float a[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) a[k] = g4[k * H];
-  if (parts == 2) {
-    const float* g5 = g4 + (int64_t)r.T * 4 * H;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) a[k] += g5[k * H];
-  }
-  const float i = sigmoidf_(a[0]), g = tanhf(a[1]), f = sigmoidf_(a[2] + 1.0f), o = sigmoidf_(a[3]);
-  const float c = f * r.c[e] + i * g;
+  float c = r.c[e];
+  const float hn = velo_cell(g4[0], g4[H], g4[2 * H], g4[3 * H], c);
   if (word) return;
   r.c[e] = c;
-  r.h[e] = o * tanhf(c);
+  r.h[e] = hn;
 }
 
 // controls[t][b] and lr_mult[t]; one warp per output
-__global__ void __launch_bounds__(NT) k_velo_heads(const pylo_velo_rnn r) {
+// h: r.h, or where k_velo_lstm has left the new one
+__global__ void __launch_bounds__(NT) k_velo_heads(const pylo_velo_rnn r, const float* __restrict__ h) {
   pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t wid = (int64_t)blockIdx.x * NWARP + (threadIdx.x >> 5);
@@ -2141,7 +2147,7 @@ __global__ void __launch_bounds__(NT) k_velo_heads(const pylo_velo_rnn r) {
   const int t = (int)(wid / B1), b = (int)(wid % B1);
   const float* wrow = b < r.B ? r.ctrl_w + (int64_t)b * H : r.step_w;
   float acc = 0.f;
-  for (int k = lane; k < H; k += 32) acc = fmaf(wrow[k], r.h[(int64_t)t * H + k], acc);
+  for (int k = lane; k < H; k += 32) acc = fmaf(wrow[k], h[(int64_t)t * H + k], acc);
   acc = warp_sum(acc);
   if (lane == 0) {
     if (b < r.B) r.controls[(int64_t)t * r.B + b] = acc + r.ctrl_b[b];
@@ -2151,11 +2157,14 @@ __global__ void __launch_bounds__(NT) k_velo_heads(const pylo_velo_rnn r) {
 
 // weights[tensor][e] = mean_b(control[b] * bank[b][e]) * 100 (VeLO_MLP.py:92-126).  Latency-bound: a block takes a quarter of a
 // tensor's 159 weights and deals the bank to sixteen groups of threads, whose sixteen reads of the usual bank are in flight
-// together (a block per tensor and four groups, eight reads at a time: 7.3 us, now 3.5).
+// together (a block per tensor and four groups, eight reads at a time: 7.3 us, now 3.5; as one launch with the heads, a cluster per tensor, the two took 12.5 instead of 7.4).
 #define MIX_GROUPS 16
 #define MIX_OUT 40
-__global__ void __launch_bounds__(MIX_OUT * MIX_GROUPS) k_velo_mix(const pylo_velo_rnn r) {
+__global__ void __launch_bounds__(MIX_OUT * MIX_GROUPS) k_velo_mix(const pylo_velo_rnn r, const float* __restrict__ h_new) {
   pdl_begin();
+  if (h_new != r.h && !reported(r.status)) {   // nobody reads the old h any more
+    for (int k = blockIdx.y * blockDim.x + threadIdx.x; k < r.H; k += gridDim.y * blockDim.x) r.h[(int64_t)blockIdx.x * r.H + k] = h_new[(int64_t)blockIdx.x * r.H + k];
+  }
   extern __shared__ float s_ctrl[];
   __shared__ float s_part[MIX_GROUPS][MIX_OUT];
   const int tensor = blockIdx.x, row = r.T - 1 - tensor;
@@ -2950,23 +2959,23 @@ int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, const pylo_velo_loss* lossbuf, 
   const int64_t TH = (int64_t)r.T * r.H;
   const pylo_velo_loss none = {};
   launch(k_velo_xmix, (r.H + NWARP - 1) / NWARP, NT, 0, s, r, lossbuf ? *lossbuf : none);
-  int parts = 1;
+  const float* h = r.h;   // the new one
   if (r.H % 128 == 0 && r.H <= 512) {
-    parts = 2;
-    const int gx = 4 * r.H / GR_ROWS, groups = (r.T + 7) / 8;
+    const int gx = r.H / GR_UNITS, groups = (r.T + 7) / 8;
     const int gy = groups * gx <= 2 * sm_count() ? groups : (2 * sm_count() / gx > 0 ? 2 * sm_count() / gx : 1);   // two CTAs per SM
     const int per = (groups + gy - 1) / gy, smem = 2 * 8 * 2 * r.H * (int)sizeof(float);
     static bool configured[4][PYLO_MAX_DEVICES] = {};
-    auto kernel = r.H == 128 ? k_velo_gates_rows<1> : r.H == 256 ? k_velo_gates_rows<2> : r.H == 384 ? k_velo_gates_rows<3> : k_velo_gates_rows<4>;
+    auto kernel = r.H == 128 ? k_velo_lstm<1> : r.H == 256 ? k_velo_lstm<2> : r.H == 384 ? k_velo_lstm<3> : k_velo_lstm<4>;
     if (int rc = allow_dynamic_smem(kernel, smem, configured[r.H / 128 - 1])) return rc;
     launch(kernel, dim3(gx, gy), NT, smem, s, r, per);
+    h = r.gates;
   } else {
     launch(k_velo_gates, dim3((4 * r.H + GT - 1) / GT, (r.T + GT - 1) / GT), NT, 0, s, r);
+    launch(k_velo_cell, (unsigned)((TH + 255) / 256), 256, 0, s, r);
   }
-  launch(k_velo_cell, (unsigned)((TH + 255) / 256), 256, 0, s, r, parts);
   const int64_t hw = (int64_t)r.T * (r.B + 1);
-  launch(k_velo_heads, (unsigned)((hw + NWARP - 1) / NWARP), NT, 0, s, r);
-  launch(k_velo_mix, dim3(r.T, 160 / MIX_OUT), MIX_OUT * MIX_GROUPS, r.B * sizeof(float), s, r);
+  launch(k_velo_heads, (unsigned)((hw + NWARP - 1) / NWARP), NT, 0, s, r, h);
+  launch(k_velo_mix, dim3(r.T, 160 / MIX_OUT), MIX_OUT * MIX_GROUPS, r.B * sizeof(float), s, r, h);
   return launch_status();
 }
 
