@@ -2319,7 +2319,7 @@ static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
   // An SM fetches a K block of 64 in half a microsecond or more, so a few tiles with a long contraction are shared by clusters
   // of CTAs: from eight blocks each on (below, bringing the sums together costs what is gained: 197 x 768, 12 blocks, 171 us
   // per chain unsplit, 174 in two), as far as three quarters of the SMs go (1001 x 1433 in 36 clusters of four found no room
-  // for all of them at once: 342 -> 446).  128 x 3000: 293 -> 194 us, 768 x 2304: 308 -> 259, 10 x 3000: 215 -> 140.
+  // for all of them at once: 342 -> 446).  768 x 2304: 308 -> 259 us; 128 x 3000 (now k_ns_cluster's): 293 -> 194.
   int blocks = 0, split = 1;
   for (int k = 0; k < grp.n; ++k) blocks = max(blocks, (grp.p[k].g.K + NF_BK - 1) / NF_BK);
   while (split < 8 && blocks >= 16 * split && tiles * 2 * split <= sms * 3 / 4) split *= 2;
