@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define PYLO_B200_ABI_VERSION 15
+#define PYLO_B200_ABI_VERSION 16
 
 /* optimizer families (which feature set / network geometry a launch uses) */
 #define PYLO_FAM_ADAFAC 0 /* AdafacLO_CUDA, ELO_CUDA: 28+11 features, 39-32-32-2 */
@@ -157,6 +157,8 @@ typedef struct pylo_step_params {
   const float* w_host;    /* HOST pointer to the network of desc.w, where it is the same for all units, or NULL.  CELO2: apply_packed
                              then takes it as an argument of its launch instead of reading the folded one of every unit;
                              ADAFAC: apply_adafac_tc its output layer */
+  float* step_squares;    /* CELO2: apply_packed leaves the sum of squares of item k's raw steps in step_squares[k] (what celo2_post_sums
+                             would make, in other pieces); may be NULL */
 } pylo_step_params;
 
 int pylo_b200_abi_version(void);

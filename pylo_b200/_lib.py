@@ -17,7 +17,7 @@ TILE_ELEMS = 16384
 A_COLS = 1024
 PREP_TABLE = 2048  # table entries (rows x hidden units) per item of pylo_b200_prep_apply
 WFOLD_STRIDE = 2432
-ABI_VERSION = 15
+ABI_VERSION = 16
 
 FAM_ADAFAC, FAM_CELO2, FAM_VELO = 0, 1, 2
 MODE_FAST2D, MODE_GENERIC, MODE_VEC1D = 0, 1, 2
@@ -58,6 +58,7 @@ class StepParams(C.Structure):
         ("eps_v", C.c_float), ("eps_feat", C.c_float), ("eps_norm", C.c_float), ("clip_val", C.c_float),
         ("no_tables", C.c_int32), ("gnorm_sq", C.c_void_p), ("sum_tiles", C.c_int32), ("bulk_copies", C.c_int32),
         ("status", C.c_void_p), ("host_status", C.c_void_p), ("w_host", C.c_void_p),
+        ("step_squares", C.c_void_p),
     ]
 
 

@@ -1490,6 +1490,8 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
   __shared__ __align__(16) float s_w[ARG ? 20 : W::SIZE];   // ARG: the normalisers of the element-wise features
   __shared__ __align__(16) float s_row[PK_STAGE * RP];
   __shared__ float s_sc[2];
+  __shared__ float s_red[40];
+  float* const squares = FAM == PYLO_FAM_CELO2 ? prm.step_squares : nullptr;
   const int tid = threadIdx.x;
   const uint32_t s_wa = smem_addr(s_w);
   int loaded = -1;
@@ -1571,6 +1573,7 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
       }
     };
     load_row(0, cg, cp, cm0, cm1, cm2, cv);
+    float sq = 0.f;   // CELO2: of this thread's raw steps
     const int sub = min(PK_ROWS, PK_STAGE / ng);   // rows per thread and stage
 #pragma unroll 1
     for (int q = 0; q < rpt; ++q) {
@@ -1701,6 +1704,14 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
           two(cp.z, cp.w, d2, d3, m2, m3, res.z, res.w);
         } else {
           res = make_float4(d0 * __expf(m0 * exp_mult), d1 * __expf(m1 * exp_mult), d2 * __expf(m2 * exp_mult), d3 * __expf(m3 * exp_mult));
+          if constexpr (RAGGED) {
+            sq += res.x * res.x;
+            if (y + tpr < Y) sq += res.y * res.y;
+            if (y + 2 * tpr < Y) sq += res.z * res.z;
+            if (y + 3 * tpr < Y) sq += res.w * res.w;
+          } else {
+            sq += res.x * res.x + res.y * res.y + res.z * res.z + res.w * res.w;
+          }
         }
         if constexpr (RAGGED) {
           const float r4[4] = {res.x, res.y, res.z, res.w};
@@ -1717,6 +1728,10 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
         }
       }
       if (q + 1 < rpt) { cg = ng_; cp = np_; cm0 = nm0; cm1 = nm1; cm2 = nm2; cv = nv; }
+    }
+    if (FAM == PYLO_FAM_CELO2 && squares) {
+      sq = block_sum(sq, s_red);
+      if (tid == 0) squares[t] = sq;
     }
   }
 }

@@ -186,6 +186,17 @@ class _Celo2Family(Optimizer):
             post.part = torch.zeros(max(post.n_tiles, 1), dtype=torch.float32, device=self.device)
             post.items["part"] = post.part.data_ptr() + 4 * post.items["tile0"].astype(np.uint64)
             plan["post"] = post
+            # where the packed sweep takes every matrix, its items' sums of squares of the raw steps stand in for a launch that reads
+            # the steps again (unless they are orthogonalised): (first item, items) of every matrix
+            pl = plan["lo"]
+            plan["squares"] = None
+            if not pl.sliced and pl.n_tiles_slow == 0 and pl.n_rtiles == 0:
+                owner = pl.ctiles.host["tensor"]   # ascending: the units in their order
+                first = np.searchsorted(owner, np.arange(len(lo)))
+                count = np.searchsorted(owner, np.arange(len(lo)), side="right") - first
+                buffer = torch.zeros(max(len(owner), 1), dtype=torch.float32, device=self.device)
+                plan["squares"] = (buffer, buffer.data_ptr() + 4 * first.astype(np.uint64), count.astype(np.int32),
+                                   post.items["part"].copy(), post.items["n_tiles"].copy())
             base_p = np.array([p.data_ptr() for p in lo], dtype=np.uint64)
             post.items["p"][:] = base_p[post.owner_t] + post.owner_off
         if adam:
@@ -278,21 +289,27 @@ class _Celo2Family(Optimizer):
         exp_mult, rmsmult = group_floats(group, "exp_mult", "rmsmult")
         lo.set_hyper(lr=lr, wd=wd, clip_norm=clip_norm, exp_mult=exp_mult)
         lo.refresh(grads)
+        squares = None if group["orthogonalize"] else plan["squares"]
+        prm.step_squares = squares[0].data_ptr() if squares else None
         lo.run(prm, stream)
+        prm.step_squares = None
         post: ItemPlan = plan["post"]
         keep = [t.out for t in lo.tensors]
         if group["orthogonalize"]:
             keep, steps = self._orthogonalise(plan, stream)
         else:
             steps = [k.data_ptr() for k in keep]
-        key = (steps, lr, wd, rmsmult)
+        key = (steps, lr, wd, rmsmult, squares is not None)
         if key != plan["post_key"]:
             it = post.items
             it["step"][:] = np.array(steps, dtype=np.uint64)[post.owner_t] + post.owner_off
             it["lr"][:], it["wd"][:], it["rmsmult"][:] = lr, wd, rmsmult
+            if plan["squares"]:
+                it["part"][:], it["n_tiles"][:] = plan["squares"][1:3] if squares else plan["squares"][3:5]
             post.upload()
             plan["post_key"] = key
-        L.check(L.lib.pylo_b200_celo2_post_sums(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_sums")
+        if not squares:
+            L.check(L.lib.pylo_b200_celo2_post_sums(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_sums")
         L.check(L.lib.pylo_b200_celo2_post_apply(post.table.ptr, post.tiles.ptr, post.n_tiles, lo.step_plan.status,
                                                  lo.step_plan.host_status, stream), "celo2_post_apply")
         self._keep = keep

@@ -460,3 +460,30 @@ def test_unaligned_rows_go_the_way_of_the_aligned_ones(family, extra, monkeypatc
     plan, = _plans(opt)
     taken = {int(t) for t in plan.atiles.host["tensor"][:plan.n_ragged]}
     assert taken == {0, 1, 2, 3, 5} and len({int(u) for u in plan.rtiles.host["tensor"]}) == (0 if family == "adafaclo" else 5)
+
+
+def test_squares_of_the_raw_steps_from_the_apply_sweep():
+    """CELO2 without orthogonalisation: the apply sweep's sums of squares against the launch that reads the steps again, tiles and
+    rows with remainders, several items a matrix; and a group that changes its mind between steps."""
+    shapes = [(40, 24), (300, 1028), (1031, 68), (5, 4)]
+    case = dict(shapes=shapes, init_seed=51, init_scale=0.1, grad_seed=52, grad_scale=0.3)
+    runs = []
+    for own in (False, True):
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+        opt = _make("celo2", params, orthogonalize=False)
+        for t in (1, 2, 3, 4):
+            for p, g in zip(params, cases.grads_at(case, t)):
+                p.grad = g.cuda()
+            opt.param_groups[0]["orthogonalize"] = t == 3
+            opt.step()
+            plan = opt._plans[0][1]
+            if t == 1:
+                assert plan["squares"] is not None
+                if own:
+                    it = plan["post"].items
+                    it["part"][:], it["n_tiles"][:] = plan["squares"][3:5]
+                    plan["squares"] = plan["post_key"] = None
+        runs.append([p.detach().clone() for p in params])
+    for a, b, init in zip(runs[0], runs[1], cases.init_values(case)):
+        # the same terms in another order: each sum to a few 2^-24 of itself, half of that in its root
+        assert float((a - b).abs().max()) <= 1e-5 * float((b - init.cuda()).abs().max()) + 2 ** -23 * float(b.abs().max())
