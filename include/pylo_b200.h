@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define PYLO_B200_ABI_VERSION 16
+#define PYLO_B200_ABI_VERSION 17
 
 /* optimizer families (which feature set / network geometry a launch uses) */
 #define PYLO_FAM_ADAFAC 0 /* AdafacLO_CUDA, ELO_CUDA: 28+11 features, 39-32-32-2 */
@@ -305,9 +305,10 @@ int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* t
  * index, pad_ = threads per row (8 .. 256, a thread owns 4 columns) | rows per thread << 16 (0: 16); a tile has
  * rows * (256 / threads) rows and 4 * threads columns.  ragged != 0: the items are on GENERIC matrices with tables (any Y, any
  * alignment).  For these families pylo_b200_prep_apply stores desc.h_a as (v, v) pairs, [X][H][2], and
- * for every family desc.h_b transposed, [H][Y]. */
+ * for every family desc.h_b transposed, [H][Y].  tiles: other tensors' for
+ * pylo_b200_apply, done in the same launch for VELO and in one after it for CELO2. */
 int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles, int ragged,
-                           const pylo_step_params* prm, void* stream);
+                           const pylo_tile* tiles, int n_tiles, const pylo_step_params* prm, void* stream);
 
 /* Batched fp32-faithful matrix product on the tensor cores, for the Newton-Schulz orthogonalisation of the CELO2
  * family (orthogonalize_via_newton_schulz, CELO2_naive.py:59-73, called at CELO2_cuda.py:332-335; the reference runs

@@ -17,7 +17,7 @@ TILE_ELEMS = 16384
 A_COLS = 1024
 PREP_TABLE = 2048  # table entries (rows x hidden units) per item of pylo_b200_prep_apply
 WFOLD_STRIDE = 2432
-ABI_VERSION = 16
+ABI_VERSION = 17
 
 FAM_ADAFAC, FAM_CELO2, FAM_VELO = 0, 1, 2
 MODE_FAST2D, MODE_GENERIC, MODE_VEC1D = 0, 1, 2
@@ -137,7 +137,7 @@ def _load():
         "pylo_b200_apply": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply_adafac_cols": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply_adafac_tc": [vp, vp, i32, i32, C.POINTER(StepParams), vp, vp, vp],
-        "pylo_b200_apply_packed": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
+        "pylo_b200_apply_packed": [vp, vp, i32, i32, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_gemm_tn_3xtf32": [C.POINTER(GemmDesc), vp, vp],
         "pylo_b200_transpose": [vp, vp, i32, i32, i32, i32, C.c_int64, C.c_int64, i32, i32, vp],
         "pylo_b200_newton_schulz_workspace": [i32, i32, i32, i32],

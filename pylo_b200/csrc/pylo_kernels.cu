@@ -1035,11 +1035,10 @@ __device__ __forceinline__ float finish(float p, float o0, float o1, const Fin& 
   return pn;
 }
 
+// word: of the step's status (0 for CELO2, whose parameters k_post_apply writes); block, blocks: of those that share the tiles
 template <int FAM>
-__global__ void __launch_bounds__(NT) k_apply(const pylo_tensor_desc* __restrict__ descs,
-                                              const pylo_tile* __restrict__ tiles, int n_tiles, int reverse,
-                                              const pylo_step_params prm) {
-  pdl_begin();
+__device__ __forceinline__ void apply_tiles(const pylo_tensor_desc* __restrict__ descs, const pylo_tile* __restrict__ tiles, int n_tiles,
+                                            int reverse, const pylo_step_params& prm, int word, int block, int blocks) {
   using F = Fam<FAM>;
   using L = Fold<FAM>;
   constexpr int H = F::H;
@@ -1047,12 +1046,11 @@ __global__ void __launch_bounds__(NT) k_apply(const pylo_tensor_desc* __restrict
   const int tid = threadIdx.x;
   const uint32_t s_wa = smem_addr(s_w);
   int loaded = -1;
-  for (int tt = blockIdx.x; tt < n_tiles; tt += gridDim.x) {
+  for (int tt = block; tt < n_tiles; tt += blocks) {
     const int t = reverse ? (n_tiles - 1 - tt) : tt;
     const pylo_tile tl = tiles[t];
     const pylo_tensor_desc& d = descs[tl.tensor];
     if (loaded != tl.tensor) {
-      const int word = FAM == PYLO_FAM_CELO2 ? 0 : reported(prm.status);   // CELO2's parameters are written by k_post_apply
       __syncthreads();
 #pragma unroll 4
       for (int e = tid; e < L::SIZE; e += NT) s_w[e] = __ldg(d.wfold + e);
@@ -1126,6 +1124,13 @@ __global__ void __launch_bounds__(NT) k_apply(const pylo_tensor_desc* __restrict
       }
     }
   }
+}
+template <int FAM>
+__global__ void __launch_bounds__(NT) k_apply(const pylo_tensor_desc* __restrict__ descs,
+                                              const pylo_tile* __restrict__ tiles, int n_tiles, int reverse,
+                                              const pylo_step_params prm) {
+  pdl_begin();
+  apply_tiles<FAM>(descs, tiles, n_tiles, reverse, prm, FAM == PYLO_FAM_CELO2 ? 0 : reported(prm.status), blockIdx.x, gridDim.x);
 }
 
 // ================================================================================================
@@ -1478,10 +1483,8 @@ __device__ __forceinline__ float4 ld4_early(const float* p) {
 // RAGGED: matrices whose rows do not start on 16-byte boundaries: a thread's four columns are a tile's quarter apart, so that a
 // warp's single accesses are to neighbouring elements.
 template <int FAM, bool ARG, bool RAGGED>
-__global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_CTAS_CELO2) k_apply_packed(const pylo_tensor_desc* __restrict__ descs,
-                                                        const pylo_atile* __restrict__ ctiles, int n_ctiles,
-                                                        const pylo_step_params prm, const __grid_constant__ PkNet<FAM> net) {
-  pdl_begin();
+__device__ __forceinline__ void packed_tiles(const pylo_tensor_desc* __restrict__ descs, const pylo_atile* __restrict__ ctiles, int n_ctiles,
+                                             const pylo_step_params& prm, const PkNet<FAM>& net, int word, int block, int blocks) {
   using F = Fam<FAM>;
   using L = Fold<FAM>;
   using W = PkW<FAM>;
@@ -1495,7 +1498,7 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
   const int tid = threadIdx.x;
   const uint32_t s_wa = smem_addr(s_w);
   int loaded = -1;
-  for (int t = blockIdx.x; t < n_ctiles; t += gridDim.x) {
+  for (int t = block; t < n_ctiles; t += blocks) {
     const pylo_atile ct = ctiles[t];
     const pylo_tensor_desc& d = descs[ct.tensor];
     const int X = d.X, Y = d.Y;
@@ -1505,7 +1508,6 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
     const int rt = rpt * ng;          // rows per tile
     const int x0 = ct.strip * rt, y0 = ct.cb * tpr * 4;
     if (loaded != ct.tensor) {
-      const int word = FAM == PYLO_FAM_CELO2 ? 0 : reported(prm.status);
       __syncthreads();
       const float* __restrict__ wf = d.wfold;
       if (ARG) {
@@ -1733,6 +1735,24 @@ __global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_C
       sq = block_sum(sq, s_red);
       if (tid == 0) squares[t] = sq;
     }
+  }
+}
+// VeLO: the items on the first `packed` CTAs and other units' tiles (those of k_apply) on the rest, at the same time, instead of two
+// launches one after the other, 7.5 and 4.7 us on a perceptron of 118 K: one of 7.6 us (step 48.3 -> 44.5 us; unaligned 1001-wide
+// layers 127 -> 123, 110 M transformer 726 -> 721, convolutions with five tiles per item 318 -> 316).  Not CELO2: its vectors are not
+// in the plan, and tiles at one CTA per SM, which its items want, are slow (convolutions 15.6 -> 24.9 ms).
+template <int FAM, bool ARG, bool RAGGED>
+__global__ void __launch_bounds__(NT, FAM == PYLO_FAM_VELO ? PK_CTAS_VELO : PK_CTAS_CELO2) k_apply_packed(const pylo_tensor_desc* __restrict__ descs,
+                                                        const pylo_atile* __restrict__ ctiles, int n_ctiles, int packed,
+                                                        const pylo_tile* __restrict__ tiles, int n_tiles,
+                                                        const pylo_step_params prm, const __grid_constant__ PkNet<FAM> net) {
+  pdl_begin();
+  if constexpr (FAM == PYLO_FAM_VELO) {
+    const int word = reported(prm.status);
+    if ((int)blockIdx.x < packed) packed_tiles<FAM, ARG, RAGGED>(descs, ctiles, n_ctiles, prm, net, word, blockIdx.x, packed);
+    else apply_tiles<FAM>(descs, tiles, n_tiles, 0, prm, word, blockIdx.x - packed, gridDim.x - packed);
+  } else {
+    packed_tiles<FAM, ARG, RAGGED>(descs, ctiles, n_ctiles, prm, net, 0, blockIdx.x, gridDim.x);   // k_post_apply writes the parameters
   }
 }
 
@@ -2898,9 +2918,9 @@ int pylo_b200_newton_schulz_launches(const pylo_ns_desc* descs, int n) {
 }
 
 int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles, int ragged,
-                           const pylo_step_params* prm, void* stream) {
-  CHECK_ARG(descs && ctiles && prm && n_ctiles >= 0);
-  if (n_ctiles == 0) return 0;
+                           const pylo_tile* tiles, int n_tiles, const pylo_step_params* prm, void* stream) {
+  CHECK_ARG(descs && (ctiles || !n_ctiles) && (tiles || !n_tiles) && prm && n_ctiles >= 0 && n_tiles >= 0);
+  if (n_ctiles == 0) return n_tiles ? pylo_b200_apply(descs, tiles, n_tiles, 0, prm, stream) : 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
     case PYLO_FAM_CELO2: {
@@ -2915,15 +2935,19 @@ int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctil
       }
       auto kernel = prm->w_host ? (ragged ? k_apply_packed<PYLO_FAM_CELO2, true, true> : k_apply_packed<PYLO_FAM_CELO2, true, false>)
                                 : (ragged ? k_apply_packed<PYLO_FAM_CELO2, false, true> : k_apply_packed<PYLO_FAM_CELO2, false, false>);
-      launch(kernel, grid_for(n_ctiles, PK_CTAS_CELO2), NT, 0, s, descs, ctiles, n_ctiles, *prm, net);
+      const int packed = grid_for(n_ctiles, PK_CTAS_CELO2);
+      launch(kernel, packed, NT, 0, s, descs, ctiles, n_ctiles, packed, (const pylo_tile*)nullptr, 0, *prm, net);
+      if (n_tiles) return pylo_b200_apply(descs, tiles, n_tiles, 0, prm, stream);
       break;
     }
     // four times the CTAs that fit: an SM that is done takes the next (17 M parameters: 341 -> 327 us per step, 67 M: 1104 ->
     // 1091); CELO2's larger network is loaded by every CTA, which costs more than that gives
-    case PYLO_FAM_VELO:
-      launch(ragged ? k_apply_packed<PYLO_FAM_VELO, false, true> : k_apply_packed<PYLO_FAM_VELO, false, false>, grid_for(n_ctiles, 4 * PK_CTAS_VELO), NT, 0, s,
-             descs, ctiles, n_ctiles, *prm, PkNet<PYLO_FAM_VELO>{});
+    case PYLO_FAM_VELO: {
+      const int packed = grid_for(n_ctiles, 4 * PK_CTAS_VELO);
+      launch(ragged ? k_apply_packed<PYLO_FAM_VELO, false, true> : k_apply_packed<PYLO_FAM_VELO, false, false>, packed + grid_for(n_tiles, 4), NT, 0, s,
+             descs, ctiles, n_ctiles, packed, tiles, n_tiles, *prm, PkNet<PYLO_FAM_VELO>{});
       break;
+    }
     default: return -2;
   }
   return launch_status();
@@ -3036,15 +3060,17 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
     if (main && (rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles + first, p->n_ctiles - first, p->n_ctiles_gen > first, &q, p->status, p->host_status, stream))) return rc;
     return 0;
   }
-  if (main && p->n_ctiles) {
-    rc = q.family == PYLO_FAM_ADAFAC ? pylo_b200_apply_adafac_cols(p->desc, p->ctiles, p->n_ctiles, &q, stream)
-                                     : pylo_b200_apply_packed(p->desc, p->ctiles, p->n_ctiles, 0, &q, stream);
-    if (rc) return rc;
+  if (q.family == PYLO_FAM_ADAFAC) {
+    if (main && p->n_ctiles && (rc = pylo_b200_apply_adafac_cols(p->desc, p->ctiles, p->n_ctiles, &q, stream))) return rc;
+    return rest && p->n_tiles_slow ? pylo_b200_apply(p->desc, p->tiles_slow, p->n_tiles_slow, 0, &q, stream) : 0;
   }
-  if (rest && p->n_rtiles)
-    if ((rc = pylo_b200_apply_packed(p->desc, p->rtiles, p->n_rtiles, 1, &q, stream))) return rc;
-  if (rest && p->n_tiles_slow) return pylo_b200_apply(p->desc, p->tiles_slow, p->n_tiles_slow, 0, &q, stream);
-  return 0;
+  // the tiles go with the first launch of packed items that there is
+  int n_slow = rest ? p->n_tiles_slow : 0;
+  if (main && p->n_ctiles) {
+    if ((rc = pylo_b200_apply_packed(p->desc, p->ctiles, p->n_ctiles, 0, p->tiles_slow, n_slow, &q, stream))) return rc;
+    n_slow = 0;
+  }
+  return rest ? pylo_b200_apply_packed(p->desc, p->rtiles, p->n_rtiles, 1, p->tiles_slow, n_slow, &q, stream) : 0;
 }
 
 int pylo_b200_advance_steps(double* const* steps, int n, double* first, int* equal) {

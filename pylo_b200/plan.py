@@ -588,6 +588,8 @@ class LoPlan:
         other = "k_apply_adafac_tc<true>" if self.tensor_cores else "k_apply"
         apply = [(L.STEP_APPLY, self.apply_kernel if self.n_ctiles > self.n_ctiles_gen else other, main)]
         apply.insert(0 if self.tensor_cores else 1, (L.STEP_APPLY_REST, other, rest))
+        if self.family == L.FAM_VELO and (self.n_ctiles or self.n_rtiles):   # the packed sweep takes the other units' tiles along
+            apply = [(L.STEP_APPLY | L.STEP_APPLY_REST, self.apply_kernel, int(self.n_ctiles > 0) + int(self.n_rtiles > 0))]
         front = [(L.STEP_SUMS, "rowcol_sums", (self.n_ragged > 0) + (self.n_atiles > self.n_ragged) + (self.n_gitems > 0)), (L.STEP_FACTORS, "factor_update", 1),
                  (L.STEP_STATE, "state_moments", 1)]
         if self.small:

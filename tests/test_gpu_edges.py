@@ -409,6 +409,39 @@ def test_small_models_front_in_one_launch(family, extra, shapes, monkeypatch):
                 assert torch.allclose(x, sb[key], rtol=4e-6, atol=1e-12), key
 
 
+@pytest.mark.parametrize("shapes,launches", [([(40, 24), (24,)], 1), ([(65, 77), (7,), (1,)], 1), ([(1001, 1028), (65, 77), (16385,), (3, 3, 5, 5)], 2),
+                                             ([(3000, 2048), (2048,)], 1), ([(64, 64)], 1), ([(13,), (4099,)], 1)],
+                         ids=["aligned", "ragged", "both", "many items", "matrices only", "vectors only"])
+def test_velo_units_of_both_sweeps_in_one_launch(shapes, launches):
+    """VeLO's packed items and the other units' tiles by one launch, against a launch for each: the same numbers."""
+    from pylo_b200 import _lib as L
+
+    case = dict(shapes=shapes, init_seed=53, init_scale=0.1, grad_seed=54, grad_scale=0.3)
+    runs = []
+    for apart in (False, True):
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+        opt = _make("velo", params)
+        for t in (1, 2):
+            for p, g in zip(params, cases.grads_at(case, t)):
+                p.grad = g.cuda()
+            if t == 2:
+                plan, = _plans(opt)
+                assert sum(n for ph, _, n in plan._phases() if ph & (L.STEP_APPLY | L.STEP_APPLY_REST)) == launches
+                if apart:   # neither phase alone has both kinds
+                    whole = plan._phases
+
+                    def phases():
+                        kept = [ph for ph in whole() if not ph[0] & (L.STEP_APPLY | L.STEP_APPLY_REST)]
+                        return kept + [(L.STEP_APPLY, "items", 1), (L.STEP_APPLY_REST, "tiles", 1)]
+                    plan._phases = phases
+                    plan.enable_profile()
+            _step(opt, "velo", t)
+        torch.cuda.synchronize()
+        runs.append([p.detach().clone() for p in params])
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+    assert all(float((a - v.cuda()).abs().max()) > 0 for a, v in zip(runs[0], cases.init_values(case)) if v.numel() > 1)
+
+
 @pytest.mark.parametrize("shapes", [[(40, 24), (33, 28)], [(300, 1028), (7, 4)]], ids=["small", "blocks"])
 @pytest.mark.parametrize("family,extra", [("celo2", {"orthogonalize": False}), ("adafaclo", {})])
 def test_network_as_an_argument_is_the_folded_one(family, extra, shapes):
