@@ -325,6 +325,7 @@ __device__ __forceinline__ void cluster_store(float* p, uint32_t rank, float v) 
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
+__device__ __forceinline__ void cluster_store(int* p, uint32_t rank, int v) { cluster_store(reinterpret_cast<float*>(p), rank, __int_as_float(v)); }
 
 __device__ __forceinline__ float cluster_load(const float* p, uint32_t rank) {
   uint32_t a;

@@ -27,6 +27,7 @@ struct NcSmem {
   float part[NC_SIDE * NC_SIDE];                  // [column][row]: this CTA's share of a, then the sums
   float red[40];
   float sumsq[16];                                // of the CTAs' columns
+  int sent[16];                                   // by the cluster's CTAs, at the end: 2 x rounds of copies, + 1 after a wait that ran out
   uint64_t bar, got[2], free;
   uint32_t tmem_base;
   volatile int abort;
@@ -94,19 +95,15 @@ __global__ void __launch_bounds__(NC_THREADS, 1) k_ns_cluster(const __grid_const
   const bool rows_here = quarter * 32 < nr, mine = rows_here && 32 * group < nr;   // the same for the whole warp
   const uint32_t t_row = tmem + ((uint32_t)(quarter * 32) << 16);
   pdl_begin();
-  if (matrix >= it.batch) {   // fills the item's last cluster up
-    cluster_wait();
-  } else if (it.parts == 0) {
-    ns_small_body<NC_THREADS>(it.x + base, it.out + base, it.rows, it.cols, grp.iters, it.c0, it.c1, it.c2, it.eps, reinterpret_cast<float*>(&sm), sm.red);
-    cluster_wait();
-  } else {
+  const bool busy = matrix < it.batch;              // the others fill the item's last cluster up
+  const bool shared = busy && it.parts > 0;
   float xr[COLS / 64][16], acc = 0.f;
 #pragma unroll
   for (int q = 0; q < COLS / 64; ++q) {
     const int col = 16 * (group + 4 * q), kk = k0 + col;
 #pragma unroll
     for (int j = 0; j < 16; ++j) xr[q][j] = 0.f;
-    if (row < r && col < cs) {
+    if (shared && row < r && col < cs) {
       if (tall) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) if (kk + j < c) xr[q][j] = it.x[base + (long long)(kk + j) * r + row];
@@ -125,21 +122,31 @@ __global__ void __launch_bounds__(NC_THREADS, 1) k_ns_cluster(const __grid_const
       for (int j = 0; j < 16; ++j) acc = fmaf(xr[q][j], xr[q][j], acc);
     }
   }
-  acc = block_sum(acc, sm.red);
+  if (shared) acc = block_sum(acc, sm.red);
+  else if (busy)
+    ns_small_body<NC_THREADS>(it.x + base, it.out + base, it.rows, it.cols, grp.iters, it.c0, it.c1, it.c2, it.eps, reinterpret_cast<float*>(&sm), sm.red);
+  cluster_wait();
+  // A wait that runs out is one answer for the warp (`dead`), which waits for nothing from then on.  The first warp, which issues
+  // the CTA's products and copies and speaks to the other CTAs, does none of that any more either: so every barrier has had
+  // exactly as many arrivals and bytes as `products` and the CTAs' `sent` say, and what is still in flight can be waited for.
   uint32_t parity = 0, exchanged = 0, freed = 0;
+  int products = 0, sent = 0;
   bool dead = false;
+  auto wait = [&](uint64_t* bar, uint32_t phase) {
+    if (!dead) dead = !__all_sync(0xffffffffu, ns_wait(bar, phase, &sm.abort));
+  };
   // Told to the others: this CTA has read what they sent.  wait_free: all of them have said so.
   auto say_free = [&]() {
-    if (warp == 0 && lane < parts && lane != rank)
+    if (warp == 0 && !dead && lane < parts && lane != rank)
       asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(nf_at_rank(&sm.free, first + lane)) : "memory");
   };
   auto wait_free = [&]() {
-    if (!dead && !ns_wait(&sm.free, freed, &sm.abort)) dead = true;
+    wait(&sm.free, freed);
     __syncwarp();
     asm volatile("fence.acq_rel.cluster;" ::: "memory");
     freed ^= 1;
   };
-  cluster_wait();
+  if (shared) {
   double tot = (double)acc;
   if (parts > 1) {
     if (warp == 0 && lane < parts)
@@ -172,7 +179,8 @@ __global__ void __launch_bounds__(NC_THREADS, 1) k_ns_cluster(const __grid_const
     fence_async_smem();   // the operands were written through the generic proxy
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) {
+    if (warp == 0 && !dead) {
+      ++products;
       if (elect_one()) {
         tc_fence_after();
         const uint32_t ah = smem_addr(a_hi), al = smem_addr(a_lo), bh = smem_addr(b_hi), bl = smem_addr(b_lo);
@@ -196,7 +204,7 @@ __global__ void __launch_bounds__(NC_THREADS, 1) k_ns_cluster(const __grid_const
       }
       __syncwarp();
     }
-    if (!dead && !ns_wait(&sm.bar, parity, &sm.abort)) dead = true;
+    wait(&sm.bar, parity);
     parity ^= 1;
     __syncwarp();
     tc_fence_after();
@@ -224,14 +232,15 @@ __global__ void __launch_bounds__(NC_THREADS, 1) k_ns_cluster(const __grid_const
   auto send = [&](int which, const float* src, int step, float* dst) {
     asm volatile("fence.proxy.async;" ::: "memory");   // the pieces were written through the generic proxy
     __syncthreads();
-    if (warp == 0) {
+    if (warp == 0 && !dead) {
+      ++sent;
       if (lane == 0) nf_expect(&sm.got[which], (parts - 1) * block * 4);
       if (lane < parts && lane != rank)
         asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                      ::"r"(nf_at_rank(dst + rank * block, first + lane)), "r"(smem_addr(src + lane * step)), "r"(block * 4), "r"(nf_at_rank(&sm.got[which], first + lane)) : "memory");
       __syncwarp();
     }
-    if (!dead && !ns_wait(&sm.got[which], exchanged, &sm.abort)) dead = true;
+    wait(&sm.got[which], exchanged);
     __syncwarp();
   };
 
@@ -291,7 +300,7 @@ __global__ void __launch_bounds__(NC_THREADS, 1) k_ns_cluster(const __grid_const
     put_m();
     // ---- x' = c0 x + b x
     multiply(sm.m[0], sm.m[1], sm.x[0], sm.x[1], cs, nr / 16, true);
-    if (parts > 1) say_free();   // a's sums are read, and so is b: the next round's copies may come
+    if (parts > 1 && round + 1 < grp.iters) say_free();   // a's sums are read, and so is b: the next round's copies may come
 #pragma unroll
     for (int q = 0; q < COLS / 64; ++q) {
       const int col = 16 * (group + 4 * q);
@@ -319,11 +328,33 @@ __global__ void __launch_bounds__(NC_THREADS, 1) k_ns_cluster(const __grid_const
       }
     }
   }
-  if (parts > 1) wait_free();
   }
+  // After a wait that ran out nothing may be on its way when a CTA leaves: neither this CTA's products, nor copies into its shared
+  // memory, nor copies out of another's.  All CTAs say what they have sent; behind the barrier, where nobody sends any more, the
+  // failed ones take in what is theirs, and all of them stay until that is done.  A copy belongs to the phase of `got` that this
+  // CTA announced last, or to the next one, which it has not announced: another CTA is at most one round of copies ahead,
+  // and then only if the last announced phase is complete.
+  if (warp == 0 && lane < (int)cluster_size()) cluster_store(&sm.sent[cluster_rank()], lane, 2 * sent + (dead ? 1 : 0));
   tc_fence_before();
   __syncthreads();
   cluster_sync();   // no CTA leaves while another may write to its shared memory
+  if (__any_sync(0xffffffffu, lane < (int)cluster_size() && (sm.sent[lane] & 1))) {   // the same in all CTAs of the cluster
+    if (warp == 0 && dead) {
+      if (products) pipe_wait(&sm.bar, (uint32_t)(products - 1) & 1);
+      const int bytes = ((r + 31) & ~31) / parts * NC_SIDE * 4;
+      for (int which = 0; which < 2 && parts > 1; ++which) {
+        const int own = (sent + 1 - which) / 2;
+        const int theirs = lane < parts && lane != rank ? ((sm.sent[first + lane] >> 1) + 1 - which) / 2 : own;
+        const int missing = __popc(__ballot_sync(0xffffffffu, theirs < own)), ahead = __popc(__ballot_sync(0xffffffffu, theirs > own));
+        if (missing && lane == 0)   // these never come
+          asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&sm.got[which])), "r"(missing * bytes) : "memory");
+        if (own) pipe_wait(&sm.got[which], (uint32_t)(own - 1) & 1);
+        if (ahead && lane == 0) nf_expect(&sm.got[which], ahead * bytes);
+        if (ahead) pipe_wait(&sm.got[which], (uint32_t)own & 1);
+      }
+    }
+    cluster_sync();
+  }
   if (tid == 0 && sm.abort && status) atomicOr(status, 4);
   if (warp == 1) tc_dealloc(tmem, 512);
 }

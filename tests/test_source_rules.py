@@ -50,3 +50,19 @@ def test_a_failed_wait_of_the_ring_ends_the_whole_cta():
     assert "__all_sync(0xffffffffu, ok)" in bodies["pipe_wait"]
     sweep = bodies["k_state_moments"]
     assert sweep.index("block_reduce_store<NACC>") < sweep.index("dead = __syncthreads_or(dead)")
+
+
+def test_the_cluster_chain_takes_in_its_copies_after_a_failed_wait():
+    """k_ns_cluster's bulk copies land in other CTAs: after a wait that ran out every CTA stays until those of all are in, and the
+    products are done.  That can be counted only if the failed warp starts nothing more."""
+    body = functions()["k_ns_cluster"]
+    assert body.count("ns_wait(") == 1 and "!__all_sync(0xffffffffu, ns_wait(" in body   # one answer for the warp
+    for start in ("++products;", "++sent;"):   # products and copies of a warp that still waits only, all of them counted
+        assert re.search(r"if \(warp == 0 && !dead\) \{\s*" + re.escape(start), body), start
+    for word, start in (("nf_mma<", "++products;"), ("cp.async.bulk", "++sent;")):
+        assert body.index(start) < body.index(word) and body.count(word) == 1
+    for arrival in re.finditer(r"mbarrier\.arrive\.release\.cluster", body):
+        assert "!dead" in body[body.rindex("if (", 0, arrival.start()):arrival.start()]
+    told, stopped, gone = body.index("cluster_store(&sm.sent"), body.index("cluster_sync();"), body.rindex("cluster_sync();")
+    assert told < stopped < body.index("pipe_wait(&sm.bar") < gone and stopped < body.index("pipe_wait(&sm.got") < gone
+    assert max(body.rindex(word) for word in ("++products;", "++sent;", "say_free()")) < told
