@@ -31,7 +31,7 @@ from torch.optim import Optimizer
 
 from .. import _lib as L
 from ..models.Meta_MLP import MetaMLP
-from ..plan import GradNorm, LoPlan, LoTensor, current_stream_ptr, one_minus, with_gradients
+from ..plan import GradNorm, LoPlan, LoTensor, current_stream_ptr, model_shapes, one_minus, with_gradients
 from ._common import StepCounters, factored_dims_sorted, optimizer_step, require_cuda_param
 
 
@@ -94,6 +94,15 @@ class _AdafacFamily(Optimizer):
         super().add_param_group(param_group)
         self._plans = {}
 
+    @staticmethod
+    def _factoring(shape):
+        """(shape, factored axes, axis of row_col_mean)."""
+        fd, axis = factored_dims_sorted(shape), 0
+        if fd is not None:
+            dc, dr = fd
+            axis = dc - 1 if dc > dr else dc  # AdafacLO_cuda.py:342 (axis 0 is the decay axis)
+        return shape, fd, axis
+
     def _build_plan(self, plist):
         tensors = []
         for p in plist:
@@ -101,16 +110,14 @@ class _AdafacFamily(Optimizer):
             st = self.state[p]
             if len(st) == 0:
                 self._init_state(st, p)
-            fd = factored_dims_sorted(tuple(p.shape))
-            axis = 0
-            if fd is not None:
-                dc, dr = fd
-                axis = dc - 1 if dc > dr else dc  # AdafacLO_cuda.py:342 (axis 0 is the decay axis)
+            _, fd, axis = self._factoring(tuple(p.shape))
             tensors.append(LoTensor(
                 p=p.data, m=st["exp_avg"], v=st["exp_avg_sq"], fac_r=st["exp_avg_sq_r"], fac_c=st["exp_avg_sq_c"],
                 fdims=fd, rcm_axis=axis, w=self._w_flat, peer_ptrs=getattr(p, "_pylo_peer_ptrs", None),
                 peer_multicast=getattr(p, "_pylo_peer_multicast", False)))
-        return LoPlan(L.FAM_ADAFAC, tensors, self.device, tensor_cores=(self.mlp_precision == "3xtf32"))
+        model = model_shapes(plist)
+        return LoPlan(L.FAM_ADAFAC, tensors, self.device, tensor_cores=(self.mlp_precision == "3xtf32"),
+                      model=model and [self._factoring(s) for s in model])
 
     def check_status(self):
         """Synchronise and raise if a kernel of an earlier step reported a wait that ran out."""

@@ -29,7 +29,7 @@ from torch.optim import Optimizer
 from .. import _lib as L
 from ..models.VeLO_MLP import VeLOMLP
 from ..models.VeLO_RNN import VeLORNN
-from ..plan import LoPlan, LoTensor, current_stream_ptr, one_minus
+from ..plan import LoPlan, LoTensor, current_stream_ptr, one_minus, share_of
 from ._common import factored_dims_velo, group_floats, optimizer_step, require_cuda_param
 
 
@@ -231,7 +231,11 @@ class VeLO_CUDA(Optimizer):
                 tensors.append(LoTensor(fac_r=st["fac_vec_row"], fac_c=st["fac_vec_col"], rcm_axis=fd[0] + 1, **common))
             else:
                 tensors.append(LoTensor(fac_r=st["fac_vec_v"], fac_c=None, **common))
-        plan = LoPlan(L.FAM_VELO, tensors, dev)
+        model = None
+        if self._all_shapes is not None and share_of(plist, self._all_shapes):
+            dims = [(s, factored_dims_velo(s)) for s in self._all_shapes]
+            model = [(s, fd, 0 if fd is None else fd[0] + 1) for s, fd in dims]
+        plan = LoPlan(L.FAM_VELO, tensors, dev, model=model)
         w = self._rnn_w
         r = L.VeloRnn()
         r.mix2_w, r.mix2_b = w["mix_layer2.weight"].data_ptr(), w["mix_layer2.bias"].data_ptr()

@@ -9,8 +9,9 @@ sequence of one step.  Nothing here touches tensor values on the host.
 from __future__ import annotations
 
 import ctypes as C
+from collections import Counter
 from dataclasses import dataclass
-from typing import List, Optional, Sequence, Tuple
+from typing import List, NamedTuple, Optional, Sequence, Tuple
 
 import numpy as np
 import torch
@@ -72,6 +73,29 @@ def geometry(shape: Sequence[int], fdims):
     Y = int(shape[ay])
     I = _prod(shape[ay + 1:])
     return O, X, M, Y, I, int(dr == ay)
+
+
+def fill_geometry(d, shape: Sequence[int], fdims, rcm_axis: int, sliced: bool = False, tensors=()):
+    """The descriptor fields of a tensor of this shape that say how it is walked through; ``sliced``: its features are
+    normalised per matrix, ``tensors``: what has to be aligned for the fast mode.  Returns its (O, X, M, Y, I) and whether the mode
+    is FAST2D, or None for fewer than 2 dims."""
+    d["n"] = n = _prod(shape)
+    if fdims is None:
+        d["mode"] = L.MODE_VEC1D
+        d["O"] = d["X"] = d["M"] = d["I"] = 1
+        d["Y"] = min(n, 2**31 - 1)
+        d["r_is_a"] = 1
+        d["rcm_pre"] = d["rcm_A"] = d["rcm_post"] = 1
+        return None
+    O, X, M, Y, I, r_is_a = geometry(shape, fdims)
+    d["O"], d["X"], d["M"], d["Y"], d["I"], d["r_is_a"] = O, X, M, Y, I, r_is_a
+    d["La"], d["Lb"] = n // Y, n // X
+    rshape = [3] + list(shape)   # of the row accumulator
+    rshape[1 + fdims[1]] = 1
+    d["rcm_pre"], d["rcm_A"], d["rcm_post"] = _prod(rshape[:rcm_axis]), rshape[rcm_axis], _prod(rshape[rcm_axis + 1:])
+    fast = O == 1 and M == 1 and I == 1 and Y % 4 == 0 and n < 2**31 and not sliced and _aligned16(*tensors)
+    d["mode"] = L.MODE_FAST2D if fast else L.MODE_GENERIC
+    return O, X, M, Y, I, fast
 
 
 def _aligned16(*tensors) -> bool:
@@ -274,6 +298,51 @@ def small_front(mats: Sequence[Tuple[int, int]], vectors: Sequence[int]):
     return found or next((q for q in map(share, [cl for cl in (1, 2, 4, 8, 16) if T * cl <= 2 * SMALL_CTAS]) if q), None)
 
 
+class SumOrder(NamedTuple):
+    """How the sums over a tensor are made.  All of it decides in which order a tensor's terms are added up."""
+
+    small: Optional[Tuple[int, int, int, int]]   # see small_front
+    elems: int          # elements of a tile where that does not cut the tensors
+    sum_tiles: bool     # no launch for phase B2: of small units phase P adds the tile partials up, for VeLO the LSTM's input kernel does
+    bulk_copies: bool   # the state sweep reads through a ring of bulk copies
+
+    def tiles(self, sizes):
+        return equal_tiles(sizes, self.small[0]) if self.small else make_tiles(sizes, self.elems)
+
+
+def sum_order(family: int, d: np.ndarray, sizes: Sequence[int], modes: np.ndarray, sliced: bool) -> SumOrder:
+    """The rule, for tensors with these descriptors and their units of these sizes and modes.
+
+    Tiles: four 256-thread CTAs per SM, one pass of a CTA is 1024 elements; below ~10 M elements smaller tiles fill the GPU, above
+    they would only multiply the block reductions.
+
+    The state sweep's ring of bulk copies leaves little L1 cache to the units that are not FAST2D and keeps the launches around it
+    apart, so it has to have enough to do: from 64 M elements on (VeLO on 100 M: 1615 -> 1580 us per step, on 17 M: 341 -> 351;
+    AdafacLO on 25 M: 837 -> 851, on 86 M even), nearly all of them FAST2D."""
+    total, small = int(sum(sizes)), None
+    if not sliced and total <= 2 * SMALL_CTAS * L.SMALL_SLICE:
+        vectors = d["mode"] == L.MODE_VEC1D
+        if (vectors | plain_matrices(d)).all():
+            small = small_front(list(zip(d["X"][~vectors].tolist(), d["Y"][~vectors].tolist())), d["n"][vectors].tolist())
+    elems = tile_elems(total, 1024, 4 * L.SM_COUNT)
+    most = small[0] if small else -(-max(sizes, default=0) // elems)
+    fast = int(sum(n for n, m in zip(sizes, modes.tolist()) if m == L.MODE_FAST2D))
+    return SumOrder(small, elems, family == L.FAM_VELO or most <= SUM_TILES_MOST, fast >= L.BULK_COPY_ELEMS and 8 * fast >= 7 * total)
+
+
+def model_shapes(params) -> Optional[Sequence[Tuple[int, ...]]]:
+    """The shapes of all tensors of the model that these parameters are a rank's share of (the sharded steps of
+    :mod:`pylo_b200.zero` note them), or None where there is no such note or it does not fit them."""
+    noted = [getattr(p, "_pylo_model_shapes", None) for p in params]
+    first = noted[0] if noted else None
+    return first if first is not None and all(q is first or q == first for q in noted) and share_of(params, first) else None
+
+
+def share_of(params, shapes) -> bool:
+    """Whether these parameters can be some of a model's tensors of these shapes."""
+    return not Counter(tuple(p.shape) for p in params) - Counter(shapes)
+
+
 class LoPlan:
     """Descriptor tables, tile lists and workspace for the tensors of one optimizer instance.
 
@@ -284,7 +353,9 @@ class LoPlan:
 
     H = {L.FAM_ADAFAC: 32, L.FAM_CELO2: 8, L.FAM_VELO: 4}
 
-    def __init__(self, family: int, tensors: List[LoTensor], device, tensor_cores=False):
+    def __init__(self, family: int, tensors: List[LoTensor], device, tensor_cores=False, model=None):
+        """``model``: (shape, factored axes, rcm_axis) of all tensors of the model, in any order, of which ``tensors`` are a rank's
+        share; their step is then the one that a plan over the whole model makes, to the last bit."""
         self.family = family
         # whether the AdafacLO family's FAST2D tensors take the tensor-core apply kernel (TF32 operands)
         self.tensor_cores = bool(tensor_cores) and family == L.FAM_ADAFAC
@@ -296,7 +367,6 @@ class LoPlan:
         ws_items = []  # (table, row, field, count)
         atiles, ratiles, gitems = [], [], []
         ws_bytes = 0  # the library's own count of the workspace, checked against the layout below
-        plain = []    # per tensor: whether it is a matrix that phase A takes in strips and blocks of columns
         for i, t in enumerate(tensors):
             shape = tuple(t.p.shape)
             n = t.p.numel()
@@ -307,7 +377,9 @@ class LoPlan:
                 if x is not None and not (x.is_cuda and x.dtype == torch.float32 and x.is_contiguous()):
                     raise ValueError(f"{name} of tensor {i} must be a contiguous fp32 CUDA tensor")
             d = tdesc[i]
-            d["n"], d["m_stride"], d["idx0"] = n, n, 0
+            d["m_stride"], d["idx0"] = n, 0
+            sliced = t.slice_last2 and len(shape) > 2
+            sides = fill_geometry(d, shape, t.fdims, t.rcm_axis, sliced, (t.p, t.m, t.v, t.out))
             d["lr"], d["wd"], d["clip_norm"] = t.lr, t.wd, t.clip_norm
             d["exp_mult"], d["step_mult"] = t.exp_mult, t.step_mult
             d["p"], d["m"], d["v"] = t.p.data_ptr(), t.m.data_ptr(), t.v.data_ptr()
@@ -320,32 +392,17 @@ class LoPlan:
                 d["p_peer"][: len(t.peer_ptrs)] = list(t.peer_ptrs)
                 d["n_peer"] = -1 if t.peer_multicast else len(t.peer_ptrs)
             if t.fdims is None:
-                plain.append(False)
-                d["mode"] = L.MODE_VEC1D
-                d["O"] = d["X"] = d["M"] = d["I"] = 1
-                d["Y"] = min(n, 2**31 - 1)
-                d["r_is_a"] = 1
+                ws = L.workspace_layout(family, L.MODE_VEC1D, n)
                 d["fac_a"] = t.fac_r.data_ptr()
                 d["fac_b"] = t.fac_c.data_ptr() if t.fac_c is not None else 0
-                d["rcm_pre"] = d["rcm_A"] = d["rcm_post"] = 1
             else:
-                O, X, M, Y, I, r_is_a = geometry(shape, t.fdims)
-                d["O"], d["X"], d["M"], d["Y"], d["I"], d["r_is_a"] = O, X, M, Y, I, r_is_a
+                O, X, M, Y, I, fast = sides
                 La, Lb = n // Y, n // X
-                d["La"], d["Lb"] = La, Lb
-                fac_a, fac_b = (t.fac_r, t.fac_c) if r_is_a else (t.fac_c, t.fac_r)
+                fac_a, fac_b = (t.fac_r, t.fac_c) if t.fdims[1] > t.fdims[0] else (t.fac_c, t.fac_r)
                 d["fac_a"], d["fac_b"] = fac_a.data_ptr(), fac_b.data_ptr()
-                rshape = list(t.fac_r.shape)
-                ax = t.rcm_axis
-                d["rcm_pre"], d["rcm_A"], d["rcm_post"] = _prod(rshape[:ax]), rshape[ax], _prod(rshape[ax + 1:])
-                fast = (O == 1 and M == 1 and I == 1 and Y % 4 == 0 and n < 2**31
-                        and not (t.slice_last2 and t.p.dim() > 2) and _aligned16(t.p, t.m, t.v, t.out))
-                d["mode"] = L.MODE_FAST2D if fast else L.MODE_GENERIC
                 # matrices whose rows are not aligned go the way of the others with single accesses, where a warp finds its 32
                 # columns twice: 3.4 M VeLO parameters in rows of 1433 and 1001, sums 25.8 -> 13.5 us, apply sweep 68 -> 33
-                sliced = t.slice_last2 and t.p.dim() > 2
                 ragged = not fast and not sliced and O == M == I == 1 and Y >= 64
-                plain.append(fast or ragged)
                 # sub-buffer sizes and the phase-A tiling come from the library (pylo_b200_workspace_layout), so that
                 # this table and a table built by any other host of the C ABI agree
                 ws = L.workspace_layout(family, int(d["mode"]), n, La, Lb, X if fast or ragged else 0, Y if fast or ragged else 0)
@@ -362,9 +419,7 @@ class LoPlan:
                     rows[:, 2] = per
                     gitems.append(rows)
             ws_items.append(("t", i, "closed", L.STAT_STRIDE))
-            ws_bytes += L.lib.pylo_b200_workspace_bytes(
-                C.byref(L.workspace_layout(family, int(d["mode"]), n, int(d["La"]), int(d["Lb"]),
-                                           int(d["X"]) if plain[i] else 0, int(d["Y"]) if plain[i] else 0)), 1, 0)
+            ws_bytes += L.lib.pylo_b200_workspace_bytes(C.byref(ws), 1, 0)
 
         # units of element-wise work
         self.sliced = any(t.slice_last2 and t.p.dim() > 2 for t in tensors)
@@ -392,17 +447,15 @@ class LoPlan:
         else:
             udesc = tdesc
         sizes = [int(udesc["n"][u]) for u in range(U)]
-        # phase B: four 256-thread CTAs per SM, one pass of a CTA is 1024 elements; below ~10 M elements smaller tiles
-        # fill the GPU, above they would only multiply the block reductions
-        self.small = None
-        if not self.sliced and sum(sizes) <= 2 * SMALL_CTAS * L.SMALL_SLICE:
-            vectors = tdesc["mode"] == L.MODE_VEC1D
-            if (vectors | plain_matrices(tdesc)).all():
-                self.small = small_front(list(zip(tdesc["X"][~vectors].tolist(), tdesc["Y"][~vectors].tolist())), tdesc["n"][vectors].tolist())
-        if self.small:   # as many tiles a tensor as CTAs take its rows
-            tiles, ranges = equal_tiles(sizes, self.small[0])
+        if model is None:
+            order = sum_order(family, tdesc, sizes, udesc["mode"], self.sliced)
         else:
-            tiles, ranges = make_tiles(sizes, tile_elems(sum(sizes), 1024, 4 * L.SM_COUNT))
+            whole = np.zeros(len(model), dtype=L.DESC_DTYPE)
+            for d, (shape, fdims, rcm_axis) in zip(whole, model):
+                fill_geometry(d, shape, fdims, rcm_axis)   # the other ranks' buffers are aligned
+            order = sum_order(family, whole, whole["n"].tolist(), whole["mode"], False)
+        self.small = order.small   # as many tiles a tensor as CTAs take its rows
+        tiles, ranges = order.tiles(sizes)
         for u, (t0, k) in enumerate(ranges):
             udesc["tile0"][u], udesc["n_tiles"][u] = t0, k
             ws = L.workspace_layout(family, L.MODE_VEC1D, sizes[u])  # the per-unit part depends on the element count only
@@ -487,13 +540,7 @@ class LoPlan:
         self.tiles_slow = FixedTable(slow)
         self.n_tiles_slow = len(slow)
         self._fixed = FixedTable.place([self.tiles, self.atiles, self.gitems, self.ctiles, self.rtiles, self.pitems, self.tiles_slow], self.device)
-        #: no launch for phase B2: of small units phase P adds the tile partials up, for VeLO the LSTM's input kernel does.
-        self.sum_tiles = family == L.FAM_VELO or max((k for _, k in ranges), default=0) <= SUM_TILES_MOST
-        # The state sweep's ring of bulk copies leaves little L1 cache to the units that are not FAST2D and keeps the launches
-        # around it apart, so it has to have enough to do: from 64 M elements on (VeLO on 100 M: 1615 -> 1580 us per step, on
-        # 17 M: 341 -> 351; AdafacLO on 25 M: 837 -> 851, on 86 M even), nearly all of them FAST2D.
-        fast_elems = sum(sizes[u] for u in range(U) if udesc["mode"][u] == L.MODE_FAST2D)
-        self.bulk_copies = int(fast_elems >= L.BULK_COPY_ELEMS and 8 * fast_elems >= 7 * self.total_elems)
+        self.sum_tiles, self.bulk_copies = order.sum_tiles, int(order.bulk_copies)
         #: everything pylo_b200_step needs for a step over these tensors
         self.step_plan = L.StepPlan(
             tdesc=self.tdesc.ptr, desc=self.desc.ptr, atiles=self.atiles.ptr, gitems=self.gitems.ptr, pitems=self.pitems.ptr,

@@ -99,6 +99,18 @@ def partition_blocks(shapes: Sequence[Tuple[int, ...]], world_size: int, blocks:
     return owner, block, offsets, subs
 
 
+def _note_model(params: Sequence[torch.Tensor]):
+    """Note on every parameter the shapes of the whole model.
+
+    The order in which a step adds up the terms of a tensor's sums (tiles, clusters of CTAs) depends on how much the model gives
+    the GPU to do.  A rank's optimizer takes the model's order, not that of its share, so that its step is the single
+    process's to the last bit (see ``plan.sum_order``; the CELO2 family's tail and Newton-Schulz depend on
+    the share all the same: equal up to rounding)."""
+    shapes = tuple(tuple(p.shape) for p in params)
+    for p in params:
+        p._pylo_model_shapes = shapes
+
+
 class _GradIntake:
     """Gradient intake for a sharded step: data-parallel replicas reduce-scatter their gradients so that every rank
     receives exactly the gradients of the tensors it owns, already summed (docs/concepts.rst:274-283 describes the
@@ -178,6 +190,8 @@ class ShardedStep(_GradIntake):
             if copy_values:
                 view.copy_(p.data)
             p.data = view
+        if self.world > 1:
+            _note_model(self.params)
         self.owned = [i for i, r in enumerate(self.owner) if r == self.rank]
 
     @classmethod
@@ -200,6 +214,8 @@ class ShardedStep(_GradIntake):
             gen.manual_seed(seed * 1000003 + i)
             view.normal_(0.0, init_scale, generator=gen)
             self.params.append(torch.nn.Parameter(view, requires_grad=True))
+        if self.world > 1:
+            _note_model(self.params)
         self.owned = [i for i, r in enumerate(self.owner) if r == self.rank]
         return self
 
@@ -284,6 +300,8 @@ class FusedShardedStep(_GradIntake):
             gen.manual_seed(seed * 1000003 + i)
             view.normal_(0.0, init_scale, generator=gen)
             self.params.append(torch.nn.Parameter(view, requires_grad=True))
+        if self.world > 1:
+            _note_model(self.params)
         self.owned = [i for i, r in enumerate(self.owner) if r == self.rank]
         self.push = push if self.world > 1 else "stores"
         self._group_ranges, self._pushed = [], False
@@ -377,6 +395,8 @@ class StagedShardedStep(_GradIntake):
             gen.manual_seed(seed * 1000003 + i)
             view.normal_(0.0, init_scale, generator=gen)
             self.params.append(torch.nn.Parameter(view, requires_grad=True))
+        if self.world > 1:
+            _note_model(self.params)
         self.owned = [i for i, r in enumerate(self.owner) if r == self.rank]
         self.shard = sum(self.subs)
         self._comm = torch.cuda.Stream(device=device) if self.world > 1 and torch.device(device).type == "cuda" else None

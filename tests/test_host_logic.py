@@ -296,3 +296,29 @@ def test_small_models_are_dealt_to_clusters_that_hold_them():
             mine = tiles[t0:t0 + m]
             assert m == k and (mine["tensor"] == i).all() and (mine["elems"] % 4 == 0).all()
             assert int(np.clip(n - mine["start"], 0, mine["elems"]).sum()) == n
+
+
+def test_a_rank_s_plan_takes_the_order_of_sums_of_the_whole_model():
+    """What ShardedStep notes on the parameters, when the plan takes it, and that the order then does not depend on the share."""
+    from pylo_b200.optim.AdafacLO_cuda import AdafacLO_CUDA
+
+    shapes = ((96, 64), (64,), (8, 6, 5), (300, 260))
+    params = [torch.nn.Parameter(torch.zeros(s)) for s in shapes]
+    assert plan.model_shapes(params) is None
+    zero._note_model(params)
+    assert plan.model_shapes(params) == shapes and plan.model_shapes(params[2:]) == shapes
+    assert plan.model_shapes(params[:1] + [torch.nn.Parameter(torch.zeros(7))]) is None      # a tensor without the note
+    foreign = torch.nn.Parameter(torch.zeros(500, 500))
+    foreign._pylo_model_shapes = shapes
+    assert plan.model_shapes([foreign]) is None and plan.model_shapes([params[3], params[3]]) is None   # not of this model
+    assert plan.model_shapes([]) is None
+
+    def order(which):
+        d = np.zeros(len(which), dtype=L.DESC_DTYPE)
+        for row, s in zip(d, which):
+            _, fd, axis = AdafacLO_CUDA._factoring(s)
+            plan.fill_geometry(row, s, fd, axis)
+        return plan.sum_order(L.FAM_ADAFAC, d, d["n"].tolist(), d["mode"], False)
+
+    # the share alone would take the launch of small models, which the whole one does not: why the note is needed
+    assert order(shapes[3:]).small and not order(shapes).small
