@@ -347,8 +347,10 @@ int pylo_b200_transpose(const float* src, float* dst, int rows, int cols, int ld
  * x and out are [batch][rows][cols], contiguous, different; x is left as it is.  Operands are kept as two fp16 planes of one
  * power-of-two scale (22 significant bits, as many as a TF32 high and low part), which is sound while every |x| of the chain
  * stays below 10: the caller checks its coefficients.  Matrices of a few thousand elements run in plain fp32 instead,
- * those of up to 128 rows (their shorter side) and 3072 columns in one launch, a cluster of CTAs each, without a workspace.
- * work: pylo_b200_newton_schulz_workspace(...) bytes of device memory (may be NULL where that is 0), 256-byte aligned.
+ * those of up to 128 rows (their shorter side) and 3072 columns in one launch, a cluster of CTAs each, without a workspace, or
+ * in the launches of larger stacks of the same call.
+ * work: pylo_b200_newton_schulz_workspaces(...) bytes of device memory (may be NULL where that is 0), 256-byte aligned;
+ * pylo_b200_newton_schulz_workspace(...), what a stack needs at least, does too.
  * descs is a HOST array; all stacks run the same number of iterations.  status: device int, bit 2 is ORed in if a bounded wait ran out; may be NULL.  Returns -5 where the
  * driver offers no tensor maps. */
 typedef struct pylo_ns_desc {
@@ -360,8 +362,11 @@ typedef struct pylo_ns_desc {
   float c0, c1, c2, eps;
 } pylo_ns_desc;
 int64_t pylo_b200_newton_schulz_workspace(int rows, int cols, int batch, int iters);
+/* The bytes for every stack of one call, which may be more than what the stack needs at least: a few matrices of up to 128 rows run
+ * fastest in the launches of larger ones beside them.  x, out and work of the descs are not looked at. */
+int pylo_b200_newton_schulz_workspaces(const pylo_ns_desc* descs, int n, int64_t* bytes);
 int pylo_b200_newton_schulz(const pylo_ns_desc* descs, int n, int* status, void* stream);
-/* how many kernels that call launches (shapes, batches and iteration counts are looked at, no pointer) */
+/* how many kernels that call launches (x and out are not looked at) */
 int pylo_b200_newton_schulz_launches(const pylo_ns_desc* descs, int n);
 
 /* CELO2 tail (CELO2_cuda.py:336-339): step * rsqrt(mean(step^2 over the last two axes) + 1e-9) * rmsmult,

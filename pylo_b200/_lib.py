@@ -141,6 +141,7 @@ def _load():
         "pylo_b200_gemm_tn_3xtf32": [C.POINTER(GemmDesc), vp, vp],
         "pylo_b200_transpose": [vp, vp, i32, i32, i32, i32, C.c_int64, C.c_int64, i32, i32, vp],
         "pylo_b200_newton_schulz_workspace": [i32, i32, i32, i32],
+        "pylo_b200_newton_schulz_workspaces": [C.POINTER(NsDesc), i32, C.POINTER(C.c_int64)],
         "pylo_b200_newton_schulz": [C.POINTER(NsDesc), i32, vp, vp],
         "pylo_b200_newton_schulz_launches": [C.POINTER(NsDesc), i32],
         "pylo_b200_celo2_post_sums": [vp, vp, i32, vp],

@@ -2390,7 +2390,7 @@ static bool ns_is_small(int rows, int cols, int iters) {
 }
 
 // How a stack is run: 0, by single CTAs in plain fp32; 1 to 16, by so many CTAs a matrix (k_ns_cluster); -1, as a chain of
-// launches.  What fits clusters is faster there for any number of matrices (us per chain, launches / clusters, two of each run
+// launches.  Alone, what fits clusters is faster there for any number of matrices (us per chain, launches / clusters, two of each run
 // within 1 %: 128 x 784 155 / 64, 128 x 3072 184 / 83, 24 x 128 x 1000 288 / 140, 48 x 128 x 1000 413 / 280, 400 x 128 x 128
 // 833 / 120, 300 x 64 x 256 642 / 205), with as few CTAs a matrix as hold it (48 matrices of 128 x 128 to 128 x 512, with
 // up to 192 columns per CTA 73, with 128 125).
@@ -2402,15 +2402,68 @@ static int ns_parts(int rows, int cols, int iters) {
   while ((c + parts - 1) / parts > NC_COLS) parts *= 2;
   return parts;
 }
-// Whether a stack goes into the launch of clusters: what they take, and, where there is such a launch, a few small matrices.
-static bool ns_any_clusters(const pylo_ns_desc* descs, int n) {
-  for (int k = 0; k < n; ++k) if (ns_parts(descs[k].rows, descs[k].cols, descs[k].iters) > 0) return true;
-  return false;
+struct NsWork {   // byte offsets into the workspace, every buffer on a 1024-byte boundary
+  int64_t xp[2], ap, bp, a, x, part, inv, total;
+  int r, c, ldx, lda_p, lda, slices;
+};
+static NsWork ns_work(int rows, int cols, int batch) {
+  NsWork w = {};
+  w.r = rows < cols ? rows : cols;
+  w.c = rows < cols ? cols : rows;
+  w.ldx = (cols + 7) / 8 * 8;
+  w.lda_p = (w.r + 7) / 8 * 8;
+  w.lda = (w.r + 3) / 4 * 4;
+  const int64_t n = (int64_t)rows * cols;
+  w.slices = (int)((n + NF_SLICE - 1) / NF_SLICE);
+  int64_t at = 0;
+  auto take = [&](int64_t bytes) { const int64_t o = at; at += (bytes + 1023) / 1024 * 1024; return o; };
+  const int64_t planes_x = (int64_t)batch * rows * w.ldx * 4, planes_a = (int64_t)batch * w.r * w.lda_p * 4;
+  w.xp[0] = take(planes_x);
+  w.xp[1] = take(planes_x);
+  w.ap = take(planes_a);
+  w.bp = take(planes_a);
+  w.a = take((int64_t)batch * w.r * w.lda * 4);
+  w.x = take((int64_t)batch * n * 4);
+  w.part = take((int64_t)batch * w.slices * 4);
+  w.inv = take((int64_t)batch * 4);
+  w.total = at;
+  return w;
 }
-static bool ns_in_clusters(const pylo_ns_desc& d, bool clusters) {
-  const int parts = ns_parts(d.rows, d.cols, d.iters);
-  return parts > 0 || (clusters && parts == 0 && d.batch <= 16);
-}
+
+// Where a stack goes: the chain of launches, the launch of clusters, or a launch of single CTAs of its own.
+enum NsRoute { NS_CHAIN, NS_CLUSTERS, NS_SINGLE };
+struct NsRoutes {
+  bool chain = false, clusters = false;   // whether a stack needs the chain; whether there is a launch of clusters
+  long long fitting = 0;                  // matrices that would fit clusters
+  NsRoutes(const pylo_ns_desc* descs, int n) {
+    for (int k = 0; k < n; ++k) {
+      const int parts = ns_parts(descs[k].rows, descs[k].cols, descs[k].iters);
+      chain |= parts < 0;
+      if (parts > 0) fitting += descs[k].batch;
+    }
+    for (int k = 0; k < n; ++k) clusters |= by_size(descs[k]) == NS_CLUSTERS;
+  }
+  // Whether a stack goes with the chain: where it must, and beside larger ones also where it would fit clusters, as long as it is
+  // no more than a few tiles in launches that are there anyway: a launch of clusters before them costs its own 40 to 80 us (us per
+  // call, clusters first / riding: 512 x 512, 128 x 512, 1792 x 512 299 / 233; 512 x 784, 512 x 512, 100 x 512 285 / 219; 16 of
+  // 768 rows and one 50 x 768 1245 / 1167; 256 x 256 and 48 of 128 x 128 186 / 152).  64 matrices make the symmetric products take
+  // tiles of 256 x 256, three quarters of each for padding, and clusters are the better place (256 x 256 and 64 of 128 x 128 187 /
+  // 247, of 128 x 512 284 / 318; 512 x 512 and 400 of 128 x 128 308 / 909).
+  bool rides(int parts) const { return parts < 0 || (parts > 0 && chain && fitting < 64); }
+  // What has no workspace for the chain and fits clusters stays there.
+  NsRoute by_size(const pylo_ns_desc& d) const {
+    const int parts = ns_parts(d.rows, d.cols, d.iters);
+    if (parts == 0) return NS_SINGLE;
+    if (parts < 0) return NS_CHAIN;
+    return rides(parts) && d.work && ((uintptr_t)d.work & 255) == 0 && d.work_bytes >= ns_work(d.rows, d.cols, d.batch).total ? NS_CHAIN : NS_CLUSTERS;
+  }
+  // A launch of clusters takes a few small matrices along.
+  NsRoute operator()(const pylo_ns_desc& d) const {
+    const NsRoute to = by_size(d);
+    return to == NS_SINGLE && clusters && d.batch <= 16 ? NS_CLUSTERS : to;
+  }
+};
+
 // One launch: clusters as large as the most CTAs that share a matrix.
 template <int COLS>
 static int nc_launch(const nc_group& grp, int ctas, int cluster, int* status, cudaStream_t s) {
@@ -2732,37 +2785,18 @@ int pylo_b200_transpose(const float* src, float* dst, int rows, int cols, int ld
 // ------------------------------------------------------------------------------------------------
 // Newton-Schulz chain
 // ------------------------------------------------------------------------------------------------
-struct NsWork {   // byte offsets into the workspace, every buffer on a 1024-byte boundary
-  int64_t xp[2], ap, bp, a, x, part, inv, total;
-  int r, c, ldx, lda_p, lda, slices;
-};
-static NsWork ns_work(int rows, int cols, int batch) {
-  NsWork w = {};
-  w.r = rows < cols ? rows : cols;
-  w.c = rows < cols ? cols : rows;
-  w.ldx = (cols + 7) / 8 * 8;
-  w.lda_p = (w.r + 7) / 8 * 8;
-  w.lda = (w.r + 3) / 4 * 4;
-  const int64_t n = (int64_t)rows * cols;
-  w.slices = (int)((n + NF_SLICE - 1) / NF_SLICE);
-  int64_t at = 0;
-  auto take = [&](int64_t bytes) { const int64_t o = at; at += (bytes + 1023) / 1024 * 1024; return o; };
-  const int64_t planes_x = (int64_t)batch * rows * w.ldx * 4, planes_a = (int64_t)batch * w.r * w.lda_p * 4;
-  w.xp[0] = take(planes_x);
-  w.xp[1] = take(planes_x);
-  w.ap = take(planes_a);
-  w.bp = take(planes_a);
-  w.a = take((int64_t)batch * w.r * w.lda * 4);
-  w.x = take((int64_t)batch * n * 4);
-  w.part = take((int64_t)batch * w.slices * 4);
-  w.inv = take((int64_t)batch * 4);
-  w.total = at;
-  return w;
-}
-
 int64_t pylo_b200_newton_schulz_workspace(int rows, int cols, int batch, int iters) {
   if (rows <= 0 || cols <= 0 || batch <= 0 || iters < 0) return -1;
   return ns_parts(rows, cols, iters) >= 0 ? 0 : ns_work(rows, cols, batch).total;
+}
+
+int pylo_b200_newton_schulz_workspaces(const pylo_ns_desc* descs, int n, int64_t* bytes) {
+  CHECK_ARG(descs && bytes && n >= 0);
+  for (int k = 0; k < n; ++k) CHECK_ARG(descs[k].rows > 0 && descs[k].cols > 0 && descs[k].batch > 0 && descs[k].iters >= 0);
+  const NsRoutes route(descs, n);
+  for (int k = 0; k < n; ++k)
+    bytes[k] = route.rides(ns_parts(descs[k].rows, descs[k].cols, descs[k].iters)) ? ns_work(descs[k].rows, descs[k].cols, descs[k].batch).total : 0;
+  return 0;
 }
 
 typedef CUresult (*TensorMapEncode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -2879,15 +2913,15 @@ int pylo_b200_newton_schulz(const pylo_ns_desc* descs, int n, int* status, void*
   nc_group small = {};
   small.iters = n ? descs[0].iters : 0;
   auto run_clusters = [&]() { const int rc = small.n ? ns_clusters(small, status, s) : 0; small.n = 0; return rc; };
-  const bool clusters = ns_any_clusters(descs, n);
+  const NsRoutes route(descs, n);
   for (int k = 0; k < n; ++k) {
     const pylo_ns_desc& d = descs[k];
-    const int parts = ns_parts(d.rows, d.cols, d.iters);
-    if (ns_in_clusters(d, clusters)) {
-      small.p[small.n++] = {d.x, d.out, d.rows, d.cols, d.batch, parts, 0, d.c0, d.c1, d.c2, d.eps};
+    const NsRoute to = route(d);
+    if (to == NS_CLUSTERS) {
+      small.p[small.n++] = {d.x, d.out, d.rows, d.cols, d.batch, ns_parts(d.rows, d.cols, d.iters), 0, d.c0, d.c1, d.c2, d.eps};
       if (small.n == NF_GROUP)
         if (int rc = run_clusters()) return rc;
-    } else if (parts == 0) {
+    } else if (to == NS_SINGLE) {
       static bool configured[PYLO_MAX_DEVICES] = {};
       if (int rc = allow_dynamic_smem(k_ns_small, 200 * 1024, configured)) return rc;
       launch(k_ns_small, d.batch, NT, (size_t)ns_small_floats(d.rows, d.cols) * 4, s, d.x, d.out, d.rows, d.cols, d.iters, d.c0, d.c1, d.c2, d.eps);
@@ -2907,15 +2941,11 @@ int pylo_b200_newton_schulz(const pylo_ns_desc* descs, int n, int* status, void*
 
 int pylo_b200_newton_schulz_launches(const pylo_ns_desc* descs, int n) {
   CHECK_ARG(descs && n >= 0);
-  const bool clusters = ns_any_clusters(descs, n);
-  int in_clusters = 0, single = 0, chains = 0;
-  for (int k = 0; k < n; ++k) {
-    if (ns_in_clusters(descs[k], clusters)) ++in_clusters;
-    else if (ns_parts(descs[k].rows, descs[k].cols, descs[k].iters) == 0) ++single;
-    else ++chains;
-  }
+  const NsRoutes route(descs, n);
+  int of[3] = {};
+  for (int k = 0; k < n; ++k) ++of[route(descs[k])];
   auto groups = [](int m) { return (m + NF_GROUP - 1) / NF_GROUP; };
-  return groups(in_clusters) + single + groups(chains) * (2 + 3 * (n ? descs[0].iters : 0));
+  return groups(of[NS_CLUSTERS]) + of[NS_SINGLE] + groups(of[NS_CHAIN]) * (2 + 3 * (n ? descs[0].iters : 0));
 }
 
 int pylo_b200_apply_packed(const pylo_tensor_desc* descs, const pylo_atile* ctiles, int n_ctiles, int ragged,

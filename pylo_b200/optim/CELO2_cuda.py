@@ -31,8 +31,8 @@ from .. import _lib as L
 from ..models.CELO2_MLP import CELO2MLP
 from ..plan import (GradNorm, LoPlan, LoTensor, current_stream_ptr, fp32_gradient, grad_pointers, one_minus, tile_elems,
                     with_gradients)
-from ._common import (ItemPlan, factored_dims_argsort, group_floats, newton_schulz, newton_schulz_bounded, newton_schulz_buffers,
-                      newton_schulz_native, newton_schulz_tc, optimizer_step, require_cuda_param)
+from ._common import (ItemPlan, factored_dims_argsort, group_floats, newton_schulz, newton_schulz_bounded,
+                      newton_schulz_group_buffers, newton_schulz_native, newton_schulz_tc, optimizer_step, require_cuda_param)
 
 _IN, _HID = 30, 8
 _KEPT_FLOATS = 4 << 20  # elements up to which a plan keeps Newton-Schulz results and workspaces between steps
@@ -323,7 +323,7 @@ class _Celo2Family(Optimizer):
             results = group["kept"]
             if native:
                 if results is None:
-                    results = [newton_schulz_buffers(part, self.ns_iters) for part, _ in group["parts"]]
+                    results = newton_schulz_group_buffers([part for part, _ in group["parts"]], self.ns_iters)
                     if group["floats"] <= _KEPT_FLOATS:
                         # small models: results and workspaces stay with the plan; large ones take them from the allocator
                         # on every step, so that the training step can have the memory in between

@@ -117,15 +117,21 @@ def newton_schulz_bounded(coeffs, iters: int) -> bool:
     return iters >= 1
 
 
+def _ns_descs(stacks, iters):
+    descs = (L.NsDesc * len(stacks))()
+    for d, x in zip(descs, stacks):
+        d.rows, d.cols, d.iters = x.shape[-2], x.shape[-1], iters
+        d.batch = x.numel() // (d.rows * d.cols)
+    return descs
+
+
 def newton_schulz_native(stacks, outs, works, coeffs, iters, eps, status, stream):
     """One native call for the chains of several stacks of matrices (contiguous, 16-byte aligned): ``outs`` the results,
-    ``works`` uint8 tensors of at least :func:`newton_schulz_workspace` bytes (None where that is 0).  Returns the number of
-    launches."""
-    descs = (L.NsDesc * len(stacks))()
+    ``works`` their workspaces (:func:`newton_schulz_group_buffers`).  Returns the number of launches."""
+    descs = _ns_descs(stacks, iters)
     for d, x, out, work in zip(descs, stacks, outs, works):
         d.x, d.out = x.data_ptr(), out.data_ptr()
-        d.rows, d.cols, d.iters, d.eps = x.shape[-2], x.shape[-1], iters, eps
-        d.batch = x.numel() // (d.rows * d.cols)
+        d.eps = eps
         d.c0, d.c1, d.c2 = coeffs
         if work is not None:
             d.work, d.work_bytes = work.data_ptr(), work.numel()
@@ -134,10 +140,15 @@ def newton_schulz_native(stacks, outs, works, coeffs, iters, eps, status, stream
 
 
 def newton_schulz_buffers(x: torch.Tensor, iters: int):
-    """(result, workspace or None) for one stack of :func:`newton_schulz_native`."""
-    r, c = x.shape[-2:]
-    n = int(L.lib.pylo_b200_newton_schulz_workspace(r, c, x.numel() // (r * c), iters))
-    return torch.empty_like(x), torch.empty(n, dtype=torch.uint8, device=x.device) if n else None
+    """(result, workspace or None) for one stack of :func:`newton_schulz_native` that is alone in its call."""
+    return newton_schulz_group_buffers([x], iters)[0]
+
+
+def newton_schulz_group_buffers(stacks, iters: int):
+    """(result, workspace or None) for every stack of one call of :func:`newton_schulz_native`."""
+    need = (C_.c_int64 * len(stacks))()
+    L.check(L.lib.pylo_b200_newton_schulz_workspaces(_ns_descs(stacks, iters), len(stacks), need), "newton_schulz_workspaces")
+    return [(torch.empty_like(x), torch.empty(n, dtype=torch.uint8, device=x.device) if n else None) for x, n in zip(stacks, need)]
 
 
 def newton_schulz_tc(x: torch.Tensor, coeffs, iters: int = 5, eps: float = 1e-8, status=None, stream=None) -> torch.Tensor:

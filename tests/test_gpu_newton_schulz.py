@@ -173,3 +173,26 @@ def test_chain_in_one_launch(shapes, coeffs, iters):
         if max(x.shape) > 128:
             assert torch.equal(run([x])[0], out)
     assert int(status.item()) == 0
+
+
+# in the launches of larger stacks: up to 128 rows, wide and tall, odd pitches, one and many of them, and a single-CTA matrix
+RIDERS = [[(300, 260), (128, 512)], [(129, 129), (5, 97, 193), (3071, 128), (65, 65), (10, 128)], [(200, 200), (63, 70, 72)]]
+
+
+@pytest.mark.parametrize("shapes", RIDERS, ids=[str(s[0]) for s in RIDERS])
+def test_small_matrices_in_the_launches_of_larger_ones(shapes):
+    """Against fp64, under the bound of the chain of launches."""
+    from pylo_b200.optim import _common as K
+
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    xs = [torch.randn(s, device="cuda", generator=gen) * torch.exp(torch.randn(s[:-1] + (1,), device="cuda", generator=gen)) for s in shapes]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    bufs = K.newton_schulz_group_buffers(xs, 5)
+    launches = K.newton_schulz_native(xs, [o for o, _ in bufs], [w for _, w in bufs], COEFFS, 5, 1e-8, status, stream)
+    assert launches == 17 + sum(w is None for _, w in bufs)
+    for x, (out, _) in zip(xs, bufs):
+        exact = K.newton_schulz(x.double(), COEFFS)
+        e32 = float((K.newton_schulz(x, COEFFS).double() - exact).norm() / exact.norm())
+        assert float((out.double() - exact).norm() / exact.norm()) < max(4 * e32, 1e-5)
+    assert int(status.item()) == 0

@@ -1,5 +1,7 @@
 """Host-side logic that needs no GPU: factored-dims rules, geometry, tiling, ownership, flat layout."""
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -322,3 +324,34 @@ def test_a_rank_s_plan_takes_the_order_of_sums_of_the_whole_model():
 
     # the share alone would take the launch of small models, which the whole one does not: why the note is needed
     assert order(shapes[3:]).small and not order(shapes).small
+
+
+# (stacks of one call, launches, which of them have a workspace): a chain is two launches and three a round
+NS_ROUTES = [([(1, 512, 512), (1, 128, 512), (1, 1792, 512)], 17, (1, 1, 1)),
+             ([(1, 512, 784), (1, 512, 512), (1, 100, 512)], 17, (1, 1, 1)),
+             ([(12, 768, 768), (1, 50, 768), (4, 768, 3072), (1, 10, 128)], 18, (1, 1, 1, 0)),
+             ([(1, 256, 256), (63, 128, 128)], 17, (1, 1)),
+             ([(1, 256, 256), (40, 128, 128), (24, 128, 512)], 18, (1, 0, 0)),   # too many to ride: clusters, then the chain
+             ([(1, 256, 256), (64, 128, 128), (1, 10, 128)], 18, (1, 0, 0)),     # which take a small matrix along
+             ([(1, 128, 784), (1, 128, 128), (1, 10, 128)], 1, (0, 0, 0)),
+             ([(1, 65, 64)], 1, (0,)), ([(2, 10, 128)], 1, (0,)), ([(1, 129, 129)], 17, (1,))]
+
+
+@pytest.mark.parametrize("stacks,launches,spaces", NS_ROUTES, ids=[str(s[:2]) for s, _, _ in NS_ROUTES])
+def test_small_matrices_ride_in_the_newton_schulz_launches_of_larger_ones(stacks, launches, spaces):
+    """Up to 63 matrices that would fit a cluster add no launch to a call that has larger ones; without a workspace they do."""
+    descs = K._ns_descs([torch.empty(s, device="meta") for s in stacks], 5)
+    need = (ctypes.c_int64 * len(stacks))()
+    assert L.lib.pylo_b200_newton_schulz_workspaces(descs, len(stacks), need) == 0
+    assert tuple(int(b > 0) for b in need) == spaces
+    for d, b in zip(descs, need):
+        if b:
+            d.work, d.work_bytes = 1 << 20, b
+    assert L.lib.pylo_b200_newton_schulz_launches(descs, len(stacks)) == launches
+    for d in descs:   # what a caller has that asks for every stack by itself
+        d.work_bytes = L.lib.pylo_b200_newton_schulz_workspace(d.rows, d.cols, d.batch, d.iters)
+        d.work = (1 << 20) if d.work_bytes else None
+    small = any(b and not d.work_bytes for b, d in zip(need, descs))
+    assert L.lib.pylo_b200_newton_schulz_launches(descs, len(stacks)) == launches + (small and not (10, 128) in [s[1:] for s in stacks])
+    descs[0].rows = 0
+    assert L.lib.pylo_b200_newton_schulz_workspaces(descs, len(stacks), need) == -1
