@@ -186,17 +186,6 @@ class _Celo2Family(Optimizer):
             post.part = torch.zeros(max(post.n_tiles, 1), dtype=torch.float32, device=self.device)
             post.items["part"] = post.part.data_ptr() + 4 * post.items["tile0"].astype(np.uint64)
             plan["post"] = post
-            # where the packed sweep takes every matrix, its items' sums of squares of the raw steps stand in for a launch that reads
-            # the steps again (unless they are orthogonalised): (first item, items) of every matrix
-            pl = plan["lo"]
-            plan["squares"] = None
-            if not pl.sliced and pl.n_tiles_slow == 0 and pl.n_rtiles == 0:
-                owner = pl.ctiles.host["tensor"]   # ascending: the units in their order
-                first = np.searchsorted(owner, np.arange(len(lo)))
-                count = np.searchsorted(owner, np.arange(len(lo)), side="right") - first
-                buffer = torch.zeros(max(len(owner), 1), dtype=torch.float32, device=self.device)
-                plan["squares"] = (buffer, buffer.data_ptr() + 4 * first.astype(np.uint64), count.astype(np.int32),
-                                   post.items["part"].copy(), post.items["n_tiles"].copy())
             base_p = np.array([p.data_ptr() for p in lo], dtype=np.uint64)
             post.items["p"][:] = base_p[post.owner_t] + post.owner_off
         if adam:
@@ -209,6 +198,20 @@ class _Celo2Family(Optimizer):
             it["m"][:] = [st[keys[0]].data_ptr() for st in plan["adam_states"]]
             it["v"][:] = [st[keys[1]].data_ptr() for st in plan["adam_states"]]
         return plan
+
+    def _build_squares(self, plan):
+        """Where the packed sweep takes every matrix, its items' sums of squares of the raw steps stand in for a launch that reads
+        the steps again: (their buffer, first item and items of every matrix, what the table says otherwise); else None."""
+        lo, items = plan["lo"], plan["post"].items
+        if lo.sliced or lo.n_tiles_slow or lo.n_rtiles:
+            return None
+        owner = lo.ctiles.host["tensor"]   # ascending: the units in their order
+        units = np.arange(len(plan["lo_params"]))
+        first = np.searchsorted(owner, units)
+        count = np.searchsorted(owner, units, side="right") - first
+        buffer = torch.zeros(max(len(owner), 1), dtype=torch.float32, device=self.device)
+        return (buffer, buffer.data_ptr() + 4 * first.astype(np.uint64), count.astype(np.int32),
+                items["part"].copy(), items["n_tiles"].copy())
 
     def _params_struct(self, group, gnorm_ptr):
         prm = self._prm
@@ -289,7 +292,11 @@ class _Celo2Family(Optimizer):
         exp_mult, rmsmult = group_floats(group, "exp_mult", "rmsmult")
         lo.set_hyper(lr=lr, wd=wd, clip_norm=clip_norm, exp_mult=exp_mult)
         lo.refresh(grads)
-        squares = None if group["orthogonalize"] else plan["squares"]
+        squares = None
+        if not group["orthogonalize"]:   # steps that are orthogonalised have other squares: their groups need none of it
+            if "squares" not in plan:
+                plan["squares"] = self._build_squares(plan)
+            squares = plan["squares"]
         prm.step_squares = squares[0].data_ptr() if squares else None
         lo.run(prm, stream)
         prm.step_squares = None
@@ -304,7 +311,7 @@ class _Celo2Family(Optimizer):
             it = post.items
             it["step"][:] = np.array(steps, dtype=np.uint64)[post.owner_t] + post.owner_off
             it["lr"][:], it["wd"][:], it["rmsmult"][:] = lr, wd, rmsmult
-            if plan["squares"]:
+            if plan.get("squares"):
                 it["part"][:], it["n_tiles"][:] = plan["squares"][1:3] if squares else plan["squares"][3:5]
             post.upload()
             plan["post_key"] = key

@@ -520,3 +520,27 @@ def test_squares_of_the_raw_steps_from_the_apply_sweep():
     for a, b, init in zip(runs[0], runs[1], cases.init_values(case)):
         # the same terms in another order: each sum to a few 2^-24 of itself, half of that in its root
         assert float((a - b).abs().max()) <= 1e-5 * float((b - init.cuda()).abs().max()) + 2 ** -23 * float(b.abs().max())
+
+
+def test_orthogonalised_groups_build_no_tables_of_squares():
+    """They are made at the first step without orthogonalisation, with the results of the launch that reads the steps again."""
+    case = dict(shapes=[(40, 24), (300, 1028), (5, 4)], init_seed=53, init_scale=0.1, grad_seed=54, grad_scale=0.3)
+    runs = []
+    for own in (False, True):
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+        opt = _make("celo2", params, orthogonalize=True)
+        for t in (1, 2, 3, 4):
+            for p, g in zip(params, cases.grads_at(case, t)):
+                p.grad = g.cuda()
+            opt.param_groups[0]["orthogonalize"] = t % 2 == 1
+            opt.step()
+            plan = opt._plans[0][1]
+            if t == 1:
+                assert plan.get("squares") is None
+                if own:
+                    plan["squares"] = None
+        assert own or plan["squares"] is not None
+        runs.append([p.detach().clone() for p in params])
+    for a, b, init in zip(runs[0], runs[1], cases.init_values(case)):
+        # the same terms in another order: each sum to a few 2^-24 of itself, half of that in its root
+        assert float((a - b).abs().max()) <= 1e-5 * float((b - init.cuda()).abs().max()) + 2 ** -23 * float(b.abs().max())
