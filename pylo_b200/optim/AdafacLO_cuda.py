@@ -32,7 +32,7 @@ from torch.optim import Optimizer
 from .. import _lib as L
 from ..models.Meta_MLP import MetaMLP
 from ..plan import GradNorm, LoPlan, LoTensor, current_stream_ptr, model_shapes, one_minus, with_gradients
-from ._common import StepCounters, factored_dims_sorted, optimizer_step, require_cuda_param
+from ._common import FlatWeights, StepCounters, factored_dims_sorted, optimizer_step, require_cuda_param
 
 
 def _decay_to_param(x):
@@ -54,8 +54,7 @@ class _AdafacFamily(Optimizer):
         flat = network.flat_weights()
         if tuple(flat[0].shape) != (32, 39):
             raise ValueError(f"{self._name} kernel only supports the 39->32->32->2 MetaMLP.")
-        self._w_flat = torch.cat([t.reshape(-1) for t in flat]).to(self.device).contiguous()
-        self._w_host = self._w_flat.cpu().numpy()   # the apply sweep's launch carries its output layer
+        self._weights = FlatWeights(flat, self.device)   # the apply sweep's launch carries the output layer
         self._plans = {}
         self._gnorm = None
         if self.mlp_precision not in ("fp32", "3xtf32"):
@@ -68,6 +67,10 @@ class _AdafacFamily(Optimizer):
         self._w_m, self._w_f = one_minus(self.beta_m), one_minus(self.beta_adafactor)
         self._w_v = one_minus(self.beta_rms)[0]
         self._prm = None   # the launch constants, made once
+
+    @property
+    def _w_flat(self):
+        return self._weights.flat
 
     def _init_state(self, state, p):
         """AdafacLO_cuda.py:227-256 / ELO_cuda.py:160-176."""
@@ -154,13 +157,13 @@ class _AdafacFamily(Optimizer):
         prm = self._prm
         if prm is None:
             prm = self._prm = L.StepParams()
-            prm.w_host = self._w_host.ctypes.data
             prm.family = L.FAM_ADAFAC
             for k in range(3):
                 prm.w_m[k], prm.w_f[k] = self._w_m[k], self._w_f[k]
             prm.w_v = self._w_v
             prm.eps_feat, prm.eps_norm = 1e-6, 1e-5
             prm.clip_val = float("inf")
+        prm.w_host = self._weights.host()
         prm.nan_to_num, prm.wd_mode, prm.eps_v, prm.gnorm_sq = nan_to_num, wd_mode, eps_v, gnorm_ptr
         return prm
 

@@ -31,7 +31,7 @@ from .. import _lib as L
 from ..models.CELO2_MLP import CELO2MLP
 from ..plan import (GradNorm, LoPlan, LoTensor, current_stream_ptr, fp32_gradient, grad_pointers, one_minus, tile_elems,
                     with_gradients)
-from ._common import (ItemPlan, factored_dims_argsort, group_floats, newton_schulz, newton_schulz_bounded,
+from ._common import (FlatWeights, ItemPlan, factored_dims_argsort, group_floats, newton_schulz, newton_schulz_bounded,
                       newton_schulz_group_buffers, newton_schulz_native, newton_schulz_tc, optimizer_step, require_cuda_param)
 
 _IN, _HID = 30, 8
@@ -73,8 +73,7 @@ class _Celo2Family(Optimizer):
             raise ValueError(f"{self._name} kernel only supports ff_hidden_size=8, ff_hidden_layers=2.")
         self.w_in, self.b_in, self.w_h, self.b_h, self.w_out, self.b_out = (
             t.to(dev) for t in self.network.flat_weights())
-        self._w_flat = torch.cat([t.reshape(-1) for t in (self.w_in, self.b_in, self.w_h, self.b_h, self.w_out, self.b_out)]).contiguous()
-        self._w_host = self._w_flat.cpu().numpy()   # the apply sweep's launch carries it
+        self._weights = FlatWeights((self.w_in, self.b_in, self.w_h, self.b_h, self.w_out, self.b_out), dev)   # the apply sweep's launch carries them
         self._plans = {}
         self._gnorm = None
         # "3xtf32" (default): the Newton-Schulz products on the tensor cores (this library's kernels, operands split
@@ -92,6 +91,10 @@ class _Celo2Family(Optimizer):
         self._w_v = float(1 - self.beta_rms[-1])
         self._prm = None   # the launch constants, made once
         self._b1_shared, self._b2_shared = float(self.beta_m[0]), float(self.beta_rms[-1])
+
+    @property
+    def _w_flat(self):
+        return self._weights.flat
 
     # ------------------------------------------------------------------ state
     def _init_lo_state(self, state, p):
@@ -222,7 +225,7 @@ class _Celo2Family(Optimizer):
                 prm.w_m[k], prm.w_f[k] = self._w_m[k], self._w_f[k]
             prm.w_v = self._w_v
             prm.eps_feat, prm.eps_norm = 1e-8, 1e-9
-            prm.w_host = self._w_host.ctypes.data
+        prm.w_host = self._weights.host()
         prm.clip_val, prm.gnorm_sq = float(group["grad_clip_val"]), gnorm_ptr
         return prm
 

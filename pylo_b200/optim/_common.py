@@ -235,6 +235,27 @@ def optimizer_step(step):
     return run
 
 
+class FlatWeights:
+    """A small network's weights, one after the other: ``flat`` on the device, which descriptors point to, and on the host what
+    launches carry as arguments.
+
+    The host's values are read from ``flat`` here and nowhere else, again after every write to it that autograd's version counter
+    sees (not one through ``.data`` or by a foreign kernel), so that a step does not mix old and new ones."""
+
+    def __init__(self, parts, device):
+        with torch.inference_mode(False):   # a tensor made in inference mode counts nothing
+            self.flat = torch.cat([t.detach().reshape(-1) for t in parts]).to(device).contiguous()
+        self._version = None
+
+    def host(self) -> int:
+        """Address of the host's copy, good until the next call."""
+        version = self.flat._version
+        if version != self._version:
+            self._values = self.flat.detach().cpu().numpy()
+            self._address, self._version = self._values.ctypes.data, version
+        return self._address
+
+
 class StepCounters:
     """The ``step`` entries of some parameters' states, advanced together.
 

@@ -1,6 +1,8 @@
 """GPU checks at the sizes where the work lists, the generic paths and the Newton-Schulz chain can go wrong: edges of tiles,
 remainders, the smallest and the largest of a range; against the CPU oracle or an fp64 evaluation."""
 
+import copy
+
 import pytest
 import torch
 
@@ -544,3 +546,37 @@ def test_orthogonalised_groups_build_no_tables_of_squares():
     for a, b, init in zip(runs[0], runs[1], cases.init_values(case)):
         # the same terms in another order: each sum to a few 2^-24 of itself, half of that in its root
         assert float((a - b).abs().max()) <= 1e-5 * float((b - init.cuda()).abs().max()) + 2 ** -23 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("family", ["adafaclo", "elo", "celo2", "elo_celo2"])
+def test_new_weights_of_the_network_reach_all_launches(family):
+    """Weights written into the flat tensor between steps act as those of an optimizer that is made with them: parts of the network
+    reach the kernels through descriptors, others as arguments of a launch."""
+    from pylo_b200 import optim
+
+    cls = {"adafaclo": optim.AdafacLO_CUDA, "elo": optim.ELO_CUDA, "celo2": optim.CELO2_CUDA, "elo_celo2": optim.ELO_CELO2_CUDA}[family]
+    case = dict(shapes=[(40, 24), (300, 1028), (33, 35), (24,)], init_seed=55, init_scale=0.1, grad_seed=56, grad_scale=0.3)
+    new = _nets(family)
+    with torch.no_grad():
+        for w in new.parameters():
+            w.mul_(1.5)
+    runs = []
+    for late in (False, True):
+        params = [torch.nn.Parameter(v.cuda()) for v in cases.init_values(case)]
+        opt = cls(params, lr=1e-2, network=_nets(family))
+        for t in (1, 2):
+            for p, g in zip(params, cases.grads_at(case, t)):
+                p.grad = g.cuda()
+            if t == 2:
+                made = cls(params, lr=1e-2, network=copy.deepcopy(new))
+                if late:
+                    opt._w_flat.copy_(made._w_flat)
+                else:
+                    made.load_state_dict(opt.state_dict())
+                    opt = made
+            opt.step()
+        runs.append([p.detach().clone() for p in params])
+    for a, b in zip(*runs):
+        assert torch.equal(a, b)
+    with pytest.raises(AttributeError):   # plans point to the old one
+        opt._w_flat = made._w_flat
