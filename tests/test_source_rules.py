@@ -23,23 +23,42 @@ def functions():
     return out
 
 
+REACH = re.compile(r"\b(cluster_store|cluster_load|nf_at_rank)\(")
+
+
+def barriers(body):
+    """Cluster barriers that all threads pass, whatever branch they took: [(place, whether it orders memory accesses)]."""
+    top = lambda at: body.count("{", 0, at) == body.count("}", 0, at)
+    places = lambda text: [m.start() for m in re.finditer(re.escape(text), body) if top(m.start())]
+    release, acquire = places('asm volatile("barrier.cluster.arrive.release'), places('asm volatile("barrier.cluster.wait.acquire')
+    halves = [(at, False) for at in places("cluster_wait();")[len(places("cluster_arrive();")) - 1:]]
+    return sorted([(at, True) for at in places("cluster_sync();")] + halves + [(w, True) for w in acquire if any(r < w for r in release)])
+
+
 def test_no_cta_reaches_into_another_before_it_is_known_to_run():
-    """Distributed shared memory may be accessed only once every CTA of the cluster has started (a cluster barrier)."""
+    """Distributed shared memory may be accessed only once every CTA of the cluster has started (a cluster barrier), and read only
+    behind one that orders the accesses before it; and no CTA leaves before a barrier behind the last access."""
     bodies = functions()
-    assert {"k_factor_update", "nf_gemm_body"} <= set(bodies)
+    seen = set()
     for name, body in bodies.items():
-        reach = re.search(r"\b(cluster_store|nf_at_rank)\(", body)
-        if name in ("cluster_store", "nf_at_rank") or not reach or "cluster_rank()" not in body:
+        reach = list(REACH.finditer(body))
+        if name in ("cluster_store", "cluster_load", "nf_at_rank") or not reach or "cluster_rank()" not in body:
             continue
-        before = body[:reach.start()]
-        assert "cluster_sync();" in before or re.search(r"cluster_arrive\(\);.*cluster_wait\(\);", before, re.S), name
+        seen.add(name)
+        first, last = reach[0].start(), reach[-1].start()
+        assert any(at < first for at, _ in barriers(body)), name
+        assert any(at > last for at, ordered in barriers(body) if ordered), name
+        for look in re.finditer(r"\bcluster_load\(", body):
+            assert any(at < look.start() for at, ordered in barriers(body) if ordered), name
+    assert {"k_factor_update", "k_small_front", "k_ns_cluster", "nf_gemm_body"} <= seen
 
 
 def test_kernels_that_write_parameters_look_at_the_status_word():
-    """After a wait that ran out the step's sums are incomplete; no kernel may write parameters from them.  (k_adamw reads
+    """After a wait that ran out the step's sums are incomplete; no kernel may write parameters, or VeLO's LSTM state, from them.  (k_adamw reads
     nothing that an earlier kernel of the step makes.)"""
     bodies = functions()
-    for name in ("k_apply", "k_apply_adafac_cols", "k_apply_packed", "k_post_apply", "k_velo_cell", "k_velo_xmix"):
+    for name in ("k_apply", "k_apply_adafac_cols", "k_apply_packed", "k_post_apply", "k_velo_lstm", "k_velo_mix", "k_velo_cell",
+                 "k_velo_xmix"):
         assert "reported(" in bodies[name], name
     assert "poisoned" in bodies["k_apply_adafac_tc"]
 
