@@ -2038,9 +2038,10 @@ __device__ __forceinline__ float velo_cell(float i, float g, float f, float o, f
 // hidden unit (one half of their columns: those that meet x', or those that meet h) in registers and takes eight tensors at a time
 // from shared memory: 512 FMAs per lane on 32 shared-memory reads, then the 32 sums are reduced over the lanes together, 31
 // shuffles in all, and lane l ends with the sum of tensor l / 4 and gate l % 4.  The other half's sums come from the warp beside
-// it, the four gates of a tensor from the lanes beside.  512 hidden units: 6 tensors 68.6 -> 3.6 us, 292 tensors 124 -> 46 us (the
-// tiled kernel below, which is kept for hidden sizes that are not multiples of 128, or above 512), and the cell was another launch
-// of 2.8.  Other CTAs still read h: the new one is left in `gates` ([T][H]), k_velo_mix takes it over.
+// it, the four gates of a tensor from the lanes beside.  512 hidden units, the gates alone: 6 tensors 3.6 us, 292 tensors 46, in the
+// tiled kernel below, which is for hidden sizes that are not multiples of 128 or above 512, 68.6 and 124; with the cell, which
+// would be another launch of 2.8, 6.7 and 57 as launches by themselves under the profiler.  Other CTAs still read h: the new one is
+// left in `gates` ([T][H]), k_velo_mix takes it over.
 #define GR_UNITS 4   // hidden units per CTA: one per pair of warps
 template <int NI>    // float4 per lane and row: H = 128 * NI
 __global__ void __launch_bounds__(NT, 2) k_velo_lstm(const pylo_velo_rnn r, int groups_per_cta) {

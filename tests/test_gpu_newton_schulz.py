@@ -152,7 +152,8 @@ CLUSTERED = [[(65, 65)], [(128, 128)], [(128, 192)], [(5, 97, 193)], [(33, 769)]
 @pytest.mark.parametrize("coeffs,iters", [(COEFFS, 5), ((1.5, -0.5, 0.0), 3)])
 def test_chain_in_one_launch(shapes, coeffs, iters):
     """Against fp64, as close as the fp32 chain (both round every entry of three products a round to 2^-22 or less of its
-    largest terms: the same bound as for the chain of launches); and what a matrix gives does not depend on its company."""
+    largest terms: the same bound as for the chain of launches); and what a matrix gives does not depend on its company, but
+    for those that a single CTA takes, which are summed by as many threads as the launch has."""
     from pylo_b200.optim import _common as K
 
     gen = torch.Generator(device="cuda").manual_seed(11)
@@ -170,7 +171,7 @@ def test_chain_in_one_launch(shapes, coeffs, iters):
         exact = K.newton_schulz(x.double(), coeffs, iters)
         e32 = float((K.newton_schulz(x, coeffs, iters).double() - exact).norm() / exact.norm())
         assert float((out.double() - exact).norm() / exact.norm()) < max(4 * e32, 1e-5)
-        if max(x.shape) > 128:
+        if tuple(x.shape) != (10, 128):
             assert torch.equal(run([x])[0], out)
     assert int(status.item()) == 0
 
