@@ -246,6 +246,7 @@ class FlatWeights:
         with torch.inference_mode(False):   # a tensor made in inference mode counts nothing
             self.flat = torch.cat([t.detach().reshape(-1) for t in parts]).to(device).contiguous()
         self._version = None
+        self.host()   # now, not in the first step
 
     def host(self) -> int:
         """Address of the host's copy, good until the next call."""
