@@ -462,7 +462,10 @@ int pylo_b200_velo_loss_features(float* means, int32_t* iteration, float* runnin
 #define PYLO_STEP_APPLY_REST 64
 #define PYLO_STEP_FRONT (PYLO_STEP_SUMS | PYLO_STEP_FACTORS | PYLO_STEP_STATE | PYLO_STEP_MOMENTS)
 #define PYLO_STEP_BACK (PYLO_STEP_PREP | PYLO_STEP_APPLY | PYLO_STEP_APPLY_REST)
-#define PYLO_TC_ONE_LAUNCH 4736 /* items below which one launch takes both kinds of items of apply_adafac_tc */
+#define PYLO_TC_ONE_LAUNCH 4736 /* items on FAST2D units below which one launch of apply_adafac_tc takes both kinds of items: \
+                                  the variant that takes both is 2 % slower on FAST2D items (ViT-B/16 2700 / 2751 us per \
+                                  step, two Llama-3-8B blocks 12640 / 12925), a launch more costs about 10 us (convolutions \
+                                  of 11 M parameters with a 0.5 M classifier 308.6 / 302.7) */
 typedef struct pylo_step_plan {
   const pylo_tensor_desc *tdesc, *desc; /* per tensor, per unit */
   const pylo_atile *atiles, *gitems, *pitems, *ctiles;

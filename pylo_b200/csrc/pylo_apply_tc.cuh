@@ -221,7 +221,7 @@ struct TcSmem {
 struct TcHeads { float w[64], b[2]; };
 
 // GENERIC: the launch may hold items on tensors that are not FAST2D.  The variant without them is the faster one on large
-// models (their body costs the other one registers: 1 % of the sweep over two Llama blocks).
+// models (their body costs the other one registers: 2 % of the step over two Llama blocks).
 template <bool GENERIC, bool ARG>
 __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const pylo_tensor_desc* __restrict__ descs,
                                                               const pylo_atile* __restrict__ ttiles, int n_ttiles,

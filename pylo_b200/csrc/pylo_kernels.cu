@@ -3087,7 +3087,7 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
   const bool main = phases & PYLO_STEP_APPLY, rest = phases & PYLO_STEP_APPLY_REST;
   if (p->tensor_cores) {
     // small models: one launch; large ones: what is not FAST2D first, then the others through the leaner variant
-    const int first = p->n_ctiles < PYLO_TC_ONE_LAUNCH ? 0 : p->n_ctiles_gen;
+    const int first = p->n_ctiles - p->n_ctiles_gen < PYLO_TC_ONE_LAUNCH ? 0 : p->n_ctiles_gen;
     if (rest && (rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles, first, 1, &q, p->status, p->host_status, stream))) return rc;
     if (main && (rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles + first, p->n_ctiles - first, p->n_ctiles_gen > first, &q, p->status, p->host_status, stream))) return rc;
     return 0;

@@ -264,9 +264,15 @@ def apply_items(family: int, tensor_cores: bool, fast, slow, least: int = 8) -> 
     """Work list of the tiled apply sweep: ``fast`` = [(unit, rows, columns)] of the FAST2D units, ``slow`` = [(unit,
     elements)] of the others, which only the tensor-core kernel takes (as runs of 128 elements, first in the list)."""
     if tensor_cores:
-        parts = [(u, -(-n // 128), 128, L.TC_GEN_ITEM) for u, n in slow] + [(u, X, Y, 0) for u, X, Y in fast]
-        rt = tensor_core_rows([(X, Y) for _, X, Y, _ in parts])
-        parts = [(u, X, Y, rt, 128, tag | rt) for u, X, Y, tag in parts]
+        slow = [(u, -(-n // 128), 128) for u, n in slow]
+        rows = lambda parts: tensor_core_rows([(X, Y) for _, X, Y in parts])
+        gen = both = rows(slow + fast)
+        if sum(-(-X // both) * -(-Y // 128) for _, X, Y in fast) >= L.TC_ONE_LAUNCH and slow:
+            # A large model's slow units have a launch of their own, which is over when its longest item is: their height follows
+            # from them alone.  At the FAST2D units' 64 rows a ViT-B/16's patch embedding was 72 items of 64 tiles for 592
+            # workers, and the SMs that had them came late to the FAST2D launch (133 us by itself, now 21)
+            gen, both = rows(slow), rows(fast)
+        parts = [(u, X, Y, gen, 128, L.TC_GEN_ITEM | gen) for u, X, Y in slow] + [(u, X, Y, both, 128, both) for u, X, Y in fast]
     else:
         parts = [(u, X, Y) + apply_tile_shape(family, X, Y, least) for u, X, Y in fast]
         if family != L.FAM_ADAFAC:
@@ -629,7 +635,7 @@ class LoPlan:
 
     def _phases(self):
         """[(phase of pylo_b200_step, name, launches)] in the step's order, without those that launch nothing."""
-        split = self.tensor_cores and self.n_ctiles >= L.TC_ONE_LAUNCH   # a launch of its own for what is not FAST2D
+        split = self.tensor_cores and self.n_ctiles - self.n_ctiles_gen >= L.TC_ONE_LAUNCH   # a launch of its own for what is not FAST2D
         rest = int(split and self.n_ctiles_gen > 0) if self.tensor_cores else int(self.n_tiles_slow > 0) + int(self.n_rtiles > 0)
         main = int(self.n_ctiles > (self.n_ctiles_gen if split else 0))
         other = "k_apply_adafac_tc<true>" if self.tensor_cores else "k_apply"

@@ -165,6 +165,19 @@ def test_apply_work_lists_cover_all_units_exactly_once(family, tc, fast, slow):
     assert all((x == 1).all() for x in list(seen.values()) + list(runs.values()))
 
 
+@pytest.mark.parametrize("layers,height", [(1, None), (2, None), (48, 8)])
+def test_slow_units_of_a_large_model_have_a_height_of_their_own(layers, height):
+    """From PYLO_TC_ONE_LAUNCH items on FAST2D units on, the others have a launch that ends with its longest item."""
+    fast, slow = [(1 + k, 768, 3072) for k in range(layers)], [(0, 768 * 768), (99, 130)]
+    items = plan.apply_items(L.FAM_ADAFAC, True, fast, slow)
+    gen = items["pad_"] >= L.TC_GEN_ITEM
+    of_slow, of_fast = set((items["pad_"][gen] & 0xffff).tolist()), set(items["pad_"][~gen].tolist())
+    assert len(of_slow) == len(of_fast) == 1
+    assert ((~gen).sum() >= L.TC_ONE_LAUNCH) == (height is not None)
+    assert of_slow == ({height} if height else of_fast)
+    assert gen.sum() == sum(-(-n // (128 * min(of_slow))) for _, n in slow)
+
+
 def test_packed_rows_give_every_sm_its_tiles():
     """Rows per thread of the packed sweep: the most that still leave sixteen tiles per SM (four below 32 rows)."""
     for X, Y in ((4096, 4096), (1024, 1024), (300, 260), (16, 8), (50257, 768)):
