@@ -50,8 +50,8 @@ B_BYTES = 40  # state_moments sweep: reads g, p, m(3), v; writes m(3), v
 # DRAM bytes per element (dram__bytes_read.sum + dram__bytes_write.sum) of the dominant kernels: CONSTANTS taken
 # from ncu captures of a 4096 x 4096 case, not measured in this run; traffic grows in proportion to the elements
 NCU_TRAFFIC_PER_ELEM = {"k_apply_adafac_cols": 27.58, "k_apply_adafac_tc": 27.44}
-# TF32 / fp16 multiply-adds the tensor-core apply kernels issue per parameter (products x N x K, M = the element)
-TC_ISSUED_FMA_PER_PARAM = {"3xtf32": (9 + 12 + 1) * 32 * 8}   # 22 products of N = 32, K = 8 per element row
+# fp16 multiply-adds the tensor-core apply kernels issue per parameter (products x N x K, M = the element)
+TC_ISSUED_FMA_PER_PARAM = {"3xtf32": 14 * 32 * 16}   # 14 products of N = 32, K = 16 per element row
 
 
 def parse(argv=None):
@@ -69,7 +69,7 @@ def parse(argv=None):
                          "into TF32 high and low parts), or as fp32 torch.matmul (the reference's arithmetic; a library call)")
     ap.add_argument("--mlp-precision", default="3xtf32", choices=["fp32", "3xtf32"],
                     help="adafaclo / elo: the network's hidden layers as scalar fp32 FMAs, or as tensor-core products of "
-                         "operands split into two TF32 parts (fp32-faithful: hi x hi + hi x lo + lo x hi)")
+                         "operands split into two parts (fp32-faithful: hi x hi + hi x lo + lo x hi)")
     ap.add_argument("--blocks", type=int, default=8, help="N>1: stages whose parameter all-gathers overlap the next stage")
     ap.add_argument("--exchange", default="auto", choices=["auto", "fused", "copy", "staged"],
                     help="N>1: how updated parameters reach the other ranks (fused: peer stores from the apply kernels; "
@@ -544,7 +544,7 @@ def measure(args, dev, world, rank, local, headline):
             per_param = TC_ISSUED_FMA_PER_PARAM[args.mlp_precision]
             issued = per_launch_elems * per_param * 2 / (phase_ms[dominant] * 1e-3)
             roofline["tensor"] = {"network_fma_per_param": 1600, "issued_fma_per_param": per_param,
-                                  "operands": "tf32", "products_per_128_params": 22,
+                                  "operands": "fp16 planes", "products_per_128_params": 14,
                                   "issued_tflops": issued / 1e12,
                                   "network_fp32_equiv_tflops": per_launch_elems * 3200 / (phase_ms[dominant] * 1e-3) / 1e12}
         elif args.optimizer in ("adafaclo", "elo") and dominant in ("k_apply", "k_apply_adafac_cols") and clocks and clocks.get("sm_mhz"):

@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define PYLO_B200_ABI_VERSION 17
+#define PYLO_B200_ABI_VERSION 18
 
 /* optimizer families (which feature set / network geometry a launch uses) */
 #define PYLO_FAM_ADAFAC 0 /* AdafacLO_CUDA, ELO_CUDA: 28+11 features, 39-32-32-2 */
@@ -50,7 +50,7 @@ extern "C" {
 #define PYLO_STAT_STRIDE 40  /* floats per tile partial / per tensor sums: 30 feature slots + 8 VeLO statistics */
 #define PYLO_TILE_ELEMS 16384 /* elements per element-wise tile (at most) */
 #define PYLO_A_COLS 1024      /* columns per row/column-sum tile */
-#define PYLO_WFOLD_STRIDE 2432 /* floats reserved per tensor for the folded network */
+#define PYLO_WFOLD_STRIDE 4800 /* floats reserved per tensor for the folded network and the tensor cores' operands */
 #define PYLO_SMALL_FLOATS 52224 /* shared memory of pylo_b200_small_front, in floats */
 #define PYLO_MAX_PEERS 7       /* other GPUs of one box */
 
@@ -144,8 +144,8 @@ typedef struct pylo_step_params {
   float eps_feat;         /* inside rsqrt(v + eps): 1e-6 AdafacLO/ELO/VeLO, 1e-8 CELO2 */
   float eps_norm;         /* inside rsqrt(S/n + eps): 1e-5 AdafacLO/ELO/VeLO, 1e-9 CELO2 */
   float clip_val;         /* element-wise clamp of the gradient; +inf for none */
-  int32_t no_tables;      /* prep_apply: 0 = make the per-row (desc.h_a) and per-column (desc.h_b) first-layer tables,
-                             1 = neither, 2 = the per-row table only (what the tensor-core apply kernel reads) */
+  int32_t no_tables;      /* prep_apply: 0 = make the per-row (desc.h_a) and per-column (desc.h_b) first-layer tables, and for ADAFAC
+                             what apply_adafac_tc reads; 1 = neither; 2 = only what apply_adafac_tc reads (ADAFAC); 3 = the tables only */
   const float* gnorm_sq;  /* device scalar: sum of squares of all gradients, or NULL */
   int32_t sum_tiles;      /* prep_apply: 1 = add the tile partials up itself (finalize_moments was not called) */
   int32_t bulk_copies;    /* state_moments: 1 = FAST2D tiles come through a ring of bulk copies, for large models that consist
@@ -285,10 +285,10 @@ int pylo_b200_apply_adafac_cols(const pylo_tensor_desc* descs, const pylo_atile*
                                 const pylo_step_params* prm, void* stream);
 
 /* Phase C for the tensors of the ADAFAC family on the tensor cores (no reference counterpart: the
- * reference evaluates the network with scalar FMAs, lo_kernel_apply learned_optimizer.cu:236-284).  Same inputs
- * and outputs as pylo_b200_apply_adafac_cols, except that of the two first-layer tables it reads only desc.h_a
- * (run pylo_b200_prep_apply with no_tables = 2 or 0).  The two hidden layers run as tcgen05 TF32 products with
- * every operand split into a high and a low TF32 part (hi x hi + hi x lo + lo x hi), which keeps a 32-term dot
+ * reference evaluates the network with scalar FMAs, lo_kernel_apply learned_optimizer.cu:236-284).  Same outputs
+ * as pylo_b200_apply_adafac_cols; it reads no first-layer tables, but the operands that pylo_b200_prep_apply makes
+ * with no_tables = 2 or 0.  The two hidden layers run as tcgen05 products of
+ * operands split into a high and a low fp16 plane of a common power-of-two scale (hi x hi + hi x lo + lo x hi), which keeps a 32-term dot
  * product within ~3e-7 of the sum of its terms' magnitudes; non-finite features give NaN where the scalar path may
  * give an infinity.  ttiles: strip = row-strip index, cb = block of 128 columns, pad_ = rows per work item (one
  * warpgroup of a CTA takes a whole item).  Units that are not FAST2D: pad_ = 0x10000 | tiles per work item, strip = item

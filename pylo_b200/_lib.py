@@ -16,8 +16,8 @@ SUMS_STRIDE = 48
 TILE_ELEMS = 16384
 A_COLS = 1024
 PREP_TABLE = 2048  # table entries (rows x hidden units) per item of pylo_b200_prep_apply
-WFOLD_STRIDE = 2432
-ABI_VERSION = 17
+WFOLD_STRIDE = 4800
+ABI_VERSION = 18
 
 FAM_ADAFAC, FAM_CELO2, FAM_VELO = 0, 1, 2
 MODE_FAST2D, MODE_GENERIC, MODE_VEC1D = 0, 1, 2

@@ -1,6 +1,7 @@
 // Shared device helpers for the pylo_b200 kernels (sm_100a).
 #pragma once
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
@@ -57,7 +58,25 @@ struct Fold {
   static constexpr int SN = W3P + 2 * F::H;       // [NF]: the features' normalisers
   static constexpr int SIZE = SN;                 // of what a kernel with the folded network needs
 };
-static_assert(Fold<PYLO_FAM_ADAFAC>::SN + Fam<PYLO_FAM_ADAFAC>::NF <= PYLO_WFOLD_STRIDE, "wfold too small");
+
+// What the tensor-core sweep reads of a unit, behind the folded network in desc.wfold: the operands B of its products as they lie
+// in shared memory (fp16 planes in the K-major no-swizzle layout: 8-row x 16-byte core matrices), then the features' scales.
+struct __align__(128) TcImage {
+  uint16_t b1[64 * 32];     // first layer, rows 0..31 the high planes, 32..63 the low planes; K = 32 slots (see tc_slot_feature)
+  uint16_t b2[64 * 32];     // second layer
+  uint16_t bias1[32 * 16];  // K = 16: column 0 the bias's high plane, column 1 what that leaves, times 2^11
+  uint16_t bias2[32 * 16];
+  float sn[32];             // [slot] normaliser times the features' power of two; [28] the scale of the second layer's sums
+};
+constexpr int TC_IMAGE = (Fold<PYLO_FAM_ADAFAC>::SN + Fam<PYLO_FAM_ADAFAC>::NF + 31) / 32 * 32;   // floats
+static_assert(TC_IMAGE + (int)sizeof(TcImage) / 4 <= PYLO_WFOLD_STRIDE, "wfold too small");
+// Which feature the first layer's operand A holds in slot k < 28: 0..12 and 25..27, then the six of one vector and the six of the
+// other ("r" first, or "c" first where swap is set)
+__host__ __device__ constexpr int tc_slot_feature(int k, bool swap) {
+  using F = Fam<PYLO_FAM_ADAFAC>;
+  return k < 13 ? k : k < 16 ? k + 12 : k < 19 ? (swap ? F::C : F::R) + k - 16 : k < 22 ? (swap ? F::RC : F::RR) + k - 19
+         : k < 25 ? (swap ? F::R : F::C) + k - 22 : (swap ? F::RR : F::RC) + k - 25;
+}
 
 // compile-time loop: guarantees static register indexing however large the unrolled body gets
 template <int I, int N, class Fn>

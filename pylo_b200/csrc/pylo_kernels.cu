@@ -919,6 +919,135 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
   }
 }
 
+// What the tensor-core sweep reads of a unit (TcImage): the network as operands B, the features' normalisers as scales of operand A.
+// One CTA per unit; latency-bound like the kernel above.
+//
+// Operands are two fp16 planes, so every operand gets a power of two that keeps it inside fp16's range whatever the gradients are.
+// A feature over its root mean square is at most sqrt(n) (all of the tensor's sum of squares in one element), so 2^q sqrt(n) <= 2^15;
+// a first-layer sum is at most its weights' magnitudes times sqrt(n), plus the bias, so 2^e1 times that is <= 2^15; and weights are
+// taken as large as they go, up to 2^a = 2^(e1 + TC_SHIFT - q): the shift between is undone by the tensor core, which scales the
+// sums by 2^-TC_SHIFT as it adds the bias.  A plane's last bit is 2^-25 of the scaled unit: of a feature 2^-(25 + q) of its root mean square
+// (q = 3 at 16 M elements), of a weight 2^-(25 + a), a = 7 to 10.
+#define TC_SHIFT 10
+__constant__ float TIME_SCALES[11] = {1.f, 3.f, 10.f, 30.f, 100.f, 300.f, 1000.f, 3000.f, 10000.f, 30000.f, 100000.f};
+__device__ __forceinline__ int tc_room(float x) {   // the largest e (up to 60) for which x 2^e is known to be below 2^15
+  return x > 0.f ? max(-60, min(60, 141 - (int)((__float_as_uint(x) >> 23) & 255))) : 60;
+}
+__device__ __forceinline__ float tc_pow2(int e) { return __uint_as_float((uint32_t)(127 + max(-126, min(127, e))) << 23); }
+__device__ __forceinline__ uint32_t tc_plane(float x, float scale, float& rest) {   // fp16 of x; rest: what it leaves, scaled
+  const __half h = __float2half_rn(x);
+  rest = (x - __half2float(h)) * scale;
+  return __half_as_ushort(h);
+}
+__global__ void __launch_bounds__(NT) k_prep_tc(const pylo_tensor_desc* __restrict__ descs, const pylo_atile* __restrict__ items,
+                                                const pylo_step_params prm) {
+  pdl_begin();
+  using F = Fam<PYLO_FAM_ADAFAC>;
+  using L = Fold<PYLO_FAM_ADAFAC>;
+  constexpr int H = F::H, NF = F::NF, NIN = F::NIN;
+  constexpr int o_b1 = NIN * H, o_w2 = o_b1 + H, o_b2 = o_w2 + H * H, o_w3 = o_b2 + H, o_b3 = o_w3 + 2 * H, o_end = o_b3 + 2;
+  __shared__ float s_net[o_end + H];            // the second layer's rows are H + 1 apart, so that lanes on different rows do not collide
+  __shared__ float s_scale[NF], s_b1[H], s_pow[6];
+  __shared__ float s_part[4][NT / 32][32];
+  __shared__ double s_d[6][PYLO_STAT_STRIDE];
+  const pylo_atile it = items[blockIdx.x];
+  if (it.strip) return;   // the whole CTA
+  const pylo_tensor_desc& d = descs[it.tensor];
+  const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5;
+  auto at = [](int e) { return e < o_w2 ? e : e < o_b2 ? e + (e - o_w2) / H : e + H; };
+  for (int e = tid; e < o_end; e += NT)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(s_net + at(e))), "l"(d.w + e) : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  const float n = (float)d.n;
+  if (prm.sum_tiles) {
+    const double tot = unit_sum<6>(d, s_d);
+    if (tid < NF) s_scale[tid] = rsqrtf((float)tot / n + prm.eps_norm);
+    if (tid < PYLO_STAT_STRIDE) store_unit_sum(d, tot);
+  } else if (tid < NF) {
+    s_scale[tid] = rsqrtf(d.sums[tid] / n + prm.eps_norm);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  {  // a hidden unit per lane, its inputs dealt to the warps
+    const float step = d.step + prm.step_delta;
+    float sum = 0.f, most = 0.f, most2 = 0.f, time = 0.f;
+    for (int k = part; k < NF; k += NT / 32) {
+      const float a = fabsf(s_net[lane * NIN + k]);
+      sum += a;
+      most = fmaxf(most, a);
+    }
+    for (int t = part; t < 11; t += NT / 32) time = fmaf(s_net[lane * NIN + NF + t], tanhf(step / TIME_SCALES[t] - 1.0f), time);
+    for (int k = part; k < H; k += NT / 32) most2 = fmaxf(most2, fabsf(s_net[o_w2 + lane * (H + 1) + k]));
+    s_part[0][part][lane] = sum; s_part[1][part][lane] = most; s_part[2][part][lane] = most2; s_part[3][part][lane] = time;
+  }
+  __syncthreads();
+  if (part == 0) {
+    float sum = 0.f, most = 0.f, most2 = 0.f, b1 = s_net[o_b1 + lane];
+    for (int q = 0; q < NT / 32; ++q) {
+      sum += s_part[0][q][lane];
+      most = fmaxf(most, s_part[1][q][lane]);
+      most2 = fmaxf(most2, s_part[2][q][lane]);
+      b1 += s_part[3][q][lane];
+    }
+    s_b1[lane] = b1;
+    const float spread = sqrtf(n) * 1.001f;
+    float bound = fmaf(sum, spread, fabsf(b1)), b2 = fabsf(s_net[at(o_b2 + lane)]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      bound = fmaxf(bound, __shfl_xor_sync(0xffffffffu, bound, o));
+      most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+      most2 = fmaxf(most2, __shfl_xor_sync(0xffffffffu, most2, o));
+      b2 = fmaxf(b2, __shfl_xor_sync(0xffffffffu, b2, o));
+    }
+    const int q = min(6, tc_room(spread));
+    const int a = min(min(6, tc_room(bound)) + TC_SHIFT - q, tc_room(most)), e1 = a + q - TC_SHIFT;
+    const int a2 = min(tc_room(most2) - 1, tc_room(b2) + TC_SHIFT - e1), e2 = e1 + a2 - TC_SHIFT;
+    if (lane == 0) {
+      s_pow[0] = tc_pow2(q); s_pow[1] = tc_pow2(a); s_pow[2] = tc_pow2(e1); s_pow[3] = tc_pow2(a2); s_pow[4] = tc_pow2(e2); s_pow[5] = tc_pow2(-e2);
+    }
+  }
+  __syncthreads();
+  TcImage& o = *reinterpret_cast<TcImage*>(d.wfold + TC_IMAGE);
+  const bool swap = d.mode == PYLO_MODE_FAST2D && d.r_is_a;   // FAST2D: the column vector's features come first
+  {  // both layers: a thread makes eight weights of one hidden unit, 16 bytes of each plane
+    const int layer = tid >> 7, kc = part & 3;
+    const float scale = s_pow[layer ? 3 : 1];
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      uint32_t h[2], l[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int k = kc * 8 + i + u;
+        const float x = layer ? s_net[o_w2 + lane * (H + 1) + k] : k < NF ? s_net[lane * NIN + tc_slot_feature(k, swap)] : 0.f;
+        float rest, none;
+        h[u] = tc_plane(x * scale, 1.f, rest);
+        l[u] = tc_plane(rest, 0.f, none);
+      }
+      hi[i / 2] = h[0] | h[1] << 16;
+      lo[i / 2] = l[0] | l[1] << 16;
+    }
+    char* b = reinterpret_cast<char*>(layer ? o.b2 : o.b1) + kc * 1024 + (lane >> 3) * 128 + (lane & 7) * 16;
+    *reinterpret_cast<uint4*>(b) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(b + 512) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+  if (part < 4) {
+    const int layer = part >> 1, kc = part & 1;
+    float rest, none;
+    uint32_t word = tc_plane(layer ? s_net[at(o_b2 + lane)] * s_pow[4] : s_b1[lane] * s_pow[2], 2048.f, rest);
+    word |= tc_plane(rest, 0.f, none) << 16;
+    char* b = reinterpret_cast<char*>(layer ? o.bias2 : o.bias1) + kc * 512 + (lane >> 3) * 128 + (lane & 7) * 16;
+    *reinterpret_cast<uint4*>(b) = make_uint4(kc ? 0u : word, 0u, 0u, 0u);
+  } else if (part == 4) {
+    o.sn[lane] = lane < NF ? s_scale[tc_slot_feature(lane, swap)] * s_pow[0] : lane == NF ? s_pow[5] : 0.f;
+    if (lane < 2) d.wfold[L::B3 + lane] = s_net[at(o_b3 + lane)];
+    if (lane == 0) d.wfold[L::SC + 1] = d.lr_mult ? d.lr * d.lr_mult[0] : d.lr;
+  } else if (part < 7) {   // pair-major copy of the output layer
+    const int e = lane + 32 * (part - 5), k = 2 * (e / 4) + (e & 1), q = (e % 4) >> 1;
+    d.wfold[L::W3P + e] = s_net[at(o_w3 + q * H + k)];
+  }
+}
+
 // ================================================================================================
 // Phase C: features -> network -> parameter / raw step
 // ================================================================================================
@@ -2696,7 +2825,10 @@ int pylo_b200_prep_apply(const pylo_tensor_desc* descs, const pylo_atile* items,
   if (n_items == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: launch(k_prep_apply<PYLO_FAM_ADAFAC>, n_items, NT, 0, s, descs, items, *prm); break;
+    case PYLO_FAM_ADAFAC:
+      if (prm->no_tables != 2) launch(k_prep_apply<PYLO_FAM_ADAFAC>, n_items, NT, 0, s, descs, items, *prm);
+      if (prm->no_tables == 2 || prm->no_tables == 0) launch(k_prep_tc, n_items, NT, 0, s, descs, items, *prm);
+      break;
     case PYLO_FAM_CELO2: launch(k_prep_apply<PYLO_FAM_CELO2>, n_items, NT, 0, s, descs, items, *prm); break;
     case PYLO_FAM_VELO: launch(k_prep_apply<PYLO_FAM_VELO>, n_items, NT, 0, s, descs, items, *prm); break;
     default: return -2;
@@ -3081,7 +3213,7 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
   if (!(phases & PYLO_STEP_BACK)) return 0;
   pylo_step_params q = *prm;
   q.sum_tiles = p->sum_tiles && q.family != PYLO_FAM_VELO;
-  q.no_tables = p->tensor_cores ? 2 : 0;   // the tensor-core kernel reads the per-row table only
+  q.no_tables = p->tensor_cores ? 2 : 3;
   if (phases & PYLO_STEP_PREP)
     if ((rc = pylo_b200_prep_apply(p->desc, p->pitems, p->n_pitems, &q, stream))) return rc;
   const bool main = phases & PYLO_STEP_APPLY, rest = phases & PYLO_STEP_APPLY_REST;

@@ -36,6 +36,16 @@
 // tensor memory is freed.
 #pragma once
 
+// instruction descriptor: fp32 accumulate, TF32 x TF32, both operands K-major, M = 128
+__host__ __device__ constexpr uint32_t tc_idesc(uint32_t n) { return (1u << 4) | (2u << 7) | (2u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
+// D[128 x N] (+)= A[128 x 8] * B[N x 8]^T, both through shared-memory descriptors
+__device__ __forceinline__ void tc_mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
 #define NS_BM 128
 #define NS_BN 256
 #define NS_BK 32

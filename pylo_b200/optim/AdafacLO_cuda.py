@@ -16,7 +16,7 @@ coordinates.
 
 ``mlp_precision`` (an addition) selects how the network's two hidden layers are
 evaluated on factored 2-D tensors: ``"3xtf32"`` (default) as tcgen05 tensor-core
-products with every operand split into a high and a low TF32 part, three
+products with every operand split into a high and a low fp16 plane, three
 products per layer, which reproduces the fp32 result to ~3e-7 of a dot
 product's magnitude; ``"fp32"`` as scalar fp32 FMAs on the CUDA cores, the
 arithmetic of the reference kernel.  Both meet the same parity bounds.

@@ -363,7 +363,7 @@ class LoPlan:
         """``model``: (shape, factored axes, rcm_axis) of all tensors of the model, in any order, of which ``tensors`` are a rank's
         share; their step is then the one that a plan over the whole model makes, to the last bit."""
         self.family = family
-        # whether the AdafacLO family's FAST2D tensors take the tensor-core apply kernel (TF32 operands)
+        # whether the AdafacLO family's FAST2D tensors take the tensor-core apply kernel
         self.tensor_cores = bool(tensor_cores) and family == L.FAM_ADAFAC
         self.tensors = tensors
         self.device = torch.device(device)
@@ -512,9 +512,8 @@ class LoPlan:
             if not tdesc["h_a"][i]:
                 continue
             X, Y = int(tdesc["X"][i]), int(tdesc["Y"][i])
-            # the tensor-core kernel reads the per-row table only, the CUDA-core kernels both
-            parts = (X + per - 1) // per + (0 if self.tensor_cores else (Y + per - 1) // per)
-            pitems.append(atile_grid(unit_of[i], parts, 1)[1:])
+            if not self.tensor_cores:   # the tensor-core kernel reads no tables
+                pitems.append(atile_grid(unit_of[i], (X + per - 1) // per + (Y + per - 1) // per, 1)[1:])
             (fast if tdesc["mode"][i] == L.MODE_FAST2D else ragged).append((unit_of[i], X, Y))
         slow_units = [u for u in range(U) if not tdesc["h_a"][unit_owner[u][0]]]
         self.ctiles = FixedTable(apply_items(family, self.tensor_cores, fast, [(u, sizes[u]) for u in slow_units]))
