@@ -45,6 +45,8 @@ extern "C" {
 /* how a tensor is traversed */
 #define PYLO_MODE_FAST2D 0  /* contiguous [X,Y], Y % 4 == 0, 16-byte aligned: float4 path */
 #define PYLO_MODE_GENERIC 1 /* any contiguous [O,X,M,Y,I] view, scalar loads */
+#define PYLO_MODE_KERNEL 3  /* contiguous [X,Y,I] with I <= 32 positions (convolution weights; O = M = 1), Y * I % 4 == 0, 16-byte aligned: a
+                               matrix of Y * I columns whose "a" vectors have an entry per row and position; for pylo_b200_apply as GENERIC */
 #define PYLO_MODE_VEC1D 2   /* fewer than two dims: accumulators are full size ("vector_like") */
 
 #define PYLO_STAT_STRIDE 40  /* floats per tile partial / per tensor sums: 30 feature slots + 8 VeLO statistics */
@@ -74,10 +76,10 @@ typedef struct pylo_tensor_desc {
   float* fac_b;   /* factored accumulator state, [3][Lb] (VEC1D: the column one or NULL) */
   float* f_a;     /* workspace [3][La]: rsqrt factor in "a" orientation */
   float* f_b;     /* workspace [3][Lb] */
-  float* fx;      /* workspace [La][4]: f_a interleaved per index (FAST2D, and GENERIC matrices with tables, see workspace_layout; else NULL) */
+  float* fx;      /* workspace [La][4]: f_a interleaved per index (FAST2D, KERNEL, and GENERIC matrices with tables, see workspace_layout; else NULL) */
   float* sum_a;   /* workspace [La]: sum over Y of g'^2 + 1e-30 */
   float* sum_b;   /* workspace [Lb]: sum over X */
-  float* part_a;  /* workspace [X][n_cb]  row-sum partials (tensors in atiles; else NULL) */
+  float* part_a;  /* workspace [X][n_cb]  row-sum partials (tensors in atiles; else NULL); KERNEL: [La][2 n_cb] */
   float* part_b;  /* workspace [n_strips][Lb] column-sum partials */
   float* h_a;     /* workspace [La][H] (ADAFAC) or [La][H][2] (CELO2, VELO): first-layer term of the "a" features (+ bias) */
   float* h_b;     /* workspace [H][Lb]: first-layer term of the "b" features */
@@ -101,7 +103,7 @@ typedef struct pylo_tensor_desc {
   int32_t mode;
   int32_t r_is_a;
   int32_t rcm_pre, rcm_A, rcm_post; /* row_col_mean: the row accumulator viewed [pre][A][post], mean over A */
-  int32_t rb, n_strips, n_cb;       /* phase-A tiling: rows per strip, strips, column blocks (FAST2D) */
+  int32_t rb, n_strips, n_cb;       /* phase-A tiling: rows per strip, strips, column blocks (tensors in atiles) */
   int32_t tile0, n_tiles;           /* this tensor's range in the element-wise tile list */
   int32_t vec_elementwise;          /* 1: this unit is a slice of a tensor (its normalisers cover the slice only),
                                        so the vector-only features are accumulated per element, not in closed form */
@@ -172,7 +174,7 @@ int pylo_b200_sizeof_params(void);
  * pylo_b200_workspace_layout fills, for one tensor of the given family, traversal mode and geometry, the size
  * in floats of every workspace sub-buffer that pylo_tensor_desc points at (0 where the mode does not use it),
  * and the phase-A tiling (rb, n_strips, n_cb) and the number of element-wise tiles that go into the descriptor.  A GENERIC tensor
- * that is a plain matrix (O = M = I = 1) may be given with its X and Y: its sums then go into the items of FAST2D tensors (atiles),
+ * that is a plain matrix (O = M = I = 1) may be given with its X and Y (a KERNEL one is, with its X and its Y * I columns): its sums then go into the items of FAST2D tensors (atiles),
  * and for CELO2 and VELO it has the tables of pylo_b200_apply_packed's ragged items.
  * A unit of element-wise work that is a slice of a tensor (vec_elementwise = 1) owns only the last three
  * sub-buffers (sums, wfold, tile_part), sized with n = the slice's elements, plus a zero-filled `closed`; the
@@ -226,17 +228,18 @@ int pylo_b200_grad_sumsq_static(const pylo_gvec* items, const pylo_tile* tiles, 
 
 /* Phase A: row and column sums of g'^2 + 1e-30 (the reductions inside
  * grad_sqr.mean(dim=dr / dc), AdafacLO_cuda.py:333-340, CELO2_cuda.py:218-224, velo_cuda.py:531-541).
- * atiles cover the FAST2D tensors, and GENERIC matrices laid out like them (the first n_ragged; strip x 1024-column block each; they leave per-strip column partials, which
- * pylo_b200_factor_update adds up).  gitems cover the GENERIC tensors: items with pad_ = 1 take 256 of the Lb columns
+ * atiles cover the FAST2D tensors, GENERIC matrices laid out like them (the first n_ragged) and KERNEL tensors (the next n_kernel):
+ * a strip x 1024-column block each; they leave per-strip column partials, which pylo_b200_factor_update adds up.  gitems cover the GENERIC tensors: items with pad_ = 1 take 256 of the Lb columns
  * (cb) over the rows of a strip (desc.rb of the X rows), items with pad_ = 0 take cb of the La / I
  * blocks that have I row sums each, from block strip * cb on. */
-int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles, int n_ragged,
+int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles, int n_ragged, int n_kernel,
                           const pylo_atile* gitems, int n_gitems, const pylo_step_params* prm, void* stream);
 
 /* Phase A2, one cluster of CTAs per tensor: the sums over strips and column blocks of phase A's partials, EMA of the factored accumulators, row_col_mean,
  * row/column rsqrt factors (AdafacLO_cuda.py:342-345, CELO2_cuda.py:229-231, velo_cuda.py:716-729)
- * and the closed-form feature moments of the twelve vector-only features. */
-int pylo_b200_factor_update(const pylo_tensor_desc* descs, int n_tensors, const pylo_step_params* prm,
+ * and the closed-form feature moments of the twelve vector-only features.  mats: DEVICE list of the n_tensors tensors to take (VEC1D ones
+ * have nothing to do, as long as their `closed` is zero), or NULL for the first n_tensors. */
+int pylo_b200_factor_update(const pylo_tensor_desc* descs, const int32_t* mats, int n_tensors, const pylo_step_params* prm,
                             void* stream);
 
 /* Phase B: momentum / second-moment EMA in place and per-tile sums of squares of
@@ -291,7 +294,7 @@ int pylo_b200_apply_adafac_cols(const pylo_tensor_desc* descs, const pylo_atile*
  * operands split into a high and a low fp16 plane of a common power-of-two scale (hi x hi + hi x lo + lo x hi), which keeps a 32-term dot
  * product within ~3e-7 of the sum of its terms' magnitudes; non-finite features give NaN where the scalar path may
  * give an infinity.  ttiles: strip = row-strip index, cb = block of 128 columns, pad_ = rows per work item (one
- * warpgroup of a CTA takes a whole item).  Units that are not FAST2D: pad_ = 0x10000 | tiles per work item, strip = item
+ * warpgroup of a CTA takes a whole item).  Units that are neither FAST2D nor KERNEL: pad_ = 0x10000 | tiles per work item, strip = item
  * index, cb = 0; an item is that many runs of 128 consecutive elements; generic != 0 says that the list may hold such
  * items.  status: device int; the kernel ORs 1 into it if a wait on the tensor
  * core ran out (the parameters it could not finish then keep their old values), and a launch that finds it
@@ -462,6 +465,7 @@ int pylo_b200_velo_loss_features(float* means, int32_t* iteration, float* runnin
 #define PYLO_STEP_APPLY_REST 64
 #define PYLO_STEP_FRONT (PYLO_STEP_SUMS | PYLO_STEP_FACTORS | PYLO_STEP_STATE | PYLO_STEP_MOMENTS)
 #define PYLO_STEP_BACK (PYLO_STEP_PREP | PYLO_STEP_APPLY | PYLO_STEP_APPLY_REST)
+#define PYLO_ROWCOL_ONE_LAUNCH 2368 /* items of rowcol_sums up to which the GENERIC tensors' items join their launch (KERNEL items: always) */
 #define PYLO_TC_ONE_LAUNCH 4736 /* items on FAST2D units below which one launch of apply_adafac_tc takes both kinds of items: \
                                   the variant that takes both is 2 % slower on FAST2D items (ViT-B/16 2700 / 2751 us per \
                                   step, two Llama-3-8B blocks 12640 / 12925), a launch more costs about 10 us (convolutions \
@@ -471,6 +475,7 @@ typedef struct pylo_step_plan {
   const pylo_atile *atiles, *gitems, *pitems, *ctiles;
   const pylo_tile *tiles, *tiles_slow;
   const pylo_atile* rtiles; /* CELO2, VELO: items of apply_packed on matrices with tables whose rows are not aligned */
+  const int32_t* mats;      /* the tensors that are not VEC1D */
   int *status, *host_status;
   int32_t n_tensors, n_units, n_atiles, n_gitems, n_pitems, n_ctiles, n_ctiles_gen, n_tiles, n_tiles_slow, tensor_cores;
   int32_t sum_tiles; /* 1: leave finalize_moments out and let prep_apply add up the tile partials, for units of up to
@@ -478,7 +483,8 @@ typedef struct pylo_step_plan {
   int32_t n_ragged, n_rtiles; /* of atiles, the first that are not on FAST2D tensors; of rtiles */
   int32_t small_cluster, small_slice, small_rows, small_cols; /* small_cluster > 0: SUMS, FACTORS and STATE, asked for together,
                         are one launch of pylo_b200_small_front */
-  int32_t pad_;
+  int32_t n_kernel; /* of atiles, those behind the first n_ragged that are on KERNEL tensors */
+  int32_t n_mats, pad_;
 } pylo_step_plan;
 int pylo_b200_step(const pylo_step_plan* plan, const pylo_step_params* prm, int phases, void* stream);
 /* Host only: adds 1 to n step counters (HOST pointers to doubles); first: the old value of the first, equal: whether all

@@ -20,7 +20,7 @@ WFOLD_STRIDE = 4800
 ABI_VERSION = 18
 
 FAM_ADAFAC, FAM_CELO2, FAM_VELO = 0, 1, 2
-MODE_FAST2D, MODE_GENERIC, MODE_VEC1D = 0, 1, 2
+MODE_FAST2D, MODE_GENERIC, MODE_VEC1D, MODE_KERNEL = 0, 1, 2, 3
 
 _PTR_FIELDS = [
     "g", "p", "m", "v", "fac_a", "fac_b", "f_a", "f_b", "fx", "sum_a", "sum_b", "part_a", "part_b",
@@ -99,10 +99,10 @@ class VeloLoss(C.Structure):
 class StepPlan(C.Structure):
     """pylo_step_plan: all tables of one optimizer's tensors."""
     _fields_ = [(name, C.c_void_p) for name in (
-        "tdesc", "desc", "atiles", "gitems", "pitems", "ctiles", "tiles", "tiles_slow", "rtiles", "status", "host_status")] + [
+        "tdesc", "desc", "atiles", "gitems", "pitems", "ctiles", "tiles", "tiles_slow", "rtiles", "mats", "status", "host_status")] + [
         (name, C.c_int32) for name in ("n_tensors", "n_units", "n_atiles", "n_gitems", "n_pitems", "n_ctiles", "n_ctiles_gen",
                                        "n_tiles", "n_tiles_slow", "tensor_cores", "sum_tiles", "n_ragged", "n_rtiles", "small_cluster", "small_slice",
-                                       "small_rows", "small_cols", "pad_")]
+                                       "small_rows", "small_cols", "n_kernel", "n_mats", "pad_")]
 
 
 class PyloLibError(RuntimeError):
@@ -128,8 +128,8 @@ def _load():
         "pylo_b200_workspace_bytes": [C.POINTER(WsLayout), i32, i32],
         "pylo_b200_grad_sumsq": [vp, vp, i32, vp, vp, vp],
         "pylo_b200_grad_sumsq_static": [vp, vp, i32, vp, vp],
-        "pylo_b200_rowcol_sums": [vp, vp, i32, i32, vp, i32, C.POINTER(StepParams), vp],
-        "pylo_b200_factor_update": [vp, i32, C.POINTER(StepParams), vp],
+        "pylo_b200_rowcol_sums": [vp, vp, i32, i32, i32, vp, i32, C.POINTER(StepParams), vp],
+        "pylo_b200_factor_update": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_state_moments": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_small_front": [vp, i32, i32, i32, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_finalize_moments": [vp, i32, vp],
@@ -173,6 +173,7 @@ TC_GEN_ITEM = 1 << 16  # tag bit of its items on tensors that are not FAST2D
 STEP_SUMS, STEP_FACTORS, STEP_STATE, STEP_MOMENTS, STEP_PREP, STEP_APPLY, STEP_APPLY_REST = (1 << k for k in range(7))
 STEP_FRONT = STEP_SUMS | STEP_FACTORS | STEP_STATE | STEP_MOMENTS
 STEP_BACK = STEP_PREP | STEP_APPLY | STEP_APPLY_REST
+ROWCOL_ONE_LAUNCH = 2368  # items of rowcol_sums up to which the GENERIC tensors' items join their launch
 TC_ONE_LAUNCH = 8 * TC_WORKERS  # FAST2D items below which one launch of the tensor-core kernel takes both kinds of items
 BULK_COPY_ELEMS = 1 << 26  # FAST2D elements from which the state sweep reads through a ring of bulk copies
 SMALL_SLICE, SMALL_FLOATS = 8192, 52224   # of pylo_b200_small_front: elements of a CTA's rows, floats of shared memory

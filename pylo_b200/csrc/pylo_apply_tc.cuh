@@ -8,7 +8,8 @@
 //     into tensor memory, where they are operand A (lane = element, column = two features);
 //   * the six features that depend only on the element's column join operand A from registers, where they stay for
 //     all rows of a work item; the six that depend only on its row come from shared memory, where a warpgroup makes
-//     them for up to 64 rows at a time.  First layer: K = 28 of 32;
+//     them for up to 64 rows at a time (of convolution weights, KERNEL, the row's features differ from one position to the
+//     next: 14 rows of 9 positions).  First layer: K = 28 of 32;
 //   * fp32 accuracy is kept by splitting every operand into two fp16 planes (11 + 11 significant bits) and running
 //     three products per layer and K step (hi x hi, hi x lo, lo x hi) into one accumulator of 32 columns.  The features
 //     are normalised before they are split: over its root mean square no feature exceeds sqrt(n), so that powers of two
@@ -20,7 +21,7 @@
 //     (K = 8), twice the operand stores, and the row's features through operand B: 8192 x 4096 elements 714 -> 678 us, step over ViT-B/16
 //     2760 -> 2378, two Llama blocks 12610 -> 11320; the movement's error against fp64 is half of what it was
 //     (4096 x 4096, normal gradients: 1.6e-7 -> 0.9e-7 rms);
-//   * tensors that are not FAST2D (ragged rows, more than two dims, vectors) are taken as 128 consecutive elements that
+//   * other tensors (ragged rows, vectors, odd convolutions) are taken as 128 consecutive elements that
 //     may lie in several rows (GEN items): their twelve vector features are made per element (the scalar kernel that took them before needed 752
 //     us for the 5 M parameters of a small convolutional network, FMA-bound);
 //   * relu, the split of the hidden activations (whose conversions to fp16 clamp at zero by themselves), the two output heads and
@@ -55,7 +56,8 @@
 #endif
 #define TC_COLS 128              // tensor columns per work item: one per lane of the accumulator tile
 #define TC_WG_TMEM 64            // tensor-memory columns per warpgroup: [0,16) operand A high planes, [16,32) low planes, [32,64) accumulator
-#define TC_ROWS 64               // tensor rows whose features and factors a warpgroup makes at once
+#define TC_ROWS 64               // FAST2D: tensor rows whose factors and features a warpgroup makes at once
+#define TC_RECORDS 128           // KERNEL: the same of rows and positions
 #define TC_GEN_ITEM (1 << 16)    // set in an item's tag: `strip` counts items of `rows` x 128 consecutive elements
 #define TC_SPIN_LIMIT (1 << 20)
 #ifndef TC_POLL_SLEEP_NS
@@ -182,7 +184,7 @@ __device__ __forceinline__ void tc_split2(uint64_t x, uint32_t& hi, uint32_t& lo
 // wait on one another.
 struct __align__(128) TcWgSmem {
   TcImage img;               // of the unit of the present item
-  float row[TC_ROWS][12];    // FAST2D, per tensor row: three factors, then its six features as three words of high and three of low planes
+  float row[TC_RECORDS][12]; // FAST2D, KERNEL, per tensor row (and position): three factors, then its six features as three words of high and three of low planes
   float w3[64 + 4];          // output layer, pair-major (Fold::W3P), then its two biases
   uint64_t bar;
 };
@@ -244,10 +246,11 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
     const pylo_atile ct = ttiles[t];
     const pylo_tensor_desc& d = descs[ct.tensor];
     const int rows_item = ct.pad_ & (TC_GEN_ITEM - 1);  // rows (tiles of 128 elements) per work item
-    // One item; GEN: the tensor is not FAST2D.  Two bodies, so that neither holds the other's registers.
-    auto item = [&](auto gen_tag) {
-    constexpr bool GEN = decltype(gen_tag)::value;
-    const int X = d.X, Y = d.Y;
+    // One item: on a FAST2D tensor, a KERNEL one, or (GEN) any other.  A body for each, so that none holds another's registers.
+    auto item = [&](auto mode_tag) {
+    constexpr bool GEN = decltype(mode_tag)::value == PYLO_MODE_GENERIC, KERNEL = decltype(mode_tag)::value == PYLO_MODE_KERNEL;
+    const int I = KERNEL ? d.I : 1;   // positions; a matrix of Y * I columns
+    const int X = d.X, Y = d.Y * I;
     const int64_t n = d.n;
     const int y = ct.cb * TC_COLS + col;
     const int x0 = ct.strip * rows_item;
@@ -330,18 +333,23 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
       if (colok) planes6(16, fc[0], fc[1], fc[2], chi, clo);
     TC_CLK(7)  // item set-up
 #pragma unroll 1
+    const float* rec = nullptr;   // KERNEL: of this row and this thread's position
+    int ready = 0;                // rows ahead whose factors and features are there
     for (int x = x0; x < x_end; ++x) {   // the same for the whole warpgroup
       const int i = x - x0;
-      if (!GEN && (i & (TC_ROWS - 1)) == 0) {   // the next rows' factors and features (the previous ones were read before a barrier)
-        if (col < TC_ROWS && x + col < x_end) {
-          const float4 f = ld4(d.fx + 4 * (int64_t)(x + col));
+      if (KERNEL ? ready == 0 : !GEN && (i & (TC_ROWS - 1)) == 0) {   // the next rows' factors and features (the previous ones were read before a barrier)
+        ready = min(KERNEL ? TC_RECORDS / I : TC_ROWS, x_end - x);
+        if (col < ready * I) {
+          const int64_t a = (int64_t)x * I + col, La = (int64_t)X * I;
+          const float4 f = ld4(d.fx + 4 * a);
           uint32_t hi[3], lo[3];
-          planes6(22, d.fac_a[x + col], d.fac_a[(int64_t)X + x + col], d.fac_a[2 * (int64_t)X + x + col], hi, lo);
+          planes6(22, d.fac_a[a], d.fac_a[La + a], d.fac_a[2 * La + a], hi, lo);
           float* q = sm.row[col];
           st4(q, make_float4(f.x, f.y, f.z, __uint_as_float(hi[0])));
           st4(q + 4, make_float4(__uint_as_float(hi[1]), __uint_as_float(hi[2]), __uint_as_float(lo[0]), __uint_as_float(lo[1])));
           q[8] = __uint_as_float(lo[2]);
         }
+        if (KERNEL) rec = sm.row[yc % I];
         wg_barrier(wg);
       }
       TC_CLK(8)  // loop overhead, rows' features
@@ -363,13 +371,14 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
 #pragma unroll
           for (int j = 0; j < 3; ++j) { hi[11 + j] = h[j]; lo[11 + j] = l[j]; }
         } else {
-          const float* q = sm.row[i & (TC_ROWS - 1)];
+          const float* q = KERNEL ? rec : sm.row[i & (TC_ROWS - 1)];
           const float4 r0 = ld4(q), r1 = ld4(q + 4);
           k0 = r0.x * fb0; k1 = r0.y * fb1; k2 = r0.z * fb2;
 #pragma unroll
           for (int j = 0; j < 3; ++j) { hi[8 + j] = chi[j]; lo[8 + j] = clo[j]; }
           hi[11] = __float_as_uint(r0.w); hi[12] = __float_as_uint(r1.x); hi[13] = __float_as_uint(r1.y);
           lo[11] = __float_as_uint(r1.z); lo[12] = __float_as_uint(r1.w); lo[13] = __float_as_uint(q[8]);
+          if (KERNEL) { rec += 12 * I; --ready; }
         }
         hi[14] = hi[15] = lo[14] = lo[15] = 0u;
         const uint64_t fe[8] = {pack2(g, cp), pack2(cm0, cm1), pack2(cm2, cv), pack2(cm0 * rs, cm1 * rs), pack2(cm2 * rs, rs),
@@ -492,10 +501,11 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
     }
     };
     if constexpr (GENERIC) {
-      if (ct.pad_ & TC_GEN_ITEM) item(std::true_type{});
-      else item(std::false_type{});
+      if (ct.pad_ & TC_GEN_ITEM) item(std::integral_constant<int, PYLO_MODE_GENERIC>{});
+      else if (d.mode == PYLO_MODE_KERNEL) item(std::integral_constant<int, PYLO_MODE_KERNEL>{});
+      else item(std::integral_constant<int, PYLO_MODE_FAST2D>{});
     } else {
-      item(std::false_type{});
+      item(std::integral_constant<int, PYLO_MODE_FAST2D>{});
     }
   }
   TC_CLK_FLUSH

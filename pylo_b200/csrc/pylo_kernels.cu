@@ -90,105 +90,6 @@ __global__ void __launch_bounds__(1024) k_sum_final(const float* __restrict__ sc
 // ================================================================================================
 // Phase A: row / column sums of g'^2 + 1e-30
 // ================================================================================================
-// Bound by HBM.  Of the CTA's eight warps, four pairs take every fourth row of the strip and the warps of a pair one half
-// (512 columns) of the block each, so that a lane keeps 16 column accumulators (not 32) and has room to request its next
-// row before it adds up the present one: the loads of the next row fly during the shuffles of this one's row sum.
-// 355 M elements (GPT-2-medium shapes): 417 us before (a warp per row, 32 accumulators, no row ahead).
-// Matrices whose rows are not aligned (GENERIC, with part_a) go the same way with single loads (not VEC), a piece's columns 32 apart.
-#define RC_GROUPS 4
-template <bool VEC>
-__global__ void __launch_bounds__(NT, VEC ? 4 : 3) k_rowcol_fast(const pylo_tensor_desc* __restrict__ descs,
-                                                       const pylo_atile* __restrict__ atiles, int n_atiles,
-                                                       const pylo_step_params prm) {
-  pdl_begin();
-  __shared__ float s_col[RC_GROUPS][PYLO_A_COLS];
-  __shared__ float s_row[PYLO_A_ROWS_MAX][2];
-  const int lane = threadIdx.x & 31, half = (threadIdx.x >> 5) & 1, grp = threadIdx.x >> 6;
-  for (int t = blockIdx.x; t < n_atiles; t += gridDim.x) {
-    const pylo_atile at = atiles[t];
-    const pylo_tensor_desc& d = descs[at.tensor];
-    const int X = d.X, Y = d.Y, rb = d.rb;
-    const int row0 = at.strip * rb;
-    const int rows = min(rb, X - row0);
-    const int col0 = at.cb * PYLO_A_COLS;
-    const float gs = grad_scale_of(d, prm);
-    const bool plain = plain_grad(gs, prm);
-    const int c0 = half * 512 + (VEC ? lane * 4 : lane);
-    const float* base = d.g + (int64_t)row0 * Y + col0 + c0;
-    const int left = Y - col0 - c0;   // columns of this lane's pieces that exist: VEC: piece j is there if j * 128 < left, else column k if k * 32 is
-    float colacc[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) colacc[j] = 0.f;
-    float4 cur[4], nxt[4];
-    auto load = [&](int r, float4 (&q)[4]) {
-      const float* p = base + (int64_t)r * Y;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if constexpr (VEC) {
-          if (j * 128 < left) q[j] = ldg4(p + j * 128);
-        } else {
-          if (j * 128 < left) q[j].x = __ldg(p + j * 128);
-          if (j * 128 + 32 < left) q[j].y = __ldg(p + j * 128 + 32);
-          if (j * 128 + 64 < left) q[j].z = __ldg(p + j * 128 + 64);
-          if (j * 128 + 96 < left) q[j].w = __ldg(p + j * 128 + 96);
-        }
-      }
-    };
-    if (grp < rows) load(grp, cur);
-    for (int r = grp; r < rows; r += RC_GROUPS) {
-      if (r + RC_GROUPS < rows) load(r + RC_GROUPS, nxt);
-      float rowsum = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j * 128 < left) {
-          const float e[4] = {cur[j].x, cur[j].y, cur[j].z, cur[j].w};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (!VEC && j * 128 + u * 32 >= left) continue;
-            const float g = plain ? e[u] : xform_grad(e[u], gs, prm.clip_val, prm.nan_to_num);
-            const float q = g * g + 1e-30f;
-            colacc[j * 4 + u] += q;
-            rowsum += q;
-          }
-        }
-      }
-      rowsum = warp_sum(rowsum);
-      if (lane == 0) s_row[r][half] = rowsum;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) cur[j] = nxt[j];
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if constexpr (VEC) st4(&s_col[grp][c0 + j * 128], make_float4(colacc[j * 4], colacc[j * 4 + 1], colacc[j * 4 + 2], colacc[j * 4 + 3]));
-      else
-#pragma unroll
-        for (int u = 0; u < 4; ++u) s_col[grp][c0 + j * 128 + u * 32] = colacc[j * 4 + u];
-    }
-    __syncthreads();
-    if constexpr (VEC) {
-      const int c = threadIdx.x * 4;
-      if (col0 + c < Y) {
-        float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int w = 0; w < RC_GROUPS; ++w) {
-          const float4 q = ld4(&s_col[w][c]);
-          tot.x += q.x; tot.y += q.y; tot.z += q.z; tot.w += q.w;
-        }
-        st4(d.part_b + (int64_t)at.strip * Y + col0 + c, tot);
-      }
-    } else {
-      for (int c = threadIdx.x; c < PYLO_A_COLS && col0 + c < Y; c += NT) {
-        float tot = 0.f;
-#pragma unroll
-        for (int w = 0; w < RC_GROUPS; ++w) tot += s_col[w][c];
-        d.part_b[(int64_t)at.strip * Y + col0 + c] = tot;
-      }
-    }
-    if (threadIdx.x < rows) d.part_a[(int64_t)(row0 + threadIdx.x) * d.n_cb + at.cb] = s_row[threadIdx.x][0] + s_row[threadIdx.x][1];
-    __syncthreads();
-  }
-}
-
 // GENERIC tensors, seen as a matrix of O*X rows of C = M*Y*I (see GenPos).  Two kinds of work item, told apart by pad_:
 //   1: column sums: 256 of the Lb columns, one per thread, over the rows of a strip (partials as on the float4 path);
 //   0: row sums: a row is M blocks of Y*I consecutive elements, every block has I sums over y.  A group of lanes takes a
@@ -196,12 +97,8 @@ __global__ void __launch_bounds__(NT, VEC ? 4 : 3) k_rowcol_fast(const pylo_tens
 // Both read whole lines.  (One warp per output with lanes along the reduced axis, as it was, read one element per line
 // wherever that axis is not the last: 211 us for 5 M parameters of 3x3 convolutions, 302 us for a ViT patch embedding.)
 #define GA_LONG 1024      // from this block length on (I <= 32) a CTA, not a warp, takes a block: the loads of a block are a serial chain
-__global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* __restrict__ descs,
-                                                       const pylo_atile* __restrict__ items,
-                                                       const pylo_step_params prm) {
-  pdl_begin();
-  __shared__ float s_red[NT];
-  const pylo_atile it = items[blockIdx.x];
+__device__ __forceinline__ void rowcol_generic(const pylo_tensor_desc* __restrict__ descs, const pylo_atile it, const pylo_step_params& prm,
+                                               float* s_red) {   // s_red: NT floats
   const pylo_tensor_desc& d = descs[it.tensor];
   const float gs = grad_scale_of(d, prm);
   const bool plain = plain_grad(gs, prm);
@@ -284,6 +181,140 @@ __global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* _
   }
 }
 
+// Bound by HBM.  Of the CTA's eight warps, four pairs take every fourth row of the strip and the warps of a pair one half
+// (512 columns) of the block each, so that a lane keeps 16 column accumulators (not 32) and has room to request its next
+// row before it adds up the present one: the loads of the next row fly during the shuffles of this one's row sum.
+// 355 M elements (GPT-2-medium shapes): 417 us before (a warp per row, 32 accumulators, no row ahead).
+// Matrices whose rows are not aligned (GENERIC, with part_a) go the same way with single loads (not VEC), a piece's columns 32 apart.
+#define RC_GROUPS 4
+// MIX: the list may hold convolution weights, and the first n_gitems CTAs take the GENERIC tensors' items, one each: a launch of their own
+// took 13 us for the one 64 x 3 x 7 x 7 tensor of a convolutional network, a chain of latencies.  Both cost registers, so this
+// variant has three CTAs per SM and large models do without it (with it, spilling, 355 M elements 277 -> 340 us).
+template <bool VEC, bool MIX>
+__global__ void __launch_bounds__(NT, VEC && !MIX ? 4 : 3) k_rowcol_fast(const pylo_tensor_desc* __restrict__ descs,
+                                                       const pylo_atile* __restrict__ atiles, int n_atiles,
+                                                       const pylo_atile* __restrict__ gitems, int n_gitems,
+                                                       const pylo_step_params prm) {
+  pdl_begin();
+  __shared__ float s_col[RC_GROUPS][PYLO_A_COLS];
+  if (MIX && (int)blockIdx.x < n_gitems) {
+    rowcol_generic(descs, gitems[blockIdx.x], prm, s_col[0]);
+    return;
+  }
+  const int cta = MIX ? blockIdx.x - n_gitems : blockIdx.x, ctas = MIX ? gridDim.x - n_gitems : gridDim.x;
+  __shared__ float s_row[PYLO_A_ROWS_MAX][2];
+  const int lane = threadIdx.x & 31, half = (threadIdx.x >> 5) & 1, grp = threadIdx.x >> 6;
+  for (int t = cta; t < n_atiles; t += ctas) {
+    const pylo_atile at = atiles[t];
+    const pylo_tensor_desc& d = descs[at.tensor];
+    const int I = MIX ? d.I : 1;   // a row has a sum per position
+    const int X = d.X, Y = d.Y * I, rb = d.rb;
+    const int row0 = at.strip * rb;
+    const int rows = min(rb, X - row0);
+    const int col0 = at.cb * PYLO_A_COLS;
+    const float gs = grad_scale_of(d, prm);
+    const bool plain = plain_grad(gs, prm);
+    const int c0 = half * 512 + (VEC ? lane * 4 : lane);
+    const float* base = d.g + (int64_t)row0 * Y + col0 + c0;
+    const int left = Y - col0 - c0;   // columns of this lane's pieces that exist: VEC: piece j is there if j * 128 < left, else column k if k * 32 is
+    float colacc[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) colacc[j] = 0.f;
+    const int lanes = 32 / I * I, first = (col0 + half * 512) % I;   // lanes that add up, and the position of the half's first column
+    float* const own = &s_col[grp][half * 512];
+    float4 cur[4], nxt[4];
+    auto load = [&](int r, float4 (&q)[4]) {
+      const float* p = base + (int64_t)r * Y;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if constexpr (VEC) {
+          if (j * 128 < left) q[j] = ldg4(p + j * 128);
+        } else {
+          if (j * 128 < left) q[j].x = __ldg(p + j * 128);
+          if (j * 128 + 32 < left) q[j].y = __ldg(p + j * 128 + 32);
+          if (j * 128 + 64 < left) q[j].z = __ldg(p + j * 128 + 64);
+          if (j * 128 + 96 < left) q[j].w = __ldg(p + j * 128 + 96);
+        }
+      }
+    };
+    if (grp < rows) load(grp, cur);
+    for (int r = grp; r < rows; r += RC_GROUPS) {
+      if (r + RC_GROUPS < rows) load(r + RC_GROUPS, nxt);
+      float rowsum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float sq[4] = {0.f, 0.f, 0.f, 0.f};
+        if (j * 128 < left) {
+          const float e[4] = {cur[j].x, cur[j].y, cur[j].z, cur[j].w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (!VEC && j * 128 + u * 32 >= left) continue;
+            const float g = plain ? e[u] : xform_grad(e[u], gs, prm.clip_val, prm.nan_to_num);
+            const float q = g * g + 1e-30f;
+            colacc[j * 4 + u] += q;
+            rowsum += q;
+            sq[u] = q;
+          }
+        }
+        if (I > 1) st4(own + lane * 4 + j * 128, make_float4(sq[0], sq[1], sq[2], sq[3]));
+      }
+      if (I == 1) {
+        rowsum = warp_sum(rowsum);
+        if (lane == 0) s_row[r][half] = rowsum;
+      } else {   // through shared memory, where a lane stays on one position because the lanes' stride is a multiple of I
+        __syncwarp();
+        float acc = 0.f;
+        if (lane < lanes)
+#pragma unroll 8
+          for (int e = lane; e < 512; e += lanes) acc += own[e];
+        float tot = acc;
+        for (int q = I; q < lanes; q += I) tot += __shfl_sync(0xffffffffu, acc, (lane + q) & 31);   // read by lanes < I only
+        const int i = first + lane < I ? first + lane : first + lane - I;
+        if (lane < I) d.part_a[((int64_t)(row0 + r) * I + i) * (2 * d.n_cb) + 2 * at.cb + half] = tot;
+        __syncwarp();
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cur[j] = nxt[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if constexpr (VEC) st4(&s_col[grp][c0 + j * 128], make_float4(colacc[j * 4], colacc[j * 4 + 1], colacc[j * 4 + 2], colacc[j * 4 + 3]));
+      else
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s_col[grp][c0 + j * 128 + u * 32] = colacc[j * 4 + u];
+    }
+    __syncthreads();
+    if constexpr (VEC) {
+      const int c = threadIdx.x * 4;
+      if (col0 + c < Y) {
+        float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < RC_GROUPS; ++w) {
+          const float4 q = ld4(&s_col[w][c]);
+          tot.x += q.x; tot.y += q.y; tot.z += q.z; tot.w += q.w;
+        }
+        st4(d.part_b + (int64_t)at.strip * Y + col0 + c, tot);
+      }
+    } else {
+      for (int c = threadIdx.x; c < PYLO_A_COLS && col0 + c < Y; c += NT) {
+        float tot = 0.f;
+#pragma unroll
+        for (int w = 0; w < RC_GROUPS; ++w) tot += s_col[w][c];
+        d.part_b[(int64_t)at.strip * Y + col0 + c] = tot;
+      }
+    }
+    if (I == 1 && threadIdx.x < rows) d.part_a[(int64_t)(row0 + threadIdx.x) * d.n_cb + at.cb] = s_row[threadIdx.x][0] + s_row[threadIdx.x][1];
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* __restrict__ descs, const pylo_atile* __restrict__ items,
+                                                       const pylo_step_params prm) {
+  pdl_begin();
+  __shared__ float s_red[NT];
+  rowcol_generic(descs, items[blockIdx.x], prm, s_red);
+}
+
 // ================================================================================================
 // Phase A2: factored accumulators, factors, closed-form vector-feature moments.  One cluster of eight CTAs per tensor.
 //
@@ -335,17 +366,18 @@ __device__ __forceinline__ float cluster_load(const float* p, uint32_t rank) {
   return v;
 }
 
-template <int FAM>
-__global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_factor_update(const pylo_tensor_desc* __restrict__ descs,
-                                                                                          const pylo_step_params prm) {
+// mats: which tensors (those with fewer than two dims have no factors, and their closed forms stay zero), or NULL for all.
+template <int FAM, int THREADS>
+__global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(THREADS, A2_NT / THREADS) k_factor_update(const pylo_tensor_desc* __restrict__ descs,
+                                                                                          const int* __restrict__ mats, const pylo_step_params prm) {
   pdl_begin();
   using F = Fam<FAM>;
   constexpr int NS = 15;  // sums per CTA: row accumulator (its mean), then the four closed forms, three decays each
-  __shared__ float s_part[A2_NT / 128][128];
-  __shared__ float s_warp[A2_NT / 32][NS];
+  __shared__ __align__(16) float s_part[THREADS / 128][512];
+  __shared__ float s_warp[THREADS / 32][NS];
   __shared__ float s_cta[A2_CL][NS + 1];
   __shared__ float s_tot[NS + 1];
-  const pylo_tensor_desc& d = descs[blockIdx.x / A2_CL];
+  const pylo_tensor_desc& d = descs[mats ? mats[blockIdx.x / A2_CL] : blockIdx.x / A2_CL];
   const int tid = threadIdx.x, rank = (int)cluster_rank();
   if (d.mode == PYLO_MODE_VEC1D) {  // the same for all CTAs of the cluster
     if (rank == 0 && tid < PYLO_STAT_STRIDE) d.closed[tid] = 0.f;
@@ -354,6 +386,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
   cluster_arrive();   // waited for below, before the first store into another CTA
   const bool blocks = d.part_a != nullptr, r_is_a = d.r_is_a != 0;   // blocks: phase A has left row sums per block of columns
   const int64_t La = d.La, Lb = d.Lb;
+  const int parts = d.mode == PYLO_MODE_KERNEL ? 2 * d.n_cb : d.n_cb;
   const float inv_n_a = (float)d.Y, inv_n_b = (float)d.X;
   float acc[NS];
 #pragma unroll
@@ -365,8 +398,8 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
   };
 
   // 1. "a" vectors: finish the row sums, EMA of the accumulator lerp(acc, mean, 1 - beta_fac[k])
-  const int gtid = rank * A2_NT + tid;
-  for (int64_t i = gtid; i < La; i += A2_CL * A2_NT) {
+  const int gtid = rank * THREADS + tid;
+  for (int64_t i = gtid; i < La; i += A2_CL * THREADS) {
     float old[3];  // requested before the partials are added up
 #pragma unroll
     for (int k = 0; k < 3; ++k) old[k] = d.fac_a[k * La + i];
@@ -374,7 +407,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
     if (blocks) {
       s = 0.f;
 #pragma unroll 4
-      for (int c = 0; c < d.n_cb; ++c) s += d.part_a[i * d.n_cb + c];
+      for (int c = 0; c < parts; ++c) s += d.part_a[i * parts + c];
       d.sum_a[i] = s;
     } else {
       s = d.sum_a[i];
@@ -394,37 +427,55 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
       if (d.fx) st4(d.fx + 4 * i, make_float4(f[0], f[1], f[2], 0.f));
     }
   }
-  // 2. "b" vectors: sum over the strips (in a fixed order), EMA
-  for (int64_t c0 = (int64_t)rank * 128; c0 < Lb; c0 += A2_CL * 128) {
-    const int64_t i = c0 + (tid & 127);
-    float s = 0.f, old[3] = {0.f, 0.f, 0.f};
-    if (tid < 128 && i < Lb) {
+  // 2. "b" vectors: sum over the strips (in a fixed order), EMA.  A pass takes 128 columns, or 512 where there are enough of them, its
+  // strips dealt to the groups of 128 threads.
+  auto columns = [&](auto width) {
+    constexpr int V = decltype(width)::value, W = 128 * V;
+    for (int64_t c0 = (int64_t)rank * W; c0 < Lb; c0 += A2_CL * W) {
+      const int64_t i = c0 + V * (tid & 127);
+      float s[V], old[3] = {0.f, 0.f, 0.f};
+      if (tid < W && c0 + tid < Lb) {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) old[k] = d.fac_b[k * Lb + i];
-    }
-    if (i < Lb) {
-      const float* __restrict__ src = d.part_b + i;
-#pragma unroll 8
-      for (int r = tid >> 7; r < d.n_strips; r += A2_NT / 128) s += src[(int64_t)r * Lb];
-    }
-    s_part[tid >> 7][tid & 127] = s;
-    __syncthreads();
-    if (tid < 128 && i < Lb) {
-      s = 0.f;
-#pragma unroll
-      for (int w = 0; w < A2_NT / 128; ++w) s += s_part[w][tid];
-      d.sum_b[i] = s;
-      const float mean = s / inv_n_b;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float v = lerp_torch(old[k], mean, prm.w_f[k]);
-        d.fac_b[k * Lb + i] = v;
-        add(!r_is_a, k, v);
-        if (r_is_a) d.f_b[k * Lb + i] = safe_rsqrt(v);
+        for (int k = 0; k < 3; ++k) old[k] = d.fac_b[k * Lb + c0 + tid];
       }
+#pragma unroll
+      for (int u = 0; u < V; ++u) s[u] = 0.f;
+      if (i < Lb) {
+        const float* __restrict__ src = d.part_b + i;
+#pragma unroll 8
+        for (int r = tid >> 7; r < d.n_strips; r += THREADS / 128) {
+          if constexpr (V == 4) {
+            const float4 q = ld4(src + (int64_t)r * Lb);
+            s[0] += q.x; s[1] += q.y; s[2] += q.z; s[3] += q.w;
+          } else {
+            s[0] += src[(int64_t)r * Lb];
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < V; ++u) s_part[tid >> 7][V * (tid & 127) + u] = s[u];
+      __syncthreads();
+      if (tid < W && c0 + tid < Lb) {
+        const int64_t j = c0 + tid;
+        float tot = 0.f;
+#pragma unroll
+        for (int w = 0; w < THREADS / 128; ++w) tot += s_part[w][tid];
+        d.sum_b[j] = tot;
+        const float mean = tot / inv_n_b;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const float v = lerp_torch(old[k], mean, prm.w_f[k]);
+          d.fac_b[k * Lb + j] = v;
+          add(!r_is_a, k, v);
+          if (r_is_a) d.f_b[k * Lb + j] = safe_rsqrt(v);
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
-  }
+  };
+  static_assert(THREADS >= 512, "a pass of 512 columns is finished by a thread per column");
+  if (Lb % 4 == 0 && Lb > A2_CL * 128) columns(std::integral_constant<int, 4>{});
+  else columns(std::integral_constant<int, 1>{});
   // 3. the fifteen sums over the tensor, in every CTA
 #pragma unroll
   for (int j = 0; j < NS; ++j) {
@@ -435,7 +486,7 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
   cluster_wait();
   if (tid < NS) {
     float v = 0.f;
-    for (int w = 0; w < A2_NT / 32; ++w) v += s_warp[w][tid];
+    for (int w = 0; w < THREADS / 32; ++w) v += s_warp[w][tid];
     for (uint32_t q = 0; q < A2_CL; ++q) cluster_store(&s_cta[rank][tid], q, v);
   }
   cluster_sync();  // also: every CTA's accumulators are visible to the others
@@ -451,10 +502,17 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
   float* f_r = r_is_a ? d.f_a : d.f_b;
   const int64_t Lr = r_is_a ? La : Lb;
   const int64_t pre = d.rcm_pre, A = d.rcm_A, post = d.rcm_post;
+  auto put = [&](int64_t e, float v) {   // entry e of [3][Lr]
+    f_r[e] = v;
+    if (d.fx && r_is_a) {
+      const int64_t k = e >= 2 * Lr ? 2 : e >= Lr ? 1 : 0;
+      d.fx[4 * (e - k * Lr) + k] = v;
+    }
+  };
   if ((pre == 3 && A == Lr) || (pre == 1 && A == 3 && post == Lr)) {
     // the mean of each decay's whole vector, or (the decay axis is the reduce axis) of each entry's three decays
     const bool whole = pre == 3 && A == Lr;
-    for (int64_t i = gtid; i < Lr; i += A2_CL * A2_NT) {
+    for (int64_t i = gtid; i < Lr; i += A2_CL * THREADS) {
       const float v0 = fac_r[i], v1 = fac_r[Lr + i], v2 = fac_r[2 * Lr + i];
       const float own = (v0 + v1 + v2) / 3.0f;
       const float f0 = safe_rsqrt(v0 / ((whole ? s_tot[0] / (float)A : own) + 1e-9f));
@@ -463,23 +521,17 @@ __global__ void __cluster_dims__(A2_CL, 1, 1) __launch_bounds__(A2_NT, 1) k_fact
       f_r[i] = f0; f_r[Lr + i] = f1; f_r[2 * Lr + i] = f2;
       if (d.fx && r_is_a) st4(d.fx + 4 * i, make_float4(f0, f1, f2, 0.f));
     }
-  } else if (post == 1) {
+  } else {   // a warp per mean (a thread per mean, one after the other, took 55 us for VeLO over 3x3 convolutions: 27 means of 512 entries)
     const int lane = tid & 31;
-    for (int64_t pr = gtid >> 5; pr < pre; pr += A2_CL * A2_NT / 32) {
+    for (int64_t o = gtid >> 5; o < pre * post; o += A2_CL * THREADS / 32) {
+      const int64_t first = o / post * A * post + o % post;
       float m = 0.f;
-      for (int64_t a = lane; a < A; a += 32) m += fac_r[pr * A + a];
+#pragma unroll 4
+      for (int64_t a = lane; a < A; a += 32) m += fac_r[first + a * post];
       m = __shfl_sync(0xffffffffu, warp_sum(m), 0) / (float)A;
-      for (int64_t a = lane; a < A; a += 32) f_r[pr * A + a] = safe_rsqrt(fac_r[pr * A + a] / (m + 1e-9f));
-    }
-  } else {
-    for (int64_t o = gtid; o < pre * post; o += A2_CL * A2_NT) {
-      const int64_t pr = o / post, po = o % post;
-      float m = 0.f;
-      for (int64_t a = 0; a < A; ++a) m += fac_r[(pr * A + a) * post + po];
-      m /= (float)A;
-      for (int64_t a = 0; a < A; ++a) {
-        const int64_t e = (pr * A + a) * post + po;
-        f_r[e] = safe_rsqrt(fac_r[e] / (m + 1e-9f));
+      for (int64_t a = lane; a < A; a += 32) {
+        const int64_t e = first + a * post;
+        put(e, safe_rsqrt(fac_r[e] / (m + 1e-9f)));
       }
     }
   }
@@ -621,15 +673,15 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
     const float* gp = d.g + start;
     const float* pp = d.p + start;
 
-    if (d.mode == PYLO_MODE_FAST2D) {
-      const uint32_t Y = d.Y;
+    if (d.mode == PYLO_MODE_FAST2D || (!RING && d.mode == PYLO_MODE_KERNEL)) {
+      const uint32_t Y = RING ? d.Y : d.Y * d.I;
       // this thread's row and column (n < 2^31 here), moved on by a stage's length
       const uint32_t first = (uint32_t)start + tid * 4;
       uint32_t x = first / Y, y = first - x * Y;
       const uint32_t dx = PIPE_ELEMS / Y, dy = PIPE_ELEMS - dx * Y;
       const float* __restrict__ fxp = d.fx;
       const float* __restrict__ fbp = d.f_b;
-      auto update4 = [&](int i, float4 g4, float4 p4, float4 a0, float4 a1, float4 a2, float4 v4, float4 fa, float4 b0, float4 b1, float4 b2) {
+      auto update4 = [&](int i, float4 g4, float4 p4, float4 a0, float4 a1, float4 a2, float4 v4, auto row, float4 b0, float4 b1, float4 b2) {
         float ge[4] = {g4.x, g4.y, g4.z, g4.w}, pe[4] = {p4.x, p4.y, p4.z, p4.w};
         float m0e[4] = {a0.x, a0.y, a0.z, a0.w}, m1e[4] = {a1.x, a1.y, a1.z, a1.w}, m2e[4] = {a2.x, a2.y, a2.z, a2.w};
         float ve[4] = {v4.x, v4.y, v4.z, v4.w};
@@ -644,6 +696,7 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
           ve[u] = lerp_torch(ve[u], g * g + prm.eps_v, prm.w_v);
           const float rs = rsqrtf(ve[u] + prm.eps_feat);
           float f[F::NF];
+          const float4 fa = row(u);
           elem_features<FAM>(f, g, pe[u], m0e[u], m1e[u], m2e[u], ve[u], rs, fa.x * b0e[u], fa.y * b1e[u], fa.z * b2e[u]);
           accumulate<FAM, false>(acc, f);
         }
@@ -652,6 +705,25 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
         st4(m2p + i, make_float4(m2e[0], m2e[1], m2e[2], m2e[3]));
         st4(vp + i, make_float4(ve[0], ve[1], ve[2], ve[3]));
       };
+      if (!RING && d.mode == PYLO_MODE_KERNEL) {   // the four columns are four positions in turn, each with row factors of its own
+        const uint32_t I = d.I;
+        uint32_t pos = y % I;
+        const uint32_t dpos = dy % I;   // Y is a multiple of I
+        for (int i = tid * 4; i < cnt; i += PIPE_ELEMS) {
+          float4 fa[4];
+#pragma unroll
+          for (uint32_t u = 0; u < 4; ++u) {
+            uint32_t q = pos + u;
+            while (q >= I) q -= I;
+            fa[u] = ld4(fxp + 4 * ((int64_t)x * I + q));
+          }
+          update4(i, ldg4(gp + i), ld4(pp + i), ld4(m0p + i), ld4(m1p + i), ld4(m2p + i), ld4(vp + i), [&](int u) { return fa[u]; }, ld4(fbp + y),
+                  ld4(fbp + Y + y), ld4(fbp + 2 * (int64_t)Y + y));
+          x += dx; y += dy; pos += dpos;
+          if (y >= Y) { y -= Y; ++x; }
+          if (pos >= I) pos -= I;
+        }
+      } else
       for (int i = tid * 4; i - tid * 4 < cnt; i += PIPE_ELEMS) {
         const bool ok = i < cnt;
         float4 fa = make_float4(0.f, 0.f, 0.f, 0.f), b0 = fa, b1 = fa, b2 = fa;
@@ -666,13 +738,13 @@ __global__ void __launch_bounds__(NT, 2) k_state_moments(const pylo_tensor_desc*
           if (!pipe_wait_full(pipe, k)) { dead = true; break; }
           const float(*st)[PIPE_ELEMS] = pipe.st[k % PIPE_STAGES];
           if (ok) update4(i, ld4(&st[0][tid * 4]), ld4(&st[1][tid * 4]), ld4(&st[2][tid * 4]), ld4(&st[3][tid * 4]), ld4(&st[4][tid * 4]),
-                          ld4(&st[5][tid * 4]), fa, b0, b1, b2);
+                          ld4(&st[5][tid * 4]), [&](int) { return fa; }, b0, b1, b2);
           pipe_release(pipe, k++);
         } else if (ok) {
-          update4(i, ldg4(gp + i), ld4(pp + i), ld4(m0p + i), ld4(m1p + i), ld4(m2p + i), ld4(vp + i), fa, b0, b1, b2);
+          update4(i, ldg4(gp + i), ld4(pp + i), ld4(m0p + i), ld4(m1p + i), ld4(m2p + i), ld4(vp + i), [&](int) { return fa; }, b0, b1, b2);
         }
       }
-    } else if (d.mode == PYLO_MODE_GENERIC) {
+    } else if (d.mode == PYLO_MODE_GENERIC || (RING && d.mode == PYLO_MODE_KERNEL)) {
       const int64_t La = d.La, Lb = d.Lb;
       const bool vecf = d.vec_elementwise != 0;
       GenPos pos(d, d.idx0 + start + tid, NT);
@@ -825,7 +897,7 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
   for (int e = tid; e < o_end; e += NT) copy(s_net + e, d.w + e);
   // the table entries of this item: of the "a" or of the "b" index
   const int La = d.X, Lb = d.Y, items_a = (La + PER - 1) / PER;
-  const bool tables = d.fx && prm.no_tables != 1, of_a = it.strip < items_a;
+  const bool tables = d.h_a && prm.no_tables != 1, of_a = it.strip < items_a;
   const int i0 = (of_a ? it.strip : it.strip - items_a) * PER, end = tables && (of_a || prm.no_tables != 2) ? min(of_a ? La : Lb, i0 + PER) : 0;
   for (int e = tid; e < 3 * PER; e += NT) {
     const int k = e / PER, i = i0 + e % PER;
@@ -1008,7 +1080,7 @@ __global__ void __launch_bounds__(NT) k_prep_tc(const pylo_tensor_desc* __restri
   }
   __syncthreads();
   TcImage& o = *reinterpret_cast<TcImage*>(d.wfold + TC_IMAGE);
-  const bool swap = d.mode == PYLO_MODE_FAST2D && d.r_is_a;   // FAST2D: the column vector's features come first
+  const bool swap = (d.mode == PYLO_MODE_FAST2D || d.mode == PYLO_MODE_KERNEL) && d.r_is_a;   // there the column vector's features come first
   {  // both layers: a thread makes eight weights of one hidden unit, 16 bytes of each plane
     const int layer = tid >> 7, kc = part & 3;
     const float scale = s_pow[layer ? 3 : 1];
@@ -2493,6 +2565,13 @@ static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
   return ns_launch<NfSmem<128, false>, k_gemm_f16x2>(grp, (int)(tiles < sms ? tiles : sms), status, s);
 }
 
+// More clusters than run at once share the SMs two and two, so that one's barriers and latencies are another's time.
+template <int FAM>
+static void factor_update_launch(const pylo_tensor_desc* descs, const int32_t* mats, int n, const pylo_step_params& prm, cudaStream_t s) {
+  if (n * A2_CL <= sm_count()) launch(k_factor_update<FAM, A2_NT>, n * A2_CL, A2_NT, 0, s, descs, mats, prm);
+  else launch(k_factor_update<FAM, A2_NT / 2>, n * A2_CL, A2_NT / 2, 0, s, descs, mats, prm);
+}
+
 template <int FAM>
 static int state_moments_launch(const pylo_tensor_desc* descs, const pylo_tile* tiles, int n_tiles, int reverse,
                                 const pylo_step_params& prm, cudaStream_t s) {
@@ -2641,7 +2720,7 @@ int pylo_b200_workspace_layout(int family, int mode, int64_t n, int64_t La, int6
                                pylo_ws_layout* out) {
   CHECK_ARG(out && n > 0);
   CHECK_ARG(family == PYLO_FAM_ADAFAC || family == PYLO_FAM_CELO2 || family == PYLO_FAM_VELO);
-  CHECK_ARG(mode == PYLO_MODE_FAST2D || mode == PYLO_MODE_GENERIC || mode == PYLO_MODE_VEC1D);
+  CHECK_ARG(mode == PYLO_MODE_FAST2D || mode == PYLO_MODE_GENERIC || mode == PYLO_MODE_VEC1D || mode == PYLO_MODE_KERNEL);
   const int64_t H = family == PYLO_FAM_ADAFAC ? 32 : (family == PYLO_FAM_CELO2 ? 8 : 4);
   pylo_ws_layout w = {};
   if (mode != PYLO_MODE_VEC1D) {
@@ -2656,7 +2735,8 @@ int pylo_b200_workspace_layout(int family, int mode, int64_t n, int64_t La, int6
     w.n_strips = (int32_t)((rows + w.rb - 1) / w.rb);
     w.part_b = w.n_strips * Lb;
   } else if (mode != PYLO_MODE_VEC1D) {
-    CHECK_ARG(X > 0 && Y > 0 && La == X && Lb == Y && (Y % 4 == 0 || mode == PYLO_MODE_GENERIC));
+    const bool kernel = mode == PYLO_MODE_KERNEL;
+    CHECK_ARG(X > 0 && Y > 0 && (La == X || (kernel && La % X == 0 && La / X <= 32)) && Lb == Y && (Y % 4 == 0 || mode == PYLO_MODE_GENERIC));
     // rows per strip: about X / 128, a multiple of 8, within [32, 128].  Up to 512 rows a tensor gives too few strips of
     // 32 to fill the GPU and the launch is all latency: strips of 8 (one or two rows per warp) there.
     int rb = (((X + 127) / 128 + 7) / 8) * 8;
@@ -2664,9 +2744,11 @@ int pylo_b200_workspace_layout(int family, int mode, int64_t n, int64_t La, int6
     w.rb = rb;
     w.n_strips = (X + rb - 1) / rb;
     w.n_cb = (Y + PYLO_A_COLS - 1) / PYLO_A_COLS;
-    w.part_a = (int64_t)X * w.n_cb;
+    w.part_a = kernel ? 2 * La * w.n_cb : (int64_t)X * w.n_cb;
     w.part_b = (int64_t)w.n_strips * Y;
-    if (mode == PYLO_MODE_FAST2D || family != PYLO_FAM_ADAFAC) {   // what the tiled apply sweeps read
+    if (kernel) {
+      w.fx = 4 * La;
+    } else if (mode == PYLO_MODE_FAST2D || family != PYLO_FAM_ADAFAC) {   // what the tiled apply sweeps read
       w.fx = 4 * La;
       w.h_a = La * H * 2;
       w.h_b = Lb * H;
@@ -2751,27 +2833,31 @@ int pylo_b200_grad_sumsq_static(const pylo_gvec* items, const pylo_tile* tiles, 
   return launch_status();
 }
 
-int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles, int n_ragged,
+int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atiles, int n_atiles, int n_ragged, int n_kernel,
                           const pylo_atile* gitems, int n_gitems, const pylo_step_params* prm, void* stream) {
-  CHECK_ARG(descs && prm && n_ragged >= 0 && n_atiles >= n_ragged && n_gitems >= 0 && (atiles || !n_atiles));
+  CHECK_ARG(descs && prm && n_ragged >= 0 && n_kernel >= 0 && n_atiles >= n_ragged + n_kernel && n_gitems >= 0 && (atiles || !n_atiles));
   cudaStream_t s = (cudaStream_t)stream;
-  if (n_ragged > 0) launch(k_rowcol_fast<false>, grid_for(n_ragged, 3), NT, 0, s, descs, atiles, n_ragged, *prm);
-  if (n_atiles > n_ragged) launch(k_rowcol_fast<true>, grid_for(n_atiles - n_ragged, 4), NT, 0, s, descs, atiles + n_ragged, n_atiles - n_ragged, *prm);
-  if (n_gitems > 0) {
-    CHECK_ARG(gitems);
-    launch(k_rowcol_generic, n_gitems, NT, 0, s, descs, gitems, *prm);
+  CHECK_ARG(gitems || !n_gitems);
+  const pylo_atile* fast = atiles + n_ragged;
+  const int n_fast = n_atiles - n_ragged;
+  if (n_ragged > 0) launch(k_rowcol_fast<false, false>, grid_for(n_ragged, 3), NT, 0, s, descs, atiles, n_ragged, gitems, 0, *prm);
+  if (n_kernel > 0 || (n_gitems > 0 && n_fast > 0 && n_fast <= PYLO_ROWCOL_ONE_LAUNCH)) {
+    launch(k_rowcol_fast<true, true>, n_gitems + grid_for(n_fast, 3), NT, 0, s, descs, fast, n_fast, gitems, n_gitems, *prm);
+  } else {
+    if (n_fast > 0) launch(k_rowcol_fast<true, false>, grid_for(n_fast, 4), NT, 0, s, descs, fast, n_fast, gitems, 0, *prm);
+    if (n_gitems > 0) launch(k_rowcol_generic, n_gitems, NT, 0, s, descs, gitems, *prm);
   }
   return launch_status();
 }
 
-int pylo_b200_factor_update(const pylo_tensor_desc* descs, int n_tensors, const pylo_step_params* prm, void* stream) {
+int pylo_b200_factor_update(const pylo_tensor_desc* descs, const int32_t* mats, int n_tensors, const pylo_step_params* prm, void* stream) {
   CHECK_ARG(descs && prm && n_tensors >= 0);
   if (n_tensors == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: launch(k_factor_update<PYLO_FAM_ADAFAC>, n_tensors * A2_CL, A2_NT, 0, s, descs, *prm); break;
-    case PYLO_FAM_CELO2: launch(k_factor_update<PYLO_FAM_CELO2>, n_tensors * A2_CL, A2_NT, 0, s, descs, *prm); break;
-    case PYLO_FAM_VELO: launch(k_factor_update<PYLO_FAM_VELO>, n_tensors * A2_CL, A2_NT, 0, s, descs, *prm); break;
+    case PYLO_FAM_ADAFAC: factor_update_launch<PYLO_FAM_ADAFAC>(descs, mats, n_tensors, *prm, s); break;
+    case PYLO_FAM_CELO2: factor_update_launch<PYLO_FAM_CELO2>(descs, mats, n_tensors, *prm, s); break;
+    case PYLO_FAM_VELO: factor_update_launch<PYLO_FAM_VELO>(descs, mats, n_tensors, *prm, s); break;
     default: return -2;
   }
   return launch_status();
@@ -3203,9 +3289,9 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
     phases &= ~front;
   }
   if ((phases & PYLO_STEP_SUMS) && (p->n_atiles || p->n_gitems))
-    if ((rc = pylo_b200_rowcol_sums(p->tdesc, p->atiles, p->n_atiles, p->n_ragged, p->gitems, p->n_gitems, prm, stream))) return rc;
+    if ((rc = pylo_b200_rowcol_sums(p->tdesc, p->atiles, p->n_atiles, p->n_ragged, p->n_kernel, p->gitems, p->n_gitems, prm, stream))) return rc;
   if (phases & PYLO_STEP_FACTORS)
-    if ((rc = pylo_b200_factor_update(p->tdesc, p->n_tensors, prm, stream))) return rc;
+    if ((rc = pylo_b200_factor_update(p->tdesc, p->mats, p->n_mats, prm, stream))) return rc;
   if (phases & PYLO_STEP_STATE)
     if ((rc = pylo_b200_state_moments(p->desc, p->tiles, p->n_tiles, 1, prm, stream))) return rc;
   if ((phases & PYLO_STEP_MOMENTS) && !p->sum_tiles)

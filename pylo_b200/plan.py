@@ -93,8 +93,12 @@ def fill_geometry(d, shape: Sequence[int], fdims, rcm_axis: int, sliced: bool = 
     rshape = [3] + list(shape)   # of the row accumulator
     rshape[1 + fdims[1]] = 1
     d["rcm_pre"], d["rcm_A"], d["rcm_post"] = _prod(rshape[:rcm_axis]), rshape[rcm_axis], _prod(rshape[rcm_axis + 1:])
-    fast = O == 1 and M == 1 and I == 1 and Y % 4 == 0 and n < 2**31 and not sliced and _aligned16(*tensors)
-    d["mode"] = L.MODE_FAST2D if fast else L.MODE_GENERIC
+    vec = O == 1 and M == 1 and Y * I % 4 == 0 and n < 2**31 and not sliced and _aligned16(*tensors)
+    fast = vec and I == 1
+    # convolution weights of at least half a block of 128 columns: matrices whose row vectors have an entry per position (5 M parameters
+    # of 3x3 convolutions, AdafacLO, us per step 275 -> 228: state 60 -> 46, network 160 -> 128; 205 with the sums in one launch)
+    kernel = vec and 1 < I <= 32 and Y * I >= 64
+    d["mode"] = L.MODE_FAST2D if fast else L.MODE_KERNEL if kernel else L.MODE_GENERIC
     return O, X, M, Y, I, fast
 
 
@@ -260,19 +264,21 @@ def ragged_rows(family: int, tiles: Sequence[Tuple[int, int, int, int]]) -> int:
     return min((64, 32, 16, 8, 4), key=lambda k: -(-n_items(k) // ctas) * (k + 1))
 
 
-def apply_items(family: int, tensor_cores: bool, fast, slow, least: int = 8) -> np.ndarray:
+def apply_items(family: int, tensor_cores: bool, fast, slow, least: int = 8, kernel=()) -> np.ndarray:
     """Work list of the tiled apply sweep: ``fast`` = [(unit, rows, columns)] of the FAST2D units, ``slow`` = [(unit,
-    elements)] of the others, which only the tensor-core kernel takes (as runs of 128 elements, first in the list)."""
+    elements)] of the others, which only the tensor-core kernel takes (as runs of 128 elements, first in the list), ``kernel`` =
+    [(unit, rows, columns)] of the KERNEL ones, which it takes as matrices of all positions' columns (next in the list)."""
     if tensor_cores:
+        kernel = list(kernel)
         slow = [(u, -(-n // 128), 128) for u, n in slow]
         rows = lambda parts: tensor_core_rows([(X, Y) for _, X, Y in parts])
-        gen = both = rows(slow + fast)
-        if sum(-(-X // both) * -(-Y // 128) for _, X, Y in fast) >= L.TC_ONE_LAUNCH and slow:
+        gen = both = rows(slow + kernel + fast)
+        if sum(-(-X // both) * -(-Y // 128) for _, X, Y in fast) >= L.TC_ONE_LAUNCH and slow + kernel:
             # A large model's slow units have a launch of their own, which is over when its longest item is: their height follows
             # from them alone.  At the FAST2D units' 64 rows a ViT-B/16's patch embedding was 72 items of 64 tiles for 592
             # workers, and the SMs that had them came late to the FAST2D launch (133 us by itself, now 21)
-            gen, both = rows(slow), rows(fast)
-        parts = [(u, X, Y, gen, 128, L.TC_GEN_ITEM | gen) for u, X, Y in slow] + [(u, X, Y, both, 128, both) for u, X, Y in fast]
+            gen, both = rows(slow + kernel), rows(fast)
+        parts = [(u, X, Y, gen, 128, L.TC_GEN_ITEM | gen) for u, X, Y in slow] + [(u, X, Y, gen, 128, gen) for u, X, Y in kernel] + [(u, X, Y, both, 128, both) for u, X, Y in fast]
     else:
         parts = [(u, X, Y) + apply_tile_shape(family, X, Y, least) for u, X, Y in fast]
         if family != L.FAM_ADAFAC:
@@ -371,7 +377,7 @@ class LoPlan:
         H = self.H[family]
         tdesc = np.zeros(T, dtype=L.DESC_DTYPE)
         ws_items = []  # (table, row, field, count)
-        atiles, ratiles, gitems = [], [], []
+        atiles, ratiles, katiles, gitems = [], [], [], []
         ws_bytes = 0  # the library's own count of the workspace, checked against the layout below
         for i, t in enumerate(tensors):
             shape = tuple(t.p.shape)
@@ -411,12 +417,14 @@ class LoPlan:
                 ragged = not fast and not sliced and O == M == I == 1 and Y >= 64
                 # sub-buffer sizes and the phase-A tiling come from the library (pylo_b200_workspace_layout), so that
                 # this table and a table built by any other host of the C ABI agree
-                ws = L.workspace_layout(family, int(d["mode"]), n, La, Lb, X if fast or ragged else 0, Y if fast or ragged else 0)
+                kernel = int(d["mode"]) == L.MODE_KERNEL
+                in_atiles = fast or ragged or kernel
+                ws = L.workspace_layout(family, int(d["mode"]), n, La, Lb, X if in_atiles else 0, Lb if in_atiles else 0)
                 ws_items += [("t", i, f, getattr(ws, f)) for f in ("f_a", "f_b", "sum_a", "sum_b")]
                 d["rb"], d["n_strips"], d["n_cb"] = ws.rb, ws.n_strips, ws.n_cb
-                if fast or ragged:
+                if in_atiles:
                     ws_items += [("t", i, f, getattr(ws, f)) for f in ("fx", "part_a", "part_b", "h_a", "h_b") if getattr(ws, f)]
-                    (atiles if fast else ratiles).append(atile_grid(i, ws.n_strips, ws.n_cb))
+                    (ratiles if ragged else katiles if kernel else atiles).append(atile_grid(i, ws.n_strips, ws.n_cb))
                 else:
                     ws_items.append(("t", i, "part_b", ws.part_b))
                     gitems.append(atile_grid(i, ws.n_strips, (Lb + 255) // 256, 1))
@@ -491,17 +499,19 @@ class LoPlan:
         self.desc = DeviceTable(udesc, self.device) if self.sliced else self.tdesc
         self.tiles = FixedTable(tiles)
         self.n_tiles = len(tiles)
-        self.atiles = FixedTable(atile_list(ratiles + atiles))
+        self.atiles = FixedTable(atile_list(ratiles + katiles + atiles))
         self.n_atiles, self.n_ragged = len(self.atiles.host), len(atile_list(ratiles))
         self.gitems = FixedTable(atile_list(gitems))
         self.n_gitems = len(self.gitems.host)
+        self.mats = FixedTable(np.flatnonzero(tdesc["mode"] != L.MODE_VEC1D).astype(np.int32))   # the tensors with factors
+        self.n_mats = len(self.mats.host)
         self.n_tensors = T
         self.n_units = U
         self.total_elems = int(sum(sizes))
         self._keepalive = []
         # FAST2D tensors take a tiled apply kernel (see apply_items); everything else the generic one, or, with
         # tensor cores, items of the same kernel
-        fast = []
+        fast, kernel = [], []
         # phase P: item 0 of every unit folds the network, the further ones (and item 0) make the tables' parts
         pitems = [np.zeros((U, 4), dtype=np.int32)]
         pitems[0][:, 0] = np.arange(U)
@@ -509,19 +519,22 @@ class LoPlan:
         unit_of = {i: u for u, (i, _) in enumerate(unit_owner)}  # a FAST2D tensor is never sliced: one unit
         ragged = []
         for i in range(T):
+            X, Y = int(tdesc["X"][i]), int(tdesc["Y"][i])
+            if tdesc["mode"][i] == L.MODE_KERNEL and self.tensor_cores:
+                kernel.append((unit_of[i], X, Y * int(tdesc["I"][i])))
             if not tdesc["h_a"][i]:
                 continue
-            X, Y = int(tdesc["X"][i]), int(tdesc["Y"][i])
             if not self.tensor_cores:   # the tensor-core kernel reads no tables
                 pitems.append(atile_grid(unit_of[i], (X + per - 1) // per + (Y + per - 1) // per, 1)[1:])
             (fast if tdesc["mode"][i] == L.MODE_FAST2D else ragged).append((unit_of[i], X, Y))
-        slow_units = [u for u in range(U) if not tdesc["h_a"][unit_owner[u][0]]]
-        self.ctiles = FixedTable(apply_items(family, self.tensor_cores, fast, [(u, sizes[u]) for u in slow_units]))
+        tiled = {u for u, _, _ in fast + ragged + kernel}
+        slow_units = [u for u in range(U) if u not in tiled]
+        self.ctiles = FixedTable(apply_items(family, self.tensor_cores, fast, [(u, sizes[u]) for u in slow_units], kernel=kernel))
         self.n_ctiles = len(self.ctiles.host)
         self.rtiles = FixedTable(apply_items(family, False, ragged, [], 32))
         self.n_rtiles = len(self.rtiles.host)
         #: how many of them, at the front of the list, are on tensors that are not FAST2D (tensor cores only)
-        self.n_ctiles_gen = int((self.ctiles.host["pad_"] >= L.TC_GEN_ITEM).sum()) if self.tensor_cores else 0
+        self.n_ctiles_gen = int((~np.isin(self.ctiles.host["tensor"], [u for u, _, _ in fast])).sum()) if self.tensor_cores else 0
         self.pitems = FixedTable(atile_list(pitems))
         self.n_pitems = len(self.pitems.host)
         #: the kernel that takes the FAST2D tensors' apply sweep (also the key of its timings in phase_times())
@@ -544,15 +557,16 @@ class LoPlan:
         slow["tensor"] = np.asarray(slow_units, dtype=np.int32)[slow["tensor"]] if len(slow) else slow["tensor"]
         self.tiles_slow = FixedTable(slow)
         self.n_tiles_slow = len(slow)
-        self._fixed = FixedTable.place([self.tiles, self.atiles, self.gitems, self.ctiles, self.rtiles, self.pitems, self.tiles_slow], self.device)
+        self._fixed = FixedTable.place([self.tiles, self.atiles, self.gitems, self.ctiles, self.rtiles, self.pitems, self.tiles_slow, self.mats], self.device)
         self.sum_tiles, self.bulk_copies = order.sum_tiles, int(order.bulk_copies)
         #: everything pylo_b200_step needs for a step over these tensors
         self.step_plan = L.StepPlan(
             tdesc=self.tdesc.ptr, desc=self.desc.ptr, atiles=self.atiles.ptr, gitems=self.gitems.ptr, pitems=self.pitems.ptr,
-            ctiles=self.ctiles.ptr, tiles=self.tiles.ptr, tiles_slow=self.tiles_slow.ptr, rtiles=self.rtiles.ptr,
+            ctiles=self.ctiles.ptr, tiles=self.tiles.ptr, tiles_slow=self.tiles_slow.ptr, rtiles=self.rtiles.ptr, mats=self.mats.ptr, n_mats=self.n_mats,
             status=self.status.data_ptr(), host_status=self._status_host.data_ptr(),
             n_tensors=T, n_units=U, n_atiles=self.n_atiles, n_gitems=self.n_gitems, n_pitems=self.n_pitems,
             n_ctiles=self.n_ctiles, n_ctiles_gen=self.n_ctiles_gen, n_tiles=self.n_tiles, n_tiles_slow=self.n_tiles_slow, n_ragged=self.n_ragged, n_rtiles=self.n_rtiles,
+            n_kernel=sum(len(a) for a in katiles),
             tensor_cores=int(self.tensor_cores), sum_tiles=int(self.sum_tiles))
         if self.small:
             (self.step_plan.small_cluster, self.step_plan.small_slice, self.step_plan.small_rows, self.step_plan.small_cols) = self.small
@@ -642,7 +656,10 @@ class LoPlan:
         apply.insert(0 if self.tensor_cores else 1, (L.STEP_APPLY_REST, other, rest))
         if self.family == L.FAM_VELO and (self.n_ctiles or self.n_rtiles):   # the packed sweep takes the other units' tiles along
             apply = [(L.STEP_APPLY | L.STEP_APPLY_REST, self.apply_kernel, int(self.n_ctiles > 0) + int(self.n_rtiles > 0))]
-        front = [(L.STEP_SUMS, "rowcol_sums", (self.n_ragged > 0) + (self.n_atiles > self.n_ragged) + (self.n_gitems > 0)), (L.STEP_FACTORS, "factor_update", 1),
+        fast = self.n_atiles - self.n_ragged
+        joined = self.step_plan.n_kernel > 0 or 0 < fast <= L.ROWCOL_ONE_LAUNCH   # the generic items go with the others
+        front = [(L.STEP_SUMS, "rowcol_sums", (self.n_ragged > 0) + (fast > 0) + int(self.n_gitems > 0 and not joined)),
+                 (L.STEP_FACTORS, "factor_update", int(self.n_mats > 0)),
                  (L.STEP_STATE, "state_moments", 1)]
         if self.small:
             front = [(L.STEP_SUMS | L.STEP_FACTORS | L.STEP_STATE, "small_front", 1)]
