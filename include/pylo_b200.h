@@ -147,7 +147,8 @@ typedef struct pylo_step_params {
   float eps_norm;         /* inside rsqrt(S/n + eps): 1e-5 AdafacLO/ELO/VeLO, 1e-9 CELO2 */
   float clip_val;         /* element-wise clamp of the gradient; +inf for none */
   int32_t no_tables;      /* prep_apply: 0 = make the per-row (desc.h_a) and per-column (desc.h_b) first-layer tables, and for ADAFAC
-                             what apply_adafac_tc reads; 1 = neither; 2 = only what apply_adafac_tc reads (ADAFAC); 3 = the tables only */
+                             what apply_adafac_tc reads; 1 = neither; 2 = only what apply_adafac_tc reads (ADAFAC); 3 = the tables only.
+                             apply_adafac_tc: 4 = small_front has made the networks; the features' scales come from the tile partials */
   const float* gnorm_sq;  /* device scalar: sum of squares of all gradients, or NULL */
   int32_t sum_tiles;      /* prep_apply: 1 = add the tile partials up itself (finalize_moments was not called) */
   int32_t bulk_copies;    /* state_moments: 1 = FAST2D tiles come through a ring of bulk copies, for large models that consist
@@ -254,8 +255,9 @@ int pylo_b200_state_moments(const pylo_tensor_desc* descs, const pylo_tile* tile
  * contiguous matrix (O = M = I = 1) whose row_col_mean is over the whole vector (rcm_pre = 3) or over the decays (rcm_pre = 1,
  * rcm_A = 3); the units are the tensors.  slice: the most elements of a CTA's ceil(X / cluster) rows, up to 8192 (of a vector:
  * any); rows, cols: the most such rows and columns; 6 slice + 4 rows + 5 cols, each rounded up to 4, fit PYLO_SMALL_FLOATS.
- * Every tensor leaves `cluster` rows of tile_part, so desc.n_tiles has to be that. */
-int pylo_b200_small_front(const pylo_tensor_desc* descs, int n_tensors, int cluster, int slice, int rows, int cols,
+ * Every tensor leaves `cluster` rows of tile_part, so desc.n_tiles has to be that.  networks (ADAFAC): further clusters that make the
+ * networks apply_adafac_tc reads, which then (no_tables = 4) adds up the partials itself; prep_apply is not needed. */
+int pylo_b200_small_front(const pylo_tensor_desc* descs, int n_tensors, int cluster, int slice, int rows, int cols, int networks,
                           const pylo_step_params* prm, void* stream);
 
 /* Phase B2, one CTA per tensor: fixed-order reduction of the tile partials into desc.sums. */
@@ -484,7 +486,8 @@ typedef struct pylo_step_plan {
   int32_t small_cluster, small_slice, small_rows, small_cols; /* small_cluster > 0: SUMS, FACTORS and STATE, asked for together,
                         are one launch of pylo_b200_small_front */
   int32_t n_kernel; /* of atiles, those behind the first n_ragged that are on KERNEL tensors */
-  int32_t n_mats, pad_;
+  int32_t n_mats;
+  int32_t small_networks; /* clusters of small_front that make the networks; > 0: no prep_apply (ADAFAC with tensor_cores) */
 } pylo_step_plan;
 int pylo_b200_step(const pylo_step_plan* plan, const pylo_step_params* prm, int phases, void* stream);
 /* Host only: adds 1 to n step counters (HOST pointers to doubles); first: the old value of the first, equal: whether all

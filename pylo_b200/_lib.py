@@ -102,7 +102,7 @@ class StepPlan(C.Structure):
         "tdesc", "desc", "atiles", "gitems", "pitems", "ctiles", "tiles", "tiles_slow", "rtiles", "mats", "status", "host_status")] + [
         (name, C.c_int32) for name in ("n_tensors", "n_units", "n_atiles", "n_gitems", "n_pitems", "n_ctiles", "n_ctiles_gen",
                                        "n_tiles", "n_tiles_slow", "tensor_cores", "sum_tiles", "n_ragged", "n_rtiles", "small_cluster", "small_slice",
-                                       "small_rows", "small_cols", "n_kernel", "n_mats", "pad_")]
+                                       "small_rows", "small_cols", "n_kernel", "n_mats", "small_networks")]
 
 
 class PyloLibError(RuntimeError):
@@ -131,7 +131,7 @@ def _load():
         "pylo_b200_rowcol_sums": [vp, vp, i32, i32, i32, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_factor_update": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_state_moments": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
-        "pylo_b200_small_front": [vp, i32, i32, i32, i32, i32, C.POINTER(StepParams), vp],
+        "pylo_b200_small_front": [vp, i32, i32, i32, i32, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_finalize_moments": [vp, i32, vp],
         "pylo_b200_prep_apply": [vp, vp, i32, C.POINTER(StepParams), vp],
         "pylo_b200_apply": [vp, vp, i32, i32, C.POINTER(StepParams), vp],

@@ -1001,6 +1001,8 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
 // sums by 2^-TC_SHIFT as it adds the bias.  A plane's last bit is 2^-25 of the scaled unit: of a feature 2^-(25 + q) of its root mean square
 // (q = 3 at 16 M elements), of a weight 2^-(25 + a), a = 7 to 10.
 #define TC_SHIFT 10
+// where a unit's column has features of its own for all rows (FAST2D, KERNEL), those come first
+__device__ __forceinline__ bool tc_swap(const pylo_tensor_desc& d) { return (d.mode == PYLO_MODE_FAST2D || d.mode == PYLO_MODE_KERNEL) && d.r_is_a; }
 __constant__ float TIME_SCALES[11] = {1.f, 3.f, 10.f, 30.f, 100.f, 300.f, 1000.f, 3000.f, 10000.f, 30000.f, 100000.f};
 __device__ __forceinline__ int tc_room(float x) {   // the largest e (up to 60) for which x 2^e is known to be below 2^15
   return x > 0.f ? max(-60, min(60, 141 - (int)((__float_as_uint(x) >> 23) & 255))) : 60;
@@ -1011,59 +1013,53 @@ __device__ __forceinline__ uint32_t tc_plane(float x, float scale, float& rest) 
   rest = (x - __half2float(h)) * scale;
   return __half_as_ushort(h);
 }
-__global__ void __launch_bounds__(NT) k_prep_tc(const pylo_tensor_desc* __restrict__ descs, const pylo_atile* __restrict__ items,
-                                                const pylo_step_params prm) {
-  pdl_begin();
-  using F = Fam<PYLO_FAM_ADAFAC>;
-  using L = Fold<PYLO_FAM_ADAFAC>;
-  constexpr int H = F::H, NF = F::NF, NIN = F::NIN;
-  constexpr int o_b1 = NIN * H, o_w2 = o_b1 + H, o_b2 = o_w2 + H * H, o_w3 = o_b2 + H, o_b3 = o_w3 + 2 * H, o_end = o_b3 + 2;
-  __shared__ float s_net[o_end + H];            // the second layer's rows are H + 1 apart, so that lanes on different rows do not collide
-  __shared__ float s_scale[NF], s_b1[H], s_pow[6];
-  __shared__ float s_part[4][NT / 32][32];
-  __shared__ double s_d[6][PYLO_STAT_STRIDE];
-  const pylo_atile it = items[blockIdx.x];
-  if (it.strip) return;   // the whole CTA
-  const pylo_tensor_desc& d = descs[it.tensor];
-  const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5;
-  auto at = [](int e) { return e < o_w2 ? e : e < o_b2 ? e + (e - o_w2) / H : e + H; };
-  for (int e = tid; e < o_end; e += NT)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(s_net + at(e))), "l"(d.w + e) : "memory");
+// The network's part of a unit's TcImage, and in sn[28] and [29] the scale of the second layer's sums and that of the features.  Called
+// by all of a CTA's THREADS threads with room for TcNet in shared memory; the network is asked for by the caller (tc_ask_network).
+struct TcNet {
+  static constexpr int H = 32, NIN = 39, o_b1 = NIN * H, o_w2 = o_b1 + H, o_b2 = o_w2 + H * H, o_w3 = o_b2 + H, o_b3 = o_w3 + 2 * H, o_end = o_b3 + 2;
+  float net[o_end + H];   // the second layer's rows are H + 1 apart, so that lanes on different rows do not collide
+  float b1[H], pow[6];
+  float part[4][NT / 32][32];
+  __host__ __device__ static constexpr int at(int e) { return e < o_w2 ? e : e < o_b2 ? e + (e - o_w2) / H : e + H; }
+};
+template <int THREADS>
+__device__ __forceinline__ void tc_ask_network(const pylo_tensor_desc& d, TcNet& s) {
+  for (int e = threadIdx.x; e < TcNet::o_end; e += THREADS)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(s.net + TcNet::at(e))), "l"(d.w + e) : "memory");
   asm volatile("cp.async.commit_group;" ::: "memory");
-  const float n = (float)d.n;
-  if (prm.sum_tiles) {
-    const double tot = unit_sum<6>(d, s_d);
-    if (tid < NF) s_scale[tid] = rsqrtf((float)tot / n + prm.eps_norm);
-    if (tid < PYLO_STAT_STRIDE) store_unit_sum(d, tot);
-  } else if (tid < NF) {
-    s_scale[tid] = rsqrtf(d.sums[tid] / n + prm.eps_norm);
-  }
+}
+template <int THREADS>
+__device__ __forceinline__ void tc_network(const pylo_tensor_desc& d, const pylo_step_params& prm, TcNet& s) {
+  using L = Fold<PYLO_FAM_ADAFAC>;
+  using N = TcNet;
+  constexpr int H = N::H, NF = Fam<PYLO_FAM_ADAFAC>::NF, PARTS = NT / 32;
+  const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5;
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  {  // a hidden unit per lane, its inputs dealt to the warps
+  if (part < PARTS) {  // a hidden unit per lane, its inputs dealt to eight warps
     const float step = d.step + prm.step_delta;
     float sum = 0.f, most = 0.f, most2 = 0.f, time = 0.f;
-    for (int k = part; k < NF; k += NT / 32) {
-      const float a = fabsf(s_net[lane * NIN + k]);
+    for (int k = part; k < NF; k += PARTS) {
+      const float a = fabsf(s.net[lane * N::NIN + k]);
       sum += a;
       most = fmaxf(most, a);
     }
-    for (int t = part; t < 11; t += NT / 32) time = fmaf(s_net[lane * NIN + NF + t], tanhf(step / TIME_SCALES[t] - 1.0f), time);
-    for (int k = part; k < H; k += NT / 32) most2 = fmaxf(most2, fabsf(s_net[o_w2 + lane * (H + 1) + k]));
-    s_part[0][part][lane] = sum; s_part[1][part][lane] = most; s_part[2][part][lane] = most2; s_part[3][part][lane] = time;
+    for (int t = part; t < 11; t += PARTS) time = fmaf(s.net[lane * N::NIN + NF + t], tanhf(step / TIME_SCALES[t] - 1.0f), time);
+    for (int k = part; k < H; k += PARTS) most2 = fmaxf(most2, fabsf(s.net[N::o_w2 + lane * (H + 1) + k]));
+    s.part[0][part][lane] = sum; s.part[1][part][lane] = most; s.part[2][part][lane] = most2; s.part[3][part][lane] = time;
   }
   __syncthreads();
   if (part == 0) {
-    float sum = 0.f, most = 0.f, most2 = 0.f, b1 = s_net[o_b1 + lane];
-    for (int q = 0; q < NT / 32; ++q) {
-      sum += s_part[0][q][lane];
-      most = fmaxf(most, s_part[1][q][lane]);
-      most2 = fmaxf(most2, s_part[2][q][lane]);
-      b1 += s_part[3][q][lane];
+    float sum = 0.f, most = 0.f, most2 = 0.f, b1 = s.net[N::o_b1 + lane];
+    for (int q = 0; q < PARTS; ++q) {
+      sum += s.part[0][q][lane];
+      most = fmaxf(most, s.part[1][q][lane]);
+      most2 = fmaxf(most2, s.part[2][q][lane]);
+      b1 += s.part[3][q][lane];
     }
-    s_b1[lane] = b1;
-    const float spread = sqrtf(n) * 1.001f;
-    float bound = fmaf(sum, spread, fabsf(b1)), b2 = fabsf(s_net[at(o_b2 + lane)]);
+    s.b1[lane] = b1;
+    const float spread = sqrtf((float)d.n) * 1.001f;
+    float bound = fmaf(sum, spread, fabsf(b1)), b2 = fabsf(s.net[N::at(N::o_b2 + lane)]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       bound = fmaxf(bound, __shfl_xor_sync(0xffffffffu, bound, o));
@@ -1075,15 +1071,15 @@ __global__ void __launch_bounds__(NT) k_prep_tc(const pylo_tensor_desc* __restri
     const int a = min(min(6, tc_room(bound)) + TC_SHIFT - q, tc_room(most)), e1 = a + q - TC_SHIFT;
     const int a2 = min(tc_room(most2) - 1, tc_room(b2) + TC_SHIFT - e1), e2 = e1 + a2 - TC_SHIFT;
     if (lane == 0) {
-      s_pow[0] = tc_pow2(q); s_pow[1] = tc_pow2(a); s_pow[2] = tc_pow2(e1); s_pow[3] = tc_pow2(a2); s_pow[4] = tc_pow2(e2); s_pow[5] = tc_pow2(-e2);
+      s.pow[0] = tc_pow2(q); s.pow[1] = tc_pow2(a); s.pow[2] = tc_pow2(e1); s.pow[3] = tc_pow2(a2); s.pow[4] = tc_pow2(e2); s.pow[5] = tc_pow2(-e2);
     }
   }
   __syncthreads();
   TcImage& o = *reinterpret_cast<TcImage*>(d.wfold + TC_IMAGE);
-  const bool swap = (d.mode == PYLO_MODE_FAST2D || d.mode == PYLO_MODE_KERNEL) && d.r_is_a;   // there the column vector's features come first
-  {  // both layers: a thread makes eight weights of one hidden unit, 16 bytes of each plane
+  const bool swap = tc_swap(d);
+  if (tid < 256) {  // both layers: a thread makes eight weights of one hidden unit, 16 bytes of each plane
     const int layer = tid >> 7, kc = part & 3;
-    const float scale = s_pow[layer ? 3 : 1];
+    const float scale = s.pow[layer ? 3 : 1];
     uint32_t hi[4], lo[4];
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
@@ -1091,7 +1087,7 @@ __global__ void __launch_bounds__(NT) k_prep_tc(const pylo_tensor_desc* __restri
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int k = kc * 8 + i + u;
-        const float x = layer ? s_net[o_w2 + lane * (H + 1) + k] : k < NF ? s_net[lane * NIN + tc_slot_feature(k, swap)] : 0.f;
+        const float x = layer ? s.net[N::o_w2 + lane * (H + 1) + k] : k < NF ? s.net[lane * N::NIN + tc_slot_feature(k, swap)] : 0.f;
         float rest, none;
         h[u] = tc_plane(x * scale, 1.f, rest);
         l[u] = tc_plane(rest, 0.f, none);
@@ -1106,18 +1102,43 @@ __global__ void __launch_bounds__(NT) k_prep_tc(const pylo_tensor_desc* __restri
   if (part < 4) {
     const int layer = part >> 1, kc = part & 1;
     float rest, none;
-    uint32_t word = tc_plane(layer ? s_net[at(o_b2 + lane)] * s_pow[4] : s_b1[lane] * s_pow[2], 2048.f, rest);
+    uint32_t word = tc_plane(layer ? s.net[N::at(N::o_b2 + lane)] * s.pow[4] : s.b1[lane] * s.pow[2], 2048.f, rest);
     word |= tc_plane(rest, 0.f, none) << 16;
     char* b = reinterpret_cast<char*>(layer ? o.bias2 : o.bias1) + kc * 512 + (lane >> 3) * 128 + (lane & 7) * 16;
     *reinterpret_cast<uint4*>(b) = make_uint4(kc ? 0u : word, 0u, 0u, 0u);
   } else if (part == 4) {
-    o.sn[lane] = lane < NF ? s_scale[tc_slot_feature(lane, swap)] * s_pow[0] : lane == NF ? s_pow[5] : 0.f;
-    if (lane < 2) d.wfold[L::B3 + lane] = s_net[at(o_b3 + lane)];
-    if (lane == 0) d.wfold[L::SC + 1] = d.lr_mult ? d.lr * d.lr_mult[0] : d.lr;
+    if (lane < 2) {
+      o.sn[NF + lane] = s.pow[lane ? 0 : 5];
+      d.wfold[L::B3 + lane] = s.net[N::at(N::o_b3 + lane)];
+    }
+    if (lane == 2) d.wfold[L::SC + 1] = d.lr_mult ? d.lr * d.lr_mult[0] : d.lr;
   } else if (part < 7) {   // pair-major copy of the output layer
     const int e = lane + 32 * (part - 5), k = 2 * (e / 4) + (e & 1), q = (e % 4) >> 1;
-    d.wfold[L::W3P + e] = s_net[at(o_w3 + q * H + k)];
+    d.wfold[L::W3P + e] = s.net[N::at(N::o_w3 + q * H + k)];
   }
+}
+__global__ void __launch_bounds__(NT) k_prep_tc(const pylo_tensor_desc* __restrict__ descs, const pylo_atile* __restrict__ items,
+                                                const pylo_step_params prm) {
+  pdl_begin();
+  constexpr int NF = Fam<PYLO_FAM_ADAFAC>::NF;
+  __shared__ TcNet s;
+  __shared__ float s_scale[NF];
+  __shared__ double s_d[6][PYLO_STAT_STRIDE];
+  const pylo_atile it = items[blockIdx.x];
+  if (it.strip) return;   // the whole CTA
+  const pylo_tensor_desc& d = descs[it.tensor];
+  const int tid = threadIdx.x;
+  tc_ask_network<NT>(d, s);
+  const float n = (float)d.n;
+  if (prm.sum_tiles) {
+    const double tot = unit_sum<6>(d, s_d);
+    if (tid < NF) s_scale[tid] = rsqrtf((float)tot / n + prm.eps_norm);
+    if (tid < PYLO_STAT_STRIDE) store_unit_sum(d, tot);
+  } else if (tid < NF) {
+    s_scale[tid] = rsqrtf(d.sums[tid] / n + prm.eps_norm);
+  }
+  tc_network<NT>(d, prm, s);
+  if (tid < NF) reinterpret_cast<TcImage*>(d.wfold + TC_IMAGE)->sn[tid] = s_scale[tc_slot_feature(tid, tc_swap(d))] * s.pow[0];
 }
 
 // ================================================================================================
@@ -2701,12 +2722,14 @@ static int ns_clusters(nc_group& grp, int* status, cudaStream_t s) {
 }
 
 template <int FAM>
-static int small_front_launch(const pylo_tensor_desc* descs, int ctas, int cluster, const SfShape& q, const pylo_step_params& prm, cudaStream_t s) {
+static int small_front_launch(const pylo_tensor_desc* descs, int n, int cluster, const SfShape& q, int networks, const pylo_step_params& prm, cudaStream_t s) {
   static bool configured[PYLO_MAX_DEVICES] = {}, wide[PYLO_MAX_DEVICES] = {};
   if (int rc = allow_dynamic_smem(k_small_front<FAM>, PYLO_SMALL_FLOATS * 4, configured)) return rc;
   if (cluster > 8)
     if (int rc = allow_wide_clusters(k_small_front<FAM>, wide)) return rc;
-  launch_clusters(k_small_front<FAM>, ctas, SF_NT, cluster, (size_t)sf_floats(q) * 4, s, descs, q, prm);
+  size_t smem = (size_t)sf_floats(q) * 4;
+  if (networks && smem < sizeof(TcNet)) smem = sizeof(TcNet);
+  launch_clusters(k_small_front<FAM>, (n + networks) * cluster, SF_NT, cluster, smem, s, descs, n, q, prm);
   return launch_status();
 }
 
@@ -2879,9 +2902,9 @@ int pylo_b200_state_moments(const pylo_tensor_desc* descs, const pylo_tile* tile
   return launch_status();
 }
 
-int pylo_b200_small_front(const pylo_tensor_desc* descs, int n_tensors, int cluster, int slice, int rows, int cols,
+int pylo_b200_small_front(const pylo_tensor_desc* descs, int n_tensors, int cluster, int slice, int rows, int cols, int networks,
                           const pylo_step_params* prm, void* stream) {
-  CHECK_ARG(descs && prm && n_tensors >= 0);
+  CHECK_ARG(descs && prm && n_tensors >= 0 && networks >= 0 && (networks == 0 || prm->family == PYLO_FAM_ADAFAC));
   CHECK_ARG(((uintptr_t)descs & 15) == 0);   // a descriptor is read in pieces of 16 bytes
   CHECK_ARG(cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8 || cluster == 16);
   const SfShape q = {(slice + 3) & ~3, (rows + 3) & ~3, (cols + 3) & ~3};   // the arrays start on 16-byte boundaries
@@ -2889,9 +2912,9 @@ int pylo_b200_small_front(const pylo_tensor_desc* descs, int n_tensors, int clus
   if (n_tensors == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: return small_front_launch<PYLO_FAM_ADAFAC>(descs, n_tensors * cluster, cluster, q, *prm, s);
-    case PYLO_FAM_CELO2: return small_front_launch<PYLO_FAM_CELO2>(descs, n_tensors * cluster, cluster, q, *prm, s);
-    case PYLO_FAM_VELO: return small_front_launch<PYLO_FAM_VELO>(descs, n_tensors * cluster, cluster, q, *prm, s);
+    case PYLO_FAM_ADAFAC: return small_front_launch<PYLO_FAM_ADAFAC>(descs, n_tensors, cluster, q, networks, *prm, s);
+    case PYLO_FAM_CELO2: return small_front_launch<PYLO_FAM_CELO2>(descs, n_tensors, cluster, q, 0, *prm, s);
+    case PYLO_FAM_VELO: return small_front_launch<PYLO_FAM_VELO>(descs, n_tensors, cluster, q, 0, *prm, s);
     default: return -2;
   }
 }
@@ -3285,7 +3308,7 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
   int rc = 0;
   constexpr int front = PYLO_STEP_SUMS | PYLO_STEP_FACTORS | PYLO_STEP_STATE;
   if (p->small_cluster && (phases & front) == front) {
-    if ((rc = pylo_b200_small_front(p->tdesc, p->n_tensors, p->small_cluster, p->small_slice, p->small_rows, p->small_cols, prm, stream))) return rc;
+    if ((rc = pylo_b200_small_front(p->tdesc, p->n_tensors, p->small_cluster, p->small_slice, p->small_rows, p->small_cols, p->small_networks, prm, stream))) return rc;
     phases &= ~front;
   }
   if ((phases & PYLO_STEP_SUMS) && (p->n_atiles || p->n_gitems))
@@ -3294,20 +3317,26 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
     if ((rc = pylo_b200_factor_update(p->tdesc, p->mats, p->n_mats, prm, stream))) return rc;
   if (phases & PYLO_STEP_STATE)
     if ((rc = pylo_b200_state_moments(p->desc, p->tiles, p->n_tiles, 1, prm, stream))) return rc;
+  if ((phases & PYLO_STEP_STATE) && p->small_networks) {   // the phases one by one: what the launch of all of them would have left
+    pylo_step_params q = *prm;
+    q.no_tables = 2;
+    q.sum_tiles = 1;
+    if ((rc = pylo_b200_prep_apply(p->desc, p->pitems, p->n_pitems, &q, stream))) return rc;
+  }
   if ((phases & PYLO_STEP_MOMENTS) && !p->sum_tiles)
     if ((rc = pylo_b200_finalize_moments(p->desc, p->n_units, stream))) return rc;
   if (!(phases & PYLO_STEP_BACK)) return 0;
   pylo_step_params q = *prm;
   q.sum_tiles = p->sum_tiles && q.family != PYLO_FAM_VELO;
-  q.no_tables = p->tensor_cores ? 2 : 3;
-  if (phases & PYLO_STEP_PREP)
+  q.no_tables = p->small_networks ? 4 : p->tensor_cores ? 2 : 3;
+  if ((phases & PYLO_STEP_PREP) && !p->small_networks)
     if ((rc = pylo_b200_prep_apply(p->desc, p->pitems, p->n_pitems, &q, stream))) return rc;
   const bool main = phases & PYLO_STEP_APPLY, rest = phases & PYLO_STEP_APPLY_REST;
   if (p->tensor_cores) {
     // small models: one launch; large ones: what is not FAST2D first, then the others through the leaner variant
     const int first = p->n_ctiles - p->n_ctiles_gen < PYLO_TC_ONE_LAUNCH ? 0 : p->n_ctiles_gen;
     if (rest && (rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles, first, 1, &q, p->status, p->host_status, stream))) return rc;
-    if (main && (rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles + first, p->n_ctiles - first, p->n_ctiles_gen > first, &q, p->status, p->host_status, stream))) return rc;
+    if (main && (rc = pylo_b200_apply_adafac_tc(p->desc, p->ctiles + first, p->n_ctiles - first, p->n_ctiles_gen > first || p->small_networks, &q, p->status, p->host_status, stream))) return rc;
     return 0;
   }
   if (q.family == PYLO_FAM_ADAFAC) {

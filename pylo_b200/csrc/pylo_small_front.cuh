@@ -7,6 +7,8 @@
 // sums through distributed shared memory.  It takes 11.3 us there: a step of 33.9 us takes 27.3.  Bound by latency (descriptor and
 // copies 2 us, sums 1.5, the two exchanges 2.5, factors 1) and, in the state update (2.5), by the issue slots of a tensor's
 // sixteen SMs.
+// AdafacLO, ELO: clusters behind the tensors' make the networks of the tensor-core sweep meanwhile, which then only needs the features'
+// scales; it adds the few partials up itself, and there is no launch in between (perceptron: us per step 23.5 -> 19.5).
 // The host chooses it (LoPlan) where every tensor is a vector or a plain matrix whose share fits.
 #pragma once
 
@@ -28,7 +30,7 @@ __device__ __forceinline__ void sf_copy(float* dst, const float* src, int cnt) {
 }
 
 template <int FAM>
-__global__ void __launch_bounds__(SF_NT, 1) k_small_front(const pylo_tensor_desc* __restrict__ descs, const SfShape shape,
+__global__ void __launch_bounds__(SF_NT, 1) k_small_front(const pylo_tensor_desc* __restrict__ descs, int n_tensors, const SfShape shape,
                                                           const pylo_step_params prm) {
   pdl_begin();
   using F = Fam<FAM>;
@@ -37,6 +39,19 @@ __global__ void __launch_bounds__(SF_NT, 1) k_small_front(const pylo_tensor_desc
   __shared__ float s_red[WARPS * NACC];
   __shared__ float s_warp[WARPS][NS], s_cta[16][NS + 1], s_tot[NS + 1], s_scr[SF_NT];
   const int tid = threadIdx.x, lane = tid & 31, rank = (int)cluster_rank(), parts = (int)cluster_size();
+  if constexpr (FAM == PYLO_FAM_ADAFAC) {
+    // further clusters: the tensors' networks as the tensor-core sweep reads them, which need nothing that is made here
+    const int first = n_tensors * parts;
+    if ((int)blockIdx.x >= first) {
+      TcNet& net = *reinterpret_cast<TcNet*>(sf);
+      for (int u = blockIdx.x - first; u < n_tensors; u += gridDim.x - first) {
+        tc_ask_network<SF_NT>(descs[u], net);
+        tc_network<SF_NT>(descs[u], prm, net);
+        __syncthreads();
+      }
+      return;
+    }
+  }
   __shared__ pylo_tensor_desc d;   // all of it at once: read field by field between the copies it costs a trip to L2 each time
   static_assert(sizeof(d) % 16 == 0 && sizeof(d) / 16 <= SF_NT, "a thread per 16 bytes");
   if (tid < (int)(sizeof(d) / 16)) reinterpret_cast<uint4*>(&d)[tid] = __ldg(reinterpret_cast<const uint4*>(descs + blockIdx.x / parts) + tid);

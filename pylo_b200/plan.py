@@ -310,6 +310,13 @@ def small_front(mats: Sequence[Tuple[int, int]], vectors: Sequence[int]):
     return found or next((q for q in map(share, [cl for cl in (1, 2, 4, 8, 16) if T * cl <= 2 * SMALL_CTAS]) if q), None)
 
 
+def small_networks(n_tensors: int, cluster: int) -> bool:
+    """Whether one more cluster of this size, which makes the networks of the tensor-core sweep, costs no further turn: a cluster lies
+    in one of eight groups of at least 18 SMs."""
+    at_once = 8 * (18 // cluster)
+    return -(-(n_tensors + 1) // at_once) == -(-n_tensors // at_once)
+
+
 class SumOrder(NamedTuple):
     """How the sums over a tensor are made.  All of it decides in which order a tensor's terms are added up."""
 
@@ -570,6 +577,7 @@ class LoPlan:
             tensor_cores=int(self.tensor_cores), sum_tiles=int(self.sum_tiles))
         if self.small:
             (self.step_plan.small_cluster, self.step_plan.small_slice, self.step_plan.small_rows, self.step_plan.small_cols) = self.small
+            self.step_plan.small_networks = int(self.tensor_cores and small_networks(T, self.small[0]))
         self._step_plan_ref = C.byref(self.step_plan)
         self._hyper = None          # what set_hyper last wrote
         self._grad_ptrs = None      # the gradient addresses the table holds
@@ -664,7 +672,7 @@ class LoPlan:
         if self.small:
             front = [(L.STEP_SUMS | L.STEP_FACTORS | L.STEP_STATE, "small_front", 1)]
         phases = front + [(L.STEP_MOMENTS, "finalize_moments", int(not self.sum_tiles)),
-                  (L.STEP_PREP, "prep_apply", 1)] + apply
+                  (L.STEP_PREP, "prep_apply", int(not self.step_plan.small_networks))] + apply
         return [ph for ph in phases if ph[2]]
 
     def enable_profile(self, on: bool = True):

@@ -90,3 +90,32 @@ def test_a_gradient_that_is_not_a_number_counts_as_no_activation(shape):
     o = W[4] @ torch.relu(W[3]) + W[5]
     want = before.double() - LR * float(opt.step_mult) * o[0] * torch.exp(o[1] * float(opt.exp_mult))
     assert torch.allclose(p.detach().double(), want, rtol=1e-5, atol=0)
+
+
+@pytest.mark.parametrize("family", ["adafaclo", "elo"])
+@pytest.mark.parametrize("shapes", [[(5, 3)], [(128, 96), (128,), (10, 128), (10,)], [(33, 37), (40,)] * 3 + [(300, 64)],
+                                    [(24, 16), (24,)] * 12, [(3, 5)] * 150])
+def test_networks_made_by_the_front_launch(family, shapes, monkeypatch):
+    """One launch less than with a preparation of its own, and the same step: the sums over a tensor's tiles are added up in fp64."""
+    from pylo_b200 import plan
+    from test_gpu_properties import _make
+
+    outs = []
+    for joined in (True, False):
+        if not joined:
+            monkeypatch.setattr(plan, "small_networks", lambda n, cluster: False)
+        gen = torch.Generator(device="cuda").manual_seed(11)
+        params = [torch.nn.Parameter(torch.randn(*s, device="cuda", generator=gen) * 0.1) for s in shapes]
+        opt = _make(family, params)
+        for _ in range(3):
+            for p in params:
+                p.grad = torch.randn(*p.shape, device="cuda", generator=gen) * 0.3
+            opt.step()
+        opt.check_status()
+        plans = [pl for _, pl in opt._plans.values()]
+        assert all(pl.small for pl in plans)
+        want = plan.small_networks(len(shapes), plans[0].small[0])
+        assert all(bool(pl.step_plan.small_networks) == want for pl in plans)
+        outs.append([p.detach().clone() for p in params])
+    for a, b in zip(*outs):
+        assert torch.allclose(a, b, rtol=1e-6, atol=1e-8)
