@@ -429,7 +429,8 @@ typedef struct pylo_velo_rnn {
   float *controls;                                /* workspace [T][B] */
   float *weights;                                 /* out [T][160] */
   float *lr_mult;                                 /* out [T] */
-  int32_t T, H, B, pad_;
+  int32_t T, H, B;
+  int32_t mixed;                                  /* 1: pylo_b200_velo_inputs has made xmix */
 } pylo_velo_rnn;
 /* The loss buffer (BufferLossAccumulators, velo_cuda.py:170-211): means[10], iteration, running_min[10], decays[10], and
  * the step's loss, a device scalar or (loss == NULL) value. */
@@ -449,6 +450,10 @@ int pylo_b200_velo_tensor_features(const pylo_tensor_desc* descs, int n_local, c
                                    int n_total, const float* rank_onehot, float fraction,
                                    const pylo_velo_loss* lossbuf, float* x_in, void* stream);
 int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, const pylo_velo_loss* lossbuf, void* stream);
+/* velo_tensor_features and the first layer of velo_rnn in one launch, for all (up to 16) tensors of a model, of up to 16 tiles each, and H a
+ * multiple of 128 up to 512; velo_rnn with mixed = 1 comes next. */
+int pylo_b200_velo_inputs(const pylo_tensor_desc* descs, const int32_t* layer_of, const float* rank_onehot, float fraction,
+                          const pylo_velo_loss* lossbuf, const pylo_velo_rnn* rnn, void* stream);
 /* The loss buffer's update and features alone, for a host with a front end of its own: writes loss9[9]. */
 int pylo_b200_velo_loss_features(float* means, int32_t* iteration, float* running_min, const float* decays,
                                  const float* loss, float* loss9, void* stream);

@@ -87,7 +87,7 @@ class VeloRnn(C.Structure):
     _fields_ = [(name, C.c_void_p) for name in (
         "mix2_w", "mix2_b", "fmix_w", "fmix_b", "lstm_w", "lstm_b", "ctrl_w", "ctrl_b", "step_w", "step_b",
         "bank", "h", "c", "x_in", "status", "xmix", "gates", "controls", "weights", "lr_mult")] + [
-        ("T", C.c_int32), ("H", C.c_int32), ("B", C.c_int32), ("pad_", C.c_int32)]
+        ("T", C.c_int32), ("H", C.c_int32), ("B", C.c_int32), ("mixed", C.c_int32)]
 
 
 class VeloLoss(C.Structure):
@@ -148,6 +148,7 @@ def _load():
         "pylo_b200_celo2_post_apply": [vp, vp, i32, vp, vp, vp],
         "pylo_b200_adamw": [vp, vp, i32, i32] + [f32] * 7 + [C.POINTER(StepParams), vp],
         "pylo_b200_velo_tensor_features": [vp, i32, vp, i32, vp, f32, C.POINTER(VeloLoss), vp, vp],
+        "pylo_b200_velo_inputs": [vp, vp, vp, f32, C.POINTER(VeloLoss), C.POINTER(VeloRnn), vp],
         "pylo_b200_velo_rnn": [C.POINTER(VeloRnn), C.POINTER(VeloLoss), vp],
         "pylo_b200_velo_loss_features": [vp, vp, vp, vp, vp, vp, vp],
         "pylo_b200_step": [C.POINTER(StepPlan), C.POINTER(StepParams), i32, vp],
@@ -168,6 +169,7 @@ lib, EXPORTED = _load()
 
 
 SM_COUNT = 148        # of a B200; sizes of work lists only, the kernels ask the device
+VELO_INPUTS_MOST = 16  # tensors that pylo_b200_velo_inputs takes, and their tiles
 TC_WORKERS = SM_COUNT * 4  # warpgroups the tensor-core apply kernel runs at once (four per SM)
 TC_GEN_ITEM = 1 << 16  # tag bit of its items on tensors that are not FAST2D
 STEP_SUMS, STEP_FACTORS, STEP_STATE, STEP_MOMENTS, STEP_PREP, STEP_APPLY, STEP_APPLY_REST = (1 << k for k in range(7))

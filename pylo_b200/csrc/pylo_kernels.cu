@@ -838,8 +838,7 @@ __device__ __forceinline__ double unit_sum(const pylo_tensor_desc& d, double (&s
   }
   return tot;
 }
-__device__ __forceinline__ void store_unit_sum(const pylo_tensor_desc& d, double tot) {
-  const int j = threadIdx.x;
+__device__ __forceinline__ void store_unit_sum(const pylo_tensor_desc& d, double tot, int j = threadIdx.x) {
   const float hi = (float)tot;
   d.sums[j] = hi;
   if (j >= 30 && j < 38) d.sums[SUMS_LO + (j - 30)] = (float)(tot - (double)hi);
@@ -2170,6 +2169,34 @@ __global__ void k_velo_loss(const pylo_velo_loss b, float* __restrict__ loss9) {
   velo_loss_update(b, loss9, true);
 }
 
+// Entry `lane` (< 30) of a tensor's LSTM inputs from its sums (s_sum, 40 of them) and the loss features.
+__device__ __forceinline__ float velo_feature(int lane, const pylo_tensor_desc& d, const double* s_sum, const float* s_loss9, const float* rank_onehot,
+                                              float fraction) {
+  const double n = (double)d.n;
+  // as the stored sums have them: 32 bits, the VeLO statistics 32 + 32
+  auto stat = [&](int j) { const float hi = (float)s_sum[30 + j]; return (double)hi + (double)(float)(s_sum[30 + j] - (double)hi); };
+  const float mean_p2 = (float)((double)(float)s_sum[2] / n);
+  const double norm = (double)rsqrtf(fmaxf(mean_p2, 1e-9f));
+  const double mean_v = stat(6) / n, e_v2 = stat(7) / n;
+  float o = 0.f;
+  if (lane < 9) {  // tanh((x - t) * 10) (velo_cuda.py:155-162)
+    const float at[9] = {0.03f, 0.1f, 0.2f, 0.4f, 0.6f, 0.8f, 0.9f, 1.0f, 1.1f};
+#pragma unroll
+    for (int j = 0; j < 9; ++j) if (lane == j) o = tanhf((fraction - at[j]) * 10.0f);
+  }
+  else if (lane < 18) o = s_loss9[lane - 9];
+  else if (lane == 18) o = clip_log_abs10((float)(norm * mean_v));
+  else if (lane < 24) o = rank_onehot[lane - 19];
+  else if (lane < 30) {
+    const int k = (lane - 24) % 3;
+    const double mu = stat(k) / n, e_m2 = stat(3 + k) / n;
+    const double var = lane < 27 ? fmax(e_m2 - mu * mu, 0.0)
+                                : fmax(e_v2 - 2.0 * mu * mean_v + mu * mu, 0.0);  // mean((rms - mean_m)^2), velo_cuda.py:243
+    o = clip_log_abs10((float)(norm * norm * var));
+  }
+  return o;
+}
+
 // The 30 LSTM inputs of a tensor from the statistics gathered in phase B (velo_cuda.py:213-252).  One CTA per tensor, which
 // first does phase B2 for it (a launch less), while its last warp works out the loss features: every CTA for itself and
 // without advancing the loss buffer, which is left to a kernel that runs when all of them are done (k_velo_xmix).
@@ -2193,28 +2220,7 @@ __global__ void __launch_bounds__(ROWS * PYLO_STAT_STRIDE + 32) k_velo_tensor_fe
   __syncthreads();
   if (tid >= 32) return;
   const int layer = layer_of ? layer_of[t] : t;  // position of this tensor among all T tensors of the model
-  const double n = (double)d.n;
-  // as the stored sums have them: 32 bits, the VeLO statistics 32 + 32
-  auto stat = [&](int j) { const float hi = (float)s_sum[30 + j]; return (double)hi + (double)(float)(s_sum[30 + j] - (double)hi); };
-  const float mean_p2 = (float)((double)(float)s_sum[2] / n);
-  const double norm = (double)rsqrtf(fmaxf(mean_p2, 1e-9f));
-  const double mean_v = stat(6) / n, e_v2 = stat(7) / n;
-  float o = 0.f;
-  if (tid < 9) {  // tanh((x - t) * 10) (velo_cuda.py:155-162)
-    const float at[9] = {0.03f, 0.1f, 0.2f, 0.4f, 0.6f, 0.8f, 0.9f, 1.0f, 1.1f};
-#pragma unroll
-    for (int j = 0; j < 9; ++j) if (tid == j) o = tanhf((fraction - at[j]) * 10.0f);
-  }
-  else if (tid < 18) o = s_loss9[tid - 9];
-  else if (tid == 18) o = clip_log_abs10((float)(norm * mean_v));
-  else if (tid < 24) o = rank_onehot[t * 5 + tid - 19];
-  else if (tid < 30) {
-    const int k = (tid - 24) % 3;
-    const double mu = stat(k) / n, e_m2 = stat(3 + k) / n;
-    const double var = tid < 27 ? fmax(e_m2 - mu * mu, 0.0)
-                                : fmax(e_v2 - 2.0 * mu * mean_v + mu * mu, 0.0);  // mean((rms - mean_m)^2), velo_cuda.py:243
-    o = clip_log_abs10((float)(norm * norm * var));
-  }
+  const float o = velo_feature(tid, d, s_sum, s_loss9, rank_onehot + t * 5, fraction);
   if (tid < 30) x_in[(int64_t)(T - 1 - layer) * 30 + tid] = o;  // rows are flipped (velo_cuda.py:422)
 }
 
@@ -2246,6 +2252,64 @@ __global__ void __launch_bounds__(NT) k_velo_xmix(const pylo_velo_rnn r, const p
   for (int t = lane; t < r.T; t += 32) r.xmix[(int64_t)t * r.H + h] += best;
 }
 
+// The two above in one launch for small models (up to VI_TENSORS tensors of up to VI_TILES tiles): every CTA makes all tensors' inputs for itself,
+// from sums in the order of unit_sum, and its eight hidden units' x'.  The loss buffer, which all CTAs read here, is written by
+// k_velo_lstm.  Latency-bound; in place of two launches: perceptron, us per step 44.4 -> 42.2.
+#define VI_TENSORS 16
+#define VI_TILES 16
+__global__ void __launch_bounds__(NT) k_velo_inputs(const pylo_tensor_desc* __restrict__ descs, const int32_t* __restrict__ layer_of,
+                                                    const float* __restrict__ rank_onehot, float fraction, const pylo_velo_loss lossbuf,
+                                                    const pylo_velo_rnn r) {
+  pdl_begin();
+  __shared__ double s_sum[VI_TENSORS][PYLO_STAT_STRIDE];
+  __shared__ float s_x[VI_TENSORS][31], s_loss9[9];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, j = tid % PYLO_STAT_STRIDE, T = r.T;
+  const int h = blockIdx.x * NWARP + warp;
+  const bool unit = h < r.H;
+  const float w2 = unit && lane < 30 ? __ldg(r.mix2_w + h * 30 + lane) : 0.f, wf = unit && lane < 30 ? __ldg(r.fmix_w + h * 30 + lane) : 0.f;
+  const float b2 = unit ? __ldg(r.mix2_b + h) : 0.f, bf = unit ? __ldg(r.fmix_b + h) : 0.f;
+  if (tid < 5 * PYLO_STAT_STRIDE) {
+    for (int t = tid / PYLO_STAT_STRIDE; t < T; t += 5) {
+      const pylo_tensor_desc& d = descs[t];
+      const float* __restrict__ src = d.tile_part + j;
+      const int n = d.n_tiles;
+      float v[VI_TILES];
+#pragma unroll
+      for (int q = 0; q < VI_TILES; ++q) v[q] = q < n ? src[q * PYLO_STAT_STRIDE] : 0.f;
+      double tot = 0.0;
+#pragma unroll
+      for (int q = 0; q < VI_TILES; ++q) tot += (double)v[q];
+      tot += (double)d.closed[j];
+      s_sum[t][j] = tot;
+      if (blockIdx.x == 0) store_unit_sum(d, tot, j);
+    }
+  } else if (warp == NWARP - 1) {
+    velo_loss_update(lossbuf, s_loss9, false);
+  }
+  __syncthreads();
+  for (int t = warp; t < T; t += NWARP) {
+    const int row = T - 1 - (layer_of ? layer_of[t] : t);  // rows are flipped (velo_cuda.py:422)
+    const float o = velo_feature(lane, descs[t], s_sum[t], s_loss9, rank_onehot + t * 5, fraction);
+    if (lane < 30) {
+      s_x[row][lane] = o;
+      if (blockIdx.x == 0) r.x_in[row * 30 + lane] = o;
+    }
+  }
+  __syncthreads();
+  float m = b2, f = bf;
+  const float* x = s_x[lane < T ? lane : 0];   // a lane per tensor
+#pragma unroll
+  for (int k = 0; k < 30; ++k) {
+    const float v = x[k];
+    m = fmaf(__shfl_sync(0xffffffffu, w2, k), v, m);
+    f = fmaf(__shfl_sync(0xffffffffu, wf, k), v, f);
+  }
+  float best = lane < T ? fmaxf(m, 0.f) : 0.f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if (unit && lane < T) r.xmix[(int64_t)lane * r.H + h] = f + best;
+}
+
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 // cell update of one hidden unit; gate order i, g, f, o with f + 1 (VeLO_RNN.py:57-65)
 __device__ __forceinline__ float velo_cell(float i, float g, float f, float o, float& c) {
@@ -2266,13 +2330,14 @@ __device__ __forceinline__ float velo_cell(float i, float g, float f, float o, f
 // left in `gates` ([T][H]), k_velo_mix takes it over.
 #define GR_UNITS 4   // hidden units per CTA: one per pair of warps
 template <int NI>    // float4 per lane and row: H = 128 * NI
-__global__ void __launch_bounds__(NT, 2) k_velo_lstm(const pylo_velo_rnn r, int groups_per_cta) {
+__global__ void __launch_bounds__(NT, 2) k_velo_lstm(const pylo_velo_rnn r, const pylo_velo_loss lossbuf, int groups_per_cta) {
   pdl_begin();
   extern __shared__ __align__(16) float s_x[];   // [2][8][2H]
   __shared__ float s_half[GR_UNITS][32];
   constexpr int H = 128 * NI;
   const int tid = threadIdx.x, lane = tid & 31, half = (tid >> 5) & 1, unit = tid >> 6, h = blockIdx.x * GR_UNITS + unit;
   const int word = reported(r.status);
+  if (lossbuf.means && blockIdx.x == 0 && blockIdx.y == 0 && tid < 32) velo_loss_update(lossbuf, nullptr, !word);   // behind k_velo_inputs
   const int groups = (r.T + 7) / 8, g0 = blockIdx.y * groups_per_cta, g1 = min(g0 + groups_per_cta, groups);
   auto stage = [&](int g) {
     float* dst = s_x + (g & 1) * 16 * H;
@@ -3264,22 +3329,32 @@ int pylo_b200_velo_tensor_features(const pylo_tensor_desc* descs, int n_local, c
   return launch_status();
 }
 
+int pylo_b200_velo_inputs(const pylo_tensor_desc* descs, const int32_t* layer_of, const float* rank_onehot, float fraction,
+                          const pylo_velo_loss* lossbuf, const pylo_velo_rnn* rnn, void* stream) {
+  CHECK_ARG(descs && rank_onehot && rnn && rnn->T > 0 && rnn->T <= VI_TENSORS && rnn->x_in && rnn->xmix);
+  CHECK_ARG(lossbuf && lossbuf->means && lossbuf->iteration && lossbuf->running_min && lossbuf->decays);
+  launch(k_velo_inputs, (rnn->H + NWARP - 1) / NWARP, NT, 0, (cudaStream_t)stream, descs, layer_of, rank_onehot, fraction, *lossbuf, *rnn);
+  return launch_status();
+}
+
 int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, const pylo_velo_loss* lossbuf, void* stream) {
   CHECK_ARG(rnn && rnn->T > 0 && rnn->H > 0 && rnn->B > 0 && rnn->B <= 1024);
   cudaStream_t s = (cudaStream_t)stream;
   const pylo_velo_rnn r = *rnn;
   const int64_t TH = (int64_t)r.T * r.H;
   const pylo_velo_loss none = {};
-  launch(k_velo_xmix, (r.H + NWARP - 1) / NWARP, NT, 0, s, r, lossbuf ? *lossbuf : none);
+  const bool tiled = !(r.H % 128 == 0 && r.H <= 512);   // the LSTM's other kernels
+  CHECK_ARG(!r.mixed || !tiled);
+  if (!r.mixed) launch(k_velo_xmix, (r.H + NWARP - 1) / NWARP, NT, 0, s, r, lossbuf ? *lossbuf : none);
   const float* h = r.h;   // the new one
-  if (r.H % 128 == 0 && r.H <= 512) {
+  if (!tiled) {
     const int gx = r.H / GR_UNITS, groups = (r.T + 7) / 8;
     const int gy = groups * gx <= 2 * sm_count() ? groups : (2 * sm_count() / gx > 0 ? 2 * sm_count() / gx : 1);   // two CTAs per SM
     const int per = (groups + gy - 1) / gy, smem = 2 * 8 * 2 * r.H * (int)sizeof(float);
     static bool configured[4][PYLO_MAX_DEVICES] = {};
     auto kernel = r.H == 128 ? k_velo_lstm<1> : r.H == 256 ? k_velo_lstm<2> : r.H == 384 ? k_velo_lstm<3> : k_velo_lstm<4>;
     if (int rc = allow_dynamic_smem(kernel, smem, configured[r.H / 128 - 1])) return rc;
-    launch(kernel, dim3(gx, gy), NT, smem, s, r, per);
+    launch(kernel, dim3(gx, gy), NT, smem, s, r, r.mixed && lossbuf ? *lossbuf : none, per);
     h = r.gates;
   } else {
     launch(k_velo_gates, dim3((4 * r.H + GT - 1) / GT, (r.T + GT - 1) / GT), NT, 0, s, r);

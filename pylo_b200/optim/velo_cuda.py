@@ -248,6 +248,8 @@ class VeLO_CUDA(Optimizer):
         for k in ("x_in", "xmix", "gates", "controls", "weights", "lr_mult"):
             setattr(r, k, buf[k].data_ptr())
         r.T, r.H, r.B = T, H, B
+        # a small model that this process has all of: the LSTM's inputs and its first layer in one launch
+        r.mixed = int(self._owned is None and plan.small is not None and T <= L.VELO_INPUTS_MOST and H % 128 == 0 and H <= 512)
         return {"plan": plan, "buf": buf, "rnn": r, "loss": L.VeloLoss(), "hyper": None}
 
     # ------------------------------------------------------------------ step
@@ -313,10 +315,14 @@ class VeLO_CUDA(Optimizer):
         sharded = self._owned is not None
         if sharded:
             buf["x_in"].zero_()
-        L.check(L.lib.pylo_b200_velo_tensor_features(plan.desc.ptr, plan.n_tensors, buf["layer_of"].data_ptr(), int(r.T),
-                                                     buf["rank"].data_ptr(), float(fraction), C.byref(loss_arg),
-                                                     buf["x_in"].data_ptr(), stream),
-                "velo_tensor_features")
+        if r.mixed:
+            L.check(L.lib.pylo_b200_velo_inputs(plan.desc.ptr, buf["layer_of"].data_ptr(), buf["rank"].data_ptr(), float(fraction),
+                                                C.byref(loss_arg), C.byref(r), stream), "velo_inputs")
+        else:
+            L.check(L.lib.pylo_b200_velo_tensor_features(plan.desc.ptr, plan.n_tensors, buf["layer_of"].data_ptr(), int(r.T),
+                                                         buf["rank"].data_ptr(), float(fraction), C.byref(loss_arg),
+                                                         buf["x_in"].data_ptr(), stream),
+                    "velo_tensor_features")
         if sharded and torch.distributed.is_initialized() and torch.distributed.get_world_size(self._pg) > 1:
             torch.distributed.all_reduce(buf["x_in"], group=self._pg)
         L.check(L.lib.pylo_b200_velo_rnn(C.byref(r), C.byref(loss_arg), stream), "velo_rnn")
