@@ -144,25 +144,18 @@ def tile_elems(total: int, least: int, tiles_wanted: int) -> int:
     return e
 
 
-def state_tile(family: int, sizes: Sequence[int]) -> int:
+def state_tile(sizes: Sequence[int]) -> int:
     """Elements per tile of the state sweep over units of these sizes: the multiple of 1024 (one pass of a CTA) with which the CTAs that
     run at once, two per SM, are done first, where that saves a sixth over the power of two that gives four CTAs per SM a tile.  A
-    tile's start and its block reduction cost about a pass; a launch that adds up the partials of units of more than SUM_TILES_MOST
-    tiles costs about as much as two.  Two full turns are no gain (the CTAs of a turn start, read and reduce together): 5 M parameters
-    of convolutions 206.8 with the power of two, 214.9 us per step in two turns, 202.7 in three; VeLO on a ViT of 5 M 174.5 and 185.7.
-    One turn or three: perceptrons 156.1 -> 146.0 (4 M), VeLO 295.0 -> 283.2 (11 M, odd sizes), CELO2 on 11 M 317.3 -> 305.0.
-    """
+    tile's start and its block reduction cost about a pass.  Two full turns are no gain (the CTAs of a turn start, read and reduce
+    together): 5 M parameters of convolutions 206.8 with the power of two, 214.9 us per step in two turns, 202.7 in three; VeLO on a
+    ViT of 5 M 174.5 and 185.7.  One turn or three: perceptrons 156.1 -> 146.0 (4 M), VeLO 295.0 -> 283.2 (11 M, odd sizes), CELO2 on
+    11 M 317.3 -> 305.0."""
     n, at_once = np.asarray(sizes, dtype=np.int64), 2 * L.SM_COUNT
-
-    def cost(e):
-        tiles = -(-n // e)
-        return -(-int(tiles.sum()) // at_once) * (e + 1024) + 1750 * (family != L.FAM_VELO and int(tiles.max(initial=0)) > SUM_TILES_MOST)
-
-    def turns(e):
-        return -(-int((-(-n // e)).sum()) // at_once)
-
     plain = tile_elems(int(n.sum()), 1024, 4 * L.SM_COUNT)
-    best = min([e for e in range(L.TILE_ELEMS, 0, -1024) if turns(e) != 2 or e == 1024], key=cost)
+    turns = {e: -(-int((-(-n // e)).sum()) // at_once) for e in range(L.TILE_ELEMS, 0, -1024)}
+    cost = lambda e: turns[e] * (e + 1024)
+    best = min([e for e in turns if turns[e] != 2 or e == plain], key=cost)
     return best if cost(best) < 0.83 * cost(plain) else plain
 
 
@@ -354,7 +347,7 @@ class SumOrder(NamedTuple):
 def sum_order(family: int, d: np.ndarray, sizes: Sequence[int], modes: np.ndarray, sliced: bool) -> SumOrder:
     """The rule, for tensors with these descriptors and their units of these sizes and modes.
 
-    Tiles: see :func:`state_tile`; a large model's are as large as they can be.
+    Tiles: see :func:`state_tile`.
 
     The state sweep's ring of bulk copies leaves little L1 cache to the units that are not FAST2D and keeps the launches around it
     apart, so it has to have enough to do: from 64 M elements on (VeLO on 100 M: 1615 -> 1580 us per step, on 17 M: 341 -> 351;
@@ -364,7 +357,7 @@ def sum_order(family: int, d: np.ndarray, sizes: Sequence[int], modes: np.ndarra
         vectors = d["mode"] == L.MODE_VEC1D
         if (vectors | plain_matrices(d)).all():
             small = small_front(list(zip(d["X"][~vectors].tolist(), d["Y"][~vectors].tolist())), d["n"][vectors].tolist())
-    elems = state_tile(family, sizes) if total < L.BULK_COPY_ELEMS else L.TILE_ELEMS
+    elems = state_tile(sizes)
     most = small[0] if small else -(-max(sizes, default=0) // elems)
     fast = int(sum(n for n, m in zip(sizes, modes.tolist()) if m == L.MODE_FAST2D))
     return SumOrder(small, elems, family == L.FAM_VELO or most <= SUM_TILES_MOST, fast >= L.BULK_COPY_ELEMS and 8 * fast >= 7 * total)
