@@ -406,6 +406,11 @@ typedef struct pylo_adam_item {
 int pylo_b200_adamw(const pylo_adam_item* items, const pylo_tile* tiles, int n_tiles, int independent,
                     float beta1, float one_minus_beta1, float beta2, float one_minus_beta2, float eps,
                     float bc1, float bc2, const pylo_step_params* prm, void* stream);
+/* celo2_post_apply and adamw in one launch, for small models (up to PYLO_TAIL_ONE_LAUNCH tiles of both). */
+#define PYLO_TAIL_ONE_LAUNCH 592
+int pylo_b200_celo2_tail(const pylo_post_item* post, const pylo_tile* post_tiles, int n_post, const int* status, int* host_status,
+                         const pylo_adam_item* items, const pylo_tile* tiles, int n_tiles, int independent, float beta1, float one_minus_beta1,
+                         float beta2, float one_minus_beta2, float eps, float bc1, float bc2, const pylo_step_params* prm, void* stream);
 
 /* VeLO front end.  velo_tensor_features: desc.sums -> the [T][30] LSTM input rows, row T-1-t for
  * tensor t (velo_cuda.py:213-252,419-422); loss features and fraction features are passed in.

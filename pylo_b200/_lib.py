@@ -147,6 +147,7 @@ def _load():
         "pylo_b200_celo2_post_sums": [vp, vp, i32, vp],
         "pylo_b200_celo2_post_apply": [vp, vp, i32, vp, vp, vp],
         "pylo_b200_adamw": [vp, vp, i32, i32] + [f32] * 7 + [C.POINTER(StepParams), vp],
+        "pylo_b200_celo2_tail": [vp, vp, i32, vp, vp] + [vp, vp, i32, i32] + [f32] * 7 + [C.POINTER(StepParams), vp],
         "pylo_b200_velo_tensor_features": [vp, i32, vp, i32, vp, f32, C.POINTER(VeloLoss), vp, vp],
         "pylo_b200_velo_inputs": [vp, vp, vp, f32, C.POINTER(VeloLoss), C.POINTER(VeloRnn), vp],
         "pylo_b200_velo_rnn": [C.POINTER(VeloRnn), C.POINTER(VeloLoss), vp],
@@ -170,6 +171,7 @@ lib, EXPORTED = _load()
 
 SM_COUNT = 148        # of a B200; sizes of work lists only, the kernels ask the device
 VELO_INPUTS_MOST = 16  # tensors that pylo_b200_velo_inputs takes, and their tiles
+TAIL_ONE_LAUNCH = 592  # tiles of CELO2's tail and AdamW up to which they share a launch
 TC_WORKERS = SM_COUNT * 4  # warpgroups the tensor-core apply kernel runs at once (four per SM)
 TC_GEN_ITEM = 1 << 16  # tag bit of its items on tensors that are not FAST2D
 STEP_SUMS, STEP_FACTORS, STEP_STATE, STEP_MOMENTS, STEP_PREP, STEP_APPLY, STEP_APPLY_REST = (1 << k for k in range(7))

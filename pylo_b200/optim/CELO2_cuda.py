@@ -281,10 +281,11 @@ class _Celo2Family(Optimizer):
             prm = self._params_struct(group, gnorm_ptr)
             clip_norm = float(group["clip_norm"]) if group["clip_grad"] else 0.0
             lr, wd = group_floats(group, "lr", "weight_decay")
+            tail = ()   # what the matrices' last launch still has to do, where it waits for AdamW's
             if plan["lo"] is not None:
-                self._lo_step(group, plan, [g for g, lo in zip(grads, plan["in_lo"]) if lo], prm, clip_norm, lr, wd, stream)
+                tail = self._lo_step(group, plan, [g for g, lo in zip(grads, plan["in_lo"]) if lo], prm, clip_norm, lr, wd, stream)
             if plan["adam"] is not None:
-                self._adam_step(group, plan, [g for g, lo in zip(grads, plan["in_lo"]) if not lo], prm, clip_norm, lr, stream)
+                self._adam_step(group, plan, [g for g, lo in zip(grads, plan["in_lo"]) if not lo], prm, clip_norm, lr, stream, tail)
             if self.after_group is not None:
                 self.after_group(gi)
         return loss
@@ -320,9 +321,12 @@ class _Celo2Family(Optimizer):
             plan["post_key"] = key
         if not squares:
             L.check(L.lib.pylo_b200_celo2_post_sums(post.table.ptr, post.tiles.ptr, post.n_tiles, stream), "celo2_post_sums")
-        L.check(L.lib.pylo_b200_celo2_post_apply(post.table.ptr, post.tiles.ptr, post.n_tiles, lo.step_plan.status,
-                                                 lo.step_plan.host_status, stream), "celo2_post_apply")
         self._keep = keep
+        tail = (post.table.ptr, post.tiles.ptr, post.n_tiles, lo.step_plan.status, lo.step_plan.host_status)
+        if plan["adam"] is not None and post.n_tiles + plan["adam"].n_tiles <= L.TAIL_ONE_LAUNCH:
+            return tail
+        L.check(L.lib.pylo_b200_celo2_post_apply(*tail, stream), "celo2_post_apply")
+        return ()
 
     def _orthogonalise(self, plan, stream):
         """Newton-Schulz over the plan's stacks of raw steps: (the results to keep alive, address of every tensor's)."""
@@ -355,7 +359,7 @@ class _Celo2Family(Optimizer):
                     steps[ti] = at + n * j
         return keep, steps
 
-    def _adam_step(self, group, plan, grads, prm, clip_norm, lr, stream):
+    def _adam_step(self, group, plan, grads, prm, clip_norm, lr, stream, tail=()):
         adam: ItemPlan = plan["adam"]
         it = adam.items
         ptrs = grad_pointers(grads)
@@ -381,8 +385,9 @@ class _Celo2Family(Optimizer):
             adam.upload()
             plan["adam_key"] = key
         bc1, bc2 = (1.0 - b1 ** ts[0], 1.0 - b2 ** ts[0]) if same else (0.0, 0.0)
-        L.check(L.lib.pylo_b200_adamw(adam.table.ptr, adam.tiles.ptr, adam.n_tiles, int(not self._shared_adam),
-                                      b1, 1 - b1, b2, 1 - b2, eps, bc1, bc2, C.byref(prm), stream), "adamw")
+        launch = L.lib.pylo_b200_celo2_tail if tail else L.lib.pylo_b200_adamw
+        L.check(launch(*tail, adam.table.ptr, adam.tiles.ptr, adam.n_tiles, int(not self._shared_adam),
+                       b1, 1 - b1, b2, 1 - b2, eps, bc1, bc2, C.byref(prm), stream), "adamw")
         self._keepg = copies
 
 
