@@ -487,7 +487,7 @@ typedef struct pylo_step_plan {
   const pylo_atile *atiles, *gitems, *pitems, *ctiles;
   const pylo_tile *tiles, *tiles_slow;
   const pylo_atile* rtiles; /* CELO2, VELO: items of apply_packed on matrices with tables whose rows are not aligned */
-  const int32_t* mats;      /* the tensors that are not VEC1D */
+  const int32_t* mats;      /* the n_mats tensors that are not VEC1D, or NULL: the first n_mats */
   int *status, *host_status;
   int32_t n_tensors, n_units, n_atiles, n_gitems, n_pitems, n_ctiles, n_ctiles_gen, n_tiles, n_tiles_slow, tensor_cores;
   int32_t sum_tiles; /* 1: leave finalize_moments out and let prep_apply add up the tile partials, for units of up to

@@ -172,6 +172,7 @@ lib, EXPORTED = _load()
 SM_COUNT = 148        # of a B200; sizes of work lists only, the kernels ask the device
 VELO_INPUTS_MOST = 16  # tensors that pylo_b200_velo_inputs takes, and their tiles
 TAIL_ONE_LAUNCH = 592  # tiles of CELO2's tail and AdamW up to which they share a launch
+FACTOR_CLUSTER = 8  # CTAs per tensor of pylo_b200_factor_update
 TC_WORKERS = SM_COUNT * 4  # warpgroups the tensor-core apply kernel runs at once (four per SM)
 TC_GEN_ITEM = 1 << 16  # tag bit of its items on tensors that are not FAST2D
 STEP_SUMS, STEP_FACTORS, STEP_STATE, STEP_MOMENTS, STEP_PREP, STEP_APPLY, STEP_APPLY_REST = (1 << k for k in range(7))

@@ -326,10 +326,11 @@ def small_front(mats: Sequence[Tuple[int, int]], vectors: Sequence[int]):
 
 
 def small_networks(n_tensors: int, cluster: int) -> bool:
-    """Whether one more cluster of this size, which makes the networks of the tensor-core sweep, costs no further turn: a cluster lies
-    in one of eight groups of at least 18 SMs."""
+    """Whether one more cluster of this size makes the networks of the tensor-core sweep: where each of its CTAs has two at most (they
+    take 3 us each, the tensors' own work 11; the 101 vectors of a ViT-B/16 in clusters of two CTAs: 170 us), and it costs no
+    further turn: a cluster lies in one of eight groups of at least 18 SMs."""
     at_once = 8 * (18 // cluster)
-    return -(-(n_tensors + 1) // at_once) == -(-n_tensors // at_once)
+    return n_tensors <= 2 * cluster and -(-(n_tensors + 1) // at_once) == -(-n_tensors // at_once)
 
 
 class SumOrder(NamedTuple):
@@ -583,7 +584,8 @@ class LoPlan:
         #: everything pylo_b200_step needs for a step over these tensors
         self.step_plan = L.StepPlan(
             tdesc=self.tdesc.ptr, desc=self.desc.ptr, atiles=self.atiles.ptr, gitems=self.gitems.ptr, pitems=self.pitems.ptr,
-            ctiles=self.ctiles.ptr, tiles=self.tiles.ptr, tiles_slow=self.tiles_slow.ptr, rtiles=self.rtiles.ptr, mats=self.mats.ptr, n_mats=self.n_mats,
+            ctiles=self.ctiles.ptr, tiles=self.tiles.ptr, tiles_slow=self.tiles_slow.ptr, rtiles=self.rtiles.ptr, mats=self.mats.ptr if T * L.FACTOR_CLUSTER > L.SM_COUNT else 0,
+            n_mats=self.n_mats if T * L.FACTOR_CLUSTER > L.SM_COUNT else T,   # few tensors: all of them, which costs nothing
             status=self.status.data_ptr(), host_status=self._status_host.data_ptr(),
             n_tensors=T, n_units=U, n_atiles=self.n_atiles, n_gitems=self.n_gitems, n_pitems=self.n_pitems,
             n_ctiles=self.n_ctiles, n_ctiles_gen=self.n_ctiles_gen, n_tiles=self.n_tiles, n_tiles_slow=self.n_tiles_slow, n_ragged=self.n_ragged, n_rtiles=self.n_rtiles,
@@ -681,7 +683,7 @@ class LoPlan:
         fast = self.n_atiles - self.n_ragged
         joined = self.step_plan.n_kernel > 0 or 0 < fast <= L.ROWCOL_ONE_LAUNCH   # the generic items go with the others
         front = [(L.STEP_SUMS, "rowcol_sums", (self.n_ragged > 0) + (fast > 0) + int(self.n_gitems > 0 and not joined)),
-                 (L.STEP_FACTORS, "factor_update", int(self.n_mats > 0)),
+                 (L.STEP_FACTORS, "factor_update", int(self.step_plan.n_mats > 0)),
                  (L.STEP_STATE, "state_moments", 1)]
         if self.small:
             front = [(L.STEP_SUMS | L.STEP_FACTORS | L.STEP_STATE, "small_front", 1)]
