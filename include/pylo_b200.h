@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define PYLO_B200_ABI_VERSION 18
+#define PYLO_B200_ABI_VERSION 19
 
 /* optimizer families (which feature set / network geometry a launch uses) */
 #define PYLO_FAM_ADAFAC 0 /* AdafacLO_CUDA, ELO_CUDA: 28+11 features, 39-32-32-2 */
@@ -239,8 +239,9 @@ int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atile
 /* Phase A2, one cluster of CTAs per tensor: the sums over strips and column blocks of phase A's partials, EMA of the factored accumulators, row_col_mean,
  * row/column rsqrt factors (AdafacLO_cuda.py:342-345, CELO2_cuda.py:229-231, velo_cuda.py:716-729)
  * and the closed-form feature moments of the twelve vector-only features.  mats: DEVICE list of the n_tensors tensors to take (VEC1D ones
- * have nothing to do, as long as their `closed` is zero), or NULL for the first n_tensors. */
-int pylo_b200_factor_update(const pylo_tensor_desc* descs, const int32_t* mats, int n_tensors, const pylo_step_params* prm,
+ * have nothing to do, as long as their `closed` is zero), or NULL for the first n_tensors.  threads: 1024 or 512 per CTA, which decides
+ * the order of the sums; 512 is faster for more tensors than run at once (eight CTAs each). */
+int pylo_b200_factor_update(const pylo_tensor_desc* descs, const int32_t* mats, int n_tensors, int threads, const pylo_step_params* prm,
                             void* stream);
 
 /* Phase B: momentum / second-moment EMA in place and per-tile sums of squares of
@@ -498,6 +499,8 @@ typedef struct pylo_step_plan {
   int32_t n_kernel; /* of atiles, those behind the first n_ragged that are on KERNEL tensors */
   int32_t n_mats;
   int32_t small_networks; /* clusters of small_front that make the networks; > 0: no prep_apply (ADAFAC with tensor_cores) */
+  int32_t factor_threads; /* of factor_update */
+  int32_t pad_;
 } pylo_step_plan;
 int pylo_b200_step(const pylo_step_plan* plan, const pylo_step_params* prm, int phases, void* stream);
 /* Host only: adds 1 to n step counters (HOST pointers to doubles); first: the old value of the first, equal: whether all

@@ -17,7 +17,7 @@ TILE_ELEMS = 16384
 A_COLS = 1024
 PREP_TABLE = 2048  # table entries (rows x hidden units) per item of pylo_b200_prep_apply
 WFOLD_STRIDE = 4800
-ABI_VERSION = 18
+ABI_VERSION = 19
 
 FAM_ADAFAC, FAM_CELO2, FAM_VELO = 0, 1, 2
 MODE_FAST2D, MODE_GENERIC, MODE_VEC1D, MODE_KERNEL = 0, 1, 2, 3
@@ -102,7 +102,7 @@ class StepPlan(C.Structure):
         "tdesc", "desc", "atiles", "gitems", "pitems", "ctiles", "tiles", "tiles_slow", "rtiles", "mats", "status", "host_status")] + [
         (name, C.c_int32) for name in ("n_tensors", "n_units", "n_atiles", "n_gitems", "n_pitems", "n_ctiles", "n_ctiles_gen",
                                        "n_tiles", "n_tiles_slow", "tensor_cores", "sum_tiles", "n_ragged", "n_rtiles", "small_cluster", "small_slice",
-                                       "small_rows", "small_cols", "n_kernel", "n_mats", "small_networks")]
+                                       "small_rows", "small_cols", "n_kernel", "n_mats", "small_networks", "factor_threads", "pad_")]
 
 
 class PyloLibError(RuntimeError):
@@ -129,7 +129,7 @@ def _load():
         "pylo_b200_grad_sumsq": [vp, vp, i32, vp, vp, vp],
         "pylo_b200_grad_sumsq_static": [vp, vp, i32, vp, vp],
         "pylo_b200_rowcol_sums": [vp, vp, i32, i32, i32, vp, i32, C.POINTER(StepParams), vp],
-        "pylo_b200_factor_update": [vp, vp, i32, C.POINTER(StepParams), vp],
+        "pylo_b200_factor_update": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_state_moments": [vp, vp, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_small_front": [vp, i32, i32, i32, i32, i32, i32, C.POINTER(StepParams), vp],
         "pylo_b200_finalize_moments": [vp, i32, vp],

@@ -317,16 +317,19 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
       if (!ARG && col < 64) sm.w3[col] = __ldg(d.wfold + L::W3P + col);
       if (!ARG && col < 2) sm.w3[64 + col] = __ldg(d.wfold + L::B3 + col);
       loaded = ct.tensor;
-      // small models: k_small_front has left the network and the partial sums of squares; the features' scales are made here
+      // small models: k_small_front has left the network and the partial sums of squares; the features' scales are made here, the
+      // partials added up as unit_sum does
       if (GENERIC && prm.no_tables == 4) {
         double(*const part)[32] = reinterpret_cast<double(*)[32]>(sm.row);
+        static_assert(TC_SUM_ROWS == 4, "a warp per row");
         const int q = warp & 3, j = col & 31, f = tc_slot_feature(j < F::NF ? j : 0, tc_swap(d));
-        double acc = q == 0 ? (double)d.closed[f] : 0.0;
-        for (int t = q; t < d.n_tiles; t += 4) acc += (double)d.tile_part[(int64_t)t * PYLO_STAT_STRIDE + f];
+        const float closed = d.closed[f];
+        double acc = 0.0;
+        for (int t = q; t < d.n_tiles; t += TC_SUM_ROWS) acc += (double)d.tile_part[(int64_t)t * PYLO_STAT_STRIDE + f];
         part[q][j] = acc;
         wg_barrier(wg);
         if (col < F::NF) {
-          const float tot = (float)(part[0][col] + part[1][col] + part[2][col] + part[3][col]);
+          const float tot = (float)(part[0][col] + part[1][col] + part[2][col] + part[3][col] + (double)closed);
           sm.img.sn[col] = rsqrtf(tot / (float)n + prm.eps_norm) * sm.img.sn[F::NF + 1];
           if (ct.strip == 0 && ct.cb == 0) d.sums[f] = tot;
         }

@@ -322,7 +322,9 @@ __global__ void __launch_bounds__(NT) k_rowcol_generic(const pylo_tensor_desc* _
 // A and the factors need the mean of the whole vector.  Eight CTAs share the tensor (one CTA took 185 us for the 50257
 // rows of a GPT-2 embedding) and exchange their partial sums through distributed shared memory; every CTA adds the eight
 // in rank order, so the result does not depend on timing.  The sum over the strips is part of this kernel: 128 columns
-// per pass, the strips dealt to eight groups of 128 threads.
+// per pass (512 where there are enough), the strips dealt to eight groups of 128 threads, or to four: a CTA has A2_NT threads, or half
+// of them where the model has more clusters than run at once, which then share the SMs two and two, so that one's barriers and
+// latencies are another's time.  The number of threads decides the order of the sums; the host takes it from the whole model (sum_order).
 // ================================================================================================
 #define A2_NT 1024
 #define A2_CL 8
@@ -1000,6 +1002,7 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
 // sums by 2^-TC_SHIFT as it adds the bias.  A plane's last bit is 2^-25 of the scaled unit: of a feature 2^-(25 + q) of its root mean square
 // (q = 3 at 16 M elements), of a weight 2^-(25 + a), a = 7 to 10.
 #define TC_SHIFT 10
+#define TC_SUM_ROWS 4   // of unit_sum, for what k_small_front leaves (up to 16 tiles): as the sweep's warpgroups do it where they add the partials up
 // where a unit's column has features of its own for all rows (FAST2D, KERNEL), those come first
 __device__ __forceinline__ bool tc_swap(const pylo_tensor_desc& d) { return (d.mode == PYLO_MODE_FAST2D || d.mode == PYLO_MODE_KERNEL) && d.r_is_a; }
 __constant__ float TIME_SCALES[11] = {1.f, 3.f, 10.f, 30.f, 100.f, 300.f, 1000.f, 3000.f, 10000.f, 30000.f, 100000.f};
@@ -1122,7 +1125,7 @@ __global__ void __launch_bounds__(NT) k_prep_tc(const pylo_tensor_desc* __restri
   constexpr int NF = Fam<PYLO_FAM_ADAFAC>::NF;
   __shared__ TcNet s;
   __shared__ float s_scale[NF];
-  __shared__ double s_d[6][PYLO_STAT_STRIDE];
+  __shared__ double s_d[6][PYLO_STAT_STRIDE], s_few[TC_SUM_ROWS][PYLO_STAT_STRIDE];
   const pylo_atile it = items[blockIdx.x];
   if (it.strip) return;   // the whole CTA
   const pylo_tensor_desc& d = descs[it.tensor];
@@ -1130,7 +1133,7 @@ __global__ void __launch_bounds__(NT) k_prep_tc(const pylo_tensor_desc* __restri
   tc_ask_network<NT>(d, s);
   const float n = (float)d.n;
   if (prm.sum_tiles) {
-    const double tot = unit_sum<6>(d, s_d);
+    const double tot = d.n_tiles <= 16 ? unit_sum<TC_SUM_ROWS>(d, s_few) : unit_sum<6>(d, s_d);
     if (tid < NF) s_scale[tid] = rsqrtf((float)tot / n + prm.eps_norm);
     if (tid < PYLO_STAT_STRIDE) store_unit_sum(d, tot);
   } else if (tid < NF) {
@@ -2671,10 +2674,9 @@ static int ns_gemm(nf_group& grp, int* status, cudaStream_t s) {
   return ns_launch<NfSmem<128, false>, k_gemm_f16x2>(grp, (int)(tiles < sms ? tiles : sms), status, s);
 }
 
-// More clusters than run at once share the SMs two and two, so that one's barriers and latencies are another's time.
 template <int FAM>
-static void factor_update_launch(const pylo_tensor_desc* descs, const int32_t* mats, int n, const pylo_step_params& prm, cudaStream_t s) {
-  if (n * A2_CL <= sm_count()) launch(k_factor_update<FAM, A2_NT>, n * A2_CL, A2_NT, 0, s, descs, mats, prm);
+static void factor_update_launch(const pylo_tensor_desc* descs, const int32_t* mats, int n, int threads, const pylo_step_params& prm, cudaStream_t s) {
+  if (threads == A2_NT) launch(k_factor_update<FAM, A2_NT>, n * A2_CL, A2_NT, 0, s, descs, mats, prm);
   else launch(k_factor_update<FAM, A2_NT / 2>, n * A2_CL, A2_NT / 2, 0, s, descs, mats, prm);
 }
 
@@ -2958,14 +2960,14 @@ int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atile
   return launch_status();
 }
 
-int pylo_b200_factor_update(const pylo_tensor_desc* descs, const int32_t* mats, int n_tensors, const pylo_step_params* prm, void* stream) {
-  CHECK_ARG(descs && prm && n_tensors >= 0);
+int pylo_b200_factor_update(const pylo_tensor_desc* descs, const int32_t* mats, int n_tensors, int threads, const pylo_step_params* prm, void* stream) {
+  CHECK_ARG(descs && prm && n_tensors >= 0 && (threads == A2_NT || threads == A2_NT / 2));
   if (n_tensors == 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   switch (prm->family) {
-    case PYLO_FAM_ADAFAC: factor_update_launch<PYLO_FAM_ADAFAC>(descs, mats, n_tensors, *prm, s); break;
-    case PYLO_FAM_CELO2: factor_update_launch<PYLO_FAM_CELO2>(descs, mats, n_tensors, *prm, s); break;
-    case PYLO_FAM_VELO: factor_update_launch<PYLO_FAM_VELO>(descs, mats, n_tensors, *prm, s); break;
+    case PYLO_FAM_ADAFAC: factor_update_launch<PYLO_FAM_ADAFAC>(descs, mats, n_tensors, threads, *prm, s); break;
+    case PYLO_FAM_CELO2: factor_update_launch<PYLO_FAM_CELO2>(descs, mats, n_tensors, threads, *prm, s); break;
+    case PYLO_FAM_VELO: factor_update_launch<PYLO_FAM_VELO>(descs, mats, n_tensors, threads, *prm, s); break;
     default: return -2;
   }
   return launch_status();
@@ -3419,7 +3421,7 @@ int pylo_b200_step(const pylo_step_plan* p, const pylo_step_params* prm, int pha
   if ((phases & PYLO_STEP_SUMS) && (p->n_atiles || p->n_gitems))
     if ((rc = pylo_b200_rowcol_sums(p->tdesc, p->atiles, p->n_atiles, p->n_ragged, p->n_kernel, p->gitems, p->n_gitems, prm, stream))) return rc;
   if (phases & PYLO_STEP_FACTORS)
-    if ((rc = pylo_b200_factor_update(p->tdesc, p->mats, p->n_mats, prm, stream))) return rc;
+    if ((rc = pylo_b200_factor_update(p->tdesc, p->mats, p->n_mats, p->factor_threads, prm, stream))) return rc;
   if (phases & PYLO_STEP_STATE)
     if ((rc = pylo_b200_state_moments(p->desc, p->tiles, p->n_tiles, 1, prm, stream))) return rc;
   if ((phases & PYLO_STEP_STATE) && p->small_networks) {   // the phases one by one: what the launch of all of them would have left

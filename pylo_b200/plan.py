@@ -340,6 +340,7 @@ class SumOrder(NamedTuple):
     elems: int          # elements of a tile where that does not cut the tensors
     sum_tiles: bool     # no launch for phase B2: of small units phase P adds the tile partials up, for VeLO the LSTM's input kernel does
     bulk_copies: bool   # the state sweep reads through a ring of bulk copies
+    factor_threads: int = 1024   # per CTA of the factor phase
 
     def tiles(self, sizes):
         return equal_tiles(sizes, self.small[0]) if self.small else make_tiles(sizes, self.elems)
@@ -352,7 +353,9 @@ def sum_order(family: int, d: np.ndarray, sizes: Sequence[int], modes: np.ndarra
 
     The state sweep's ring of bulk copies leaves little L1 cache to the units that are not FAST2D and keeps the launches around it
     apart, so it has to have enough to do: from 64 M elements on (VeLO on 100 M: 1615 -> 1580 us per step, on 17 M: 341 -> 351;
-    AdafacLO on 25 M: 837 -> 851, on 86 M even), nearly all of them FAST2D."""
+    AdafacLO on 25 M: 837 -> 851, on 86 M even), nearly all of them FAST2D.
+
+    The factor phase has a cluster of eight CTAs per tensor with factors: half as many threads each where not all run at once."""
     total, small = int(sum(sizes)), None
     if not sliced and total <= 2 * SMALL_CTAS * L.SMALL_SLICE:
         vectors = d["mode"] == L.MODE_VEC1D
@@ -361,7 +364,9 @@ def sum_order(family: int, d: np.ndarray, sizes: Sequence[int], modes: np.ndarra
     elems = state_tile(sizes)
     most = small[0] if small else -(-max(sizes, default=0) // elems)
     fast = int(sum(n for n, m in zip(sizes, modes.tolist()) if m == L.MODE_FAST2D))
-    return SumOrder(small, elems, family == L.FAM_VELO or most <= SUM_TILES_MOST, fast >= L.BULK_COPY_ELEMS and 8 * fast >= 7 * total)
+    together = int((d["mode"] != L.MODE_VEC1D).sum()) * L.FACTOR_CLUSTER <= L.SM_COUNT
+    return SumOrder(small, elems, family == L.FAM_VELO or most <= SUM_TILES_MOST, fast >= L.BULK_COPY_ELEMS and 8 * fast >= 7 * total,
+                    1024 if together else 512)
 
 
 def model_shapes(params) -> Optional[Sequence[Tuple[int, ...]]]:
@@ -589,7 +594,7 @@ class LoPlan:
             status=self.status.data_ptr(), host_status=self._status_host.data_ptr(),
             n_tensors=T, n_units=U, n_atiles=self.n_atiles, n_gitems=self.n_gitems, n_pitems=self.n_pitems,
             n_ctiles=self.n_ctiles, n_ctiles_gen=self.n_ctiles_gen, n_tiles=self.n_tiles, n_tiles_slow=self.n_tiles_slow, n_ragged=self.n_ragged, n_rtiles=self.n_rtiles,
-            n_kernel=sum(len(a) for a in katiles),
+            n_kernel=sum(len(a) for a in katiles), factor_threads=order.factor_threads,
             tensor_cores=int(self.tensor_cores), sum_tiles=int(self.sum_tiles))
         if self.small:
             (self.step_plan.small_cluster, self.step_plan.small_slice, self.step_plan.small_rows, self.step_plan.small_cols) = self.small
