@@ -13,7 +13,7 @@
 //   * fp32 accuracy is kept by splitting every operand into two fp16 planes (11 + 11 significant bits) and running
 //     three products per layer and K step (hi x hi, hi x lo, lo x hi) into one accumulator of 32 columns.  The features
 //     are normalised before they are split: over its root mean square no feature exceeds sqrt(n), so that powers of two
-//     can be found that keep both layers' operands in fp16's range for any gradient (k_prep_tc).  Operand
+//     can be found, for every hidden unit, that keep both layers' operands in fp16's range for any gradient (tc_network).  Operand
 //     B holds the high planes in rows 0..31 and the low planes in rows 32..63 of one block; a product addresses
 //     either half through its descriptor's start address;
 //   * a layer's last product is of a constant operand A (in shared memory) with a block that holds the bias; the tensor

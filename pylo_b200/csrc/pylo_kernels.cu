@@ -997,10 +997,13 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
 //
 // Operands are two fp16 planes, so every operand gets a power of two that keeps it inside fp16's range whatever the gradients are.
 // A feature over its root mean square is at most sqrt(n) (all of the tensor's sum of squares in one element), so 2^q sqrt(n) <= 2^15;
-// a first-layer sum is at most its weights' magnitudes times sqrt(n), plus the bias, so 2^e1 times that is <= 2^15; and weights are
+// a hidden unit's first-layer sum is at most its weights' magnitudes times sqrt(n), plus the bias, so 2^e1 times that is <= 2^15, with
+// an e1 for every unit, which its column of the second layer undoes; and weights are
 // taken as large as they go, up to 2^a = 2^(e1 + TC_SHIFT - q): the shift between is undone by the tensor core, which scales the
-// sums by 2^-TC_SHIFT as it adds the bias.  A plane's last bit is 2^-25 of the scaled unit: of a feature 2^-(25 + q) of its root mean square
-// (q = 3 at 16 M elements), of a weight 2^-(25 + a), a = 7 to 10.
+// sums by 2^-TC_SHIFT as it adds the bias.  What a network's units are scaled by (by s, and their columns by 1 / s) therefore changes
+// nothing: with one e1 for all units, the largest one's, half of the units times 1e-4 were off by 5e-6 to 5e-5 of the sum of the terms'
+// magnitudes at 16 M elements, now 5e-9 to 2e-8 (restated on the CPU, normal and heavy-tailed features).  A plane's last bit is 2^-25 of the scaled unit: of a feature 2^-(25 + q) of its root mean square
+// (q = 6 up to 65 K elements, 2 at 16 M, 0 at 268 M), of a unit's activation 2^-(25 + e1), i.e. 2^-39 or less of its largest possible one.
 #define TC_SHIFT 10
 #define TC_SUM_ROWS 4   // of unit_sum, for what k_small_front leaves (up to 16 tiles): as the sweep's warpgroups do it where they add the partials up
 // where a unit's column has features of its own for all rows (FAST2D, KERNEL), those come first
@@ -1015,12 +1018,12 @@ __device__ __forceinline__ uint32_t tc_plane(float x, float scale, float& rest) 
   rest = (x - __half2float(h)) * scale;
   return __half_as_ushort(h);
 }
-// The network's part of a unit's TcImage, and in sn[28] and [29] the scale of the second layer's sums and that of the features.  Called
+// The network's part of a unit's TcImage, and in sn[28] and [29] what undoes the scale of the second layer's sums and that of the features.  Called
 // by all of a CTA's THREADS threads with room for TcNet in shared memory; the network is asked for by the caller (tc_ask_network).
 struct TcNet {
   static constexpr int H = 32, NIN = 39, o_b1 = NIN * H, o_w2 = o_b1 + H, o_b2 = o_w2 + H * H, o_w3 = o_b2 + H, o_b3 = o_w3 + 2 * H, o_end = o_b3 + 2;
   float net[o_end + H];   // the second layer's rows are H + 1 apart, so that lanes on different rows do not collide
-  float b1[H], pow[6];
+  float b1[H], row[H], column[H], pow[3];   // first layer's bias (scaled), scales of its rows and of the second layer's columns; see below
   float part[4][NT / 32][32];
   __host__ __device__ static constexpr int at(int e) { return e < o_w2 ? e : e < o_b2 ? e + (e - o_w2) / H : e + H; }
 };
@@ -1047,7 +1050,7 @@ __device__ __forceinline__ void tc_network(const pylo_tensor_desc& d, const pylo
       most = fmaxf(most, a);
     }
     for (int t = part; t < 11; t += PARTS) time = fmaf(s.net[lane * N::NIN + NF + t], tanhf(step / TIME_SCALES[t] - 1.0f), time);
-    for (int k = part; k < H; k += PARTS) most2 = fmaxf(most2, fabsf(s.net[N::o_w2 + lane * (H + 1) + k]));
+    for (int k = part; k < H; k += PARTS) most2 = fmaxf(most2, fabsf(s.net[N::o_w2 + k * (H + 1) + lane]));   // of the unit's column
     s.part[0][part][lane] = sum; s.part[1][part][lane] = most; s.part[2][part][lane] = most2; s.part[3][part][lane] = time;
   }
   __syncthreads();
@@ -1059,29 +1062,21 @@ __device__ __forceinline__ void tc_network(const pylo_tensor_desc& d, const pylo
       most2 = fmaxf(most2, s.part[2][q][lane]);
       b1 += s.part[3][q][lane];
     }
-    s.b1[lane] = b1;
-    const float spread = sqrtf((float)d.n) * 1.001f;
-    float bound = fmaf(sum, spread, fabsf(b1)), b2 = fabsf(s.net[N::at(N::o_b2 + lane)]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      bound = fmaxf(bound, __shfl_xor_sync(0xffffffffu, bound, o));
-      most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
-      most2 = fmaxf(most2, __shfl_xor_sync(0xffffffffu, most2, o));
-      b2 = fmaxf(b2, __shfl_xor_sync(0xffffffffu, b2, o));
-    }
+    const float spread = sqrtf((float)d.n) * 1.001f, bound = fmaf(sum, spread, fabsf(b1));
     const int q = min(6, tc_room(spread));
-    const int a = min(min(6, tc_room(bound)) + TC_SHIFT - q, tc_room(most)), e1 = a + q - TC_SHIFT;
-    const int a2 = min(tc_room(most2) - 1, tc_room(b2) + TC_SHIFT - e1), e2 = e1 + a2 - TC_SHIFT;
-    if (lane == 0) {
-      s.pow[0] = tc_pow2(q); s.pow[1] = tc_pow2(a); s.pow[2] = tc_pow2(e1); s.pow[3] = tc_pow2(a2); s.pow[4] = tc_pow2(e2); s.pow[5] = tc_pow2(-e2);
-    }
+    const int a = min(tc_room(bound) + TC_SHIFT - q, tc_room(most)), e1 = a + q - TC_SHIFT;
+    // second-layer sums times 2^a2: as large as every column's weights, which get 2^(a2 - e1), and the biases allow
+    int a2 = min(tc_room(most2) - 1 + e1, tc_room(fabsf(s.net[N::at(N::o_b2 + lane)])) + TC_SHIFT);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a2 = min(a2, __shfl_xor_sync(0xffffffffu, a2, o));
+    s.b1[lane] = b1 * tc_pow2(e1); s.row[lane] = tc_pow2(a); s.column[lane] = tc_pow2(a2 - e1);
+    if (lane == 0) { s.pow[0] = tc_pow2(q); s.pow[1] = tc_pow2(a2 - TC_SHIFT); s.pow[2] = tc_pow2(TC_SHIFT - a2); }
   }
   __syncthreads();
   TcImage& o = *reinterpret_cast<TcImage*>(d.wfold + TC_IMAGE);
   const bool swap = tc_swap(d);
   if (tid < 256) {  // both layers: a thread makes eight weights of one hidden unit, 16 bytes of each plane
     const int layer = tid >> 7, kc = part & 3;
-    const float scale = s.pow[layer ? 3 : 1];
     uint32_t hi[4], lo[4];
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
@@ -1091,7 +1086,7 @@ __device__ __forceinline__ void tc_network(const pylo_tensor_desc& d, const pylo
         const int k = kc * 8 + i + u;
         const float x = layer ? s.net[N::o_w2 + lane * (H + 1) + k] : k < NF ? s.net[lane * N::NIN + tc_slot_feature(k, swap)] : 0.f;
         float rest, none;
-        h[u] = tc_plane(x * scale, 1.f, rest);
+        h[u] = tc_plane(x * (layer ? s.column[k] : s.row[lane]), 1.f, rest);
         l[u] = tc_plane(rest, 0.f, none);
       }
       hi[i / 2] = h[0] | h[1] << 16;
@@ -1104,13 +1099,13 @@ __device__ __forceinline__ void tc_network(const pylo_tensor_desc& d, const pylo
   if (part < 4) {
     const int layer = part >> 1, kc = part & 1;
     float rest, none;
-    uint32_t word = tc_plane(layer ? s.net[N::at(N::o_b2 + lane)] * s.pow[4] : s.b1[lane] * s.pow[2], 2048.f, rest);
+    uint32_t word = tc_plane(layer ? s.net[N::at(N::o_b2 + lane)] * s.pow[1] : s.b1[lane], 2048.f, rest);
     word |= tc_plane(rest, 0.f, none) << 16;
     char* b = reinterpret_cast<char*>(layer ? o.bias2 : o.bias1) + kc * 512 + (lane >> 3) * 128 + (lane & 7) * 16;
     *reinterpret_cast<uint4*>(b) = make_uint4(kc ? 0u : word, 0u, 0u, 0u);
   } else if (part == 4) {
     if (lane < 2) {
-      o.sn[NF + lane] = s.pow[lane ? 0 : 5];
+      o.sn[NF + lane] = s.pow[lane ? 0 : 2];
       d.wfold[L::B3 + lane] = s.net[N::at(N::o_b3 + lane)];
     }
     if (lane == 2) d.wfold[L::SC + 1] = d.lr_mult ? d.lr * d.lr_mult[0] : d.lr;
