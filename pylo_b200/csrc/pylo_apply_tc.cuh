@@ -161,23 +161,20 @@ constexpr uint32_t TC_IDESC = (1u << 4) | ((32u >> 3) << 17) | ((128u >> 4) << 2
 #define TC_CLK_FLUSH
 #endif
 
-// Two values as fp16 planes: hi the values cut to 11 significant bits, lo what that leaves, rounded; packed, the first value in the
-// lower half.  RELU: of the values' positive parts: a cut value and what the cut leaves have the value's sign, so both conversions clamp
-// at zero by themselves.  The rest is x + (-(x & mask)), the mask and sign flip being one three-input logic operation.
+// Two values as fp16 planes: hi the values cut to fp16, lo what that leaves, rounded; packed, the first value in the
+// lower half.  RELU: of the values' positive parts: the high plane of a negative value is zero and what it leaves negative, so both
+// conversions clamp at zero by themselves.
 template <bool RELU>
 __device__ __forceinline__ void tc_split2(uint64_t x, uint32_t& hi, uint32_t& lo) {
   float a, b;
   unpack2(x, a, b);
-  auto cut = [](float v) { return __uint_as_float((__float_as_uint(v) & 0xffffe000u) ^ 0x80000000u); };
+  if constexpr (RELU) asm("cvt.rz.relu.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
+  else asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
+  const float2 cut = __half22float2(*reinterpret_cast<const __half2*>(&hi));
   float ra, rb;
-  unpack2(add2(x, pack2(cut(a), cut(b))), ra, rb);
-  if constexpr (RELU) {
-    asm("cvt.rz.relu.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
-    asm("cvt.rn.relu.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(rb), "f"(ra));
-  } else {
-    asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
-    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(rb), "f"(ra));
-  }
+  unpack2(add2(x, pack2(-cut.x, -cut.y)), ra, rb);
+  if constexpr (RELU) asm("cvt.rn.relu.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(rb), "f"(ra));
+  else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(rb), "f"(ra));
 }
 
 // One warpgroup's private shared memory: its copy of the weights and its tensor-core barrier.  Warpgroups never

@@ -123,3 +123,35 @@ def test_units_with_scales_of_their_own(shape, units, kind):
 @pytest.mark.parametrize("shape", [(4096, 14336), (32000, 4096)])
 def test_large_tensors(shape, kind, grad):
     _check(*_run(shape, grad, kind, 16))
+
+
+@pytest.mark.parametrize("shape", [(64, 128), (37, 53), (1024, 1024), (64, 48, 3, 3)])
+def test_small_values_are_rounded_not_cut(shape):
+    """A network that hands one feature through, and a gradient whose entries but one lie below fp16's normal range after scaling: what
+    the two planes hold is within half of fp16's smallest step, whichever way."""
+    from pylo_b200 import models, optim
+
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    net = models.MetaMLP(39, 32, 1)
+    with torch.no_grad():
+        for w in net.parameters():
+            w.zero_()
+        w1, _, w2, _, w3, _ = net.parameters()
+        w1[0, 0] = w2[0, 0] = w3[0, 0] = 1.0
+    p = torch.nn.Parameter(torch.zeros(*shape, device="cuda"))
+    n = p.numel()
+    q = min(6, 14 - math.floor(math.log2(1.001 * math.sqrt(n))))
+    rms = 10.0
+    g = torch.rand(shape, device="cuda", generator=gen) * (rms * 2.0 ** (-14 - q))
+    g.view(-1)[n // 3] = rms * math.sqrt(n)
+    p.grad = g
+    opt = optim.AdafacLO_CUDA([p], lr=LR, network=net)
+    opt.step()
+    opt.check_status()
+    scale = 1.0 / math.sqrt(float(g.double().pow(2).mean()) + 1e-5)
+    got = -p.detach().double() / (LR * float(opt.step_mult))
+    error = (got - g.double() * scale).view(-1)
+    error[n // 3] = 0.0
+    half = 2.0 ** (-25 - q)
+    assert float(error.abs().max()) <= 1.01 * half, float(error.abs().max()) / half
+    assert abs(float(error.mean())) <= 0.1 * half
