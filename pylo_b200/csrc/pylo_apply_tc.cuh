@@ -346,9 +346,9 @@ __global__ void __launch_bounds__(TC_BOUND_THREADS, 1) k_apply_adafac_tc(const p
     if constexpr (!GEN)
       if (colok) planes6(16, fc[0], fc[1], fc[2], chi, clo);
     TC_CLK(7)  // item set-up
-#pragma unroll 1
     const float* rec = nullptr;   // KERNEL: of this row and this thread's position
     int ready = 0;                // rows ahead whose factors and features are there
+#pragma unroll 1
     for (int x = x0; x < x_end; ++x) {   // the same for the whole warpgroup
       const int i = x - x0;
       if (KERNEL ? ready == 0 : !GEN && (i & (TC_ROWS - 1)) == 0) {   // the next rows' factors and features (the previous ones were read before a barrier)
