@@ -52,7 +52,7 @@ extern "C" {
 #define PYLO_STAT_STRIDE 40  /* floats per tile partial / per tensor sums: 30 feature slots + 8 VeLO statistics */
 #define PYLO_TILE_ELEMS 16384 /* elements per element-wise tile (at most) */
 #define PYLO_A_COLS 1024      /* columns per row/column-sum tile */
-#define PYLO_WFOLD_STRIDE 4800 /* floats reserved per tensor for the folded network and the tensor cores' operands */
+#define PYLO_WFOLD_STRIDE 4800 /* ADAFAC: floats of desc.wfold, the folded network and the tensor cores' operands (the others: see workspace_layout) */
 #define PYLO_SMALL_FLOATS 52224 /* shared memory of pylo_b200_small_front, in floats */
 #define PYLO_MAX_PEERS 7       /* other GPUs of one box */
 
@@ -85,7 +85,7 @@ typedef struct pylo_tensor_desc {
   float* h_b;     /* workspace [H][Lb]: first-layer term of the "b" features */
   float* closed;  /* workspace [PYLO_STAT_STRIDE]: closed-form sums of squares of vector features */
   float* sums;    /* workspace [48]: per-tensor sums (30 feature slots, 8 VeLO statistics, their 8 low-order parts) */
-  float* wfold;   /* workspace [PYLO_WFOLD_STRIDE]: network with normalisers folded in */
+  float* wfold;   /* workspace: network with normalisers folded in; ADAFAC: [PYLO_WFOLD_STRIDE], the tensor cores' operands behind it */
   float* tile_part; /* workspace [n_tiles][PYLO_STAT_STRIDE] */
   float* out;     /* CELO2: raw step output [n]; else NULL */
   const float* w; /* network weights for this tensor, family layout (see pylo_b200_prep_apply) */

@@ -2862,7 +2862,11 @@ int pylo_b200_workspace_layout(int family, int mode, int64_t n, int64_t La, int6
   w.closed = PYLO_STAT_STRIDE;
   w.n_tiles = (int32_t)((n + PYLO_TILE_ELEMS - 1) / PYLO_TILE_ELEMS);
   w.sums = SUMS_STRIDE;
-  w.wfold = PYLO_WFOLD_STRIDE;
+  switch (family) {   // the tensor cores' operands are behind the network for ADAFAC alone; CELO2 has a unit per matrix, down to 3 x 3
+    case PYLO_FAM_ADAFAC: w.wfold = PYLO_WFOLD_STRIDE; break;
+    case PYLO_FAM_CELO2: w.wfold = Fold<PYLO_FAM_CELO2>::SN + Fam<PYLO_FAM_CELO2>::NF; break;
+    default: w.wfold = Fold<PYLO_FAM_VELO>::SN + Fam<PYLO_FAM_VELO>::NF; break;
+  }
   w.tile_part = (int64_t)w.n_tiles * PYLO_STAT_STRIDE;
   *out = w;
   return 0;
