@@ -81,7 +81,8 @@ typedef struct pylo_tensor_desc {
   float* sum_b;   /* workspace [Lb]: sum over X */
   float* part_a;  /* workspace [X][n_cb]  row-sum partials (tensors in atiles; else NULL); KERNEL: [La][2 n_cb] */
   float* part_b;  /* workspace [n_strips][Lb] column-sum partials */
-  float* h_a;     /* workspace [La][H] (ADAFAC) or [La][H][2] (CELO2, VELO): first-layer term of the "a" features (+ bias) */
+  float* h_a;     /* workspace [La][H] (ADAFAC) or [La][H][2] (CELO2, VELO): first-layer term of the "a" features (+ bias); h_a, h_b: NULL
+                     where apply_adafac_tc is the only sweep over the tensor, which reads no tables */
   float* h_b;     /* workspace [H][Lb]: first-layer term of the "b" features */
   float* closed;  /* workspace [PYLO_STAT_STRIDE]: closed-form sums of squares of vector features */
   float* sums;    /* workspace [48]: per-tensor sums (30 feature slots, 8 VeLO statistics, their 8 low-order parts) */

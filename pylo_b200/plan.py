@@ -447,6 +447,8 @@ class LoPlan:
                 kernel = int(d["mode"]) == L.MODE_KERNEL
                 in_atiles = fast or ragged or kernel
                 ws = L.workspace_layout(family, int(d["mode"]), n, La, Lb, X if in_atiles else 0, Lb if in_atiles else 0)
+                if self.tensor_cores:   # the tensor-core sweep reads no tables
+                    ws.h_a = ws.h_b = 0
                 ws_items += [("t", i, f, getattr(ws, f)) for f in ("f_a", "f_b", "sum_a", "sum_b")]
                 d["rb"], d["n_strips"], d["n_cb"] = ws.rb, ws.n_strips, ws.n_cb
                 if in_atiles:
@@ -549,9 +551,9 @@ class LoPlan:
             X, Y = int(tdesc["X"][i]), int(tdesc["Y"][i])
             if tdesc["mode"][i] == L.MODE_KERNEL and self.tensor_cores:
                 kernel.append((unit_of[i], X, Y * int(tdesc["I"][i])))
-            if not tdesc["h_a"][i]:
+            if tdesc["mode"][i] != L.MODE_FAST2D and not tdesc["h_a"][i]:
                 continue
-            if not self.tensor_cores:   # the tensor-core kernel reads no tables
+            if tdesc["h_a"][i]:   # the tables' parts
                 pitems.append(atile_grid(unit_of[i], (X + per - 1) // per + (Y + per - 1) // per, 1)[1:])
             (fast if tdesc["mode"][i] == L.MODE_FAST2D else ragged).append((unit_of[i], X, Y))
         tiled = {u for u, _, _ in fast + ragged + kernel}

@@ -1,6 +1,10 @@
 """Workspace sizes follow from what a family's kernels read."""
 
+import pytest
+import torch
+
 from pylo_b200 import _lib as L
+from pylo_b200 import models, optim
 
 
 def test_the_folded_network_is_as_long_as_the_family_needs():
@@ -10,3 +14,15 @@ def test_the_folded_network_is_as_long_as_the_family_needs():
     for family, hidden in ((L.FAM_CELO2, 8), (L.FAM_VELO, 4)):
         network = 30 * hidden + hidden + hidden * hidden + hidden + 2 * hidden + 2   # the two outputs that are used
         assert network + 30 <= floats[family] < 2 * network + 64
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["3xtf32", "fp32"])
+def test_tables_only_where_a_sweep_reads_them(precision):
+    p = torch.nn.Parameter(torch.zeros(600, 260, device="cuda"))
+    p.grad = torch.ones_like(p)
+    opt = optim.AdafacLO_CUDA([p], network=models.MetaMLP(39, 32, 1), mlp_precision=precision)
+    opt.step()
+    (_, plan), = opt._plans.values()
+    tables = [bool(plan.tdesc.host[f][0]) for f in ("h_a", "h_b")]
+    assert tables == [precision == "fp32"] * 2
