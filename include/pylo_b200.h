@@ -479,7 +479,10 @@ int pylo_b200_velo_loss_features(float* means, int32_t* iteration, float* runnin
 #define PYLO_STEP_APPLY_REST 64
 #define PYLO_STEP_FRONT (PYLO_STEP_SUMS | PYLO_STEP_FACTORS | PYLO_STEP_STATE | PYLO_STEP_MOMENTS)
 #define PYLO_STEP_BACK (PYLO_STEP_PREP | PYLO_STEP_APPLY | PYLO_STEP_APPLY_REST)
-#define PYLO_ROWCOL_ONE_LAUNCH 2368 /* items of rowcol_sums up to which the GENERIC tensors' items join their launch (KERNEL items: always) */
+#define PYLO_ROWCOL_ONE_LAUNCH 2368 /* items of rowcol_sums on FAST2D tensors up to which the GENERIC tensors' items join their launch */
+#define PYLO_ROWCOL_KERNEL_APART 2960 /* the same where there are KERNEL items, with which the GENERIC tensors' go in either case: one or two \
+                                       convolution weights beside matrices of 300 M elements (9216 items) 320 us joined, 261 apart; 85 M \
+                                       (3168) 111 / 105; 31 M (3840) 60 / 60; 25 M (3072) 66 / 65; 21 M (2560) 47.5 / 49.8 */
 #define PYLO_TC_ONE_LAUNCH 4736 /* items on FAST2D units below which one launch of apply_adafac_tc takes both kinds of items: \
                                   the variant that takes both is 2 % slower on FAST2D items (ViT-B/16 2700 / 2751 us per \
                                   step, two Llama-3-8B blocks 12640 / 12925), a launch more costs about 10 us (convolutions \

@@ -178,7 +178,8 @@ TC_GEN_ITEM = 1 << 16  # tag bit of its items on tensors that are not FAST2D
 STEP_SUMS, STEP_FACTORS, STEP_STATE, STEP_MOMENTS, STEP_PREP, STEP_APPLY, STEP_APPLY_REST = (1 << k for k in range(7))
 STEP_FRONT = STEP_SUMS | STEP_FACTORS | STEP_STATE | STEP_MOMENTS
 STEP_BACK = STEP_PREP | STEP_APPLY | STEP_APPLY_REST
-ROWCOL_ONE_LAUNCH = 2368  # items of rowcol_sums up to which the GENERIC tensors' items join their launch
+ROWCOL_ONE_LAUNCH = 2368  # items of rowcol_sums on FAST2D tensors up to which the GENERIC tensors' items join their launch
+ROWCOL_KERNEL_APART = 2960  # the same where there are KERNEL items
 TC_ONE_LAUNCH = 8 * TC_WORKERS  # FAST2D items below which one launch of the tensor-core kernel takes both kinds of items
 BULK_COPY_ELEMS = 1 << 26  # FAST2D elements from which the state sweep reads through a ring of bulk copies
 SMALL_SLICE, SMALL_FLOATS = 8192, 52224   # of pylo_b200_small_front: elements of a CTA's rows, floats of shared memory

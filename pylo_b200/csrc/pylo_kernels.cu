@@ -2950,12 +2950,12 @@ int pylo_b200_rowcol_sums(const pylo_tensor_desc* descs, const pylo_atile* atile
   const pylo_atile* fast = atiles + n_ragged;
   const int n_fast = n_atiles - n_ragged;
   if (n_ragged > 0) launch(k_rowcol_fast<false, false>, grid_for(n_ragged, 3), NT, 0, s, descs, atiles, n_ragged, gitems, 0, *prm);
-  if (n_kernel > 0 || (n_gitems > 0 && n_fast > 0 && n_fast <= PYLO_ROWCOL_ONE_LAUNCH)) {
-    launch(k_rowcol_fast<true, true>, n_gitems + grid_for(n_fast, 3), NT, 0, s, descs, fast, n_fast, gitems, n_gitems, *prm);
-  } else {
-    if (n_fast > 0) launch(k_rowcol_fast<true, false>, grid_for(n_fast, 4), NT, 0, s, descs, fast, n_fast, gitems, 0, *prm);
-    if (n_gitems > 0) launch(k_rowcol_generic, n_gitems, NT, 0, s, descs, gitems, *prm);
-  }
+  // how many of the aligned items go with the variant that takes KERNEL and GENERIC tensors along: all of a small model's, else the KERNEL ones
+  const int most = n_kernel > 0 ? PYLO_ROWCOL_KERNEL_APART : PYLO_ROWCOL_ONE_LAUNCH;
+  const int mixed = n_fast - n_kernel > most ? n_kernel : n_kernel > 0 || n_gitems > 0 ? n_fast : 0;
+  if (mixed > 0) launch(k_rowcol_fast<true, true>, n_gitems + grid_for(mixed, 3), NT, 0, s, descs, fast, mixed, gitems, n_gitems, *prm);
+  else if (n_gitems > 0) launch(k_rowcol_generic, n_gitems, NT, 0, s, descs, gitems, *prm);
+  if (n_fast > mixed) launch(k_rowcol_fast<true, false>, grid_for(n_fast - mixed, 4), NT, 0, s, descs, fast + mixed, n_fast - mixed, gitems, 0, *prm);
   return launch_status();
 }
 

@@ -687,9 +687,11 @@ class LoPlan:
         apply.insert(0 if self.tensor_cores else 1, (L.STEP_APPLY_REST, other, rest))
         if self.family == L.FAM_VELO and (self.n_ctiles or self.n_rtiles):   # the packed sweep takes the other units' tiles along
             apply = [(L.STEP_APPLY | L.STEP_APPLY_REST, self.apply_kernel, int(self.n_ctiles > 0) + int(self.n_rtiles > 0))]
-        fast = self.n_atiles - self.n_ragged
-        joined = self.step_plan.n_kernel > 0 or 0 < fast <= L.ROWCOL_ONE_LAUNCH   # the generic items go with the others
-        front = [(L.STEP_SUMS, "rowcol_sums", (self.n_ragged > 0) + (fast > 0) + int(self.n_gitems > 0 and not joined)),
+        kernel = self.step_plan.n_kernel
+        fast = self.n_atiles - self.n_ragged - kernel
+        mixed = kernel > 0 or self.n_gitems > 0
+        joined = mixed and 0 < fast <= (L.ROWCOL_KERNEL_APART if kernel else L.ROWCOL_ONE_LAUNCH)   # all kinds of items in one launch
+        front = [(L.STEP_SUMS, "rowcol_sums", (self.n_ragged > 0) + int(mixed) + int(fast > 0 and not joined)),
                  (L.STEP_FACTORS, "factor_update", int(self.step_plan.n_mats > 0)),
                  (L.STEP_STATE, "state_moments", 1)]
         if self.small:
