@@ -300,7 +300,7 @@ int pylo_b200_apply_adafac_cols(const pylo_tensor_desc* descs, const pylo_atile*
  * give an infinity.  ttiles: strip = row-strip index, cb = block of 128 columns, pad_ = rows per work item (one
  * warpgroup of a CTA takes a whole item).  Units that are neither FAST2D nor KERNEL: pad_ = 0x10000 | tiles per work item, strip = item
  * index, cb = 0; an item is that many runs of 128 consecutive elements; generic != 0 says that the list may hold such
- * items.  status: device int; the kernel ORs 1 into it if a wait on the tensor
+ * items, or items on KERNEL units; no_tables = 4 is refused without it.  status: device int; the kernel ORs 1 into it if a wait on the tensor
  * core ran out (the parameters it could not finish then keep their old values), and a launch that finds it
  * non-zero stores nothing; may be NULL.  host_status: a word of pinned (device-accessible) host memory that both events
  * are also written to, so that the host can look without asking the device; may be NULL. */

@@ -3059,6 +3059,7 @@ int pylo_b200_apply_adafac_tc(const pylo_tensor_desc* descs, const pylo_atile* t
                               const pylo_step_params* prm, int* status, int* host_status, void* stream) {
   CHECK_ARG(descs && ttiles && prm && n_ttiles >= 0 && prm->family == PYLO_FAM_ADAFAC);
   if (n_ttiles == 0) return 0;
+  CHECK_ARG(generic || prm->no_tables != 4);   // the other variant makes no scales
   // more than half an SM's shared memory is requested: one CTA per SM, which then owns all of the SM's tensor memory
   constexpr int smem = sizeof(TcSmem) > 120 * 1024 ? (int)sizeof(TcSmem) : 120 * 1024;
   static bool configured[4][PYLO_MAX_DEVICES] = {};
