@@ -457,8 +457,8 @@ int pylo_b200_velo_tensor_features(const pylo_tensor_desc* descs, int n_local, c
                                    int n_total, const float* rank_onehot, float fraction,
                                    const pylo_velo_loss* lossbuf, float* x_in, void* stream);
 int pylo_b200_velo_rnn(const pylo_velo_rnn* rnn, const pylo_velo_loss* lossbuf, void* stream);
-/* velo_tensor_features and the first layer of velo_rnn in one launch, for all (up to 16) tensors of a model, of up to 16 tiles each, and H a
- * multiple of 128 up to 512; velo_rnn with mixed = 1 comes next. */
+/* velo_tensor_features and the first layer of velo_rnn in one launch, for all (up to 16) tensors of a model (made for up to 16 tiles each: every
+ * CTA adds them all up; the same sums to the last bit up to 20), and H a multiple of 128 up to 512; velo_rnn with mixed = 1 comes next. */
 int pylo_b200_velo_inputs(const pylo_tensor_desc* descs, const int32_t* layer_of, const float* rank_onehot, float fraction,
                           const pylo_velo_loss* lossbuf, const pylo_velo_rnn* rnn, void* stream);
 /* The loss buffer's update and features alone, for a host with a front end of its own: writes loss9[9]. */

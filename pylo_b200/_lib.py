@@ -170,7 +170,7 @@ lib, EXPORTED = _load()
 
 
 SM_COUNT = 148        # of a B200; sizes of work lists only, the kernels ask the device
-VELO_INPUTS_MOST = 16  # tensors that pylo_b200_velo_inputs takes, and their tiles
+VELO_INPUTS_MOST = 16  # tensors that pylo_b200_velo_inputs takes
 TAIL_ONE_LAUNCH = 592  # tiles of CELO2's tail and AdamW up to which they share a launch
 FACTOR_CLUSTER = 8  # CTAs per tensor of pylo_b200_factor_update
 TC_WORKERS = SM_COUNT * 4  # warpgroups the tensor-core apply kernel runs at once (four per SM)

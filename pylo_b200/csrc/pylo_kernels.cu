@@ -2270,7 +2270,7 @@ __global__ void __launch_bounds__(NT) k_velo_xmix(const pylo_velo_rnn r, const p
   for (int t = lane; t < r.T; t += 32) r.xmix[(int64_t)t * r.H + h] += best;
 }
 
-// The two above in one launch for small models (up to VI_TENSORS tensors of up to VI_TILES tiles): every CTA makes all tensors' inputs for itself,
+// The two above in one launch for small models (up to VI_TENSORS tensors, best of up to VI_TILES tiles): every CTA makes all tensors' inputs for itself,
 // from sums in the order of unit_sum, and its eight hidden units' x'.  The loss buffer, which all CTAs read here, is written by
 // k_velo_lstm.  Latency-bound; in place of two launches: perceptron, us per step 44.4 -> 42.2.
 #define VI_TENSORS 16
@@ -2297,6 +2297,8 @@ __global__ void __launch_bounds__(NT) k_velo_inputs(const pylo_tensor_desc* __re
       double tot = 0.0;
 #pragma unroll
       for (int q = 0; q < VI_TILES; ++q) tot += (double)v[q];
+#pragma unroll 1
+      for (int q = VI_TILES; q < n; ++q) tot += (double)src[(int64_t)q * PYLO_STAT_STRIDE];   // none in the plans of small models
       tot += (double)d.closed[j];
       s_sum[t][j] = tot;
       if (blockIdx.x == 0) store_unit_sum(d, tot, j);
