@@ -144,19 +144,38 @@ def tile_elems(total: int, least: int, tiles_wanted: int) -> int:
     return e
 
 
-def state_tile(sizes: Sequence[int]) -> int:
+_TILES = np.arange(L.TILE_ELEMS, 0, -1024, dtype=np.int64)   # what a tile of the state sweep may have: multiples of a CTA's pass
+
+
+def state_tile(sizes: Sequence[int], alike: bool = False, slow: int = 0) -> int:
     """Elements per tile of the state sweep over units of these sizes: the multiple of 1024 (one pass of a CTA) with which the CTAs that
-    run at once, two per SM, are done first, where that saves a sixth over the power of two that gives four CTAs per SM a tile.  A
-    tile's start and its block reduction cost about a pass.  Two full turns are no gain (the CTAs of a turn start, read and reduce
-    together): 5 M parameters of convolutions 206.8 with the power of two, 214.9 us per step in two turns, 202.7 in three; VeLO on a
-    ViT of 5 M 174.5 and 185.7.  One turn or three: perceptrons 156.1 -> 146.0 (4 M), VeLO 295.0 -> 283.2 (11 M, odd sizes), CELO2 on
-    11 M 317.3 -> 305.0."""
-    n, at_once = np.asarray(sizes, dtype=np.int64), 2 * L.SM_COUNT
-    plain = tile_elems(int(n.sum()), 1024, 4 * L.SM_COUNT)
-    turns = {e: -(-int((-(-n // e)).sum()) // at_once) for e in range(L.TILE_ELEMS, 0, -1024)}
-    cost = lambda e: turns[e] * (e + 1024)
-    best = min([e for e in turns if turns[e] != 2 or e == plain], key=cost)
-    return best if cost(best) < 0.83 * cost(plain) else plain
+    run at once, two per SM, have least to do in their turns, where that saves a tenth over the power of two that gives four CTAs per
+    SM a tile.  A tile's start and its block reduction cost about three passes.
+
+    Units that are read element by element across inner axes take longer and, as a model's first tensors, come last: ``slow`` is the
+    largest such unit, and in one turn a tile that is no more than a part of it costs as much again.  Two turns
+    are the best number only where all units go the same way (``alike``).  us per step in one turn / two / three: VeLO on ViTs, 3.9 M 157 / 146 / 139,
+    2.9 M 133 / 125 / 119; AdafacLO on convolutions, 4.7 M - / 174 / 163, 2.7 M 121 / 129 / 124.  Alike: VeLO on transformers, 5.3 M
+    - / 146 / 152, 4.8 M - / 132 / 138, AdafacLO on 8.6 M - / 287 / 293, CELO2 on perceptrons of 4.5 M 162 / 162 / 163.  Over 202 models of
+    all kinds from 0.4 to 50 M a step takes 0.87 to 1.02 of what it took with whole turns for all kinds alike (saving a sixth, a pass for the
+    start, never two turns), 0.90 to 1.02 of what it takes with the power of two, and 0.6 % more than with the best tile; over 60 further
+    ones 0.86 to 1.04 and 0.92 to 1.03."""
+    at_once, total = 2 * L.SM_COUNT, sum(sizes)
+    plain = tile_elems(total, 1024, 4 * L.SM_COUNT)
+    if not 0 < total <= 16 * at_once * L.TILE_ELEMS:   # more turns than a better last one would show in
+        return plain
+    n, e = np.asarray(sizes, dtype=np.int64), _TILES[:, None]
+    turns = -(-(-(-n // e)).sum(1) // at_once)
+    cost = turns * (_TILES + 3072)
+    if len(n) >= at_once:   # whole turns of units that are less than half a tile, CELO2's matrices: they cost what is in them
+        short = 2 * n < e
+        cost += (short * n).sum(1) // at_once - short.sum(1) // at_once * _TILES
+    if slow:
+        cost += (turns == 1) * (slow > _TILES) * _TILES
+    if not alike:
+        cost += (turns == 2) * (_TILES != plain) * cost[0]
+    best = int(cost.argmin())
+    return int(_TILES[best]) if cost[best] < 0.9 * cost[L.TILE_ELEMS // 1024 - plain // 1024] else plain
 
 
 def atile_grid(tensor: int, n_strips: int, n_cb: int, tag: int = 0) -> np.ndarray:
@@ -361,7 +380,13 @@ def sum_order(family: int, d: np.ndarray, sizes: Sequence[int], modes: np.ndarra
         vectors = d["mode"] == L.MODE_VEC1D
         if (vectors | plain_matrices(d)).all():
             small = small_front(list(zip(d["X"][~vectors].tolist(), d["Y"][~vectors].tolist())), d["n"][vectors].tolist())
-    elems = state_tile(sizes)
+    elems = L.TILE_ELEMS
+    if small is None:
+        across = modes == L.MODE_GENERIC   # inner axes between an element and the next of its row
+        if across.any() and not sliced:
+            across &= ~plain_matrices(d)
+        slow = max([sizes[u] for u in np.flatnonzero(across)], default=0)
+        elems = state_tile(sizes, not slow and not (modes == L.MODE_KERNEL).any(), slow)
     most = small[0] if small else -(-max(sizes, default=0) // elems)
     fast = int(sum(n for n, m in zip(sizes, modes.tolist()) if m == L.MODE_FAST2D))
     together = int((d["mode"] != L.MODE_VEC1D).sum()) * L.FACTOR_CLUSTER <= L.SM_COUNT
