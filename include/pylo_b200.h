@@ -295,8 +295,10 @@ int pylo_b200_apply_adafac_cols(const pylo_tensor_desc* descs, const pylo_atile*
  * reference evaluates the network with scalar FMAs, lo_kernel_apply learned_optimizer.cu:236-284).  Same outputs
  * as pylo_b200_apply_adafac_cols; it reads no first-layer tables, but the operands that pylo_b200_prep_apply makes
  * with no_tables = 2 or 0.  The two hidden layers run as tcgen05 products of
- * operands split into a high and a low fp16 plane of a common power-of-two scale (hi x hi + hi x lo + lo x hi), which keeps a 32-term dot
- * product within ~3e-7 of the sum of its terms' magnitudes; non-finite features give NaN where the scalar path may
+ * operands split into a high and a low fp16 plane (hi x hi + hi x lo + lo x hi), features scaled by one power of two and every hidden unit
+ * by one of its own, which keeps a 32-term dot product within ~3e-7 of the sum of its terms' magnitudes, whatever the units' scales, with a
+ * floor under a feature's magnitude: 2^-(25 + q) of its root mean square over the unit, 2^q sqrt(n) <= 2^15 and q <= 6 (2^-27 at 16 M
+ * elements).  A feature that is not a number or infinite makes the element's hidden activations zero, where the scalar path may
  * give an infinity.  ttiles: strip = row-strip index, cb = block of 128 columns, pad_ = rows per work item (one
  * warpgroup of a CTA takes a whole item).  Units that are neither FAST2D nor KERNEL: pad_ = 0x10000 | tiles per work item, strip = item
  * index, cb = 0; an item is that many runs of 128 consecutive elements; generic != 0 says that the list may hold such

@@ -19,7 +19,7 @@
 //   * a layer's last product is of a constant operand A (in shared memory) with a block that holds the bias; the tensor
 //     core scales the sums before it by 2^-TC_SHIFT.  A tile takes 7 + 7 products of width 32 (K = 16).  TF32 planes took 22
 //     (K = 8), twice the operand stores, and the row's features through operand B: 8192 x 4096 elements 714 -> 678 us, step over ViT-B/16
-//     2760 -> 2378, two Llama blocks 12610 -> 11320; the movement's error against fp64 is half of what it was
+//     2647 -> 2287, two Llama blocks 12770 -> 11480 (one GPU, in turn); the movement's error against fp64 is half of what it was
 //     (4096 x 4096, normal gradients: 1.6e-7 -> 0.9e-7 rms);
 //   * other tensors (ragged rows, vectors, odd convolutions) are taken as 128 consecutive elements that
 //     may lie in several rows (GEN items): their twelve vector features are made per element (the scalar kernel that took them before needed 752
@@ -47,7 +47,8 @@
 
 #ifndef TC_WGS
 // Warpgroups per CTA.  More hide more of a tile's chain, but have fewer registers each (six: 80), and at the power limit instructions
-// per element count: us per step with 3, 4, 5, 6: ViT-B/16 2643, 2533, 2757, 2668, two Llama blocks 12530, 11926, 12740, 12625.
+// per element count: us per step with 3, 4, 5, 6 (the first version on fp16 planes): ViT-B/16 2643, 2533, 2757, 2668, two Llama blocks
+// 12530, 11926, 12740, 12625.
 #define TC_WGS 4
 #endif
 #define TC_NT (TC_WGS * 128)

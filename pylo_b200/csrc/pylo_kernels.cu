@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(NT) k_prep_apply(const pylo_tensor_desc* __res
   // the table entries of this item: of the "a" or of the "b" index
   const int La = d.X, Lb = d.Y, items_a = (La + PER - 1) / PER;
   const bool tables = d.h_a && prm.no_tables != 1, of_a = it.strip < items_a;
-  const int i0 = (of_a ? it.strip : it.strip - items_a) * PER, end = tables && (of_a || prm.no_tables != 2) ? min(of_a ? La : Lb, i0 + PER) : 0;
+  const int i0 = (of_a ? it.strip : it.strip - items_a) * PER, end = tables ? min(of_a ? La : Lb, i0 + PER) : 0;
   for (int e = tid; e < 3 * PER; e += NT) {
     const int k = e / PER, i = i0 + e % PER;
     if (i < end) copy(&s_fac[k][i - i0], (of_a ? d.fac_a + (int64_t)k * La : d.fac_b + (int64_t)k * Lb) + i);

@@ -18,7 +18,8 @@ coordinates.
 evaluated on factored 2-D tensors: ``"3xtf32"`` (default) as tcgen05 tensor-core
 products with every operand split into a high and a low fp16 plane, three
 products per layer, which reproduces the fp32 result to ~3e-7 of a dot
-product's magnitude; ``"fp32"`` as scalar fp32 FMAs on the CUDA cores, the
+product's magnitude whatever the hidden units' scales (features below 2^-27
+of their root mean square, at 16 M elements, count as zero); ``"fp32"`` as scalar fp32 FMAs on the CUDA cores, the
 arithmetic of the reference kernel.  Both meet the same parity bounds.
 """
 
