@@ -173,7 +173,7 @@ __device__ __forceinline__ void tc_split2(uint64_t x, uint32_t& hi, uint32_t& lo
   else asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
   const float2 cut = __half22float2(*reinterpret_cast<const __half2*>(&hi));
   float ra, rb;
-  unpack2(add2(x, pack2(-cut.x, -cut.y)), ra, rb);
+  unpack2(fma2(pack2(cut.x, cut.y), pack2(-1.f, -1.f), x), ra, rb);   // exact
   if constexpr (RELU) asm("cvt.rn.relu.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(rb), "f"(ra));
   else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(rb), "f"(ra));
 }
