@@ -75,9 +75,17 @@ def geometry(shape: Sequence[int], fdims):
     return O, X, M, Y, I, int(dr == ay)
 
 
-def fill_geometry(d, shape: Sequence[int], fdims, rcm_axis: int, sliced: bool = False, tensors=()):
+#: how much of its blocks of 128 columns a convolution weight has to fill for the tensor-core sweep to take it as a matrix (a block's
+#: empty lanes cost what full ones do), and from which size on: small ones are all latency, and fewer launches as matrices.  AdafacLO, 60 tensors of 50 K
+#: elements, (n, c, 3, 3), us per step as matrices / the general way: c = 8 (0.56 full) 220 / 195, 16 (0.56) 200 / 188, 20 (0.70) 166 / 183,
+#: 32 (0.75) 156 / 180, 24 (0.84) 149 / 176, 64 (0.90) 138 / 175; (n, 20, 2, 2) (0.63) 210 / 188; of 17 K elements 101 / 94, 96 / 91, 85 / 86;
+#: 32 of (64, 16, 3, 3) 44 / 52
+KERNEL_FULL, KERNEL_FULL_FROM = 2 / 3, 32768
+
+
+def fill_geometry(d, shape: Sequence[int], fdims, rcm_axis: int, sliced: bool = False, tensors=(), full: float = 0.0):
     """The descriptor fields of a tensor of this shape that say how it is walked through; ``sliced``: its features are
-    normalised per matrix, ``tensors``: what has to be aligned for the fast mode.  Returns its (O, X, M, Y, I) and whether the mode
+    normalised per matrix, ``tensors``: what has to be aligned for the fast mode, ``full``: see KERNEL_FULL.  Returns its (O, X, M, Y, I) and whether the mode
     is FAST2D, or None for fewer than 2 dims."""
     d["n"] = n = _prod(shape)
     if fdims is None:
@@ -97,7 +105,7 @@ def fill_geometry(d, shape: Sequence[int], fdims, rcm_axis: int, sliced: bool = 
     fast = vec and I == 1
     # convolution weights of at least half a block of 128 columns: matrices whose row vectors have an entry per position (5 M parameters
     # of 3x3 convolutions, AdafacLO, us per step 275 -> 228: state 60 -> 46, network 160 -> 128; 205 with the sums in one launch)
-    kernel = vec and 1 < I <= 32 and Y * I >= 64
+    kernel = vec and 1 < I <= 32 and Y * I >= 64 and (n < KERNEL_FULL_FROM or Y * I >= full * 128 * -(-Y * I // 128))
     d["mode"] = L.MODE_FAST2D if fast else L.MODE_KERNEL if kernel else L.MODE_GENERIC
     return O, X, M, Y, I, fast
 
@@ -427,6 +435,7 @@ class LoPlan:
         self.device = torch.device(device)
         T = len(tensors)
         H = self.H[family]
+        full = KERNEL_FULL if self.tensor_cores else 0.0
         tdesc = np.zeros(T, dtype=L.DESC_DTYPE)
         ws_items = []  # (table, row, field, count)
         atiles, ratiles, katiles, gitems = [], [], [], []
@@ -443,7 +452,7 @@ class LoPlan:
             d = tdesc[i]
             d["m_stride"], d["idx0"] = n, 0
             sliced = t.slice_last2 and len(shape) > 2
-            sides = fill_geometry(d, shape, t.fdims, t.rcm_axis, sliced, (t.p, t.m, t.v, t.out))
+            sides = fill_geometry(d, shape, t.fdims, t.rcm_axis, sliced, (t.p, t.m, t.v, t.out), full)
             d["lr"], d["wd"], d["clip_norm"] = t.lr, t.wd, t.clip_norm
             d["exp_mult"], d["step_mult"] = t.exp_mult, t.step_mult
             d["p"], d["m"], d["v"] = t.p.data_ptr(), t.m.data_ptr(), t.v.data_ptr()
@@ -520,7 +529,7 @@ class LoPlan:
         else:
             whole = np.zeros(len(model), dtype=L.DESC_DTYPE)
             for d, (shape, fdims, rcm_axis) in zip(whole, model):
-                fill_geometry(d, shape, fdims, rcm_axis)   # the other ranks' buffers are aligned
+                fill_geometry(d, shape, fdims, rcm_axis, full=full)   # the other ranks' buffers are aligned
             order = sum_order(family, whole, whole["n"].tolist(), whole["mode"], False)
         self.small = order.small   # as many tiles a tensor as CTAs take its rows
         tiles, ranges = order.tiles(sizes)
