@@ -49,7 +49,7 @@ APPLY_BYTES = 28
 B_BYTES = 40  # state_moments sweep: reads g, p, m(3), v; writes m(3), v
 # DRAM bytes per element (dram__bytes_read.sum + dram__bytes_write.sum) of the dominant kernels: CONSTANTS taken
 # from ncu captures of a 4096 x 4096 case, not measured in this run; traffic grows in proportion to the elements
-NCU_TRAFFIC_PER_ELEM = {"k_apply_adafac_cols": 27.58, "k_apply_adafac_tc": 27.44}
+NCU_TRAFFIC_PER_ELEM = {"k_apply_adafac_cols": 27.58, "k_apply_adafac_tc": 27.42}
 # fp16 multiply-adds the tensor-core apply kernels issue per parameter (products x N x K, M = the element)
 TC_ISSUED_FMA_PER_PARAM = {"3xtf32": 14 * 32 * 16}   # 14 products of N = 32, K = 16 per element row
 

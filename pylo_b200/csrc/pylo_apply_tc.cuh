@@ -35,10 +35,10 @@
 //     a branch on the thread index, each product cost its thread ~52 cycles; this way ~24.
 //   * the output layer, one network's for all units, is an argument of the launch: read from shared memory, with no registers
 //     to ask ahead, each pair of units waited for its weights (the heads took 700 of a tile's 2970 cycles, as an argument 500).
-// What bounds it: issue slots (367 instructions per element, 62 % of the slots) and the latency of a tile's stages, one serial chain of
-// 2630 cycles with four tiles per SM in flight, one per warpgroup (features 356, operand stores and next row's requests 158, first products
-// 439, relu and split 414, second products 438, heads and store 525, waits and barriers 79, loop 110); on large models the GPU's power
-// limit.  Tensor pipe 38 %, ALU pipe 51 %, DRAM 19 %.
+// What bounds it: issue slots (386 instructions per element, 66 % of the slots) and the latency of a tile's stages, one serial chain of
+// 2500 cycles with four tiles per SM in flight, one per warpgroup (features 292, operand stores and next row's requests 169, first products
+// 403, relu and split 424, second products 407, heads and store 523, waits and barriers 85, loop 110); on large models the GPU's power
+// limit.  Tensor pipe 38 %, ALU pipe 38 %, fma pipe 41 %, DRAM 19 %.
 // Every wait on the tensor core is bounded.  A thread whose wait ran out records it in *status (and in *host_status, a word
 // of pinned host memory that the host looks at without asking the device), stops waiting
 // and stops storing (its parameters, and their copies on the peers, keep their old values), and goes on to
